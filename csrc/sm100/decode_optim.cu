@@ -1,12 +1,5 @@
 // Small kernels of the RL loop.
 //
-//   attention_decode: one new query token per sequence against a KV cache (rollout phase).
-//       One CTA per (sequence, KV head): the query heads of a GQA group share every K / V
-//       load. Scores: a warp per key, lanes over the head dimension. Output: the keys are cut
-//       into four interleaved sets, each thread owns two output dimensions of one set, and the
-//       four partial sums are added in a fixed order, so the result does not depend on the
-//       batch. (Groups that are not 1, 2, 4 or 8 heads wide take the older one-CTA-per-head
-//       kernel.)
 //   decode_qkv_rope_cache: what lies between the fused qkv projection and attention in a decode
 //       step, in one launch: split q / k / v, rotate q and k, write k and v into the cache slot.
 //   adamw_step: fused AdamW update over a flat parameter group: bf16 parameter, fp32 master
@@ -17,173 +10,11 @@
 #include <cstdint>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
-#include <math_constants.h>
-
-#include "common/ptx.cuh"
 
 namespace ka {
 namespace {
 
 constexpr int kD = 128;
-constexpr int kDecThreads = 128;
-constexpr float kLog2e = 1.4426950408889634f;
-
-// q: [B, Hq, D]; cache_k / cache_v: [B, max_len, Hkv, D]; lens[b]: valid keys (incl. the new
-// token); out: [B, Hq, D].
-__global__ void __launch_bounds__(kDecThreads)
-attention_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache_k,
-                        const __nv_bfloat16* __restrict__ cache_v, const int* __restrict__ lens,
-                        __nv_bfloat16* __restrict__ out, int hq, int hkv, int max_len, float scale) {
-  extern __shared__ float s_scores[];  // [max_len]
-  __shared__ float s_q[kD];
-  __shared__ float s_red[kDecThreads / 32];
-  const int b = blockIdx.x / hq, h = blockIdx.x % hq;
-  const int hk = h / (hq / hkv);
-  const int n = lens[b];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  s_q[tid] = __bfloat162float(q[(static_cast<size_t>(b) * hq + h) * kD + tid]);
-  __syncthreads();
-  const float c = scale * kLog2e;
-  // scores: one warp per key, lanes split the head dimension
-  float wmax = -CUDART_INF_F;
-  for (int j = warp; j < n; j += kDecThreads / 32) {
-    const __nv_bfloat16* kp = cache_k + ((static_cast<size_t>(b) * max_len + j) * hkv + hk) * kD;
-    float acc = 0.f;
-#pragma unroll
-    for (int t = 0; t < kD / 32; ++t) acc = __fmaf_rn(s_q[lane + 32 * t], __bfloat162float(kp[lane + 32 * t]), acc);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
-    if (lane == 0) s_scores[j] = acc;
-    wmax = fmaxf(wmax, acc);
-  }
-  if (lane == 0) s_red[warp] = wmax;
-  __syncthreads();
-  float m = s_red[0];
-  for (int w = 1; w < kDecThreads / 32; ++w) m = fmaxf(m, s_red[w]);
-  // probabilities; the normaliser is summed by one thread in key order
-  for (int j = tid; j < n; j += kDecThreads) s_scores[j] = ex2_approx(__fmul_rn(__fsub_rn(s_scores[j], m), c));
-  __syncthreads();
-  // output: thread d owns one element of the head dimension, keys in order
-  float acc = 0.f, l = 0.f;
-  for (int j = 0; j < n; ++j) {
-    const float p = s_scores[j];
-    l = __fadd_rn(l, p);
-    acc = __fmaf_rn(p, __bfloat162float(cache_v[((static_cast<size_t>(b) * max_len + j) * hkv + hk) * kD + tid]), acc);
-  }
-  out[(static_cast<size_t>(b) * hq + h) * kD + tid] = __float2bfloat16_rn(__fdiv_rn(acc, l));
-}
-
-// q: [B, Hq, D]; caches: [B, max_len, Hkv, D]; one CTA per (sequence, KV head), GQ = Hq / Hkv.
-constexpr int kGqaThreads = 256;
-constexpr int kKeySplits = 4;
-
-template <int GQ>
-__global__ void __launch_bounds__(kGqaThreads)
-attention_decode_gqa_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache_k,
-                            const __nv_bfloat16* __restrict__ cache_v, const int* __restrict__ lens,
-                            __nv_bfloat16* __restrict__ out, int hq, int hkv, int max_len, float scale) {
-  extern __shared__ float s_scores[];  // [GQ][max_len]
-  __shared__ float s_q[GQ][kD];
-  __shared__ float s_part[kKeySplits][GQ][kD];
-  __shared__ float s_l[kKeySplits][GQ];
-  __shared__ float s_max[kGqaThreads / 32][GQ];
-  const int b = blockIdx.x / hkv, hk = blockIdx.x % hkv;
-  const int n = lens[b];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const size_t kv_row = static_cast<size_t>(hkv) * kD;  // elements between consecutive keys
-  const __nv_bfloat16* kbase = cache_k + (static_cast<size_t>(b) * max_len * hkv + hk) * kD;
-  const __nv_bfloat16* vbase = cache_v + (static_cast<size_t>(b) * max_len * hkv + hk) * kD;
-  for (int i = tid; i < GQ * kD; i += kGqaThreads)
-    s_q[i / kD][i % kD] = __bfloat162float(q[(static_cast<size_t>(b) * hq + hk * GQ + i / kD) * kD + i % kD]);
-  __syncthreads();
-
-  // ---- scores: warp w takes keys w, w + 8, ...; lane l holds dimensions 4l .. 4l + 3
-  float qr[GQ][4], wmax[GQ];
-#pragma unroll
-  for (int g = 0; g < GQ; ++g) {
-    wmax[g] = -CUDART_INF_F;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) qr[g][e] = s_q[g][4 * lane + e];
-  }
-#pragma unroll 4
-  for (int j = warp; j < n; j += kGqaThreads / 32) {
-    const uint2 raw = *reinterpret_cast<const uint2*>(kbase + j * kv_row + 4 * lane);
-    const __nv_bfloat162 k01 = *reinterpret_cast<const __nv_bfloat162*>(&raw.x);
-    const __nv_bfloat162 k23 = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
-    const float kf[4] = {__bfloat162float(k01.x), __bfloat162float(k01.y), __bfloat162float(k23.x),
-                         __bfloat162float(k23.y)};
-    float acc[GQ];
-#pragma unroll
-    for (int g = 0; g < GQ; ++g) {
-      float a = __fmul_rn(qr[g][0], kf[0]);
-      a = __fmaf_rn(qr[g][1], kf[1], a);
-      a = __fmaf_rn(qr[g][2], kf[2], a);
-      a = __fmaf_rn(qr[g][3], kf[3], a);
-      acc[g] = a;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int g = 0; g < GQ; ++g) acc[g] = __fadd_rn(acc[g], __shfl_xor_sync(0xffffffffu, acc[g], o));
-    if (lane == 0) {
-#pragma unroll
-      for (int g = 0; g < GQ; ++g) s_scores[g * max_len + j] = acc[g];
-    }
-#pragma unroll
-    for (int g = 0; g < GQ; ++g) wmax[g] = fmaxf(wmax[g], acc[g]);
-  }
-  if (lane == 0) {
-#pragma unroll
-    for (int g = 0; g < GQ; ++g) s_max[warp][g] = wmax[g];
-  }
-  __syncthreads();
-  const float c = scale * kLog2e;
-#pragma unroll
-  for (int g = 0; g < GQ; ++g) {
-    float m = s_max[0][g];
-#pragma unroll
-    for (int w = 1; w < kGqaThreads / 32; ++w) m = fmaxf(m, s_max[w][g]);
-    for (int j = tid; j < n; j += kGqaThreads)
-      s_scores[g * max_len + j] = ex2_approx(__fmul_rn(__fsub_rn(s_scores[g * max_len + j], m), c));
-  }
-  __syncthreads();
-
-  // ---- output: thread = (key set, dimension pair); a key set is j = set, set + 4, ...
-  const int d2 = tid & 63, set = tid >> 6;
-  float acc[GQ][2], l[GQ];
-#pragma unroll
-  for (int g = 0; g < GQ; ++g) {
-    acc[g][0] = 0.f;
-    acc[g][1] = 0.f;
-    l[g] = 0.f;
-  }
-#pragma unroll 8
-  for (int j = set; j < n; j += kKeySplits) {
-    const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(vbase + j * kv_row + 2 * d2);
-    const float v0 = __bfloat162float(v.x), v1 = __bfloat162float(v.y);
-#pragma unroll
-    for (int g = 0; g < GQ; ++g) {
-      const float p = s_scores[g * max_len + j];
-      l[g] = __fadd_rn(l[g], p);
-      acc[g][0] = __fmaf_rn(p, v0, acc[g][0]);
-      acc[g][1] = __fmaf_rn(p, v1, acc[g][1]);
-    }
-  }
-#pragma unroll
-  for (int g = 0; g < GQ; ++g) {
-    s_part[set][g][2 * d2] = acc[g][0];
-    s_part[set][g][2 * d2 + 1] = acc[g][1];
-    if (d2 == 0) s_l[set][g] = l[g];
-  }
-  __syncthreads();
-  for (int i = tid; i < GQ * kD; i += kGqaThreads) {
-    const int g = i / kD, d = i % kD;
-    const float a = __fadd_rn(__fadd_rn(s_part[0][g][d], s_part[1][g][d]), __fadd_rn(s_part[2][g][d], s_part[3][g][d]));
-    const float ls = __fadd_rn(__fadd_rn(s_l[0][g], s_l[1][g]), __fadd_rn(s_l[2][g], s_l[3][g]));
-    out[(static_cast<size_t>(b) * hq + hk * GQ + g) * kD + d] = __float2bfloat16_rn(__fdiv_rn(a, ls));
-  }
-}
-
 // qkv: [B, (hq + 2 hkv) * 128] bf16 (row stride qkv_stride), the output of the fused projection.
 // pos [B]: position of the new token; slot [1]: cache row to write (both on the device, so a
 // CUDA graph can replay the launch). q_out [B, hq, 128] rotated; cache_k / cache_v
@@ -281,49 +112,6 @@ adamw_kernel(__nv_bfloat16* __restrict__ param, float* __restrict__ master, cons
 }  // namespace ka
 
 extern "C" {
-
-int ka_attention_decode(const void* q, const void* cache_k, const void* cache_v, const int* lens, void* out, int batch,
-                        int hq, int hkv, int head_dim, int max_len, float scale, void* stream) {
-  using namespace ka;
-  if (batch <= 0) return 0;
-  if (head_dim != kD || hq % hkv != 0 || max_len * 4 > 200 * 1024) return -1;
-  const int gq = hq / hkv;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if ((gq == 1 || gq == 2 || gq == 4 || gq == 8) && static_cast<long long>(gq) * max_len * 4 <= 160 * 1024) {
-    const int smem_g = gq * max_len * 4;
-    const __nv_bfloat16* qb = static_cast<const __nv_bfloat16*>(q);
-    const __nv_bfloat16* kb = static_cast<const __nv_bfloat16*>(cache_k);
-    const __nv_bfloat16* vb = static_cast<const __nv_bfloat16*>(cache_v);
-    __nv_bfloat16* ob = static_cast<__nv_bfloat16*>(out);
-    // the shared-memory opt-in is per device and cheap: set it on every call that needs it
-#define KA_LAUNCH_GQA(GQ)                                                                                       \
-  do {                                                                                                          \
-    if (smem_g > 40 * 1024 &&                                                                                   \
-        cudaFuncSetAttribute(attention_decode_gqa_kernel<GQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
-                             smem_g) != cudaSuccess)                                                            \
-      return -10;                                                                                               \
-    attention_decode_gqa_kernel<GQ><<<batch * hkv, kGqaThreads, smem_g, st>>>(qb, kb, vb, lens, ob, hq, hkv,    \
-                                                                               max_len, scale);                 \
-  } while (0)
-    if (gq == 1) KA_LAUNCH_GQA(1);
-    else if (gq == 2) KA_LAUNCH_GQA(2);
-    else if (gq == 4) KA_LAUNCH_GQA(4);
-    else KA_LAUNCH_GQA(8);
-#undef KA_LAUNCH_GQA
-    return cudaGetLastError() == cudaSuccess ? 0 : -11;
-  }
-  static int configured_bytes = 0;
-  const int smem = max_len * 4;
-  if (smem > 48 * 1024 && smem > configured_bytes) {
-    if (cudaFuncSetAttribute(attention_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return -10;
-    configured_bytes = smem;
-  }
-  attention_decode_kernel<<<batch * hq, kDecThreads, smem, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(cache_k),
-      static_cast<const __nv_bfloat16*>(cache_v), lens, static_cast<__nv_bfloat16*>(out), hq, hkv, max_len, scale);
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
-}
 
 // See decode_qkv_rope_cache_kernel. head_dim is 128.
 int ka_decode_qkv_rope_cache(const void* qkv, long long qkv_stride, const long long* pos, const long long* slot,

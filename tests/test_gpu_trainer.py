@@ -124,3 +124,30 @@ def test_grpo_step_is_bitwise_repeatable_and_resumable(cuda_device, tmp_path):
     assert lb0 == la[0]                       # run-to-run bitwise equal loss
     assert lc == la[1:]                       # resume reproduces the uninterrupted run
     assert la[0] != la[1] or la[1] != la[2]   # the policy actually moved
+
+
+@pytest.mark.parametrize("hq,hkv", [(4, 4), (4, 2), (8, 2), (8, 1), (6, 2)])
+def test_decode_attention_bits_do_not_depend_on_how_many_ctas_share_a_sequence(cuda_device, hq, hkv):
+    """A cluster of up to eight CTAs works on a (sequence, KV head), fewer in a large batch; the
+    decomposition of the keys is the same. Lengths around the block and stripe boundaries."""
+    lens = torch.tensor([1, 2, 15, 16, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1025],
+                        dtype=torch.int32, device=cuda_device)
+    g = torch.Generator(device=cuda_device).manual_seed(3)
+    n = lens.numel()
+    q = torch.randn(n, hq, 128, device=cuda_device, generator=g).to(torch.bfloat16)
+    ck = torch.randn(n, 1030, hkv, 128, device=cuda_device, generator=g).to(torch.bfloat16)
+    cv = torch.randn(n, 1030, hkv, 128, device=cuda_device, generator=g).to(torch.bfloat16)
+    out = attention_decode(q, ck, cv, lens)
+    ref = attention_decode(q.cpu().float(), ck.cpu().float(), cv.cpu().float(), lens.cpu())
+    # fp32 arithmetic, rounded once to bf16: half a unit in the last place of the largest value
+    assert (out.cpu().float() - ref).abs().max().item() <= 2 ** -8 * ref.abs().max().item()
+    for reps in (4, 30):
+        wide = attention_decode(q.repeat(reps, 1, 1), ck.repeat(reps, 1, 1, 1), cv.repeat(reps, 1, 1, 1), lens.repeat(reps))
+        assert torch.equal(wide.view(reps, n, hq, 128), out.expand(reps, n, hq, 128))
+    one = [attention_decode(q[i:i + 1], ck[i:i + 1], cv[i:i + 1], lens[i:i + 1]) for i in range(n)]
+    assert torch.equal(torch.cat(one), out)
+    # a cache that is not 16-byte aligned takes the general kernel
+    flat = torch.empty(ck.numel() + 1, dtype=torch.bfloat16, device=cuda_device)
+    flat[1:] = ck.reshape(-1)
+    off = attention_decode(q, flat[1:].view_as(ck), cv, lens)
+    assert (off.float() - out.float()).abs().max().item() <= 2 ** -7 * ref.abs().max().item()
