@@ -3,15 +3,20 @@
 //
 // With a handful of rows the product is a stream of the weight matrix, so the operands are
 // swapped: the WEIGHTS are the 128-row A operand of tcgen05.mma and the activations the narrow
-// B operand (N = the batch padded to 16 / 32 / 64), D^T[n, m] accumulating in TMEM. Every CTA
-// owns 128 weight rows and walks the whole K in one accumulation chain (no split-K: the order
-// of the sum over K is the one the tiled kernel uses, so a row's result does not depend on
-// which of the two kernels its batch size selects). Nearly all shared memory is a TMA ring of
-// weight tiles (11 stages x 16 KiB in flight per SM), which is what a memory-bound stream
-// needs. Measured: a CTA streams about 80 GB/s, bounded by load latency over that ring, so
-// shapes with N >= 128 x (number of SMs) run near the HBM rate and N = 4096 (32 CTAs) at about
-// a quarter of it; taking fewer weight rows per CTA did not help (the K loop then becomes
-// bound by the rate of MMA instructions), and splitting K would change the order of the sum.
+// B operand (N = the batch padded to 16 / 32 / 64), D^T[n, m] accumulating in TMEM. An output
+// element is one accumulation chain over K (no split-K: the order of the sum over K is the one
+// the tiled kernel uses, so a row's result does not depend on which of the two kernels its batch
+// size selects).
+//
+// What bounds it is the weight stream, and an SM pulls at most about 80 GB/s, so every SM has
+// to have its share of the rows: the N rows are cut into tiles of R rows (R a multiple of 8, at
+// most 128) such that the tiles fill the SMs evenly, N = 4096 into 128 tiles of 32 rows instead
+// of 32 tiles of 128. The MMA still reads 128 rows of shared memory; what lies behind a shorter
+// tile (the next stage, or slack at the end) only reaches accumulator rows that nobody stores.
+// A CTA walks its tiles persistently; the ring of 128-wide K blocks runs on across tiles and the
+// accumulator is double-buffered.
+// Measured, 8 rows (64 rows): the four products of a Llama-3-8B decoder layer (436 MB of weights)
+// take 98 us (110 us); with 128 weight rows per CTA everywhere they took 157 us (164 us).
 //
 // The reference has no GEMM of its own (it names backends in rl_engine/kernels/registry.py:41-55).
 #include <cstdint>
@@ -25,26 +30,18 @@ namespace ka {
 namespace {
 
 constexpr int kMmaRows = 128;  // M of the MMA (rows of shared memory it reads per K step)
-constexpr int kBK = 64;        // K per stage: one 128-byte swizzled row
+constexpr int kBox = 64;       // K columns of a TMA box: one 128-byte swizzled row
+constexpr int kBoxes = 2;      // boxes per stage
 constexpr int kThreads = 192;  // four epilogue warps, one TMA warp, one MMA warp
 constexpr int kMaxStages = 32;
-
-// NB: batch rows padded (the MMA's N); R: weight rows per CTA
-template <int NB, int R>
-struct Cfg {
-  static constexpr int kWBytes = R * kBK * 2;
-  static constexpr int kXBytes = NB * kBK * 2;
-  static constexpr int kStageBytes = kWBytes + kXBytes;
-  static constexpr int kStages = (196 * 1024) / kStageBytes > kMaxStages ? kMaxStages : (196 * 1024) / kStageBytes;
-  // slack: the MMA of the last stage reads kMmaRows rows starting at its (shorter) weight tile
-  static constexpr int kSlack = (kMmaRows - R) * kBK * 2;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kSlack + 1024 + 1024;
-};
+constexpr int kRingBytes = 192 * 1024;
+constexpr int kSmemBytes = kRingBytes + kMmaRows * kBox * 2 + 2048;   // ring, slack behind it, control
 
 struct Control {
   uint64_t full[kMaxStages];
   uint64_t empty[kMaxStages];
-  uint64_t acc_full;
+  uint64_t acc_full[2];
+  uint64_t acc_empty[2];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -53,38 +50,54 @@ struct SkinnyParams {
   __nv_bfloat16* out;   // [M, N], row stride ldc
   long long ldc;
   int m, n, k;
+  int tile_rows, n_tiles, stages;
   int* status;
   unsigned long long timeout_ns;
 };
 
-template <int NB, int R>
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
+// NB: batch rows padded (the MMA's N)
+template <int NB>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                    const __grid_constant__ SkinnyParams p) {
-  using C = Cfg<NB, R>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - raw_addr);
-  Control* ctl = reinterpret_cast<Control*>(smem + C::kStages * C::kStageBytes + C::kSlack);
+  Control* ctl = reinterpret_cast<Control*>(smem + kRingBytes + kMmaRows * kBox * 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * R;
-  const int num_kb = (p.k + kBK - 1) / kBK;
-  constexpr int kTmemCols = NB < 32 ? 32 : NB;
+  const int w_bytes = p.tile_rows * kBox * 2;                 // one box of the weight tile
+  constexpr int kXBytes = NB * kBox * 2;
+  const int box_bytes = w_bytes + kXBytes, stage_bytes = kBoxes * box_bytes;
+  const int n_boxes = (p.k + kBox - 1) / kBox, num_kb = (n_boxes + kBoxes - 1) / kBoxes;
+  constexpr int kTmemCols = 2 * NB < 32 ? 32 : 2 * NB;
 
   WaitCtx wctx{&ctl->abort_flag, p.status, p.timeout_ns};
   if (threadIdx.x == 0) {
-    for (int s = 0; s < C::kStages; ++s) {
+    for (int s = 0; s < p.stages; ++s) {
       mbar_init(smem_u32(&ctl->full[s]), 1);
       mbar_init(smem_u32(&ctl->empty[s]), 1);
     }
-    mbar_init(smem_u32(&ctl->acc_full), 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&ctl->acc_full[b]), 1);
+      mbar_init(smem_u32(&ctl->acc_empty[b]), 4);
+    }
     ctl->abort_flag = 0;
     fence_mbar_init_cluster();
   }
   if (warp == 5) {
     tmem_alloc<1>(smem_u32(&ctl->tmem_base), kTmemCols);
     tmem_relinquish<1>();
+  }
+  if (warp == 4 && lane == 0) {
+    tma_prefetch_desc(&tm_w);
+    tma_prefetch_desc(&tm_x);
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -93,58 +106,106 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 
   if (warp == 4) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      for (int kb = 0; kb < num_kb; ++kb) {
-        const int s = kb % C::kStages;
-        if (!mbar_wait_bounded(smem_u32(&ctl->empty[s]), ((kb / C::kStages) & 1) ^ 1u, wctx, 61, s)) break;
-        const uint32_t full = smem_u32(&ctl->full[s]);
-        const uint32_t wt = base + s * C::kStageBytes, xt = wt + C::kWBytes;
-        mbar_arrive_expect_tx(full, C::kStageBytes);
-        tma_load_2d(wt, &tm_w, kb * kBK, n0, full);
-        tma_load_2d(xt, &tm_x, kb * kBK, 0, full);
+    if (elect_one()) {
+      int s = 0;
+      uint32_t phase = 1;
+      bool ok = true;
+      for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
+        for (int kb = 0; kb < num_kb; ++kb) {
+          ok = mbar_wait_bounded(smem_u32(&ctl->empty[s]), phase, wctx, 61, s);
+          if (!ok) break;
+          const uint32_t full = smem_u32(&ctl->full[s]);
+          const uint32_t dst = base + s * stage_bytes;
+          const int boxes = min(kBoxes, n_boxes - kb * kBoxes);
+          mbar_arrive_expect_tx(full, boxes * box_bytes);
+          for (int x = 0; x < boxes; ++x) {
+            const int k0 = (kb * kBoxes + x) * kBox;
+            tma_load_2d(dst + x * w_bytes, &tm_w, k0, t * p.tile_rows, full);
+            tma_load_2d(dst + kBoxes * w_bytes + x * kXBytes, &tm_x, k0, 0, full);
+          }
+          if (++s == p.stages) {
+            s = 0;
+            phase ^= 1u;
+          }
+        }
       }
     }
   } else if (warp == 5) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_bf16_f32(kMmaRows, NB);
+    if (elect_one()) {
+      constexpr uint32_t idesc = umma_idesc_bf16_f32(kMmaRows, NB);
+      const uint64_t d0 = umma_desc_k_sw128(base);
+      int s = 0, i = 0;
+      uint32_t phase = 0;
       bool ok = true;
-      for (int kb = 0; kb < num_kb && ok; ++kb) {
-        const int s = kb % C::kStages;
-        ok = mbar_wait_bounded(smem_u32(&ctl->full[s]), (kb / C::kStages) & 1, wctx, 62, s);
+      for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x, ++i) {
+        const int b = i & 1;
+        ok = mbar_wait_bounded(smem_u32(&ctl->acc_empty[b]), ((i >> 1) & 1) ^ 1u, wctx, 64, i);
         if (!ok) break;
         tc_fence_after_sync();
-        const uint32_t wt = base + s * C::kStageBytes, xt = wt + C::kWBytes;
+        const uint32_t acc = tmem_base + static_cast<uint32_t>(b * NB);
+        for (int kb = 0; kb < num_kb; ++kb) {
+          ok = mbar_wait_bounded(smem_u32(&ctl->full[s]), phase, wctx, 62, s);
+          if (!ok) break;
+          tc_fence_after_sync();
+          const uint64_t dw = d0 + static_cast<uint64_t>((s * stage_bytes) >> 4);
+          const uint64_t dx = dw + static_cast<uint64_t>((kBoxes * w_bytes) >> 4);
+          const int boxes = min(kBoxes, n_boxes - kb * kBoxes);
 #pragma unroll
-        for (int k = 0; k < kBK / 16; ++k)
-          umma_bf16<1>(tmem_base, umma_desc_k_sw128(wt + k * 32), umma_desc_k_sw128(xt + k * 32), idesc,
-                       (kb > 0 || k > 0) ? 1u : 0u);
-        umma_commit<1>(smem_u32(&ctl->empty[s]));
+          for (int x = 0; x < kBoxes; ++x) {
+            if (x >= boxes) break;
+#pragma unroll
+            for (int k = 0; k < kBox / 16; ++k)
+              umma_bf16<1>(acc, dw + static_cast<uint64_t>((x * w_bytes) >> 4) + k * 2,
+                           dx + static_cast<uint64_t>((x * kXBytes) >> 4) + k * 2, idesc,
+                           (kb > 0 || x > 0 || k > 0) ? 1u : 0u);
+          }
+          umma_commit<1>(smem_u32(&ctl->empty[s]));
+          if (++s == p.stages) {
+            s = 0;
+            phase ^= 1u;
+          }
+        }
+        if (ok) umma_commit<1>(smem_u32(&ctl->acc_full[b]));
       }
-      if (ok) umma_commit<1>(smem_u32(&ctl->acc_full));
     }
   } else {
     // ------------------------------------------------------------------ epilogue
     // TMEM lane = weight row (output column n), TMEM column = batch row m.
-    const bool mine = mbar_wait_bounded(smem_u32(&ctl->acc_full), 0, wctx, 63, 0);
-    const bool ok = __all_sync(0xffffffffu, mine) != 0;
-    if (ok && warp * 32 < R) {
+    int i = 0;
+    for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x, ++i) {
+      const int b = i & 1;
+      const bool mine = mbar_wait_bounded(smem_u32(&ctl->acc_full[b]), (i >> 1) & 1, wctx, 63, i);
+      if (__all_sync(0xffffffffu, mine) == 0) break;
       tc_fence_after_sync();
-      const int n = n0 + warp * 32 + lane;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+      const int r = warp * 32 + lane, n = t * p.tile_rows + r;
+      const bool row_ok = r < p.tile_rows && n < p.n;
+      const uint32_t taddr = tmem_base + static_cast<uint32_t>(b * NB) + (static_cast<uint32_t>(warp * 32) << 16);
+      if (warp * 32 < p.tile_rows) {
 #pragma unroll
-      for (int c0 = 0; c0 < kTmemCols; c0 += 32) {
-        uint32_t v[32];
-        tmem_ld_32x32(taddr + c0, v);
-        tmem_ld_wait();
-        if (n < p.n) {
+        for (int c0 = 0; c0 < NB; c0 += 16) {
+          if (c0 >= p.m) break;
+          uint32_t v[16];
+          __syncwarp();
+          tmem_ld_32x16(taddr + c0, v);
+          // the wait names the registers, so that no use of them moves in front of it
+          asm volatile("tcgen05.wait::ld.sync.aligned;"
+                       : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                         "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]),
+                         "+r"(v[15])
+                       :
+                       : "memory");
+          if (row_ok) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int m = c0 + i;
-            if (m < p.m) p.out[static_cast<long long>(m) * p.ldc + n] = __float2bfloat16_rn(__uint_as_float(v[i]));
+            for (int j = 0; j < 16; ++j)
+              if (c0 + j < p.m)
+                p.out[static_cast<long long>(c0 + j) * p.ldc + n] = __float2bfloat16_rn(__uint_as_float(v[j]));
           }
         }
       }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&ctl->acc_empty[b]));
     }
   }
 
@@ -158,24 +219,32 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   }
 }
 
-template <int NB, int R>
-int launch(const void* a, long long lda, const void* w, long long ldw, const SkinnyParams& p, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gemm_skinny_kernel<NB, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             Cfg<NB, R>::kSmemBytes) != cudaSuccess)
-      return -10;
-    configured = true;
-  }
+template <int NB>
+int launch(const void* a, long long lda, const void* w, long long ldw, SkinnyParams p, cudaStream_t stream) {
+  if (cudaFuncSetAttribute(gemm_skinny_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) !=
+      cudaSuccess)
+    return -10;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+    return -12;
+  // Rows per tile: as many tiles as SMs, or a whole multiple of that when a tile would exceed the
+  // MMA's 128 rows, rounded up to the 8 rows of a swizzle atom.
+  const int rounds = (p.n + sms * kMmaRows - 1) / (sms * kMmaRows);
+  const int per = (p.n + sms * rounds - 1) / (sms * rounds);
+  p.tile_rows = (per + 7) / 8 * 8;
+  p.n_tiles = (p.n + p.tile_rows - 1) / p.tile_rows;
+  const int stage_bytes = kBoxes * (p.tile_rows + NB) * kBox * 2;
+  p.stages = kRingBytes / stage_bytes < kMaxStages ? kRingBytes / stage_bytes : kMaxStages;
   CUtensorMap tw, tx;
   int rc = make_tmap_2d_16bit_sw128(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, w, static_cast<uint64_t>(p.n),
-                                    static_cast<uint64_t>(p.k), ldw, R, kBK);
+                                    static_cast<uint64_t>(p.k), ldw, static_cast<uint32_t>(p.tile_rows), kBox);
   if (rc) return -20 + rc;
   rc = make_tmap_2d_16bit_sw128(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a, static_cast<uint64_t>(p.m),
-                                static_cast<uint64_t>(p.k), lda, NB, kBK);
+                                static_cast<uint64_t>(p.k), lda, NB, kBox);
   if (rc) return -40 + rc;
-  const unsigned grid = static_cast<unsigned>((p.n + R - 1) / R);
-  gemm_skinny_kernel<NB, R><<<grid, kThreads, Cfg<NB, R>::kSmemBytes, stream>>>(tw, tx, p);
+  const unsigned grid = static_cast<unsigned>(p.n_tiles < sms ? p.n_tiles : sms);
+  gemm_skinny_kernel<NB><<<grid, kThreads, kSmemBytes, stream>>>(tw, tx, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -190,7 +259,6 @@ extern "C" int ka_gemm_skinny_bf16(const void* a, long long lda, const void* w, 
   using namespace ka;
   if (m <= 0 || n <= 0) return 0;
   if (m > 64 || k <= 0) return -1;
-  const int nb = m <= 16 ? 16 : (m <= 32 ? 32 : 64);
   SkinnyParams p = {};
   p.out = static_cast<__nv_bfloat16*>(out);
   p.ldc = ldc;
@@ -200,7 +268,7 @@ extern "C" int ka_gemm_skinny_bf16(const void* a, long long lda, const void* w, 
   p.status = status;
   p.timeout_ns = timeout_ns;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (nb == 16) return launch<16, 128>(a, lda, w, ldw, p, st);
-  if (nb == 32) return launch<32, 128>(a, lda, w, ldw, p, st);
-  return launch<64, 128>(a, lda, w, ldw, p, st);
+  if (m <= 16) return launch<16>(a, lda, w, ldw, p, st);
+  if (m <= 32) return launch<32>(a, lda, w, ldw, p, st);
+  return launch<64>(a, lda, w, ldw, p, st);
 }

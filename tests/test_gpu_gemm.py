@@ -57,7 +57,8 @@ def test_linear_autograd(cuda_device):
 
 
 @pytest.mark.parametrize("m", [1, 8, 16, 17, 33, 64])
-@pytest.mark.parametrize("n,k", [(4096, 4096), (1000, 520), (28672, 4096), (4096, 14336)])
+@pytest.mark.parametrize("n,k", [(4096, 4096), (1000, 520), (28672, 4096), (4096, 14336), (8, 64), (6144, 200),
+                                 (19008, 192), (128256, 256)])
 def test_skinny_gemm_equals_tiled_kernel_bitwise(cuda_device, m, n, k, monkeypatch):
     """The weight-streaming kernel for decode-sized batches must give the bits of the tiled
     kernel: otherwise a row's result would depend on the batch size it is computed in."""
