@@ -86,6 +86,19 @@ __device__ __forceinline__ void decode_unit(const GemmParams& p, int tiles_m, in
     out.m_blk = (out.m_blk + static_cast<int>((static_cast<long long>(p.rank) * p.rows_per_rank) / (kBM * kG))) % tiles_m;
 }
 
+// The units of a CTA pair, in order. Plain modes deal units (tile, slice) round robin over the
+// pairs; tree mode (kTree) deals whole tiles, so that all slices of a tile follow one another on
+// the pair that combines them.
+template <bool kTree>
+__device__ __forceinline__ int first_unit(int pair_id, int k_slices) {
+  return kTree ? pair_id * k_slices : pair_id;
+}
+template <bool kTree>
+__device__ __forceinline__ int next_unit(int u, int n_pairs, int k_slices) {
+  if (!kTree) return u + n_pairs;
+  return (u + 1) % k_slices != 0 ? u + 1 : u + 1 + (n_pairs - 1) * k_slices;
+}
+
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory"); }
 
 __device__ __forceinline__ void tmem_ld_wait_dep(uint32_t (&v)[32]) {
@@ -213,6 +226,111 @@ __device__ __forceinline__ float4 add4(float4 a, float4 b) {
   return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
 }
 
+// ---- tree mode: the eight canonical K slices of a tile summed where they are computed.
+// A thread of the epilogue owns one row and 128 columns of the tile. Slice partials are rounded
+// to bf16 once and added in fp32 as ((0+1)+(2+3))+((4+5)+(6+7)), the reduce-scatter tail's
+// order, so the bits are those of the staged path. Even slices stay in registers as packed
+// bf16; (0+1), then (0+1)+(2+3), and (4+5) wait in two fp32 slots of a per-CTA scratch block
+// (2 x 128 KiB, 38 MB over the device: it stays in L2) that only this thread reads back.
+constexpr int kTreeSlices = 8;
+constexpr int kTreeSlotFloats = kBM * kBN;
+
+__device__ __forceinline__ float4* tree_slot(float* scratch, int cta, int slot, int warp, int g, int lane) {
+  return reinterpret_cast<float4*>(scratch + (static_cast<size_t>(cta) * 2 + slot) * kTreeSlotFloats) +
+         (warp * (kBN / 64) + g) * 8 * 32 + lane;   // eight float4 per thread and group, 32 apart
+}
+
+__device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
+
+// One 32-column group of slice `s`. `v`: the accumulators; `leaf`: the packed even slice of the
+// pair. Returns true when the tile is finished: `v` then holds 32 sums.
+__device__ __forceinline__ bool tree_group(float* scratch, int s, int warp, int g, int lane, uint32_t (&v)[32],
+                                           uint32_t (&leaf)[16]) {
+  if ((s & 1) == 0) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) leaf[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+    return false;
+  }
+  float4* s0 = tree_slot(scratch, blockIdx.x, 0, warp, g, lane);
+  float4* s1 = tree_slot(scratch, blockIdx.x, 1, warp, g, lane);
+  float4 t[8];
+  if (s == 3 || s == 7) {
+    const float4* src = s == 3 ? s0 : s1;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t[i] = src[i * 32];
+  }
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const uint32_t w = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+    v[2 * j] = __float_as_uint(__fadd_rn(bf16_lo(leaf[j]), bf16_lo(w)));
+    v[2 * j + 1] = __float_as_uint(__fadd_rn(bf16_hi(leaf[j]), bf16_hi(w)));
+  }
+  if (s == 3 || s == 7) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float4 a = add4(t[i], make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
+                                              __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3])));
+      v[4 * i] = __float_as_uint(a.x);
+      v[4 * i + 1] = __float_as_uint(a.y);
+      v[4 * i + 2] = __float_as_uint(a.z);
+      v[4 * i + 3] = __float_as_uint(a.w);
+    }
+  }
+  if (s == 7) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t[i] = s0[i * 32];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float4 a = add4(t[i], make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
+                                              __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3])));
+      v[4 * i] = __float_as_uint(a.x);
+      v[4 * i + 1] = __float_as_uint(a.y);
+      v[4 * i + 2] = __float_as_uint(a.z);
+      v[4 * i + 3] = __float_as_uint(a.w);
+    }
+    return true;
+  }
+  float4* dst = s == 5 ? s1 : s0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    dst[i * 32] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]), __uint_as_float(v[4 * i + 2]),
+                              __uint_as_float(v[4 * i + 3]));
+  return false;
+}
+
+// Store two finished 32-column groups (`half` 0 stages, 1 stores) with the optional residual:
+// the sum is rounded to bf16 first, as a separate bf16 linear + add would.
+__device__ __forceinline__ void tree_store(const GemmParams& p, const uint32_t (&v)[32], uint32_t* wbuf,
+                                           long long row_w0, int col, int lane, int half) {
+  uint32_t* mine = wbuf + lane * 33 + half * 16;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) mine[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+  __syncwarp();
+  if (half == 0) return;
+  const int c = lane & 7, r0 = lane >> 3;
+  const bool col_ok = col + c * 8 + 8 <= p.n;
+#pragma unroll
+  for (int it = 0; it < 8; ++it) {
+    const int r = r0 + 4 * it;
+    if (col_ok && row_w0 + r < p.m) {
+      const uint32_t* src = wbuf + r * 33 + c * 4;
+      const long long off = (row_w0 + r) * p.n + col + c * 8;
+      uint4 o = make_uint4(src[0], src[1], src[2], src[3]);
+      if (p.residual) {
+        const uint4 rr = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.residual) + off);
+        o.x = pack_bf16(__fadd_rn(bf16_lo(o.x), bf16_lo(rr.x)), __fadd_rn(bf16_hi(o.x), bf16_hi(rr.x)));
+        o.y = pack_bf16(__fadd_rn(bf16_lo(o.y), bf16_lo(rr.y)), __fadd_rn(bf16_hi(o.y), bf16_hi(rr.y)));
+        o.z = pack_bf16(__fadd_rn(bf16_lo(o.z), bf16_lo(rr.z)), __fadd_rn(bf16_hi(o.z), bf16_hi(rr.z)));
+        o.w = pack_bf16(__fadd_rn(bf16_lo(o.w), bf16_lo(rr.w)), __fadd_rn(bf16_hi(o.w), bf16_hi(rr.w)));
+      }
+      *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(p.out) + off) = o;
+    }
+  }
+  __syncwarp();
+}
+
+template <bool kTree>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                  const __grid_constant__ GemmParams p) {
@@ -270,7 +388,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int u = pair_id; u < n_units && ok; u += n_pairs) {
+      for (int u = first_unit<kTree>(pair_id, p.k_slices); u < n_units && ok; u = next_unit<kTree>(u, n_pairs, p.k_slices)) {
         Unit un;
         decode_unit(p, tiles_m, tiles_n, u, un);
         const int row0 = un.m_blk * (kBM * kG) + static_cast<int>(cta_rank) * kBM;
@@ -326,7 +444,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       int abuf = 0;
       uint32_t aphase = 0;
       bool ok = true;
-      for (int u = pair_id; u < n_units && ok; u += n_pairs) {
+      for (int u = first_unit<kTree>(pair_id, p.k_slices); u < n_units && ok; u = next_unit<kTree>(u, n_pairs, p.k_slices)) {
         ok = mbar_wait_bounded(smem_u32(&ctl->tempty[abuf]), aphase ^ 1u, wctx, kWMmaTmem, abuf);
         if (!ok) break;
         tc_fence_after_sync();
@@ -407,7 +525,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     int abuf = 0;
     uint32_t aphase = 0;
     const uint32_t tempty_leader = mapa_u32(smem_u32(&ctl->tempty[0]), 0);
-    for (int u = pair_id; u < n_units; u += n_pairs) {
+    uint32_t leaf[kTree ? kBN / 64 : 1][16];
+    for (int u = first_unit<kTree>(pair_id, p.k_slices); u < n_units; u = next_unit<kTree>(u, n_pairs, p.k_slices)) {
       Unit un;
       decode_unit(p, tiles_m, tiles_n, u, un);
       const long long row_w0 = static_cast<long long>(un.m_blk) * (kBM * kG) + cta_rank * kBM + wq * 32;
@@ -427,6 +546,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         rc.tgt = p.row_ids[row] - p.col_offset;
       }
       uint32_t* wbuf = epi_buf + warp * kEpiBufWords;
+      if constexpr (kTree) {
+#pragma unroll
+        for (int g = 0; g < kBN / 64; ++g) {
+          uint32_t v[32];
+          __syncwarp();
+          tmem_ld_32x32(trow + g * 32, v);
+          tmem_ld_wait_dep(v);
+          if (tree_group(p.tree_scratch, un.slice, warp, g, lane, v, leaf[g]))
+            tree_store(p, v, wbuf, row_w0, col0 + (g & ~1) * 32, lane, g & 1);
+        }
+      } else {
       uint32_t va[32], vb[32];
       tmem_ld_32x32(trow, va);
       tmem_ld_wait_dep(va);
@@ -441,6 +571,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         store_group_warp(p, vb, wbuf, row_w0, col0 + (g + 1) * 32, slice_global, rc, lane, 1);
         __syncwarp();
         if (g + 2 < kBN / 64) tmem_ld_wait_dep(va);
+      }
       }
       tc_fence_before_sync();
       __syncwarp();
@@ -561,10 +692,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   }
 }
 
+template <bool kTree>
 int max_ctas(int num_sms) {
   static int cached = 0;
   if (cached > 0) return cached;
-  if (cudaFuncSetAttribute(gemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
+  if (cudaFuncSetAttribute(gemm_bf16_kernel<kTree>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
     return -1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(num_sms / 2 * 2));
@@ -578,7 +710,7 @@ int max_ctas(int num_sms) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, gemm_bf16_kernel, &cfg) != cudaSuccess || clusters <= 0) {
+  if (cudaOccupancyMaxActiveClusters(&clusters, gemm_bf16_kernel<kTree>, &cfg) != cudaSuccess || clusters <= 0) {
     cudaGetLastError();
     clusters = num_sms / 2;
   }
@@ -610,10 +742,12 @@ int gemm_launch(const void* a, long long lda, const void* b, long long ldb, cons
   else
     rc = make_tmap_2d_16bit_sw128(&tm_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, b, p.k, p.n, ldb, kBK, 64);
   if (rc != 0) return -40 + rc;
-  int ctas = max_ctas(num_sms);
+  const bool tree = p.epilogue == kEpiTreeBf16;
+  if (tree && (p.k_slices != kTreeSlices || !p.tree_scratch)) return -4;
+  int ctas = tree ? max_ctas<true>(num_sms) : max_ctas<false>(num_sms);
   if (ctas <= 0) return -10;
   const int tiles_m = (p.m + kBM * kG - 1) / (kBM * kG), tiles_n = (p.n + kBN - 1) / kBN;
-  const int units = tiles_m * tiles_n * p.k_slices;
+  const int units = tiles_m * tiles_n * (tree ? 1 : p.k_slices);
   if (!full_grid && units * kG < ctas) ctas = units * kG;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(ctas));
@@ -627,7 +761,8 @@ int gemm_launch(const void* a, long long lda, const void* b, long long ldb, cons
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_bf16_kernel, tm_a, tm_b, p);
+  const cudaError_t e = tree ? cudaLaunchKernelEx(&cfg, gemm_bf16_kernel<true>, tm_a, tm_b, p)
+                             : cudaLaunchKernelEx(&cfg, gemm_bf16_kernel<false>, tm_a, tm_b, p);
   if (e != cudaSuccess) {
     fprintf(stderr, "[kernel_align_b200] gemm launch failed: %s\n", cudaGetErrorString(e));
     return -11;
@@ -651,6 +786,36 @@ extern "C" int ka_gemm_bf16(const void* a, long long lda, int a_major, const voi
   p.ldc = ldc;
   p.k_slices = 1;
   p.total_slices = 1;
+  p.world = 1;
+  p.status = status;
+  p.timeout_ns = timeout_ns;
+  return ka::gemm_launch(a, lda, b, ldb, p, num_sms, false, static_cast<cudaStream_t>(stream));
+}
+
+// Bytes of scratch ka_gemm_tree8 needs on a device with num_sms SMs (uninitialised memory).
+extern "C" size_t ka_gemm_tree8_scratch_bytes(int num_sms) {
+  return static_cast<size_t>(num_sms) * 2 * ka::kTreeSlotFloats * sizeof(float);
+}
+
+// out[m, n] (bf16, row-major) = a[m, k] times b^T (+ residual) with K cut into the eight
+// canonical slices of the tensor-parallel linears, every slice rounded to bf16 once and summed in
+// fp32 in the fixed tree order: what ka_gemm_reduce_scatter computes on one rank, bit for bit,
+// without its staging buffers. b: [n, k] (b_major = 0) or [k, n] (b_major = 1).
+extern "C" int ka_gemm_tree8(const void* a, long long lda, const void* b, long long ldb, int b_major, void* out,
+                             const void* residual, void* scratch, int m, int n, int k, int* status, int num_sms,
+                             unsigned long long timeout_ns, void* stream) {
+  if (n % 8 != 0) return -51;
+  ka::GemmParams p = {};
+  p.m = m;
+  p.n = n;
+  p.k = k;
+  p.b_major = b_major ? 1 : 0;
+  p.epilogue = ka::kEpiTreeBf16;
+  p.out = out;
+  p.residual = residual;
+  p.tree_scratch = static_cast<float*>(scratch);
+  p.k_slices = ka::kTreeSlices;
+  p.total_slices = ka::kTreeSlices;
   p.world = 1;
   p.status = status;
   p.timeout_ns = timeout_ns;

@@ -24,6 +24,7 @@ enum GemmEpilogue : int {
   kEpiStoreBf16 = 0,    // C bf16 [M, N]
   kEpiStoreF32 = 1,     // C fp32 [M, N]
   kEpiPartialF32 = 2,   // K-slice partial (fp32 accumulated, stored as bf16), pushed to the row owner's staging buffer
+  kEpiTreeBf16 = 4,     // the eight K slices of a tile summed in the kernel, `out` bf16 [M, N] (+ residual)
   kEpiLogitsGrad = 3    // C bf16 = g[row] * scale * (onehot(ids[row]) - exp(scale * acc - lse[row]))
 };
 
@@ -44,6 +45,7 @@ struct GemmParams {
   unsigned epoch;
   void* out;              // reduced bf16 [rows_per_rank, n] of this rank
   const void* residual;   // optional bf16 [rows_per_rank, n] added after the reduction
+  float* tree_scratch;    // kEpiTreeBf16: two fp32 tiles per CTA
   // --- all-gather of A (a_gather != 0): A is read from `a` = this rank's gather buffer
   //     [world * rows_per_rank_a, k]; rows of rank r become valid when a_flags[r * blocks + b] == epoch
   int a_gather;

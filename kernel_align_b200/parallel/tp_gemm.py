@@ -84,6 +84,11 @@ def _lib():
     lib.ka_gemm_reduce_scatter.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_void_p, c_void_p,
                                            c_void_p, c_int, c_int, c_int, c_int, c_int, c_uint, c_void_p, c_int,
                                            c_ulonglong, c_void_p]
+    lib.ka_gemm_tree8_scratch_bytes.restype = c_size_t
+    lib.ka_gemm_tree8_scratch_bytes.argtypes = [c_int]
+    lib.ka_gemm_tree8.restype = c_int
+    lib.ka_gemm_tree8.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_int,
+                                  c_int, c_int, c_void_p, c_int, c_ulonglong, c_void_p]
     lib.ka_all_gather_gemm.restype = c_int
     lib.ka_all_gather_gemm.argtypes = [c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_void_p, c_int,
                                        c_int, c_int, c_int, c_int, c_uint, c_void_p, c_int, c_ulonglong, c_void_p]
@@ -126,6 +131,22 @@ def _gemm_reduce_scatter_cpu(x, w_shard, ctx, residual, trans_b, keep_padding):
     return out if keep_padding else out[:rows_valid]
 
 
+def _tree_pays(m: int, n: int, k: int, num_sms: int) -> bool:
+    """Whether one rank sums the eight K slices of a tile in the kernel that computes them
+    (``ka_gemm_tree8``) or stages them (``ka_gemm_reduce_scatter``). The bits are the same.
+
+    A CTA pair that keeps a tile walks its eight slices one after the other, while staged slices
+    spread over all pairs but cost a pass over the partials and the wait for them. Measured on
+    148 SMs, staged / kept in us: 4096 rows, N = 4096: 399 / 184 (K = 4096), 1077 / 884 (28672);
+    32 tiles: 75 / 46 (4096), 110 / 97 (14336), 148 / 162 (28672); 16 tiles: 55 / 41 (4096),
+    62 / 58 (6144), 74 / 95 (14336). A slice round takes about 5.4e-3 us per K column, staging
+    about 20 us plus 1.2 us per tile; the rule compares the two."""
+    pairs = max(1, num_sms // 2)
+    tiles = -(-m // 256) * -(-n // 256)
+    extra_rounds = -(-tiles // pairs) * 8 - -(-8 * tiles // pairs)
+    return extra_rounds * (k / 8) * 5.4e-3 < 20 + 1.2 * tiles
+
+
 @profiled("gemm_reduce_scatter")
 def gemm_reduce_scatter(x: torch.Tensor, w_shard: torch.Tensor, ctx: TPContext,
                         residual: Optional[torch.Tensor] = None, trans_b: bool = False,
@@ -144,8 +165,6 @@ def gemm_reduce_scatter(x: torch.Tensor, w_shard: torch.Tensor, ctx: TPContext,
     x = x.contiguous()
     w = w_shard.contiguous()
     rpr = rows_per_rank(m, ctx.world)
-    nbytes = lib.ka_gemm_rs_exchange_bytes(m, n, ctx.world)
-    arena, epoch = ctx.arena(("rs", m, n), nbytes)
     rows_valid = max(0, min(rpr, m - ctx.rank * rpr))
     out = torch.empty(rpr, n, dtype=torch.bfloat16, device=x.device)
     res = None
@@ -153,8 +172,20 @@ def gemm_reduce_scatter(x: torch.Tensor, w_shard: torch.Tensor, ctx: TPContext,
         res = residual.contiguous()
         if res.shape[0] < rpr:
             res = torch.cat([res, res.new_zeros(rpr - res.shape[0], n)])
-    ptrs = (c_void_p * ctx.world)(*arena.ptrs)
     props = torch.cuda.get_device_properties(x.device)
+    if ctx.world == 1 and _tree_pays(m, n, k_local, props.multi_processor_count):
+        scratch = torch.empty(lib.ka_gemm_tree8_scratch_bytes(props.multi_processor_count), dtype=torch.uint8,
+                              device=x.device)
+        rc = lib.ka_gemm_tree8(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), int(trans_b), out.data_ptr(),
+                               res.data_ptr() if res is not None else None, scratch.data_ptr(), m, n, k_local,
+                               status_buffer(x.device).data_ptr(), props.multi_processor_count, default_timeout_ns(),
+                               torch.cuda.current_stream(x.device).cuda_stream)
+        if rc != 0:
+            raise RuntimeError(f"ka_gemm_tree8 rejected its arguments (code {rc})")
+        return out if keep_padding else out[:rows_valid]
+    nbytes = lib.ka_gemm_rs_exchange_bytes(m, n, ctx.world)
+    arena, epoch = ctx.arena(("rs", m, n), nbytes)
+    ptrs = (c_void_p * ctx.world)(*arena.ptrs)
     rc = lib.ka_gemm_reduce_scatter(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), int(trans_b), out.data_ptr(),
                                     res.data_ptr() if res is not None else None, ptrs, m, n, k_local, ctx.world,
                                     ctx.rank, epoch & 0xFFFFFFFF, status_buffer(x.device).data_ptr(),

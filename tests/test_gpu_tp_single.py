@@ -43,3 +43,23 @@ def test_reduce_scatter_matches_cpu_rank_emulator(cuda_device):
     diff = (out.cpu().float() - emu).abs()
     assert diff.max().item() <= 0.02 * emu.abs().max().item()
     assert (diff > 0).float().mean().item() < 0.2
+
+
+@pytest.mark.parametrize("m,n,k,trans_b", [(1, 8, 512, False), (300, 264, 512, False), (1000, 768, 1536, True),
+                                           (2049, 1032, 1024, False), (19000, 256, 512, True)])
+def test_slices_summed_in_the_kernel_equal_the_staged_ones_bitwise(cuda_device, m, n, k, trans_b, monkeypatch):
+    """One rank may sum the eight K slices of a tile where they are computed; the staged path,
+    which the multi-rank kernels share, defines the bits."""
+    from kernel_align_b200.parallel import tp_gemm
+
+    ctx = TPContext(device=cuda_device)
+    g = torch.Generator(device=cuda_device).manual_seed(m + n)
+    x = torch.randn(m, k, device=cuda_device, generator=g).to(torch.bfloat16)
+    w = (torch.randn(*((k, n) if trans_b else (n, k)), device=cuda_device, generator=g) * 0.05).to(torch.bfloat16)
+    r = torch.randn(m, n, device=cuda_device, generator=g).to(torch.bfloat16)
+    outs = []
+    for tree in (False, True):
+        monkeypatch.setattr(tp_gemm, "_tree_pays", lambda *a, t=tree: t)
+        outs += [[gemm_reduce_scatter(x, w, ctx, residual=res, trans_b=trans_b) for res in (None, r)]]
+    gemm.check_status(cuda_device)
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
