@@ -140,6 +140,65 @@ rope_vec8_kernel(__nv_bfloat16* __restrict__ x, long long token_stride, const lo
   }
 }
 
+// The fused qkv projection cut into its parts with q and k rotated, and the way back:
+//   kBackward = false: qkv [rows, (hq + 2 hkv) * 128] -> q, k (rotated), v, each [tokens, heads, 128]
+//   kBackward = true:  dq, dk (rotated by the opposite angle), dv -> dqkv; rows past `tokens` are zeroed
+// Bound by the bytes: every element is read once and written once, 16 bytes per access. A thread
+// takes eight pairs of one head (rope_vec8_kernel's arithmetic, the same bits) for two tokens;
+// a block is 32 heads x 8 groups of pairs, so no index is divided.
+// 4096 tokens, 32 + 8 + 8 heads: slices, copies, rotation and their autograd took about 300 us of
+// a layer's forward and backward, this takes two launches.
+constexpr int kQkvTokens = 2;
+
+template <bool kBackward>
+__global__ void __launch_bounds__(256)
+qkv_rope_kernel(__nv_bfloat16* __restrict__ qkv, long long qkv_stride, const long long* __restrict__ positions,
+                const float* __restrict__ cos_t, const float* __restrict__ sin_t, __nv_bfloat16* __restrict__ q,
+                __nv_bfloat16* __restrict__ k, __nv_bfloat16* __restrict__ v, int rows, int tokens, int hq, int hkv) {
+  constexpr int kHd = 128, kHalf = 64;
+  const int head = blockIdx.y * 32 + (threadIdx.x >> 3), j = (threadIdx.x & 7) * 8;
+  if (head >= hq + 2 * hkv) return;
+  __nv_bfloat16* part = head < hq ? q : (head < hq + hkv ? k : v);
+  const int heads = head < hq ? hq : hkv, h = head < hq ? head : (head < hq + hkv ? head - hq : head - hq - hkv);
+  const bool rotate = head < hq + hkv;
+#pragma unroll
+  for (int n = 0; n < kQkvTokens; ++n) {
+    const long long t = static_cast<long long>(blockIdx.x) * kQkvTokens + n;
+    if (t >= rows) return;
+    __nv_bfloat16* joint = qkv + t * qkv_stride + static_cast<long long>(head) * kHd + j;
+    __nv_bfloat16* own = part + (t * heads + h) * kHd + j;
+    Bf16x8 lo, hi;
+    if (t < tokens) {
+      const __nv_bfloat16* src = kBackward ? own : joint;
+      lo = *reinterpret_cast<const Bf16x8*>(src);
+      hi = *reinterpret_cast<const Bf16x8*>(src + kHalf);
+      if (rotate) {
+        const long long pos = positions[t];
+        const float4* cp = reinterpret_cast<const float4*>(cos_t + pos * kHalf + j);
+        const float4* sp = reinterpret_cast<const float4*>(sin_t + pos * kHalf + j);
+        const float4 c0 = cp[0], c1 = cp[1], s0 = sp[0], s1 = sp[1];
+        const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+        const float sn[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float a = __bfloat162float(lo.v[e]), b = __bfloat162float(hi.v[e]);
+          const float se = kBackward ? -sn[e] : sn[e];
+          lo.v[e] = __float2bfloat16_rn(__fsub_rn(__fmul_rn(a, c[e]), __fmul_rn(b, se)));
+          hi.v[e] = __float2bfloat16_rn(__fadd_rn(__fmul_rn(b, c[e]), __fmul_rn(a, se)));
+        }
+      }
+    } else if constexpr (kBackward) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) lo.v[e] = hi.v[e] = __float2bfloat16_rn(0.f);
+    } else {
+      return;
+    }
+    __nv_bfloat16* dst = kBackward ? joint : own;
+    *reinterpret_cast<Bf16x8*>(dst) = lo;
+    *reinterpret_cast<Bf16x8*>(dst + kHalf) = hi;
+  }
+}
+
 __device__ __forceinline__ float tanh_approx(float x) {
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -206,10 +265,12 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* _
 // Backward of y = bf16(bf16(x * inv) * w).
 //   dx = inv * (dy*w - n * mean(dy*w*n)),  n = x * inv;   dw_partial[chunk] = sum_rows dy * n
 // One CTA per chunk of kRmsChunk rows (fixed, so the order in which rows enter d_w does not
-// depend on the grid); threads own columns. kRows rows are in flight at once: their x and dy
+// depend on the grid); 16 rows give 4096 tokens 256 CTAs, one wave of two per SM (64 rows left
+// more than half of the SMs idle: 92 us). With `d_res` the gradient that reaches x past the norm
+// (the residual stream) is added to the rounded dx, which saves a pass. Threads own columns. kRows rows are in flight at once: their x and dy
 // vectors are loaded once into registers and serve all three steps (sum of squares, the dot
 // product, dx / dw), and the block reductions of the kRows rows share their two barriers.
-constexpr int kRmsChunk = 64;
+constexpr int kRmsChunk = 16;
 
 // Fixed-order sums of R values per thread over the CTA (8 warps): lanes by xor-shuffle, then the
 // eight warp sums left to right, the same in every thread.
@@ -237,8 +298,8 @@ __device__ __forceinline__ void block_sum_fixed_multi(float (&v)[R], float (*s_w
 template <int VPT, int kRows>
 __global__ void __launch_bounds__(256, 2)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                   const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part,
-                   int rows, int d, float eps) {
+                   const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ d_res,
+                   __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part, int rows, int d, float eps) {
   __shared__ float s_warp[kRows][8];
   const int chunk = blockIdx.x;
   const int r0 = chunk * kRmsChunk, r1 = min(rows, r0 + kRmsChunk);
@@ -321,6 +382,12 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
           o.v[j] = __float2bfloat16_rn(__fmul_rn(inv[r], __fsub_rn(gw, __fmul_rn(n, mean_dot))));
           dw_acc[a][j] = __fmaf_rn(g, n, dw_acc[a][j]);  // rows enter in increasing order
         }
+        if (d_res) {
+          const Bf16x8 rr = reinterpret_cast<const Bf16x8*>(d_res + static_cast<size_t>(row) * d)[i];
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            o.v[j] = __float2bfloat16_rn(__fadd_rn(__bfloat162float(o.v[j]), __bfloat162float(rr.v[j])));
+        }
         reinterpret_cast<Bf16x8*>(dx + static_cast<size_t>(row) * d)[i] = o;
       }
     }
@@ -335,13 +402,25 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   }
 }
 
-// d_w[c] = sum over chunks (in index order) of dw_part[chunk][c]
-__global__ void rmsnorm_dw_kernel(const float* __restrict__ dw_part, __nv_bfloat16* __restrict__ dw, int chunks, int d) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d) return;
+// d_w[c] = sum over chunks of dw_part[chunk][c]: eight interleaved sets of chunks (each in index
+// order), then the sets in order. A block is 32 columns x 8 sets, so that 256 chunks are 32
+// dependent adds and not 256.
+__global__ void __launch_bounds__(256)
+rmsnorm_dw_kernel(const float* __restrict__ dw_part, __nv_bfloat16* __restrict__ dw, int chunks, int d) {
+  __shared__ float s_part[8][32];
+  const int col = threadIdx.x & 31, set = threadIdx.x >> 5, c = blockIdx.x * 32 + col;
   float acc = 0.f;
-  for (int k = 0; k < chunks; ++k) acc = __fadd_rn(acc, dw_part[static_cast<size_t>(k) * d + c]);
-  dw[c] = __float2bfloat16_rn(acc);
+  if (c < d) {
+#pragma unroll 4
+    for (int k = set; k < chunks; k += 8) acc = __fadd_rn(acc, dw_part[static_cast<size_t>(k) * d + c]);
+  }
+  s_part[set][col] = acc;
+  __syncthreads();
+  if (set == 0 && c < d) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) acc = __fadd_rn(acc, s_part[w][col]);
+    dw[c] = __float2bfloat16_rn(acc);
+  }
 }
 
 int grid_for(long long work_items, int threads, int num_sms) {
@@ -386,6 +465,21 @@ int ka_rope(void* x, long long token_stride, const long long* positions, const f
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
+// See qkv_rope_kernel. head_dim is 128, qkv rows 16-byte aligned, positions [tokens] on the device.
+int ka_qkv_rope(void* qkv, long long qkv_stride, const long long* positions, const float* cos_t, const float* sin_t,
+                void* q, void* k, void* v, int rows, int tokens, int hq, int hkv, int backward, void* stream) {
+  using namespace ka;
+  if (rows <= 0) return 0;
+  if (qkv_stride % 8 != 0 || (reinterpret_cast<uintptr_t>(qkv) & 15u) != 0 || tokens > rows) return -1;
+  const dim3 grid(static_cast<unsigned>((rows + kQkvTokens - 1) / kQkvTokens),
+                  static_cast<unsigned>((hq + 2 * hkv + 31) / 32));
+  auto* kernel = backward ? qkv_rope_kernel<true> : qkv_rope_kernel<false>;
+  kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<__nv_bfloat16*>(qkv), qkv_stride, positions, cos_t, sin_t, static_cast<__nv_bfloat16*>(q),
+      static_cast<__nv_bfloat16*>(k), static_cast<__nv_bfloat16*>(v), rows, tokens, hq, hkv);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
 int ka_swiglu(const void* gate, const void* up, long long in_stride, void* out, int rows, int f, int num_sms,
               void* stream) {
   using namespace ka;
@@ -414,10 +508,10 @@ int ka_swiglu_bwd(const void* gate, const void* up, long long in_stride, const v
 // Rows per partial sum of the weight gradient (the size of dw_part follows from it).
 int ka_rmsnorm_bwd_chunk() { return ka::kRmsChunk; }
 
-// x, dy: [rows, d] bf16; dx: [rows, d] bf16; dw: [d] bf16; dw_part: scratch of
+// x, dy: [rows, d] bf16; d_res: null or [rows, d], added to dx; dx: [rows, d] bf16; dw: [d] bf16; dw_part: scratch of
 // ceil(rows / ka_rmsnorm_bwd_chunk()) * d floats. d % 8 == 0 and d <= 8192.
-int ka_rmsnorm_bwd(const void* x, const void* w, const void* dy, void* dx, void* dw, float* dw_part, int rows, int d,
-                   float eps, void* stream) {
+int ka_rmsnorm_bwd(const void* x, const void* w, const void* dy, const void* d_res, void* dx, void* dw, float* dw_part,
+                   int rows, int d, float eps, void* stream) {
   using namespace ka;
   if (rows <= 0) return 0;
   if (d % 8 != 0 || d > 8192) return -1;
@@ -426,15 +520,16 @@ int ka_rmsnorm_bwd(const void* x, const void* w, const void* dy, void* dx, void*
   const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
   const __nv_bfloat16* wb = static_cast<const __nv_bfloat16*>(w);
   const __nv_bfloat16* gb = static_cast<const __nv_bfloat16*>(dy);
+  const __nv_bfloat16* rb = static_cast<const __nv_bfloat16*>(d_res);
   __nv_bfloat16* ob = static_cast<__nv_bfloat16*>(dx);
   const int vpt = (d / 8 + 255) / 256;
   if (vpt <= 1)
-    rmsnorm_bwd_kernel<1, 4><<<chunks, 256, 0, st>>>(xb, wb, gb, ob, dw_part, rows, d, eps);
+    rmsnorm_bwd_kernel<1, 4><<<chunks, 256, 0, st>>>(xb, wb, gb, rb, ob, dw_part, rows, d, eps);
   else if (vpt == 2)
-    rmsnorm_bwd_kernel<2, 2><<<chunks, 256, 0, st>>>(xb, wb, gb, ob, dw_part, rows, d, eps);
+    rmsnorm_bwd_kernel<2, 2><<<chunks, 256, 0, st>>>(xb, wb, gb, rb, ob, dw_part, rows, d, eps);
   else
-    rmsnorm_bwd_kernel<4, 1><<<chunks, 256, 0, st>>>(xb, wb, gb, ob, dw_part, rows, d, eps);
-  rmsnorm_dw_kernel<<<(d + 255) / 256, 256, 0, st>>>(dw_part, static_cast<__nv_bfloat16*>(dw), chunks, d);
+    rmsnorm_bwd_kernel<4, 1><<<chunks, 256, 0, st>>>(xb, wb, gb, rb, ob, dw_part, rows, d, eps);
+  rmsnorm_dw_kernel<<<(d + 31) / 32, 256, 0, st>>>(dw_part, static_cast<__nv_bfloat16*>(dw), chunks, d);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 

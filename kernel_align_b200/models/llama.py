@@ -28,7 +28,7 @@ import torch.nn as nn
 import torch.utils.checkpoint
 
 from ..ops.attention import attention_fn
-from ..ops.layer_ops import rmsnorm_fn, rope_fn, rope_tables, swiglu_fn
+from ..ops.layer_ops import qkv_rope_fn, rmsnorm_fn, rmsnorm_fork_fn, rope_tables, swiglu_fn
 from ..parallel.tp_gemm import TPContext, rows_per_rank
 from ..parallel.tp_layers import column_parallel_linear, row_parallel_linear
 
@@ -101,20 +101,17 @@ class DecoderLayer(nn.Module):
         cfg, tp = self.cfg, self.tp
         hd = cfg.head_dim
         tokens = batch * seq_len
-        h = rmsnorm_fn(x_local, self.norm1, cfg.rms_eps)
+        h, x_local = rmsnorm_fork_fn(x_local, self.norm1, cfg.rms_eps)
         qkv = column_parallel_linear(h, self.wqkv, tp)                       # [M_pad, (hq + 2 hkv) * hd]
-        qkv = qkv[:tokens]
-        q = qkv[:, : self.hq * hd].reshape(tokens, self.hq, hd)
-        k = qkv[:, self.hq * hd:(self.hq + self.hkv) * hd].reshape(tokens, self.hkv, hd)
-        v = qkv[:, (self.hq + self.hkv) * hd:].reshape(batch, seq_len, self.hkv, hd)
-        q = rope_fn(q, positions, cos, sin).view(batch, seq_len, self.hq, hd)
-        k = rope_fn(k, positions, cos, sin).view(batch, seq_len, self.hkv, hd)
+        q, k, v = qkv_rope_fn(qkv, positions, cos, sin, self.hq, self.hkv, hd)
+        q = q.view(batch, seq_len, self.hq, hd)
+        k, v = k.view(batch, seq_len, self.hkv, hd), v.view(batch, seq_len, self.hkv, hd)
         a = attention_fn(q, k, v, causal=True).reshape(tokens, self.hq * hd)
         m_pad = x_local.shape[0] * tp.world
         if m_pad != tokens:
             a = torch.cat([a, a.new_zeros(m_pad - tokens, a.shape[1])])
         x_local = row_parallel_linear(a, self.wo, tp, residual=x_local)
-        h = rmsnorm_fn(x_local, self.norm2, cfg.rms_eps)
+        h, x_local = rmsnorm_fork_fn(x_local, self.norm2, cfg.rms_eps)
         gu = column_parallel_linear(h, self.wgu, tp)                         # [M_pad, 2 * ffn / world]
         f = swiglu_fn(gu)
         x_local = row_parallel_linear(f, self.wdown, tp, residual=x_local)

@@ -140,6 +140,35 @@ def swiglu(gate_up: torch.Tensor, up: Optional[torch.Tensor] = None) -> torch.Te
 # Differentiable wrappers: on CUDA forward and backward both run the hand-written kernels; on
 # CPU the forward is the C++ library and the backward the same formulas in PyTorch fp32.
 # --------------------------------------------------------------------------------------------
+def _rmsnorm_backward(x, weight, eps, dy, d_res):
+    """``(dx, dw)`` of RMSNorm; ``d_res`` (or None) is added to the rounded ``dx``."""
+    d = x.shape[-1]
+    x2 = x.reshape(-1, d).contiguous()
+    dy2 = dy.reshape(-1, d).contiguous()
+    rows = x2.shape[0]
+    if x.device.type != "cuda":
+        xf, gf, wf = x2.float(), dy2.float(), weight.float()
+        r = torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps)
+        gw = gf * wf
+        dx = r * gw - xf * (r.pow(3) * (gw * xf).mean(-1, keepdim=True))
+        dw = (gf * xf * r).sum(0)
+        dx = dx.to(x.dtype).reshape(x.shape)
+        return (dx if d_res is None else dx + d_res), dw.to(weight.dtype)
+    res2 = d_res.reshape(-1, d).contiguous() if d_res is not None else None
+    dx = torch.empty_like(x2)
+    dw = torch.empty_like(weight)
+    chunk = int(_native.cuda().ka_rmsnorm_bwd_chunk())
+    part = torch.empty((rows + chunk - 1) // chunk, d, dtype=torch.float32, device=x.device)
+    fn = _native.cuda().ka_rmsnorm_bwd
+    fn.restype = c_int
+    fn.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float,
+                   c_void_p]
+    _check(fn(x2.data_ptr(), weight.contiguous().data_ptr(), dy2.data_ptr(),
+              res2.data_ptr() if res2 is not None else None, dx.data_ptr(), dw.data_ptr(), part.data_ptr(), rows, d,
+              float(eps), _stream(x)), "ka_rmsnorm_bwd")
+    return dx.reshape(x.shape), dw
+
+
 class _RMSNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, eps):
@@ -150,27 +179,7 @@ class _RMSNormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, weight = ctx.saved_tensors
-        d = x.shape[-1]
-        x2 = x.reshape(-1, d).contiguous()
-        dy2 = dy.reshape(-1, d).contiguous()
-        rows = x2.shape[0]
-        if x.device.type != "cuda":
-            xf, gf, wf = x2.float(), dy2.float(), weight.float()
-            r = torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + ctx.eps)
-            gw = gf * wf
-            dx = r * gw - xf * (r.pow(3) * (gw * xf).mean(-1, keepdim=True))
-            dw = (gf * xf * r).sum(0)
-            return dx.to(x.dtype).reshape(x.shape), dw.to(weight.dtype), None
-        dx = torch.empty_like(x2)
-        dw = torch.empty_like(weight)
-        chunk = int(_native.cuda().ka_rmsnorm_bwd_chunk())
-        part = torch.empty((rows + chunk - 1) // chunk, d, dtype=torch.float32, device=x.device)
-        fn = _native.cuda().ka_rmsnorm_bwd
-        fn.restype = c_int
-        fn.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_void_p]
-        _check(fn(x2.data_ptr(), weight.contiguous().data_ptr(), dy2.data_ptr(), dx.data_ptr(), dw.data_ptr(),
-                  part.data_ptr(), rows, d, float(ctx.eps), _stream(x)), "ka_rmsnorm_bwd")
-        return dx.reshape(x.shape), dw, None
+        return (*_rmsnorm_backward(x, weight, ctx.eps, dy, None), None)
 
 
 def rmsnorm_fn(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5) -> torch.Tensor:
@@ -178,6 +187,30 @@ def rmsnorm_fn(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5) -> torc
     if not (x.requires_grad or weight.requires_grad) or not torch.is_grad_enabled():
         return rmsnorm(x, weight, eps)
     return _RMSNormFn.apply(x, weight, eps)
+
+
+class _RMSNormForkFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, weight, eps):
+        ctx.set_materialize_grads(False)
+        ctx.save_for_backward(x, weight)
+        ctx.eps = eps
+        return rmsnorm(x, weight, eps), x.view_as(x)
+
+    @staticmethod
+    def backward(ctx, dy, d_res):
+        x, weight = ctx.saved_tensors
+        if dy is None:
+            return d_res, None, None
+        return (*_rmsnorm_backward(x, weight, ctx.eps, dy, d_res), None)
+
+
+def rmsnorm_fork_fn(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5):
+    """``(rmsnorm(x) * weight, x)`` for a residual stream that goes both through the norm and past
+    it. Backward adds the two gradients of ``x`` inside the norm's kernel."""
+    if not (x.requires_grad or weight.requires_grad) or not torch.is_grad_enabled():
+        return rmsnorm(x, weight, eps), x
+    return _RMSNormForkFn.apply(x, weight, eps)
 
 
 class _RopeFn(torch.autograd.Function):
@@ -196,6 +229,49 @@ class _RopeFn(torch.autograd.Function):
 def rope_fn(x: torch.Tensor, positions: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
     """Out-of-place, differentiable rotary embedding of ``x`` ``[tokens, heads, head_dim]``."""
     return _RopeFn.apply(x, positions, cos, sin)
+
+
+def _qkv_rope_launch(qkv, positions, cos, sin, q, k, v, tokens, backward):
+    fn = _native.cuda().ka_qkv_rope
+    fn.restype = c_int
+    fn.argtypes = [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                   c_int, c_int, c_void_p]
+    _check(fn(qkv.data_ptr(), qkv.stride(0), positions.data_ptr(), cos.data_ptr(), sin.data_ptr(), q.data_ptr(),
+              k.data_ptr(), v.data_ptr(), qkv.shape[0], tokens, q.shape[1], k.shape[1], int(backward), _stream(qkv)),
+           "ka_qkv_rope")
+
+
+class _QkvRopeFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, qkv, positions, cos, sin, hq, hkv, tokens):
+        pos = positions.reshape(-1).to(torch.int64).contiguous()
+        ctx.save_for_backward(pos, cos, sin)
+        ctx.shape = qkv.shape
+        q, k, v = (torch.empty(tokens, h, 128, dtype=qkv.dtype, device=qkv.device) for h in (hq, hkv, hkv))
+        _qkv_rope_launch(qkv, pos, cos, sin, q, k, v, tokens, False)
+        return q, k, v
+
+    @staticmethod
+    def backward(ctx, dq, dk, dv):
+        pos, cos, sin = ctx.saved_tensors
+        dqkv = torch.empty(ctx.shape, dtype=dq.dtype, device=dq.device)
+        _qkv_rope_launch(dqkv, pos, cos, sin, dq.contiguous(), dk.contiguous(), dv.contiguous(), dq.shape[0], True)
+        return dqkv, None, None, None, None, None, None
+
+
+def qkv_rope_fn(qkv: torch.Tensor, positions: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, hq: int, hkv: int,
+                head_dim: int):
+    """Cut a fused projection ``[rows, (hq + 2 hkv) * head_dim]`` into ``q``, ``k`` (rotated at
+    ``positions [tokens]``) and ``v``, each ``[tokens, heads, head_dim]``; rows past ``tokens`` are
+    padding. Differentiable; the bits of slicing and :func:`rope_fn`, in one launch per direction."""
+    tokens = positions.numel()
+    aligned = qkv.dim() == 2 and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0
+    if qkv.device.type == "cuda" and head_dim == 128 and qkv.dtype == torch.bfloat16 and aligned and 0 < tokens:
+        return _QkvRopeFn.apply(qkv, positions, cos, sin, hq, hkv, tokens)
+    q = qkv[:tokens, : hq * head_dim].reshape(tokens, hq, head_dim)
+    k = qkv[:tokens, hq * head_dim:(hq + hkv) * head_dim].reshape(tokens, hkv, head_dim)
+    v = qkv[:tokens, (hq + hkv) * head_dim:].reshape(tokens, hkv, head_dim)
+    return rope_fn(q, positions, cos, sin), rope_fn(k, positions, cos, sin), v
 
 
 class _SwigluFn(torch.autograd.Function):

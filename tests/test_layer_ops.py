@@ -73,3 +73,47 @@ def test_gpu_layer_ops_match_cpu_library(cuda_device):
     assert (out.float() - want.float()).abs().max() <= 0.07
     sep = swiglu(gu[:, :14336].contiguous().to(cuda_device), gu[:, 14336:].contiguous().to(cuda_device)).cpu()
     assert torch.equal(sep, out)
+
+
+@pytest.mark.parametrize("dev", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+@pytest.mark.parametrize("tokens,rows,hq,hkv", [(1, 128, 4, 2), (130, 256, 32, 8), (257, 257, 3, 1)])
+def test_qkv_rope_equals_slices_and_rope_bitwise(dev, tokens, rows, hq, hkv):
+    from kernel_align_b200.ops.layer_ops import qkv_rope_fn, rope_fn, rope_tables
+
+    g = torch.Generator(device=dev).manual_seed(tokens)
+    width = (hq + 2 * hkv) * 128
+    x = torch.randn(rows, width, device=dev, generator=g).to(torch.bfloat16)
+    cos, sin = rope_tables(64, 128, device=dev)
+    pos = torch.randint(0, 64, (tokens,), device=dev, generator=g)
+    a, b = x.clone().requires_grad_(), x.clone().requires_grad_()
+    got = qkv_rope_fn(a, pos, cos, sin, hq, hkv, 128)
+    cut = [b[:tokens, lo * 128:hi * 128].reshape(tokens, hi - lo, 128)
+           for lo, hi in ((0, hq), (hq, hq + hkv), (hq + hkv, hq + 2 * hkv))]
+    want = rope_fn(cut[0], pos, cos, sin), rope_fn(cut[1], pos, cos, sin), cut[2]
+    d = [torch.randn(t.shape, device=dev, generator=g).to(torch.bfloat16) for t in want]
+    torch.autograd.backward(got, d)
+    torch.autograd.backward(want, d)
+    assert all(torch.equal(p, q) for p, q in zip(got, want)) and torch.equal(a.grad, b.grad)
+
+
+@pytest.mark.parametrize("dev", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+@pytest.mark.parametrize("rows,d", [(1, 128), (17, 1024), (300, 4096), (64, 8192)])
+def test_rmsnorm_fork_adds_the_two_gradients(dev, rows, d):
+    from kernel_align_b200.ops.layer_ops import rmsnorm_fn, rmsnorm_fork_fn
+
+    g = torch.Generator(device=dev).manual_seed(rows)
+    x = torch.randn(rows, d, device=dev, generator=g).to(torch.bfloat16)
+    w = (torch.randn(d, device=dev, generator=g) * 0.1 + 1).to(torch.bfloat16)
+    dy, dr = (torch.randn(rows, d, device=dev, generator=g).to(torch.bfloat16) for _ in range(2))
+    grads = []
+    for fork in (True, False):
+        xi, wi = x.clone().requires_grad_(), w.clone().requires_grad_()
+        y, r = rmsnorm_fork_fn(xi, wi) if fork else (rmsnorm_fn(xi, wi), xi.clone())
+        assert torch.equal(r, x)
+        torch.autograd.backward((y, r), (dy, dr))
+        grads.append((y, xi.grad, wi.grad))
+    assert all(torch.equal(p, q) for p, q in zip(*grads))
+    # only one of the two outputs used
+    xi = x.clone().requires_grad_()
+    rmsnorm_fork_fn(xi, w)[1].backward(dr)
+    assert torch.equal(xi.grad, dr)
