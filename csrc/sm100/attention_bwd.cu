@@ -49,56 +49,94 @@ struct BwdParams {
   unsigned long long timeout_ns;
 };
 
-// delta[b, h, i] = sum_d dO * O (fp32), one warp per (token, head)
-__global__ void attention_delta_kernel(const __nv_bfloat16* __restrict__ o, long long o_stride,
-                                       const __nv_bfloat16* __restrict__ d_o, long long do_stride,
-                                       float* __restrict__ delta, int batch, int seq_len, int hq) {
-  const long long w = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const long long total = static_cast<long long>(batch) * seq_len * hq;
-  if (w >= total) return;
-  const int h = static_cast<int>(w % hq);
-  const long long tok = w / hq;
-  const uint2 a = *reinterpret_cast<const uint2*>(o + tok * o_stride + h * kD + lane * 4);
-  const uint2 b = *reinterpret_cast<const uint2*>(d_o + tok * do_stride + h * kD + lane * 4);
-  float acc = 0.f;
-  acc = __fmaf_rn(__uint_as_float(a.x << 16), __uint_as_float(b.x << 16), acc);
-  acc = __fmaf_rn(__uint_as_float(a.x & 0xFFFF0000u), __uint_as_float(b.x & 0xFFFF0000u), acc);
-  acc = __fmaf_rn(__uint_as_float(a.y << 16), __uint_as_float(b.y << 16), acc);
-  acc = __fmaf_rn(__uint_as_float(a.y & 0xFFFF0000u), __uint_as_float(b.y & 0xFFFF0000u), acc);
+// delta[b, h, i] = sum_d dO * O (fp32): 16 lanes x 16 bytes per (token, head), a block takes
+// kDeltaTokens consecutive tokens of one head, so that its results are contiguous and every
+// thread has four pairs of loads in flight (one 8-byte pair per warp and row took three times
+// the time of the bytes: 34 us for 4096 tokens x 32 heads, 67 MB).
+constexpr int kDeltaTokens = 64;
+
+__global__ void __launch_bounds__(256)
+attention_delta_kernel(const __nv_bfloat16* __restrict__ o, long long o_stride, const __nv_bfloat16* __restrict__ d_o,
+                       long long do_stride, float* __restrict__ delta, int seq_len, int hq) {
+  constexpr int kPer = kDeltaTokens / 16;
+  const int groups = (seq_len + kDeltaTokens - 1) / kDeltaTokens;
+  const int b = blockIdx.x / groups, h = blockIdx.y, ln = threadIdx.x & 15;
+  const int i0 = (blockIdx.x % groups) * kDeltaTokens + (threadIdx.x >> 4);
+  uint4 a[kPer], g[kPer];
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, off));
-  if (lane == 0) {
-    const int b_ = static_cast<int>(tok / seq_len), i = static_cast<int>(tok % seq_len);
-    delta[(static_cast<long long>(b_) * hq + h) * seq_len + i] = acc;
+  for (int n = 0; n < kPer; ++n) {
+    const int i = i0 + n * 16;
+    const long long tok = static_cast<long long>(b) * seq_len + i;
+    if (i < seq_len) {
+      a[n] = *reinterpret_cast<const uint4*>(o + tok * o_stride + h * kD + ln * 8);
+      g[n] = *reinterpret_cast<const uint4*>(d_o + tok * do_stride + h * kD + ln * 8);
+    } else {
+      a[n] = g[n] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < kPer; ++n) {
+    const uint32_t x[4] = {a[n].x, a[n].y, a[n].z, a[n].w}, y[4] = {g[n].x, g[n].y, g[n].z, g[n].w};
+    float acc = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      acc = __fmaf_rn(__uint_as_float(x[e] << 16), __uint_as_float(y[e] << 16), acc);
+      acc = __fmaf_rn(__uint_as_float(x[e] & 0xFFFF0000u), __uint_as_float(y[e] & 0xFFFF0000u), acc);
+    }
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, off));
+    const int i = i0 + n * 16;
+    if (ln == 0 && i < seq_len) delta[(static_cast<long long>(b) * hq + h) * seq_len + i] = acc;
   }
 }
 
+// (d0, d1) = (a0, a1) * (b0, b1), each lane rounded like mul.rn
+__device__ __forceinline__ void mul2(float& d0, float& d1, float a0, float a1, float b0, float b1) {
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "mul.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d0), "=f"(d1)
+      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+}
+
+// Offset (in 16-byte descriptor units) of K step kk of a 128 x 128 tile: K-major, MN-major.
+__device__ __forceinline__ constexpr uint64_t kstep(int kk) { return ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4; }
+__device__ __forceinline__ constexpr uint64_t mnstep(int kk) { return (kk * 2048) >> 4; }
+// Column of K step kk of a bf16 A operand that overlays a 128-column fp32 region: the threads of
+// part 0 write 32 packed columns over their own fp32 columns [0, 64), part 1 over [64, 128).
+__device__ __forceinline__ constexpr uint32_t tcol(int kk) { return kk < 4 ? kk * 8 : 64 + (kk - 4) * 8; }
+
+// ------------------------------------------------------------------------------------------------
+// Both kernels overlap the tensor core with the element-wise work: the operand of the next
+// iteration is in a second shared-memory stage, the next S and dP products are issued as soon as
+// their TMEM columns have been read, and the 16-bit operand that comes out of S goes back to TMEM
+// over the columns of S (the A operand of the product that follows), which leaves shared memory
+// to the loaded tiles. Tiles that need no mask take a path without comparisons.
+// One iteration is three products of 512 cycles (dQ) or four (dK / dV); with a single stage and
+// everything in sequence it took about 9000 cycles. B = 2, L = 4000, 32 / 8 heads, causal:
+// dQ 891 -> 521 us, dK / dV 1466 -> 1074 us; B = 8, L = 512: dQ 114 -> 68 us, dK / dV 173 -> 117 us.
+// ------------------------------------------------------------------------------------------------
 struct CtlDq {
-  uint64_t qdo_full;      // Q and dO tiles loaded
-  uint64_t kv_full, kv_empty;
-  uint64_t s_full;        // S and dP ready in TMEM
-  uint64_t ds_full;       // dS tile written (count: softmax warps)
-  uint64_t acc_full;      // final dQ ready
+  uint64_t qdo_full;                 // Q and dO tiles loaded
+  uint64_t kv_full[2], kv_empty[2];
+  uint64_t s_full[2];                // S ready in its TMEM buffer
+  uint64_t dp_full, dp_read;         // dP ready / read into registers (count: softmax warps)
+  uint64_t ds_full;                  // dS written over S (count: softmax warps)
+  uint64_t acc_full;                 // final dQ ready
   uint32_t tmem_base;
   int abort_flag;
 };
 
 // ------------------------------------------------------------------------------------------------
-// dQ kernel
+// dQ kernel. TMEM: S (two buffers), dP, dQ. Shared memory: Q, dO, two stages of (K, V).
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads, 1)
 attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                         const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                         const __grid_constant__ BwdParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t raw_addr = smem_u32(smem_raw);
-  const uint32_t base = (raw_addr + 1023u) & ~1023u;
-  uint8_t* smem = smem_raw + (base - raw_addr);
-  const uint32_t q_tile = base, do_tile = base + kTileBytes, k_tile = base + 2 * kTileBytes,
-                 v_tile = base + 3 * kTileBytes, ds_tile = base + 4 * kTileBytes;
-  uint8_t* ds_ptr = smem + 4 * kTileBytes;
-  CtlDq* ctl = reinterpret_cast<CtlDq*>(smem + 5 * kTileBytes);
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t base = smem_u32(smem_raw);
+  const uint32_t q_tile = base, do_tile = base + kTileBytes, ring = base + 2 * kTileBytes;  // stage: K, V
+  CtlDq* ctl = reinterpret_cast<CtlDq*>(smem_raw + 6 * kTileBytes);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_qt = (p.seq_len + kT - 1) / kT;
@@ -113,9 +151,13 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
 
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&ctl->qdo_full), 1);
-    mbar_init(smem_u32(&ctl->kv_full), 1);
-    mbar_init(smem_u32(&ctl->kv_empty), 1);
-    mbar_init(smem_u32(&ctl->s_full), 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(smem_u32(&ctl->kv_full[s]), 1);
+      mbar_init(smem_u32(&ctl->kv_empty[s]), 1);
+      mbar_init(smem_u32(&ctl->s_full[s]), 1);
+    }
+    mbar_init(smem_u32(&ctl->dp_full), 1);
+    mbar_init(smem_u32(&ctl->dp_read), kSoftThreads / 32);
     mbar_init(smem_u32(&ctl->ds_full), kSoftThreads / 32);
     mbar_init(smem_u32(&ctl->acc_full), 1);
     ctl->abort_flag = 0;
@@ -129,7 +171,7 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = ctl->tmem_base;
-  const uint32_t tmem_s = tmem_base, tmem_dp = tmem_base + 128, tmem_dq = tmem_base + 256;
+  const uint32_t tmem_dp = tmem_base + 256, tmem_dq = tmem_base + 384;   // S: tmem_base + 128 * buffer
 
   if (warp == kWarpTma) {
     if (lane == 0) {
@@ -140,8 +182,10 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       tma_load_2d(do_tile, &tm_do, h * kD, tok0 + q_row0, f);
       tma_load_2d(do_tile + 16384, &tm_do, h * kD + 64, tok0 + q_row0, f);
       for (int j = 0; j < n_kv; ++j) {
-        if (!mbar_wait_bounded(smem_u32(&ctl->kv_empty), (j & 1) ^ 1u, wctx, 41, j)) break;
-        const uint32_t full = smem_u32(&ctl->kv_full);
+        const int s = j & 1;
+        if (!mbar_wait_bounded(smem_u32(&ctl->kv_empty[s]), ((j >> 1) & 1) ^ 1u, wctx, 41, j)) break;
+        const uint32_t full = smem_u32(&ctl->kv_full[s]);
+        const uint32_t k_tile = ring + s * 2 * kTileBytes, v_tile = k_tile + kTileBytes;
         mbar_arrive_expect_tx(full, 2 * kTileBytes);
         const int row = tok0 + j * kT;
         tma_load_2d(k_tile, &tm_k, hk * kD, row, full);
@@ -154,25 +198,52 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     if (lane == 0) {
       const uint32_t idesc_kk = umma_idesc_bf16_f32(kT, kT);             // both operands K-major
       const uint32_t idesc_kmn = umma_idesc_bf16_f32(kT, kD) | (1u << 16);  // B MN-major
-      bool ok = mbar_wait_bounded(smem_u32(&ctl->qdo_full), 0, wctx, 42, 0);
-      for (int j = 0; j < n_kv && ok; ++j) {
-        ok = mbar_wait_bounded(smem_u32(&ctl->kv_full), j & 1, wctx, 43, j);
-        if (!ok) break;
+      const uint64_t d_q = desc_kmajor(q_tile, 0), d_do = desc_kmajor(do_tile, 0), d_ring = desc_kmajor(ring, 0),
+                     d_ring_mn = desc_mnmajor(ring, 0);
+      constexpr uint64_t kStage = (2 * kTileBytes) >> 4, kTile = kTileBytes >> 4;
+      auto issue_s = [&](int j) {      // S = Q K^T
+        const uint64_t dk = d_ring + (j & 1) * kStage;
+#pragma unroll
+        for (int kk = 0; kk < kD / 16; ++kk)
+          umma_bf16<1>(tmem_base + (j & 1) * 128, d_q + kstep(kk), dk + kstep(kk), idesc_kk, kk > 0 ? 1u : 0u);
+        umma_commit<1>(smem_u32(&ctl->s_full[j & 1]));
+      };
+      auto issue_dp = [&](int j) {     // dP = dO V^T
+        const uint64_t dv = d_ring + (j & 1) * kStage + kTile;
+#pragma unroll
+        for (int kk = 0; kk < kD / 16; ++kk)
+          umma_bf16<1>(tmem_dp, d_do + kstep(kk), dv + kstep(kk), idesc_kk, kk > 0 ? 1u : 0u);
+        umma_commit<1>(smem_u32(&ctl->dp_full));
+      };
+      bool ok = mbar_wait_bounded(smem_u32(&ctl->qdo_full), 0, wctx, 42, 0) &&
+                mbar_wait_bounded(smem_u32(&ctl->kv_full[0]), 0, wctx, 43, 0);
+      if (ok) {
         tc_fence_after_sync();
-#pragma unroll
-        for (int kk = 0; kk < kD / 16; ++kk)  // S = Q K^T
-          umma_bf16<1>(tmem_s, desc_kmajor(q_tile, kk), desc_kmajor(k_tile, kk), idesc_kk, kk > 0 ? 1u : 0u);
-#pragma unroll
-        for (int kk = 0; kk < kD / 16; ++kk)  // dP = dO V^T
-          umma_bf16<1>(tmem_dp, desc_kmajor(do_tile, kk), desc_kmajor(v_tile, kk), idesc_kk, kk > 0 ? 1u : 0u);
-        umma_commit<1>(smem_u32(&ctl->s_full));
+        issue_s(0);
+        issue_dp(0);
+      }
+      for (int j = 0; j < n_kv && ok; ++j) {
+        if (j + 1 < n_kv) {
+          // S(j + 1) goes over dS(j - 1), whose product was issued an iteration ago; the tensor
+          // core executes in issue order
+          ok = mbar_wait_bounded(smem_u32(&ctl->kv_full[(j + 1) & 1]), ((j + 1) >> 1) & 1, wctx, 43, j + 1);
+          if (!ok) break;
+          tc_fence_after_sync();
+          issue_s(j + 1);
+          ok = mbar_wait_bounded(smem_u32(&ctl->dp_read), j & 1, wctx, 47, j);
+          if (!ok) break;
+          tc_fence_after_sync();
+          issue_dp(j + 1);
+        }
         ok = mbar_wait_bounded(smem_u32(&ctl->ds_full), j & 1, wctx, 44, j);
         if (!ok) break;
         tc_fence_after_sync();
+        const uint64_t dk = d_ring_mn + (j & 1) * kStage;
 #pragma unroll
         for (int kk = 0; kk < kT / 16; ++kk)  // dQ += dS K
-          umma_bf16<1>(tmem_dq, desc_kmajor(ds_tile, kk), desc_mnmajor(k_tile, kk), idesc_kmn, (j > 0 || kk > 0) ? 1u : 0u);
-        umma_commit<1>(smem_u32(&ctl->kv_empty));
+          umma_bf16_ts(tmem_dq, tmem_base + (j & 1) * 128 + tcol(kk), dk + mnstep(kk), idesc_kmn,
+                       (j > 0 || kk > 0) ? 1u : 0u);
+        umma_commit<1>(smem_u32(&ctl->kv_empty[j & 1]));
         if (j + 1 == n_kv) umma_commit<1>(smem_u32(&ctl->acc_full));
       }
     }
@@ -185,41 +256,67 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     const bool row_ok = q_pos < p.seq_len;
     const long long stat = (static_cast<long long>(b) * p.hq + h) * p.seq_len + q_pos;
     const float neg_lse2 = row_ok ? __fmul_rn(-p.lse[stat], kLog2e) : 0.f;
-    const float dlt = row_ok ? p.delta[stat] : 0.f;
+    const float neg_dlt = row_ok ? -p.delta[stat] : 0.f;
     bool ok = true;
     for (int j = 0; j < n_kv && ok; ++j) {
-      const bool mine = mbar_wait_bounded(smem_u32(&ctl->s_full), j & 1, wctx, 45, j);
+      bool mine = mbar_wait_bounded(smem_u32(&ctl->s_full[j & 1]), (j >> 1) & 1, wctx, 45, j);
       ok = __all_sync(0xffffffffu, mine) != 0;
       if (!ok) break;
       tc_fence_after_sync();
+      const uint32_t tmem_s = tmem_base + static_cast<uint32_t>((j & 1) * 128 + part * 64) + lane_base;
+      uint32_t s0[32], s1[32], g0[32], g1[32];
+      __syncwarp();
+      tmem_ld_32x32(tmem_s, s0);
+      tmem_ld_32x32(tmem_s + 32, s1);
+      tmem_ld_wait_dep(s0);
+      tmem_ld_wait_dep(s1);
       const int kv0 = j * kT + part * 64;
-      const int limit = row_ok ? ((p.causal ? min(q_pos, p.seq_len - 1) : p.seq_len - 1) - kv0) : -1;
-#pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        uint32_t sv[32], dv[32];
-        __syncwarp();
-        tmem_ld_32x32(tmem_s + lane_base + part * 64 + g * 32, sv);
-        tmem_ld_32x32(tmem_dp + lane_base + part * 64 + g * 32, dv);
-        tmem_ld_wait_dep(sv);
-        tmem_ld_wait_dep(dv);
-        uint32_t w[16];
+      const bool full = p.causal ? j < qt : (j + 1) * kT <= p.seq_len;   // uniform over the CTA
+      const int limit = full ? 64 : (row_ok ? ((p.causal ? q_pos : p.seq_len - 1) - kv0) : -1);
+      auto probs = [&](uint32_t (&sv)[32]) {
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          float d0 = 0.f, d1 = 0.f;
-          if (g * 32 + i <= limit) {
-            const float pr = ex2_approx(__fmaf_rn(__uint_as_float(sv[i]), c, neg_lse2));
-            d0 = __fmul_rn(__fmul_rn(pr, __fsub_rn(__uint_as_float(dv[i]), dlt)), p.scale);
-          }
-          if (g * 32 + i + 1 <= limit) {
-            const float pr = ex2_approx(__fmaf_rn(__uint_as_float(sv[i + 1]), c, neg_lse2));
-            d1 = __fmul_rn(__fmul_rn(pr, __fsub_rn(__uint_as_float(dv[i + 1]), dlt)), p.scale);
-          }
-          w[i >> 1] = pack_bf16(d0, d1);
+          float e0, e1;
+          fma2(e0, e1, __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]), c, c, neg_lse2, neg_lse2);
+          sv[i] = __float_as_uint(ex2_approx(e0));
+          sv[i + 1] = __float_as_uint(ex2_approx(e1));
         }
-        store_tile_row32(ds_ptr, row, part * 64 + g * 32, w);
-      }
+      };
+      probs(s0);
+      probs(s1);
+      mine = mbar_wait_bounded(smem_u32(&ctl->dp_full), j & 1, wctx, 45, j);
+      ok = __all_sync(0xffffffffu, mine) != 0;
+      if (!ok) break;
+      tc_fence_after_sync();
+      __syncwarp();
+      tmem_ld_32x32(tmem_dp + lane_base + part * 64, g0);
+      tmem_ld_32x32(tmem_dp + lane_base + part * 64 + 32, g1);
+      tmem_ld_wait_dep(g0);
+      tmem_ld_wait_dep(g1);
       tc_fence_before_sync();
-      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&ctl->dp_read));
+      auto grads = [&](uint32_t (&sv)[32], uint32_t (&gv)[32], int col) {   // packed into sv[0 .. 15]
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          float d0, d1;
+          add2(d0, d1, __uint_as_float(gv[i]), __uint_as_float(gv[i + 1]), neg_dlt, neg_dlt);
+          mul2(d0, d1, __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]), d0, d1);
+          mul2(d0, d1, d0, d1, p.scale, p.scale);
+          if (!full) {
+            if (col + i > limit) d0 = 0.f;
+            if (col + i + 1 > limit) d1 = 0.f;
+          }
+          sv[i >> 1] = pack_bf16(d0, d1);
+        }
+      };
+      grads(s0, g0, 0);
+      grads(s1, g1, 32);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) s0[16 + i] = s1[i];
+      tmem_st_32x32(tmem_s, s0);
+      tmem_st_wait();
+      tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&ctl->ds_full));
     }
@@ -259,33 +356,33 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
 }
 
 // ------------------------------------------------------------------------------------------------
-// dK / dV kernel
+// dK / dV kernel. TMEM: S^T (then P^T as bf16 over it), dP^T, dV, dK. Shared memory: K, V, two
+// stages of (Q, dO), dS^T.
 // ------------------------------------------------------------------------------------------------
 struct CtlDkv {
-  uint64_t kv_full;       // K and V tiles loaded (once)
-  uint64_t qdo_full, qdo_empty;
-  uint64_t st_full;       // S^T and dP^T ready in TMEM
-  uint64_t pds_full;      // P^T and dS^T tiles written (count: softmax warps)
+  uint64_t kv_full;                  // K and V tiles loaded (once)
+  uint64_t qdo_full[2], qdo_empty[2];
+  uint64_t st_full;                  // S^T ready in TMEM
+  uint64_t p_full;                   // P^T written over S^T (count: softmax warps)
+  uint64_t dp_full, dp_read;         // dP^T ready / read into registers (count: softmax warps)
+  uint64_t ds_full, ds_empty;        // dS^T tile written (count: softmax warps) / consumed
   uint64_t acc_full;
   uint32_t tmem_base;
   int abort_flag;
-  float lse2[2][kT];      // -lse * log2(e) of the current q tile, double-buffered by iteration
-  float delta[2][kT];
+  alignas(16) float lse2[2][kT];     // -lse * log2(e) of the current q tile, double-buffered by iteration
+  alignas(16) float neg_delta[2][kT];
 };
 
 __global__ void __launch_bounds__(kThreads, 1)
 attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                          const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                          const __grid_constant__ BwdParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t raw_addr = smem_u32(smem_raw);
-  const uint32_t base = (raw_addr + 1023u) & ~1023u;
-  uint8_t* smem = smem_raw + (base - raw_addr);
-  const uint32_t k_tile = base, v_tile = base + kTileBytes, q_tile = base + 2 * kTileBytes,
-                 do_tile = base + 3 * kTileBytes, pt_tile = base + 4 * kTileBytes, dst_tile = base + 5 * kTileBytes;
-  uint8_t* pt_ptr = smem + 4 * kTileBytes;
-  uint8_t* dst_ptr = smem + 5 * kTileBytes;
-  CtlDkv* ctl = reinterpret_cast<CtlDkv*>(smem + 6 * kTileBytes);
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t base = smem_u32(smem_raw);
+  const uint32_t k_tile = base, v_tile = base + kTileBytes, ring = base + 2 * kTileBytes,   // stage: Q, dO
+                 dst_tile = base + 6 * kTileBytes;
+  uint8_t* dst_ptr = smem_raw + 6 * kTileBytes;
+  CtlDkv* ctl = reinterpret_cast<CtlDkv*>(smem_raw + 7 * kTileBytes);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_t = (p.seq_len + kT - 1) / kT;
@@ -301,10 +398,16 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
 
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&ctl->kv_full), 1);
-    mbar_init(smem_u32(&ctl->qdo_full), 1);
-    mbar_init(smem_u32(&ctl->qdo_empty), 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(smem_u32(&ctl->qdo_full[s]), 1);
+      mbar_init(smem_u32(&ctl->qdo_empty[s]), 1);
+    }
     mbar_init(smem_u32(&ctl->st_full), 1);
-    mbar_init(smem_u32(&ctl->pds_full), kSoftThreads / 32);
+    mbar_init(smem_u32(&ctl->p_full), kSoftThreads / 32);
+    mbar_init(smem_u32(&ctl->dp_full), 1);
+    mbar_init(smem_u32(&ctl->dp_read), kSoftThreads / 32);
+    mbar_init(smem_u32(&ctl->ds_full), kSoftThreads / 32);
+    mbar_init(smem_u32(&ctl->ds_empty), 1);
     mbar_init(smem_u32(&ctl->acc_full), 1);
     ctl->abort_flag = 0;
     fence_mbar_init_cluster();
@@ -328,9 +431,10 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       tma_load_2d(v_tile, &tm_v, hk * kD, tok0 + kv_row0, f);
       tma_load_2d(v_tile + 16384, &tm_v, hk * kD + 64, tok0 + kv_row0, f);
       for (int n = 0; n < n_iter; ++n) {
-        const int h = hk * group + n / n_q, qt = qt0 + n % n_q;
-        if (!mbar_wait_bounded(smem_u32(&ctl->qdo_empty), (n & 1) ^ 1u, wctx, 51, n)) break;
-        const uint32_t full = smem_u32(&ctl->qdo_full);
+        const int h = hk * group + n / n_q, qt = qt0 + n % n_q, s = n & 1;
+        if (!mbar_wait_bounded(smem_u32(&ctl->qdo_empty[s]), ((n >> 1) & 1) ^ 1u, wctx, 51, n)) break;
+        const uint32_t full = smem_u32(&ctl->qdo_full[s]);
+        const uint32_t q_tile = ring + s * 2 * kTileBytes, do_tile = q_tile + kTileBytes;
         mbar_arrive_expect_tx(full, 2 * kTileBytes);
         const int row = tok0 + qt * kT;
         tma_load_2d(q_tile, &tm_q, h * kD, row, full);
@@ -343,28 +447,58 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     if (lane == 0) {
       const uint32_t idesc_kk = umma_idesc_bf16_f32(kT, kT);
       const uint32_t idesc_kmn = umma_idesc_bf16_f32(kT, kD) | (1u << 16);
-      bool ok = mbar_wait_bounded(smem_u32(&ctl->kv_full), 0, wctx, 52, 0);
-      for (int n = 0; n < n_iter && ok; ++n) {
-        ok = mbar_wait_bounded(smem_u32(&ctl->qdo_full), n & 1, wctx, 53, n);
-        if (!ok) break;
-        tc_fence_after_sync();
+      const uint64_t d_k = desc_kmajor(k_tile, 0), d_v = desc_kmajor(v_tile, 0), d_ring = desc_kmajor(ring, 0),
+                     d_ring_mn = desc_mnmajor(ring, 0), d_ds = desc_kmajor(dst_tile, 0);
+      constexpr uint64_t kStage = (2 * kTileBytes) >> 4, kTile = kTileBytes >> 4;
+      auto issue_st = [&](int n) {     // S^T = K Q^T
+        const uint64_t dq = d_ring + (n & 1) * kStage;
 #pragma unroll
-        for (int kk = 0; kk < kD / 16; ++kk)  // S^T = K Q^T
-          umma_bf16<1>(tmem_st, desc_kmajor(k_tile, kk), desc_kmajor(q_tile, kk), idesc_kk, kk > 0 ? 1u : 0u);
-#pragma unroll
-        for (int kk = 0; kk < kD / 16; ++kk)  // dP^T = V dO^T
-          umma_bf16<1>(tmem_dpt, desc_kmajor(v_tile, kk), desc_kmajor(do_tile, kk), idesc_kk, kk > 0 ? 1u : 0u);
+        for (int kk = 0; kk < kD / 16; ++kk)
+          umma_bf16<1>(tmem_st, d_k + kstep(kk), dq + kstep(kk), idesc_kk, kk > 0 ? 1u : 0u);
         umma_commit<1>(smem_u32(&ctl->st_full));
-        ok = mbar_wait_bounded(smem_u32(&ctl->pds_full), n & 1, wctx, 54, n);
+      };
+      auto issue_dpt = [&](int n) {    // dP^T = V dO^T
+        const uint64_t ddo = d_ring + (n & 1) * kStage + kTile;
+#pragma unroll
+        for (int kk = 0; kk < kD / 16; ++kk)
+          umma_bf16<1>(tmem_dpt, d_v + kstep(kk), ddo + kstep(kk), idesc_kk, kk > 0 ? 1u : 0u);
+        umma_commit<1>(smem_u32(&ctl->dp_full));
+      };
+      bool ok = mbar_wait_bounded(smem_u32(&ctl->kv_full), 0, wctx, 52, 0) &&
+                mbar_wait_bounded(smem_u32(&ctl->qdo_full[0]), 0, wctx, 53, 0);
+      if (ok) {
+        tc_fence_after_sync();
+        issue_st(0);
+        issue_dpt(0);
+      }
+      for (int n = 0; n < n_iter && ok; ++n) {
+        ok = mbar_wait_bounded(smem_u32(&ctl->p_full), n & 1, wctx, 54, n);
         if (!ok) break;
         tc_fence_after_sync();
+        const uint64_t ddo = d_ring_mn + (n & 1) * kStage + kTile;
 #pragma unroll
         for (int kk = 0; kk < kT / 16; ++kk)  // dV += P^T dO
-          umma_bf16<1>(tmem_dv, desc_kmajor(pt_tile, kk), desc_mnmajor(do_tile, kk), idesc_kmn, (n > 0 || kk > 0) ? 1u : 0u);
+          umma_bf16_ts(tmem_dv, tmem_st + tcol(kk), ddo + mnstep(kk), idesc_kmn, (n > 0 || kk > 0) ? 1u : 0u);
+        if (n + 1 < n_iter) {
+          // S^T(n + 1) goes over P^T(n): the tensor core executes in issue order
+          ok = mbar_wait_bounded(smem_u32(&ctl->qdo_full[(n + 1) & 1]), ((n + 1) >> 1) & 1, wctx, 53, n + 1);
+          if (!ok) break;
+          tc_fence_after_sync();
+          issue_st(n + 1);
+          ok = mbar_wait_bounded(smem_u32(&ctl->dp_read), n & 1, wctx, 57, n);
+          if (!ok) break;
+          tc_fence_after_sync();
+          issue_dpt(n + 1);
+        }
+        ok = mbar_wait_bounded(smem_u32(&ctl->ds_full), n & 1, wctx, 58, n);
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint64_t dq = d_ring_mn + (n & 1) * kStage;
 #pragma unroll
         for (int kk = 0; kk < kT / 16; ++kk)  // dK += dS^T Q
-          umma_bf16<1>(tmem_dk, desc_kmajor(dst_tile, kk), desc_mnmajor(q_tile, kk), idesc_kmn, (n > 0 || kk > 0) ? 1u : 0u);
-        umma_commit<1>(smem_u32(&ctl->qdo_empty));
+          umma_bf16<1>(tmem_dk, d_ds + kstep(kk), dq + mnstep(kk), idesc_kmn, (n > 0 || kk > 0) ? 1u : 0u);
+        umma_commit<1>(smem_u32(&ctl->ds_empty));
+        umma_commit<1>(smem_u32(&ctl->qdo_empty[n & 1]));
         if (n + 1 == n_iter) umma_commit<1>(smem_u32(&ctl->acc_full));
       }
     }
@@ -377,18 +511,22 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     const bool row_ok = kv_pos < p.seq_len;
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const float c = p.scale * kLog2e;
+    const uint32_t tmem_s = tmem_st + lane_base + part * 64, tmem_g = tmem_dpt + lane_base + part * 64;
     bool ok = true;
+    // row statistics of the q tile of iteration n: threads 0..127 the log-sum-exp, 128..255 delta
+    auto stat_of = [&](int n) {
+      const int h = hk * group + n / n_q, qp = (qt0 + n % n_q) * kT + row;
+      if (qp >= p.seq_len) return 0.f;
+      const long long at = (static_cast<long long>(b) * p.hq + h) * p.seq_len + qp;
+      return part == 0 ? __fmul_rn(-p.lse[at], kLog2e) : -p.delta[at];
+    };
+    float next_stat = n_iter > 0 ? stat_of(0) : 0.f;
     for (int n = 0; n < n_iter; ++n) {
-      const int h = hk * group + n / n_q, qt = qt0 + n % n_q;
+      const int qt = qt0 + n % n_q;
       const int buf = n & 1;
-      if (tid < kT) {
-        const int qp = qt * kT + tid;
-        const long long stat = (static_cast<long long>(b) * p.hq + h) * p.seq_len + qp;
-        const bool v_ok = qp < p.seq_len;
-        ctl->lse2[buf][tid] = v_ok ? __fmul_rn(-p.lse[stat], kLog2e) : 0.f;
-        ctl->delta[buf][tid] = v_ok ? p.delta[stat] : 0.f;
-      }
+      (part == 0 ? ctl->lse2[buf] : ctl->neg_delta[buf])[row] = next_stat;
       asm volatile("bar.sync 1, %0;" ::"n"(kSoftThreads) : "memory");
+      if (n + 1 < n_iter) next_stat = stat_of(n + 1);
       if (ctl->abort_flag) ok = false;
       if (ok) {
         const bool mine = mbar_wait_bounded(smem_u32(&ctl->st_full), n & 1, wctx, 55, n);
@@ -397,41 +535,99 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       if (!ok) continue;
       tc_fence_after_sync();
       const int q0 = qt * kT + part * 64;  // first query column of this thread
+      const bool full = (!p.causal || qt > jt) && (qt + 1) * kT <= p.seq_len;   // uniform over the CTA
+      const float4* lse4 = reinterpret_cast<const float4*>(&ctl->lse2[buf][part * 64]);
+      const float4* dlt4 = reinterpret_cast<const float4*>(&ctl->neg_delta[buf][part * 64]);
+      uint32_t s0[32], s1[32];
+      __syncwarp();
+      tmem_ld_32x32(tmem_s, s0);
+      tmem_ld_32x32(tmem_s + 32, s1);
+      tmem_ld_wait_dep(s0);
+      tmem_ld_wait_dep(s1);
+      // P (kept in fp32 for dS), packed for the product
+      uint32_t w[32];
+      auto probs = [&](uint32_t (&sv)[32], int g) {
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        uint32_t sv[32], dv[32];
-        __syncwarp();
-        tmem_ld_32x32(tmem_st + lane_base + part * 64 + g * 32, sv);
-        tmem_ld_32x32(tmem_dpt + lane_base + part * 64 + g * 32, dv);
-        tmem_ld_wait_dep(sv);
-        tmem_ld_wait_dep(dv);
-        uint32_t wp[16], wd[16];
+        for (int i = 0; i < 32; i += 4) {
+          const float4 l = lse4[(g * 32 + i) >> 2];
+          float e[4];
+          fma2(e[0], e[1], __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]), c, c, l.x, l.y);
+          fma2(e[2], e[3], __uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3]), c, c, l.z, l.w);
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float pv[2], dsv[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int col = part * 64 + g * 32 + i + e;   // inside the q tile
-            const int qp = q0 + g * 32 + i + e;           // position in the sequence
-            const bool valid = row_ok && qp < p.seq_len && (!p.causal || kv_pos <= qp);
-            float pr = 0.f, ds = 0.f;
-            if (valid) {
-              pr = ex2_approx(__fmaf_rn(__uint_as_float(sv[i + e]), c, ctl->lse2[buf][col]));
-              ds = __fmul_rn(__fmul_rn(pr, __fsub_rn(__uint_as_float(dv[i + e]), ctl->delta[buf][col])), p.scale);
+          for (int k = 0; k < 4; ++k) {
+            e[k] = ex2_approx(e[k]);
+            if (!full) {
+              const int qp = q0 + g * 32 + i + k;
+              if (!(row_ok && qp < p.seq_len && (!p.causal || kv_pos <= qp))) e[k] = 0.f;
             }
-            pv[e] = pr;
-            dsv[e] = ds;
+            sv[i + k] = __float_as_uint(e[k]);
           }
-          wp[i >> 1] = pack_bf16(pv[0], pv[1]);
-          wd[i >> 1] = pack_bf16(dsv[0], dsv[1]);
+          w[(g * 32 + i) >> 1] = pack_bf16(e[0], e[1]);
+          w[((g * 32 + i) >> 1) + 1] = pack_bf16(e[2], e[3]);
         }
-        store_tile_row32(pt_ptr, row, part * 64 + g * 32, wp);
-        store_tile_row32(dst_ptr, row, part * 64 + g * 32, wd);
-      }
+      };
+      probs(s0, 0);
+      probs(s1, 1);
+      tmem_st_32x32(tmem_s, w);
+      tmem_st_wait();
       tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&ctl->p_full));
+      bool mine = mbar_wait_bounded(smem_u32(&ctl->dp_full), n & 1, wctx, 55, n);
+      ok = __all_sync(0xffffffffu, mine) != 0;
+      if (!ok) continue;
+      tc_fence_after_sync();
+      uint32_t g0[32], g1[32];
+      __syncwarp();
+      tmem_ld_32x32(tmem_g, g0);
+      tmem_ld_32x32(tmem_g + 32, g1);
+      tmem_ld_wait_dep(g0);
+      tmem_ld_wait_dep(g1);
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&ctl->dp_read));
+      auto grads = [&](const uint32_t (&pv)[32], const uint32_t (&gv)[32], int g) {
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+          const float4 d = dlt4[(g * 32 + i) >> 2];
+          float t[4];
+          add2(t[0], t[1], __uint_as_float(gv[i]), __uint_as_float(gv[i + 1]), d.x, d.y);
+          add2(t[2], t[3], __uint_as_float(gv[i + 2]), __uint_as_float(gv[i + 3]), d.z, d.w);
+          mul2(t[0], t[1], __uint_as_float(pv[i]), __uint_as_float(pv[i + 1]), t[0], t[1]);
+          mul2(t[2], t[3], __uint_as_float(pv[i + 2]), __uint_as_float(pv[i + 3]), t[2], t[3]);
+          mul2(t[0], t[1], t[0], t[1], p.scale, p.scale);
+          mul2(t[2], t[3], t[2], t[3], p.scale, p.scale);
+          if (!full) {       // a masked column may hold anything: 0 * it need not be 0
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const int qp = q0 + g * 32 + i + k;
+              if (!(row_ok && qp < p.seq_len && (!p.causal || kv_pos <= qp))) t[k] = 0.f;
+            }
+          }
+          w[(g * 32 + i) >> 1] = pack_bf16(t[0], t[1]);
+          w[((g * 32 + i) >> 1) + 1] = pack_bf16(t[2], t[3]);
+        }
+      };
+      grads(s0, g0, 0);
+      grads(s1, g1, 1);
+      if (n > 0) {           // the product of the previous dS^T has read the tile
+        mine = mbar_wait_bounded(smem_u32(&ctl->ds_empty), (n - 1) & 1, wctx, 59, n);
+        ok = __all_sync(0xffffffffu, mine) != 0;
+        if (!ok) continue;
+      }
+      {
+        uint32_t lo[16], hi[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          lo[i] = w[i];
+          hi[i] = w[16 + i];
+        }
+        store_tile_row32(dst_ptr, row, part * 64, lo);
+        store_tile_row32(dst_ptr, row, part * 64 + 32, hi);
+      }
       fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&ctl->pds_full));
+      if (lane == 0) mbar_arrive(smem_u32(&ctl->ds_full));
     }
     if (ok && n_iter > 0) {
       const bool mine = mbar_wait_bounded(smem_u32(&ctl->acc_full), 0, wctx, 56, 0);
@@ -492,8 +688,9 @@ extern "C" int ka_attention_bwd(const void* q, long long q_stride, const void* k
   if (batch <= 0 || seq_len <= 0) return 0;
   if (head_dim != kD || hq % hkv != 0) return -1;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  constexpr int kSmemDq = 5 * kTileBytes + 1024 + 256;
-  constexpr int kSmemDkv = 6 * kTileBytes + 1024 + 2304;
+  constexpr int kSmemDq = 6 * kTileBytes + 256;
+  constexpr int kSmemDkv = 7 * kTileBytes + 2304;
+  static_assert(sizeof(CtlDq) <= 256 && sizeof(CtlDkv) <= 2304 && kSmemDkv <= 227 * 1024, "shared memory layout");
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(attention_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemDq) != cudaSuccess ||
@@ -515,10 +712,11 @@ extern "C" int ka_attention_bwd(const void* q, long long q_stride, const void* k
   rc = make_tmap_2d_16bit_sw128(&tdo, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, d_o, tokens, static_cast<uint64_t>(hq) * kD,
                                 do_stride, kT, 64);
   if (rc) return -80 + rc;
-  const long long n_warps = static_cast<long long>(tokens) * hq;
-  attention_delta_kernel<<<static_cast<unsigned>((n_warps * 32 + 255) / 256), 256, 0, st>>>(
-      static_cast<const __nv_bfloat16*>(o), o_stride, static_cast<const __nv_bfloat16*>(d_o), do_stride, delta, batch,
-      seq_len, hq);
+  const dim3 delta_grid(static_cast<unsigned>((seq_len + kDeltaTokens - 1) / kDeltaTokens) * batch,
+                        static_cast<unsigned>(hq));
+  attention_delta_kernel<<<delta_grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(o), o_stride,
+                                                     static_cast<const __nv_bfloat16*>(d_o), do_stride, delta, seq_len,
+                                                     hq);
   BwdParams p = {};
   p.lse = lse;
   p.delta = delta;

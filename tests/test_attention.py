@@ -65,7 +65,8 @@ def test_gpu_attention_invariance_and_fused_qkv_views(cuda_device):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("b,l,hq,hkv,causal", [(2, 128, 4, 2, True), (2, 512, 8, 2, True), (1, 300, 4, 4, True),
-                                                (2, 256, 4, 1, False)])
+                                                (2, 256, 4, 1, False), (2, 1, 4, 2, True), (1, 129, 8, 1, True),
+                                                (2, 257, 2, 2, False), (1, 1030, 4, 2, True)])
 def test_gpu_attention_backward_matches_autograd(cuda_device, b, l, hq, hkv, causal):
     from kernel_align_b200.ops.attention import attention_fn
     from kernel_align_b200.ops.gemm import check_status
