@@ -785,6 +785,353 @@ __device__ void descend16(const T* rp, int v, bool vec_ok, float inv_temp, float
   __syncthreads();
 }
 
+// ---- 16-bit rows: everything from one histogram of counts per key -----------------------------
+// A bf16 or fp16 value has 65536 keys and the mass of a key is a function of the key, so one
+// pass that counts elements per key answers every question about (count, mass) prefixes: the
+// maximum, the total mass and both thresholds cost one exponential per distinct value instead
+// of one per element and pass. The draw needs sums in token-id order: the row is cut into 32
+// contiguous segments, one per warp, whose kept masses are order-free integer sums (coalesced
+// loads, masses from a table), the segment that holds the target is cut into 32 again, and only
+// the last hundred elements are walked in order.
+//   * Counters are 16 bits, two per word (128 KiB for all 65536 keys). An overflow loses at
+//     least 65535 from the sum of the counters, so "sum == v" says that none happened; a row
+//     in which one value fills more than 65535 places takes the older search.
+//   * The table of masses reuses the histogram's memory: groups of 32 keys that hold kept
+//     elements get consecutive slots (at most 1024; a row that needs more, i.e. with values in
+//     every corner of the format, takes the older search). A mass of 2^32 (probability 1) is
+//     stored as 2^32 - 1, which no smaller float maps to.
+// Measured, bf16 [200, 128256] ~ N(0, 2), T = 1, top_p = 0.9: 227 us with an exponential per
+// element for the total and ordered walks of the row in the draw, 113 us this way.
+constexpr int kGroups = 2048;                 // of 32 keys; GeneralSmem::cnt / mass hold their sums
+constexpr int kTableGroups = 1024;
+constexpr int kHistWords = 32768;
+static_assert(kGroups == kBins && kGroups == 2 * kThreads, "two groups per thread, sums kept in the descent's bins");
+
+struct FastSmem {
+  unsigned int words[kHistWords];             // 16-bit counters, then the table of masses
+  unsigned short slot[kGroups];
+  unsigned long long seg_ties[kWarps];
+  unsigned long long seg_mass[kWarps];
+  unsigned int total;
+  unsigned int max_key;
+  // result of a search / of a level of the draw
+  int sel;
+  unsigned int sel_key;
+  unsigned long long above_cnt, above_mass, present;
+  unsigned long long ties_before, target;
+};
+
+template <typename T>
+__device__ __forceinline__ float key16_float(uint32_t k16) {
+  if (k16 == 0) return key_to_float(0u);  // NaN
+  return Elem<T>::to_float(from_bits16<T>((k16 & 0x8000u) ? (k16 & 0x7FFFu) : (~k16 & 0xFFFFu)));
+}
+template <typename T>
+__device__ __forceinline__ unsigned long long key16_mass_of(uint32_t k16, float inv_temp, float y_max) {
+  return mass_fixed(exp_det(sub_rn(mul_rn(key16_float<T>(k16), inv_temp), y_max)));
+}
+
+__device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ unsigned long long warp_incl_u64(unsigned long long v) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long n = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += n;
+  }
+  return v;
+}
+
+__device__ __forceinline__ unsigned int key_count(const FastSmem& f, uint32_t k16) {
+  return (f.words[k16 >> 1] >> ((k16 & 1u) * 16u)) & 0xFFFFu;
+}
+
+// descend()'s contract on the histogram: groups by a block scan from the top, the key inside the
+// group by one warp.
+template <typename T>
+__device__ void search_groups(bool by_mass, unsigned long long limit, float inv_temp, float y_max, GeneralSmem& s,
+                              FastSmem& f) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) f.sel = -1;
+  const int g0 = kGroups - 1 - 2 * tid;       // this thread's groups, from the top: g0, g0 - 1
+  const unsigned long long c0 = s.cnt[g0], c1 = s.cnt[g0 - 1], m0 = s.mass[g0], m1 = s.mass[g0 - 1];
+  unsigned long long tot_c, tot_m;
+  unsigned long long c = block_exscan_u64(c0 + c1, s.scan, tot_c), m = block_exscan_u64(m0 + m1, s.scan, tot_m);
+  const unsigned long long pre = by_mass ? m : c, mid = pre + (by_mass ? m0 : c0), end = mid + (by_mass ? m1 : c1);
+  if (pre <= limit && end > limit) {
+    const bool second = mid <= limit;
+    f.sel = second ? g0 - 1 : g0;
+    f.above_cnt = second ? c + c0 : c;
+    f.above_mass = second ? m + m0 : m;
+  }
+  __syncthreads();
+  const int g = f.sel;
+  if (g < 0) {
+    // nothing crossed: the lowest key (NaN, mass 0), as the bitwise descent ends in bin 0
+    if (tid == 0) {
+      f.present = key_count(f, 0);
+      f.sel_key = 0;
+      f.above_cnt = tot_c - f.present;
+      f.above_mass = tot_m;
+    }
+  } else if (tid < 32) {
+    const uint32_t key = static_cast<uint32_t>(g) * 32u + 31u - lane;   // from the top
+    const unsigned long long kc = key_count(f, key);
+    const unsigned long long km = kc ? kc * key16_mass_of<T>(key, inv_temp, y_max) : 0ull;
+    const unsigned long long ic = warp_incl_u64(kc), im = warp_incl_u64(km);
+    const unsigned long long above_c = f.above_cnt, above_m = f.above_mass;
+    const bool crosses = by_mass ? above_m + im > limit : above_c + ic > limit;
+    const int first = __ffs(static_cast<int>(__ballot_sync(0xffffffffu, crosses))) - 1;
+    if (lane == first) {
+      f.sel_key = key;
+      f.above_cnt = above_c + ic - kc;
+      f.above_mass = above_m + im - km;
+      f.present = kc;
+    }
+  }
+  __syncthreads();
+}
+
+// Kept mass and ties of the elements [begin, end) of the row, summed by one warp (any order).
+template <typename T>
+__device__ __forceinline__ void sum_range(const T* rp, bool vec_ok, int begin, int end, uint32_t tau, const FastSmem& f,
+                                          unsigned long long& mass, unsigned long long& ties) {
+  const int lane = threadIdx.x & 31;
+  const unsigned short* hp = reinterpret_cast<const unsigned short*>(rp);
+  unsigned long long m = 0;
+  unsigned int n_ties = 0, n_one = 0;
+  auto take = [&](uint32_t key) {
+    if (key > tau) {
+      const unsigned int t = f.words[f.slot[key >> 5] * 32u + (key & 31u)];
+      m += t;
+      n_one += t == 0xFFFFFFFFu ? 1u : 0u;
+    } else if (key == tau) {
+      ++n_ties;
+    }
+  };
+  int i = begin;
+  if (vec_ok) {                               // begin is a multiple of 8
+    const uint4* vp = reinterpret_cast<const uint4*>(hp + begin);
+    const int nvec = (end - begin) / 8;
+    constexpr int kU = 4;
+    for (int j = lane; j < nvec; j += 32 * kU) {
+      uint4 raw[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) raw[u] = j + 32 * u < nvec ? __ldg(vp + j + 32 * u) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        if (j + 32 * u >= nvec) break;
+        const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t k2 = key16x2<T>(w[e]);
+          take(k2 & 0xFFFFu);
+          take(k2 >> 16);
+        }
+      }
+    }
+    i = begin + nvec * 8;
+  }
+  for (i += lane; i < end; i += 32) take(key16x2<T>(hp[i]) & 0xFFFFu);
+  mass = warp_sum_u64(m + n_one);
+  ties = warp_sum_u64(static_cast<unsigned long long>(n_ties));
+}
+
+// One row of 16-bit logits. Returns false (for the whole block) if the row needs the older search.
+template <typename T>
+__device__ bool sample_row16(const T* rp, int v, bool vec_ok, float inv_temp, int top_k, float top_p, uint32_t u24,
+                             GeneralSmem& s, FastSmem& f, int* out) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned short* hp = reinterpret_cast<const unsigned short*>(rp);
+  // ---- count
+  for (int i = tid; i < kHistWords / 4; i += kThreads) reinterpret_cast<uint4*>(f.words)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (tid == 0) {
+    f.total = 0;
+    f.max_key = 0;
+  }
+  __syncthreads();
+  auto add = [&](uint32_t key) { atomicAdd(&f.words[key >> 1], 1u << ((key & 1u) * 16u)); };
+  const int nvec = vec_ok ? v / 8 : 0;
+  {
+    const uint4* vp = reinterpret_cast<const uint4*>(hp);
+    constexpr int kU = 4;
+    for (int j = tid; j < nvec; j += kThreads * kU) {
+      uint4 raw[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        raw[u] = j + kThreads * u < nvec ? __ldg(vp + j + kThreads * u) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        if (j + kThreads * u >= nvec) break;
+        const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t k2 = key16x2<T>(w[e]);
+          add(k2 & 0xFFFFu);
+          add(k2 >> 16);
+        }
+      }
+    }
+    for (int i = nvec * 8 + tid; i < v; i += kThreads) add(key16x2<T>(hp[i]) & 0xFFFFu);
+  }
+  __syncthreads();
+  // ---- counts per group (group g belongs to warp g % 32), their sum, the largest key
+  {
+    unsigned int sum = 0, top = 0;
+    for (int g = warp; g < kGroups; g += kWarps) {
+      const unsigned int c = key_count(f, static_cast<uint32_t>(g * 32 + lane));
+      const unsigned int any = __ballot_sync(0xffffffffu, c != 0);
+      const unsigned int n = any ? __reduce_add_sync(0xffffffffu, c) : 0u;
+      if (lane == 0) s.cnt[g] = n;
+      sum += n;
+      if (any) top = static_cast<unsigned int>(g * 32 + 31 - __clz(static_cast<int>(any)));
+    }
+    if (lane == 0) {
+      atomicAdd(&f.total, sum);
+      atomicMax(&f.max_key, top);
+    }
+  }
+  __syncthreads();
+  if (f.total != static_cast<unsigned int>(v)) return false;   // a counter overflowed
+  const float y_max = mul_rn(key16_float<T>(f.max_key), inv_temp);
+  for (int g = warp; g < kGroups; g += kWarps) {
+    unsigned long long m = 0;
+    if (s.cnt[g]) {
+      const uint32_t key = static_cast<uint32_t>(g * 32 + lane);
+      const unsigned int c = key_count(f, key);
+      m = warp_sum_u64(c ? c * key16_mass_of<T>(key, inv_temp, y_max) : 0ull);
+    }
+    if (lane == 0) s.mass[g] = m;
+  }
+  __syncthreads();
+
+  // ---- where the kept prefix ends: the same decisions as in sample_general_kernel
+  uint32_t tau = 0;
+  unsigned long long tie_keep = ~0ull, kept_mass = 0;
+  {
+    uint32_t k_tau = 0;
+    unsigned long long k_ties = ~0ull;
+    const bool has_k = top_k > 0 && top_k < v;
+    if (has_k) {
+      search_groups<T>(false, static_cast<unsigned long long>(top_k - 1), inv_temp, y_max, s, f);
+      k_tau = f.sel_key;
+      k_ties = static_cast<unsigned long long>(top_k) - f.above_cnt;
+      kept_mass = f.above_mass + k_ties * key16_mass_of<T>(k_tau, inv_temp, y_max);
+    } else {
+      unsigned long long total;
+      block_exscan_u64(s.mass[2 * tid] + s.mass[2 * tid + 1], s.scan, total);
+      kept_mass = total;
+    }
+    tau = k_tau;
+    tie_keep = k_ties;
+    if (top_p < 1.0f) {
+      const unsigned long long limit = mass_fraction(static_cast<double>(top_p), kept_mass);
+      __syncthreads();
+      search_groups<T>(true, limit, inv_temp, y_max, s, f);
+      const uint32_t p_tau = f.sel_key;
+      const unsigned long long above = f.above_mass, q = key16_mass_of<T>(p_tau, inv_temp, y_max);
+      const unsigned long long p_ties = above > limit ? 0ull : (q == 0 ? ~0ull : (limit - above) / q + 1);
+      if (!has_k || (p_tau != k_tau ? p_tau > k_tau : p_ties < k_ties)) {
+        tau = p_tau;
+        tie_keep = p_ties < f.present ? p_ties : f.present;
+        kept_mass = above + tie_keep * q;
+      }
+    }
+  }
+  if (kept_mass == 0) return false;           // nothing has a mass: the older path picks by position
+
+  // ---- table of masses of the kept keys, over the counters
+  const int g_lo = static_cast<int>(tau >> 5);
+  unsigned long long n_slots;
+  {
+    const int g = 2 * tid;
+    const unsigned int a = g >= g_lo && s.cnt[g] ? 1u : 0u, b = g + 1 >= g_lo && s.cnt[g + 1] ? 1u : 0u;
+    const unsigned long long first = block_exscan_u64(a + b, s.scan, n_slots);
+    f.slot[g] = static_cast<unsigned short>(first);
+    f.slot[g + 1] = static_cast<unsigned short>(first + a);
+  }
+  if (n_slots > kTableGroups) return false;
+  unsigned long long present = 0;             // bit i: this lane's key of the warp's i-th group occurs
+  for (int g = warp, i = 0; g < kGroups; g += kWarps, ++i)
+    if (g >= g_lo && s.cnt[g])
+      present |= static_cast<unsigned long long>(key_count(f, static_cast<uint32_t>(g * 32 + lane)) != 0) << i;
+  __syncthreads();                            // every counter has been read
+  for (int g = warp, i = 0; g < kGroups; g += kWarps, ++i) {
+    if (g < g_lo || !s.cnt[g]) continue;
+    unsigned long long q = 0;
+    if ((present >> i) & 1ull) q = key16_mass_of<T>(static_cast<uint32_t>(g * 32 + lane), inv_temp, y_max);
+    f.words[f.slot[g] * 32 + lane] = static_cast<unsigned int>(q >> 32 ? 0xFFFFFFFFull : q);
+  }
+  __syncthreads();
+
+  // ---- draw: find the first element, in token-id order, whose cumulative kept mass exceeds target
+  const unsigned long long q_tau = key16_mass_of<T>(tau, inv_temp, y_max);
+  int begin = 0, end = v;
+  if (tid == 0) {
+    f.target = mass_scale_u24(u24, kept_mass);
+    f.ties_before = 0;
+  }
+#pragma unroll 1
+  for (int level = 0; level < 2; ++level) {
+    const int len = ((end - begin + kWarps - 1) / kWarps + 7) / 8 * 8;
+    const int b = min(end, begin + warp * len), e = min(end, b + len);
+    unsigned long long mass, ties;
+    sum_range<T>(rp, vec_ok, b, e, tau, f, mass, ties);
+    if (lane == 0) {
+      f.seg_mass[warp] = mass;
+      f.seg_ties[warp] = ties;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const unsigned long long t = f.seg_ties[lane], target = f.target;
+      const unsigned long long t0 = f.ties_before + warp_incl_u64(t) - t;
+      const unsigned long long left = tie_keep > t0 ? tie_keep - t0 : 0ull;
+      const unsigned long long m = f.seg_mass[lane] + (t < left ? t : left) * q_tau;
+      const unsigned long long inc = warp_incl_u64(m);
+      const int first = __ffs(static_cast<int>(__ballot_sync(0xffffffffu, inc > target))) - 1;
+      if (lane == first) {
+        f.sel = first;
+        f.target = target - (inc - m);
+        f.ties_before = t0;
+      }
+    }
+    __syncthreads();
+    begin = min(end, begin + f.sel * len);
+    end = min(end, begin + len);
+  }
+  if (warp == 0) {
+    const unsigned long long target = f.target;
+    unsigned long long acc = 0, t0 = f.ties_before;
+    for (int i0 = begin; i0 < end; i0 += 32) {
+      const int i = i0 + lane;
+      const uint32_t key = i < end ? key16x2<T>(hp[i]) & 0xFFFFu : 0u;
+      const bool tie = i < end && key == tau;
+      const unsigned int tie_mask = __ballot_sync(0xffffffffu, tie);
+      const unsigned long long rank = t0 + __popc(tie_mask & ((1u << lane) - 1u));
+      unsigned long long q = 0;
+      if (i < end && key > tau) {
+        const unsigned int t = f.words[f.slot[key >> 5] * 32u + (key & 31u)];
+        q = static_cast<unsigned long long>(t) + (t == 0xFFFFFFFFu ? 1ull : 0ull);
+      } else if (tie && rank < tie_keep) {
+        q = q_tau;
+      }
+      const unsigned long long inc = acc + warp_incl_u64(q);
+      const unsigned int hit = __ballot_sync(0xffffffffu, inc > target);
+      if (hit) {
+        if (lane == __ffs(static_cast<int>(hit)) - 1) *out = i;
+        break;
+      }
+      acc = __shfl_sync(0xffffffffu, inc, 31);
+      t0 += __popc(tie_mask);
+    }
+  }
+  return true;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1)
 sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v, const long long* __restrict__ row_ids,
@@ -798,6 +1145,13 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
   const int row = blockIdx.x;
   const T* rp = logits + static_cast<long long>(row) * row_stride;
   const bool vec_ok = (reinterpret_cast<uintptr_t>(rp) & 15u) == 0;
+  if constexpr (Elem<T>::kPacked) {
+    FastSmem& f = *reinterpret_cast<FastSmem*>(smem_raw + kGeneralSmemBytes);
+    const unsigned long long rid = row_ids ? static_cast<unsigned long long>(row_ids[row])
+                                           : static_cast<unsigned long long>(row);
+    if (sample_row16<T>(rp, v, vec_ok, inv_temp, top_k, top_p, uniform_u24(seed, rid, step), s, f, out + row)) return;
+    __syncthreads();
+  }
 
   // ---- row maximum
   uint32_t tmax = 0;
@@ -1056,7 +1410,8 @@ int launch_sampling(const void* logits, long long row_stride, int rows, int v, c
     sample_topk_kernel<T><<<rows, kTopkThreads, sizeof(TopkSmem), stream>>>(lp, row_stride, v, row_ids, inv_temp, top_k,
                                                                          top_p, seed, step, out);
   } else {
-    constexpr int smem = kGeneralSmemBytes + (std::is_same<T, __nv_bfloat16>::value ? kHistBytes : 0);
+    constexpr int smem = kGeneralSmemBytes + (Elem<T>::kPacked ? static_cast<int>(sizeof(FastSmem)) : 0);
+    static_assert(sizeof(FastSmem) >= kHistBytes, "the older search keeps its histogram there");
     static bool configured = false;
     if (!configured) {
       e = cudaFuncSetAttribute(sample_general_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

@@ -107,3 +107,25 @@ def test_sampler_bf16_without_top_k_threshold_among_negative_values_and_nan(cuda
                                    (100000, None, 1.0), (None, None, 1.0)):
             tok = sample(logits, top_k=top_k, top_p=top_p, temperature=temp, seed=21, step=4)
             assert torch.equal(tok.cpu(), _cpu(logits, top_k, top_p, temp, 21, 4)), (name, top_k, top_p, temp)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("vocab", [7, 1000, 50257, 140001])
+def test_sampler_16_bit_rows_without_top_k(cuda_device, dtype, vocab):
+    """One histogram of counts per key serves the search and the draw. Odd vocabularies (rows that
+    are not 16-byte aligned), one value in more than 65535 places (a counter overflows), values in
+    every corner of the format (more groups than the table holds), and nothing but -inf."""
+    g = torch.Generator(device=cuda_device).manual_seed(vocab)
+    logits = torch.randn(6, vocab, device=cuda_device, generator=g) * 2
+    logits[1] = 1.5
+    logits[2] = -logits[2].abs()
+    logits[3, : vocab // 2] = 0.25
+    logits = logits.to(dtype)
+    bits = torch.randint(-2 ** 15, 2 ** 15, (vocab,), device=cuda_device, generator=g).to(torch.int16)
+    wild = bits.view(dtype)
+    logits[4] = torch.where(torch.isinf(wild), torch.zeros_like(wild), wild)
+    logits[5] = float("-inf")
+    for top_k, top_p, temp in ((None, 0.9, 0.7), (None, None, 1.0), (None, 0.05, 1.0), (3000, 0.95, 0.7)):
+        for step in (0, 1):
+            tok = sample(logits, top_k=top_k, top_p=top_p, temperature=temp, seed=5, step=step)
+            assert torch.equal(tok.cpu(), _cpu(logits, top_k, top_p, temp, 5, step)), (top_k, top_p, temp)
