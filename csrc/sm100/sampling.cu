@@ -15,8 +15,8 @@
 //
 // Three kernels:
 //   sample_topk_kernel     top_k in [1, 1024] (greedy = top_k 1), optional top_p
-//   sample_topk_cluster_kernel  the same for 16-bit logits and few rows: a cluster of 2 or 4
-//                          CTAs per row, candidates exchanged through distributed shared memory
+//   sample_topk_held_kernel  the same for aligned 16-bit rows that 1, 2 or 4 CTAs hold in registers
+//                          (a cluster; candidates exchanged through distributed shared memory)
 //   sample_general_kernel  no top_k (or k > 1024), optional top_p: threshold search by radix
 //                          descent on (count, mass) histograms; for bf16 rows in one step on a
 //                          histogram of counts per key (the mass of a key is a function of the key)
@@ -448,10 +448,11 @@ sample_topk_kernel(const T* __restrict__ logits, long long row_stride, int v, co
 }
 
 // ------------------------------------------------------------------------------------------
-// Cluster variant of the top-k kernel for 16-bit logits and few rows: C CTAs of a thread-block
-// cluster share one row, so that C SMs pull it instead of one (a single CTA is bound by the
-// latency of its own loads; with 64 rows only 64 of the 148 SMs would work at all).
-//   1. CTA r scans its 1/C of the row and finds, as above, a bound that at least kk of its own
+// Top-k kernel for aligned rows of 16-bit logits that fit the registers of a few SMs: a cluster of
+// C CTAs (1, 2 or 4) shares a row, every thread requests its whole part (eight 16-byte vectors) at
+// once and keeps it, so the row is read once and the collection costs no second pass. One CTA
+// with eight loads per thread and step needed five round trips to memory and the same again to L2.
+//   1. CTA r keeps its 1/C of the row and finds, as above, a bound that at least kk of its own
 //      elements reach. The largest of the C bounds is valid for the whole row: the part that
 //      produced it alone holds kk elements at or above it.
 //   2. The bounds travel through distributed shared memory (one store per peer, one cluster
@@ -460,12 +461,14 @@ sample_topk_kernel(const T* __restrict__ logits, long long row_stride, int v, co
 //      its offset (remote shared-memory stores), and CTA 0 finishes as the one-CTA kernel does.
 // The survivors are the kk largest by (key desc, id asc) of a candidate set that contains them
 // all, so the token is the one the one-CTA kernel and the CPU library return. No multicast.
+// Measured (bf16 [64, 128256], k = 50, top_p = 0.9): 16.6 us, one CTA per row 22.5 us.
 // ------------------------------------------------------------------------------------------
 constexpr int kMaxCluster = 4;
 
 struct ClusterXchg {
   uint32_t low[kMaxCluster];   // bound found by each CTA of the cluster
   int cnt[kMaxCluster];        // candidates collected by each CTA
+  int hits[8][3];              // bound search: counts of a step's three thresholds
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -485,63 +488,77 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
+constexpr int kHeldThreads = 1024;
+constexpr int kHeldVecs = 8;                                          // 16-byte vectors a thread keeps
+constexpr int kHeldElems = kHeldThreads * kHeldVecs * 8;              // 16-bit elements a CTA keeps
+
 template <typename T, int C>
-__global__ void __launch_bounds__(kTopkThreads, 2)
-sample_topk_cluster_kernel(const T* __restrict__ logits, long long row_stride, int v,
-                           const long long* __restrict__ row_ids, float inv_temp, int top_k, float top_p,
-                           unsigned long long seed, unsigned long long step, int* __restrict__ out) {
-  static_assert(Elem<T>::kPacked, "the cluster kernel takes 16-bit logits");
+__global__ void __launch_bounds__(kHeldThreads, 1)
+sample_topk_held_kernel(const T* __restrict__ logits, long long row_stride, int v,
+                        const long long* __restrict__ row_ids, float inv_temp, int top_k, float top_p,
+                        unsigned long long seed, unsigned long long step, int* __restrict__ out) {
+  static_assert(Elem<T>::kPacked, "the kernel takes 16-bit logits");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TopkSmem& s = *reinterpret_cast<TopkSmem*>(smem_raw);
   ClusterXchg& x = *reinterpret_cast<ClusterXchg*>(smem_raw + sizeof(TopkSmem));
-  const int tid = threadIdx.x;
-  const int nt = blockDim.x;
+  const int tid = threadIdx.x, lane = tid & 31;
   const int row = blockIdx.x / C;
-  const int cr = static_cast<int>(cluster_rank());
+  const int cr = C == 1 ? 0 : static_cast<int>(cluster_rank());
   const T* rp = logits + static_cast<long long>(row) * row_stride;  // 16-byte aligned (checked by the host)
   const int kk = min(min(top_k, kMaxTopK), v);
-  if (tid == 0) s.count = 0;
+  if constexpr (C > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");   // waited for before the first remote store
 
   // ---- this CTA's part: vectors [v0, v1) of the row, the scalar tail goes to the last CTA
   const int nvec = v / 8;
   const int v0 = static_cast<int>(static_cast<long long>(nvec) * cr / C);
   const int v1 = static_cast<int>(static_cast<long long>(nvec) * (cr + 1) / C);
-  const uint4* vp = reinterpret_cast<const uint4*>(rp);
   const unsigned short* hp = reinterpret_cast<const unsigned short*>(rp);
-  const bool has_tail = cr == C - 1;
-  constexpr int kU = 8;
-  uint32_t tm2 = 0;
-  int i = v0 + tid;
-  for (; i + (kU - 1) * nt < v1; i += kU * nt) {
-    uint4 raw[kU];
+  const int tail = nvec * 8 + tid;                                    // at most seven elements
+  const bool has_tail = cr == C - 1 && tail < v;
+  const uint4* mine_p = reinterpret_cast<const uint4*>(rp) + v0 + tid;   // this thread's vectors, kHeldThreads apart
+  const int left = v1 - v0 - tid;
+  uint4 raw[kHeldVecs];
 #pragma unroll
-    for (int u = 0; u < kU; ++u) raw[u] = __ldg(vp + i + u * nt);
+  for (int u = 0; u < kHeldVecs; ++u)
+    raw[u] = u * kHeldThreads < left ? __ldg(mine_p + u * kHeldThreads) : make_uint4(~0u, ~0u, ~0u, ~0u);   // NaN: key 0
+  const uint32_t tail_bits = has_tail ? hp[tail] : 0xFFFFu;
+  if (tid == 0) s.count = 0;
+  if (tid < 24) x.hits[tid / 3][tid % 3] = 0;
+  __syncthreads();
+  uint32_t tm2 = key16x2<T>(tail_bits | 0xFFFF0000u);
 #pragma unroll
-    for (int u = 0; u < kU; ++u)
-      tm2 = __vmaxu2(tm2, __vmaxu2(__vmaxu2(key16x2<T>(raw[u].x), key16x2<T>(raw[u].y)),
-                                   __vmaxu2(key16x2<T>(raw[u].z), key16x2<T>(raw[u].w))));
-  }
-  for (; i < v1; i += nt) {
-    const uint4 raw = __ldg(vp + i);
-    tm2 = __vmaxu2(tm2, __vmaxu2(__vmaxu2(key16x2<T>(raw.x), key16x2<T>(raw.y)),
-                                 __vmaxu2(key16x2<T>(raw.z), key16x2<T>(raw.w))));
-  }
-  if (has_tail)
-    for (int t = nvec * 8 + tid; t < v; t += nt) tm2 = __vmaxu2(tm2, key16x2<T>(hp[t]) & 0xFFFFu);
+  for (int u = 0; u < kHeldVecs; ++u)
+    tm2 = __vmaxu2(tm2, __vmaxu2(__vmaxu2(key16x2<T>(raw[u].x), key16x2<T>(raw[u].y)),
+                                 __vmaxu2(key16x2<T>(raw[u].z), key16x2<T>(raw[u].w))));
+  // ---- the kk-th largest of the 2048 maxima, two bits of it per step: counts for the three
+  // thresholds, packed per warp (at most 64 each), one barrier
   const uint32_t m_lo = tm2 & 0xFFFFu, m_hi = tm2 >> 16;
   uint32_t low16 = 0;
-  for (int bit = 15; bit >= 0; --bit) {
-    const uint32_t cand = low16 | (1u << bit);
-    const int cnt = __syncthreads_count(m_lo >= cand) + __syncthreads_count(m_hi >= cand);
-    if (cnt >= kk) low16 = cand;
-  }
-  // ---- the largest of the C bounds serves the whole row
-  if (tid < C) st_remote_u32(map_to_cta(&x.low[cr], static_cast<uint32_t>(tid)), low16);
-  cluster_sync_all();
+#pragma unroll 1
+  for (int st = 0; st < 8; ++st) {
+    const int shift = 14 - 2 * st;
+    uint32_t packed = 0;
 #pragma unroll
-  for (int r = 0; r < C; ++r) low16 = max(low16, x.low[r]);
+    for (uint32_t t = 1; t <= 3; ++t) {
+      const uint32_t cand = low16 | (t << shift);
+      packed += ((m_lo >= cand ? 1u : 0u) + (m_hi >= cand ? 1u : 0u)) << (10 * (t - 1));
+    }
+    packed = __reduce_add_sync(0xffffffffu, packed);
+    if (lane < 3) atomicAdd(&x.hits[st][lane], static_cast<int>((packed >> (10 * lane)) & 1023u));
+    __syncthreads();
+    const int c1 = x.hits[st][0], c2 = x.hits[st][1], c3 = x.hits[st][2];
+    low16 |= static_cast<uint32_t>(c3 >= kk ? 3 : (c2 >= kk ? 2 : (c1 >= kk ? 1 : 0))) << shift;
+  }
+  if constexpr (C > 1) {
+    // ---- the largest of the C bounds serves the whole row
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");      // every CTA of the cluster runs
+    if (tid < C) st_remote_u32(map_to_cta(&x.low[cr], static_cast<uint32_t>(tid)), low16);
+    cluster_sync_all();
+#pragma unroll
+    for (int r = 0; r < C; ++r) low16 = max(low16, x.low[r]);
+  }
 
-  // ---- collect this part's elements at or above the bound (second pass: L2)
+  // ---- collect this part's elements at or above the bound
   const uint32_t low2 = low16 * 0x00010001u;
   auto push = [&](uint32_t bits16, int idx) {
     const int slot = atomicAdd(&s.count, 1);
@@ -550,50 +567,50 @@ sample_topk_cluster_kernel(const T* __restrict__ logits, long long row_stride, i
       s.cand_idx[slot] = static_cast<uint32_t>(idx);
     }
   };
-  auto scan_vec = [&](const uint4& raw, int vi) {
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-    const uint32_t h0 = __vcmpgeu2(key16x2<T>(w[0]), low2), h1 = __vcmpgeu2(key16x2<T>(w[1]), low2);
-    const uint32_t h2 = __vcmpgeu2(key16x2<T>(w[2]), low2), h3 = __vcmpgeu2(key16x2<T>(w[3]), low2);
-    if ((h0 | h1 | h2 | h3) == 0u) return;
-    const uint32_t hit[4] = {h0, h1, h2, h3};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (hit[j] & 0xFFFFu) push(w[j] & 0xFFFFu, vi * 8 + 2 * j);
-      if (hit[j] >> 16) push(w[j] >> 16, vi * 8 + 2 * j + 1);
+  for (int u = 0; u < kHeldVecs; ++u) {
+    if (u * kHeldThreads >= left) break;
+    // one bit per element (bit 4 * half + word), few of which are ever set
+    uint32_t hits = (__vcmpgeu2(key16x2<T>(raw[u].x), low2) & 0x00100001u) |
+                    (__vcmpgeu2(key16x2<T>(raw[u].y), low2) & 0x00200002u) |
+                    (__vcmpgeu2(key16x2<T>(raw[u].z), low2) & 0x00400004u) |
+                    (__vcmpgeu2(key16x2<T>(raw[u].w), low2) & 0x00800008u);
+    hits = (hits | (hits >> 16)) & 0xFFu;
+    while (hits) {
+      const int bit = __ffs(static_cast<int>(hits)) - 1;
+      hits &= hits - 1;
+      const int w = bit & 3, half = bit >> 2;
+      const uint32_t word = w == 0 ? raw[u].x : (w == 1 ? raw[u].y : (w == 2 ? raw[u].z : raw[u].w));
+      push((word >> (16 * half)) & 0xFFFFu, (v0 + tid + u * kHeldThreads) * 8 + 2 * w + half);
     }
-  };
-  i = v0 + tid;
-  for (; i + (kU - 1) * nt < v1; i += kU * nt) {
-    uint4 raw[kU];
-#pragma unroll
-    for (int u = 0; u < kU; ++u) raw[u] = __ldg(vp + i + u * nt);
-#pragma unroll
-    for (int u = 0; u < kU; ++u) scan_vec(raw[u], i + u * nt);
   }
-  for (; i < v1; i += nt) scan_vec(__ldg(vp + i), i);
-  if (has_tail)
-    for (int t = nvec * 8 + tid; t < v; t += nt)
-      if ((key16x2<T>(hp[t]) & 0xFFFFu) >= low16) push(hp[t], t);
+  if (has_tail && (key16x2<T>(tail_bits) & 0xFFFFu) >= low16) push(tail_bits, tail);
   __syncthreads();
-  const int mine = s.count;  // may exceed the buffer: then the total does too and CTA 0 searches the row exactly
-  if (tid < C) st_remote_u32(map_to_cta(&x.cnt[cr], static_cast<uint32_t>(tid)), static_cast<uint32_t>(mine));
-  cluster_sync_all();
-  int total = 0, offset = 0;
+  int total = s.count;  // may exceed the buffer: then CTA 0 searches the row exactly
+  if constexpr (C > 1) {
+    const int mine = total;
+    if (tid < C) st_remote_u32(map_to_cta(&x.cnt[cr], static_cast<uint32_t>(tid)), static_cast<uint32_t>(mine));
+    cluster_sync_all();
+    int offset = 0;
+    total = 0;
 #pragma unroll
-  for (int r = 0; r < C; ++r) {
-    if (r < cr) offset += x.cnt[r];
-    total += x.cnt[r];
-  }
-  // ---- candidates of the other CTAs move into CTA 0's list
-  if (cr != 0 && total <= kCandCap) {
-    const uint32_t dst_key = map_to_cta(&s.cand_key[0], 0u), dst_idx = map_to_cta(&s.cand_idx[0], 0u);
-    for (int j = tid; j < mine; j += nt) {
-      st_remote_u32(dst_key + 4u * static_cast<uint32_t>(offset + j), s.cand_key[j]);
-      st_remote_u32(dst_idx + 4u * static_cast<uint32_t>(offset + j), s.cand_idx[j]);
+    for (int r = 0; r < C; ++r) {
+      if (r < cr) offset += x.cnt[r];
+      total += x.cnt[r];
     }
+    // ---- candidates of the other CTAs move into CTA 0's list
+    if (cr != 0 && total <= kCandCap) {
+      const uint32_t dst_key = map_to_cta(&s.cand_key[0], 0u), dst_idx = map_to_cta(&s.cand_idx[0], 0u);
+      for (int j = tid; j < mine; j += kHeldThreads) {
+        st_remote_u32(dst_key + 4u * static_cast<uint32_t>(offset + j), s.cand_key[j]);
+        st_remote_u32(dst_idx + 4u * static_cast<uint32_t>(offset + j), s.cand_idx[j]);
+      }
+    }
+    cluster_sync_all();  // after this barrier nobody touches another CTA's shared memory
+    if (cr != 0) return;
+  } else {
+    __syncthreads();
   }
-  cluster_sync_all();  // after this barrier nobody touches another CTA's shared memory
-  if (cr != 0) return;
   topk_finish<T>(s, total, rp, v, true, kk, inv_temp, top_p, seed, step, row_ids, row, out);
 }
 
@@ -1361,38 +1378,25 @@ int launch_sampling(const void* logits, long long row_stride, int rows, int v, c
       if (e != cudaSuccess) return -10;
       configured = true;
     }
-    // few rows of 16-bit logits may be given several CTAs per row (a cluster)
-    int cluster = 1;
+    // Aligned rows that 1, 2 or 4 CTAs can keep in registers take the kernel that reads them once;
+    // it was faster at every number of rows (see its comment). KA_SAMPLE_CLUSTER = 1 keeps the
+    // other one, 2 and 4 ask for that many CTAs per row.
     if constexpr (Elem<T>::kPacked) {
-      int dev = 0, sms = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      const bool aligned = (reinterpret_cast<uintptr_t>(lp) & 15u) == 0 && (row_stride * sizeof(T)) % 16 == 0 && v >= 8192;
-      // Measured (bf16 [G, 128256], k = 50, L2 flushed): 28.7 / 28.7 / 30.6 us for 1 / 2 / 4 CTAs
-      // per row at G = 64, 31.6 / 35.7 / 50.0 at G = 128. A row's two passes are a small part of
-      // the kernel's latency chain (bound search, candidate sort, masses, draw), so more SMs per
-      // row buy nothing here; the variant stays available but is not chosen by default.
-      (void)sms;
-      if (const char* e = getenv("KA_SAMPLE_CLUSTER")) {      // 2 / 4: CTAs per row (opt-in)
-        const int c = atoi(e);
-        if (c == 1 || ((c == 2 || c == 4) && aligned)) cluster = c;
+      const bool aligned = (reinterpret_cast<uintptr_t>(lp) & 15u) == 0 && (row_stride * sizeof(T)) % 16 == 0;
+      int cluster = v <= kHeldElems ? 1 : (v <= 2 * kHeldElems ? 2 : (v <= 4 * kHeldElems ? 4 : 0));
+      if (const char* env = getenv("KA_SAMPLE_CLUSTER")) {
+        const int c = atoi(env);
+        if (c == 1) cluster = 0;
+        if ((c == 2 || c == 4) && cluster != 0 && c > cluster) cluster = c;
       }
-    }
-    if (cluster > 1) {
-      if constexpr (Elem<T>::kPacked) {
+      if (cluster > 0 && aligned) {
         const int smem = static_cast<int>(sizeof(TopkSmem) + sizeof(ClusterXchg));
-        auto* k2 = sample_topk_cluster_kernel<T, 2>;
-        auto* k4 = sample_topk_cluster_kernel<T, 4>;
-        static bool cluster_configured = false;
-        if (!cluster_configured) {
-          if (cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-              cudaFuncSetAttribute(k4, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-            return -10;
-          cluster_configured = true;
-        }
+        auto* kernel = cluster == 1 ? sample_topk_held_kernel<T, 1>
+                                    : (cluster == 2 ? sample_topk_held_kernel<T, 2> : sample_topk_held_kernel<T, 4>);
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -10;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(static_cast<unsigned>(rows * cluster));
-        cfg.blockDim = dim3(kTopkThreads);
+        cfg.gridDim = dim3(static_cast<unsigned>(rows) * cluster);
+        cfg.blockDim = dim3(kHeldThreads);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = stream;
         cudaLaunchAttribute attr[1];
@@ -1401,9 +1405,8 @@ int launch_sampling(const void* logits, long long row_stride, int rows, int v, c
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, cluster == 2 ? k2 : k4, lp, row_stride, v, row_ids, inv_temp, top_k, top_p, seed,
-                               step, out);
+        cfg.numAttrs = cluster > 1 ? 1 : 0;
+        e = cudaLaunchKernelEx(&cfg, kernel, lp, row_stride, v, row_ids, inv_temp, top_k, top_p, seed, step, out);
         return e == cudaSuccess ? 0 : -11;
       }
     }
