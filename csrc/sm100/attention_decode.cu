@@ -1,22 +1,26 @@
 // Single-token attention against a KV cache (rollout phase), grouped KV heads, head_dim 128.
 //
 // What bounds it is the read of the cache, so the keys of a sequence are spread over enough
-// CTAs that their loads fill the memory pipe, and every K and V row is loaded once, 16 bytes
-// per lane, for all query heads of its GQA group.
+// CTAs that their loads fill the memory pipe, every K and V row is loaded once, 16 bytes per
+// lane, for all query heads of its GQA group, and the instructions per key are kept few.
 //
-//   * Keys are cut into blocks of 8 * KPB. Block i belongs to stripe i % 8, and inside a block
-//     half-warp w of the CTA's eight takes keys [w * KPB, (w + 1) * KPB). A half-warp covers a
-//     row with 16 lanes x 8 dimensions and keeps its own running (max, sum, acc): the loop over
-//     blocks has no CTA-wide barrier, and the loads of the next block are in flight while the
-//     current one is computed.
-//   * The eight half-warp states of a stripe are merged in half-warp order, the eight stripes in
-//     stripe order. This decomposition depends on the number of keys alone, so a row's bits do
-//     not depend on its batch. How many CTAs work on a (sequence, KV head) does: a cluster of
-//     S = 1, 2, 4 or 8 CTAs takes 8 / S stripes each, the smallest S that gives about four CTAs
-//     per SM, and the merge reads the other CTAs' stripes through distributed shared memory.
-//   * Scores: fp32, summed over the 16 lanes by exchanging halves of the vector of (head, key)
-//     partial sums, so 32 sums cost 30 shuffles instead of 128 and each lane ends up with the
-//     scores whose exponentials it takes. Probabilities and accumulators stay in fp32.
+//   * Keys are cut into blocks of 64. Block i belongs to stripe i % 8, and inside a block warp w
+//     of the CTA's four takes keys [16 w, 16 w + 16). A warp keeps its own running (max, sum, acc)
+//     of a stripe: the loop over blocks has no CTA-wide barrier, and the loads of the next block
+//     are in flight while the current one is computed.
+//   * Scores: mma.sync m16n8k16 with the 16 keys as rows and the heads of the group as columns
+//     (products of bf16 are exact, sums in fp32). The K rows are loaded 16 bytes per lane straight
+//     into A fragments: the head dimension is permuted, the same way for K and q, which a dot
+//     product does not notice. With the scores on the fp32 pipe (32 sums over 16 lanes per half-warp)
+//     the instructions took as long as the bytes: 70 us where this takes 59 us (64 x 875 keys,
+//     32 / 8 heads; one CTA per sequence and KV head without any of this took 109 us). P V stays on the fp32 pipe: probabilities and
+//     accumulators are fp32.
+//   * The states of stripes 0-3 and of stripes 4-7 are folded in stripe order, per warp, and the
+//     eight folded states (2 halves x 4 warps) are merged in order. This decomposition depends on
+//     the number of keys alone, so a row's bits do not depend on its batch. How many CTAs work on
+//     a (sequence, KV head) does: a cluster of S = 2, 4 or 8 takes 8 / S stripes each, the
+//     smallest S that gives about four CTAs per SM. With S = 2 a CTA folds its own stripes; the
+//     rest is read from the other CTAs through distributed shared memory.
 //
 // The reference has no decode attention (its executor comments defer generation to a future
 // vLLM integration, rl_engine/executors/rollout.py:33).
@@ -81,25 +85,22 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
 }
 
 constexpr int kStripes = 8;
+constexpr int kWarps = kDecThreads / 32;
+constexpr int kWarpKeys = 16;                          // keys of a warp in a block: the rows of the MMA
+constexpr int kBlockKeys = kWarps * kWarpKeys;
 
+// A warp's state of a stripe (or of a fold of four): per head (max, sum) and the accumulator.
 template <int GQ>
-struct Split {
-  static constexpr int kKpb = GQ == 1 ? 16 : (GQ == 8 ? 4 : 8);   // keys per half-warp and block
-  static constexpr int kScores = GQ * kKpb;                       // per half-warp and block: 16 or 32
-  static constexpr int kOwn = kScores / 16;                       // scores a lane ends up with
-  static constexpr int kLanesPerHead = 16 / GQ;
-  static constexpr int kBlockKeys = 8 * kKpb;
+struct State {
+  float ml[kWarps][GQ][2];
+  float acc[kWarps][GQ][kD];
 };
 
-// Shared memory: half-warp exchange of probabilities and states, then one state per stripe.
 template <int GQ>
 struct SplitSmem {
-  float p[8][Split<GQ>::kKpb][GQ];
-  float alpha[8][GQ];
-  float hw_ml[8][GQ][2];
-  float hw_acc[8][GQ][kD];
-  float st_ml[kStripes][GQ][2];      // only the first 8 / S stripes are used
-  // followed by float st_acc[8 / S][GQ][kD]
+  float p[kWarps][kWarpKeys][GQ];
+  float alpha[kWarps][GQ];
+  // followed by State<GQ>[states per CTA]: one per stripe, or one folded state when splits == 2
 };
 
 __device__ __forceinline__ void unpack8(const uint4& r, float (&f)[8]) {
@@ -119,6 +120,15 @@ __device__ __forceinline__ void fma2(float& d0, float& d1, float a0, float a1, f
       : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
 }
 
+// D[16 keys, 8 heads] += A[16, 16] * B[16, 8], bf16 in, fp32 out.
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                          uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
@@ -131,213 +141,286 @@ __device__ __forceinline__ float state_weight(float m, float M, float c) {
   return m == -CUDART_INF_F ? 0.f : ex2_approx(__fmul_rn(__fsub_rn(m, M), c));
 }
 
+// Fold of two states, the same operations wherever it happens: weights first, then value by value.
+struct FoldWeights {
+  float m, w_old, w_new;
+};
+__device__ __forceinline__ FoldWeights fold_weights(float m_old, float m_new, float c) {
+  FoldWeights f;
+  f.m = fmaxf(m_old, m_new);
+  f.w_old = state_weight(m_old, f.m, c);
+  f.w_new = state_weight(m_new, f.m, c);
+  return f;
+}
+__device__ __forceinline__ float fold_value(const FoldWeights& f, float v_old, float v_new) {
+  return __fmaf_rn(f.w_new, v_new, __fmul_rn(f.w_old, v_old));
+}
+
 template <int GQ>
 __global__ void __launch_bounds__(kDecThreads, GQ == 8 ? 2 : 3)
 attention_decode_split_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache_k,
                               const __nv_bfloat16* __restrict__ cache_v, const int* __restrict__ lens,
                               __nv_bfloat16* __restrict__ out, int hq, int hkv, int max_len, float scale, int splits) {
-  using T = Split<GQ>;
-  constexpr int KPB = T::kKpb;
   extern __shared__ __align__(16) uint8_t smem_raw[];
   SplitSmem<GQ>& sm = *reinterpret_cast<SplitSmem<GQ>*>(smem_raw);
-  float* st_acc = reinterpret_cast<float*>(smem_raw + sizeof(SplitSmem<GQ>));   // [8 / S][GQ][kD]
+  State<GQ>* states = reinterpret_cast<State<GQ>*>(smem_raw + sizeof(SplitSmem<GQ>));
 
-  const int rank = splits == 1 ? 0 : static_cast<int>(cluster_ctarank());
+  const int rank = static_cast<int>(cluster_ctarank());
   const int bh = blockIdx.x / splits;
   const int b = bh / hkv, hk = bh % hkv;
   const int n = lens[b];
   const int per_cta = kStripes / splits;
-  const int tid = threadIdx.x, hw = tid >> 4, ln = tid & 15;
+  const bool folded = splits == 2;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const float c = scale * kLog2e;
   const size_t kv_row = static_cast<size_t>(hkv) * kD;
-  const __nv_bfloat16* kbase = cache_k + (static_cast<size_t>(b) * max_len * hkv + hk) * kD + ln * 8;
-  const __nv_bfloat16* vbase = cache_v + (static_cast<size_t>(b) * max_len * hkv + hk) * kD + ln * 8;
+  const size_t kv_off = (static_cast<size_t>(b) * max_len * hkv + hk) * kD;
+  // K fragments: lane (g, t) holds keys g and g + 8, dimensions 32 i + 8 t .. + 7 (two K steps of
+  // the MMA per 16-byte load). V: half-warp h holds keys 8 h .. 8 h + 7, lane ln dimensions 8 ln .. + 7.
+  const int g8 = lane >> 2, t4 = lane & 3, half = lane >> 4, ln = lane & 15;
+  const __nv_bfloat16* kbase = cache_k + kv_off + t4 * 8;
+  const __nv_bfloat16* vbase = cache_v + kv_off + ln * 8;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
 
-  float qr[GQ][8];
+  uint4 qf[4];                     // B fragments: head g8 of the group, the same dimensions
 #pragma unroll
-  for (int g = 0; g < GQ; ++g)
+  for (int i = 0; i < 4; ++i) {
+    qf[i] = zero;
+    if (g8 < GQ) {
+      const __nv_bfloat16* qp = q + (static_cast<size_t>(b) * hq + hk * GQ + g8) * kD + i * 32 + t4 * 8;
+      uint32_t* w = reinterpret_cast<uint32_t*>(&qf[i]);
 #pragma unroll
-    for (int e = 0; e < 8; ++e)
-      qr[g][e] = __bfloat162float(q[(static_cast<size_t>(b) * hq + hk * GQ + g) * kD + ln * 8 + e]);
+      for (int e = 0; e < 4; ++e)
+        w[e] = static_cast<uint32_t>(__bfloat16_as_ushort(qp[2 * e])) |
+               (static_cast<uint32_t>(__bfloat16_as_ushort(qp[2 * e + 1])) << 16);
+    }
+  }
 
   // The blocks of this CTA: stripes [rank * per_cta, (rank + 1) * per_cta), each stripe's blocks
-  // in increasing order. (stripe, block) walks that list.
-  const int n_blocks = (n + T::kBlockKeys - 1) / T::kBlockKeys;
-  const int stripe_end = (rank + 1) * per_cta;
-  uint4 kr[KPB], vr[KPB];
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  auto load = [&](const __nv_bfloat16* base, int blk, uint4 (&r)[KPB]) {
-    const int key0 = blk * T::kBlockKeys + hw * KPB;
+  // in increasing order.
+  const int n_blocks = (n + kBlockKeys - 1) / kBlockKeys;
+  const int stripe0 = rank * per_cta, stripe_end = stripe0 + per_cta;
+  uint4 kr[8], vr[8];
+  auto load_k = [&](int blk) {
+    const int key0 = blk * kBlockKeys + warp * kWarpKeys + g8;
 #pragma unroll
-    for (int i = 0; i < KPB; ++i)
-      r[i] = key0 + i < n ? *reinterpret_cast<const uint4*>(base + (key0 + i) * kv_row) : zero;
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        kr[r * 4 + i] = key0 + 8 * r < n
+                            ? *reinterpret_cast<const uint4*>(kbase + (key0 + 8 * r) * kv_row + i * 32)
+                            : zero;
+  };
+  auto load_v = [&](int blk) {
+    const int key0 = blk * kBlockKeys + warp * kWarpKeys + half * 8;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      vr[i] = key0 + i < n ? *reinterpret_cast<const uint4*>(vbase + (key0 + i) * kv_row) : zero;
   };
 
-  int stripe = rank * per_cta;
-  int blk = stripe;
-  if (blk < n_blocks) {
-    load(kbase, blk, kr);
-    load(vbase, blk, vr);
+  if (stripe0 < n_blocks) {
+    load_k(stripe0);
+    load_v(stripe0);
   }
-  for (; stripe < stripe_end; ++stripe) {
+  // this lane's two heads of the score fragment (columns 2 t and 2 t + 1) and whether they exist
+  const int h0 = 2 * t4;
+  const bool has0 = h0 < GQ, has1 = h0 + 1 < GQ;
+  for (int stripe = stripe0; stripe < stripe_end; ++stripe) {
     float acc[GQ][8];
 #pragma unroll
     for (int g = 0; g < GQ; ++g)
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc[g][e] = 0.f;
-    float m_run = -CUDART_INF_F, l_run = 0.f;      // of the head whose scores this lane owns
-    for (blk = stripe; blk < n_blocks; blk += kStripes) {
-      // the block after this one, in this stripe or at the start of the next
-      int nblk = blk + kStripes;
+    float m_run[2] = {-CUDART_INF_F, -CUDART_INF_F}, l_run[2] = {0.f, 0.f};
+    for (int blk = stripe; blk < n_blocks; blk += kStripes) {
+      int nblk = blk + kStripes;                    // the block after this one: of this stripe or the next
       if (nblk >= n_blocks) nblk = stripe + 1 < stripe_end ? stripe + 1 : n_blocks;
-      float s[T::kScores];                          // index = head * KPB + key
+      float s[4] = {0.f, 0.f, 0.f, 0.f};            // (key g8, heads h0, h0 + 1), (key g8 + 8, the same)
 #pragma unroll
-      for (int i = 0; i < KPB; ++i) {
-        float kf[8];
-        unpack8(kr[i], kf);
+      for (int i = 0; i < 4; ++i) {
+        mma_16816(s, kr[i].x, kr[4 + i].x, kr[i].y, kr[4 + i].y, qf[i].x, qf[i].y);
+        mma_16816(s, kr[i].z, kr[4 + i].z, kr[i].w, kr[4 + i].w, qf[i].z, qf[i].w);
+      }
+      if (nblk < n_blocks) load_k(nblk);
+      const int key0 = blk * kBlockKeys + warp * kWarpKeys + g8;
+      if (key0 >= n) s[0] = s[1] = -CUDART_INF_F;
+      if (key0 + 8 >= n) s[2] = s[3] = -CUDART_INF_F;
 #pragma unroll
-        for (int g = 0; g < GQ; ++g) {
-          float a0 = 0.f, a1 = 0.f;
+      for (int h = 0; h < 2; ++h) {
+        float mb = fmaxf(s[h], s[2 + h]);
 #pragma unroll
-          for (int e = 0; e < 8; e += 2) fma2(a0, a1, qr[g][e], qr[g][e + 1], kf[e], kf[e + 1]);
-          s[g * KPB + i] = __fadd_rn(a0, a1);
+        for (int o = 4; o < 32; o <<= 1) mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, o));
+        const float m_new = fmaxf(m_run[h], mb);
+        const float m_ref = m_new == -CUDART_INF_F ? 0.f : m_new;   // nothing but -inf so far: every weight is 0
+        const float al = m_run[h] == -CUDART_INF_F ? 0.f : ex2_approx(__fmul_rn(__fsub_rn(m_run[h], m_ref), c));
+        m_run[h] = m_new;
+        const float p0 = key0 < n ? ex2_approx(__fmul_rn(__fsub_rn(s[h], m_ref), c)) : 0.f;
+        const float p1 = key0 + 8 < n ? ex2_approx(__fmul_rn(__fsub_rn(s[2 + h], m_ref), c)) : 0.f;
+        l_run[h] = __fadd_rn(__fmul_rn(l_run[h], al), __fadd_rn(p0, p1));
+        if (h == 0 ? has0 : has1) {
+          sm.p[warp][g8][h0 + h] = p0;
+          sm.p[warp][g8 + 8][h0 + h] = p1;
+          if (g8 == 0) sm.alpha[warp][h0 + h] = al;
         }
       }
-      if (nblk < n_blocks) load(kbase, nblk, kr);
-      // sum over the 16 lanes: each step halves the vector, lane l keeps the part its bit names
-#pragma unroll
-      for (int step = 0; step < 4; ++step) {
-        const int mask = 8 >> step, half = T::kScores >> (step + 1);
-        const bool upper = (ln & mask) != 0;
-#pragma unroll
-        for (int i = 0; i < half; ++i) {
-          const float keep = upper ? s[half + i] : s[i], give = upper ? s[i] : s[half + i];
-          s[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, mask));
-        }
-      }
-      // lane ln owns scores ln * kOwn .. : head ln / kLanesPerHead
-      const int own_head = ln / T::kLanesPerHead;
-      const int own_key = (ln % T::kLanesPerHead) * T::kOwn;
-      const int key0 = blk * T::kBlockKeys + hw * KPB + own_key;
-      float mb = -CUDART_INF_F;
-#pragma unroll
-      for (int i = 0; i < T::kOwn; ++i) {
-        if (key0 + i >= n) s[i] = -CUDART_INF_F;
-        mb = fmaxf(mb, s[i]);
-      }
-#pragma unroll
-      for (int o = T::kLanesPerHead >> 1; o > 0; o >>= 1) mb = fmaxf(mb, __shfl_xor_sync(0xffffffffu, mb, o));
-      const float m_new = fmaxf(m_run, mb);
-      const float m_ref = m_new == -CUDART_INF_F ? 0.f : m_new;   // nothing but -inf so far: every weight is 0
-      const float al = m_run == -CUDART_INF_F ? 0.f : ex2_approx(__fmul_rn(__fsub_rn(m_run, m_ref), c));
-      m_run = m_new;
-      l_run = __fmul_rn(l_run, al);
-#pragma unroll
-      for (int i = 0; i < T::kOwn; ++i) {
-        const float pr = ex2_approx(__fmul_rn(__fsub_rn(s[i], m_ref), c));
-        l_run = __fadd_rn(l_run, pr);
-        sm.p[hw][own_key + i][own_head] = pr;
-      }
-      if (ln % T::kLanesPerHead == 0) sm.alpha[hw][own_head] = al;
       __syncwarp();
       float ag[GQ];
 #pragma unroll
-      for (int g = 0; g < GQ; ++g) ag[g] = sm.alpha[hw][g];
+      for (int g = 0; g < GQ; ++g) ag[g] = sm.alpha[warp][g];
 #pragma unroll
       for (int g = 0; g < GQ; ++g)
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[g][e] = __fmul_rn(acc[g][e], ag[g]);
 #pragma unroll
-      for (int i = 0; i < KPB; ++i) {
+      for (int i = 0; i < 8; ++i) {
         float vf[8], pg[GQ];
         unpack8(vr[i], vf);
 #pragma unroll
-        for (int g = 0; g < GQ; ++g) pg[g] = sm.p[hw][i][g];
+        for (int g = 0; g < GQ; ++g) pg[g] = sm.p[warp][half * 8 + i][g];
 #pragma unroll
         for (int g = 0; g < GQ; ++g)
 #pragma unroll
           for (int e = 0; e < 8; e += 2) fma2(acc[g][e], acc[g][e + 1], pg[g], pg[g], vf[e], vf[e + 1]);
       }
-      if (nblk < n_blocks) load(vbase, nblk, vr);
+      if (nblk < n_blocks) load_v(nblk);
       __syncwarp();                                 // p and alpha are rewritten by the next block
     }
-    // ---- merge the eight half-warps of this stripe (in order) into its state
+
+    // ---- the warp's state of this stripe: sums over the lanes, then stored or folded
 #pragma unroll
-    for (int o = T::kLanesPerHead >> 1; o > 0; o >>= 1) l_run = __fadd_rn(l_run, __shfl_xor_sync(0xffffffffu, l_run, o));
-    if (ln % T::kLanesPerHead == 0) {
-      sm.hw_ml[hw][ln / T::kLanesPerHead][0] = m_run;
-      sm.hw_ml[hw][ln / T::kLanesPerHead][1] = l_run;
-    }
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-    for (int g = 0; g < GQ; ++g)
+      for (int o = 4; o < 32; o <<= 1) l_run[h] = __fadd_rn(l_run[h], __shfl_xor_sync(0xffffffffu, l_run[h], o));
+    // the two half-warps add their accumulators: half h keeps heads [h * GQ / 2, (h + 1) * GQ / 2)
+    constexpr int kOwn = GQ == 1 ? 1 : GQ / 2;
+    float own[kOwn][8];
 #pragma unroll
-      for (int e = 0; e < 8; e += 4)
-        *reinterpret_cast<float4*>(&sm.hw_acc[hw][g][ln * 8 + e]) =
-            make_float4(acc[g][e], acc[g][e + 1], acc[g][e + 2], acc[g][e + 3]);
-    __syncthreads();
-    const int ls = stripe - rank * per_cta;
+    for (int g = 0; g < kOwn; ++g)
 #pragma unroll
-    for (int g = 0; g < GQ; ++g) {
-      float M = sm.hw_ml[0][g][0];
-#pragma unroll
-      for (int w = 1; w < 8; ++w) M = fmaxf(M, sm.hw_ml[w][g][0]);
-      float a = 0.f, l = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) {
-        const float wt = state_weight(sm.hw_ml[w][g][0], M, c);
-        l = __fmaf_rn(wt, sm.hw_ml[w][g][1], l);
-        a = __fmaf_rn(wt, sm.hw_acc[w][g][tid], a);
+      for (int e = 0; e < 8; ++e) {
+        if constexpr (GQ == 1) {
+          own[0][e] = __fadd_rn(acc[0][e], __shfl_xor_sync(0xffffffffu, acc[0][e], 16));
+        } else {
+          const float give = half ? acc[g][e] : acc[kOwn + g][e], keep = half ? acc[kOwn + g][e] : acc[g][e];
+          own[g][e] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, 16));
+        }
       }
-      st_acc[(ls * GQ + g) * kD + tid] = a;
-      if (tid == 0) {
-        sm.st_ml[ls][g][0] = M;
-        sm.st_ml[ls][g][1] = l;
+    State<GQ>& st = states[folded ? 0 : stripe - stripe0];
+    const bool first = !folded || stripe == stripe0;
+    const int head0 = GQ == 1 ? 0 : half * kOwn;
+    float (*dst)[kD] = &st.acc[warp][head0];
+    if (first) {
+      if (g8 == 0) {
+        if (has0) {
+          st.ml[warp][h0][0] = m_run[0];
+          st.ml[warp][h0][1] = l_run[0];
+        }
+        if (has1) {
+          st.ml[warp][h0 + 1][0] = m_run[1];
+          st.ml[warp][h0 + 1][1] = l_run[1];
+        }
+      }
+      if (GQ > 1 || half == 0) {
+#pragma unroll
+        for (int g = 0; g < kOwn; ++g)
+#pragma unroll
+          for (int e = 0; e < 8; e += 4)
+            *reinterpret_cast<float4*>(&dst[g][ln * 8 + e]) =
+                make_float4(own[g][e], own[g][e + 1], own[g][e + 2], own[g][e + 3]);
+      }
+    } else {
+      // every lane needs the maxima of the heads it keeps: head h sits in lanes t4 = h / 2, slot h % 2
+      FoldWeights fw[kOwn];
+#pragma unroll
+      for (int g = 0; g < kOwn; ++g) {
+        const int h = head0 + g;
+        const float a = __shfl_sync(0xffffffffu, m_run[0], h >> 1), d = __shfl_sync(0xffffffffu, m_run[1], h >> 1);
+        fw[g] = fold_weights(st.ml[warp][h][0], (h & 1) ? d : a, c);
+      }
+      __syncwarp();                                 // the old maxima have been read
+      if (g8 == 0) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (!(h == 0 ? has0 : has1)) continue;
+          float* ml = st.ml[warp][h0 + h];
+          const FoldWeights f = fold_weights(ml[0], m_run[h], c);
+          ml[0] = f.m;
+          ml[1] = fold_value(f, ml[1], l_run[h]);
+        }
+      }
+      if (GQ > 1 || half == 0) {
+#pragma unroll
+        for (int g = 0; g < kOwn; ++g)
+#pragma unroll
+          for (int e = 0; e < 8; e += 4) {
+            float4* at = reinterpret_cast<float4*>(&dst[g][ln * 8 + e]);
+            const float4 old = *at;
+            *at = make_float4(fold_value(fw[g], old.x, own[g][e]), fold_value(fw[g], old.y, own[g][e + 1]),
+                              fold_value(fw[g], old.z, own[g][e + 2]), fold_value(fw[g], old.w, own[g][e + 3]));
+          }
       }
     }
-    __syncthreads();
+    __syncwarp();                                   // the next stripe of this CTA reads the state
   }
 
-  // ---- merge the stripes in order; CTA r of the cluster writes its share of the outputs
-  if (splits > 1) {
-    cluster_arrive();
-    cluster_wait();
-  }
+  // ---- merge; CTA r of the cluster writes its share of the outputs
+  cluster_arrive();
+  cluster_wait();
   const int share = GQ * kD / splits;
-  const uint32_t ml_base = smem_u32(&sm.st_ml[0][0][0]), acc_base = smem_u32(st_acc);
+  const uint32_t st_base = smem_u32(states);
   for (int i = tid; i < share; i += kDecThreads) {
     const int o = rank * share + i, g = o / kD, d = o % kD;
-    float ms[kStripes], lsum[kStripes], as[kStripes];
+    float ms[2 * kWarps], ls[2 * kWarps], as[2 * kWarps];
+    auto fetch = [&](int stripe, int w, float& m, float& l, float& a) {    // stripe: of the eight, or the fold 0 / 1
+      const int owner = folded ? stripe : stripe / per_cta, slot = folded ? 0 : stripe % per_cta;
+      const uint32_t at = mapa_u32(st_base + slot * static_cast<uint32_t>(sizeof(State<GQ>)), owner);
+      const uint32_t ml = at + ((w * GQ + g) * 2) * 4;
+      m = ld_cluster_f32(ml);
+      l = ld_cluster_f32(ml + 4);
+      a = ld_cluster_f32(at + static_cast<uint32_t>(sizeof(State<GQ>::ml)) + ((w * GQ + g) * kD + d) * 4);
+    };
+    if (folded) {
 #pragma unroll
-    for (int s = 0; s < kStripes; ++s) {
-      const int owner = s / per_cta, ls = s - owner * per_cta;
-      const uint32_t ml = ml_base + (ls * GQ + g) * 8, ac = acc_base + ((ls * GQ + g) * kD + d) * 4;
-      if (splits > 1) {
-        const uint32_t mlr = mapa_u32(ml, owner);
-        ms[s] = ld_cluster_f32(mlr);
-        lsum[s] = ld_cluster_f32(mlr + 4);
-        as[s] = ld_cluster_f32(mapa_u32(ac, owner));
-      } else {
-        ms[s] = sm.st_ml[ls][g][0];
-        lsum[s] = sm.st_ml[ls][g][1];
-        as[s] = st_acc[(ls * GQ + g) * kD + d];
+      for (int f = 0; f < 2; ++f)
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) fetch(f, w, ms[f * kWarps + w], ls[f * kWarps + w], as[f * kWarps + w]);
+    } else {
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+        float m[4][kWarps], l[4][kWarps], a[4][kWarps];                    // all requested before the first is used
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+          for (int w = 0; w < kWarps; ++w) fetch(f * 4 + k, w, m[k][w], l[k][w], a[k][w]);
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+#pragma unroll
+          for (int k = 1; k < 4; ++k) {
+            const FoldWeights fw = fold_weights(m[0][w], m[k][w], c);
+            m[0][w] = fw.m;
+            l[0][w] = fold_value(fw, l[0][w], l[k][w]);
+            a[0][w] = fold_value(fw, a[0][w], a[k][w]);
+          }
+          ms[f * kWarps + w] = m[0][w];
+          ls[f * kWarps + w] = l[0][w];
+          as[f * kWarps + w] = a[0][w];
+        }
       }
     }
     float M = ms[0];
 #pragma unroll
-    for (int s = 1; s < kStripes; ++s) M = fmaxf(M, ms[s]);
+    for (int s = 1; s < 2 * kWarps; ++s) M = fmaxf(M, ms[s]);
     float a = 0.f, l = 0.f;
 #pragma unroll
-    for (int s = 0; s < kStripes; ++s) {
+    for (int s = 0; s < 2 * kWarps; ++s) {
       const float wt = state_weight(ms[s], M, c);
-      l = __fmaf_rn(wt, lsum[s], l);
+      l = __fmaf_rn(wt, ls[s], l);
       a = __fmaf_rn(wt, as[s], a);
     }
     out[(static_cast<size_t>(b) * hq + hk * GQ + g) * kD + d] = __float2bfloat16_rn(__fdiv_rn(a, l));
   }
-  if (splits > 1) {      // nobody leaves while its shared memory may still be read
-    cluster_arrive();
-    cluster_wait();
-  }
+  cluster_arrive();      // nobody leaves while its shared memory may still be read
+  cluster_wait();
 }
 
 template <int GQ>
@@ -346,9 +429,10 @@ int launch_split(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bflo
   // About four CTAs per SM of a 148-SM device keep enough loads in flight; more CTAs than that
   // only add merges. (The result does not depend on this choice.)
   constexpr long long kWanted = 4 * 148;
-  int splits = 1;
+  int splits = 2;
   while (splits < kStripes && static_cast<long long>(batch) * hkv * splits < kWanted) splits *= 2;
-  const int smem = static_cast<int>(sizeof(SplitSmem<GQ>)) + kStripes / splits * GQ * kD * 4;
+  const int smem = static_cast<int>(sizeof(SplitSmem<GQ>)) +
+                   (splits == 2 ? 1 : kStripes / splits) * static_cast<int>(sizeof(State<GQ>));
   if (smem > 48 * 1024 &&    // per device and cheap: set on every call that needs it
       cudaFuncSetAttribute(attention_decode_split_kernel<GQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
           cudaSuccess)
@@ -364,7 +448,7 @@ int launch_split(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bflo
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = splits > 1 ? 1 : 0;
+  cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, attention_decode_split_kernel<GQ>, q, k, v, lens, out, hq, hkv, max_len, scale,
                             splits) == cudaSuccess
              ? 0
