@@ -11,12 +11,15 @@
 // What bounds it is the weight stream, and an SM pulls at most about 80 GB/s, so every SM has
 // to have its share of the rows: the N rows are cut into tiles of R rows (R a multiple of 8, at
 // most 128) such that the tiles fill the SMs evenly, N = 4096 into 128 tiles of 32 rows instead
-// of 32 tiles of 128. The MMA still reads 128 rows of shared memory; what lies behind a shorter
-// tile (the next stage, or slack at the end) only reaches accumulator rows that nobody stores.
+// of 32 tiles of 128. The MMA reads 64 or 128 rows of shared memory (M = 64 for tiles of at most
+// 64 rows); what lies behind a shorter tile (the next stage, or slack at the end) only reaches
+// accumulator rows that nobody stores. M = 64 matters because those reads share the shared-memory
+// port with the arriving tiles: 39 cycles per MMA at M = 128, N = 16, 23 at M = 64, and N = 4096,
+// K = 14336 took 32.6 us with M = 128, 27.1 us with M = 64.
 // A CTA walks its tiles persistently; the ring of 128-wide K blocks runs on across tiles and the
 // accumulator is double-buffered.
 // Measured, 8 rows (64 rows): the four products of a Llama-3-8B decoder layer (436 MB of weights)
-// take 98 us (110 us); with 128 weight rows per CTA everywhere they took 157 us (164 us).
+// take 90 us (102 us); with 128 weight rows per CTA everywhere they took 157 us (164 us).
 //
 // The reference has no GEMM of its own (it names backends in rl_engine/kernels/registry.py:41-55).
 #include <cstdint>
@@ -29,13 +32,13 @@
 namespace ka {
 namespace {
 
-constexpr int kMmaRows = 128;  // M of the MMA (rows of shared memory it reads per K step)
+constexpr int kMaxRows = 128;  // largest M of the MMA (rows of shared memory it reads per K step)
 constexpr int kBox = 64;       // K columns of a TMA box: one 128-byte swizzled row
 constexpr int kBoxes = 2;      // boxes per stage
 constexpr int kThreads = 192;  // four epilogue warps, one TMA warp, one MMA warp
 constexpr int kMaxStages = 32;
 constexpr int kRingBytes = 192 * 1024;
-constexpr int kSmemBytes = kRingBytes + kMmaRows * kBox * 2 + 2048;   // ring, slack behind it, control
+constexpr int kSmemBytes = kRingBytes + kMaxRows * kBox * 2 + 2048;   // ring, slack behind it, control
 
 struct Control {
   uint64_t full[kMaxStages];
@@ -61,8 +64,8 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
-// NB: batch rows padded (the MMA's N)
-template <int NB>
+// NB: batch rows padded (the MMA's N); MR: weight rows of the MMA (its M)
+template <int NB, int MR>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                    const __grid_constant__ SkinnyParams p) {
@@ -70,7 +73,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t base = (raw_addr + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - raw_addr);
-  Control* ctl = reinterpret_cast<Control*>(smem + kRingBytes + kMmaRows * kBox * 2);
+  Control* ctl = reinterpret_cast<Control*>(smem + kRingBytes + kMaxRows * kBox * 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w_bytes = p.tile_rows * kBox * 2;                 // one box of the weight tile
   constexpr int kXBytes = NB * kBox * 2;
@@ -133,7 +136,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   } else if (warp == 5) {
     // ------------------------------------------------------------------ MMA issuer
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16_f32(kMmaRows, NB);
+      constexpr uint32_t idesc = umma_idesc_bf16_f32(MR, NB);
       const uint64_t d0 = umma_desc_k_sw128(base);
       int s = 0, i = 0;
       uint32_t phase = 0;
@@ -171,17 +174,19 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     }
   } else {
     // ------------------------------------------------------------------ epilogue
-    // TMEM lane = weight row (output column n), TMEM column = batch row m.
+    // TMEM column = batch row m. TMEM lane = weight row (output column n); with M = 64 the rows
+    // 16 w .. 16 w + 15 sit in the first half of warp w's 32 lanes.
+    constexpr int kWarpRows = MR / 4;
     int i = 0;
     for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x, ++i) {
       const int b = i & 1;
       const bool mine = mbar_wait_bounded(smem_u32(&ctl->acc_full[b]), (i >> 1) & 1, wctx, 63, i);
       if (__all_sync(0xffffffffu, mine) == 0) break;
       tc_fence_after_sync();
-      const int r = warp * 32 + lane, n = t * p.tile_rows + r;
-      const bool row_ok = r < p.tile_rows && n < p.n;
+      const int r = warp * kWarpRows + lane, n = t * p.tile_rows + r;
+      const bool row_ok = lane < kWarpRows && r < p.tile_rows && n < p.n;
       const uint32_t taddr = tmem_base + static_cast<uint32_t>(b * NB) + (static_cast<uint32_t>(warp * 32) << 16);
-      if (warp * 32 < p.tile_rows) {
+      if (warp * kWarpRows < p.tile_rows) {
 #pragma unroll
         for (int c0 = 0; c0 < NB; c0 += 16) {
           if (c0 >= p.m) break;
@@ -219,21 +224,11 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   }
 }
 
-template <int NB>
-int launch(const void* a, long long lda, const void* w, long long ldw, SkinnyParams p, cudaStream_t stream) {
-  if (cudaFuncSetAttribute(gemm_skinny_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) !=
+template <int NB, int MR>
+int launch(const void* a, long long lda, const void* w, long long ldw, SkinnyParams p, int sms, cudaStream_t stream) {
+  if (cudaFuncSetAttribute(gemm_skinny_kernel<NB, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) !=
       cudaSuccess)
     return -10;
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    return -12;
-  // Rows per tile: as many tiles as SMs, or a whole multiple of that when a tile would exceed the
-  // MMA's 128 rows, rounded up to the 8 rows of a swizzle atom.
-  const int rounds = (p.n + sms * kMmaRows - 1) / (sms * kMmaRows);
-  const int per = (p.n + sms * rounds - 1) / (sms * rounds);
-  p.tile_rows = (per + 7) / 8 * 8;
-  p.n_tiles = (p.n + p.tile_rows - 1) / p.tile_rows;
   const int stage_bytes = kBoxes * (p.tile_rows + NB) * kBox * 2;
   p.stages = kRingBytes / stage_bytes < kMaxStages ? kRingBytes / stage_bytes : kMaxStages;
   CUtensorMap tw, tx;
@@ -244,7 +239,7 @@ int launch(const void* a, long long lda, const void* w, long long ldw, SkinnyPar
                                 static_cast<uint64_t>(p.k), lda, NB, kBox);
   if (rc) return -40 + rc;
   const unsigned grid = static_cast<unsigned>(p.n_tiles < sms ? p.n_tiles : sms);
-  gemm_skinny_kernel<NB><<<grid, kThreads, kSmemBytes, stream>>>(tw, tx, p);
+  gemm_skinny_kernel<NB, MR><<<grid, kThreads, kSmemBytes, stream>>>(tw, tx, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -267,8 +262,23 @@ extern "C" int ka_gemm_skinny_bf16(const void* a, long long lda, const void* w, 
   p.k = k;
   p.status = status;
   p.timeout_ns = timeout_ns;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+    return -12;
+  // Rows per tile: as many tiles as SMs, or a whole multiple of that when a tile would exceed the
+  // MMA's 128 rows, rounded up to the 8 rows of a swizzle atom.
+  const int rounds = (p.n + sms * kMaxRows - 1) / (sms * kMaxRows);
+  const int per = (p.n + sms * rounds - 1) / (sms * rounds);
+  p.tile_rows = (per + 7) / 8 * 8;
+  p.n_tiles = (p.n + p.tile_rows - 1) / p.tile_rows;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (m <= 16) return launch<16>(a, lda, w, ldw, p, st);
-  if (m <= 32) return launch<32>(a, lda, w, ldw, p, st);
-  return launch<64>(a, lda, w, ldw, p, st);
+  if (p.tile_rows <= 64) {
+    if (m <= 16) return launch<16, 64>(a, lda, w, ldw, p, sms, st);
+    if (m <= 32) return launch<32, 64>(a, lda, w, ldw, p, sms, st);
+    return launch<64, 64>(a, lda, w, ldw, p, sms, st);
+  }
+  if (m <= 16) return launch<16, 128>(a, lda, w, ldw, p, sms, st);
+  if (m <= 32) return launch<32, 128>(a, lda, w, ldw, p, sms, st);
+  return launch<64, 128>(a, lda, w, ldw, p, sms, st);
 }
