@@ -74,7 +74,24 @@ def cuda() -> ctypes.CDLL:
         c_int,
         [c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p],
     )
+    _bind(lib, "ka_grpo_advantages", c_int, [c_void_p, c_void_p, c_int, c_int, c_float, c_void_p])
+    _bind(
+        lib,
+        "ka_grpo_loss_fwd",
+        c_int,
+        [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_float, c_float, c_int,
+         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
+    )
+    _bind(lib, "ka_grpo_loss_bwd", c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p])
     return lib
+
+
+def stream_ptr(device) -> int:
+    """The current stream of a CUDA device as the integer the kernels take."""
+    import torch
+
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    return torch._C._cuda_getCurrentRawStream(index)
 
 
 DTYPE_CODES = {"torch.float32": 0, "torch.bfloat16": 1, "torch.float16": 2}

@@ -24,10 +24,8 @@ def group_advantages(rewards: torch.Tensor, group_size: int, eps: float = 1e-4) 
     adv = torch.empty_like(r)
     n_groups = r.numel() // group_size
     if r.device.type == "cuda":
-        fn = _native.cuda().ka_grpo_advantages
-        fn.restype = c_int
-        fn.argtypes = [c_void_p, c_void_p, c_int, c_int, c_float, c_void_p]
-        rc = fn(r.data_ptr(), adv.data_ptr(), n_groups, group_size, eps, torch.cuda.current_stream(r.device).cuda_stream)
+        rc = _native.cuda().ka_grpo_advantages(r.data_ptr(), adv.data_ptr(), n_groups, group_size, eps,
+                                               _native.stream_ptr(r.device))
     else:
         fn = _native.cpu().ka_cpu_grpo_advantages
         fn.restype = c_int
@@ -41,56 +39,58 @@ def group_advantages(rewards: torch.Tensor, group_size: int, eps: float = 1e-4) 
 class _GrpoLossFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logp_new, logp_old, logp_ref, adv, mask, eps_low, eps_high, beta, seq_mean):
+        ctx.set_materialize_grads(False)
         n_seq, seq_len = logp_new.shape
-        ln = logp_new.detach().float().contiguous()
-        lo = logp_old.detach().float().contiguous()
-        lr = logp_ref.detach().float().contiguous() if logp_ref is not None else None
-        a = adv.detach().float().contiguous()
-        m = mask.to(torch.uint8).contiguous() if mask is not None else None
+        ln = logp_new.float().contiguous()
+        lo = logp_old.float().contiguous()
+        lr = logp_ref.float().contiguous() if logp_ref is not None else None
+        a = adv.float().contiguous()
+        ctx.shape = (n_seq, seq_len)
+        ctx.cuda = ln.device.type == "cuda"
         out = torch.empty(3, dtype=torch.float32, device=ln.device)
-        if ln.device.type == "cuda":
+        ctx.mark_non_differentiable(out)
+        if ctx.cuda:
+            # bytes and floats are read as they are, anything else is converted first
+            if mask is not None and mask.dtype not in (torch.bool, torch.uint8, torch.float32):
+                mask = mask.to(torch.uint8)
+            m = mask.contiguous() if mask is not None else None
             raw = torch.empty_like(ln)
             ws = torch.empty(4 * n_seq, dtype=torch.float32, device=ln.device)
-            fn = _native.cuda().ka_grpo_loss_fwd
-            fn.restype = c_int
-            fn.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_float, c_float,
-                           c_int, c_void_p, c_void_p, c_void_p, c_void_p]
-            rc = fn(ln.data_ptr(), lo.data_ptr(), lr.data_ptr() if lr is not None else None, a.data_ptr(),
-                    m.data_ptr() if m is not None else None, n_seq, seq_len, eps_low, eps_high, beta, int(seq_mean),
-                    raw.data_ptr(), ws.data_ptr(), out.data_ptr(), torch.cuda.current_stream(ln.device).cuda_stream)
+            loss = torch.empty((), dtype=torch.float32, device=ln.device)
+            rc = _native.cuda().ka_grpo_loss_fwd(
+                ln.data_ptr(), lo.data_ptr(), lr.data_ptr() if lr is not None else None, a.data_ptr(),
+                m.data_ptr() if m is not None else None, int(m is not None and m.dtype == torch.float32), n_seq,
+                seq_len, eps_low, eps_high, beta, int(seq_mean), raw.data_ptr(), ws.data_ptr(), loss.data_ptr(),
+                out.data_ptr(), _native.stream_ptr(ln.device))
             if rc != 0:
                 raise RuntimeError(f"ka_grpo_loss_fwd failed ({rc})")
             ctx.save_for_backward(raw, ws)
-            ctx.cuda = True
-        else:
-            grad = torch.empty_like(ln)
-            fn = _native.cpu().ka_cpu_grpo_loss
-            fn.restype = c_int
-            fn.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_float, c_float,
-                           c_int, c_void_p, c_void_p]
-            rc = fn(ln.data_ptr(), lo.data_ptr(), lr.data_ptr() if lr is not None else None, a.data_ptr(),
-                    m.data_ptr() if m is not None else None, n_seq, seq_len, eps_low, eps_high, beta, int(seq_mean),
-                    grad.data_ptr(), out.data_ptr())
-            if rc != 0:
-                raise RuntimeError(f"ka_cpu_grpo_loss failed ({rc})")
-            ctx.save_for_backward(grad)
-            ctx.cuda = False
-        ctx.shape = (n_seq, seq_len)
-        ctx.mark_non_differentiable(out)
+            return loss, out
+        m = mask.to(torch.uint8).contiguous() if mask is not None else None
+        grad = torch.empty_like(ln)
+        fn = _native.cpu().ka_cpu_grpo_loss
+        fn.restype = c_int
+        fn.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_float, c_float,
+                       c_int, c_void_p, c_void_p]
+        rc = fn(ln.data_ptr(), lo.data_ptr(), lr.data_ptr() if lr is not None else None, a.data_ptr(),
+                m.data_ptr() if m is not None else None, n_seq, seq_len, eps_low, eps_high, beta, int(seq_mean),
+                grad.data_ptr(), out.data_ptr())
+        if rc != 0:
+            raise RuntimeError(f"ka_cpu_grpo_loss failed ({rc})")
+        ctx.save_for_backward(grad)
         return out[0].clone(), out
 
     @staticmethod
     def backward(ctx, g_loss, _g_stats):
+        if g_loss is None:
+            return (None,) * 9
         n_seq, seq_len = ctx.shape
         if ctx.cuda:
             raw, ws = ctx.saved_tensors
             grad = torch.empty_like(raw)
-            up = g_loss.detach().float().reshape(1).contiguous()
-            fn = _native.cuda().ka_grpo_loss_bwd
-            fn.restype = c_int
-            fn.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]
-            rc = fn(raw.data_ptr(), ws[3 * n_seq:].data_ptr(), up.data_ptr(), grad.data_ptr(), n_seq, seq_len,
-                    torch.cuda.current_stream(raw.device).cuda_stream)
+            up = g_loss.float().contiguous()
+            rc = _native.cuda().ka_grpo_loss_bwd(raw.data_ptr(), ws.data_ptr() + 12 * n_seq, up.data_ptr(),
+                                                 grad.data_ptr(), n_seq, seq_len, _native.stream_ptr(raw.device))
             if rc != 0:
                 raise RuntimeError(f"ka_grpo_loss_bwd failed ({rc})")
         else:

@@ -52,6 +52,8 @@ def _check(dev):
             assert stats[2].item() == mask.sum().item()
             again = grpo_loss(ln, lo, adv, mask=mask, logp_ref=lr, beta=beta, reduction=reduction)
             assert again.item() == loss.item()  # bitwise repeatable
+            floats = grpo_loss(ln, lo, adv, mask=mask.float(), logp_ref=lr, beta=beta, reduction=reduction)
+            assert floats.item() == loss.item()
 
 
 def test_grpo_loss_cpu():
