@@ -19,7 +19,7 @@
 //     eight folded states (2 halves x 4 warps) are merged in order. This decomposition depends on
 //     the number of keys alone, so a row's bits do not depend on its batch. How many CTAs work on
 //     a (sequence, KV head) does: a cluster of S = 2, 4 or 8 takes 8 / S stripes each, the
-//     smallest S that gives about four CTAs per SM. With S = 2 a CTA folds its own stripes; the
+//     largest S whose CTAs are all resident at once. With S = 2 a CTA folds its own stripes; the
 //     rest is read from the other CTAs through distributed shared memory.
 //
 // The reference has no decode attention (its executor comments defer generation to a future
@@ -226,6 +226,16 @@ attention_decode_split_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bf
   const int h0 = 2 * t4;
   const bool has0 = h0 < GQ, has1 = h0 + 1 < GQ;
   for (int stripe = stripe0; stripe < stripe_end; ++stripe) {
+    if (stripe >= n_blocks) {      // no keys: an empty state where somebody reads one, nothing to fold otherwise
+      if (!folded || stripe == stripe0) {
+        State<GQ>& st = states[folded ? 0 : stripe - stripe0];
+        if (lane < GQ) {
+          st.ml[warp][lane][0] = -CUDART_INF_F;
+          st.ml[warp][lane][1] = 0.f;
+        }
+      }
+      continue;
+    }
     float acc[GQ][8];
 #pragma unroll
     for (int g = 0; g < GQ; ++g)
@@ -378,6 +388,7 @@ attention_decode_split_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bf
       m = ld_cluster_f32(ml);
       l = ld_cluster_f32(ml + 4);
       a = ld_cluster_f32(at + static_cast<uint32_t>(sizeof(State<GQ>::ml)) + ((w * GQ + g) * kD + d) * 4);
+      if (m == -CUDART_INF_F) a = 0.f;      // an empty state has no accumulator
     };
     if (folded) {
 #pragma unroll
@@ -426,11 +437,15 @@ attention_decode_split_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bf
 template <int GQ>
 int launch_split(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v, const int* lens,
                  __nv_bfloat16* out, int batch, int hq, int hkv, int max_len, float scale, cudaStream_t st) {
-  // About four CTAs per SM of a 148-SM device keep enough loads in flight; more CTAs than that
-  // only add merges. (The result does not depend on this choice.)
-  constexpr long long kWanted = 4 * 148;
+  // As many CTAs as are resident at once (three per SM of a 148-SM device), and no more than the
+  // cache has blocks: a second wave, or CTAs without keys, cost a set-up and two cluster barriers
+  // for nothing (8 x 448 keys, 32 / 8 heads:
+  // 10.0 us with S = 4, 13.7 with S = 8; 32 x 100 keys: 14 us, 26 us without these limits). The result does not depend on this choice.
+  constexpr long long kResident = 3 * 148;
+  const int blocks = (max_len + kBlockKeys - 1) / kBlockKeys;
   int splits = 2;
-  while (splits < kStripes && static_cast<long long>(batch) * hkv * splits < kWanted) splits *= 2;
+  while (splits < kStripes && splits < blocks && static_cast<long long>(batch) * hkv * splits * 2 <= kResident)
+    splits *= 2;
   const int smem = static_cast<int>(sizeof(SplitSmem<GQ>)) +
                    (splits == 2 ? 1 : kStripes / splits) * static_cast<int>(sizeof(State<GQ>));
   if (smem > 48 * 1024 &&    // per device and cheap: set on every call that needs it
