@@ -16,6 +16,7 @@
 // The reference has no attention kernel and no backward pass of any kind: it routes the op
 // type "attention" to a backend name (rl_engine/kernels/registry.py:41-55).
 #include <cstdint>
+#include <type_traits>
 #include <cuda_bf16.h>
 #include <math_constants.h>
 
@@ -29,7 +30,9 @@ namespace {
 
 constexpr int kD = 128;
 constexpr int kT = 128;                    // tile rows (queries or keys)
-constexpr int kSoftThreads = 256;          // 8 warps: two threads per TMEM lane (64 columns each)
+constexpr int kParts = 4;                  // threads per TMEM lane
+constexpr int kPartCols = kT / kParts;     // columns of a tile each of them takes
+constexpr int kSoftThreads = kT * kParts;  // 16 warps
 constexpr int kThreads = kSoftThreads + 64;  // + TMA warp + MMA warp
 constexpr int kWarpTma = kSoftThreads / 32, kWarpMma = kSoftThreads / 32 + 1;
 constexpr int kTileBytes = 128 * 128 * 2;
@@ -98,22 +101,34 @@ __device__ __forceinline__ void mul2(float& d0, float& d1, float a0, float a1, f
       : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
 }
 
+// 32 consecutive fp32 values of a row, as bf16.
+__device__ __forceinline__ void store_row32(__nv_bfloat16* dst, const uint32_t (&v)[32]) {
+#pragma unroll
+  for (int i = 0; i < 32; i += 8)
+    *reinterpret_cast<uint4*>(dst + i) = make_uint4(pack_bf16(__uint_as_float(v[i]), __uint_as_float(v[i + 1])),
+                                                    pack_bf16(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])),
+                                                    pack_bf16(__uint_as_float(v[i + 4]), __uint_as_float(v[i + 5])),
+                                                    pack_bf16(__uint_as_float(v[i + 6]), __uint_as_float(v[i + 7])));
+}
+
 // Offset (in 16-byte descriptor units) of K step kk of a 128 x 128 tile: K-major, MN-major.
 __device__ __forceinline__ constexpr uint64_t kstep(int kk) { return ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4; }
 __device__ __forceinline__ constexpr uint64_t mnstep(int kk) { return (kk * 2048) >> 4; }
-// Column of K step kk of a bf16 A operand that overlays a 128-column fp32 region: the threads of
-// part 0 write 32 packed columns over their own fp32 columns [0, 64), part 1 over [64, 128).
-__device__ __forceinline__ constexpr uint32_t tcol(int kk) { return kk < 4 ? kk * 8 : 64 + (kk - 4) * 8; }
+// Column of K step kk of a bf16 A operand that overlays a 128-column fp32 region: the threads of a
+// part write 16 packed columns over the first half of their own 32 fp32 columns.
+__device__ __forceinline__ constexpr uint32_t tcol(int kk) { return (kk >> 1) * kPartCols + (kk & 1) * 8; }
 
 // ------------------------------------------------------------------------------------------------
 // Both kernels overlap the tensor core with the element-wise work: the operand of the next
 // iteration is in a second shared-memory stage, the next S and dP products are issued as soon as
 // their TMEM columns have been read, and the 16-bit operand that comes out of S goes back to TMEM
 // over the columns of S (the A operand of the product that follows), which leaves shared memory
-// to the loaded tiles. Tiles that need no mask take a path without comparisons.
+// to the loaded tiles. Sixteen warps share a tile (eight issued in a quarter of the cycles: with two
+// warps per scheduler nothing covers the TMEM loads and barriers), and tiles that need no mask
+// run a loop of their own, without comparisons.
 // One iteration is three products of 512 cycles (dQ) or four (dK / dV); with a single stage and
 // everything in sequence it took about 9000 cycles. B = 2, L = 4000, 32 / 8 heads, causal:
-// dQ 891 -> 519 us, dK / dV 1466 -> 833 us; B = 8, L = 512: dQ 114 -> 68 us, dK / dV 173 -> 91 us.
+// dQ 891 -> 500 us, dK / dV 1466 -> 530 us; B = 8, L = 512: dQ 114 -> 66 us, dK / dV 173 -> 62 us.
 // ------------------------------------------------------------------------------------------------
 struct CtlDq {
   uint64_t qdo_full;                 // Q and dO tiles loaded
@@ -252,6 +267,7 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     const int row = tid & 127, part = tid >> 7;
     const int q_pos = q_row0 + row;
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t part_base = lane_base + part * kPartCols;
     const float c = p.scale * kLog2e;
     const bool row_ok = q_pos < p.seq_len;
     const long long stat = (static_cast<long long>(b) * p.hq + h) * p.seq_len + q_pos;
@@ -263,58 +279,48 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       ok = __all_sync(0xffffffffu, mine) != 0;
       if (!ok) break;
       tc_fence_after_sync();
-      const uint32_t tmem_s = tmem_base + static_cast<uint32_t>((j & 1) * 128 + part * 64) + lane_base;
-      uint32_t s0[32], s1[32], g0[32], g1[32];
+      const uint32_t tmem_s = tmem_base + static_cast<uint32_t>((j & 1) * 128) + part_base;
+      uint32_t sv[32], gv[32], w[16];
       __syncwarp();
-      tmem_ld_32x32(tmem_s, s0);
-      tmem_ld_32x32(tmem_s + 32, s1);
-      tmem_ld_wait_dep(s0);
-      tmem_ld_wait_dep(s1);
-      const int kv0 = j * kT + part * 64;
-      const bool full = p.causal ? j < qt : (j + 1) * kT <= p.seq_len;   // uniform over the CTA
-      const int limit = full ? 64 : (row_ok ? ((p.causal ? q_pos : p.seq_len - 1) - kv0) : -1);
-      auto probs = [&](uint32_t (&sv)[32]) {
+      tmem_ld_32x32(tmem_s, sv);
+      tmem_ld_wait_dep(sv);
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float e0, e1;
-          fma2(e0, e1, __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]), c, c, neg_lse2, neg_lse2);
-          sv[i] = __float_as_uint(ex2_approx(e0));
-          sv[i + 1] = __float_as_uint(ex2_approx(e1));
-        }
-      };
-      probs(s0);
-      probs(s1);
+      for (int i = 0; i < 32; i += 2) {
+        float e0, e1;
+        fma2(e0, e1, __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]), c, c, neg_lse2, neg_lse2);
+        sv[i] = __float_as_uint(ex2_approx(e0));
+        sv[i + 1] = __float_as_uint(ex2_approx(e1));
+      }
       mine = mbar_wait_bounded(smem_u32(&ctl->dp_full), j & 1, wctx, 45, j);
       ok = __all_sync(0xffffffffu, mine) != 0;
       if (!ok) break;
       tc_fence_after_sync();
       __syncwarp();
-      tmem_ld_32x32(tmem_dp + lane_base + part * 64, g0);
-      tmem_ld_32x32(tmem_dp + lane_base + part * 64 + 32, g1);
-      tmem_ld_wait_dep(g0);
-      tmem_ld_wait_dep(g1);
+      tmem_ld_32x32(tmem_dp + part_base, gv);
+      tmem_ld_wait_dep(gv);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&ctl->dp_read));
-      auto grads = [&](uint32_t (&sv)[32], uint32_t (&gv)[32], int col) {   // packed into sv[0 .. 15]
+      auto grads = [&](auto masked, int limit) {      // limit: last allowed column of this part
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
           float d0, d1;
           add2(d0, d1, __uint_as_float(gv[i]), __uint_as_float(gv[i + 1]), neg_dlt, neg_dlt);
           mul2(d0, d1, __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]), d0, d1);
           mul2(d0, d1, d0, d1, p.scale, p.scale);
-          if (!full) {
-            if (col + i > limit) d0 = 0.f;
-            if (col + i + 1 > limit) d1 = 0.f;
+          if constexpr (decltype(masked)::value) {
+            d0 = i > limit ? 0.f : d0;
+            d1 = i + 1 > limit ? 0.f : d1;
           }
-          sv[i >> 1] = pack_bf16(d0, d1);
+          w[i >> 1] = pack_bf16(d0, d1);
         }
       };
-      grads(s0, g0, 0);
-      grads(s1, g1, 32);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) s0[16 + i] = s1[i];
-      tmem_st_32x32(tmem_s, s0);
+      if (p.causal ? j < qt : (j + 1) * kT <= p.seq_len)       // uniform over the CTA
+        grads(std::false_type{}, 0);
+      else
+        grads(std::true_type{},
+              row_ok ? (p.causal ? q_pos : p.seq_len - 1) - (j * kT + part * kPartCols) : -1);
+      tmem_st_32x16(tmem_s, w);
       tmem_st_wait();
       tc_fence_before_sync();
       __syncwarp();
@@ -326,23 +332,12 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
     }
     if (ok) {
       tc_fence_after_sync();
-      __nv_bfloat16* dst = p.dq + static_cast<long long>(tok0 + q_pos) * p.dq_stride + h * kD + part * 64;
-#pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        uint32_t v[32];
-        __syncwarp();
-        tmem_ld_32x32(tmem_dq + lane_base + part * 64 + g * 32, v);
-        tmem_ld_wait_dep(v);
-        if (row_ok) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 8)
-            *reinterpret_cast<uint4*>(dst + g * 32 + i) =
-                make_uint4(pack_bf16(__uint_as_float(v[i]), __uint_as_float(v[i + 1])),
-                           pack_bf16(__uint_as_float(v[i + 2]), __uint_as_float(v[i + 3])),
-                           pack_bf16(__uint_as_float(v[i + 4]), __uint_as_float(v[i + 5])),
-                           pack_bf16(__uint_as_float(v[i + 6]), __uint_as_float(v[i + 7])));
-        }
-      }
+      __nv_bfloat16* dst = p.dq + static_cast<long long>(tok0 + q_pos) * p.dq_stride + h * kD + part * kPartCols;
+      uint32_t v[32];
+      __syncwarp();
+      tmem_ld_32x32(tmem_dq + part_base, v);
+      tmem_ld_wait_dep(v);
+      if (row_ok) store_row32(dst, v);
     }
   }
   if (ctl->abort_flag) drain_in_flight();
@@ -506,30 +501,31 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       }
     }
   } else {
-    // Thread (row, part): KV row `row` of the tile, query columns [part * 64, part * 64 + 64).
-    // One named barrier per iteration, reached by all 256 threads whatever happened before.
+    // Thread (row, part): KV row `row` of the tile, 32 query columns from part * 32.
+    // One named barrier per iteration, reached by all threads whatever happened before.
     const int tid = threadIdx.x;
     const int row = tid & 127, part = tid >> 7;
     const int kv_pos = kv_row0 + row;
     const bool row_ok = kv_pos < p.seq_len;
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t part_base = lane_base + part * kPartCols;
     const float c = p.scale * kLog2e;
-    const uint32_t tmem_s = tmem_st + lane_base + part * 64, tmem_g = tmem_dpt + lane_base + part * 64;
+    const uint32_t tmem_s = tmem_st + part_base, tmem_g = tmem_dpt + part_base;
     bool ok = true;
-    // row statistics of the q tile of iteration n: threads 0..127 the log-sum-exp, 128..255 delta
+    // row statistics of the q tile of iteration n: part 0 fetches the log-sum-exp, part 1 delta
     auto stat_of = [&](int n) {
       const int h = hk * group + n / n_q, qp = (qt0 + n % n_q) * kT + row;
       if (qp >= p.seq_len) return 0.f;
       const long long at = (static_cast<long long>(b) * p.hq + h) * p.seq_len + qp;
       return part == 0 ? __fmul_rn(-p.lse[at], kLog2e) : -p.delta[at];
     };
-    float next_stat = n_iter > 0 ? stat_of(0) : 0.f;
+    float next_stat = n_iter > 0 && part < 2 ? stat_of(0) : 0.f;
     for (int n = 0; n < n_iter; ++n) {
       const int qt = qt0 + n % n_q;
       const int buf = n & 1;
-      (part == 0 ? ctl->lse2[buf] : ctl->neg_delta[buf])[row] = next_stat;
+      if (part < 2) (part == 0 ? ctl->lse2[buf] : ctl->neg_delta[buf])[row] = next_stat;
       asm volatile("bar.sync 1, %0;" ::"n"(kSoftThreads) : "memory");
-      if (n + 1 < n_iter) next_stat = stat_of(n + 1);
+      if (n + 1 < n_iter && part < 2) next_stat = stat_of(n + 1);
       if (ctl->abort_flag) ok = false;
       if (ok) {
         const bool mine = mbar_wait_bounded(smem_u32(&ctl->st_full), n & 1, wctx, 55, n);
@@ -537,41 +533,38 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       }
       if (!ok) continue;
       tc_fence_after_sync();
-      const int q0 = qt * kT + part * 64;  // first query column of this thread
+      const int q0 = qt * kT + part * kPartCols;  // first query column of this thread
       const bool full = (!p.causal || qt > jt) && (qt + 1) * kT <= p.seq_len;   // uniform over the CTA
-      const float4* lse4 = reinterpret_cast<const float4*>(&ctl->lse2[buf][part * 64]);
-      const float4* dlt4 = reinterpret_cast<const float4*>(&ctl->neg_delta[buf][part * 64]);
-      uint32_t s0[32], s1[32];
+      // columns [first, end) of this part are allowed for this row
+      const int first = p.causal ? kv_pos - q0 : 0, end = row_ok ? p.seq_len - q0 : 0;
+      const float4* lse4 = reinterpret_cast<const float4*>(&ctl->lse2[buf][part * kPartCols]);
+      const float4* dlt4 = reinterpret_cast<const float4*>(&ctl->neg_delta[buf][part * kPartCols]);
+      uint32_t sv[32], w[16];
       __syncwarp();
-      tmem_ld_32x32(tmem_s, s0);
-      tmem_ld_32x32(tmem_s + 32, s1);
-      tmem_ld_wait_dep(s0);
-      tmem_ld_wait_dep(s1);
-      // P (kept in fp32 for dS), packed for the product
-      uint32_t w[32];
-      auto probs = [&](uint32_t (&sv)[32], int g) {
+      tmem_ld_32x32(tmem_s, sv);
+      tmem_ld_wait_dep(sv);
+      auto probs = [&](auto masked) {             // P, kept in fp32 for dS, packed for the product
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
-          const float4 l = lse4[(g * 32 + i) >> 2];
+          const float4 l = lse4[i >> 2];
           float e[4];
           fma2(e[0], e[1], __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]), c, c, l.x, l.y);
           fma2(e[2], e[3], __uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3]), c, c, l.z, l.w);
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             e[k] = ex2_approx(e[k]);
-            if (!full) {
-              const int qp = q0 + g * 32 + i + k;
-              if (!(row_ok && qp < p.seq_len && (!p.causal || kv_pos <= qp))) e[k] = 0.f;
-            }
+            if constexpr (decltype(masked)::value) e[k] = i + k >= first && i + k < end ? e[k] : 0.f;
             sv[i + k] = __float_as_uint(e[k]);
           }
-          w[(g * 32 + i) >> 1] = pack_bf16(e[0], e[1]);
-          w[((g * 32 + i) >> 1) + 1] = pack_bf16(e[2], e[3]);
+          w[i >> 1] = pack_bf16(e[0], e[1]);
+          w[(i >> 1) + 1] = pack_bf16(e[2], e[3]);
         }
       };
-      probs(s0, 0);
-      probs(s1, 1);
-      tmem_st_32x32(tmem_s, w);
+      if (full)
+        probs(std::false_type{});
+      else
+        probs(std::true_type{});
+      tmem_st_32x16(tmem_s, w);
       tmem_st_wait();
       tc_fence_before_sync();
       __syncwarp();
@@ -580,54 +573,42 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       ok = __all_sync(0xffffffffu, mine) != 0;
       if (!ok) continue;
       tc_fence_after_sync();
-      uint32_t g0[32], g1[32];
+      uint32_t gv[32];
       __syncwarp();
-      tmem_ld_32x32(tmem_g, g0);
-      tmem_ld_32x32(tmem_g + 32, g1);
-      tmem_ld_wait_dep(g0);
-      tmem_ld_wait_dep(g1);
+      tmem_ld_32x32(tmem_g, gv);
+      tmem_ld_wait_dep(gv);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&ctl->dp_read));
-      auto grads = [&](const uint32_t (&pv)[32], const uint32_t (&gv)[32], int g) {
+      auto grads = [&](auto masked) {
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
-          const float4 d = dlt4[(g * 32 + i) >> 2];
+          const float4 d = dlt4[i >> 2];
           float t[4];
           add2(t[0], t[1], __uint_as_float(gv[i]), __uint_as_float(gv[i + 1]), d.x, d.y);
           add2(t[2], t[3], __uint_as_float(gv[i + 2]), __uint_as_float(gv[i + 3]), d.z, d.w);
-          mul2(t[0], t[1], __uint_as_float(pv[i]), __uint_as_float(pv[i + 1]), t[0], t[1]);
-          mul2(t[2], t[3], __uint_as_float(pv[i + 2]), __uint_as_float(pv[i + 3]), t[2], t[3]);
+          mul2(t[0], t[1], __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]), t[0], t[1]);
+          mul2(t[2], t[3], __uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3]), t[2], t[3]);
           mul2(t[0], t[1], t[0], t[1], p.scale, p.scale);
           mul2(t[2], t[3], t[2], t[3], p.scale, p.scale);
-          if (!full) {       // a masked column may hold anything: 0 * it need not be 0
+          if constexpr (decltype(masked)::value) {       // a masked column may hold anything: 0 * it need not be 0
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const int qp = q0 + g * 32 + i + k;
-              if (!(row_ok && qp < p.seq_len && (!p.causal || kv_pos <= qp))) t[k] = 0.f;
-            }
+            for (int k = 0; k < 4; ++k) t[k] = i + k >= first && i + k < end ? t[k] : 0.f;
           }
-          w[(g * 32 + i) >> 1] = pack_bf16(t[0], t[1]);
-          w[((g * 32 + i) >> 1) + 1] = pack_bf16(t[2], t[3]);
+          w[i >> 1] = pack_bf16(t[0], t[1]);
+          w[(i >> 1) + 1] = pack_bf16(t[2], t[3]);
         }
       };
-      grads(s0, g0, 0);
-      grads(s1, g1, 1);
+      if (full)
+        grads(std::false_type{});
+      else
+        grads(std::true_type{});
       if (n > 0) {           // the product of the previous dS^T has read the tile
         mine = mbar_wait_bounded(smem_u32(&ctl->ds_empty), (n - 1) & 1, wctx, 59, n);
         ok = __all_sync(0xffffffffu, mine) != 0;
         if (!ok) continue;
       }
-      {
-        uint32_t lo[16], hi[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          lo[i] = w[i];
-          hi[i] = w[16 + i];
-        }
-        store_tile_row32(dst_ptr, row, part * 64, lo);
-        store_tile_row32(dst_ptr, row, part * 64 + 32, hi);
-      }
+      store_tile_row32(dst_ptr, row, part * kPartCols, w);
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&ctl->ds_full));
@@ -638,32 +619,17 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     }
     if (ok) {
       tc_fence_after_sync();
-      __nv_bfloat16* dk = p.dk + static_cast<long long>(tok0 + kv_pos) * p.dk_stride + hk * kD + part * 64;
-      __nv_bfloat16* dv_out = p.dv + static_cast<long long>(tok0 + kv_pos) * p.dv_stride + hk * kD + part * 64;
-#pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        uint32_t a[32], bq[32];
-        __syncwarp();
-        tmem_ld_32x32(tmem_dv + lane_base + part * 64 + g * 32, a);
-        tmem_ld_32x32(tmem_dk + lane_base + part * 64 + g * 32, bq);
-        tmem_ld_wait_dep(a);
-        tmem_ld_wait_dep(bq);
-        if (row_ok) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            *reinterpret_cast<uint4*>(dv_out + g * 32 + i) =
-                make_uint4(pack_bf16(__uint_as_float(a[i]), __uint_as_float(a[i + 1])),
-                           pack_bf16(__uint_as_float(a[i + 2]), __uint_as_float(a[i + 3])),
-                           pack_bf16(__uint_as_float(a[i + 4]), __uint_as_float(a[i + 5])),
-                           pack_bf16(__uint_as_float(a[i + 6]), __uint_as_float(a[i + 7])));
-            *reinterpret_cast<uint4*>(dk + g * 32 + i) =
-                make_uint4(pack_bf16(__uint_as_float(bq[i]), __uint_as_float(bq[i + 1])),
-                           pack_bf16(__uint_as_float(bq[i + 2]), __uint_as_float(bq[i + 3])),
-                           pack_bf16(__uint_as_float(bq[i + 4]), __uint_as_float(bq[i + 5])),
-                           pack_bf16(__uint_as_float(bq[i + 6]), __uint_as_float(bq[i + 7])));
-          }
-        }
-      }
+      const long long tok = tok0 + kv_pos;
+      const int col = hk * kD + part * kPartCols;
+      uint32_t v[32];
+      __syncwarp();
+      tmem_ld_32x32(tmem_dv + part_base, v);
+      tmem_ld_wait_dep(v);
+      if (row_ok) store_row32(p.dv + tok * p.dv_stride + col, v);
+      __syncwarp();
+      tmem_ld_32x32(tmem_dk + part_base, v);
+      tmem_ld_wait_dep(v);
+      if (row_ok) store_row32(p.dk + tok * p.dk_stride + col, v);
     }
   }
   if (ctl->abort_flag) drain_in_flight();
