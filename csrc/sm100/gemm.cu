@@ -28,23 +28,30 @@ constexpr int kEpiWarps = 8;        // two per TMEM lane quarter: columns [0,128
 constexpr int kEpiThreads = kEpiWarps * 32;
 constexpr int kWarpTma = kEpiWarps, kWarpMma = kEpiWarps + 1, kWarpPub = kEpiWarps + 2;
 constexpr int kThreads = kEpiThreads + 96;  // epilogue warps, TMA producer, MMA issuer, one spare warp
-constexpr int kStages = 6;
+constexpr int kMaxStages = 8;
 constexpr int kABytes = kBM * kBK * 2;            // 16 KiB
-constexpr int kBBytes = (kBN / kG) * kBK * 2;     // 16 KiB
-constexpr int kStageBytes = kABytes + kBBytes;
-constexpr int kTxBytes = kStageBytes * kG;
-constexpr int kTileBytes = kStages * kStageBytes;
+constexpr int kTileBytes = 192 * 1024;            // the operand ring
 constexpr int kEpiBufWords = 32 * 33;     // per epilogue warp: 32 rows x 32 words, padded
 constexpr int kSmemBytes = kTileBytes + 1024 + 512 + kEpiWarps * kEpiBufWords * 4;
 constexpr int kGroupM = 8;         // row tiles that share a column tile in the schedule
 
 struct Control {
-  uint64_t full[kStages];
-  uint64_t empty[kStages];
+  uint64_t full[kMaxStages];
+  uint64_t empty[kMaxStages];
   uint64_t tfull[2];
   uint64_t tempty[2];
   uint32_t tmem_base;
   int abort_flag;
+};
+
+// Columns per tile: BN = kBN, or half of it for small products (see narrow_tiles).
+template <int BN>
+struct Cfg {
+  static constexpr int kBBytes = (BN / kG) * kBK * 2;
+  static constexpr int kStageBytes = kABytes + kBBytes;
+  static constexpr int kTxBytes = kStageBytes * kG;
+  static constexpr int kStages = kTileBytes / kStageBytes;      // 6, or 8 for the narrow tile
+  static_assert(kStages <= kMaxStages, "barriers of the ring");
 };
 
 enum Where : int { kWProducer = 11, kWMmaFull = 12, kWMmaTmem = 13, kWEpi = 14, kWReduceFlag = 15, kWGatherFlag = 16 };
@@ -235,9 +242,10 @@ __device__ __forceinline__ float4 add4(float4 a, float4 b) {
 constexpr int kTreeSlices = 8;
 constexpr int kTreeSlotFloats = kBM * kBN;
 
+template <int BN>
 __device__ __forceinline__ float4* tree_slot(float* scratch, int cta, int slot, int warp, int g, int lane) {
   return reinterpret_cast<float4*>(scratch + (static_cast<size_t>(cta) * 2 + slot) * kTreeSlotFloats) +
-         (warp * (kBN / 64) + g) * 8 * 32 + lane;   // eight float4 per thread and group, 32 apart
+         (warp * (BN / 64) + g) * 8 * 32 + lane;   // eight float4 per thread and group, 32 apart
 }
 
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
@@ -245,6 +253,7 @@ __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w 
 
 // One 32-column group of slice `s`. `v`: the accumulators; `leaf`: the packed even slice of the
 // pair. Returns true when the tile is finished: `v` then holds 32 sums.
+template <int BN>
 __device__ __forceinline__ bool tree_group(float* scratch, int s, int warp, int g, int lane, uint32_t (&v)[32],
                                            uint32_t (&leaf)[16]) {
   if ((s & 1) == 0) {
@@ -252,8 +261,8 @@ __device__ __forceinline__ bool tree_group(float* scratch, int s, int warp, int 
     for (int j = 0; j < 16; ++j) leaf[j] = pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
     return false;
   }
-  float4* s0 = tree_slot(scratch, blockIdx.x, 0, warp, g, lane);
-  float4* s1 = tree_slot(scratch, blockIdx.x, 1, warp, g, lane);
+  float4* s0 = tree_slot<BN>(scratch, blockIdx.x, 0, warp, g, lane);
+  float4* s1 = tree_slot<BN>(scratch, blockIdx.x, 1, warp, g, lane);
   float4 t[8];
   if (s == 3 || s == 7) {
     const float4* src = s == 3 ? s0 : s1;
@@ -330,10 +339,11 @@ __device__ __forceinline__ void tree_store(const GemmParams& p, const uint32_t (
   __syncwarp();
 }
 
-template <bool kTree>
+template <bool kTree, int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                  const __grid_constant__ GemmParams p) {
+  using C = Cfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   const uint32_t tiles_addr = (raw_addr + 1023u) & ~1023u;
@@ -348,7 +358,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   const int pair_id = blockIdx.x / kG;
   const int n_pairs = gridDim.x / kG;
   const int tiles_m = (p.m + kBM * kG - 1) / (kBM * kG);
-  const int tiles_n = (p.n + kBN - 1) / kBN;
+  const int tiles_n = (p.n + BN - 1) / BN;
   const int n_units = tiles_m * tiles_n * p.k_slices;
   const int k_per_slice = p.k / p.k_slices;
   const int num_kb = (k_per_slice + kBK - 1) / kBK;
@@ -356,7 +366,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   WaitCtx wctx{&ctl->abort_flag, p.status, p.timeout_ns};
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < C::kStages; ++s) {
       mbar_init(smem_u32(&ctl->full[s]), 1);
       mbar_init(smem_u32(&ctl->empty[s]), 1);
     }
@@ -368,7 +378,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     fence_mbar_init_cluster();
   }
   if (warp == kWarpMma) {
-    tmem_alloc<kG>(smem_u32(&ctl->tmem_base), 512);
+    tmem_alloc<kG>(smem_u32(&ctl->tmem_base), 2 * BN);
     tmem_relinquish<kG>();
   }
   if (warp == kWarpTma && lane == 0) {
@@ -392,7 +402,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         Unit un;
         decode_unit(p, tiles_m, tiles_n, u, un);
         const int row0 = un.m_blk * (kBM * kG) + static_cast<int>(cta_rank) * kBM;
-        const int col0 = un.n_blk * kBN + static_cast<int>(cta_rank) * (kBN / kG);
+        const int col0 = un.n_blk * BN + static_cast<int>(cta_rank) * (BN / kG);
         const int kbase = un.slice * k_per_slice;
         if (p.a_gather) {
           // rows of another rank become readable when that rank's push has been flagged
@@ -407,10 +417,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         for (int kb = 0; kb < num_kb; ++kb) {
           ok = mbar_wait_bounded(smem_u32(&ctl->empty[stage]), phase ^ 1u, wctx, kWProducer, stage);
           if (!ok) break;
-          const uint32_t a_dst = tiles_addr + stage * kStageBytes;
+          const uint32_t a_dst = tiles_addr + stage * C::kStageBytes;
           const uint32_t b_dst = a_dst + kABytes;
           const uint32_t full = smem_u32(&ctl->full[stage]);
-          if (leader) mbar_arrive_expect_tx(full, kTxBytes);
+          if (leader) mbar_arrive_expect_tx(full, C::kTxBytes);
           const uint32_t full_leader = mapa_u32(full, 0);
           const int k0 = kbase + kb * kBK;
           if (p.a_major == 0) {
@@ -423,9 +433,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             tma_load_2d_pair(b_dst, &tm_b, k0, col0, full_leader);
           } else {
             tma_load_2d_pair(b_dst, &tm_b, col0, k0, full_leader);
-            tma_load_2d_pair(b_dst + 8192, &tm_b, col0 + 64, k0, full_leader);
+            if constexpr (BN / kG > 64) tma_load_2d_pair(b_dst + 8192, &tm_b, col0 + 64, k0, full_leader);
           }
-          if (++stage == kStages) {
+          if (++stage == C::kStages) {
             stage = 0;
             phase ^= 1u;
           }
@@ -435,7 +445,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   } else if (warp == kWarpMma) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0 && leader) {
-      const uint32_t idesc = umma_idesc_bf16_f32(kBM * kG, kBN) | (static_cast<uint32_t>(p.a_major) << 15) |
+      const uint32_t idesc = umma_idesc_bf16_f32(kBM * kG, BN) | (static_cast<uint32_t>(p.a_major) << 15) |
                              (static_cast<uint32_t>(p.b_major) << 16);
       const uint32_t a_step = p.a_major == 0 ? 2u : 128u;  // descriptor units (16 B) per K=16
       const uint32_t b_step = p.b_major == 0 ? 2u : 128u;
@@ -448,12 +458,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         ok = mbar_wait_bounded(smem_u32(&ctl->tempty[abuf]), aphase ^ 1u, wctx, kWMmaTmem, abuf);
         if (!ok) break;
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(abuf * kBN);
+        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(abuf * BN);
         for (int kb = 0; kb < num_kb; ++kb) {
           ok = mbar_wait_bounded(smem_u32(&ctl->full[stage]), phase, wctx, kWMmaFull, stage);
           if (!ok) break;
           tc_fence_after_sync();
-          const uint32_t a_addr = tiles_addr + stage * kStageBytes;
+          const uint32_t a_addr = tiles_addr + stage * C::kStageBytes;
           const uint64_t a_desc = p.a_major == 0 ? umma_desc_k_sw128(a_addr) : umma_desc_mn_sw128(a_addr);
           const uint64_t b_desc =
               p.b_major == 0 ? umma_desc_k_sw128(a_addr + kABytes) : umma_desc_mn_sw128(a_addr + kABytes);
@@ -462,7 +472,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             umma_bf16<kG>(d_tmem, a_desc + a_step * k, b_desc + b_step * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
           }
           umma_commit<kG>(smem_u32(&ctl->empty[stage]));
-          if (++stage == kStages) {
+          if (++stage == C::kStages) {
             stage = 0;
             phase ^= 1u;
           }
@@ -525,7 +535,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     int abuf = 0;
     uint32_t aphase = 0;
     const uint32_t tempty_leader = mapa_u32(smem_u32(&ctl->tempty[0]), 0);
-    uint32_t leaf[kTree ? kBN / 64 : 1][16];
+    uint32_t leaf[kTree ? BN / 64 : 1][16];
     for (int u = first_unit<kTree>(pair_id, p.k_slices); u < n_units; u = next_unit<kTree>(u, n_pairs, p.k_slices)) {
       Unit un;
       decode_unit(p, tiles_m, tiles_n, u, un);
@@ -536,8 +546,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       if (!ok) break;
       tc_fence_after_sync();
       const uint32_t trow = tmem_base + (static_cast<uint32_t>(wq * 32) << 16) +
-                            static_cast<uint32_t>(abuf * kBN + wh * (kBN / 2));
-      const int col0 = un.n_blk * kBN + wh * (kBN / 2);
+                            static_cast<uint32_t>(abuf * BN + wh * (BN / 2));
+      const int col0 = un.n_blk * BN + wh * (BN / 2);
       const int slice_global = p.slice_base + un.slice;
       RowCtx rc = {0.f, 0.f, -1};
       if (p.epilogue == kEpiLogitsGrad && row < p.m) {
@@ -548,12 +558,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       uint32_t* wbuf = epi_buf + warp * kEpiBufWords;
       if constexpr (kTree) {
 #pragma unroll
-        for (int g = 0; g < kBN / 64; ++g) {
+        for (int g = 0; g < BN / 64; ++g) {
           uint32_t v[32];
           __syncwarp();
           tmem_ld_32x32(trow + g * 32, v);
           tmem_ld_wait_dep(v);
-          if (tree_group(p.tree_scratch, un.slice, warp, g, lane, v, leaf[g]))
+          if (tree_group<BN>(p.tree_scratch, un.slice, warp, g, lane, v, leaf[g]))
             tree_store(p, v, wbuf, row_w0, col0 + (g & ~1) * 32, lane, g & 1);
         }
       } else {
@@ -561,16 +571,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       tmem_ld_32x32(trow, va);
       tmem_ld_wait_dep(va);
 #pragma unroll
-      for (int g = 0; g < kBN / 64; g += 2) {
+      for (int g = 0; g < BN / 64; g += 2) {
         __syncwarp();
         tmem_ld_32x32(trow + (g + 1) * 32, vb);
         store_group_warp(p, va, wbuf, row_w0, col0 + g * 32, slice_global, rc, lane, 0);
         __syncwarp();
         tmem_ld_wait_dep(vb);
-        if (g + 2 < kBN / 64) tmem_ld_32x32(trow + (g + 2) * 32, va);
+        if (g + 2 < BN / 64) tmem_ld_32x32(trow + (g + 2) * 32, va);
         store_group_warp(p, vb, wbuf, row_w0, col0 + (g + 1) * 32, slice_global, rc, lane, 1);
         __syncwarp();
-        if (g + 2 < kBN / 64) tmem_ld_wait_dep(va);
+        if (g + 2 < BN / 64) tmem_ld_wait_dep(va);
       }
       }
       tc_fence_before_sync();
@@ -580,7 +590,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       if (abuf == 0) aphase ^= 1u;
     }
 
-    if (p.epilogue == kEpiPartialF32) {
+    if (BN == kBN && p.epilogue == kEpiPartialF32) {
       // Publish the partial tiles: every thread makes its own stores visible system-wide, the
       // CTA meets, then the flags of all units this CTA computed are raised (the owners read
       // them in their reduce tails, which start after their own last unit anyway).
@@ -605,7 +615,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         }
       }
     }
-    if (p.epilogue == kEpiPartialF32 && ok && p.out != nullptr) {
+    if (BN == kBN && p.epilogue == kEpiPartialF32 && ok && p.out != nullptr) {
       // ---- reduce-scatter tail (skipped when the caller only wants the partials staged): the rows this rank owns, slices combined by a balanced tree
       const int rblks = p.rows_per_rank / kBM;
       const int items = rblks * tiles_n;
@@ -688,15 +698,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   if (warp == kWarpMma) {
     __syncwarp();
     tc_fence_after_sync();
-    tmem_dealloc<kG>(tmem_base, 512);
+    tmem_dealloc<kG>(tmem_base, 2 * BN);
   }
 }
 
-template <bool kTree>
+template <bool kTree, int BN>
 int max_ctas(int num_sms) {
   static int cached = 0;
   if (cached > 0) return cached;
-  if (cudaFuncSetAttribute(gemm_bf16_kernel<kTree>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
+  if (cudaFuncSetAttribute(gemm_bf16_kernel<kTree, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
     return -1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(num_sms / 2 * 2));
@@ -710,7 +720,7 @@ int max_ctas(int num_sms) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, gemm_bf16_kernel<kTree>, &cfg) != cudaSuccess || clusters <= 0) {
+  if (cudaOccupancyMaxActiveClusters(&clusters, gemm_bf16_kernel<kTree, BN>, &cfg) != cudaSuccess || clusters <= 0) {
     cudaGetLastError();
     clusters = num_sms / 2;
   }
@@ -719,6 +729,13 @@ int max_ctas(int num_sms) {
   cached = n;
   return n;
 }
+
+// Whether a product takes tiles of 128 columns instead of 256: when the narrow tiles still fit the
+// CTA pairs in one round, so that twice as many SMs load and run the epilogue. With more tiles the
+// wide ones win, they load a third less per product. Measured, 512 rows, N = 4096 (32 wide tiles on
+// 74 pairs), wide / narrow in us: slices kept in the kernel 45.5 / 35.3 (K = 4096), 97 / 86 (14336),
+// 162 / 152 (28672); plain 27.3 / 25.6 (4096), 77.0 / 75.7 (14336: both wait for L2).
+inline bool narrow_tiles(int tiles_m, int tiles_n, int pairs) { return tiles_m * tiles_n * 2 <= pairs; }
 
 }  // namespace
 
@@ -730,6 +747,16 @@ int gemm_launch(const void* a, long long lda, const void* b, long long ldb, cons
   if (p.k % 8 != 0 || p.n % 8 != 0 || lda % 8 != 0 || ldb % 8 != 0) return -1;
   if (p.k_slices < 1 || p.k % p.k_slices != 0 || (p.k_slices > 1 && (p.k / p.k_slices) % kBK != 0)) return -2;
   if (p.a_major == 1 && p.m % 8 != 0) return -3;
+  const bool tree = p.epilogue == kEpiTreeBf16;
+  if (tree && (p.k_slices != kTreeSlices || !p.tree_scratch)) return -4;
+  int ctas = tree ? max_ctas<true, kBN>(num_sms) : max_ctas<false, kBN>(num_sms);
+  if (ctas <= 0) return -10;
+  const int tiles_m = (p.m + kBM * kG - 1) / (kBM * kG);
+  const bool narrow = !full_grid && narrow_tiles(tiles_m, (p.n + kBN - 1) / kBN, ctas / kG);
+  if (narrow) ctas = tree ? max_ctas<true, kBN / 2>(num_sms) : max_ctas<false, kBN / 2>(num_sms);
+  if (ctas <= 0) return -10;
+  const int bn = narrow ? kBN / 2 : kBN;
+  const int tiles_n = (p.n + bn - 1) / bn;
   CUtensorMap tm_a, tm_b;
   int rc;
   if (p.a_major == 0)
@@ -738,15 +765,10 @@ int gemm_launch(const void* a, long long lda, const void* b, long long ldb, cons
     rc = make_tmap_2d_16bit_sw128(&tm_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a, p.k, p.m, lda, kBK, 64);
   if (rc != 0) return -20 + rc;
   if (p.b_major == 0)
-    rc = make_tmap_2d_16bit_sw128(&tm_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, b, p.n, p.k, ldb, kBN / kG, kBK);
+    rc = make_tmap_2d_16bit_sw128(&tm_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, b, p.n, p.k, ldb, bn / kG, kBK);
   else
     rc = make_tmap_2d_16bit_sw128(&tm_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, b, p.k, p.n, ldb, kBK, 64);
   if (rc != 0) return -40 + rc;
-  const bool tree = p.epilogue == kEpiTreeBf16;
-  if (tree && (p.k_slices != kTreeSlices || !p.tree_scratch)) return -4;
-  int ctas = tree ? max_ctas<true>(num_sms) : max_ctas<false>(num_sms);
-  if (ctas <= 0) return -10;
-  const int tiles_m = (p.m + kBM * kG - 1) / (kBM * kG), tiles_n = (p.n + kBN - 1) / kBN;
   const int units = tiles_m * tiles_n * (tree ? 1 : p.k_slices);
   if (!full_grid && units * kG < ctas) ctas = units * kG;
   cudaLaunchConfig_t cfg = {};
@@ -761,8 +783,9 @@ int gemm_launch(const void* a, long long lda, const void* b, long long ldb, cons
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const cudaError_t e = tree ? cudaLaunchKernelEx(&cfg, gemm_bf16_kernel<true>, tm_a, tm_b, p)
-                             : cudaLaunchKernelEx(&cfg, gemm_bf16_kernel<false>, tm_a, tm_b, p);
+  auto* kernel = narrow ? (tree ? gemm_bf16_kernel<true, kBN / 2> : gemm_bf16_kernel<false, kBN / 2>)
+                        : (tree ? gemm_bf16_kernel<true, kBN> : gemm_bf16_kernel<false, kBN>);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tm_a, tm_b, p);
   if (e != cudaSuccess) {
     fprintf(stderr, "[kernel_align_b200] gemm launch failed: %s\n", cudaGetErrorString(e));
     return -11;

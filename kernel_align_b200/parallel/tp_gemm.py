@@ -137,10 +137,10 @@ def _tree_pays(m: int, n: int, k: int, num_sms: int) -> bool:
 
     A CTA pair that keeps a tile walks its eight slices one after the other, while staged slices
     spread over all pairs but cost a pass over the partials and the wait for them. Measured on
-    148 SMs, staged / kept in us: 4096 rows, N = 4096: 399 / 184 (K = 4096), 1077 / 884 (28672);
-    32 tiles: 75 / 46 (4096), 110 / 97 (14336), 148 / 162 (28672); 16 tiles: 55 / 41 (4096),
-    62 / 58 (6144), 74 / 95 (14336). A slice round takes about 5.4e-3 us per K column, staging
-    about 20 us plus 1.2 us per tile; the rule compares the two."""
+    148 SMs, staged / kept in us: 4096 rows, N = 4096: 411 / 186 (K = 4096), 1003 / 776 (28672);
+    32 tiles: 77 / 35 (4096), 104 / 86 (14336), 145 / 152 (28672); 16 tiles: 57 / 32 (4096),
+    62 / 48 (6144), 75 / 85 (14336), 95 / 152 (28672). A slice round takes about 5.4e-3 us per
+    K column, staging about 20 us plus 1.2 us per tile; the rule compares the two."""
     pairs = max(1, num_sms // 2)
     tiles = -(-m // 256) * -(-n // 256)
     extra_rounds = -(-tiles // pairs) * 8 - -(-8 * tiles // pairs)

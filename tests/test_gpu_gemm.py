@@ -75,3 +75,21 @@ def test_skinny_gemm_equals_tiled_kernel_bitwise(cuda_device, m, n, k, monkeypat
     assert torch.equal(gemm.gemm_bi(a[:m], w), tiled[:m])
     monkeypatch.setenv("KA_GEMM_SKINNY", "0")
     assert torch.equal(gemm.gemm_bi(a[:m], w), tiled[:m])
+
+
+@pytest.mark.parametrize("n,k", [(8, 64), (136, 200), (1032, 512), (4096, 1024)])
+@pytest.mark.parametrize("trans_a,trans_b,dtype", [(False, False, torch.bfloat16), (False, True, torch.bfloat16),
+                                                   (True, True, torch.float32)])
+def test_narrow_tiles_equal_wide_ones_bitwise(cuda_device, n, k, trans_a, trans_b, dtype):
+    """Small products take tiles of 128 columns: a row must not tell which tiles it was computed in.
+    The tall product has more tiles than the narrow form accepts."""
+    g = torch.Generator(device=cuda_device).manual_seed(n + k)
+    tall = 256 * 80
+    a = torch.randn(tall, k, device=cuda_device, generator=g).to(torch.bfloat16)
+    b = (torch.randn(*((k, n) if trans_b else (n, k)), device=cuda_device, generator=g) * 0.05).to(torch.bfloat16)
+    op = (lambda t: t.t().contiguous()) if trans_a else (lambda t: t)
+    wide = gemm.gemm_bi(op(a), b, trans_a=trans_a, trans_b=trans_b, out_dtype=dtype)
+    for m in (72, 256, 264, 512):
+        narrow = gemm.gemm_bi(op(a[:m]), b, trans_a=trans_a, trans_b=trans_b, out_dtype=dtype)
+        assert torch.equal(narrow, wide[:m]), m
+    gemm.check_status(cuda_device)
