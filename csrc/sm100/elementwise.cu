@@ -336,7 +336,8 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* _
 constexpr int kRmsChunk = 16;
 
 // Fixed-order sums of R values per thread over the CTA (8 warps): lanes by xor-shuffle, then the
-// eight warp sums left to right, the same in every thread.
+// eight warp sums left to right, the same in every thread. One barrier: the caller alternates
+// between two halves of shared memory.
 template <int R>
 __device__ __forceinline__ void block_sum_fixed_multi(float (&v)[R], float (*s_warp)[8]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -354,105 +355,138 @@ __device__ __forceinline__ void block_sum_fixed_multi(float (&v)[R], float (*s_w
     for (int w = 0; w < 8; ++w) t = __fadd_rn(t, s_warp[r][w]);
     v[r] = t;
   }
-  __syncthreads();
 }
 
-// VPT: 16-byte vectors per thread and row (d <= 2048 * VPT); kRows: rows in flight.
+__device__ __forceinline__ void unpack2(uint32_t w, float& lo, float& hi) {
+  lo = __uint_as_float(w << 16);
+  hi = __uint_as_float(w & 0xFFFF0000u);
+}
+
+// VPT: 16-byte vectors per thread and row (d <= 2048 * VPT); kRows: rows in flight. Both sums of a
+// row, x^2 and (dy*w)*x, are taken in one pass (the mean of dy*w*n is the second times inv / d), and
+// the next rows are loaded before the reduction where the registers allow it (VPT <= 2): with a
+// reduction each and the loads behind them, 4096 rows of 4096 took 51 us, 38 us this way.
 template <int VPT, int kRows>
 __global__ void __launch_bounds__(256, 2)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                    const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ d_res,
                    __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part, int rows, int d, float eps) {
-  __shared__ float s_warp[kRows][8];
+  constexpr bool kAhead = VPT <= 2;
+  __shared__ float s_warp[2][2 * kRows][8];
   const int chunk = blockIdx.x;
   const int r0 = chunk * kRmsChunk, r1 = min(rows, r0 + kRmsChunk);
   const int nvec = d / 8;
+  const float inv_d = __fdiv_rn(1.f, static_cast<float>(d));
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   float dw_acc[VPT][8];
+  uint4 wv[VPT];
 #pragma unroll
-  for (int a = 0; a < VPT; ++a)
+  for (int a = 0; a < VPT; ++a) {
+    const int i = threadIdx.x + a * 256;
+    if (kAhead) wv[a] = i < nvec ? reinterpret_cast<const uint4*>(w)[i] : zero;
 #pragma unroll
     for (int j = 0; j < 8; ++j) dw_acc[a][j] = 0.f;
-  const Bf16x8* wp = reinterpret_cast<const Bf16x8*>(w);  // re-read per use: it stays in L1
-  for (int row0 = r0; row0 < r1; row0 += kRows) {
-    Bf16x8 xv[kRows][VPT], gv[kRows][VPT];
+  }
+  auto weight = [&](int a) {                  // kept, or re-read (it stays in L1)
+    const int i = threadIdx.x + a * 256;
+    if constexpr (kAhead) return wv[a];
+    return i < nvec ? reinterpret_cast<const uint4*>(w)[i] : zero;
+  };
+  uint4 xv[kRows][VPT], gv[kRows][VPT];
+  auto load = [&](int row0, uint4 (&xs)[kRows][VPT], uint4 (&gs)[kRows][VPT]) {
 #pragma unroll
-    for (int r = 0; r < kRows; ++r) {
-      const int row = row0 + r;
-#pragma unroll
-      for (int a = 0; a < VPT; ++a) {
-        const int i = threadIdx.x + a * 256;
-        if (row < r1 && i < nvec) {
-          xv[r][a] = reinterpret_cast<const Bf16x8*>(x + static_cast<size_t>(row) * d)[i];
-          gv[r][a] = reinterpret_cast<const Bf16x8*>(dy + static_cast<size_t>(row) * d)[i];
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            xv[r][a].v[j] = __float2bfloat16_rn(0.f);
-            gv[r][a].v[j] = __float2bfloat16_rn(0.f);
-          }
-        }
-      }
-    }
-    float red[kRows];
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) {
-      float ss = 0.f;
-#pragma unroll
-      for (int a = 0; a < VPT; ++a)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float f = __bfloat162float(xv[r][a].v[j]);
-          ss = __fmaf_rn(f, f, ss);
-        }
-      red[r] = ss;
-    }
-    block_sum_fixed_multi<kRows>(red, s_warp);
-    float inv[kRows];
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) {
-      inv[r] = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(__fdiv_rn(red[r], static_cast<float>(d)), eps)));
-      float dot = 0.f;
+    for (int r = 0; r < kRows; ++r)
 #pragma unroll
       for (int a = 0; a < VPT; ++a) {
         const int i = threadIdx.x + a * 256;
-        if (i >= nvec) continue;
-        const Bf16x8 wv = wp[i];
+        const bool in = row0 + r < r1 && i < nvec;
+        xs[r][a] = in ? reinterpret_cast<const uint4*>(x + static_cast<size_t>(row0 + r) * d)[i] : zero;
+        gs[r][a] = in ? reinterpret_cast<const uint4*>(dy + static_cast<size_t>(row0 + r) * d)[i] : zero;
+      }
+  };
+  int flip = 0;
+  if (kAhead) load(r0, xv, gv);
+#pragma unroll 1
+  for (int row0 = r0; row0 < r1; row0 += kRows, flip ^= 1) {
+    uint4 nx[kAhead ? kRows : 1][VPT], ng[kAhead ? kRows : 1][VPT];
+    if constexpr (kAhead)
+      load(row0 + kRows, nx, ng);
+    else
+      load(row0, xv, gv);
+    float red[2 * kRows];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float n = __fmul_rn(__bfloat162float(xv[r][a].v[j]), inv[r]);
-          dot = __fmaf_rn(__fmul_rn(__bfloat162float(gv[r][a].v[j]), __bfloat162float(wv.v[j])), n, dot);
+    for (int r = 0; r < kRows; ++r) {
+      float ss = 0.f, dot = 0.f;
+#pragma unroll
+      for (int a = 0; a < VPT; ++a) {
+        const uint4 wa = weight(a);
+        const uint32_t* xw = reinterpret_cast<const uint32_t*>(&xv[r][a]);
+        const uint32_t* gw = reinterpret_cast<const uint32_t*>(&gv[r][a]);
+        const uint32_t* ww = reinterpret_cast<const uint32_t*>(&wa);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float x0, x1, g0, g1, w0, w1;
+          unpack2(xw[j], x0, x1);
+          unpack2(gw[j], g0, g1);
+          unpack2(ww[j], w0, w1);
+          ss = __fmaf_rn(x0, x0, ss);
+          ss = __fmaf_rn(x1, x1, ss);
+          dot = __fmaf_rn(__fmul_rn(g0, w0), x0, dot);
+          dot = __fmaf_rn(__fmul_rn(g1, w1), x1, dot);
         }
       }
-      red[r] = dot;
+      red[2 * r] = ss;
+      red[2 * r + 1] = dot;
     }
-    block_sum_fixed_multi<kRows>(red, s_warp);
+    block_sum_fixed_multi<2 * kRows>(red, s_warp[flip]);
 #pragma unroll
     for (int r = 0; r < kRows; ++r) {
       const int row = row0 + r;
       if (row >= r1) break;  // uniform over the CTA
-      const float mean_dot = __fdiv_rn(red[r], static_cast<float>(d));
+      const float inv = __fdiv_rn(1.f, __fsqrt_rn(__fadd_rn(__fdiv_rn(red[2 * r], static_cast<float>(d)), eps)));
+      const float mean_dot = __fmul_rn(__fmul_rn(red[2 * r + 1], inv), inv_d);
 #pragma unroll
       for (int a = 0; a < VPT; ++a) {
         const int i = threadIdx.x + a * 256;
         if (i >= nvec) continue;
-        const Bf16x8 wv = wp[i];
-        Bf16x8 o;
+        const uint32_t* xw = reinterpret_cast<const uint32_t*>(&xv[r][a]);
+        const uint32_t* gw = reinterpret_cast<const uint32_t*>(&gv[r][a]);
+        const uint4 wa = weight(a);
+        const uint32_t* ww = reinterpret_cast<const uint32_t*>(&wa);
+        uint4 rr = zero;
+        if (d_res) rr = reinterpret_cast<const uint4*>(d_res + static_cast<size_t>(row) * d)[i];
+        const uint32_t* rw = reinterpret_cast<const uint32_t*>(&rr);
+        uint4 o;
+        uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float n = __fmul_rn(__bfloat162float(xv[r][a].v[j]), inv[r]);
-          const float g = __bfloat162float(gv[r][a].v[j]);
-          const float gw = __fmul_rn(g, __bfloat162float(wv.v[j]));
-          o.v[j] = __float2bfloat16_rn(__fmul_rn(inv[r], __fsub_rn(gw, __fmul_rn(n, mean_dot))));
-          dw_acc[a][j] = __fmaf_rn(g, n, dw_acc[a][j]);  // rows enter in increasing order
-        }
-        if (d_res) {
-          const Bf16x8 rr = reinterpret_cast<const Bf16x8*>(d_res + static_cast<size_t>(row) * d)[i];
+        for (int j = 0; j < 4; ++j) {
+          float xf[2], gf[2], wf[2], rf[2];
+          unpack2(xw[j], xf[0], xf[1]);
+          unpack2(gw[j], gf[0], gf[1]);
+          unpack2(ww[j], wf[0], wf[1]);
+          unpack2(rw[j], rf[0], rf[1]);
+          __nv_bfloat16 ob[2];
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            o.v[j] = __float2bfloat16_rn(__fadd_rn(__bfloat162float(o.v[j]), __bfloat162float(rr.v[j])));
+          for (int e = 0; e < 2; ++e) {
+            const float n = __fmul_rn(xf[e], inv);
+            ob[e] = __float2bfloat16_rn(__fmul_rn(inv, __fmaf_rn(-n, mean_dot, __fmul_rn(gf[e], wf[e]))));
+            dw_acc[a][2 * j + e] = __fmaf_rn(gf[e], n, dw_acc[a][2 * j + e]);  // rows enter in increasing order
+            if (d_res) ob[e] = __float2bfloat16_rn(__fadd_rn(__bfloat162float(ob[e]), rf[e]));
+          }
+          ow[j] = static_cast<uint32_t>(__bfloat16_as_ushort(ob[0])) |
+                  (static_cast<uint32_t>(__bfloat16_as_ushort(ob[1])) << 16);
         }
-        reinterpret_cast<Bf16x8*>(dx + static_cast<size_t>(row) * d)[i] = o;
+        reinterpret_cast<uint4*>(dx + static_cast<size_t>(row) * d)[i] = o;
       }
+    }
+    if constexpr (kAhead) {
+#pragma unroll
+      for (int r = 0; r < kRows; ++r)
+#pragma unroll
+        for (int a = 0; a < VPT; ++a) {
+          xv[r][a] = nx[r][a];
+          gv[r][a] = ng[r][a];
+        }
     }
   }
 #pragma unroll
@@ -594,9 +628,9 @@ int ka_rmsnorm_bwd(const void* x, const void* w, const void* dy, const void* d_r
   __nv_bfloat16* ob = static_cast<__nv_bfloat16*>(dx);
   const int vpt = (d / 8 + 255) / 256;
   if (vpt <= 1)
-    rmsnorm_bwd_kernel<1, 4><<<chunks, 256, 0, st>>>(xb, wb, gb, rb, ob, dw_part, rows, d, eps);
+    rmsnorm_bwd_kernel<1, 2><<<chunks, 256, 0, st>>>(xb, wb, gb, rb, ob, dw_part, rows, d, eps);
   else if (vpt == 2)
-    rmsnorm_bwd_kernel<2, 2><<<chunks, 256, 0, st>>>(xb, wb, gb, rb, ob, dw_part, rows, d, eps);
+    rmsnorm_bwd_kernel<2, 1><<<chunks, 256, 0, st>>>(xb, wb, gb, rb, ob, dw_part, rows, d, eps);
   else
     rmsnorm_bwd_kernel<4, 1><<<chunks, 256, 0, st>>>(xb, wb, gb, rb, ob, dw_part, rows, d, eps);
   rmsnorm_dw_kernel<<<(d + 31) / 32, 256, 0, st>>>(dw_part, static_cast<__nv_bfloat16*>(dw), chunks, d);
