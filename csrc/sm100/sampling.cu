@@ -17,9 +17,9 @@
 //   sample_topk_kernel     top_k in [1, 1024] (greedy = top_k 1), optional top_p
 //   sample_topk_held_kernel  the same for aligned 16-bit rows that 1, 2 or 4 CTAs hold in registers
 //                          (a cluster; candidates exchanged through distributed shared memory)
-//   sample_general_kernel  no top_k (or k > 1024), optional top_p: threshold search by radix
-//                          descent on (count, mass) histograms; for bf16 rows in one step on a
-//                          histogram of counts per key (the mass of a key is a function of the key)
+//   sample_general_kernel  no top_k (or k > 1024), optional top_p: 16-bit rows by one histogram of
+//                          counts per key (sample_row16), fp32 rows and the few 16-bit rows that
+//                          does not take by radix descent on (count, mass) histograms
 #include <cstdint>
 #include <cstdlib>
 #include <type_traits>
@@ -620,14 +620,11 @@ sample_topk_held_kernel(const T* __restrict__ logits, long long row_stride, int 
 // The kept set is a prefix of the order (key desc, id asc): the first n* elements with
 //   n* = min(k, smallest n with mass(first n) > top_p * Z_k)      (Z_k = mass of the first k)
 // The prefix is located by radix descent over the key bits (11, 11, 10) with exact integer
-// histograms of element counts and fixed-point masses (fp32 and fp16 rows), or at full key
-// resolution from a histogram of counts per key (bf16 rows, descend16 below); ties at the
-// threshold key are cut in token-id order. The draw inverts the CDF over the kept set in
-// token-id order: every thread owns a contiguous piece of the row, two block scans give it the
-// ties and the kept mass before its piece.
-// Measured, bf16 [G, 128256] ~ N(0, 2), T = 0.7, top_p = 0.9 without top_k: 108 us at G = 64 and
-// 211 us at G = 256 (two waves of one CTA per SM); with the three-level descent and a block scan
-// per 8192 elements in the draw it took about 550 us.
+// histograms of element counts and fixed-point masses (fp32 rows, and fp16 rows that sample_row16
+// hands back), or at full key resolution from two half histograms of counts per key (such bf16
+// rows, descend16 below); ties at the threshold key are cut in token-id order. The draw inverts
+// the CDF over the kept set in token-id order: every thread owns a contiguous piece of the row,
+// two block scans give it the ties and the kept mass before its piece.
 // ------------------------------------------------------------------------------------------
 constexpr int kBins = 2048;
 
