@@ -1375,17 +1375,23 @@ int launch_sampling(const void* logits, long long row_stride, int rows, int v, c
       if (e != cudaSuccess) return -10;
       configured = true;
     }
-    // Aligned rows that 1, 2 or 4 CTAs can keep in registers take the kernel that reads them once;
-    // it was faster at every number of rows (see its comment). KA_SAMPLE_CLUSTER = 1 keeps the
-    // other one, 2 and 4 ask for that many CTAs per row.
+    // Aligned rows that 1, 2 or 4 CTAs can keep in registers take the kernel that reads them once,
+    // as long as all CTAs (one per SM) are resident at once: bf16 [G, 128256], k = 50, L2 flushed:
+    // 22.6 us against 28.7 us at G = 64, but 41 against 33 us at G = 128 and 73 against 50 us at
+    // G = 256, where it comes in waves and the other kernel, two CTAs per SM, in one.
+    // KA_SAMPLE_CLUSTER = 1 keeps the other one, 2 and 4 ask for that many CTAs per row.
     if constexpr (Elem<T>::kPacked) {
       const bool aligned = (reinterpret_cast<uintptr_t>(lp) & 15u) == 0 && (row_stride * sizeof(T)) % 16 == 0;
       int cluster = v <= kHeldElems ? 1 : (v <= 2 * kHeldElems ? 2 : (v <= 4 * kHeldElems ? 4 : 0));
-      if (const char* env = getenv("KA_SAMPLE_CLUSTER")) {
-        const int c = atoi(env);
-        if (c == 1) cluster = 0;
-        if ((c == 2 || c == 4) && cluster != 0 && c > cluster) cluster = c;
-      }
+      int dev = 0, sms = 0;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      const char* env = getenv("KA_SAMPLE_CLUSTER");
+      const int asked = env ? atoi(env) : 0;
+      if (asked == 2 || asked == 4)
+        cluster = cluster != 0 && asked > cluster ? asked : cluster;
+      else if (asked == 1 || static_cast<long long>(rows) * cluster > sms)
+        cluster = 0;
       if (cluster > 0 && aligned) {
         const int smem = static_cast<int>(sizeof(TopkSmem) + sizeof(ClusterXchg));
         auto* kernel = cluster == 1 ? sample_topk_held_kernel<T, 1>
