@@ -135,7 +135,10 @@ struct CtlDq {
   uint64_t kv_full[2], kv_empty[2];
   uint64_t s_full[2];                // S ready in its TMEM buffer
   uint64_t dp_full, dp_read;         // dP ready / read into registers (count: softmax warps)
-  uint64_t ds_full;                  // dS written over S (count: softmax warps)
+  // dS written over S (count: softmax warps), one per S buffer: S(j + 1) and dP(j + 1) are issued before
+  // the wait for dS(j), so the warps may finish tile j + 1 before that wait looks. With a single barrier
+  // they would have passed two phases by then, and the wait for a parity would never end.
+  uint64_t ds_full[2];
   uint64_t acc_full;                 // final dQ ready
   uint32_t tmem_base;
   int abort_flag;
@@ -170,10 +173,10 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       mbar_init(smem_u32(&ctl->kv_full[s]), 1);
       mbar_init(smem_u32(&ctl->kv_empty[s]), 1);
       mbar_init(smem_u32(&ctl->s_full[s]), 1);
+      mbar_init(smem_u32(&ctl->ds_full[s]), kSoftThreads / 32);
     }
     mbar_init(smem_u32(&ctl->dp_full), 1);
     mbar_init(smem_u32(&ctl->dp_read), kSoftThreads / 32);
-    mbar_init(smem_u32(&ctl->ds_full), kSoftThreads / 32);
     mbar_init(smem_u32(&ctl->acc_full), 1);
     ctl->abort_flag = 0;
     fence_mbar_init_cluster();
@@ -250,7 +253,7 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
           tc_fence_after_sync();
           issue_dp(j + 1);
         }
-        ok = mbar_wait_bounded(smem_u32(&ctl->ds_full), j & 1, wctx, 44, j);
+        ok = mbar_wait_bounded(smem_u32(&ctl->ds_full[j & 1]), (j >> 1) & 1, wctx, 44, j);
         if (!ok) break;
         tc_fence_after_sync();
         const uint64_t dk = d_ring_mn + (j & 1) * kStage;
@@ -324,7 +327,7 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       tmem_st_wait();
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&ctl->ds_full));
+      if (lane == 0) mbar_arrive(smem_u32(&ctl->ds_full[j & 1]));
     }
     if (ok && n_kv > 0) {
       const bool mine = mbar_wait_bounded(smem_u32(&ctl->acc_full), 0, wctx, 46, 0);
