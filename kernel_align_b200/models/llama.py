@@ -103,7 +103,7 @@ class DecoderLayer(nn.Module):
         tokens = batch * seq_len
         h, x_local = rmsnorm_fork_fn(x_local, self.norm1, cfg.rms_eps)
         qkv = column_parallel_linear(h, self.wqkv, tp)                       # [M_pad, (hq + 2 hkv) * hd]
-        q, k, v = qkv_rope_fn(qkv, positions, cos, sin, self.hq, self.hkv, hd)
+        q, k, v = qkv_rope_fn(qkv, positions, cos, sin, self.hq, self.hkv, hd, tokens)
         q = q.view(batch, seq_len, self.hq, hd)
         k, v = k.view(batch, seq_len, self.hkv, hd), v.view(batch, seq_len, self.hkv, hd)
         a = attention_fn(q, k, v, causal=True).reshape(tokens, self.hq * hd)

@@ -260,11 +260,16 @@ class _QkvRopeFn(torch.autograd.Function):
 
 
 def qkv_rope_fn(qkv: torch.Tensor, positions: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, hq: int, hkv: int,
-                head_dim: int):
-    """Cut a fused projection ``[rows, (hq + 2 hkv) * head_dim]`` into ``q``, ``k`` (rotated at
-    ``positions [tokens]``) and ``v``, each ``[tokens, heads, head_dim]``; rows past ``tokens`` are
-    padding. Differentiable; the bits of slicing and :func:`rope_fn`, in one launch per direction."""
-    tokens = positions.numel()
+                head_dim: int, tokens: Optional[int] = None):
+    """Cut a fused projection ``[rows, (hq + 2 hkv) * head_dim]`` into ``q``, ``k`` (rotated at the
+    first ``tokens`` of ``positions``; all of them by default) and ``v``, each
+    ``[tokens, heads, head_dim]``; rows past ``tokens`` are padding. Differentiable; the bits of
+    slicing and :func:`rope_fn`, in one launch per direction."""
+    positions = positions.reshape(-1)
+    tokens = positions.numel() if tokens is None else int(tokens)
+    if positions.numel() < tokens:
+        raise ValueError(f"{positions.numel()} positions for {tokens} tokens")
+    positions = positions[:tokens]
     aligned = qkv.dim() == 2 and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0
     if qkv.device.type == "cuda" and head_dim == 128 and qkv.dtype == torch.bfloat16 and aligned and 0 < tokens:
         return _QkvRopeFn.apply(qkv, positions, cos, sin, hq, hkv, tokens)

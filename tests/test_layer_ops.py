@@ -117,3 +117,23 @@ def test_rmsnorm_fork_adds_the_two_gradients(dev, rows, d):
     xi = x.clone().requires_grad_()
     rmsnorm_fork_fn(xi, w)[1].backward(dr)
     assert torch.equal(xi.grad, dr)
+
+
+@pytest.mark.parametrize("dev", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def test_decoder_layer_takes_positions_of_the_padded_rows_too(dev):
+    from kernel_align_b200.models.llama import DecoderLayer, LlamaConfig
+    from kernel_align_b200.parallel.tp_gemm import TPContext
+
+    cfg = LlamaConfig(vocab_size=512, hidden=256, n_layers=1, n_heads=4, n_kv_heads=2, head_dim=128, ffn=512, max_pos=256)
+    layer = DecoderLayer(cfg, TPContext(device=torch.device(dev)), 1, torch.device(dev))
+    cos, sin = rope_tables(cfg.max_pos, cfg.head_dim, cfg.rope_theta, device=dev)
+    x = torch.randn(128, cfg.hidden, generator=torch.Generator().manual_seed(4)).bfloat16().to(dev)
+    pos = torch.arange(100, device=dev)
+    outs = []
+    for p in (pos, torch.cat([pos, pos.new_zeros(28)]), torch.cat([pos, pos.new_zeros(28)]).view(1, 128)):
+        xi = x.clone().requires_grad_()
+        y = layer(xi, 1, 100, p, cos, sin)
+        outs.append((y, torch.autograd.grad(y.float().square().sum(), xi)[0]))
+    assert all(torch.equal(a, b) for o in outs[1:] for a, b in zip(o, outs[0]))
+    with pytest.raises(ValueError):
+        layer(x, 1, 100, pos[:99], cos, sin)
