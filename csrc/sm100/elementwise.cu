@@ -527,6 +527,12 @@ int grid_for(long long work_items, int threads, int num_sms) {
   return g < 1 ? 1 : static_cast<int>(g);
 }
 
+// Whether every pointer is 16-byte aligned (null is).
+template <typename... P>
+bool aligned16(P... p) {
+  return ((reinterpret_cast<uintptr_t>(p) | ...) & 15u) == 0;
+}
+
 }  // namespace
 }  // namespace ka
 
@@ -557,7 +563,7 @@ int ka_rope(void* x, long long token_stride, const long long* positions, const f
   using namespace ka;
   if (tokens <= 0) return 0;
   if (hd % 2 != 0) return -1;
-  if ((hd / 2) % 8 == 0 && token_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
+  if ((hd / 2) % 8 == 0 && token_stride % 8 == 0 && aligned16(x, cos_t, sin_t)) {
     const long long groups = static_cast<long long>(tokens) * heads * (hd / 16);
     rope_vec8_kernel<<<grid_for(groups, 256, num_sms), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<__nv_bfloat16*>(x), token_stride, positions, cos_t, sin_t, tokens, heads, hd);
@@ -569,12 +575,16 @@ int ka_rope(void* x, long long token_stride, const long long* positions, const f
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
-// See qkv_rope_kernel. head_dim is 128, qkv rows 16-byte aligned, positions [tokens] on the device.
-int ka_qkv_rope(void* qkv, long long qkv_stride, const long long* positions, const float* cos_t, const float* sin_t,
-                void* q, void* k, void* v, int rows, int tokens, int hq, int hkv, int backward, void* stream) {
+// See qkv_rope_kernel. head_dim is 128, qkv [rows, width] with width = (hq + 2 hkv) * 128, positions [tokens] on
+// the device; qkv and the tables 16-byte aligned.
+int ka_qkv_rope(void* qkv, long long qkv_stride, int width, const long long* positions, const float* cos_t,
+                const float* sin_t, void* q, void* k, void* v, int rows, int tokens, int hq, int hkv, int backward,
+                void* stream) {
   using namespace ka;
   if (rows <= 0) return 0;
-  if (qkv_stride % 8 != 0 || (reinterpret_cast<uintptr_t>(qkv) & 15u) != 0 || tokens > rows) return -1;
+  if (hq < 0 || hkv < 0 || width != (hq + 2 * hkv) * 128 || qkv_stride < width || qkv_stride % 8 != 0 || tokens > rows)
+    return -1;
+  if (!aligned16(qkv, cos_t, sin_t)) return -2;
   const dim3 grid(static_cast<unsigned>((rows + kQkvTokens - 1) / kQkvTokens),
                   static_cast<unsigned>((hq + 2 * hkv + 31) / 32));
   auto* kernel = backward ? qkv_rope_kernel<true> : qkv_rope_kernel<false>;

@@ -234,11 +234,11 @@ def rope_fn(x: torch.Tensor, positions: torch.Tensor, cos: torch.Tensor, sin: to
 def _qkv_rope_launch(qkv, positions, cos, sin, q, k, v, tokens, backward):
     fn = _native.cuda().ka_qkv_rope
     fn.restype = c_int
-    fn.argtypes = [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
-                   c_int, c_int, c_void_p]
-    _check(fn(qkv.data_ptr(), qkv.stride(0), positions.data_ptr(), cos.data_ptr(), sin.data_ptr(), q.data_ptr(),
-              k.data_ptr(), v.data_ptr(), qkv.shape[0], tokens, q.shape[1], k.shape[1], int(backward), _stream(qkv)),
-           "ka_qkv_rope")
+    fn.argtypes = [c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                   c_int, c_int, c_int, c_void_p]
+    _check(fn(qkv.data_ptr(), qkv.stride(0), qkv.shape[1], positions.data_ptr(), cos.data_ptr(), sin.data_ptr(),
+              q.data_ptr(), k.data_ptr(), v.data_ptr(), qkv.shape[0], tokens, q.shape[1], k.shape[1], int(backward),
+              _stream(qkv)), "ka_qkv_rope")
 
 
 class _QkvRopeFn(torch.autograd.Function):
@@ -259,6 +259,17 @@ class _QkvRopeFn(torch.autograd.Function):
         return dqkv, None, None, None, None, None, None
 
 
+def _qkv_rope_takes(qkv, positions, cos, sin, tokens, head_dim) -> bool:
+    """Whether the fused kernel takes these tensors: it reads everything 16 bytes at a time."""
+    def table(t):
+        return (t.device == qkv.device and t.dtype == torch.float32 and t.dim() == 2 and t.shape[1] == head_dim // 2
+                and t.is_contiguous() and t.data_ptr() % 16 == 0)
+
+    return (qkv.device.type == "cuda" and qkv.dtype == torch.bfloat16 and head_dim == 128 and tokens > 0
+            and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and qkv.stride(0) >= qkv.shape[1]
+            and qkv.data_ptr() % 16 == 0 and positions.device == qkv.device and table(cos) and table(sin))
+
+
 def qkv_rope_fn(qkv: torch.Tensor, positions: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, hq: int, hkv: int,
                 head_dim: int, tokens: Optional[int] = None):
     """Cut a fused projection ``[rows, (hq + 2 hkv) * head_dim]`` into ``q``, ``k`` (rotated at the
@@ -269,9 +280,10 @@ def qkv_rope_fn(qkv: torch.Tensor, positions: torch.Tensor, cos: torch.Tensor, s
     tokens = positions.numel() if tokens is None else int(tokens)
     if positions.numel() < tokens:
         raise ValueError(f"{positions.numel()} positions for {tokens} tokens")
+    if qkv.dim() != 2 or qkv.shape[1] != (hq + 2 * hkv) * head_dim or qkv.shape[0] < tokens:
+        raise ValueError(f"a projection of {tuple(qkv.shape)} for {tokens} tokens of {hq} + 2 * {hkv} heads of {head_dim}")
     positions = positions[:tokens]
-    aligned = qkv.dim() == 2 and qkv.stride(1) == 1 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0
-    if qkv.device.type == "cuda" and head_dim == 128 and qkv.dtype == torch.bfloat16 and aligned and 0 < tokens:
+    if _qkv_rope_takes(qkv, positions, cos, sin, tokens, head_dim):
         return _QkvRopeFn.apply(qkv, positions, cos, sin, hq, hkv, tokens)
     q = qkv[:tokens, : hq * head_dim].reshape(tokens, hq, head_dim)
     k = qkv[:tokens, hq * head_dim:(hq + hkv) * head_dim].reshape(tokens, hkv, head_dim)

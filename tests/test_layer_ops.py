@@ -137,3 +137,73 @@ def test_decoder_layer_takes_positions_of_the_padded_rows_too(dev):
     assert all(torch.equal(a, b) for o in outs[1:] for a, b in zip(o, outs[0]))
     with pytest.raises(ValueError):
         layer(x, 1, 100, pos[:99], cos, sin)
+
+
+class _OnGpu:
+    """A CPU tensor that says it is on a GPU: for rules that only look at shapes, strides and addresses."""
+
+    def __init__(self, t, device="cuda:0"):
+        self.t, self.device = t, torch.device(device)
+
+    def __getattr__(self, name):
+        return getattr(self.t, name)
+
+
+def test_qkv_rope_takes_only_what_its_kernel_can_read():
+    from kernel_align_b200.ops.layer_ops import _qkv_rope_takes
+
+    width, pos = 8 * 128, torch.arange(6)
+    x = torch.zeros(9, width, dtype=torch.bfloat16)
+    cos, sin = rope_tables(16, 128)
+    odd = torch.zeros(16 * 64 + 1)[1:].view(16, 64)          # contiguous, but at an odd offset
+
+    def takes(x=x, pos=pos, cos=cos, sin=sin, tokens=6, head_dim=128, where=(None,) * 4):
+        x, pos, cos, sin = (_OnGpu(t, at or "cuda:0") for t, at in zip((x, pos, cos, sin), where))
+        return _qkv_rope_takes(x, pos, cos, sin, tokens, head_dim)
+
+    assert takes()
+    assert takes(x=torch.zeros(9, 2 * width, dtype=torch.bfloat16)[:, width:])          # rows of a wider matrix
+    assert takes(x=x[2:])
+    refused = [dict(x=x.half()), dict(x=torch.zeros(width, 9, dtype=torch.bfloat16).t()), dict(tokens=0),
+               dict(x=torch.zeros(9, width + 4, dtype=torch.bfloat16)[:, :width]),      # rows 8-byte aligned
+               dict(x=torch.zeros(9 * width + 1, dtype=torch.bfloat16)[1:].view(9, width)),
+               dict(x=torch.zeros(1, width, dtype=torch.bfloat16).expand(9, width)), dict(where=("cpu", None, None, None)),
+               dict(cos=cos.double()), dict(sin=sin.bfloat16()), dict(cos=torch.zeros(64, 16).t()), dict(cos=odd),
+               dict(sin=odd), dict(cos=cos[:, :32].contiguous()), dict(cos=cos.view(-1)), dict(head_dim=64),
+               dict(where=(None, None, None, "cpu")), dict(where=(None, None, "cuda:1", None)),
+               dict(where=(None, "cpu", None, None))]
+    for form in refused:
+        assert not takes(**form), form
+
+
+@pytest.mark.parametrize("dev", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def test_qkv_rope_refuses_a_projection_of_another_width(dev):
+    from kernel_align_b200.ops.layer_ops import qkv_rope_fn
+
+    cos, sin = rope_tables(16, 128, device=dev)
+    pos = torch.arange(6, device=dev)
+    for rows, heads in ((6, 7), (6, 9), (5, 8)):             # too narrow, too wide, too few rows
+        with pytest.raises(ValueError):
+            qkv_rope_fn(torch.zeros(rows, heads * 128, dtype=torch.bfloat16, device=dev), pos, cos, sin, 4, 2, 128)
+    # tables the fused kernel does not read take the other route
+    x = torch.randn(6, 8 * 128, generator=torch.Generator().manual_seed(0)).bfloat16().to(dev)
+    odd = torch.cat([cos.new_zeros(2), cos.reshape(-1)])[2:].view(16, 64)
+    assert all(torch.equal(a, b) for a, b in zip(qkv_rope_fn(x, pos, cos, sin, 4, 2, 128),
+                                                 qkv_rope_fn(x, pos, odd, sin, 4, 2, 128)))
+
+
+def test_qkv_rope_entry_checks_its_arguments(monkeypatch):
+    """The native entry refuses before it launches anything, so this needs no GPU."""
+    from kernel_align_b200.ops import layer_ops
+
+    monkeypatch.setattr(layer_ops, "_stream", lambda t: None)
+    x = torch.zeros(6 * 8 * 128 + 8, dtype=torch.bfloat16)[:6 * 8 * 128].view(6, 8 * 128)
+    cos, sin = rope_tables(16, 128)
+    q, k, v = (torch.zeros(6, h, 128, dtype=torch.bfloat16) for h in (4, 2, 2))
+    pos = torch.arange(6)
+    for bad in (dict(qkv=x[:, :7 * 128]), dict(qkv=x[:5]), dict(cos=cos.view(-1)[1:]), dict(sin=sin.view(-1)[1:]),
+                dict(q=q[:, :3])):
+        args = dict(dict(qkv=x, positions=pos, cos=cos, sin=sin, q=q, k=k, v=v, tokens=6), **bad)
+        for backward in (False, True):
+            with pytest.raises(RuntimeError, match=r"ka_qkv_rope failed \(-[12]\)"):
+                layer_ops._qkv_rope_launch(**args, backward=backward)
