@@ -659,6 +659,8 @@ extern "C" int ka_attention_bwd(const void* q, long long q_stride, const void* k
   using namespace ka;
   if (batch <= 0 || seq_len <= 0) return 0;
   if (head_dim != kD || hq % hkv != 0) return -1;
+  // q, k, v and d_o are checked with their tensor maps; o is read by the delta kernel alone
+  if ((reinterpret_cast<uintptr_t>(o) & 15u) != 0 || o_stride % 8 != 0) return -2;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   constexpr int kSmemDq = 6 * kTileBytes + 256;
   constexpr int kSmemDkv = 7 * kTileBytes + 2304;

@@ -576,7 +576,7 @@ int ka_rope(void* x, long long token_stride, const long long* positions, const f
 }
 
 // See qkv_rope_kernel. head_dim is 128, qkv [rows, width] with width = (hq + 2 hkv) * 128, positions [tokens] on
-// the device; qkv and the tables 16-byte aligned.
+// the device; everything but the positions 16-byte aligned.
 int ka_qkv_rope(void* qkv, long long qkv_stride, int width, const long long* positions, const float* cos_t,
                 const float* sin_t, void* q, void* k, void* v, int rows, int tokens, int hq, int hkv, int backward,
                 void* stream) {
@@ -584,7 +584,7 @@ int ka_qkv_rope(void* qkv, long long qkv_stride, int width, const long long* pos
   if (rows <= 0) return 0;
   if (hq < 0 || hkv < 0 || width != (hq + 2 * hkv) * 128 || qkv_stride < width || qkv_stride % 8 != 0 || tokens > rows)
     return -1;
-  if (!aligned16(qkv, cos_t, sin_t)) return -2;
+  if (!aligned16(qkv, cos_t, sin_t, q, k, v)) return -2;
   const dim3 grid(static_cast<unsigned>((rows + kQkvTokens - 1) / kQkvTokens),
                   static_cast<unsigned>((hq + 2 * hkv + 31) / 32));
   auto* kernel = backward ? qkv_rope_kernel<true> : qkv_rope_kernel<false>;
@@ -623,12 +623,13 @@ int ka_swiglu_bwd(const void* gate, const void* up, long long in_stride, const v
 int ka_rmsnorm_bwd_chunk() { return ka::kRmsChunk; }
 
 // x, dy: [rows, d] bf16; d_res: null or [rows, d], added to dx; dx: [rows, d] bf16; dw: [d] bf16; dw_part: scratch of
-// ceil(rows / ka_rmsnorm_bwd_chunk()) * d floats. d % 8 == 0 and d <= 8192.
+// ceil(rows / ka_rmsnorm_bwd_chunk()) * d floats. d % 8 == 0 and d <= 8192; all but dw 16-byte aligned.
 int ka_rmsnorm_bwd(const void* x, const void* w, const void* dy, const void* d_res, void* dx, void* dw, float* dw_part,
                    int rows, int d, float eps, void* stream) {
   using namespace ka;
   if (rows <= 0) return 0;
   if (d % 8 != 0 || d > 8192) return -1;
+  if (!aligned16(x, w, dy, d_res, dx, dw_part)) return -2;
   const int chunks = (rows + kRmsChunk - 1) / kRmsChunk;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);

@@ -828,6 +828,7 @@ extern "C" int ka_gemm_tree8(const void* a, long long lda, const void* b, long l
                              const void* residual, void* scratch, int m, int n, int k, int* status, int num_sms,
                              unsigned long long timeout_ns, void* stream) {
   if (n % 8 != 0) return -51;
+  if (((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(residual)) & 15u) != 0) return -54;
   ka::GemmParams p = {};
   p.m = m;
   p.n = n;

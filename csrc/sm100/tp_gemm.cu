@@ -56,6 +56,7 @@ int ka_gemm_reduce_scatter(const void* a, long long lda, const void* b, long lon
                            int* status, int num_sms, unsigned long long timeout_ns, void* stream) {
   if (!(world == 1 || world == 2 || world == 4 || world == 8) || rank < 0 || rank >= world) return -50;
   if (n % 8 != 0) return -51;
+  if (((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(residual)) & 15u) != 0) return -54;
   ka::GemmParams p = {};
   p.m = m;
   p.n = n;

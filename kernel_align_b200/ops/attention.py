@@ -85,6 +85,8 @@ def attention_backward(q, k, v, out, d_out, lse, *, causal: bool = True, scale: 
         return t if ok else t.contiguous()
 
     q, k, v, out, d_out = tok(q), tok(k), tok(v), tok(out), tok(d_out)
+    if out.data_ptr() % 16:     # contiguous at an odd offset: no tensor map looks at it, and it is read 16 bytes at a time
+        out = out.clone()
     dq = torch.empty(b, l, hq, d, dtype=torch.bfloat16, device=q.device)
     dk = torch.empty(b, l, hkv, d, dtype=torch.bfloat16, device=q.device)
     dv = torch.empty(b, l, hkv, d, dtype=torch.bfloat16, device=q.device)

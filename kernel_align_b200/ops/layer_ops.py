@@ -25,6 +25,13 @@ def _stream(t: torch.Tensor) -> int:
     return torch.cuda.current_stream(t.device).cuda_stream
 
 
+def _packed(t: torch.Tensor) -> torch.Tensor:
+    """``t`` contiguous and 16-byte aligned. Gradients come from anywhere: a piece of a packed buffer
+    is contiguous, but may start at any element, and the kernels read 16 bytes at a time."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 def _check(rc: int, name: str) -> None:
     if rc != 0:
         raise RuntimeError(f"{name} failed ({rc})")
@@ -143,8 +150,8 @@ def swiglu(gate_up: torch.Tensor, up: Optional[torch.Tensor] = None) -> torch.Te
 def _rmsnorm_backward(x, weight, eps, dy, d_res):
     """``(dx, dw)`` of RMSNorm; ``d_res`` (or None) is added to the rounded ``dx``."""
     d = x.shape[-1]
-    x2 = x.reshape(-1, d).contiguous()
-    dy2 = dy.reshape(-1, d).contiguous()
+    x2 = _packed(x.reshape(-1, d))
+    dy2 = _packed(dy.reshape(-1, d))
     rows = x2.shape[0]
     if x.device.type != "cuda":
         xf, gf, wf = x2.float(), dy2.float(), weight.float()
@@ -154,19 +161,23 @@ def _rmsnorm_backward(x, weight, eps, dy, d_res):
         dw = (gf * xf * r).sum(0)
         dx = dx.to(x.dtype).reshape(x.shape)
         return (dx if d_res is None else dx + d_res), dw.to(weight.dtype)
-    res2 = d_res.reshape(-1, d).contiguous() if d_res is not None else None
+    return _rmsnorm_backward_launch(x2, _packed(weight), eps, dy2,
+                                    _packed(d_res.reshape(-1, d)) if d_res is not None else None, x.shape)
+
+
+def _rmsnorm_backward_launch(x2, weight, eps, dy2, res2, shape):
+    rows, d = x2.shape
     dx = torch.empty_like(x2)
     dw = torch.empty_like(weight)
     chunk = int(_native.cuda().ka_rmsnorm_bwd_chunk())
-    part = torch.empty((rows + chunk - 1) // chunk, d, dtype=torch.float32, device=x.device)
+    part = torch.empty((rows + chunk - 1) // chunk, d, dtype=torch.float32, device=x2.device)
     fn = _native.cuda().ka_rmsnorm_bwd
     fn.restype = c_int
     fn.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float,
                    c_void_p]
-    _check(fn(x2.data_ptr(), weight.contiguous().data_ptr(), dy2.data_ptr(),
-              res2.data_ptr() if res2 is not None else None, dx.data_ptr(), dw.data_ptr(), part.data_ptr(), rows, d,
-              float(eps), _stream(x)), "ka_rmsnorm_bwd")
-    return dx.reshape(x.shape), dw
+    _check(fn(x2.data_ptr(), weight.data_ptr(), dy2.data_ptr(), res2.data_ptr() if res2 is not None else None,
+              dx.data_ptr(), dw.data_ptr(), part.data_ptr(), rows, d, float(eps), _stream(x2)), "ka_rmsnorm_bwd")
+    return dx.reshape(shape), dw
 
 
 class _RMSNormFn(torch.autograd.Function):
@@ -255,7 +266,7 @@ class _QkvRopeFn(torch.autograd.Function):
     def backward(ctx, dq, dk, dv):
         pos, cos, sin = ctx.saved_tensors
         dqkv = torch.empty(ctx.shape, dtype=dq.dtype, device=dq.device)
-        _qkv_rope_launch(dqkv, pos, cos, sin, dq.contiguous(), dk.contiguous(), dv.contiguous(), dq.shape[0], True)
+        _qkv_rope_launch(dqkv, pos, _packed(cos), _packed(sin), _packed(dq), _packed(dk), _packed(dv), dq.shape[0], True)
         return dqkv, None, None, None, None, None, None
 
 

@@ -172,6 +172,8 @@ def gemm_reduce_scatter(x: torch.Tensor, w_shard: torch.Tensor, ctx: TPContext,
         res = residual.contiguous()
         if res.shape[0] < rpr:
             res = torch.cat([res, res.new_zeros(rpr - res.shape[0], n)])
+        elif res.data_ptr() % 16:
+            res = res.clone()
     props = torch.cuda.get_device_properties(x.device)
     if ctx.world == 1 and _tree_pays(m, n, k_local, props.multi_processor_count):
         scratch = torch.empty(lib.ka_gemm_tree8_scratch_bytes(props.multi_processor_count), dtype=torch.uint8,

@@ -201,9 +201,76 @@ def test_qkv_rope_entry_checks_its_arguments(monkeypatch):
     cos, sin = rope_tables(16, 128)
     q, k, v = (torch.zeros(6, h, 128, dtype=torch.bfloat16) for h in (4, 2, 2))
     pos = torch.arange(6)
+    odd = torch.zeros(6 * 2 * 128 + 1, dtype=torch.bfloat16)[1:].view(6, 2, 128)
     for bad in (dict(qkv=x[:, :7 * 128]), dict(qkv=x[:5]), dict(cos=cos.view(-1)[1:]), dict(sin=sin.view(-1)[1:]),
-                dict(q=q[:, :3])):
+                dict(q=q[:, :3]), dict(v=odd), dict(k=odd)):
         args = dict(dict(qkv=x, positions=pos, cos=cos, sin=sin, q=q, k=k, v=v, tokens=6), **bad)
         for backward in (False, True):
             with pytest.raises(RuntimeError, match=r"ka_qkv_rope failed \(-[12]\)"):
                 layer_ops._qkv_rope_launch(**args, backward=backward)
+
+
+def _odd(t):
+    """The same values, contiguous, but not 16-byte aligned: a piece of a packed buffer."""
+    flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    flat[1:] = t.reshape(-1)
+    return flat[1:].view(t.shape)
+
+
+def test_gradients_reach_the_kernels_aligned(monkeypatch):
+    from kernel_align_b200.ops import layer_ops
+
+    seen = []
+
+    class Lib:
+        class _Fn:
+            def __call__(self, *args):
+                seen.extend(a % 16 for a in args if isinstance(a, int) and a > 1 << 20)
+                return 0
+        ka_qkv_rope, ka_rmsnorm_bwd = _Fn(), _Fn()
+
+        @staticmethod
+        def ka_rmsnorm_bwd_chunk():
+            return 16
+
+    monkeypatch.setattr(layer_ops._native, "cuda", lambda: Lib)
+    monkeypatch.setattr(layer_ops, "_stream", lambda t: None)
+    g = torch.zeros(4, 2, 128, dtype=torch.bfloat16)
+    cos, sin = rope_tables(16, 128)
+
+    class Ctx:
+        saved_tensors, shape = (torch.arange(4), _odd(cos), _odd(sin)), (6, 6 * 128)
+
+    layer_ops._QkvRopeFn.backward(Ctx, _odd(g), _odd(g), _odd(g))
+    x = torch.zeros(5, 64, dtype=torch.bfloat16)
+    layer_ops._rmsnorm_backward(_OnGpu(_odd(x)), _odd(x[0]), 1e-5, _odd(x), _odd(x))
+    assert len(seen) >= 12 and not any(seen)
+
+
+@pytest.mark.gpu
+def test_gpu_gradients_may_start_anywhere(cuda_device):
+    from kernel_align_b200.ops.attention import attention, attention_backward
+    from kernel_align_b200.ops.layer_ops import qkv_rope_fn, rmsnorm_fork_fn
+    from kernel_align_b200.parallel.tp_gemm import TPContext, gemm_reduce_scatter
+
+    g = torch.Generator(device=cuda_device).manual_seed(2)
+
+    def rand(*shape):
+        return torch.randn(*shape, device=cuda_device, generator=g).to(torch.bfloat16)
+
+    cos, sin = rope_tables(16, 128, device=cuda_device)
+    qkv, pos = rand(9, 8 * 128).requires_grad_(), torch.arange(7, device=cuda_device)
+    grads = [rand(7, h, 128) for h in (4, 2, 2)]
+    parts = qkv_rope_fn(qkv, pos, cos, sin, 4, 2, 128)
+    a, b = (torch.autograd.grad(parts, qkv, [f(t) for t in grads], retain_graph=True)[0] for f in (_odd, torch.clone))
+    assert torch.equal(a, b)
+    x, w, dy, dr = rand(20, 256).requires_grad_(), rand(256).requires_grad_(), rand(20, 256), rand(20, 256)
+    out = rmsnorm_fork_fn(x, w)
+    a, b = (torch.autograd.grad(out, (x, w), (f(dy), f(dr)), retain_graph=True) for f in (_odd, torch.clone))
+    assert all(torch.equal(p, q) for p, q in zip(a, b))
+    q, k, v, do = rand(2, 70, 4, 128), rand(2, 70, 2, 128), rand(2, 70, 2, 128), rand(2, 70, 4, 128)
+    o, lse = attention(q, k, v, return_lse=True)
+    assert all(torch.equal(p, r) for p, r in zip(attention_backward(q, k, v, _odd(o), do, lse),
+                                                 attention_backward(q, k, v, o, do, lse)))
+    tp, m, n, res = TPContext(device=cuda_device), rand(128, 512), rand(64, 512), rand(128, 64)
+    assert torch.equal(gemm_reduce_scatter(m, n, tp, residual=_odd(res)), gemm_reduce_scatter(m, n, tp, residual=res))
