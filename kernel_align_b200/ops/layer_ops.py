@@ -242,6 +242,7 @@ def rope_fn(x: torch.Tensor, positions: torch.Tensor, cos: torch.Tensor, sin: to
     return _RopeFn.apply(x, positions, cos, sin)
 
 
+@profiled("rope")
 def _qkv_rope_launch(qkv, positions, cos, sin, q, k, v, tokens, backward):
     fn = _native.cuda().ka_qkv_rope
     fn.restype = c_int

@@ -274,3 +274,28 @@ def test_gpu_gradients_may_start_anywhere(cuda_device):
                                                  attention_backward(q, k, v, o, do, lse)))
     tp, m, n, res = TPContext(device=cuda_device), rand(128, 512), rand(64, 512), rand(128, 64)
     assert torch.equal(gemm_reduce_scatter(m, n, tp, residual=_odd(res)), gemm_reduce_scatter(m, n, tp, residual=res))
+
+
+def test_the_fused_rotation_is_profiled_as_rope(monkeypatch):
+    from kernel_align_b200.ops import layer_ops
+    from kernel_align_b200.utils import profiler as prof
+
+    class Lib:
+        class ka_qkv_rope:
+            restype = argtypes = None
+
+            def __new__(cls, *args):
+                return 0
+
+    monkeypatch.setattr(layer_ops._native, "cuda", lambda: Lib)
+    monkeypatch.setattr(layer_ops, "_stream", lambda t: None)
+    x, pos = torch.zeros(6, 4 * 128, dtype=torch.bfloat16), torch.arange(6)
+    parts = [torch.zeros(6, h, 128, dtype=torch.bfloat16) for h in (2, 1, 1)]
+    prof.set_mode("basic")
+    prof.profiler.reset()
+    try:
+        layer_ops._qkv_rope_launch(x, pos, *rope_tables(16, 128), *parts, 6, False)
+        assert prof.profiler.summary()["rope"]["calls"] == 1
+    finally:
+        prof.set_mode("off")
+        prof.profiler.reset()

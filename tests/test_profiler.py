@@ -3,6 +3,7 @@ import math
 import os
 import sys
 
+import pytest
 import torch
 import torch.distributed as dist
 import torch.multiprocessing as mp
@@ -71,3 +72,21 @@ def test_summary_across_ranks_takes_the_slowest_rank(tmp_path):
     for r in range(2):
         s = torch.load(tmp_path / f"r{r}.pt")
         assert s["op"]["total_ms"] == 20.0 and s["other"]["total_ms"] == 1.0
+
+
+@pytest.mark.gpu
+def test_gpu_decoder_layer_has_a_range_for_every_operator(cuda_device):
+    """The rotation runs in the kernel that splits the fused projection: still under its name."""
+    cfg = LlamaConfig(vocab_size=512, hidden=256, n_layers=1, n_heads=4, n_kv_heads=2, head_dim=128, ffn=512, max_pos=256)
+    model = LlamaModel(cfg, seed=2, device=cuda_device)
+    prof.set_mode(ProfilingMode.BASIC)
+    prof.profiler.reset()
+    try:
+        model.hidden_states(torch.zeros(2, 100, dtype=torch.int64, device=cuda_device)).float().sum().backward()
+        s = prof.profiler.summary()
+    finally:
+        prof.set_mode("off")
+        prof.profiler.reset()
+    assert s["rope"]["calls"] == 2          # forward and backward
+    for name in ("rmsnorm", "attention", "attention_backward", "swiglu", "gemm_reduce_scatter"):
+        assert name in s, name
