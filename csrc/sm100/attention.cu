@@ -27,6 +27,7 @@
 #include <math_constants.h>
 
 #include "common/bounded_wait.cuh"
+#include "common/launch.cuh"
 #include "common/ptx.cuh"
 #include "common/tmap.cuh"
 #include "attention_common.cuh"
@@ -553,12 +554,8 @@ extern "C" int ka_attention_fwd(const void* q, long long q_stride, const void* k
   using namespace ka;
   if (batch <= 0 || seq_len <= 0) return 0;
   if (head_dim != kD || hq % hkv != 0) return -1;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(attention_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
-      return -10;
-    configured = true;
-  }
+  static PerDevice once;
+  if (!smem_opt_in(once, attention_fwd_kernel, kSmemBytes)) return -10;
   const uint64_t tokens = static_cast<uint64_t>(batch) * seq_len;
   CUtensorMap tq, tk, tv;
   int rc = make_tmap_2d_16bit_sw128(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, q, tokens, static_cast<uint64_t>(hq) * kD,

@@ -21,6 +21,7 @@
 #include <math_constants.h>
 
 #include "common/bounded_wait.cuh"
+#include "common/launch.cuh"
 #include "common/ptx.cuh"
 #include "common/tmap.cuh"
 #include "attention_common.cuh"
@@ -665,13 +666,10 @@ extern "C" int ka_attention_bwd(const void* q, long long q_stride, const void* k
   constexpr int kSmemDq = 6 * kTileBytes + 256;
   constexpr int kSmemDkv = 7 * kTileBytes + 2304;
   static_assert(sizeof(CtlDq) <= 256 && sizeof(CtlDkv) <= 2304 && kSmemDkv <= 227 * 1024, "shared memory layout");
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(attention_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemDq) != cudaSuccess ||
-        cudaFuncSetAttribute(attention_bwd_dkv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemDkv) != cudaSuccess)
-      return -10;
-    configured = true;
-  }
+  static PerDevice once_dq, once_dkv;
+  if (!smem_opt_in(once_dq, attention_bwd_dq_kernel, kSmemDq) ||
+      !smem_opt_in(once_dkv, attention_bwd_dkv_kernel, kSmemDkv))
+    return -10;
   const uint64_t tokens = static_cast<uint64_t>(batch) * seq_len;
   CUtensorMap tq, tk, tv, tdo;
   int rc = make_tmap_2d_16bit_sw128(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, q, tokens, static_cast<uint64_t>(hq) * kD,

@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
+#include "common/launch.cuh"
 #include "common/ptx.cuh"
 
 namespace ka {
@@ -37,6 +38,7 @@ namespace {
 constexpr int kD = 128;
 constexpr int kDecThreads = 128;
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr int kMaxScoreBytes = 200 * 1024;             // shared memory for the scores of the general form
 
 // General form, any head grouping and any alignment of the cache: one CTA per query head.
 // q: [B, Hq, D]; cache_k / cache_v: [B, max_len, Hkv, D]; lens[b]: valid keys (incl. the new
@@ -478,7 +480,7 @@ extern "C" int ka_attention_decode(const void* q, const void* cache_k, const voi
                                    int batch, int hq, int hkv, int head_dim, int max_len, float scale, void* stream) {
   using namespace ka;
   if (batch <= 0) return 0;
-  if (head_dim != kD || hq % hkv != 0 || max_len * 4 > 200 * 1024) return -1;
+  if (head_dim != kD || hq % hkv != 0 || max_len * 4 > kMaxScoreBytes) return -1;
   const int gq = hq / hkv;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const __nv_bfloat16* qb = static_cast<const __nv_bfloat16*>(q);
@@ -496,9 +498,9 @@ extern "C" int ka_attention_decode(const void* q, const void* cache_k, const voi
     }
   }
   const int smem = max_len * 4;
-  if (smem > 40 * 1024 && cudaFuncSetAttribute(attention_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               smem) != cudaSuccess)
-    return -10;
+  // the limit and not this call's size: another thread may be about to launch with a longer cache
+  static PerDevice once;
+  if (smem > 40 * 1024 && !smem_opt_in(once, attention_decode_kernel, kMaxScoreBytes)) return -10;
   attention_decode_kernel<<<batch * hq, kDecThreads, smem, st>>>(qb, kb, vb, lens, ob, hq, hkv, max_len, scale);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }

@@ -12,6 +12,7 @@
 #include <cuda_bf16.h>
 
 #include "common/bounded_wait.cuh"
+#include "common/launch.cuh"
 #include "common/ptx.cuh"
 #include "common/tmap.cuh"
 #include "gemm.h"
@@ -702,10 +703,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   }
 }
 
+// Resident CTAs of the kernel on the current device, with its shared memory opted in there.
 template <bool kTree, int BN>
-int max_ctas(int num_sms) {
-  static int cached = 0;
-  if (cached > 0) return cached;
+int setup_ctas(int num_sms) {
   if (cudaFuncSetAttribute(gemm_bf16_kernel<kTree, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
     return -1;
   cudaLaunchConfig_t cfg = {};
@@ -726,8 +726,15 @@ int max_ctas(int num_sms) {
   }
   int n = clusters * 2;
   if (n > num_sms / 2 * 2) n = num_sms / 2 * 2;
-  cached = n;
   return n;
+}
+
+template <bool kTree, int BN>
+int max_ctas(int num_sms) {
+  static PerDevice once;
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) return -1;
+  return once.get(dev, [&] { return setup_ctas<kTree, BN>(num_sms); });
 }
 
 // Whether a product takes tiles of 128 columns instead of 256: when the narrow tiles still fit the

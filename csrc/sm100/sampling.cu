@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 
 #include "../common/detmath.h"
+#include "common/launch.cuh"
 #include "sampling.h"
 
 namespace ka {
@@ -1368,13 +1369,8 @@ int launch_sampling(const void* logits, long long row_stride, int rows, int v, c
   const T* lp = static_cast<const T*>(logits);
   cudaError_t e;
   if (top_k >= 1 && top_k <= kMaxTopK) {
-    static bool configured = false;
-    if (!configured) {
-      e = cudaFuncSetAttribute(sample_topk_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(sizeof(TopkSmem)));
-      if (e != cudaSuccess) return -10;
-      configured = true;
-    }
+    static PerDevice once;
+    if (!smem_opt_in(once, sample_topk_kernel<T>, static_cast<int>(sizeof(TopkSmem)))) return -10;
     // Aligned rows that 1, 2 or 4 CTAs can keep in registers take the kernel that reads them once,
     // as long as all CTAs (one per SM) are resident at once: bf16 [G, 128256], k = 50, L2 flushed:
     // 22.6 us against 28.7 us at G = 64, but 41 against 33 us at G = 128 and 73 against 50 us at
@@ -1418,12 +1414,8 @@ int launch_sampling(const void* logits, long long row_stride, int rows, int v, c
   } else {
     constexpr int smem = kGeneralSmemBytes + (Elem<T>::kPacked ? static_cast<int>(sizeof(FastSmem)) : 0);
     static_assert(sizeof(FastSmem) >= kHistBytes, "the older search keeps its histogram there");
-    static bool configured = false;
-    if (!configured) {
-      e = cudaFuncSetAttribute(sample_general_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return -10;
-      configured = true;
-    }
+    static PerDevice once;
+    if (!smem_opt_in(once, sample_general_kernel<T>, smem)) return -10;
     sample_general_kernel<T><<<rows, kThreads, smem, stream>>>(lp, row_stride, v, row_ids, inv_temp, top_k, top_p,
                                                               seed, step, out);
   }
