@@ -92,3 +92,20 @@ def test_gpu_attention_backward_matches_autograd(cuda_device, b, l, hq, hkv, cau
     if b > 1:
         attention_fn(q3, k3, v3, causal=causal).backward(d_o[1:2])
         assert torch.equal(q3.grad, qg.grad[1:2]) and torch.equal(k3.grad, kg.grad[1:2])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("causal", [True, False])
+def test_gpu_attention_backward_reads_views_of_a_fused_projection(cuda_device, causal):
+    from kernel_align_b200.ops.attention import attention_backward
+
+    g = torch.Generator(device=cuda_device).manual_seed(6)
+    b, l, hq, hkv, d = 2, 200, 4, 2, 128
+    qkv = torch.randn(b, l, hq + 2 * hkv, d, device=cuda_device, generator=g).to(torch.bfloat16)
+    wide = torch.randn(b, l, 2 * hq, d, device=cuda_device, generator=g).to(torch.bfloat16)
+    views = qkv[:, :, :hq], qkv[:, :, hq:hq + hkv], qkv[:, :, hq + hkv:]
+    o, lse = attention(*views, causal=causal, return_lse=True)
+    wide[:, :, :hq] = o
+    strided = attention_backward(*views, wide[:, :, :hq], wide[:, :, hq:], lse, causal=causal)
+    packed = attention_backward(*(t.contiguous() for t in views), o, wide[:, :, hq:].contiguous(), lse, causal=causal)
+    assert all(torch.equal(s, p) for s, p in zip(strided, packed))

@@ -151,3 +151,31 @@ def test_decode_attention_bits_do_not_depend_on_how_many_ctas_share_a_sequence(c
     flat[1:] = ck.reshape(-1)
     off = attention_decode(q, flat[1:].view_as(ck), cv, lens)
     assert (off.float() - out.float()).abs().max().item() <= 2 ** -7 * ref.abs().max().item()
+
+
+@pytest.mark.parametrize("hq,hkv", [(4, 4), (4, 2), (8, 2), (8, 1), (6, 2)])
+def test_decode_attention_special_values(cuda_device, hq, hkv):
+    """Whatever lies behind a sequence's length is not looked at; NaN and infinities inside it come
+    out where plain softmax attention has them; an empty sequence has no result (0 / 0)."""
+    lens = torch.tensor([300, 300, 300, 300, 300, 70, 0], dtype=torch.int32, device=cuda_device)
+    g = torch.Generator(device=cuda_device).manual_seed(hq)
+    n = lens.numel()
+    q = torch.randn(n, hq, 128, device=cuda_device, generator=g).to(torch.bfloat16)
+    ck = torch.randn(n, 320, hkv, 128, device=cuda_device, generator=g).to(torch.bfloat16)
+    cv = torch.randn(n, 320, hkv, 128, device=cuda_device, generator=g).to(torch.bfloat16)
+    for i, l in enumerate(lens.tolist()):
+        ck[i, l:], cv[i, l:] = float("nan"), float("nan")
+    clean = attention_decode(q, ck, cv, lens)
+    assert torch.isfinite(clean[:6]).all() and torch.isnan(clean[6]).all()
+    ck[0, 200, 0, 5] = float("nan")              # a score is NaN: the heads of that group are
+    ck[1, 17, hkv - 1, 3] = float("inf")         # a score is +inf (NaN probabilities) or -inf (no weight)
+    cv[2, 299, 0, 7] = float("inf")              # one element of the result
+    cv[3, 64, 0, 9] = float("nan")
+    ck[4, :300, 0, 0] = float("-inf")            # every score of the group infinite
+    out = attention_decode(q, ck, cv, lens).cpu().float()
+    ref = attention_decode(q.cpu().float(), ck.cpu().float(), cv.cpu().float(), lens.cpu())
+    ref[6] = float("nan")
+    assert torch.equal(torch.isnan(out), torch.isnan(ref)) and torch.equal(torch.isinf(out), torch.isinf(ref))
+    ok = torch.isfinite(ref)
+    assert (out[ok] - ref[ok]).abs().max() <= 2 ** -8 * ref[ok].abs().max()
+    assert torch.equal(out[5], clean[5].cpu().float())

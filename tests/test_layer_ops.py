@@ -299,3 +299,25 @@ def test_the_fused_rotation_is_profiled_as_rope(monkeypatch):
     finally:
         prof.set_mode("off")
         prof.profiler.reset()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d", [128, 2048, 2056, 4096, 4104, 8192, 8200])
+def test_gpu_rmsnorm_bits_do_not_depend_on_the_number_of_rows(cuda_device, d):
+    """Few rows are kept in registers, many are read twice: the same sums in the same order."""
+    g = torch.Generator(device=cuda_device).manual_seed(d)
+    x, r = (torch.randn(1300, d, device=cuda_device, generator=g).to(torch.bfloat16) for _ in range(2))
+    w = (torch.randn(d, device=cuda_device, generator=g) * 0.1 + 1).to(torch.bfloat16)
+    y = rmsnorm(x, w)
+    yr, ro = rmsnorm(x, w, residual=r)
+    sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    for rows in (1, 17, 2 * sms, 2 * sms + 1, 4 * sms, 4 * sms + 1):
+        for lo in (0, 1300 - rows):
+            part = slice(lo, lo + rows)
+            assert torch.equal(rmsnorm(x[part], w), y[part]), rows
+            a, b = rmsnorm(x[part], w, residual=r[part])
+            assert torch.equal(a, yr[part]) and torch.equal(b, ro[part]), rows
+    want, want_ro = _rms_ref(x.cpu(), w.cpu(), 1e-5, r.cpu())
+    # both round the normalised value and the product to bf16: two units in the last place of the largest
+    assert torch.equal(ro.cpu(), want_ro)
+    assert (yr.cpu().float() - want.float()).abs().max() <= 2 ** -7 * want.float().abs().max()
