@@ -158,8 +158,12 @@ __device__ __forceinline__ float fold_value(const FoldWeights& f, float v_old, f
   return __fmaf_rn(f.w_new, v_new, __fmul_rn(f.w_old, v_old));
 }
 
+// CTAs of the split kernel that are resident on an SM: its registers are bounded for that many.
 template <int GQ>
-__global__ void __launch_bounds__(kDecThreads, GQ == 8 ? 2 : 3)
+constexpr int kCtasPerSm = GQ == 8 ? 2 : 3;
+
+template <int GQ>
+__global__ void __launch_bounds__(kDecThreads, kCtasPerSm<GQ>)
 attention_decode_split_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache_k,
                               const __nv_bfloat16* __restrict__ cache_v, const int* __restrict__ lens,
                               __nv_bfloat16* __restrict__ out, int hq, int hkv, int max_len, float scale, int splits) {
@@ -436,24 +440,62 @@ attention_decode_split_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bf
   cluster_wait();
 }
 
+// Shared memory of a CTA that is one of `splits`: the fold (2), or a state per stripe (two with 4).
+template <int GQ>
+constexpr int split_smem(int splits) {
+  return static_cast<int>(sizeof(SplitSmem<GQ>)) +
+         (splits == 2 ? 1 : kStripes / splits) * static_cast<int>(sizeof(State<GQ>));
+}
+
+// Clusters of `splits` CTAs that are resident at once on the current device. Asked of the runtime, once per device:
+// clusters must fit the SMs of a GPC, so there are fewer than kCtasPerSm * SMs / splits of them (64 / 8 heads, 9 x 448
+// keys: 72 clusters of four are 288 CTAs for 296 places, but only 71 fit: 19.5 us, as clusters of two 12.2 us).
+template <int GQ>
+int resident_clusters(int splits) {
+  static_assert(split_smem<GQ>(4) <= 48 * 1024, "the largest request, fits without an opt-in");
+  static PerDevice once[kStripes + 1];
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  return once[splits].get(dev, [&] {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(splits));
+    cfg.blockDim = dim3(kDecThreads);
+    cfg.dynamicSmemBytes = static_cast<size_t>(split_smem<GQ>(splits));
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, attention_decode_split_kernel<GQ>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return n;
+  });
+}
+
+// CTAs per (sequence, KV head): as many as are resident at once, and no more than the cache has blocks: a second wave,
+// or CTAs without keys, cost a set-up and two cluster barriers for nothing (32 / 8 heads: 8 x 448 keys 10.0 us with
+// S = 4, 13.7 with S = 8; 32 x 100 keys 14 us, 26 us without these limits; 64 / 8 heads, two CTAs per SM: 10 x 448 keys
+// 14.6 us with S = 2, 20.2 with S = 4). The result does not depend on this choice.
+template <int GQ>
+int choose_splits(int batch, int hkv, int max_len) {
+  const int blocks = (max_len + kBlockKeys - 1) / kBlockKeys;
+  int splits = 2;
+  while (splits < kStripes && splits < blocks &&
+         static_cast<long long>(batch) * hkv <= resident_clusters<GQ>(splits * 2))
+    splits *= 2;
+  return splits;
+}
+
 template <int GQ>
 int launch_split(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v, const int* lens,
                  __nv_bfloat16* out, int batch, int hq, int hkv, int max_len, float scale, cudaStream_t st) {
-  // As many CTAs as are resident at once (three per SM of a 148-SM device), and no more than the
-  // cache has blocks: a second wave, or CTAs without keys, cost a set-up and two cluster barriers
-  // for nothing (8 x 448 keys, 32 / 8 heads:
-  // 10.0 us with S = 4, 13.7 with S = 8; 32 x 100 keys: 14 us, 26 us without these limits). The result does not depend on this choice.
-  constexpr long long kResident = 3 * 148;
-  const int blocks = (max_len + kBlockKeys - 1) / kBlockKeys;
-  int splits = 2;
-  while (splits < kStripes && splits < blocks && static_cast<long long>(batch) * hkv * splits * 2 <= kResident)
-    splits *= 2;
-  const int smem = static_cast<int>(sizeof(SplitSmem<GQ>)) +
-                   (splits == 2 ? 1 : kStripes / splits) * static_cast<int>(sizeof(State<GQ>));
-  if (smem > 48 * 1024 &&    // per device and cheap: set on every call that needs it
-      cudaFuncSetAttribute(attention_decode_split_kernel<GQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-          cudaSuccess)
-    return -10;
+  const int splits = choose_splits<GQ>(batch, hkv, max_len);
+  const int smem = split_smem<GQ>(splits);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(batch) * hkv * splits);
   cfg.blockDim = dim3(kDecThreads);
@@ -503,4 +545,18 @@ extern "C" int ka_attention_decode(const void* q, const void* cache_k, const voi
   if (smem > 40 * 1024 && !smem_opt_in(once, attention_decode_kernel, kMaxScoreBytes)) return -10;
   attention_decode_kernel<<<batch * hq, kDecThreads, smem, st>>>(qb, kb, vb, lens, ob, hq, hkv, max_len, scale);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
+// How many CTAs ka_attention_decode puts on a (sequence, KV head) of an aligned cache on the current device; 1 for a
+// grouping that the general form takes.
+extern "C" int ka_attention_decode_splits(int batch, int hq, int hkv, int max_len) {
+  using namespace ka;
+  if (batch <= 0 || hkv <= 0 || hq % hkv != 0) return -1;
+  switch (hq / hkv) {
+    case 1: return choose_splits<1>(batch, hkv, max_len);
+    case 2: return choose_splits<2>(batch, hkv, max_len);
+    case 4: return choose_splits<4>(batch, hkv, max_len);
+    case 8: return choose_splits<8>(batch, hkv, max_len);
+    default: return 1;
+  }
 }

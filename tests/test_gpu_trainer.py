@@ -179,3 +179,17 @@ def test_decode_attention_special_values(cuda_device, hq, hkv):
     ok = torch.isfinite(ref)
     assert (out[ok] - ref[ok]).abs().max() <= 2 ** -8 * ref[ok].abs().max()
     assert torch.equal(out[5], clean[5].cpu().float())
+
+
+@pytest.mark.parametrize("hq,hkv,per_sm", [(8, 8, 3), (16, 8, 3), (32, 8, 3), (64, 8, 2), (8, 1, 2)])
+def test_decode_attention_ctas_are_resident_at_once(cuda_device, hq, hkv, per_sm):
+    """More than two CTAs per (sequence, KV head) only while all of them run at the same time (`per_sm`:
+    what the registers of the kernel allow), and never more than the cache has blocks."""
+    from kernel_align_b200 import _native
+
+    splits = _native.cuda().ka_attention_decode_splits
+    sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    chosen = [splits(b, hq, hkv, 4096) for b in range(1, 600)]
+    assert chosen[0] == 8 and chosen[-1] == 2 and chosen == sorted(chosen, reverse=True)
+    assert all(s == 2 or (b + 1) * hkv * s <= per_sm * sms for b, s in enumerate(chosen))
+    assert [splits(1, hq, hkv, n) for n in (1, 64, 128, 129, 256, 257)] == [2, 2, 2, 4, 4, 8]
