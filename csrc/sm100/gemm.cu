@@ -738,11 +738,18 @@ int max_ctas(int num_sms) {
 }
 
 // Whether a product takes tiles of 128 columns instead of 256: when the narrow tiles still fit the
-// CTA pairs in one round, so that twice as many SMs load and run the epilogue. With more tiles the
-// wide ones win, they load a third less per product. Measured, 512 rows, N = 4096 (32 wide tiles on
-// 74 pairs), wide / narrow in us: slices kept in the kernel 45.5 / 35.3 (K = 4096), 97 / 86 (14336),
-// 162 / 152 (28672); plain 27.3 / 25.6 (4096), 77.0 / 75.7 (14336: both wait for L2).
-inline bool narrow_tiles(int tiles_m, int tiles_n, int pairs) { return tiles_m * tiles_n * 2 <= pairs; }
+// CTA pairs in one round, so that twice as many SMs run the epilogue and the last tile's drain. What
+// that saves is the same for every K (about 1 us, 8 us where the slices are kept in the kernel), while
+// the narrow tiles load a third more per product, so a plain product with a long K takes the wide ones.
+// Measured wide / narrow in us, 4 to 36 wide tiles on 74 pairs: plain, 464 x 4096 (32 tiles): 8.1 / 6.9
+// (K = 128), 27.8 / 26.9 (4096), 76.4 / 76.1 (14336), 103.6 / 103.5 (20000), 160.4 / 161.3 (32000), 629 / 648
+// (128256: the hidden gradient of the LM head); slices kept in the kernel, 512 x 4096: 43.4 / 35.2 (4096),
+// 93.2 / 88.4 (14336), 167 / 162 (28672). More narrow tiles than pairs would need another round.
+constexpr int kNarrowMaxK = 16384;
+
+inline bool narrow_tiles(int tiles_m, int tiles_n, int k, bool tree, int pairs) {
+  return static_cast<long long>(tiles_m) * tiles_n * 2 <= pairs && (tree || k <= kNarrowMaxK);
+}
 
 }  // namespace
 
@@ -759,7 +766,7 @@ int gemm_launch(const void* a, long long lda, const void* b, long long ldb, cons
   int ctas = tree ? max_ctas<true, kBN>(num_sms) : max_ctas<false, kBN>(num_sms);
   if (ctas <= 0) return -10;
   const int tiles_m = (p.m + kBM * kG - 1) / (kBM * kG);
-  const bool narrow = !full_grid && narrow_tiles(tiles_m, (p.n + kBN - 1) / kBN, ctas / kG);
+  const bool narrow = !full_grid && narrow_tiles(tiles_m, (p.n + kBN - 1) / kBN, p.k, tree, ctas / kG);
   if (narrow) ctas = tree ? max_ctas<true, kBN / 2>(num_sms) : max_ctas<false, kBN / 2>(num_sms);
   if (ctas <= 0) return -10;
   const int bn = narrow ? kBN / 2 : kBN;
@@ -801,6 +808,13 @@ int gemm_launch(const void* a, long long lda, const void* b, long long ldb, cons
 }
 
 }  // namespace ka
+
+// Columns per tile that an m x n x k product takes on a device where `pairs` CTA pairs are resident;
+// tree: with its eight K slices summed in the kernel.
+extern "C" int ka_gemm_tile_columns(int m, int n, int k, int tree, int pairs) {
+  using namespace ka;
+  return narrow_tiles((m + kBM * kG - 1) / (kBM * kG), (n + kBN - 1) / kBN, k, tree != 0, pairs) ? kBN / 2 : kBN;
+}
 
 extern "C" int ka_gemm_bf16(const void* a, long long lda, int a_major, const void* b, long long ldb, int b_major,
                             void* c, long long ldc, int out_f32, int m, int n, int k, int* status, int num_sms,
