@@ -22,7 +22,7 @@ def main():
     ap.add_argument("--op", required=True,
                     choices=["fused_logp", "logits_logp", "sampling", "rmsnorm", "swiglu", "gemm", "attention", "attention_bwd",
                              "grpo_loss", "rope", "adamw", "decode_attention", "gemm_skinny", "rmsnorm_bwd", "logp_bwd",
-                             "decode_qkv", "sampling_top_p"])
+                             "decode_qkv", "sampling_top_p", "decoder_layer"])
     ap.add_argument("--rows", type=int, default=4736)
     ap.add_argument("--vocab", type=int, default=128256)
     ap.add_argument("--hidden", type=int, default=4096)
@@ -176,6 +176,20 @@ def main():
             w.grad = None
             lmhead_logp(h, w, ids).sum().backward()
             return h.grad
+    elif args.op == "decoder_layer":        # one sequence of 512 tokens, forward and backward
+        from kernel_align_b200.models.llama import DecoderLayer, LlamaConfig
+        from kernel_align_b200.ops.layer_ops import rope_tables
+        from kernel_align_b200.parallel.tp_gemm import TPContext
+
+        layer = DecoderLayer(LlamaConfig(n_layers=1), TPContext(device=dev), 1, dev)
+        cos, sin = rope_tables(512, 128, 500000.0, device=dev)
+        x = torch.randn(512, 4096, device=dev, generator=g).to(torch.bfloat16).requires_grad_()
+        pos = torch.arange(512, device=dev)
+
+        def fn():
+            y = layer(x, 1, 512, pos, cos, sin)
+            y.backward(torch.ones_like(y))
+            return y
     else:
         raise SystemExit(f"--op {args.op}: no profile case defined yet")
     for _ in range(args.launches):

@@ -86,8 +86,8 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
 
 // The same row in registers (d <= 2048 * VPT): x, residual and weight are requested together, the
 // row is touched once, and what is left is one memory latency, one block reduction and the
-// stores. Sums run in rmsnorm_kernel's order, so the bits are the same. (8 rows of 4096 with the
-// residual add: re-reading the row after the reduction took 4.7 us, this takes 3.0.)
+// stores. Sums run in rmsnorm_kernel's order, so the bits are the same. What it gives is beside the
+// rule that picks it, in ka_rmsnorm.
 template <int VPT>
 __global__ void __launch_bounds__(256, VPT == 4 ? 2 : 4)
 rmsnorm_reg_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
@@ -330,9 +330,10 @@ swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* _
 // One CTA per chunk of kRmsChunk rows (fixed, so the order in which rows enter d_w does not
 // depend on the grid); 16 rows give 4096 tokens 256 CTAs, one wave of two per SM (64 rows left
 // more than half of the SMs idle: 92 us). With `d_res` the gradient that reaches x past the norm
-// (the residual stream) is added to the rounded dx, which saves a pass. Threads own columns. kRows rows are in flight at once: their x and dy
-// vectors are loaded once into registers and serve all three steps (sum of squares, the dot
-// product, dx / dw), and the block reductions of the kRows rows share their two barriers.
+// (the residual stream) is added to the rounded dx, which saves a pass. Threads own columns. kRows
+// rows are worked on at once (two up to d = 2048, else one): their x and dy vectors are loaded once into
+// registers and serve both steps (the two sums, then dx / dw), and the sums of all of them share one
+// block reduction with a single barrier.
 constexpr int kRmsChunk = 16;
 
 // Fixed-order sums of R values per thread over the CTA (8 warps): lanes by xor-shuffle, then the
@@ -544,10 +545,11 @@ int ka_rmsnorm(const void* x, const void* residual, const void* w, void* y, void
   if (rows <= 0) return 0;
   if (d % 8 != 0) return -1;
   const int grid = rows < num_sms * 8 ? rows : num_sms * 8;
-  // Rows that are all resident at once take the register kernel: what counts there is one row's
-  // latency (d = 4096: 2.6 against 3.5 us for 8 rows, 3.8 against 4.6 us for 512). With more rows the
-  // other one's eight CTAs per SM hide more of it (16384 rows: 96 against 92 us; d = 8192: 246
-  // against 175 us). Both give the same bits.
+  // Rows that are all resident at once take the register kernel: what counts there is one row's latency.
+  // With the residual add, loop / register kernel in us: d = 4096: 2.9 / 2.1 (8 rows), 4.4 / 3.6 (296), 4.8 / 4.4 (592);
+  // d = 8192: 4.5 / 3.1 (8), 6.7 / 5.2 (296). With more rows the loop's eight CTAs per SM hide more of it
+  // (d = 4096: 6.9 / 6.9 for 1024 rows, 92 / 96 for 16384; d = 8192: 8.7 / 8.8 for 512, 175 / 246 for 16384). Both give
+  // the same bits.
   auto* kernel = rmsnorm_kernel;
   if (d <= 8192 && rows <= num_sms * (d <= 4096 ? 4 : 2))
     kernel = d <= 2048 ? rmsnorm_reg_kernel<1> : (d <= 4096 ? rmsnorm_reg_kernel<2> : rmsnorm_reg_kernel<4>);

@@ -1,6 +1,7 @@
 """Single-token attention against a KV cache (rollout phase) and the fused AdamW update.
 
-Kernels: ``csrc/sm100/decode_optim.cu``. CPU tensors fall back to the equivalent PyTorch math.
+Kernels: ``csrc/sm100/attention_decode.cu`` (attention) and ``csrc/sm100/decode_optim.cu`` (split /
+rotation / cache write, AdamW). CPU tensors fall back to the equivalent PyTorch math.
 """
 from __future__ import annotations
 

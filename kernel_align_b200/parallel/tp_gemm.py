@@ -137,10 +137,12 @@ def _tree_pays(m: int, n: int, k: int, num_sms: int) -> bool:
 
     A CTA pair that keeps a tile walks its eight slices one after the other, while staged slices
     spread over all pairs but cost a pass over the partials and the wait for them. Measured on
-    148 SMs, staged / kept in us: 4096 rows, N = 4096: 411 / 186 (K = 4096), 1003 / 776 (28672);
-    32 tiles: 77 / 35 (4096), 104 / 86 (14336), 145 / 152 (28672); 16 tiles: 57 / 32 (4096),
-    62 / 48 (6144), 75 / 85 (14336), 95 / 152 (28672). A slice round takes about 5.4e-3 us per
-    K column, staging about 20 us plus 1.2 us per tile; the rule compares the two."""
+    148 SMs, staged / kept in us, tiles counted as 256 x 256 (the kept form cuts up to 37 of them into
+    halves of 128 columns): 256 tiles: 385 / 156 (K = 4096), 1025 / 738 (28672); 32 tiles: 72 / 35 (4096),
+    109 / 90 (14336), 150 / 163 (28672); 16 tiles: 48 / 33 (4096), 57 / 44 (6144), 70 / 85 (14336),
+    101 / 156 (28672); 8 tiles: 39 / 33 (4096), 42 / 43 (6144), 54 / 82 (14336); 4 tiles: 39 / 33 (4096),
+    40 / 42 (6144). A slice round takes about 5.4e-3 us per K column, staging about 20 us plus 1.2 us per
+    tile; the rule compares the two."""
     pairs = max(1, num_sms // 2)
     tiles = -(-m // 256) * -(-n // 256)
     extra_rounds = -(-tiles // pairs) * 8 - -(-8 * tiles // pairs)
