@@ -15,7 +15,7 @@
 //
 // Three kernels:
 //   sample_topk_kernel     top_k in [1, 1024] (greedy = top_k 1), optional top_p
-//   sample_topk_held_kernel  the same for aligned 16-bit rows that 1, 2 or 4 CTAs hold in registers
+//   sample_topk_held_kernel  the same for 16-bit rows that 1, 2 or 4 CTAs hold in registers
 //                          (a cluster; candidates exchanged through distributed shared memory)
 //   sample_general_kernel  no top_k (or k > 1024), optional top_p: 16-bit rows by one histogram of
 //                          counts per key (sample_row16), fp32 rows and the few 16-bit rows that
@@ -36,9 +36,11 @@ namespace {
 
 constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
-constexpr int kCandCap = 4096;
+constexpr int kCandCap = 10240;
 constexpr int kMaxTopK = 1024;
 
+// `wmax` / `any_ge` work on a 32-bit register word as it was loaded (two 16-bit floats or one fp32):
+// a NaN loses against every number, fails every comparison and -0 counts as +0 in a comparison.
 template <typename T>
 struct Elem;
 template <>
@@ -48,6 +50,10 @@ struct Elem<float> {
   static constexpr bool kPacked = false;
   static constexpr uint32_t kInf2 = 0;
   __device__ static float to_float(float v) { return v; }
+  __device__ static uint32_t wmax(uint32_t a, uint32_t b) {
+    return __float_as_uint(fmaxf(__uint_as_float(a), __uint_as_float(b)));
+  }
+  __device__ static bool any_ge(uint32_t a, uint32_t b) { return __uint_as_float(a) >= __uint_as_float(b); }
 };
 template <>
 struct Elem<__nv_bfloat16> {
@@ -56,6 +62,18 @@ struct Elem<__nv_bfloat16> {
   static constexpr bool kPacked = true;
   static constexpr uint32_t kInf2 = 0x7F807F80u;  // +inf bit pattern, twice
   __device__ static float to_float(__nv_bfloat16 v) { return __bfloat162float(v); }
+  __device__ static uint32_t wmax(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+  }
+  __device__ static bool any_ge(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("{\n\t.reg .pred p, q;\n\tsetp.ge.bf16x2 p|q, %1, %2;\n\tor.pred p, p, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(d)
+        : "r"(a), "r"(b));
+    return d != 0;
+  }
 };
 template <>
 struct Elem<__half> {
@@ -64,42 +82,41 @@ struct Elem<__half> {
   static constexpr bool kPacked = true;
   static constexpr uint32_t kInf2 = 0x7C007C00u;
   __device__ static float to_float(__half v) { return __half2float(v); }
+  __device__ static uint32_t wmax(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("max.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+  }
+  __device__ static bool any_ge(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("{\n\t.reg .pred p, q;\n\tsetp.ge.f16x2 p|q, %1, %2;\n\tor.pred p, p, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(d)
+        : "r"(a), "r"(b));
+    return d != 0;
+  }
 };
 
-// Visit every element of a row once: 16-byte vector loads when the row allows it.
-template <typename T, typename F>
-__device__ __forceinline__ void for_each_key(const T* __restrict__ row, int v, bool vec_ok, F&& f) {
-  constexpr int kVec = Elem<T>::kVec;
-  const int tid = threadIdx.x;
-  if (vec_ok) {
-    const int nvec = v / kVec;
-    const uint4* p = reinterpret_cast<const uint4*>(row);
-    for (int i = tid; i < nvec; i += blockDim.x) {
-      const uint4 raw = p[i];
-      const T* e = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-      for (int j = 0; j < kVec; ++j) f(float_to_key(Elem<T>::to_float(e[j])), i * kVec + j);
-    }
-    for (int i = nvec * kVec + tid; i < v; i += blockDim.x) f(float_to_key(Elem<T>::to_float(row[i])), i);
-  } else {
-    for (int i = tid; i < v; i += blockDim.x) f(float_to_key(Elem<T>::to_float(row[i])), i);
-  }
+template <typename T>
+__device__ __forceinline__ uint32_t vec_max(const uint4& r) {
+  return Elem<T>::wmax(Elem<T>::wmax(r.x, r.y), Elem<T>::wmax(r.z, r.w));
 }
 
-// The same visit with four 16-byte loads in flight per thread (a single CTA walking a row is
-// bound by the latency of its loads). The order of the visits differs, so only for callbacks
-// that do not depend on it.
+// Elements of a row in front of its first 16-byte boundary (rows of an odd width start anywhere).
+template <typename T>
+__device__ __forceinline__ int row_head(const T* rp, int v) {
+  const int bytes = static_cast<int>((16u - (reinterpret_cast<uintptr_t>(rp) & 15u)) & 15u);
+  return min(v, bytes / static_cast<int>(sizeof(T)));
+}
+
+// Visit every element of a row once, in any order: scalars up to the first 16-byte boundary and
+// behind the last, vectors between, four of them in flight per thread (a single CTA that walks a row
+// is bound by the latency of its loads).
 template <typename T, typename F>
-__device__ __forceinline__ void for_each_key_x4(const T* __restrict__ row, int v, bool vec_ok, F&& f) {
+__device__ __forceinline__ void for_each_key(const T* __restrict__ row, int v, F&& f) {
   constexpr int kVec = Elem<T>::kVec;
-  if (!vec_ok) {
-    for_each_key<T>(row, v, false, f);
-    return;
-  }
-  const int tid = threadIdx.x;
-  const int stride = blockDim.x;
-  const int nvec = v / kVec;
-  const uint4* p = reinterpret_cast<const uint4*>(row);
+  const int tid = threadIdx.x, stride = blockDim.x;
+  const int head = row_head(row, v), nvec = (v - head) / kVec, scal = v - nvec * kVec;
+  const uint4* p = reinterpret_cast<const uint4*>(row + head);
   int i = tid;
   for (; i + 3 * stride < nvec; i += 4 * stride) {
     uint4 raw[4];
@@ -109,16 +126,19 @@ __device__ __forceinline__ void for_each_key_x4(const T* __restrict__ row, int v
     for (int u = 0; u < 4; ++u) {
       const T* e = reinterpret_cast<const T*>(&raw[u]);
 #pragma unroll
-      for (int j = 0; j < kVec; ++j) f(float_to_key(Elem<T>::to_float(e[j])), (i + u * stride) * kVec + j);
+      for (int j = 0; j < kVec; ++j) f(float_to_key(Elem<T>::to_float(e[j])), head + (i + u * stride) * kVec + j);
     }
   }
   for (; i < nvec; i += stride) {
     const uint4 raw = p[i];
     const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) f(float_to_key(Elem<T>::to_float(e[j])), i * kVec + j);
+    for (int j = 0; j < kVec; ++j) f(float_to_key(Elem<T>::to_float(e[j])), head + i * kVec + j);
   }
-  for (int k = nvec * kVec + tid; k < v; k += stride) f(float_to_key(Elem<T>::to_float(row[k])), k);
+  for (int k = tid; k < scal; k += stride) {
+    const int idx = k < head ? k : nvec * kVec + k;
+    f(float_to_key(Elem<T>::to_float(row[idx])), idx);
+  }
 }
 
 __device__ __forceinline__ int block_sum_int(int v, int* s_warp) {
@@ -159,76 +179,252 @@ __device__ __forceinline__ unsigned long long block_exscan_u64(unsigned long lon
   return warp_off + inc - v;
 }
 
+constexpr int kWarpTops = 128;    // keys that the warps of a block bring to the search for a small k
+
 struct TopkSmem {
-  uint32_t cand_key[kCandCap];
-  uint32_t cand_idx[kCandCap];
-  uint32_t sorted_key[kMaxTopK];
-  uint32_t sorted_idx[kMaxTopK];
+  unsigned long long cand[kCandCap];          // key in the high word, ~token id in the low: descending = sorted order
+  unsigned long long sorted[kMaxTopK];
   unsigned long long mass[kMaxTopK];
   unsigned long long scan[kWarps];
+  unsigned long long kept_mass;
+  unsigned int hits[2][kWarps];
+  unsigned int top[kWarpTops];                // the largest keys of every warp
+  unsigned int bound;
   int red[kWarps];
   int count;
+  int n_sorted;
+  int n_ties;
+  int keep;
+  int pick;
 };
 
-// Final step of the top-k path, run by one warp: survivors sorted by (key desc, id asc) with
-// masses q[0..n); apply top-p, draw, return the position picked. All sums are integers, so
-// the warp-parallel prefix sums give exactly the result of a serial walk.
-__device__ __forceinline__ int pick_sorted_warp(const unsigned long long* q, int n, float top_p, uint32_t u24) {
-  const int lane = threadIdx.x & 31;
-  // lane owns the contiguous slice [lane * per, lane * per + per)
-  const int per = (n + 31) / 32;
-  const int lo = min(n, lane * per), hi = min(n, lo + per);
-  unsigned long long mine = 0;
-  for (int i = lo; i < hi; ++i) mine += q[i];
-  unsigned long long inc = mine;
+__device__ __forceinline__ unsigned long long cand_of(uint32_t key, int idx) {
+  return (static_cast<unsigned long long>(key) << 32) | (~static_cast<uint32_t>(idx));
+}
+
+// Block totals of three counts, packed by thread in fields of 10 bits that a warp's sum must fit; a total
+// is at most 65535. One barrier: `hits` alternates between two rows, and the row is read before the next
+// call's barrier.
+__device__ __forceinline__ void block_count3(uint32_t packed, unsigned int (&hits)[2][kWarps], int parity, int& c1, int& c2,
+                                             int& c3) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  packed = __reduce_add_sync(0xffffffffu, packed);
+  if (lane == 0) hits[parity][warp] = packed;
+  __syncthreads();
+  const uint32_t w = lane < static_cast<int>(blockDim.x >> 5) ? hits[parity][lane] : 0u;
+  const uint32_t a = __reduce_add_sync(0xffffffffu, (w & 1023u) | (((w >> 10) & 1023u) << 16));
+  c3 = static_cast<int>(__reduce_add_sync(0xffffffffu, w >> 20));
+  c1 = static_cast<int>(a & 0xFFFFu);
+  c2 = static_cast<int>(a >> 16);
+}
+
+// Final step of the top-k path for at most 64 survivors, run by one warp: lane l holds the masses q0, q1
+// of the survivors 2 l and 2 l + 1 in sorted order; apply top-p, draw, return the position picked. All
+// sums are integers, so the warp-parallel prefix sums give exactly the result of a serial walk.
+__device__ __forceinline__ int pick_sorted_warp(unsigned long long q0, unsigned long long q1, int n, float top_p,
+                                                uint32_t u24) {
+  const int lane = threadIdx.x & 31, i = 2 * lane;
+  unsigned long long inc = q0 + q1;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
     if (lane >= o) inc += t;
   }
   const unsigned long long z = __shfl_sync(0xffffffffu, inc, 31);
-  const unsigned long long before = inc - mine;  // mass of the elements before this lane's slice
+  const unsigned long long mid = inc - q1, before = mid - q0;
+  // position of the first survivor for which a (the even one of a lane) or b (the odd one) holds, else n
+  auto first_of = [&](bool a, bool b) {
+    const uint32_t ma = __ballot_sync(0xffffffffu, a), mb = __ballot_sync(0xffffffffu, b);
+    if ((ma | mb) == 0) return n;
+    const int l = __ffs(static_cast<int>(ma | mb)) - 1;
+    return 2 * l + ((ma >> l) & 1u ? 0 : 1);
+  };
   int keep = n;
   unsigned long long zk = z;
   if (top_p < 1.0f) {
     // keep = first i > 0 with (mass before i) > limit, else n
     const unsigned long long limit = mass_fraction(static_cast<double>(top_p), z);
-    int first = n;
-    unsigned long long cum = before;
-    for (int i = lo; i < hi; ++i) {
-      if (i > 0 && cum > limit) {
-        first = i;
-        break;
-      }
-      cum += q[i];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
-    keep = first;
-    // zk = mass of the first `keep` elements
-    unsigned long long part = 0;
-    for (int i = lo; i < min(hi, keep); ++i) part += q[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    zk = part;
+    keep = first_of(i > 0 && i < n && before > limit, i + 1 < n && mid > limit);
+    zk = __shfl_sync(0xffffffffu, (keep & 1) ? mid : inc, (keep - 1) >> 1);
   }
   const unsigned long long target = mass_scale_u24(u24, zk);
-  int pick = keep - 1;
-  {
-    int first = n;
-    unsigned long long acc = before;
-    for (int i = lo; i < min(hi, keep); ++i) {
-      acc += q[i];
-      if (acc > target) {
-        first = i;
-        break;
-      }
-    }
+  const int pick = first_of(i < keep && mid > target, i + 1 < keep && inc > target);
+  return pick < keep ? pick : keep - 1;
+}
+
+// Bits that a search among keys between lo and hi has to decide, rounded up to pairs.
+__device__ __forceinline__ int open_bits(uint32_t lo, uint32_t hi) { return (33 - __clz(static_cast<int>(lo ^ hi))) & ~1; }
+__device__ __forceinline__ uint32_t above_bits(uint32_t key, int bits) { return bits >= 32 ? 0u : key >> bits << bits; }
+
+// The largest key that at least kk of the block's keys reach (0 if there are fewer above 0), two bits per
+// step; bits that all keys share need no step. A thread brings NW words: two 16-bit keys each, or one key
+// of 32 bits.
+template <int NW, int kBits>
+__device__ __forceinline__ uint32_t kth_key(const uint32_t (&w)[NW], int kk, unsigned int (&hits)[2][kWarps]) {
+  uint32_t top = 0, bottom = ~0u;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
-    if (first < keep) pick = first;
+  for (int i = 0; i < NW; ++i) {
+    if constexpr (kBits == 16) {
+      top = max(top, max(w[i] >> 16, w[i] & 0xFFFFu));
+      bottom = min(bottom, min(w[i] >> 16, w[i] & 0xFFFFu));
+    } else {
+      top = max(top, w[i]);
+      bottom = min(bottom, w[i]);
+    }
   }
-  return pick;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  top = __reduce_max_sync(0xffffffffu, top);
+  bottom = __reduce_min_sync(0xffffffffu, bottom);
+  if (lane == 0) {
+    hits[0][warp] = top;
+    hits[1][warp] = bottom;
+  }
+  __syncthreads();
+  const bool in = lane < static_cast<int>(blockDim.x >> 5);
+  top = __reduce_max_sync(0xffffffffu, in ? hits[0][lane] : 0u);
+  bottom = __reduce_min_sync(0xffffffffu, in ? hits[1][lane] : ~0u);
+  __syncthreads();
+  const int bits = open_bits(bottom, top);
+  uint32_t low = above_bits(top, bits);
+#pragma unroll 1
+  for (int shift = bits - 2, st = 0; shift >= 0; shift -= 2, ++st) {
+    uint32_t packed = 0;
+#pragma unroll
+    for (uint32_t t = 1; t <= 3; ++t) {
+      const uint32_t cand = low | (t << shift);
+      uint32_t n = 0;
+#pragma unroll
+      for (int i = 0; i < NW; ++i) {
+        if constexpr (kBits == 16)
+          n += (w[i] >= (cand << 16) ? 1u : 0u) + ((w[i] << 16) >= (cand << 16) ? 1u : 0u);
+        else
+          n += w[i] >= cand ? 1u : 0u;
+      }
+      packed += n << (10 * (t - 1));
+    }
+    int c1, c2, c3;
+    block_count3(packed, hits, st & 1, c1, c2, c3);
+    low |= static_cast<uint32_t>(c3 >= kk ? 3 : (c2 >= kk ? 2 : (c1 >= kk ? 1 : 0))) << shift;
+  }
+  __syncthreads();
+  return low;
+}
+
+// The same for kk <= 64 without a block-wide step per bit: the warps bring their largest keys, 128 in all,
+// and one warp searches among those. They are keys of the block, so at least kk of the block's reach the
+// result; it is the kk-th largest of all unless a warp holds more of those than it brings. With 1024 threads
+// 2.4k cycles; a block-wide step per two bits took 7.3k.
+template <int kBits, int kBlockWarps>
+__device__ __forceinline__ uint32_t kth_of_warp_tops(uint32_t w, int kk, TopkSmem& s) {
+  constexpr int kTops = kWarpTops / kBlockWarps;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t hi = w, lo = 0;
+  if constexpr (kBits == 16) {
+    hi = max(w >> 16, w & 0xFFFFu);
+    lo = min(w >> 16, w & 0xFFFFu);
+  }
+  uint32_t mine = 0;
+#pragma unroll
+  for (int r = 0; r < kTops; ++r) {
+    const uint32_t m = __reduce_max_sync(0xffffffffu, hi);
+    const int owner = __ffs(static_cast<int>(__ballot_sync(0xffffffffu, hi == m))) - 1;
+    if (lane == owner) {
+      hi = lo;
+      lo = 0;
+    }
+    if (lane == r) mine = m;
+  }
+  if (lane < kTops) s.top[warp * kTops + lane] = mine;
+  __syncthreads();
+  if (warp == 0) {
+    uint32_t v[kWarpTops / 32], top = 0, bottom = ~0u;
+#pragma unroll
+    for (int i = 0; i < kWarpTops / 32; ++i) {
+      v[i] = s.top[lane + 32 * i];
+      top = max(top, v[i]);
+      bottom = min(bottom, v[i]);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    bottom = __reduce_min_sync(0xffffffffu, bottom);
+    const int bits = open_bits(bottom, top);
+    uint32_t low = above_bits(top, bits);
+#pragma unroll 1
+    for (int bit = bits - 1; bit >= 0; --bit) {
+      const uint32_t cand = low | (1u << bit);
+      uint32_t c = 0;
+#pragma unroll
+      for (int i = 0; i < kWarpTops / 32; ++i) c += v[i] >= cand ? 1u : 0u;
+      if (__reduce_add_sync(0xffffffffu, c) >= static_cast<uint32_t>(kk)) low = cand;
+    }
+    if (lane == 0) s.bound = low;
+  }
+  __syncthreads();
+  return s.bound;
+}
+
+// A bound that at least kk of the keys in the block's words reach.
+template <int NW, int kBits, int kBlockWarps>
+__device__ __forceinline__ uint32_t bound_of(const uint32_t (&w)[NW], int kk, TopkSmem& s) {
+  if constexpr (NW == 1)
+    return kth_of_warp_tops<kBits, kBlockWarps>(w[0], kk, s);
+  else
+    return kth_key<NW, kBits>(w, kk, s.hits);
+}
+
+// s.sorted[0 .. 1023] descending, by 256 threads that hold four neighbours each: partners at distance 1
+// and 2 are in the same thread, up to 64 in the same warp (shuffles), farther ones go through shared memory.
+// Run by all threads of the block.
+__device__ __forceinline__ void sort_1024(TopkSmem& s) {
+  constexpr int kT = 256, kE = 4;
+  const int tid = threadIdx.x;
+  if (tid < kT) {
+    unsigned long long v[kE];
+#pragma unroll
+    for (int r = 0; r < kE; ++r) v[r] = s.sorted[tid * kE + r];
+    auto swap_if = [](unsigned long long& a, unsigned long long& b, bool desc) {
+      const bool sw = (a < b) == desc;
+      const unsigned long long t = sw ? b : a;
+      b = sw ? a : b;
+      a = t;
+    };
+#pragma unroll 1
+    for (int wb = 1; wb <= 10; ++wb) {
+#pragma unroll 1
+      for (int b = wb - 1; b >= 2; --b) {
+        // this thread's elements are the upper or the lower partners together
+        const bool upper = (tid * kE >> b) & 1, desc = ((tid * kE >> wb) & 1) == 0;
+        unsigned long long o[kE];
+        if (b >= 7) {
+          asm volatile("bar.sync 1, 256;" ::: "memory");      // the partners have read what the last exchange left
+#pragma unroll
+          for (int r = 0; r < kE; ++r) s.sorted[tid * kE + r] = v[r];
+          asm volatile("bar.sync 1, 256;" ::: "memory");
+          const int partner = (tid * kE) ^ (1 << b);
+#pragma unroll
+          for (int r = 0; r < kE; ++r) o[r] = s.sorted[partner + r];
+        } else {
+#pragma unroll
+          for (int r = 0; r < kE; ++r) o[r] = __shfl_xor_sync(0xffffffffu, v[r], 1 << (b - 2));
+        }
+#pragma unroll
+        for (int r = 0; r < kE; ++r) {
+          const bool larger = v[r] > o[r];
+          v[r] = larger == (upper != desc) ? v[r] : o[r];
+        }
+      }
+      const bool desc = ((tid * kE >> wb) & 1) == 0;
+      if (wb >= 2) {
+        swap_if(v[0], v[2], desc);
+        swap_if(v[1], v[3], desc);
+      }
+      swap_if(v[0], v[1], wb == 1 ? true : desc);
+      swap_if(v[2], v[3], wb == 1 ? false : desc);
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+#pragma unroll
+    for (int r = 0; r < kE; ++r) s.sorted[tid * kE + r] = v[r];
+  }
+  __syncthreads();
 }
 
 constexpr int kTopkThreads = 512;
@@ -248,39 +444,119 @@ __device__ __forceinline__ T from_bits16(uint32_t h) {
   return *reinterpret_cast<const T*>(&us);
 }
 
-// Second half of the top-k path, shared by the one-CTA and the cluster kernel: n_cand candidates
-// sit in s.cand_key / s.cand_idx (in any order; if there are more than the buffer holds the row
-// is searched exactly), the kk largest by (key desc, id asc) are the survivors; masses, top-p
-// and the draw follow. Run by all threads of one CTA.
+// The words a thread's largest elements are kept in: one up to this k, four for a larger one, so that the
+// number of maxima stays well above k (with as many maxima as k the bound would be the smallest of them and
+// the row's exact search the rule: k = 1000 took 334 us for 1 row of 128256 and 1365 us for 256, with four
+// words 33 and 59 us). Up to it the bound comes from what the warps bring (kth_of_warp_tops).
+constexpr int kFewK = 64;
+constexpr int kRankSort = 512;   // candidates that are sorted by counting
+
+// Key of an element given as the low bits of a register word.
 template <typename T>
-__device__ __forceinline__ void topk_finish(TopkSmem& s, int n_cand, const T* __restrict__ rp, int v, bool vec_ok,
-                                            int kk, float inv_temp, float top_p, unsigned long long seed,
-                                            unsigned long long step, const long long* __restrict__ row_ids, int row,
-                                            int* __restrict__ out) {
-  const int tid = threadIdx.x;
+__device__ __forceinline__ uint32_t key_of_bits(uint32_t bits) {
+  if constexpr (Elem<T>::kPacked)
+    return float_to_key(Elem<T>::to_float(from_bits16<T>(bits & 0xFFFFu)));
+  else
+    return float_to_key(__uint_as_float(bits));
+}
+
+// A bound on keys in the two forms the collection uses: `thr` (the same number, in every half of a word) for
+// a quick look at a vector's maximum, `low` for the exact comparison of a 32-bit key. A bound below -inf's
+// key means that NaNs qualify as well, so the quick look must let everything through.
+template <typename T>
+struct Bound {
+  uint32_t low, thr;
+  bool all;
+  __device__ __forceinline__ explicit Bound(uint32_t k) {   // k: the leading 16 bits of the key, or all 32
+    if constexpr (Elem<T>::kPacked) {
+      const uint32_t bits = (k & 0x8000u) ? (k & 0x7FFFu) : (~k & 0xFFFFu);
+      thr = bits * 0x00010001u;
+      all = k <= (~(Elem<T>::kInf2 | 0x8000u) & 0xFFFFu);
+      low = all && k == 0 ? 0u : float_to_key(Elem<T>::to_float(from_bits16<T>(bits)));
+    } else {
+      thr = __float_as_uint(key_to_float(k));
+      all = k <= ~0xFF800000u;
+      low = k;
+    }
+  }
+  __device__ __forceinline__ bool maybe(uint32_t word) const { return all || Elem<T>::any_ge(word, thr); }
+};
+
+// Keys of a thread's maxima, in place: two 16-bit keys per word, or one of 32 bits.
+template <typename T, int NW>
+__device__ __forceinline__ void words_to_keys(uint32_t (&w)[NW]) {
+#pragma unroll
+  for (int i = 0; i < NW; ++i) {
+    if constexpr (Elem<T>::kPacked)
+      w[i] = key16x2<T>(w[i]);
+    else
+      w[i] = float_to_key(__uint_as_float(w[i]));
+  }
+}
+
+// Calls f(key, idx) for the elements of `raw` that reach the bound; vector u's first element is token
+// i0 + u * step, vectors from n on are left out. Hits are rare, so a thread first notes which of its vectors
+// have one; the code behind that exists once and runs as often as the busiest lane has hits, not once per
+// vector (straight-line code that runs once per launch costs instruction fetches).
+template <typename T, int N, typename F>
+__device__ __forceinline__ void visit_hits(const uint4 (&raw)[N], int n, int i0, int step, const Bound<T>& b, F&& f) {
+  constexpr int kVec = Elem<T>::kVec;
+  uint32_t vecs = 0;
+#pragma unroll
+  for (int u = 0; u < N; ++u) vecs |= (u < n && b.maybe(vec_max<T>(raw[u])) ? 1u : 0u) << u;
+  while (vecs) {
+    const int u = __ffs(static_cast<int>(vecs)) - 1;
+    vecs &= vecs - 1;
+    uint4 r = raw[0];
+#pragma unroll
+    for (int x = 1; x < N; ++x) r = u == x ? raw[x] : r;
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+    uint32_t elems = 0;
+#pragma unroll
+    for (int j = 0; j < kVec; ++j)
+      elems |= (key_of_bits<T>(Elem<T>::kPacked ? w[j / 2] >> (16 * (j & 1)) : w[j & 3]) >= b.low ? 1u : 0u) << j;
+    while (elems) {
+      const int j = __ffs(static_cast<int>(elems)) - 1;
+      elems &= elems - 1;
+      const int wi = Elem<T>::kPacked ? j >> 1 : j;
+      const uint32_t word = wi == 0 ? w[0] : (wi == 1 ? w[1] : (wi == 2 ? w[2] : w[3]));
+      f(key_of_bits<T>(Elem<T>::kPacked ? word >> (16 * (j & 1)) : word), i0 + u * step + j);
+    }
+  }
+}
+
+// Second half of the top-k path, shared by the one-CTA and the cluster kernel: n_cand candidates
+// sit in s.cand (in any order; if there are more than the buffer holds the row is searched
+// exactly), the kk largest by (key desc, id asc) are the survivors; masses, top-p and the draw
+// follow. Run by all threads of one CTA. Few candidates are ranked by counting; from many the kk
+// largest are selected by a bit search and sorted by a bitonic network (counting grows with the square:
+// the 2100 candidates of k = 1000 in two parts of a row took 300 us that way, 12 us now).
+template <typename T>
+__device__ __forceinline__ void topk_finish(TopkSmem& s, int n_cand, const T* __restrict__ rp, int v, int kk,
+                                            float inv_temp, float top_p, uint32_t u24, int row, int* __restrict__ out) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nt = blockDim.x;
+  constexpr int kLow = Elem<T>::kLowBit;
   if (n_cand > kCandCap) {
     // ---- rare: more ties / near-ties than the candidate buffer holds. Exact radix select by
     // counting passes, then an index-ordered pick among the ties at the threshold.
     uint32_t tau = 0;
-    for (int bit = 31; bit >= 0; --bit) {
+    for (int bit = 31; bit >= kLow; --bit) {
       const uint32_t cand = tau | (1u << bit);
       int local = 0;
-      for_each_key<T>(rp, v, vec_ok, [&](uint32_t key, int) { local += (key >= cand) ? 1 : 0; });
+      for_each_key<T>(rp, v, [&](uint32_t key, int) { local += (key >= cand) ? 1 : 0; });
       if (block_sum_int(local, s.red) >= kk) tau = cand;
     }
+    // the low bits of a widened 16-bit value's key are ones below zero (and 0 is NaN's key)
+    if (tau != 0 && !(tau & 0x80000000u)) tau |= (1u << kLow) - 1u;
     int local_gt = 0;
-    for_each_key<T>(rp, v, vec_ok, [&](uint32_t key, int) { local_gt += (key > tau) ? 1 : 0; });
+    for_each_key<T>(rp, v, [&](uint32_t key, int) { local_gt += (key > tau) ? 1 : 0; });
     const int n_gt = block_sum_int(local_gt, s.red);
     const int quota = kk - n_gt;
     if (tid == 0) s.count = 0;
     __syncthreads();
-    for_each_key<T>(rp, v, vec_ok, [&](uint32_t key, int i) {
-      if (key > tau) {
-        const int slot = atomicAdd(&s.count, 1);
-        s.cand_key[slot] = key;
-        s.cand_idx[slot] = static_cast<uint32_t>(i);
-      }
+    for_each_key<T>(rp, v, [&](uint32_t key, int i) {
+      if (key > tau) s.cand[atomicAdd(&s.count, 1)] = cand_of(key, i);
     });
     __syncthreads();
     unsigned long long tie_base = 0;
@@ -297,10 +573,7 @@ __device__ __forceinline__ void topk_finish(TopkSmem& s, int n_cand, const T* __
       for (int j = 0; j < kPer; ++j) {
         const int i = i0 + j;
         if (i < v && float_to_key(Elem<T>::to_float(rp[i])) == tau) {
-          if (off < static_cast<unsigned long long>(quota)) {
-            s.cand_key[n_gt + off] = tau;
-            s.cand_idx[n_gt + off] = static_cast<uint32_t>(i);
-          }
+          if (off < static_cast<unsigned long long>(quota)) s.cand[n_gt + off] = cand_of(tau, i);
           ++off;
         }
       }
@@ -310,166 +583,245 @@ __device__ __forceinline__ void topk_finish(TopkSmem& s, int n_cand, const T* __
     n_cand = kk;
   }
 
-  // ---- rank sort of the candidates by (key desc, id asc); the first kk are the survivors
-  for (int i = tid; i < n_cand; i += nt) {
-    const uint32_t ki = s.cand_key[i], ii = s.cand_idx[i];
-    int rank = 0;
-    for (int j = 0; j < n_cand; ++j) {
-      const uint32_t kj = s.cand_key[j], ij = s.cand_idx[j];
-      rank += (kj > ki || (kj == ki && ij < ii)) ? 1 : 0;
+  // ---- the kk survivors, sorted by (key desc, id asc)
+  if (n_cand <= kRankSort) {
+    // eight lanes count for one candidate
+    for (int i0 = 0; i0 < n_cand; i0 += nt >> 3) {
+      const int i = i0 + (tid >> 3);
+      const unsigned long long mine = i < n_cand ? s.cand[i] : ~0ull;
+      uint32_t rank = 0;
+#pragma unroll 4
+      for (int j = tid & 7; j < n_cand; j += 8) rank += s.cand[j] > mine ? 1u : 0u;
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
+      if ((tid & 7) == 0 && i < n_cand && rank < static_cast<uint32_t>(kk)) s.sorted[rank] = mine;
     }
-    if (rank < kk) {
-      s.sorted_key[rank] = ki;
-      s.sorted_idx[rank] = ii;
+    __syncthreads();
+  } else {
+    // the kk-th largest key (its leading bits name it), then the kk-th largest (key, ~id) among its ties;
+    // a warp counts at most 32 * 20 candidates, which fits the fields of block_count3
+    static_assert(kCandCap <= 20 * 512, "counts per warp");
+    constexpr uint32_t kMask = ~((1u << (kLow & ~1)) - 1u);
+    uint32_t top = 0, bottom = ~0u;
+    for (int i = tid; i < n_cand; i += nt) {
+      const uint32_t key = static_cast<uint32_t>(s.cand[i] >> 32);
+      top = max(top, key);
+      bottom = min(bottom, key);
     }
+    top = __reduce_max_sync(0xffffffffu, top);
+    bottom = __reduce_min_sync(0xffffffffu, bottom);
+    if (lane == 0) {
+      s.hits[0][warp] = top;
+      s.hits[1][warp] = bottom;
+    }
+    if (tid == 0) s.n_sorted = s.n_ties = 0;
+    __syncthreads();
+    top = __reduce_max_sync(0xffffffffu, lane < nt >> 5 ? s.hits[0][lane] : 0u);
+    bottom = __reduce_min_sync(0xffffffffu, lane < nt >> 5 ? s.hits[1][lane] : ~0u);
+    __syncthreads();
+    const int bits = open_bits(bottom, top);
+    int c1, c2, c3, st = 0;
+    uint32_t tau = above_bits(top, bits) & kMask;
+    for (int bit = bits - 2; bit >= (kLow & ~1); bit -= 2, ++st) {
+      uint32_t packed = 0;
+      for (int i = tid; i < n_cand; i += nt) {
+        const uint32_t key = static_cast<uint32_t>(s.cand[i] >> 32);
+        packed += (key >= (tau | (1u << bit)) ? 1u : 0u) + (key >= (tau | (2u << bit)) ? 1u << 10 : 0u) +
+                  (key >= (tau | (3u << bit)) ? 1u << 20 : 0u);
+      }
+      block_count3(packed, s.hits, st & 1, c1, c2, c3);
+      tau |= static_cast<uint32_t>(c3 >= kk ? 3 : (c2 >= kk ? 2 : (c1 >= kk ? 1 : 0))) << bit;
+    }
+    // ---- what is above it survives, its ties go to a list of their own
+    constexpr int kTieCap = kMaxTopK;            // in s.mass, which is not in use yet
+    for (int i = tid; i < n_cand; i += nt) {
+      const unsigned long long c = s.cand[i];
+      const uint32_t key = static_cast<uint32_t>(c >> 32) & kMask;
+      if (key > tau) s.sorted[atomicAdd(&s.n_sorted, 1)] = c;
+      if (key == tau) {
+        const int slot = atomicAdd(&s.n_ties, 1);
+        if (slot < kTieCap) s.mass[slot] = c;
+      }
+    }
+    __syncthreads();
+    const int n_gt = s.n_sorted, n_ties = s.n_ties, quota = kk - n_gt;   // ties that survive: the smallest ids
+    if (n_ties <= kTieCap) {
+      for (int i = warp; i < n_ties; i += nt >> 5) {
+        const unsigned long long mine = s.mass[i];
+        uint32_t rank = 0;
+        for (int j = lane; j < n_ties; j += 32) rank += s.mass[j] > mine ? 1u : 0u;
+        rank = __reduce_add_sync(0xffffffffu, rank);
+        if (lane == 0 && rank < static_cast<uint32_t>(quota)) s.sorted[n_gt + rank] = mine;
+      }
+    } else {
+      uint32_t tie = 0;                          // the smallest ~id among those that survive
+      const int top_bit = (31 - __clz(v)) & ~1;
+      const uint32_t id_mask = top_bit == 30 ? ~0u : (4u << top_bit) - 1u;
+      for (int bit = top_bit; bit >= 0; bit -= 2, ++st) {
+        uint32_t packed = 0;
+        for (int i = tid; i < n_cand; i += nt) {
+          const unsigned long long c = s.cand[i];
+          if ((static_cast<uint32_t>(c >> 32) & kMask) != tau) continue;
+          const uint32_t id = static_cast<uint32_t>(c) & id_mask;
+          packed += (id >= (tie | (1u << bit)) ? 1u : 0u) + (id >= (tie | (2u << bit)) ? 1u << 10 : 0u) +
+                    (id >= (tie | (3u << bit)) ? 1u << 20 : 0u);
+        }
+        block_count3(packed, s.hits, st & 1, c1, c2, c3);
+        tie |= static_cast<uint32_t>(c3 >= quota ? 3 : (c2 >= quota ? 2 : (c1 >= quota ? 1 : 0))) << bit;
+      }
+      tie |= ~id_mask;
+      for (int i = tid; i < n_cand; i += nt) {
+        const unsigned long long c = s.cand[i];
+        if ((static_cast<uint32_t>(c >> 32) & kMask) == tau && static_cast<uint32_t>(c) >= tie)
+          s.sorted[atomicAdd(&s.n_sorted, 1)] = c;
+      }
+    }
+    for (int i = kk + tid; i < kMaxTopK; i += nt) s.sorted[i] = 0;   // sorts behind every candidate
+    __syncthreads();
+    sort_1024(s);
   }
-  __syncthreads();
 
   // ---- masses, top-p, draw
-  const float y0 = mul_rn(key_to_float(s.sorted_key[0]), inv_temp);
-  for (int i = tid; i < kk; i += nt) {
-    const float y = mul_rn(key_to_float(s.sorted_key[i]), inv_temp);
-    s.mass[i] = mass_fixed(exp_det(sub_rn(y, y0)));
+  auto key_at = [&](int i) { return static_cast<uint32_t>(s.sorted[i] >> 32); };
+  const float y0 = mul_rn(key_to_float(key_at(0)), inv_temp);
+  auto mass_at = [&](int i) {
+    return static_cast<unsigned long long>(mass_fixed(exp_det(sub_rn(mul_rn(key_to_float(key_at(i)), inv_temp), y0))));
+  };
+  int pos = 0;
+  if (kk <= 64) {
+    // one warp does it all
+    if (warp != 0) return;
+    const int i = 2 * lane;
+    pos = pick_sorted_warp(i < kk ? mass_at(i) : 0ull, i + 1 < kk ? mass_at(i + 1) : 0ull, kk, top_p, u24);
+  } else {
+    // thread t owns the survivors [t * per, t * per + per), per is 1 or 2
+    const int per = (kk + nt - 1) / nt, i0 = tid * per;
+    const unsigned long long q0 = i0 < kk ? mass_at(i0) : 0ull, q1 = per == 2 && i0 + 1 < kk ? mass_at(i0 + 1) : 0ull;
+    if (tid == 0) {
+      s.keep = kk;
+      s.pick = -1;
+    }
+    unsigned long long z;
+    const unsigned long long before = block_exscan_u64(q0 + q1, s.scan, z);
+    if (top_p < 1.0f) {
+      // keep = first i > 0 with (mass before i) > limit
+      const unsigned long long limit = mass_fraction(static_cast<double>(top_p), z);
+      int first = kk;
+      if (i0 > 0 && i0 < kk && before > limit)
+        first = i0;
+      else if (per == 2 && i0 + 1 < kk && before + q0 > limit)
+        first = i0 + 1;
+      first = __reduce_min_sync(0xffffffffu, first);
+      if (lane == 0 && first < kk) atomicMin(&s.keep, first);
+      __syncthreads();
+    }
+    const int keep = s.keep;
+    if (i0 < keep && i0 + per >= keep) s.kept_mass = before + q0 + (i0 + 1 < keep ? q1 : 0ull);
+    __syncthreads();
+    const unsigned long long target = mass_scale_u24(u24, s.kept_mass);
+    if (i0 < keep && before <= target && before + q0 > target)
+      s.pick = i0;
+    else if (per == 2 && i0 + 1 < keep && before + q0 <= target && before + q0 + q1 > target)
+      s.pick = i0 + 1;
+    __syncthreads();
+    pos = s.pick < 0 ? keep - 1 : s.pick;
   }
-  __syncthreads();
-  if (tid < 32) {
-    const unsigned long long rid = row_ids ? static_cast<unsigned long long>(row_ids[row])
-                                           : static_cast<unsigned long long>(row);
-    const int pos = pick_sorted_warp(s.mass, kk, top_p, uniform_u24(seed, rid, step));
-    if (tid == 0) out[row] = static_cast<int>(s.sorted_idx[pos]);
-  }
+  if (tid == 0) out[row] = static_cast<int>(~static_cast<uint32_t>(s.sorted[pos]));
 }
 
-template <typename T>
+// One CTA per row, two passes: the first (HBM) finds a bound that at least kk elements reach, the second (L2)
+// collects the elements that do. Each thread keeps the largest elements of NW groups of the row in NW words
+// as they were loaded (packed maxima: one instruction per two 16-bit elements); the kk-th largest of the
+// block's maxima bounds the kk-th largest element from below. Bound by the two passes: bf16 [256, 128256],
+// k = 50, 33 us (49 us with the keys of all elements computed); fp32 [256, 128256] 66 us (70 us), 128255
+// columns 76 us (255 us when rows off a 16-byte boundary were read by scalars).
+template <typename T, int NW>
 __global__ void __launch_bounds__(kTopkThreads, 2)
 sample_topk_kernel(const T* __restrict__ logits, long long row_stride, int v, const long long* __restrict__ row_ids,
                    float inv_temp, int top_k, float top_p, unsigned long long seed, unsigned long long step,
                    int* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TopkSmem& s = *reinterpret_cast<TopkSmem*>(smem_raw);
+  constexpr int kVec = Elem<T>::kVec, nt = kTopkThreads;
+  constexpr int kU = 8;                       // 16-byte loads in flight per thread
+  static_assert(kU % NW == 0, "every word gets its share of a batch");
   const int tid = threadIdx.x;
-  const int nt = blockDim.x;
   const int row = blockIdx.x;
   const T* rp = logits + static_cast<long long>(row) * row_stride;
-  const bool vec_ok = (reinterpret_cast<uintptr_t>(rp) & 15u) == 0;
   const int kk = min(min(top_k, kMaxTopK), v);
-  uint32_t lower = 0;  // 32-bit key: at least kk elements of the row are >= lower
-
+  const int head = row_head(rp, v), nvec = (v - head) / kVec, scal = v - nvec * kVec;
+  const uint4* vp = reinterpret_cast<const uint4*>(rp + head);
+  const int scal_idx = tid < head ? tid : nvec * kVec + tid;     // thread's scalar element, if tid < scal
+  uint32_t scal_word = ~0u;                                      // NaN
+  if (tid < scal) {
+    if constexpr (Elem<T>::kPacked)
+      scal_word = 0xFFFF0000u | reinterpret_cast<const unsigned short*>(rp)[scal_idx];
+    else
+      scal_word = __float_as_uint(rp[scal_idx]);
+  }
   if (tid == 0) s.count = 0;
-  if constexpr (Elem<T>::kPacked) {
-    // ---- 16-bit inputs: keys stay packed two per register. Each thread keeps two running
-    // maxima (even / odd elements), 1024 in all; the kk-th largest of them bounds the kk-th
-    // largest element of the row from below.
-    uint32_t tm2 = 0;
-    const int nvec = vec_ok ? v / 8 : 0;
-    const uint4* vp = reinterpret_cast<const uint4*>(rp);
-    // eight independent 16-byte loads in flight per thread: the row is latency-, not
-    // bandwidth-bound when a single CTA pulls it
-    constexpr int kU = 8;
-    int i = tid;
-    for (; i + (kU - 1) * nt < nvec; i += kU * nt) {
-      uint4 raw[kU];
+  uint32_t mx[NW];
 #pragma unroll
-      for (int u = 0; u < kU; ++u) raw[u] = __ldg(vp + i + u * nt);
+  for (int i = 0; i < NW; ++i) mx[i] = ~0u;
+  mx[0] = scal_word;
+  for (int i = tid; i < nvec; i += kU * nt) {
+    uint4 raw[kU];
 #pragma unroll
-      for (int u = 0; u < kU; ++u)
-        tm2 = __vmaxu2(tm2, __vmaxu2(__vmaxu2(key16x2<T>(raw[u].x), key16x2<T>(raw[u].y)),
-                                     __vmaxu2(key16x2<T>(raw[u].z), key16x2<T>(raw[u].w))));
-    }
-    for (; i < nvec; i += nt) {
-      const uint4 raw = __ldg(vp + i);
-      tm2 = __vmaxu2(tm2, __vmaxu2(__vmaxu2(key16x2<T>(raw.x), key16x2<T>(raw.y)),
-                                   __vmaxu2(key16x2<T>(raw.z), key16x2<T>(raw.w))));
-    }
-    const unsigned short* hp = reinterpret_cast<const unsigned short*>(rp);
-    for (int t = nvec * 8 + tid; t < v; t += nt) tm2 = __vmaxu2(tm2, key16x2<T>(hp[t]) & 0xFFFFu);
-    const uint32_t m_lo = tm2 & 0xFFFFu, m_hi = tm2 >> 16;
-    uint32_t low16 = 0;
-    for (int bit = 15; bit >= 0; --bit) {
-      const uint32_t cand = low16 | (1u << bit);
-      const int cnt = __syncthreads_count(m_lo >= cand) + __syncthreads_count(m_hi >= cand);
-      if (cnt >= kk) low16 = cand;
-    }
-    // ---- pass 2 (L2): collect every element whose 16-bit key is >= the bound
-    const uint32_t low2 = low16 * 0x00010001u;
-    auto push = [&](uint32_t bits16, int idx) {
-      const int slot = atomicAdd(&s.count, 1);
-      if (slot < kCandCap) {
-        s.cand_key[slot] = float_to_key(Elem<T>::to_float(from_bits16<T>(bits16)));
-        s.cand_idx[slot] = static_cast<uint32_t>(idx);
-      }
-    };
-    auto scan_vec = [&](const uint4& raw, int vi) {
-      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-      const uint32_t h0 = __vcmpgeu2(key16x2<T>(w[0]), low2), h1 = __vcmpgeu2(key16x2<T>(w[1]), low2);
-      const uint32_t h2 = __vcmpgeu2(key16x2<T>(w[2]), low2), h3 = __vcmpgeu2(key16x2<T>(w[3]), low2);
-      if ((h0 | h1 | h2 | h3) == 0u) return;
-      const uint32_t hit[4] = {h0, h1, h2, h3};
+    for (int u = 0; u < kU; ++u) raw[u] = i + u * nt < nvec ? __ldg(vp + i + u * nt) : make_uint4(~0u, ~0u, ~0u, ~0u);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (hit[j] & 0xFFFFu) push(w[j] & 0xFFFFu, vi * 8 + 2 * j);
-        if (hit[j] >> 16) push(w[j] >> 16, vi * 8 + 2 * j + 1);
-      }
-    };
-    i = tid;
-    for (; i + (kU - 1) * nt < nvec; i += kU * nt) {
-      uint4 raw[kU];
+    for (int u = 0; u < kU; ++u) mx[u % NW] = Elem<T>::wmax(mx[u % NW], vec_max<T>(raw[u]));
+  }
+  const unsigned long long rid = row_ids ? static_cast<unsigned long long>(row_ids[row])
+                                         : static_cast<unsigned long long>(row);
+  const uint32_t u24 = uniform_u24(seed, rid, step);
+  words_to_keys<T>(mx);
+  const Bound<T> bound(bound_of<NW, Elem<T>::kPacked ? 16 : 32, kTopkThreads / 32>(mx, kk, s));
+  auto push = [&](uint32_t key, int idx) {
+    const int slot = atomicAdd(&s.count, 1);
+    if (slot < kCandCap) s.cand[slot] = cand_of(key, idx);
+  };
+  for (int i = tid; i < nvec; i += kU * nt) {
+    uint4 raw[kU];
 #pragma unroll
-      for (int u = 0; u < kU; ++u) raw[u] = __ldg(vp + i + u * nt);
-#pragma unroll
-      for (int u = 0; u < kU; ++u) scan_vec(raw[u], i + u * nt);
-    }
-    for (; i < nvec; i += nt) scan_vec(__ldg(vp + i), i);
-    for (int t = nvec * 8 + tid; t < v; t += nt)
-      if ((key16x2<T>(hp[t]) & 0xFFFFu) >= low16) push(hp[t], t);
-  } else {
-    // ---- 32-bit inputs
-    uint32_t tm[2] = {0, 0};
-    for_each_key<T>(rp, v, vec_ok, [&](uint32_t key, int i) { tm[i & 1] = max(tm[i & 1], key); });
-    for (int bit = 31; bit >= Elem<T>::kLowBit; --bit) {
-      const uint32_t cand = lower | (1u << bit);
-      const int cnt = __syncthreads_count(tm[0] >= cand) + __syncthreads_count(tm[1] >= cand);
-      if (cnt >= kk) lower = cand;
-    }
-    for_each_key<T>(rp, v, vec_ok, [&](uint32_t key, int i) {
-      if (key >= lower) {
-        const int slot = atomicAdd(&s.count, 1);
-        if (slot < kCandCap) {
-          s.cand_key[slot] = key;
-          s.cand_idx[slot] = static_cast<uint32_t>(i);
-        }
-      }
-    });
+    for (int u = 0; u < kU; ++u) raw[u] = i + u * nt < nvec ? __ldg(vp + i + u * nt) : make_uint4(~0u, ~0u, ~0u, ~0u);
+    visit_hits<T>(raw, (nvec - i + nt - 1) / nt, head + i * kVec, nt * kVec, bound, push);
+  }
+  if (tid < scal) {
+    const uint32_t key = key_of_bits<T>(scal_word);
+    if (key >= bound.low) push(key, scal_idx);
   }
   __syncthreads();
-  int n_cand = s.count;
+  const int n_cand = s.count;
   __syncthreads();
 
-  topk_finish<T>(s, n_cand, rp, v, vec_ok, kk, inv_temp, top_p, seed, step, row_ids, row, out);
+  topk_finish<T>(s, n_cand, rp, v, kk, inv_temp, top_p, u24, row, out);
 }
 
 // ------------------------------------------------------------------------------------------
-// Top-k kernel for aligned rows of 16-bit logits that fit the registers of a few SMs: a cluster of
+// Top-k kernel for rows of 16-bit logits that fit the registers of a few SMs: a cluster of
 // C CTAs (1, 2 or 4) shares a row, every thread requests its whole part (eight 16-byte vectors) at
 // once and keeps it, so the row is read once and the collection costs no second pass. One CTA
-// with eight loads per thread and step needed five round trips to memory and the same again to L2.
+// with eight loads per thread and step needs several round trips to memory and the same again to L2.
 //   1. CTA r keeps its 1/C of the row and finds, as above, a bound that at least kk of its own
-//      elements reach. The largest of the C bounds is valid for the whole row: the part that
-//      produced it alone holds kk elements at or above it.
-//   2. The bounds travel through distributed shared memory (one store per peer, one cluster
-//      barrier); every CTA collects the elements of its part that reach the common bound.
-//   3. Counts are exchanged the same way, every CTA copies its candidates into CTA 0's list at
-//      its offset (remote shared-memory stores), and CTA 0 finishes as the one-CTA kernel does.
+//      elements reach. For a large k the bounds are exchanged through distributed shared memory and the
+//      largest serves the whole row (the part that produced it alone holds kk elements at or above it);
+//      for a small one the few more candidates cost less than the exchange.
+//   2. Every CTA collects the elements of its part that reach its bound; the others store theirs into
+//      CTA 0's shared memory and leave, CTA 0 waits at the cluster barrier and finishes as the one-CTA
+//      kernel does.
 // The survivors are the kk largest by (key desc, id asc) of a candidate set that contains them
 // all, so the token is the one the one-CTA kernel and the CPU library return. No multicast.
-// Measured (bf16 [64, 128256], k = 50, top_p = 0.9): 16.6 us, one CTA per row 22.5 us.
+// What bounds it is the chain, 18.5k cycles for bf16 [64, 128256], k = 50: load of the row 6.3k, bound 2.4k,
+// collection 1.5k, exchange 4.2k, sort 2.1k, masses and draw 1.4k (27.3k before: bound 7.4k, sort 3.6k, draw
+// 3.4k; 22.6 us a call then, 16.4 us now, the L2 flushed before each). Packed 16-bit maxima and comparisons
+// look at a vector in five instructions instead of about eighty, and rows may start anywhere: what lies
+// before the first 16-byte boundary is read as scalars (128255 columns, 64 rows: 72 us scalar, 16.4 us now).
 // ------------------------------------------------------------------------------------------
 constexpr int kMaxCluster = 4;
 
 struct ClusterXchg {
   uint32_t low[kMaxCluster];   // bound found by each CTA of the cluster
-  int cnt[kMaxCluster];        // candidates collected by each CTA
-  int hits[8][3];              // bound search: counts of a step's three thresholds
+  int cnt[kMaxCluster];        // candidates collected by each CTA (CTA 0's copy)
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -485,134 +837,113 @@ __device__ __forceinline__ uint32_t map_to_cta(const void* p, uint32_t rank) {
 __device__ __forceinline__ void st_remote_u32(uint32_t cluster_addr, uint32_t v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+__device__ __forceinline__ void st_remote_u64(uint32_t cluster_addr, unsigned long long v) {
+  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(cluster_addr), "l"(v) : "memory");
 }
+__device__ __forceinline__ int atom_add_remote(uint32_t cluster_addr, int v) {
+  int r;
+  asm volatile("atom.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(r) : "r"(cluster_addr), "r"(v) : "memory");
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive_release() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_acquire() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
 constexpr int kHeldThreads = 1024;
 constexpr int kHeldVecs = 8;                                          // 16-byte vectors a thread keeps
 constexpr int kHeldElems = kHeldThreads * kHeldVecs * 8;              // 16-bit elements a CTA keeps
 
-template <typename T, int C>
+template <typename T, int C, int NW>
 __global__ void __launch_bounds__(kHeldThreads, 1)
 sample_topk_held_kernel(const T* __restrict__ logits, long long row_stride, int v,
                         const long long* __restrict__ row_ids, float inv_temp, int top_k, float top_p,
                         unsigned long long seed, unsigned long long step, int* __restrict__ out) {
   static_assert(Elem<T>::kPacked, "the kernel takes 16-bit logits");
+  static_assert(kHeldVecs % NW == 0, "every word gets its share of the vectors");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TopkSmem& s = *reinterpret_cast<TopkSmem*>(smem_raw);
   ClusterXchg& x = *reinterpret_cast<ClusterXchg*>(smem_raw + sizeof(TopkSmem));
-  const int tid = threadIdx.x, lane = tid & 31;
+  const int tid = threadIdx.x;
   const int row = blockIdx.x / C;
   const int cr = C == 1 ? 0 : static_cast<int>(cluster_rank());
-  const T* rp = logits + static_cast<long long>(row) * row_stride;  // 16-byte aligned (checked by the host)
+  const T* rp = logits + static_cast<long long>(row) * row_stride;
   const int kk = min(min(top_k, kMaxTopK), v);
-  if constexpr (C > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");   // waited for before the first remote store
+  if (tid == 0) s.count = 0;
+  if constexpr (C > 1) cluster_arrive_release();   // waited for before the first remote access
 
-  // ---- this CTA's part: vectors [v0, v1) of the row, the scalar tail goes to the last CTA
-  const int nvec = v / 8;
+  // ---- this CTA's part: vectors [v0, v1) of the row, the scalars at its ends go to the last CTA
+  const int head = row_head(rp, v), nvec = (v - head) / 8, scal = v - nvec * 8;
   const int v0 = static_cast<int>(static_cast<long long>(nvec) * cr / C);
   const int v1 = static_cast<int>(static_cast<long long>(nvec) * (cr + 1) / C);
-  const unsigned short* hp = reinterpret_cast<const unsigned short*>(rp);
-  const int tail = nvec * 8 + tid;                                    // at most seven elements
-  const bool has_tail = cr == C - 1 && tail < v;
-  const uint4* mine_p = reinterpret_cast<const uint4*>(rp) + v0 + tid;   // this thread's vectors, kHeldThreads apart
+  const uint4* mine_p = reinterpret_cast<const uint4*>(rp + head) + v0 + tid;   // this thread's vectors, kHeldThreads apart
   const int left = v1 - v0 - tid;
   uint4 raw[kHeldVecs];
 #pragma unroll
   for (int u = 0; u < kHeldVecs; ++u)
     raw[u] = u * kHeldThreads < left ? __ldg(mine_p + u * kHeldThreads) : make_uint4(~0u, ~0u, ~0u, ~0u);   // NaN: key 0
-  const uint32_t tail_bits = has_tail ? hp[tail] : 0xFFFFu;
-  if (tid == 0) s.count = 0;
-  if (tid < 24) x.hits[tid / 3][tid % 3] = 0;
-  __syncthreads();
-  uint32_t tm2 = key16x2<T>(tail_bits | 0xFFFF0000u);
+  const bool has_scal = cr == C - 1 && tid < scal;
+  const int scal_idx = tid < head ? tid : nvec * 8 + tid;
+  const uint32_t scal_word = 0xFFFF0000u | (has_scal ? reinterpret_cast<const unsigned short*>(rp)[scal_idx] : 0xFFFFu);
+  const unsigned long long rid = row_ids ? static_cast<unsigned long long>(row_ids[row])
+                                         : static_cast<unsigned long long>(row);
+  const uint32_t u24 = uniform_u24(seed, rid, step);   // while the loads are under way
+  uint32_t mx[NW];
 #pragma unroll
-  for (int u = 0; u < kHeldVecs; ++u)
-    tm2 = __vmaxu2(tm2, __vmaxu2(__vmaxu2(key16x2<T>(raw[u].x), key16x2<T>(raw[u].y)),
-                                 __vmaxu2(key16x2<T>(raw[u].z), key16x2<T>(raw[u].w))));
-  // ---- the kk-th largest of the 2048 maxima, two bits of it per step: counts for the three
-  // thresholds, packed per warp (at most 64 each), one barrier
-  const uint32_t m_lo = tm2 & 0xFFFFu, m_hi = tm2 >> 16;
-  uint32_t low16 = 0;
-#pragma unroll 1
-  for (int st = 0; st < 8; ++st) {
-    const int shift = 14 - 2 * st;
-    uint32_t packed = 0;
+  for (int i = 0; i < NW; ++i) mx[i] = i == 0 ? scal_word : ~0u;
 #pragma unroll
-    for (uint32_t t = 1; t <= 3; ++t) {
-      const uint32_t cand = low16 | (t << shift);
-      packed += ((m_lo >= cand ? 1u : 0u) + (m_hi >= cand ? 1u : 0u)) << (10 * (t - 1));
-    }
-    packed = __reduce_add_sync(0xffffffffu, packed);
-    if (lane < 3) atomicAdd(&x.hits[st][lane], static_cast<int>((packed >> (10 * lane)) & 1023u));
-    __syncthreads();
-    const int c1 = x.hits[st][0], c2 = x.hits[st][1], c3 = x.hits[st][2];
-    low16 |= static_cast<uint32_t>(c3 >= kk ? 3 : (c2 >= kk ? 2 : (c1 >= kk ? 1 : 0))) << shift;
-  }
+  for (int u = 0; u < kHeldVecs; ++u) mx[u % NW] = Elem<T>::wmax(mx[u % NW], vec_max<T>(raw[u]));
+  words_to_keys<T>(mx);
+  uint32_t low16 = bound_of<NW, 16, kHeldThreads / 32>(mx, kk, s);
   if constexpr (C > 1) {
-    // ---- the largest of the C bounds serves the whole row
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");      // every CTA of the cluster runs
-    if (tid < C) st_remote_u32(map_to_cta(&x.low[cr], static_cast<uint32_t>(tid)), low16);
-    cluster_sync_all();
+    cluster_wait_acquire();                            // every CTA of the cluster runs, its counter is zero
+    if constexpr (NW > 1) {
+      if (tid < C) st_remote_u32(map_to_cta(&x.low[cr], static_cast<uint32_t>(tid)), low16);
+      cluster_arrive_release();
+      cluster_wait_acquire();
 #pragma unroll
-    for (int r = 0; r < C; ++r) low16 = max(low16, x.low[r]);
+      for (int r = 0; r < C; ++r) low16 = max(low16, x.low[r]);
+    }
   }
 
   // ---- collect this part's elements at or above the bound
-  const uint32_t low2 = low16 * 0x00010001u;
-  auto push = [&](uint32_t bits16, int idx) {
+  const Bound<T> bound(low16);
+  auto push = [&](uint32_t key, int idx) {
     const int slot = atomicAdd(&s.count, 1);
-    if (slot < kCandCap) {
-      s.cand_key[slot] = float_to_key(Elem<T>::to_float(from_bits16<T>(bits16)));
-      s.cand_idx[slot] = static_cast<uint32_t>(idx);
-    }
+    if (slot < kCandCap) s.cand[slot] = cand_of(key, idx);
   };
-#pragma unroll
-  for (int u = 0; u < kHeldVecs; ++u) {
-    if (u * kHeldThreads >= left) break;
-    // one bit per element (bit 4 * half + word), few of which are ever set
-    uint32_t hits = (__vcmpgeu2(key16x2<T>(raw[u].x), low2) & 0x00100001u) |
-                    (__vcmpgeu2(key16x2<T>(raw[u].y), low2) & 0x00200002u) |
-                    (__vcmpgeu2(key16x2<T>(raw[u].z), low2) & 0x00400004u) |
-                    (__vcmpgeu2(key16x2<T>(raw[u].w), low2) & 0x00800008u);
-    hits = (hits | (hits >> 16)) & 0xFFu;
-    while (hits) {
-      const int bit = __ffs(static_cast<int>(hits)) - 1;
-      hits &= hits - 1;
-      const int w = bit & 3, half = bit >> 2;
-      const uint32_t word = w == 0 ? raw[u].x : (w == 1 ? raw[u].y : (w == 2 ? raw[u].z : raw[u].w));
-      push((word >> (16 * half)) & 0xFFFFu, (v0 + tid + u * kHeldThreads) * 8 + 2 * w + half);
-    }
+  visit_hits<T>(raw, (left + kHeldThreads - 1) / kHeldThreads, head + (v0 + tid) * 8, kHeldThreads * 8, bound, push);
+  if (has_scal) {
+    const uint32_t key = key_of_bits<T>(scal_word);
+    if (key >= bound.low) push(key, scal_idx);
   }
-  if (has_tail && (key16x2<T>(tail_bits) & 0xFFFFu) >= low16) push(tail_bits, tail);
   __syncthreads();
-  int total = s.count;  // may exceed the buffer: then CTA 0 searches the row exactly
+  int total = s.count;            // may exceed the buffer: then the row is searched exactly
   if constexpr (C > 1) {
-    const int mine = total;
-    if (tid < C) st_remote_u32(map_to_cta(&x.cnt[cr], static_cast<uint32_t>(tid)), static_cast<uint32_t>(mine));
-    cluster_sync_all();
-    int offset = 0;
-    total = 0;
-#pragma unroll
-    for (int r = 0; r < C; ++r) {
-      if (r < cr) offset += x.cnt[r];
-      total += x.cnt[r];
+    // the others' candidates go to parts of CTA 0's buffer that its own do not reach; one-way stores, no
+    // round trip for a place in the list
+    constexpr int kPart = 1536, kList = kCandCap - (C - 1) * kPart;
+    if (cr != 0) {
+      const uint32_t dst = map_to_cta(&s.cand[kCandCap - cr * kPart], 0u);
+      for (int j = tid; j < total && j < kPart; j += kHeldThreads)
+        st_remote_u64(dst + 8u * static_cast<uint32_t>(j), s.cand[j]);
+      if (tid == 0) st_remote_u32(map_to_cta(&x.cnt[cr], 0u), static_cast<uint32_t>(total));
     }
-    // ---- candidates of the other CTAs move into CTA 0's list
-    if (cr != 0 && total <= kCandCap) {
-      const uint32_t dst_key = map_to_cta(&s.cand_key[0], 0u), dst_idx = map_to_cta(&s.cand_idx[0], 0u);
-      for (int j = tid; j < mine; j += kHeldThreads) {
-        st_remote_u32(dst_key + 4u * static_cast<uint32_t>(offset + j), s.cand_key[j]);
-        st_remote_u32(dst_idx + 4u * static_cast<uint32_t>(offset + j), s.cand_idx[j]);
+    cluster_arrive_release();
+    if (cr != 0) return;          // nobody reads this CTA's shared memory; CTA 0 stays until the copies are there
+    cluster_wait_acquire();
+    if (total > kList) total = kCandCap + 1;
+#pragma unroll
+    for (int r = 1; r < C; ++r) {
+      const int n = x.cnt[r];
+      if (n > kPart || total + n > kList) {
+        total = kCandCap + 1;
+      } else {                    // close the gap
+        for (int j = tid; j < n; j += kHeldThreads) s.cand[total + j] = s.cand[kCandCap - r * kPart + j];
+        total += n;
       }
     }
-    cluster_sync_all();  // after this barrier nobody touches another CTA's shared memory
-    if (cr != 0) return;
-  } else {
-    __syncthreads();
   }
-  topk_finish<T>(s, total, rp, v, true, kk, inv_temp, top_p, seed, step, row_ids, row, out);
+  __syncthreads();
+  topk_finish<T>(s, total, rp, v, kk, inv_temp, top_p, u24, row, out);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -667,7 +998,7 @@ __device__ void descend(const T* rp, int v, bool vec_ok, float inv_temp, float y
       s.mass[b] = 0;
     }
     __syncthreads();
-    for_each_key<T>(rp, v, vec_ok, [&](uint32_t key, int) {
+    for_each_key<T>(rp, v, [&](uint32_t key, int) {
       const bool match = known_bits == 0 || (key >> (32 - known_bits)) == (prefix >> (32 - known_bits));
       if (match) {
         const int bin = (key >> shift) & ((1 << w) - 1);
@@ -738,7 +1069,7 @@ __device__ void descend16(const T* rp, int v, bool vec_ok, float inv_temp, float
     for (int b = tid; b < kHalfBins; b += kThreads) hist[b] = 0;
     if (tid == 0) s.sel_bin = -1;
     __syncthreads();
-    for_each_key_x4<T>(rp, v, vec_ok, [&](uint32_t key, int) {
+    for_each_key<T>(rp, v, [&](uint32_t key, int) {
       const uint32_t k16 = key >> 16;
       if (static_cast<int>(k16 >> 15) == half) atomicAdd(&hist[k16 & 0x7FFFu], 1u);
     });
@@ -1170,7 +1501,7 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
 
   // ---- row maximum
   uint32_t tmax = 0;
-  for_each_key_x4<T>(rp, v, vec_ok, [&](uint32_t key, int) { tmax = max(tmax, key); });
+  for_each_key<T>(rp, v, [&](uint32_t key, int) { tmax = max(tmax, key); });
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) tmax = max(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
   if (tid == 0) s.max_key = 0;
@@ -1205,7 +1536,7 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
     } else {
       // everything is kept by the count criterion: Z = total mass
       unsigned long long local = 0;
-      for_each_key_x4<T>(rp, v, vec_ok, [&](uint32_t key, int) {
+      for_each_key<T>(rp, v, [&](uint32_t key, int) {
         const float y = mul_rn(key_to_float(key), inv_temp);
         local += mass_fixed(exp_det(sub_rn(y, y_max)));
       });
@@ -1255,7 +1586,7 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
           present = p_present;  // the histogram had the count
         } else {
           int local = 0;
-          for_each_key<T>(rp, v, vec_ok, [&](uint32_t key, int) { local += (key == p_tau) ? 1 : 0; });
+          for_each_key<T>(rp, v, [&](uint32_t key, int) { local += (key == p_tau) ? 1 : 0; });
           present = static_cast<unsigned long long>(block_sum_int(local, s.red));
         }
         const unsigned long long used = p_ties < present ? p_ties : present;
@@ -1362,55 +1693,63 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
   if (tid == 0) out[row] = s.pick;
 }
 
+template <typename T, int NW>
+int launch_topk(const T* lp, long long row_stride, int rows, int v, const long long* row_ids, float inv_temp, int top_k,
+                float top_p, unsigned long long seed, unsigned long long step, int* out, cudaStream_t stream) {
+  // 16-bit rows that 1, 2 or 4 CTAs can keep in registers take the kernel that reads them once, as long as
+  // all CTAs (one per SM) are resident at once; otherwise they would come in waves where the other kernel,
+  // two CTAs per SM, needs one. KA_SAMPLE_CLUSTER = 1 keeps the other one, 2 and 4 ask for that many CTAs
+  // per row.
+  if constexpr (Elem<T>::kPacked) {
+    int cluster = v <= kHeldElems ? 1 : (v <= 2 * kHeldElems ? 2 : (v <= 4 * kHeldElems ? 4 : 0));
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const char* env = getenv("KA_SAMPLE_CLUSTER");
+    const int asked = env ? atoi(env) : 0;
+    if (asked == 2 || asked == 4)
+      cluster = cluster != 0 && asked > cluster ? asked : cluster;
+    else if (asked == 1 || static_cast<long long>(rows) * cluster > sms)
+      cluster = 0;
+    if (cluster > 0) {
+      const int smem = static_cast<int>(sizeof(TopkSmem) + sizeof(ClusterXchg));
+      auto* kernel = cluster == 1 ? sample_topk_held_kernel<T, 1, NW>
+                                  : (cluster == 2 ? sample_topk_held_kernel<T, 2, NW> : sample_topk_held_kernel<T, 4, NW>);
+      static PerDevice once[3];
+      if (!smem_opt_in(once[cluster / 2], kernel, smem)) return -10;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(static_cast<unsigned>(rows) * cluster);
+      cfg.blockDim = dim3(kHeldThreads);
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = stream;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = cluster > 1 ? 1 : 0;
+      return cudaLaunchKernelEx(&cfg, kernel, lp, row_stride, v, row_ids, inv_temp, top_k, top_p, seed, step, out) ==
+                     cudaSuccess
+                 ? 0
+                 : -11;
+    }
+  }
+  static PerDevice once;
+  if (!smem_opt_in(once, sample_topk_kernel<T, NW>, static_cast<int>(sizeof(TopkSmem)))) return -10;
+  sample_topk_kernel<T, NW><<<rows, kTopkThreads, sizeof(TopkSmem), stream>>>(lp, row_stride, v, row_ids, inv_temp, top_k,
+                                                                           top_p, seed, step, out);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
 template <typename T>
 int launch_sampling(const void* logits, long long row_stride, int rows, int v, const long long* row_ids,
                     float inv_temp, int top_k, float top_p, unsigned long long seed, unsigned long long step,
                     int* out, cudaStream_t stream) {
   const T* lp = static_cast<const T*>(logits);
-  cudaError_t e;
   if (top_k >= 1 && top_k <= kMaxTopK) {
-    static PerDevice once;
-    if (!smem_opt_in(once, sample_topk_kernel<T>, static_cast<int>(sizeof(TopkSmem)))) return -10;
-    // Aligned rows that 1, 2 or 4 CTAs can keep in registers take the kernel that reads them once,
-    // as long as all CTAs (one per SM) are resident at once: bf16 [G, 128256], k = 50, L2 flushed:
-    // 22.6 us against 28.7 us at G = 64, but 41 against 33 us at G = 128 and 73 against 50 us at
-    // G = 256, where it comes in waves and the other kernel, two CTAs per SM, in one.
-    // KA_SAMPLE_CLUSTER = 1 keeps the other one, 2 and 4 ask for that many CTAs per row.
-    if constexpr (Elem<T>::kPacked) {
-      const bool aligned = (reinterpret_cast<uintptr_t>(lp) & 15u) == 0 && (row_stride * sizeof(T)) % 16 == 0;
-      int cluster = v <= kHeldElems ? 1 : (v <= 2 * kHeldElems ? 2 : (v <= 4 * kHeldElems ? 4 : 0));
-      int dev = 0, sms = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      const char* env = getenv("KA_SAMPLE_CLUSTER");
-      const int asked = env ? atoi(env) : 0;
-      if (asked == 2 || asked == 4)
-        cluster = cluster != 0 && asked > cluster ? asked : cluster;
-      else if (asked == 1 || static_cast<long long>(rows) * cluster > sms)
-        cluster = 0;
-      if (cluster > 0 && aligned) {
-        const int smem = static_cast<int>(sizeof(TopkSmem) + sizeof(ClusterXchg));
-        auto* kernel = cluster == 1 ? sample_topk_held_kernel<T, 1>
-                                    : (cluster == 2 ? sample_topk_held_kernel<T, 2> : sample_topk_held_kernel<T, 4>);
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -10;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(static_cast<unsigned>(rows) * cluster);
-        cfg.blockDim = dim3(kHeldThreads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = cluster > 1 ? 1 : 0;
-        e = cudaLaunchKernelEx(&cfg, kernel, lp, row_stride, v, row_ids, inv_temp, top_k, top_p, seed, step, out);
-        return e == cudaSuccess ? 0 : -11;
-      }
-    }
-    sample_topk_kernel<T><<<rows, kTopkThreads, sizeof(TopkSmem), stream>>>(lp, row_stride, v, row_ids, inv_temp, top_k,
-                                                                         top_p, seed, step, out);
+    return top_k <= kFewK ? launch_topk<T, 1>(lp, row_stride, rows, v, row_ids, inv_temp, top_k, top_p, seed, step, out, stream)
+                          : launch_topk<T, 4>(lp, row_stride, rows, v, row_ids, inv_temp, top_k, top_p, seed, step, out, stream);
   } else {
     constexpr int smem = kGeneralSmemBytes + (Elem<T>::kPacked ? static_cast<int>(sizeof(FastSmem)) : 0);
     static_assert(sizeof(FastSmem) >= kHistBytes, "the older search keeps its histogram there");
@@ -1419,8 +1758,7 @@ int launch_sampling(const void* logits, long long row_stride, int rows, int v, c
     sample_general_kernel<T><<<rows, kThreads, smem, stream>>>(lp, row_stride, v, row_ids, inv_temp, top_k, top_p,
                                                               seed, step, out);
   }
-  e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -11;
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
 }  // namespace

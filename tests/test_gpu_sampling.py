@@ -61,6 +61,31 @@ def test_sampler_cluster_variants_equal_cpu_definition(cuda_device, cluster, mon
     assert torch.equal(tok, sample(llama, top_k=50, top_p=0.9, temperature=0.7, seed=1, step=5))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, torch.float16])
+@pytest.mark.parametrize("vocab,rows", [(5, 3), (1023, 3), (65537, 3), (131081, 2), (33001, 200)])
+def test_sampler_top_k_bounds_and_row_starts(cuda_device, dtype, vocab, rows):
+    """Both sides of the small-k bound, candidates by the thousand, rows that start off a 16-byte
+    boundary, one to four CTAs per row and more rows than are resident; values: plain, heavy ties,
+    mostly -inf or the type's lowest, sorted (the largest all in one part of the row), NaN and +inf."""
+    g = torch.Generator(device=cuda_device).manual_seed(vocab)
+    x = torch.randn(rows, vocab, device=cuda_device, generator=g) * 2
+    u = torch.rand(x.shape, device=cuda_device, generator=g)
+    values = {"plain": x, "ties": x.round(), "masked": torch.where(u < 0.999, float("-inf"), x),
+              "lowest": torch.where(u < 0.9, torch.finfo(dtype).min, x), "sorted": x.sort(1, descending=True).values,
+              "special": torch.where(u < 0.01, float("nan"), torch.where(u > 0.9999, float("inf"), x))}
+    buf = torch.empty(rows * (vocab + 1) + 3, dtype=dtype, device=cuda_device)
+    for name, val in values.items():
+        for off, width in ((0, vocab), (3, vocab + 1)):
+            logits = buf[off:off + rows * width].view(rows, width)[:, :vocab]
+            logits.copy_(val)
+            for top_k, top_p in ((1, None), (64, 0.9), (65, 0.5), (1000, 0.95), (1024, None)):
+                if top_k >= vocab:
+                    continue
+                tok = sample(logits, top_k=top_k, top_p=top_p, temperature=0.7, seed=4, step=off)
+                ref = _cpu(logits[:4], top_k, top_p, 0.7, 4, off)
+                assert torch.equal(tok[:4].cpu(), ref), (name, off, top_k, top_p)
+
+
 def test_sampler_heavy_ties(cuda_device):
     # constant rows overflow the candidate list: the exact-select path cuts ties by token id
     logits = torch.zeros(4, 20000, device=cuda_device, dtype=torch.bfloat16)
