@@ -981,7 +981,7 @@ constexpr int kGeneralSmemBytes = (static_cast<int>(sizeof(GeneralSmem)) + 15) /
 //   by count: first key where count_above + count(key) >  limit  (limit = k - 1)
 //   by mass : first key where mass_above  + mass(key)  >  limit
 template <typename T>
-__device__ void descend(const T* rp, int v, bool vec_ok, float inv_temp, float y_max, bool by_mass,
+__device__ void descend(const T* rp, int v, float inv_temp, float y_max, bool by_mass,
                         unsigned long long limit, GeneralSmem& s, uint32_t& tau, unsigned long long& above_cnt,
                         unsigned long long& above_mass) {
   const int tid = threadIdx.x;
@@ -1058,7 +1058,7 @@ __device__ __forceinline__ unsigned long long key16_mass(uint32_t k16, float inv
 
 // Same contract as descend(); `present` additionally receives the number of elements equal to tau.
 template <typename T>
-__device__ void descend16(const T* rp, int v, bool vec_ok, float inv_temp, float y_max, bool by_mass,
+__device__ void descend16(const T* rp, int v, float inv_temp, float y_max, bool by_mass,
                           unsigned long long limit, GeneralSmem& s, unsigned int* hist, uint32_t& tau,
                           unsigned long long& above_cnt, unsigned long long& above_mass,
                           unsigned long long& present) {
@@ -1131,50 +1131,73 @@ __device__ void descend16(const T* rp, int v, bool vec_ok, float inv_temp, float
   __syncthreads();
 }
 
-// ---- 16-bit rows: everything from one histogram of counts per key -----------------------------
-// A bf16 or fp16 value has 65536 keys and the mass of a key is a function of the key, so one
-// pass that counts elements per key answers every question about (count, mass) prefixes: the
-// maximum, the total mass and both thresholds cost one exponential per distinct value instead
-// of one per element and pass. The draw needs sums in token-id order: the row is cut into 32
-// contiguous segments, one per warp, whose kept masses are order-free integer sums (coalesced
-// loads, masses from a table), the segment that holds the target is cut into 32 again, and only
-// the last hundred elements are walked in order.
-//   * Counters are 16 bits, two per word (128 KiB for all 65536 keys). An overflow loses at
-//     least 65535 from the sum of the counters, so "sum == v" says that none happened; a row
-//     in which one value fills more than 65535 places takes the older search.
-//   * The table of masses reuses the histogram's memory: groups of 32 keys that hold kept
-//     elements get consecutive slots (at most 1024; a row that needs more, i.e. with values in
-//     every corner of the format, takes the older search). A mass of 2^32 (probability 1) is
-//     stored as 2^32 - 1, which no smaller float maps to.
-// Measured, bf16 [200, 128256] ~ N(0, 2), T = 1, top_p = 0.9: 227 us with an exponential per
-// element for the total and ordered walks of the row in the draw, 113 us this way.
-constexpr int kGroups = 2048;                 // of 32 keys; GeneralSmem::cnt / mass hold their sums
-constexpr int kTableGroups = 1024;
-constexpr int kHistWords = 32768;
-static_assert(kGroups == kBins && kGroups == 2 * kThreads, "two groups per thread, sums kept in the descent's bins");
-
-struct FastSmem {
-  unsigned int words[kHistWords];             // 16-bit counters, then the table of masses
-  unsigned short slot[kGroups];
-  unsigned long long seg_ties[kWarps];
-  unsigned long long seg_mass[kWarps];
-  unsigned int total;
-  unsigned int max_key;
-  // result of a search / of a level of the draw
-  int sel;
-  unsigned int sel_key;
-  unsigned long long above_cnt, above_mass, present;
-  unsigned long long ties_before, target;
+// ---- masses by arithmetic -------------------------------------------------------------------
+// mass_fixed(exp_det(x * inv_temp - y_max)) of two elements at a time, the same integers without the
+// conversion instructions (a quarter of the rate of the others): rounding to an integer by adding and
+// subtracting 1.5 * 2^23, the exponent taken from that sum's bits, the float-to-integer step by a shift of
+// the mantissa. The products and sums are the packed two-element instructions, which round each half as the
+// scalar ones do. 19 instructions an element: a draw over
+// all 128256 elements (temperature only) takes 25 us for one row, with a histogram and a table in front of it
+// it took 62 us; fp32 25 us, with exp_det per element 168 us.
+struct MassArgs {
+  float inv_temp, neg_y_max;
 };
 
-template <typename T>
-__device__ __forceinline__ float key16_float(uint32_t k16) {
-  if (k16 == 0) return key_to_float(0u);  // NaN
-  return Elem<T>::to_float(from_bits16<T>((k16 & 0x8000u) ? (k16 & 0x7FFFu) : (~k16 & 0xFFFFu)));
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
 }
-template <typename T>
-__device__ __forceinline__ unsigned long long key16_mass_of(uint32_t k16, float inv_temp, float y_max) {
-  return mass_fixed(exp_det(sub_rn(mul_rn(key16_float<T>(k16), inv_temp), y_max)));
+__device__ __forceinline__ void unpack2(unsigned long long v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long both(float a) { return pack2(a, a); }
+
+__device__ __forceinline__ void mass_pair(float x0, float x1, const MassArgs& a, unsigned long long& sum) {
+  constexpr float kRound = 12582912.0f;                       // 1.5 * 2^23
+  // the first product is scalar: the assembler joins a packed product and the packed sum behind it into one
+  // rounding, .rn or not
+  const unsigned long long y = pack2(__fmul_rn(x0, a.inv_temp), __fmul_rn(x1, a.inv_temp));
+  unsigned long long t = mul2(add2(y, both(a.neg_y_max)), both(1.4426950408889634f));
+  float t0, t1;
+  unpack2(t, t0, t1);
+  t = pack2(fmaxf(t0, -64.f), fmaxf(t1, -64.f));              // below 2^-33 the mass is 0; NaN becomes -64
+  const unsigned long long r = add2(t, both(kRound));
+  const unsigned long long f = fma2(add2(r, both(-kRound)), both(-1.f), t);
+  unsigned long long p = both(1.5403530393381609e-4f);
+  p = fma2(p, f, both(1.3333558146428443e-3f));
+  p = fma2(p, f, both(9.6181291076284772e-3f));
+  p = fma2(p, f, both(5.5504108664821580e-2f));
+  p = fma2(p, f, both(2.4022650695910071e-1f));
+  p = fma2(p, f, both(6.9314718055994531e-1f));
+  p = fma2(p, f, both(1.0f));
+  float r0, r1, p0, p1;
+  unpack2(r, r0, r1);
+  unpack2(p, p0, p1);
+  auto add = [&](float rr, float pp) {
+    const uint32_t pb = __float_as_uint(pp);
+    // floor(p 2^(n + 32)) = mantissa (bit 31 down) >> shift, with n in the low bits of rr
+    const uint32_t shift = 126u + 0x4B400000u - (pb >> 23) - __float_as_uint(rr);
+    const uint32_t m = __funnelshift_rc((pb << 8) | 0x80000000u, 0u, shift);   // a shift of 32 or more gives 0
+    sum += (static_cast<unsigned long long>(shift >> 31) << 32) | m;           // shift -1: p = 1, n = 0
+  };
+  add(r0, p0);
+  add(r1, p1);
 }
 
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
@@ -1192,27 +1215,96 @@ __device__ __forceinline__ unsigned long long warp_incl_u64(unsigned long long v
   return v;
 }
 
-__device__ __forceinline__ unsigned int key_count(const FastSmem& f, uint32_t k16) {
-  return (f.words[k16 >> 1] >> ((k16 & 1u) * 16u)) & 0xFFFFu;
+// ---- 16-bit rows: everything from one histogram of counts per key -----------------------------
+// A bf16 or fp16 value has 65536 keys and the mass of a key is a function of the key, so one
+// pass that counts elements per key answers every question about (count, mass) prefixes: the
+// maximum, the total mass and both thresholds cost one exponential per distinct value instead
+// of one per element and pass.
+//   * Counters are 16 bits, two per word (128 KiB), named by the value's bits as they are; only what reads
+//     them puts them in the order of keys, by groups of 32. An overflow loses at least 65535 from the sum
+//     of the counters, so "sum == v" says that none happened; a row in which one value fills more than
+//     65535 places takes the older search, and so does a row with NaNs.
+//   * Only groups that occur are visited when masses are added up (150 of 2048 for bf16 logits).
+//   * The masses of the keys above the threshold go to a table in the counters' place if there are fewer
+//     than 16384 of them (a few hundred for top-p on bf16 logits). Its entries are 64 bits, so that a tie at
+//     the threshold counts itself in the high bits and a lookup needs no branch.
+// What bounds it: bf16 [148, 128256] ~ N(0, 2), T = 1, top_p = 0.9 takes a CTA 52.9k cycles: 18k for the
+// histogram (a shared-memory atomic per element, about four conflicting lanes each), 17k for the draw (a
+// table lookup per element), 10k for the searches between, 7k for clearing, table and the end of the draw.
+// 107k before: groups that do not occur were visited, lookups went through two tables and behind a branch
+// (33k for the draw with one table and the branch). 62 us a call then, 35 us now.
+constexpr int kGroups = 2048;                 // of 32 keys; GeneralSmem::cnt / mass hold their sums
+constexpr int kTable = 16384;
+constexpr int kTieShift = 48;                 // a thread's masses add up to less than 2^48 (at most 2^15 elements of 2^32)
+constexpr int kTableMaxVocab = 1 << 25;       // ... which 32 warps' lanes see in rows of at most this many elements
+constexpr int kHistWords = 32768;
+static_assert(kGroups == kBins && kGroups == 2 * kThreads, "two groups per thread, sums kept in the descent's bins");
+
+struct FastSmem {
+  union {
+    unsigned int words[kHistWords];             // 16-bit counters
+    unsigned long long table[kTable];           // then masses by distance from the largest key
+  };
+  unsigned short list[kGroups];               // groups that occur
+  unsigned int n_list;
+  unsigned int total;
+  unsigned int nans;
+  unsigned int top_group;
+  // result of a search
+  int sel;
+  unsigned int sel_key;
+  unsigned long long above_cnt, above_mass, present;
+};
+
+// What the draw keeps: keys above tau, and of the ties at tau the first tie_keep in token-id order.
+struct Kept {
+  uint32_t tau;                  // 32-bit key
+  unsigned long long tie_keep, q_tau;
+  MassArgs args;
+  const unsigned long long* table;   // kByTable: masses by distance from the largest key, a tie, 0
+  uint32_t top2, last2;              // in both halves of a word: the largest 16-bit key + 1, the distance of what has no mass
+};
+struct DrawSmem {
+  unsigned long long seg_ties[kWarps];
+  unsigned long long seg_mass[kWarps];
+  unsigned long long ties_before, target;
+  int sel;
+};
+enum : int { kAll = 0, kByExp = 1, kByTable = 2 };   // all elements are kept / masses computed / looked up
+
+template <typename T>
+__device__ __forceinline__ float key16_float(uint32_t k16) {
+  if (k16 == 0) return key_to_float(0u);  // NaN
+  return Elem<T>::to_float(from_bits16<T>((k16 & 0x8000u) ? (k16 & 0x7FFFu) : (~k16 & 0xFFFFu)));
+}
+template <typename T>
+__device__ __forceinline__ unsigned long long key16_mass_of(uint32_t k16, float inv_temp, float y_max) {
+  return mass_fixed(exp_det(sub_rn(mul_rn(key16_float<T>(k16), inv_temp), y_max)));
 }
 
-// descend()'s contract on the histogram: groups by a block scan from the top, the key inside the
-// group by one warp.
+__device__ __forceinline__ unsigned int key_count(const FastSmem& f, uint32_t k16) {
+  const uint32_t bits = (k16 & 0x8000u) ? (k16 & 0x7FFFu) : (0xFFFFu - k16);
+  return (f.words[bits >> 1] >> ((bits & 1u) * 16u)) & 0xFFFFu;
+}
+
+// descend()'s contract on the histogram, from the prefix sums of this thread's two groups (pre_c / pre_m: what
+// lies above them): the group that holds the crossing, then the key inside it by one warp. above_cnt is only
+// valid if counts were summed.
 template <typename T>
-__device__ void search_groups(bool by_mass, unsigned long long limit, float inv_temp, float y_max, GeneralSmem& s,
-                              FastSmem& f) {
+__device__ void search_groups(bool by_mass, unsigned long long limit, float inv_temp, float y_max,
+                              unsigned long long pre_c, unsigned long long pre_m, unsigned long long tot_c,
+                              unsigned long long tot_m, const GeneralSmem& s, FastSmem& f) {
   const int tid = threadIdx.x, lane = tid & 31;
   if (tid == 0) f.sel = -1;
+  __syncthreads();
   const int g0 = kGroups - 1 - 2 * tid;       // this thread's groups, from the top: g0, g0 - 1
   const unsigned long long c0 = s.cnt[g0], c1 = s.cnt[g0 - 1], m0 = s.mass[g0], m1 = s.mass[g0 - 1];
-  unsigned long long tot_c, tot_m;
-  unsigned long long c = block_exscan_u64(c0 + c1, s.scan, tot_c), m = block_exscan_u64(m0 + m1, s.scan, tot_m);
-  const unsigned long long pre = by_mass ? m : c, mid = pre + (by_mass ? m0 : c0), end = mid + (by_mass ? m1 : c1);
+  const unsigned long long pre = by_mass ? pre_m : pre_c, mid = pre + (by_mass ? m0 : c0), end = mid + (by_mass ? m1 : c1);
   if (pre <= limit && end > limit) {
     const bool second = mid <= limit;
     f.sel = second ? g0 - 1 : g0;
-    f.above_cnt = second ? c + c0 : c;
-    f.above_mass = second ? m + m0 : m;
+    f.above_cnt = second ? pre_c + c0 : pre_c;
+    f.above_mass = second ? pre_m + m0 : pre_m;
   }
   __syncthreads();
   const int g = f.sel;
@@ -1243,228 +1335,142 @@ __device__ void search_groups(bool by_mass, unsigned long long limit, float inv_
 }
 
 // Kept mass and ties of the elements [begin, end) of the row, summed by one warp (any order).
-template <typename T>
-__device__ __forceinline__ void sum_range(const T* rp, bool vec_ok, int begin, int end, uint32_t tau, const FastSmem& f,
-                                          unsigned long long& mass, unsigned long long& ties) {
+template <typename T, int kMode>
+__device__ __forceinline__ void sum_range(const T* rp, int begin, int end, const Kept& k, unsigned long long& mass,
+                                          unsigned long long& ties) {
+  constexpr int kVec = Elem<T>::kVec, kU = 4;
+  static_assert(kMode != kByTable || Elem<T>::kPacked, "the table is indexed by 16-bit keys");
   const int lane = threadIdx.x & 31;
-  const unsigned short* hp = reinterpret_cast<const unsigned short*>(rp);
+  const T* p = rp + begin;
+  const int n = end - begin, head = row_head(p, n), nvec = (n - head) / kVec, scal = n - nvec * kVec;
   unsigned long long m = 0;
-  unsigned int n_ties = 0, n_one = 0;
-  auto take = [&](uint32_t key) {
-    if (key > tau) {
-      const unsigned int t = f.words[f.slot[key >> 5] * 32u + (key & 31u)];
-      m += t;
-      n_one += t == 0xFFFFFFFFu ? 1u : 0u;
-    } else if (key == tau) {
-      ++n_ties;
+  unsigned int n_ties = 0;
+  const int tau_o = static_cast<int>(k.tau ^ 0x80000000u);    // keys as signed numbers
+  auto ordered = [](float x) {
+    const int b = __float_as_int(x);
+    return b ^ ((b >> 31) & 0x7FFFFFFF);
+  };
+  auto take2 = [&](float x0, float x1) {
+    if constexpr (kMode != kAll) {
+      const int o0 = ordered(x0), o1 = ordered(x1);
+      n_ties += (o0 == tau_o ? 1u : 0u) + (o1 == tau_o ? 1u : 0u);
+      x0 = o0 > tau_o ? x0 : __uint_as_float(0xFF800000u);
+      x1 = o1 > tau_o ? x1 : __uint_as_float(0xFF800000u);
+    }
+    mass_pair(x0, x1, k.args, m);
+  };
+  auto take_word = [&](uint32_t w) {
+    if constexpr (kMode == kByTable) {
+      // distance of both keys from the largest one, cut off behind the tie's: min(top - key, last)
+      const uint32_t not_key = ~(w ^ (((w >> 15) & 0x00010001u) * 0x7FFFu));   // keys as signed numbers
+      const uint32_t i2 = __viaddmin_u16x2(not_key, k.top2, k.last2);
+      m += k.table[i2 & 0xFFFFu];
+      m += k.table[i2 >> 16];
+    } else if constexpr (Elem<T>::kPacked) {
+      take2(Elem<T>::to_float(from_bits16<T>(w & 0xFFFFu)), Elem<T>::to_float(from_bits16<T>(w >> 16)));
     }
   };
-  int i = begin;
-  if (vec_ok) {                               // begin is a multiple of 8
-    const uint4* vp = reinterpret_cast<const uint4*>(hp + begin);
-    const int nvec = (end - begin) / 8;
-    constexpr int kU = 4;
-    for (int j = lane; j < nvec; j += 32 * kU) {
-      uint4 raw[kU];
+  const uint4* vp = reinterpret_cast<const uint4*>(p + head);
+  for (int j = lane; j < nvec; j += 32 * kU) {
+    uint4 raw[kU];
 #pragma unroll
-      for (int u = 0; u < kU; ++u) raw[u] = j + 32 * u < nvec ? __ldg(vp + j + 32 * u) : make_uint4(0u, 0u, 0u, 0u);
+    for (int u = 0; u < kU; ++u)
+      if (j + 32 * u < nvec) raw[u] = __ldg(vp + j + 32 * u);
 #pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        if (j + 32 * u >= nvec) break;
-        const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint32_t k2 = key16x2<T>(w[e]);
-          take(k2 & 0xFFFFu);
-          take(k2 >> 16);
-        }
+    for (int u = 0; u < kU; ++u) {
+      if (j + 32 * u >= nvec) break;
+      if constexpr (Elem<T>::kPacked) {
+        take_word(raw[u].x);
+        take_word(raw[u].y);
+        take_word(raw[u].z);
+        take_word(raw[u].w);
+      } else {
+        take2(__uint_as_float(raw[u].x), __uint_as_float(raw[u].y));
+        take2(__uint_as_float(raw[u].z), __uint_as_float(raw[u].w));
       }
     }
-    i = begin + nvec * 8;
   }
-  for (i += lane; i < end; i += 32) take(key16x2<T>(hp[i]) & 0xFFFFu);
-  mass = warp_sum_u64(m + n_one);
-  ties = warp_sum_u64(static_cast<unsigned long long>(n_ties));
+  if (lane < scal) {
+    // one element; its partner is -inf, which has no mass and is no tie (-inf as a threshold has mass 0)
+    const T e = p[lane < head ? lane : nvec * kVec + lane];
+    if constexpr (kMode == kByTable) {
+      const uint32_t w = *reinterpret_cast<const unsigned short*>(&e);
+      m += k.table[__viaddmin_u16x2(~(w ^ ((w >> 15) * 0x7FFFu)), k.top2, k.last2) & 0xFFFFu];
+    } else {
+      const float x = Elem<T>::to_float(e);
+      const unsigned int before = n_ties;
+      take2(x, __uint_as_float(0xFF800000u));
+      n_ties = before + (kMode != kAll && ordered(x) == tau_o ? 1u : 0u);
+    }
+  }
+  if constexpr (kMode == kByTable) {
+    n_ties = static_cast<unsigned int>(m >> kTieShift);
+    m &= (1ull << kTieShift) - 1;
+  }
+  mass = warp_sum_u64(m);
+  ties = kMode == kAll ? 0ull : __reduce_add_sync(0xffffffffu, n_ties);
 }
 
-// One row of 16-bit logits. Returns false (for the whole block) if the row needs the older search.
-template <typename T>
-__device__ bool sample_row16(const T* rp, int v, bool vec_ok, float inv_temp, int top_k, float top_p, uint32_t u24,
-                             GeneralSmem& s, FastSmem& f, int* out) {
+// First element, in token-id order, whose cumulative kept mass exceeds the target: the row is cut into
+// 32 contiguous segments, one per warp, whose kept masses are order-free integer sums (coalesced loads),
+// the segment that holds the target is cut into 32 again, and only the last hundred elements are walked
+// in order. With kAll the kept mass is what the first level adds up; false if it is 0.
+template <typename T, int kMode>
+__device__ bool draw(const T* rp, int v, const Kept& k, unsigned long long kept_mass, uint32_t u24, DrawSmem& d, int* out) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const unsigned short* hp = reinterpret_cast<const unsigned short*>(rp);
-  // ---- count
-  for (int i = tid; i < kHistWords / 4; i += kThreads) reinterpret_cast<uint4*>(f.words)[i] = make_uint4(0u, 0u, 0u, 0u);
-  if (tid == 0) {
-    f.total = 0;
-    f.max_key = 0;
-  }
-  __syncthreads();
-  auto add = [&](uint32_t key) { atomicAdd(&f.words[key >> 1], 1u << ((key & 1u) * 16u)); };
-  const int nvec = vec_ok ? v / 8 : 0;
-  {
-    const uint4* vp = reinterpret_cast<const uint4*>(hp);
-    constexpr int kU = 4;
-    for (int j = tid; j < nvec; j += kThreads * kU) {
-      uint4 raw[kU];
-#pragma unroll
-      for (int u = 0; u < kU; ++u)
-        raw[u] = j + kThreads * u < nvec ? __ldg(vp + j + kThreads * u) : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        if (j + kThreads * u >= nvec) break;
-        const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint32_t k2 = key16x2<T>(w[e]);
-          add(k2 & 0xFFFFu);
-          add(k2 >> 16);
-        }
-      }
-    }
-    for (int i = nvec * 8 + tid; i < v; i += kThreads) add(key16x2<T>(hp[i]) & 0xFFFFu);
-  }
-  __syncthreads();
-  // ---- counts per group (group g belongs to warp g % 32), their sum, the largest key
-  {
-    unsigned int sum = 0, top = 0;
-    for (int g = warp; g < kGroups; g += kWarps) {
-      const unsigned int c = key_count(f, static_cast<uint32_t>(g * 32 + lane));
-      const unsigned int any = __ballot_sync(0xffffffffu, c != 0);
-      const unsigned int n = any ? __reduce_add_sync(0xffffffffu, c) : 0u;
-      if (lane == 0) s.cnt[g] = n;
-      sum += n;
-      if (any) top = static_cast<unsigned int>(g * 32 + 31 - __clz(static_cast<int>(any)));
-    }
-    if (lane == 0) {
-      atomicAdd(&f.total, sum);
-      atomicMax(&f.max_key, top);
-    }
-  }
-  __syncthreads();
-  if (f.total != static_cast<unsigned int>(v)) return false;   // a counter overflowed
-  const float y_max = mul_rn(key16_float<T>(f.max_key), inv_temp);
-  for (int g = warp; g < kGroups; g += kWarps) {
-    unsigned long long m = 0;
-    if (s.cnt[g]) {
-      const uint32_t key = static_cast<uint32_t>(g * 32 + lane);
-      const unsigned int c = key_count(f, key);
-      m = warp_sum_u64(c ? c * key16_mass_of<T>(key, inv_temp, y_max) : 0ull);
-    }
-    if (lane == 0) s.mass[g] = m;
-  }
-  __syncthreads();
-
-  // ---- where the kept prefix ends: the same decisions as in sample_general_kernel
-  uint32_t tau = 0;
-  unsigned long long tie_keep = ~0ull, kept_mass = 0;
-  {
-    uint32_t k_tau = 0;
-    unsigned long long k_ties = ~0ull;
-    const bool has_k = top_k > 0 && top_k < v;
-    if (has_k) {
-      search_groups<T>(false, static_cast<unsigned long long>(top_k - 1), inv_temp, y_max, s, f);
-      k_tau = f.sel_key;
-      k_ties = static_cast<unsigned long long>(top_k) - f.above_cnt;
-      kept_mass = f.above_mass + k_ties * key16_mass_of<T>(k_tau, inv_temp, y_max);
-    } else {
-      unsigned long long total;
-      block_exscan_u64(s.mass[2 * tid] + s.mass[2 * tid + 1], s.scan, total);
-      kept_mass = total;
-    }
-    tau = k_tau;
-    tie_keep = k_ties;
-    if (top_p < 1.0f) {
-      const unsigned long long limit = mass_fraction(static_cast<double>(top_p), kept_mass);
-      __syncthreads();
-      search_groups<T>(true, limit, inv_temp, y_max, s, f);
-      const uint32_t p_tau = f.sel_key;
-      const unsigned long long above = f.above_mass, q = key16_mass_of<T>(p_tau, inv_temp, y_max);
-      const unsigned long long p_ties = above > limit ? 0ull : (q == 0 ? ~0ull : (limit - above) / q + 1);
-      if (!has_k || (p_tau != k_tau ? p_tau > k_tau : p_ties < k_ties)) {
-        tau = p_tau;
-        tie_keep = p_ties < f.present ? p_ties : f.present;
-        kept_mass = above + tie_keep * q;
-      }
-    }
-  }
-  if (kept_mass == 0) return false;           // nothing has a mass: the older path picks by position
-
-  // ---- table of masses of the kept keys, over the counters
-  const int g_lo = static_cast<int>(tau >> 5);
-  unsigned long long n_slots;
-  {
-    const int g = 2 * tid;
-    const unsigned int a = g >= g_lo && s.cnt[g] ? 1u : 0u, b = g + 1 >= g_lo && s.cnt[g + 1] ? 1u : 0u;
-    const unsigned long long first = block_exscan_u64(a + b, s.scan, n_slots);
-    f.slot[g] = static_cast<unsigned short>(first);
-    f.slot[g + 1] = static_cast<unsigned short>(first + a);
-  }
-  if (n_slots > kTableGroups) return false;
-  unsigned long long present = 0;             // bit i: this lane's key of the warp's i-th group occurs
-  for (int g = warp, i = 0; g < kGroups; g += kWarps, ++i)
-    if (g >= g_lo && s.cnt[g])
-      present |= static_cast<unsigned long long>(key_count(f, static_cast<uint32_t>(g * 32 + lane)) != 0) << i;
-  __syncthreads();                            // every counter has been read
-  for (int g = warp, i = 0; g < kGroups; g += kWarps, ++i) {
-    if (g < g_lo || !s.cnt[g]) continue;
-    unsigned long long q = 0;
-    if ((present >> i) & 1ull) q = key16_mass_of<T>(static_cast<uint32_t>(g * 32 + lane), inv_temp, y_max);
-    f.words[f.slot[g] * 32 + lane] = static_cast<unsigned int>(q >> 32 ? 0xFFFFFFFFull : q);
-  }
-  __syncthreads();
-
-  // ---- draw: find the first element, in token-id order, whose cumulative kept mass exceeds target
-  const unsigned long long q_tau = key16_mass_of<T>(tau, inv_temp, y_max);
   int begin = 0, end = v;
   if (tid == 0) {
-    f.target = mass_scale_u24(u24, kept_mass);
-    f.ties_before = 0;
+    d.target = mass_scale_u24(u24, kept_mass);
+    d.ties_before = 0;
+    d.sel = -1;
   }
 #pragma unroll 1
   for (int level = 0; level < 2; ++level) {
     const int len = ((end - begin + kWarps - 1) / kWarps + 7) / 8 * 8;
     const int b = min(end, begin + warp * len), e = min(end, b + len);
     unsigned long long mass, ties;
-    sum_range<T>(rp, vec_ok, b, e, tau, f, mass, ties);
+    sum_range<T, kMode>(rp, b, e, k, mass, ties);
     if (lane == 0) {
-      f.seg_mass[warp] = mass;
-      f.seg_ties[warp] = ties;
+      d.seg_mass[warp] = mass;
+      d.seg_ties[warp] = ties;
     }
     __syncthreads();
     if (warp == 0) {
-      const unsigned long long t = f.seg_ties[lane], target = f.target;
-      const unsigned long long t0 = f.ties_before + warp_incl_u64(t) - t;
-      const unsigned long long left = tie_keep > t0 ? tie_keep - t0 : 0ull;
-      const unsigned long long m = f.seg_mass[lane] + (t < left ? t : left) * q_tau;
+      const unsigned long long t = d.seg_ties[lane];
+      const unsigned long long t0 = d.ties_before + warp_incl_u64(t) - t;
+      const unsigned long long left = k.tie_keep > t0 ? k.tie_keep - t0 : 0ull;
+      const unsigned long long m = d.seg_mass[lane] + (t < left ? t : left) * k.q_tau;
       const unsigned long long inc = warp_incl_u64(m);
+      unsigned long long target = d.target;
+      if (kMode == kAll && level == 0) target = mass_scale_u24(u24, __shfl_sync(0xffffffffu, inc, 31));
       const int first = __ffs(static_cast<int>(__ballot_sync(0xffffffffu, inc > target))) - 1;
       if (lane == first) {
-        f.sel = first;
-        f.target = target - (inc - m);
-        f.ties_before = t0;
+        d.sel = first;
+        d.target = target - (inc - m);
+        d.ties_before = t0;
       }
     }
     __syncthreads();
-    begin = min(end, begin + f.sel * len);
+    if (d.sel < 0) return false;
+    begin = min(end, begin + d.sel * len);
     end = min(end, begin + len);
   }
   if (warp == 0) {
-    const unsigned long long target = f.target;
-    unsigned long long acc = 0, t0 = f.ties_before;
+    const unsigned long long target = d.target;
+    const float y_max = -k.args.neg_y_max;
+    unsigned long long acc = 0, t0 = d.ties_before;
     for (int i0 = begin; i0 < end; i0 += 32) {
       const int i = i0 + lane;
-      const uint32_t key = i < end ? key16x2<T>(hp[i]) & 0xFFFFu : 0u;
-      const bool tie = i < end && key == tau;
+      const float x = i < end ? Elem<T>::to_float(rp[i]) : 0.f;
+      const uint32_t key = float_to_key(x);
+      const bool tie = i < end && kMode != kAll && key == k.tau;
       const unsigned int tie_mask = __ballot_sync(0xffffffffu, tie);
       const unsigned long long rank = t0 + __popc(tie_mask & ((1u << lane) - 1u));
       unsigned long long q = 0;
-      if (i < end && key > tau) {
-        const unsigned int t = f.words[f.slot[key >> 5] * 32u + (key & 31u)];
-        q = static_cast<unsigned long long>(t) + (t == 0xFFFFFFFFu ? 1ull : 0ull);
-      } else if (tie && rank < tie_keep) {
-        q = q_tau;
-      }
+      if (i < end && (kMode == kAll || key > k.tau))
+        q = mass_fixed(exp_det(sub_rn(mul_rn(key_to_float(key), k.args.inv_temp), y_max)));
+      else if (tie && rank < k.tie_keep)
+        q = k.q_tau;
       const unsigned long long inc = acc + warp_incl_u64(q);
       const unsigned int hit = __ballot_sync(0xffffffffu, inc > target);
       if (hit) {
@@ -1478,37 +1484,272 @@ __device__ bool sample_row16(const T* rp, int v, bool vec_ok, float inv_temp, in
   return true;
 }
 
+// One row of 16-bit logits with a top-p or a large top-k. Returns false (for the whole block) if the row
+// needs the older search.
+template <typename T>
+__device__ bool sample_row16(const T* rp, int v, float inv_temp, int top_k, float top_p, uint32_t u24, GeneralSmem& s,
+                             FastSmem& f, DrawSmem& d, int* out) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned short* hp = reinterpret_cast<const unsigned short*>(rp);
+  // ---- count
+  for (int i = tid; i < kHistWords / 4; i += kThreads) reinterpret_cast<uint4*>(f.words)[i] = make_uint4(0u, 0u, 0u, 0u);
+  s.mass[2 * tid] = s.mass[2 * tid + 1] = 0;
+  if (tid == 0) f.n_list = f.total = f.nans = f.top_group = 0;
+  __syncthreads();
+  {
+    // the counter of bits b is half b & 1 of word b >> 1
+    auto add_word = [&](uint32_t w) {
+      unsigned char* base = reinterpret_cast<unsigned char*>(f.words);
+      atomicAdd(reinterpret_cast<unsigned int*>(base + ((w << 1) & 0x1FFFCu)), max((w << 16) & 0x10000u, 1u));
+      atomicAdd(reinterpret_cast<unsigned int*>(base + ((w >> 15) & 0x1FFFCu)), max(w & 0x10000u, 1u));
+    };
+    const int head = row_head(rp, v), nvec = (v - head) / 8, scal = v - nvec * 8;
+    const uint4* vp = reinterpret_cast<const uint4*>(hp + head);
+    constexpr int kU = 4;
+    for (int j = tid; j < nvec; j += kThreads * kU) {
+      uint4 raw[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (j + kThreads * u < nvec) raw[u] = __ldg(vp + j + kThreads * u);
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        if (j + kThreads * u >= nvec) break;
+        add_word(raw[u].x);
+        add_word(raw[u].y);
+        add_word(raw[u].z);
+        add_word(raw[u].w);
+      }
+    }
+    if (tid < scal) {
+      const uint32_t w = hp[tid < head ? tid : nvec * 8 + tid];
+      atomicAdd(&f.words[w >> 1], 1u << ((w & 1u) * 16u));
+    }
+  }
+  __syncthreads();
+  // ---- counts per group of 32 keys (four threads' vectors of eight counters), their sum, which groups occur
+  {
+    constexpr uint32_t kInf = Elem<T>::kInf2 & 0xFFFFu;
+    constexpr int kN = kHistWords / 4 / kThreads;
+    unsigned int n[kN], occurs[kN], sum = 0, nans = 0, top = 0, found = 0;
+    const bool lead = (lane & 3) == 0;
+    auto group_of = [&](int i) {
+      const int bg = (i * kThreads + tid) >> 2;
+      return bg < kGroups / 2 ? kGroups / 2 + bg : kGroups - 1 - bg;
+    };
+#pragma unroll
+    for (int i = 0; i < kN; ++i) {
+      const int at = i * kThreads + tid;
+      const uint4 q = reinterpret_cast<const uint4*>(f.words)[at];
+      n[i] = (q.x & 0xFFFFu) + (q.x >> 16) + (q.y & 0xFFFFu) + (q.y >> 16) + (q.z & 0xFFFFu) + (q.z >> 16) +
+             (q.w & 0xFFFFu) + (q.w >> 16);
+      const uint32_t mag = static_cast<uint32_t>(at * 8) & 0x7FFFu;
+      if (mag >= kInf) nans += n[i] - (mag == kInf ? q.x & 0xFFFFu : 0u);
+    }
+#pragma unroll
+    for (int i = 0; i < kN; ++i) {
+      n[i] += __shfl_xor_sync(0xffffffffu, n[i], 1);
+      n[i] += __shfl_xor_sync(0xffffffffu, n[i], 2);
+      occurs[i] = __ballot_sync(0xffffffffu, lead && n[i] != 0);
+      found += __popc(occurs[i]);
+    }
+    unsigned int slot = 0;
+    if (lane == 0 && found) slot = atomicAdd(&f.n_list, found);
+    slot = __shfl_sync(0xffffffffu, slot, 0);
+#pragma unroll
+    for (int i = 0; i < kN; ++i) {
+      if (lead) {
+        const int g = group_of(i);
+        s.cnt[g] = n[i];
+        sum += n[i];
+        if (n[i]) {
+          f.list[slot + __popc(occurs[i] & ((1u << lane) - 1u))] = static_cast<unsigned short>(g);
+          top = max(top, static_cast<unsigned int>(g));
+        }
+      }
+      slot += __popc(occurs[i]);
+    }
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    nans = __reduce_add_sync(0xffffffffu, nans);
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0) {
+      atomicAdd(&f.total, sum);
+      if (nans) atomicAdd(&f.nans, nans);
+      atomicMax(&f.top_group, top);
+    }
+  }
+  __syncthreads();
+  if (f.total != static_cast<unsigned int>(v) || f.nans != 0) return false;   // a counter overflowed, or NaNs
+  uint32_t max_key;
+  {
+    const uint32_t key = f.top_group * 32u + static_cast<uint32_t>(lane);
+    max_key = f.top_group * 32u + 31u - __clz(static_cast<int>(__ballot_sync(0xffffffffu, key_count(f, key) != 0)));
+  }
+  const float y_max = mul_rn(key16_float<T>(max_key), inv_temp);
+  // four groups per warp at a time, eight lanes with four keys each
+  for (unsigned int j0 = warp * 4; j0 < f.n_list; j0 += kWarps * 4) {
+    const unsigned int j = j0 + (lane >> 3);
+    unsigned long long m = 0;
+    if (j < f.n_list) {
+      const uint32_t key0 = f.list[j] * 32u + static_cast<uint32_t>(lane & 7) * 4u;
+      // four neighbours' counters are one 64-bit word, in rising order of bits: falling keys below zero
+      const bool neg = key0 < 0x8000u;
+      const uint32_t bits0 = neg ? 0xFFFCu - key0 : key0 - 0x8000u;
+      const uint2 c = *reinterpret_cast<const uint2*>(&f.words[bits0 >> 1]);
+      const uint32_t cnt[4] = {c.x & 0xFFFFu, c.x >> 16, c.y & 0xFFFFu, c.y >> 16};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) m += cnt[e] * key16_mass_of<T>(neg ? key0 + 3 - e : key0 + e, inv_temp, y_max);
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+    if (j < f.n_list && (lane & 7) == 0) s.mass[f.list[j]] = m;
+  }
+  __syncthreads();
+
+  // ---- where the kept prefix ends: the same decisions as in sample_general_kernel
+  uint32_t tau = 0;
+  unsigned long long tie_keep = ~0ull, kept_mass = 0;
+  {
+    uint32_t k_tau = 0;
+    unsigned long long k_ties = ~0ull;
+    const bool has_k = top_k > 0 && top_k < v;
+    const int g0 = kGroups - 1 - 2 * tid;
+    unsigned long long tot_m, tot_c = v, pre_c = 0;
+    const unsigned long long pre_m = block_exscan_u64(s.mass[g0] + s.mass[g0 - 1], s.scan, tot_m);
+    kept_mass = tot_m;
+    if (has_k) {
+      pre_c = block_exscan_u64(s.cnt[g0] + s.cnt[g0 - 1], s.scan, tot_c);
+      search_groups<T>(false, static_cast<unsigned long long>(top_k - 1), inv_temp, y_max, pre_c, pre_m, tot_c, tot_m, s, f);
+      k_tau = f.sel_key;
+      k_ties = static_cast<unsigned long long>(top_k) - f.above_cnt;
+      kept_mass = f.above_mass + k_ties * key16_mass_of<T>(k_tau, inv_temp, y_max);
+    }
+    tau = k_tau;
+    tie_keep = k_ties;
+    if (top_p < 1.0f) {
+      const unsigned long long limit = mass_fraction(static_cast<double>(top_p), kept_mass);
+      __syncthreads();
+      search_groups<T>(true, limit, inv_temp, y_max, pre_c, pre_m, tot_c, tot_m, s, f);
+      const uint32_t p_tau = f.sel_key;
+      const unsigned long long above = f.above_mass, q = key16_mass_of<T>(p_tau, inv_temp, y_max);
+      const unsigned long long p_ties = above > limit ? 0ull : (q == 0 ? ~0ull : (limit - above) / q + 1);
+      if (!has_k || (p_tau != k_tau ? p_tau > k_tau : p_ties < k_ties)) {
+        tau = p_tau;
+        tie_keep = p_ties < f.present ? p_ties : f.present;
+        kept_mass = above + tie_keep * q;
+      }
+    }
+  }
+  if (kept_mass == 0) return false;           // nothing has a mass: the older path picks by position
+
+  Kept k;
+  k.tau = float_to_key(key16_float<T>(tau));
+  k.tie_keep = tie_keep;
+  k.q_tau = key16_mass_of<T>(tau, inv_temp, y_max);
+  k.args = {inv_temp, -y_max};
+  const uint32_t range = max_key - tau;       // keys above the threshold
+  if (range + 2 <= kTable && v <= kTableMaxVocab) {
+    // table[i]: the key max_key - i; tau's entry counts ties, what is below has nothing
+    for (unsigned int i = tid; i < range; i += kThreads) f.table[i] = key16_mass_of<T>(max_key - i, inv_temp, y_max);
+    if (tid == 0) {
+      f.table[range] = 1ull << kTieShift;
+      f.table[range + 1] = 0;
+    }
+    k.table = f.table;
+    k.top2 = ((max_key + 0x8001u) & 0xFFFFu) * 0x00010001u;   // as a signed number, + 1: ~key + 1 = -key
+    k.last2 = (range + 1) * 0x00010001u;
+    __syncthreads();
+    return draw<T, kByTable>(rp, v, k, kept_mass, u24, d, out);
+  }
+  return draw<T, kByExp>(rp, v, k, kept_mass, u24, d, out);
+}
+
+// The last kept element of a row in which nothing has a mass (-1: none is kept).
+template <typename T>
+__device__ int last_kept(const T* rp, int v, uint32_t tau, unsigned long long tie_keep, GeneralSmem& s) {
+  const int tid = threadIdx.x;
+  const int chunk = (v + kThreads - 1) / kThreads;
+  const int begin = min(v, tid * chunk), end = min(v, begin + chunk);
+  unsigned long long ties = 0, total;
+  for (int i = begin; i < end; ++i) ties += float_to_key(Elem<T>::to_float(rp[i])) == tau ? 1u : 0u;
+  unsigned long long rank = block_exscan_u64(ties, s.scan, total);
+  int last = -1;
+  for (int i = begin; i < end; ++i) {
+    const uint32_t key = float_to_key(Elem<T>::to_float(rp[i]));
+    if (key > tau || (key == tau && rank < tie_keep)) last = i;
+    rank += key == tau ? 1u : 0u;
+  }
+  last = __reduce_max_sync(0xffffffffu, last);
+  __syncthreads();
+  if (tid == 0) s.pick = -1;
+  __syncthreads();
+  if ((tid & 31) == 0) atomicMax(&s.pick, last);
+  __syncthreads();
+  return s.pick;
+}
+
+// Largest key of the row, for the whole block.
+template <typename T>
+__device__ uint32_t row_max_key(const T* rp, int v, GeneralSmem& s) {
+  constexpr int kVec = Elem<T>::kVec, kU = 8;
+  const int tid = threadIdx.x;
+  const int head = row_head(rp, v), nvec = (v - head) / kVec, scal = v - nvec * kVec;
+  const uint4* vp = reinterpret_cast<const uint4*>(rp + head);
+  uint32_t w[1] = {~0u};                      // NaN: key 0
+  for (int j = tid; j < nvec; j += kThreads * kU) {
+    uint4 raw[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) raw[u] = j + kThreads * u < nvec ? __ldg(vp + j + kThreads * u) : make_uint4(~0u, ~0u, ~0u, ~0u);
+#pragma unroll
+    for (int u = 0; u < kU; ++u) w[0] = Elem<T>::wmax(w[0], vec_max<T>(raw[u]));
+  }
+  words_to_keys<T>(w);
+  uint32_t top;
+  if constexpr (Elem<T>::kPacked) {
+    top = max(w[0] >> 16, w[0] & 0xFFFFu);
+    top = top == 0 ? 0u : float_to_key(key16_float<T>(top));
+  } else {
+    top = w[0];
+  }
+  if (tid < scal) top = max(top, float_to_key(Elem<T>::to_float(rp[tid < head ? tid : nvec * kVec + tid])));
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (tid == 0) s.max_key = 0;
+  __syncthreads();
+  if ((tid & 31) == 0) atomicMax(&s.max_key, top);
+  __syncthreads();
+  return s.max_key;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1)
 sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v, const long long* __restrict__ row_ids,
                       float inv_temp, int top_k, float top_p, unsigned long long seed, unsigned long long step,
                       int* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ DrawSmem d;
   GeneralSmem& s = *reinterpret_cast<GeneralSmem*>(smem_raw);
   constexpr bool kKey16 = std::is_same<T, __nv_bfloat16>::value;
   unsigned int* hist = reinterpret_cast<unsigned int*>(smem_raw + kGeneralSmemBytes);  // kKey16 only
   const int tid = threadIdx.x;
   const int row = blockIdx.x;
   const T* rp = logits + static_cast<long long>(row) * row_stride;
-  const bool vec_ok = (reinterpret_cast<uintptr_t>(rp) & 15u) == 0;
+  const unsigned long long rid = row_ids ? static_cast<unsigned long long>(row_ids[row])
+                                         : static_cast<unsigned long long>(row);
+  const uint32_t u24 = uniform_u24(seed, rid, step);
+  const bool has_k = top_k > 0 && top_k < v;
   if constexpr (Elem<T>::kPacked) {
     FastSmem& f = *reinterpret_cast<FastSmem*>(smem_raw + kGeneralSmemBytes);
-    const unsigned long long rid = row_ids ? static_cast<unsigned long long>(row_ids[row])
-                                           : static_cast<unsigned long long>(row);
-    if (sample_row16<T>(rp, v, vec_ok, inv_temp, top_k, top_p, uniform_u24(seed, rid, step), s, f, out + row)) return;
+    if ((has_k || top_p < 1.0f) && sample_row16<T>(rp, v, inv_temp, top_k, top_p, u24, s, f, d, out + row)) return;
     __syncthreads();
   }
-
-  // ---- row maximum
-  uint32_t tmax = 0;
-  for_each_key<T>(rp, v, [&](uint32_t key, int) { tmax = max(tmax, key); });
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) tmax = max(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
-  if (tid == 0) s.max_key = 0;
-  __syncthreads();
-  if ((tid & 31) == 0) atomicMax(&s.max_key, tmax);
-  __syncthreads();
-  const float y_max = mul_rn(key_to_float(s.max_key), inv_temp);
+  const float y_max = mul_rn(key_to_float(row_max_key(rp, v, s)), inv_temp);
+  Kept k;
+  k.args = {inv_temp, -y_max};
+  k.q_tau = 0;
+  if (!has_k && top_p >= 1.0f) {              // everything is kept: the sums of the draw are the only pass
+    k.tie_keep = 0;
+    if (!draw<T, kAll>(rp, v, k, 0, u24, d, out + row) && tid == 0) out[row] = v - 1;
+    return;
+  }
 
   // ---- where the kept prefix ends: (tau, number of ties at tau that are kept)
   uint32_t tau = 0;                     // threshold key
@@ -1520,28 +1761,25 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
     uint32_t k_tau = 0;
     unsigned long long k_ties = ~0ull;
     unsigned long long zk;
-    const bool has_k = top_k > 0 && top_k < v;
     if (has_k) {
       if constexpr (kKey16) {
         unsigned long long unused;
-        descend16<T>(rp, v, vec_ok, inv_temp, y_max, false, static_cast<unsigned long long>(top_k - 1), s, hist,
-                     k_tau, k_above_cnt, k_above_mass, unused);
+        descend16<T>(rp, v, inv_temp, y_max, false, static_cast<unsigned long long>(top_k - 1), s, hist, k_tau,
+                     k_above_cnt, k_above_mass, unused);
       } else {
-        descend<T>(rp, v, vec_ok, inv_temp, y_max, false, static_cast<unsigned long long>(top_k - 1), s, k_tau,
-                   k_above_cnt, k_above_mass);
+        descend<T>(rp, v, inv_temp, y_max, false, static_cast<unsigned long long>(top_k - 1), s, k_tau, k_above_cnt,
+                   k_above_mass);
       }
       k_ties = static_cast<unsigned long long>(top_k) - k_above_cnt;
       const float y = mul_rn(key_to_float(k_tau), inv_temp);
       zk = k_above_mass + k_ties * mass_fixed(exp_det(sub_rn(y, y_max)));
     } else {
       // everything is kept by the count criterion: Z = total mass
-      unsigned long long local = 0;
-      for_each_key<T>(rp, v, [&](uint32_t key, int) {
-        const float y = mul_rn(key_to_float(key), inv_temp);
-        local += mass_fixed(exp_det(sub_rn(y, y_max)));
-      });
-      unsigned long long total;
-      block_exscan_u64(local, s.scan, total);
+      const int len = ((v + kWarps - 1) / kWarps + 7) / 8 * 8;
+      const int b = min(v, (tid >> 5) * len);
+      unsigned long long part, unused, total;
+      sum_range<T, kAll>(rp, b, min(v, b + len), k, part, unused);
+      block_exscan_u64((tid & 31) == 0 ? part : 0ull, s.scan, total);
       zk = total;
     }
     tau = has_k ? k_tau : 0u;
@@ -1552,10 +1790,9 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
       uint32_t p_tau;
       unsigned long long p_above_cnt, p_above_mass, p_present = 0;
       if constexpr (kKey16) {
-        descend16<T>(rp, v, vec_ok, inv_temp, y_max, true, limit, s, hist, p_tau, p_above_cnt, p_above_mass,
-                     p_present);
+        descend16<T>(rp, v, inv_temp, y_max, true, limit, s, hist, p_tau, p_above_cnt, p_above_mass, p_present);
       } else {
-        descend<T>(rp, v, vec_ok, inv_temp, y_max, true, limit, s, p_tau, p_above_cnt, p_above_mass);
+        descend<T>(rp, v, inv_temp, y_max, true, limit, s, p_tau, p_above_cnt, p_above_mass);
       }
       // element i (in sorted order) is kept while the mass before it is <= limit
       const float y = mul_rn(key_to_float(p_tau), inv_temp);
@@ -1597,100 +1834,14 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
   }
 
   // ---- draw: invert the CDF over the kept set in token-id order
-  const unsigned long long rid = row_ids ? static_cast<unsigned long long>(row_ids[row])
-                                         : static_cast<unsigned long long>(row);
-  const unsigned long long target = mass_scale_u24(uniform_u24(seed, rid, step), kept_mass);
-  if (tid == 0) s.pick = -1;
-  // Thread t owns the elements [t * chunk, (t + 1) * chunk) and walks them in order, up to three
-  // times: the ties before a thread and the kept mass before it come from two block scans.
-  constexpr int kVec = Elem<T>::kVec;
-  const int chunk = ((v + kThreads - 1) / kThreads + 7) & ~7;
-  const int begin = min(v, tid * chunk), end = min(v, begin + chunk);
-  auto walk = [&](auto&& f) {
-    int i = begin;
-    if (vec_ok) {
-      for (; i + kVec <= end; i += kVec) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(rp + i);
-        const T* e = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-        for (int j = 0; j < kVec; ++j) f(float_to_key(Elem<T>::to_float(e[j])), i + j);
-      }
-    }
-    for (; i < end; ++i) f(float_to_key(Elem<T>::to_float(rp[i])), i);
-  };
-  unsigned long long my_ties = 0;
-  walk([&](uint32_t key, int) { my_ties += (key == tau) ? 1u : 0u; });
-  unsigned long long tie_total;
-  const unsigned long long tie_first = block_exscan_u64(my_ties, s.scan, tie_total);
-  // Visit the kept elements of the chunk in id order. The walk only sets a flag per element
-  // (64 at a time); the masses are then computed for the flagged ones alone, so that a warp
-  // runs the exponential as often as its busiest lane has kept elements, not once per element.
-  auto walk_kept = [&](auto&& f) {
-    unsigned long long tie_off = tie_first, bits = 0;
-    int bits_base = begin;
-    auto flush = [&]() {
-      while (bits) {
-        const int j = __ffsll(static_cast<long long>(bits)) - 1;
-        bits &= bits - 1;
-        const int i = bits_base + j;
-        f(float_to_key(Elem<T>::to_float(rp[i])), i);
-      }
-    };
-    walk([&](uint32_t key, int i) {
-      if (i - bits_base == 64) {
-        flush();
-        bits_base = i;
-      }
-      bool kept = key > tau;
-      if (key == tau) {
-        kept = tie_off < tie_keep;
-        ++tie_off;
-      }
-      bits |= static_cast<unsigned long long>(kept ? 1u : 0u) << (i - bits_base);
-    });
-    flush();
-  };
-  auto mass_of = [&](uint32_t key) {
-    const float y = mul_rn(key_to_float(key), inv_temp);
-    return static_cast<unsigned long long>(mass_fixed(exp_det(sub_rn(y, y_max))));
-  };
-  unsigned long long my_mass = 0;
-  int last_kept = -1;
-  walk_kept([&](uint32_t key, int i) {
-    my_mass += mass_of(key);
-    last_kept = i;
-  });
-  unsigned long long mass_total;
-  const unsigned long long mass_first = block_exscan_u64(my_mass, s.scan, mass_total);
-  if (mass_first <= target && mass_first + my_mass > target) {  // exactly one thread
-    unsigned long long acc = mass_first;
-    int found = -1;
-    walk_kept([&](uint32_t key, int i) {
-      const unsigned long long q = mass_of(key);
-      acc += q;
-      if (found < 0 && q != 0 && acc > target) found = i;
-    });
-    s.pick = found;
-  }
-  __syncthreads();
+  k.tau = tau;
+  k.tie_keep = tie_keep;
+  k.q_tau = mass_fixed(exp_det(sub_rn(mul_rn(key_to_float(tau), inv_temp), y_max)));
+  if (draw<T, kByExp>(rp, v, k, kept_mass, u24, d, out + row)) return;
   // target == kept_mass can only happen when kept_mass is 0 (all masses underflowed):
-  // fall back to the last kept element, or the row maximum position.
-  if (s.pick < 0) {
-    const int cand = last_kept;
-    int best = cand;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
-    __syncthreads();
-    if ((tid & 31) == 0) s.red[tid >> 5] = best;
-    __syncthreads();
-    if (tid == 0) {
-      int b = -1;
-      for (int w = 0; w < kWarps; ++w) b = max(b, s.red[w]);
-      s.pick = b < 0 ? 0 : b;
-    }
-    __syncthreads();
-  }
-  if (tid == 0) out[row] = s.pick;
+  // fall back to the last kept element
+  const int last = last_kept<T>(rp, v, tau, tie_keep, s);
+  if (tid == 0) out[row] = last < 0 ? 0 : last;
 }
 
 template <typename T, int NW>

@@ -154,3 +154,29 @@ def test_sampler_16_bit_rows_without_top_k(cuda_device, dtype, vocab):
         for step in (0, 1):
             tok = sample(logits, top_k=top_k, top_p=top_p, temperature=temp, seed=5, step=step)
             assert torch.equal(tok.cpu(), _cpu(logits, top_k, top_p, temp, 5, step)), (top_k, top_p, temp)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, torch.float16])
+@pytest.mark.parametrize("vocab", [3, 1025, 33001])
+def test_sampler_without_small_top_k_special_values(cuda_device, dtype, vocab):
+    """Draws over all elements, and over what a top-p or a large top-k keeps: thresholds close to the
+    maximum and far below it (masses from the table, and computed), rows that start off a 16-byte
+    boundary, masses of 2^32 by rounding, nothing that has a mass."""
+    g = torch.Generator(device=cuda_device).manual_seed(vocab)
+    x = torch.randn(4, vocab, device=cuda_device, generator=g) * 2
+    u = torch.rand(x.shape, device=cuda_device, generator=g)
+    values = {"plain": x, "wide": x * 10, "below_zero": -x.abs() - 1, "masked": torch.where(u < 0.99, float("-inf"), x),
+              "lowest": torch.where(u < 0.9, torch.finfo(dtype).min, x), "tiny": x * 1e-6, "zeros": (x * 0).where(u < 0.7, -1.0),
+              "inf": torch.where(u > 0.999, float("inf"), x), "nan": torch.where(u < 0.01, float("nan"), x),
+              "all_masked": torch.full_like(x, float("-inf"))}
+    buf = torch.empty(4 * (vocab + 1) + 3, dtype=dtype, device=cuda_device)
+    for name, val in values.items():
+        for off, width in ((0, vocab), (3, vocab + 1)):
+            logits = buf[off:off + 4 * width].view(4, width)[:, :vocab]
+            logits.copy_(val)
+            for top_k, top_p, temperature in ((None, None, 0.7), (None, 0.9, 1.0), (None, 0.9999, 2.0), (1500, 0.8, 1.0),
+                                              (1500, None, 0.3)):
+                k = None if top_k is not None and top_k >= vocab else top_k
+                tok = sample(logits, top_k=k, top_p=top_p, temperature=temperature, seed=8, step=off)
+                ref = _cpu(logits, k, top_p, temperature, 8, off)
+                assert torch.equal(tok.cpu(), ref), (name, off, k, top_p)
