@@ -53,7 +53,7 @@ struct Elem<float> {
   __device__ static uint32_t wmax(uint32_t a, uint32_t b) {
     return __float_as_uint(fmaxf(__uint_as_float(a), __uint_as_float(b)));
   }
-  __device__ static bool any_ge(uint32_t a, uint32_t b) { return __uint_as_float(a) >= __uint_as_float(b); }
+  static __device__ bool any_ge(uint32_t a, uint32_t b) { return __uint_as_float(a) >= __uint_as_float(b); }
 };
 template <>
 struct Elem<__nv_bfloat16> {
@@ -67,7 +67,7 @@ struct Elem<__nv_bfloat16> {
     asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
   }
-  __device__ static bool any_ge(uint32_t a, uint32_t b) {
+  static __device__ bool any_ge(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("{\n\t.reg .pred p, q;\n\tsetp.ge.bf16x2 p|q, %1, %2;\n\tor.pred p, p, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(d)
@@ -87,7 +87,7 @@ struct Elem<__half> {
     asm("max.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
   }
-  __device__ static bool any_ge(uint32_t a, uint32_t b) {
+  static __device__ bool any_ge(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("{\n\t.reg .pred p, q;\n\tsetp.ge.f16x2 p|q, %1, %2;\n\tor.pred p, p, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(d)
