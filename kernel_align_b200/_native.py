@@ -83,15 +83,56 @@ def cuda() -> ctypes.CDLL:
          c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     )
     _bind(lib, "ka_grpo_loss_bwd", c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p])
+    # prototypes are set here, once: setting them costs a call several microseconds
+    p, i, ll, f, ull = c_void_p, c_int, c_longlong, c_float, c_ulonglong
+    _bind(lib, "ka_rmsnorm", c_int, [p, p, p, p, p, i, i, f, i, p])
+    _bind(lib, "ka_rmsnorm_bwd", c_int, [p, p, p, p, p, p, p, i, i, f, p])
+    _bind(lib, "ka_rope", c_int, [p, ll, p, p, p, i, i, i, i, p])
+    _bind(lib, "ka_qkv_rope", c_int, [p, ll, i, p, p, p, p, p, p, i, i, i, i, i, p])
+    _bind(lib, "ka_swiglu", c_int, [p, p, ll, p, i, i, i, p])
+    _bind(lib, "ka_swiglu_bwd", c_int, [p, p, ll, p, p, p, ll, i, i, i, p])
+    _bind(lib, "ka_attention_fwd", c_int, [p, ll, p, ll, p, ll, p, ll, p, i, i, i, i, i, f, i, p, ull, p])
+    _bind(lib, "ka_attention_bwd", c_int,
+          [p, ll, p, ll, p, ll, p, ll, p, ll, p, p, p, ll, p, ll, p, ll, i, i, i, i, i, f, i, p, ull, p])
+    _bind(lib, "ka_attention_decode", c_int, [p, p, p, p, p, i, i, i, i, i, f, p])
+    _bind(lib, "ka_decode_qkv_rope_cache", c_int, [p, ll, p, p, p, p, p, p, p, i, i, i, i, p])
+    _bind(lib, "ka_adamw_step", c_int, [p, p, p, i, p, p, ll, f, f, f, f, f, i, f, i, p])
+    _bind(lib, "ka_gemm_bf16", c_int, [p, ll, i, p, ll, i, p, ll, i, i, i, i, p, i, ull, p])
+    _bind(lib, "ka_gemm_skinny_bf16", c_int, [p, ll, p, ll, p, ll, i, i, i, p, ull, p])
+    _bind(lib, "ka_lmhead_logits_grad", c_int, [p, p, p, p, p, p, ll, i, i, i, f, i, p, i, ull, p])
+    _bind(lib, "ka_gemm_rs_exchange_bytes", c_size_t, [i, i, i])
+    _bind(lib, "ka_gemm_rs_rows_per_rank", c_int, [i, i])
+    _bind(lib, "ka_ag_gemm_exchange_bytes", c_size_t, [i, i, i])
+    _bind(lib, "ka_gemm_reduce_scatter", c_int, [p, ll, p, ll, i, p, p, p, i, i, i, i, i, c_uint, p, i, ull, p])
+    _bind(lib, "ka_gemm_tree8_scratch_bytes", c_size_t, [i])
+    _bind(lib, "ka_gemm_tree8", c_int, [p, ll, p, ll, i, p, p, p, i, i, i, p, i, ull, p])
+    _bind(lib, "ka_all_gather_gemm", c_int, [p, p, ll, i, p, ll, p, i, i, i, i, i, c_uint, p, i, ull, p])
     return lib
+
+
+def _device_index(device) -> int:
+    import torch
+
+    return device.index if device.index is not None else torch.cuda.current_device()
 
 
 def stream_ptr(device) -> int:
     """The current stream of a CUDA device as the integer the kernels take."""
     import torch
 
-    index = device.index if device.index is not None else torch.cuda.current_device()
-    return torch._C._cuda_getCurrentRawStream(index)
+    return torch._C._cuda_getCurrentRawStream(_device_index(device))
+
+
+@lru_cache(maxsize=None)
+def _sm_count(index: int) -> int:
+    import torch
+
+    return torch.cuda.get_device_properties(index).multi_processor_count
+
+
+def sm_count(device) -> int:
+    """SMs of a CUDA device (asked once per device ordinal)."""
+    return _sm_count(_device_index(device))
 
 
 DTYPE_CODES = {"torch.float32": 0, "torch.bfloat16": 1, "torch.float16": 2}

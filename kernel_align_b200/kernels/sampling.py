@@ -41,7 +41,6 @@ class SamplerBackend(nn.Module):
     def set_rng_state(self, state: dict) -> None:
         self.seed, self.step = int(state["seed"]), int(state["step"])
 
-    @torch.inference_mode()
     def sample(self, logits, top_k: Optional[int] = None, top_p: Optional[float] = None,
                temperature: float = 1.0, deterministic: bool = True, *, row_ids=None,
                step: Optional[int] = None) -> torch.Tensor:
@@ -50,11 +49,12 @@ class SamplerBackend(nn.Module):
         Every draw is reproducible, so ``deterministic`` is accepted and ignored. Each call
         consumes one step of the stream unless ``step`` is given explicitly.
         """
-        if logits.dim() == 1:
-            logits = logits.unsqueeze(0)
         use_step = self.step if step is None else int(step)
-        out = _sampling.sample(logits, top_k=top_k, top_p=top_p, temperature=temperature,
-                               seed=self.seed, step=use_step, row_ids=row_ids)
+        with torch.inference_mode():     # not as a decorator, which makes a new context manager by copying one
+            if logits.dim() == 1:
+                logits = logits.unsqueeze(0)
+            out = _sampling.sample(logits, top_k=top_k, top_p=top_p, temperature=temperature,
+                                   seed=self.seed, step=use_step, row_ids=row_ids)
         if step is None:
             self.step += 1
         return out

@@ -7,7 +7,7 @@ backend name only (rl_engine/kernels/registry.py:41-55).
 from __future__ import annotations
 
 import math
-from ctypes import c_float, c_int, c_longlong, c_ulonglong, c_void_p
+from ctypes import c_float, c_int, c_void_p
 from typing import Optional
 
 import torch
@@ -16,6 +16,13 @@ from .. import _native
 from .fused_logp import default_timeout_ns
 from .gemm import status_buffer
 from ..utils.profiler import profiled
+
+
+def _token_view(t: torch.Tensor) -> torch.Tensor:
+    """``t`` ``[B, L, H, D]`` itself if the kernels can walk it as rows of tokens, else a contiguous copy."""
+    s0, s1, s2, s3 = t.stride()
+    ok = s3 == 1 and s2 == t.shape[3] and s0 == t.shape[1] * s1 and s1 % 8 == 0 and t.data_ptr() % 16 == 0
+    return t if ok else t.contiguous()
 
 
 @profiled("attention")
@@ -47,22 +54,13 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal: bool
     if d != 128 or q.dtype != torch.bfloat16:
         raise ValueError("the sm_100a attention kernel takes bf16 with head_dim 128")
 
-    def tok_view(t, heads):
-        ok = t.stride(3) == 1 and t.stride(2) == d and t.stride(0) == l * t.stride(1) and t.stride(1) % 8 == 0 \
-            and t.data_ptr() % 16 == 0
-        return t if ok else t.contiguous()
-
-    q, k, v = tok_view(q, hq), tok_view(k, hkv), tok_view(v, hkv)
+    q, k, v = _token_view(q), _token_view(k), _token_view(v)
     out = torch.empty(b, l, hq, d, dtype=torch.bfloat16, device=q.device)
     lse = torch.empty(b, hq, l, dtype=torch.float32, device=q.device) if return_lse else None
-    lib = _native.cuda()
-    fn = lib.ka_attention_fwd
-    fn.restype = c_int
-    fn.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p,
-                   c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_ulonglong, c_void_p]
-    rc = fn(q.data_ptr(), q.stride(1), k.data_ptr(), k.stride(1), v.data_ptr(), v.stride(1), out.data_ptr(),
-            out.stride(1), lse.data_ptr() if lse is not None else None, b, l, hq, hkv, d, sc, int(causal),
-            status_buffer(q.device).data_ptr(), default_timeout_ns(), torch.cuda.current_stream(q.device).cuda_stream)
+    rc = _native.cuda().ka_attention_fwd(
+        q.data_ptr(), q.stride(1), k.data_ptr(), k.stride(1), v.data_ptr(), v.stride(1), out.data_ptr(), hq * d,
+        lse.data_ptr() if lse is not None else None, b, l, hq, hkv, d, sc, int(causal),
+        status_buffer(q.device).data_ptr(), default_timeout_ns(), _native.stream_ptr(q.device))
     if rc != 0:
         raise RuntimeError(f"ka_attention_fwd rejected its arguments (code {rc})")
     return (out, lse) if return_lse else out
@@ -79,12 +77,7 @@ def attention_backward(q, k, v, out, d_out, lse, *, causal: bool = True, scale: 
     if q.device.type != "cuda" or d != 128 or q.dtype != torch.bfloat16:
         return _attention_backward_math(q, k, v, out, d_out, lse, causal, sc)
 
-    def tok(t):
-        ok = t.stride(3) == 1 and t.stride(2) == d and t.stride(0) == l * t.stride(1) and t.stride(1) % 8 == 0 \
-            and t.data_ptr() % 16 == 0
-        return t if ok else t.contiguous()
-
-    q, k, v, out, d_out = tok(q), tok(k), tok(v), tok(out), tok(d_out)
+    q, k, v, out, d_out = (_token_view(t) for t in (q, k, v, out, d_out))
     if out.data_ptr() % 16:     # contiguous at an odd offset: no tensor map looks at it, and it is read 16 bytes at a time
         out = out.clone()
     dq = torch.empty(b, l, hq, d, dtype=torch.bfloat16, device=q.device)
@@ -92,15 +85,11 @@ def attention_backward(q, k, v, out, d_out, lse, *, causal: bool = True, scale: 
     dv = torch.empty(b, l, hkv, d, dtype=torch.bfloat16, device=q.device)
     delta = torch.empty(b, hq, l, dtype=torch.float32, device=q.device)
     lse = lse.contiguous()
-    fn = _native.cuda().ka_attention_bwd
-    fn.restype = c_int
-    fn.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p,
-                   c_longlong, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong,
-                   c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_ulonglong, c_void_p]
-    rc = fn(q.data_ptr(), q.stride(1), k.data_ptr(), k.stride(1), v.data_ptr(), v.stride(1), out.data_ptr(),
-            out.stride(1), d_out.data_ptr(), d_out.stride(1), lse.data_ptr(), delta.data_ptr(), dq.data_ptr(),
-            dq.stride(1), dk.data_ptr(), dk.stride(1), dv.data_ptr(), dv.stride(1), b, l, hq, hkv, d, sc, int(causal),
-            status_buffer(q.device).data_ptr(), default_timeout_ns(), torch.cuda.current_stream(q.device).cuda_stream)
+    rc = _native.cuda().ka_attention_bwd(
+        q.data_ptr(), q.stride(1), k.data_ptr(), k.stride(1), v.data_ptr(), v.stride(1), out.data_ptr(),
+        out.stride(1), d_out.data_ptr(), d_out.stride(1), lse.data_ptr(), delta.data_ptr(), dq.data_ptr(), hq * d,
+        dk.data_ptr(), hkv * d, dv.data_ptr(), hkv * d, b, l, hq, hkv, d, sc, int(causal),
+        status_buffer(q.device).data_ptr(), default_timeout_ns(), _native.stream_ptr(q.device))
     if rc != 0:
         raise RuntimeError(f"ka_attention_bwd rejected its arguments (code {rc})")
     return dq, dk, dv

@@ -6,7 +6,6 @@ rotation / cache write, AdamW). CPU tensors fall back to the equivalent PyTorch 
 from __future__ import annotations
 
 import math
-from ctypes import c_float, c_int, c_longlong, c_void_p
 
 import torch
 
@@ -33,10 +32,8 @@ def attention_decode(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tens
         return out
     out = torch.empty_like(q)
     fn = _native.cuda().ka_attention_decode
-    fn.restype = c_int
-    fn.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p]
     rc = fn(q.contiguous().data_ptr(), cache_k.data_ptr(), cache_v.data_ptr(), lens.to(torch.int32).contiguous().data_ptr(),
-            out.data_ptr(), b, hq, hkv, d, max_len, sc, torch.cuda.current_stream(q.device).cuda_stream)
+            out.data_ptr(), b, hq, hkv, d, max_len, sc, _native.stream_ptr(q.device))
     if rc != 0:
         raise RuntimeError(f"ka_attention_decode failed ({rc})")
     return out
@@ -68,12 +65,9 @@ def decode_qkv_rope_cache(qkv: torch.Tensor, pos: torch.Tensor, slot: torch.Tens
         raise ValueError("decode_qkv_rope_cache takes a row-major qkv and contiguous caches")
     q = torch.empty(b, hq, d, dtype=qkv.dtype, device=qkv.device)
     fn = _native.cuda().ka_decode_qkv_rope_cache
-    fn.restype = c_int
-    fn.argtypes = [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
-                   c_int, c_int, c_int, c_void_p]
     rc = fn(qkv.data_ptr(), qkv.stride(0), pos.data_ptr(), slot.data_ptr(), cos.data_ptr(), sin.data_ptr(),
             q.data_ptr(), cache_k.data_ptr(), cache_v.data_ptr(), b, hq, hkv, cache_k.shape[1],
-            torch.cuda.current_stream(qkv.device).cuda_stream)
+            _native.stream_ptr(qkv.device))
     if rc != 0:
         raise RuntimeError(f"ka_decode_qkv_rope_cache failed ({rc})")
     return q
@@ -116,13 +110,10 @@ class FusedAdamW:
                 p.copy_(st["master"].to(p.dtype))
                 continue
             fn = _native.cuda().ka_adamw_step
-            fn.restype = c_int
-            fn.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_float, c_float, c_float,
-                           c_float, c_float, c_int, c_float, c_int, c_void_p]
-            sms = torch.cuda.get_device_properties(p.device).multi_processor_count
+            sms = _native.sm_count(p.device)
             rc = fn(p.data_ptr(), st["master"].data_ptr(), g.data_ptr(), int(g.dtype == torch.bfloat16),
                     st["m"].data_ptr(), st["v"].data_ptr(), p.numel(), self.lr, b1, b2, self.eps, self.weight_decay,
-                    self.step_count, grad_scale, sms, torch.cuda.current_stream(p.device).cuda_stream)
+                    self.step_count, grad_scale, sms, _native.stream_ptr(p.device))
             if rc != 0:
                 raise RuntimeError(f"ka_adamw_step failed ({rc})")
 

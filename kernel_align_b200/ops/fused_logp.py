@@ -319,8 +319,8 @@ def _lmhead_logp_forward(
     n_panels = -(-m // (panel_rows // world)) if sharded else -(-m // panel_rows)
     peer_arr = (ctypes.c_void_p * world)(*group.exchange_ptrs) if world > 1 else None
     gather_arr = (ctypes.c_void_p * world)(*group.gather_arena_ptrs(k)) if sharded else None
-    props = torch.cuda.get_device_properties(hidden.device)
-    stream = torch.cuda.current_stream(hidden.device).cuda_stream
+    sms = _native.sm_count(hidden.device)
+    stream = _native.stream_ptr(hidden.device)
 
     def launch(g: int, cg: int, m_fast: int = 0, hint: int = 0) -> None:
         """Enqueue one forward with the given schedule (consumes the epochs of its panels)."""
@@ -337,7 +337,7 @@ def _lmhead_logp_forward(
                 ws.buf.data_ptr(), ws.nbytes, peer_arr, gather_arr,
                 m, k, v_global, hi - lo, lo, world, rank,
                 epoch & 0xFFFFFFFF, float(scale), panel_rows, 1 if gather_output else 0, g, cg, m_fast, hint,
-                props.multi_processor_count, default_timeout_ns(), stream,
+                sms, default_timeout_ns(), stream,
             )
         else:
             rc = lib.ka_lmhead_logp_forward_sched(
@@ -345,7 +345,7 @@ def _lmhead_logp_forward(
                 lse.data_ptr() if lse is not None else None,
                 ws.buf.data_ptr(), ws.nbytes, peer_arr,
                 m, k, v_global, hi - lo, lo, world, rank,
-                epoch & 0xFFFFFFFF, float(scale), panel_rows, g, cg, m_fast, hint, props.multi_processor_count,
+                epoch & 0xFFFFFFFF, float(scale), panel_rows, g, cg, m_fast, hint, sms,
                 default_timeout_ns(), stream,
             )
         if rc != 0:
@@ -425,12 +425,8 @@ def _logp_backward(hidden, weight, ids, lse, g, scale, vocab, group, need_dh, ne
         m += pad
     lib = _native.cuda()
     fn = lib.ka_lmhead_logits_grad
-    fn.restype = ctypes.c_int
-    fn.argtypes = [ctypes.c_void_p] * 6 + [ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_int,
-                                           ctypes.c_float, ctypes.c_int, ctypes.c_void_p, ctypes.c_int,
-                                           ctypes.c_ulonglong, ctypes.c_void_p]
-    props = torch.cuda.get_device_properties(h2.device)
-    stream = torch.cuda.current_stream(h2.device).cuda_stream
+    sms = _native.sm_count(h2.device)
+    stream = _native.stream_ptr(h2.device)
     rows_per_panel = max(256, min(m, (_GRAD_PANEL_BYTES // max(1, v_local * 2)) // 256 * 256))
     d_hidden = torch.empty_like(h2) if need_dh else None
     d_weight = None
@@ -440,7 +436,7 @@ def _logp_backward(hidden, weight, ids, lse, g, scale, vocab, group, need_dh, ne
         d_logits = torch.empty(r1 - r0, v_local, dtype=torch.bfloat16, device=h2.device)
         rc = fn(h2[r0:r1].data_ptr(), w.data_ptr(), ids64[r0:r1].data_ptr(), lse32[r0:r1].data_ptr(),
                 g32[r0:r1].data_ptr(), d_logits.data_ptr(), v_local, r1 - r0, v_local, k, float(scale), lo,
-                _gemm.status_buffer(h2.device).data_ptr(), props.multi_processor_count, default_timeout_ns(),
+                _gemm.status_buffer(h2.device).data_ptr(), sms, default_timeout_ns(),
                 stream)
         if rc != 0:
             raise RuntimeError(f"ka_lmhead_logits_grad rejected its arguments (code {rc})")

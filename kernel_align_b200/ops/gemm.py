@@ -18,7 +18,6 @@ same order), which gives the same bits; ``KA_GEMM_SKINNY=0`` keeps everything on
 from __future__ import annotations
 
 import os
-from ctypes import c_int, c_longlong, c_ulonglong, c_void_p
 
 from typing import Optional
 
@@ -46,24 +45,7 @@ def check_status(device: torch.device) -> None:
         raise RuntimeError(f"gemm kernel gave up: code {st[0]} at site {st[1]}, block {st[2]}, aux {st[3:6]}")
 
 
-def _fn():
-    lib = _native.cuda()
-    fn = lib.ka_gemm_bf16
-    fn.restype = c_int
-    fn.argtypes = [c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_int, c_int,
-                   c_int, c_void_p, c_int, c_ulonglong, c_void_p]
-    return fn
-
-
 SKINNY_MAX_ROWS = 64
-
-
-def _skinny_fn():
-    fn = _native.cuda().ka_gemm_skinny_bf16
-    fn.restype = c_int
-    fn.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_int, c_void_p,
-                   c_ulonglong, c_void_p]
-    return fn
 
 
 @profiled("gemm_skinny")
@@ -87,9 +69,9 @@ def gemm_skinny(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = 
         out = torch.empty(m, n, dtype=torch.bfloat16, device=a.device)
     else:
         _check_out(out, m, n, torch.bfloat16)
-    rc = _skinny_fn()(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), m, n, k,
-                      status_buffer(a.device).data_ptr(), default_timeout_ns(),
-                      torch.cuda.current_stream(a.device).cuda_stream)
+    rc = _native.cuda().ka_gemm_skinny_bf16(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(),
+                                            out.stride(0), m, n, k, status_buffer(a.device).data_ptr(),
+                                            default_timeout_ns(), _native.stream_ptr(a.device))
     if rc != 0:
         raise RuntimeError(f"ka_gemm_skinny_bf16 rejected its arguments (code {rc})")
     return out
@@ -128,10 +110,10 @@ def gemm_bi(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b:
         out = torch.empty(m, n, dtype=out_dtype, device=a.device)
     else:
         _check_out(out, m, n, out_dtype)
-    props = torch.cuda.get_device_properties(a.device)
-    rc = _fn()(a.data_ptr(), a.stride(0), int(trans_a), b.data_ptr(), b.stride(0), int(trans_b), out.data_ptr(),
-               out.stride(0), int(out_dtype == torch.float32), m, n, k, status_buffer(a.device).data_ptr(),
-               props.multi_processor_count, default_timeout_ns(), torch.cuda.current_stream(a.device).cuda_stream)
+    rc = _native.cuda().ka_gemm_bf16(a.data_ptr(), a.stride(0), int(trans_a), b.data_ptr(), b.stride(0), int(trans_b),
+                                     out.data_ptr(), out.stride(0), int(out_dtype == torch.float32), m, n, k,
+                                     status_buffer(a.device).data_ptr(), _native.sm_count(a.device),
+                                     default_timeout_ns(), _native.stream_ptr(a.device))
     if rc != 0:
         raise RuntimeError(f"ka_gemm_bf16 rejected its arguments (code {rc})")
     return out

@@ -18,7 +18,7 @@ from ..utils.profiler import profiled
 def group_advantages(rewards: torch.Tensor, group_size: int, eps: float = 1e-4) -> torch.Tensor:
     """``(r - mean_group) / (std_group + eps)`` over consecutive groups of ``group_size``
     rewards (unbiased standard deviation)."""
-    r = rewards.reshape(-1).float().contiguous()
+    r = (rewards if rewards.dim() == 1 else rewards.reshape(-1)).float().contiguous()
     if r.numel() % group_size:
         raise ValueError("the number of rewards must be a multiple of the group size")
     adv = torch.empty_like(r)
@@ -33,12 +33,12 @@ def group_advantages(rewards: torch.Tensor, group_size: int, eps: float = 1e-4) 
         rc = fn(r.data_ptr(), adv.data_ptr(), n_groups, group_size, eps)
     if rc != 0:
         raise RuntimeError(f"grpo advantages failed ({rc})")
-    return adv.reshape(rewards.shape)
+    return adv if rewards.dim() == 1 else adv.reshape(rewards.shape)
 
 
 class _GrpoLossFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, logp_new, logp_old, logp_ref, adv, mask, eps_low, eps_high, beta, seq_mean):
+    def forward(ctx, logp_new, logp_old, logp_ref, adv, mask, eps_low, eps_high, beta, seq_mean, with_stats):
         ctx.set_materialize_grads(False)
         n_seq, seq_len = logp_new.shape
         ln = logp_new.float().contiguous()
@@ -47,27 +47,30 @@ class _GrpoLossFn(torch.autograd.Function):
         a = adv.float().contiguous()
         ctx.shape = (n_seq, seq_len)
         ctx.cuda = ln.device.type == "cuda"
-        out = torch.empty(3, dtype=torch.float32, device=ln.device)
-        ctx.mark_non_differentiable(out)
         if ctx.cuda:
             # bytes and floats are read as they are, anything else is converted first
             if mask is not None and mask.dtype not in (torch.bool, torch.uint8, torch.float32):
                 mask = mask.to(torch.uint8)
             m = mask.contiguous() if mask is not None else None
             raw = torch.empty_like(ln)
-            ws = torch.empty(4 * n_seq, dtype=torch.float32, device=ln.device)
+            ws = torch.empty(4 * n_seq + 3, dtype=torch.float32, device=ln.device)   # per sequence, then the statistics
             loss = torch.empty((), dtype=torch.float32, device=ln.device)
+            out = torch.empty(3, dtype=torch.float32, device=ln.device) if with_stats else None
             rc = _native.cuda().ka_grpo_loss_fwd(
                 ln.data_ptr(), lo.data_ptr(), lr.data_ptr() if lr is not None else None, a.data_ptr(),
                 m.data_ptr() if m is not None else None, int(m is not None and m.dtype == torch.float32), n_seq,
                 seq_len, eps_low, eps_high, beta, int(seq_mean), raw.data_ptr(), ws.data_ptr(), loss.data_ptr(),
-                out.data_ptr(), _native.stream_ptr(ln.device))
+                out.data_ptr() if with_stats else ws.data_ptr() + 16 * n_seq, _native.stream_ptr(ln.device))
             if rc != 0:
                 raise RuntimeError(f"ka_grpo_loss_fwd failed ({rc})")
             ctx.save_for_backward(raw, ws)
+            if not with_stats:
+                return loss
+            ctx.mark_non_differentiable(out)
             return loss, out
         m = mask.to(torch.uint8).contiguous() if mask is not None else None
         grad = torch.empty_like(ln)
+        out = torch.empty(3, dtype=torch.float32)
         fn = _native.cpu().ka_cpu_grpo_loss
         fn.restype = c_int
         fn.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_float, c_float,
@@ -78,12 +81,15 @@ class _GrpoLossFn(torch.autograd.Function):
         if rc != 0:
             raise RuntimeError(f"ka_cpu_grpo_loss failed ({rc})")
         ctx.save_for_backward(grad)
+        if not with_stats:
+            return out[0].clone()
+        ctx.mark_non_differentiable(out)
         return out[0].clone(), out
 
     @staticmethod
-    def backward(ctx, g_loss, _g_stats):
+    def backward(ctx, g_loss, _g_stats=None):
         if g_loss is None:
-            return (None,) * 9
+            return (None,) * 10
         n_seq, seq_len = ctx.shape
         if ctx.cuda:
             raw, ws = ctx.saved_tensors
@@ -96,7 +102,7 @@ class _GrpoLossFn(torch.autograd.Function):
         else:
             (g,) = ctx.saved_tensors
             grad = g * g_loss
-        return grad, None, None, None, None, None, None, None, None
+        return (grad,) + (None,) * 9
 
 
 @profiled("grpo_loss")
@@ -113,6 +119,5 @@ def grpo_loss(logp_new: torch.Tensor, logp_old: torch.Tensor, advantages: torch.
     if reduction not in ("token_mean", "seq_mean"):
         raise ValueError("reduction must be 'token_mean' or 'seq_mean'")
     hi = eps_low if eps_high is None else eps_high
-    loss, stats = _GrpoLossFn.apply(logp_new, logp_old, logp_ref, advantages, mask, float(eps_low), float(hi),
-                                    float(beta), reduction == "seq_mean")
-    return (loss, stats) if return_stats else loss
+    return _GrpoLossFn.apply(logp_new, logp_old, logp_ref, advantages, mask, float(eps_low), float(hi), float(beta),
+                             reduction == "seq_mean", bool(return_stats))

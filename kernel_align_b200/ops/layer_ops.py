@@ -7,7 +7,6 @@ rl_engine/platforms/constants.py:75-80).
 """
 from __future__ import annotations
 
-import ctypes
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import Optional
 
@@ -18,11 +17,11 @@ from ..utils.profiler import profiled
 
 
 def _sms(t: torch.Tensor) -> int:
-    return torch.cuda.get_device_properties(t.device).multi_processor_count
+    return _native.sm_count(t.device)
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _native.stream_ptr(t.device)
 
 
 def _packed(t: torch.Tensor) -> torch.Tensor:
@@ -63,10 +62,7 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5, residual: 
     r2 = residual.reshape(-1, d).contiguous() if residual is not None else None
     y = torch.empty_like(x2)
     ro = torch.empty_like(x2) if residual is not None else None
-    lib = _native.cuda()
-    fn = lib.ka_rmsnorm
-    fn.restype = c_int
-    fn.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_void_p]
+    fn = _native.cuda().ka_rmsnorm
     _check(fn(x2.data_ptr(), r2.data_ptr() if r2 is not None else None, weight.contiguous().data_ptr(), y.data_ptr(),
               ro.data_ptr() if ro is not None else None, rows, d, float(eps), _sms(x), _stream(x)), "ka_rmsnorm")
     y = y.reshape(x.shape)
@@ -98,10 +94,7 @@ def rope_(x: torch.Tensor, positions: torch.Tensor, cos: torch.Tensor, sin: torc
         return x
     if x.dtype != torch.bfloat16 or x.stride(2) != 1 or x.stride(1) != hd:
         raise ValueError("rope_ takes bf16 [tokens, heads, head_dim] with contiguous heads")
-    lib = _native.cuda()
-    fn = lib.ka_rope
-    fn.restype = c_int
-    fn.argtypes = [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]
+    fn = _native.cuda().ka_rope
     _check(fn(x.data_ptr(), x.stride(0), pos.data_ptr(), cos.data_ptr(), sin.data_ptr(), tokens, heads, hd, _sms(x),
               _stream(x)), "ka_rope")
     return x
@@ -134,10 +127,7 @@ def swiglu(gate_up: torch.Tensor, up: Optional[torch.Tensor] = None) -> torch.Te
     if up is None and not gate_up.is_contiguous():
         return swiglu(gate_up.contiguous())
     out = torch.empty(rows, f, dtype=torch.bfloat16, device=gate_up.device)
-    lib = _native.cuda()
-    fn = lib.ka_swiglu
-    fn.restype = c_int
-    fn.argtypes = [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_void_p]
+    fn = _native.cuda().ka_swiglu
     _check(fn(gate_v.data_ptr(), up_v.data_ptr(), stride, out.data_ptr(), rows, f, _sms(out), _stream(out)),
            "ka_swiglu")
     return out.reshape(*lead, f)
@@ -172,9 +162,6 @@ def _rmsnorm_backward_launch(x2, weight, eps, dy2, res2, shape):
     chunk = int(_native.cuda().ka_rmsnorm_bwd_chunk())
     part = torch.empty((rows + chunk - 1) // chunk, d, dtype=torch.float32, device=x2.device)
     fn = _native.cuda().ka_rmsnorm_bwd
-    fn.restype = c_int
-    fn.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float,
-                   c_void_p]
     _check(fn(x2.data_ptr(), weight.data_ptr(), dy2.data_ptr(), res2.data_ptr() if res2 is not None else None,
               dx.data_ptr(), dw.data_ptr(), part.data_ptr(), rows, d, float(eps), _stream(x2)), "ka_rmsnorm_bwd")
     return dx.reshape(shape), dw
@@ -245,9 +232,6 @@ def rope_fn(x: torch.Tensor, positions: torch.Tensor, cos: torch.Tensor, sin: to
 @profiled("rope")
 def _qkv_rope_launch(qkv, positions, cos, sin, q, k, v, tokens, backward):
     fn = _native.cuda().ka_qkv_rope
-    fn.restype = c_int
-    fn.argtypes = [c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
-                   c_int, c_int, c_int, c_void_p]
     _check(fn(qkv.data_ptr(), qkv.stride(0), qkv.shape[1], positions.data_ptr(), cos.data_ptr(), sin.data_ptr(),
               q.data_ptr(), k.data_ptr(), v.data_ptr(), qkv.shape[0], tokens, q.shape[1], k.shape[1], int(backward),
               _stream(qkv)), "ka_qkv_rope")
@@ -323,9 +307,6 @@ class _SwigluFn(torch.autograd.Function):
             return grad.to(gate_up.dtype).reshape(gate_up.shape)
         grad = torch.empty_like(gu)
         fn = _native.cuda().ka_swiglu_bwd
-        fn.restype = c_int
-        fn.argtypes = [c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int,
-                       c_void_p]
         _check(fn(gu.data_ptr(), gu.data_ptr() + 2 * f, 2 * f, d2.data_ptr(), grad.data_ptr(),
                   grad.data_ptr() + 2 * f, 2 * f, rows, f, _sms(gu), _stream(gu)), "ka_swiglu_bwd")
         return grad.reshape(gate_up.shape)

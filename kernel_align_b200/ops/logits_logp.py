@@ -37,11 +37,10 @@ def logits_logp(logits: torch.Tensor, ids: torch.Tensor, *, scale: float = 1.0, 
     ids64 = ids.reshape(-1).to(torch.int64).contiguous()
     logp = torch.empty(rows, dtype=torch.float32, device=x.device)
     lse = torch.empty(rows, dtype=torch.float32, device=x.device) if return_lse else None
-    props = torch.cuda.get_device_properties(x.device)
     rc = _native.cuda().ka_logits_logp(
         x.data_ptr(), _native.dtype_code(x.dtype), x.stride(0), rows, v, ids64.data_ptr(), float(scale),
-        logp.data_ptr(), lse.data_ptr() if lse is not None else None, props.multi_processor_count,
-        torch.cuda.current_stream(x.device).cuda_stream,
+        logp.data_ptr(), lse.data_ptr() if lse is not None else None, _native.sm_count(x.device),
+        _native.stream_ptr(x.device),
     )
     if rc != 0:
         raise RuntimeError(f"ka_logits_logp failed ({rc})")

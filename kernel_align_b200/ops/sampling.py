@@ -65,7 +65,7 @@ def sample(
         x.data_ptr(), _native.dtype_code(x.dtype), x.stride(0), b, v,
         rid.data_ptr() if rid is not None else None, inv_t, k, p,
         int(seed) & (2**64 - 1), int(step) & (2**64 - 1), out.data_ptr(),
-        torch.cuda.current_stream(x.device).cuda_stream,
+        _native.stream_ptr(x.device),
     )
     if rc != 0:
         raise RuntimeError(f"ka_sample failed ({rc})")

@@ -16,8 +16,7 @@ invariant in the number of ranks for the same reason the kernels are.
 """
 from __future__ import annotations
 
-import ctypes
-from ctypes import c_int, c_longlong, c_size_t, c_uint, c_ulonglong, c_void_p
+from ctypes import c_void_p
 from typing import Optional
 
 import torch
@@ -70,29 +69,6 @@ class TPContext:
             self._arenas[key] = ent
         ent[1] += 1
         return ent[0], ent[1]
-
-
-def _lib():
-    lib = _native.cuda()
-    lib.ka_gemm_rs_exchange_bytes.restype = c_size_t
-    lib.ka_gemm_rs_exchange_bytes.argtypes = [c_int, c_int, c_int]
-    lib.ka_gemm_rs_rows_per_rank.restype = c_int
-    lib.ka_gemm_rs_rows_per_rank.argtypes = [c_int, c_int]
-    lib.ka_ag_gemm_exchange_bytes.restype = c_size_t
-    lib.ka_ag_gemm_exchange_bytes.argtypes = [c_int, c_int, c_int]
-    lib.ka_gemm_reduce_scatter.restype = c_int
-    lib.ka_gemm_reduce_scatter.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_void_p, c_void_p,
-                                           c_void_p, c_int, c_int, c_int, c_int, c_int, c_uint, c_void_p, c_int,
-                                           c_ulonglong, c_void_p]
-    lib.ka_gemm_tree8_scratch_bytes.restype = c_size_t
-    lib.ka_gemm_tree8_scratch_bytes.argtypes = [c_int]
-    lib.ka_gemm_tree8.restype = c_int
-    lib.ka_gemm_tree8.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_int,
-                                  c_int, c_int, c_void_p, c_int, c_ulonglong, c_void_p]
-    lib.ka_all_gather_gemm.restype = c_int
-    lib.ka_all_gather_gemm.argtypes = [c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_void_p, c_int,
-                                       c_int, c_int, c_int, c_int, c_uint, c_void_p, c_int, c_ulonglong, c_void_p]
-    return lib
 
 
 def _tree8(p: torch.Tensor) -> torch.Tensor:
@@ -163,7 +139,7 @@ def gemm_reduce_scatter(x: torch.Tensor, w_shard: torch.Tensor, ctx: TPContext,
         raise ValueError("the K shard must split into whole 64-wide blocks per canonical slice")
     if x.device.type != "cuda":
         return _gemm_reduce_scatter_cpu(x, w_shard, ctx, residual, trans_b, keep_padding)
-    lib = _lib()
+    lib = _native.cuda()
     x = x.contiguous()
     w = w_shard.contiguous()
     rpr = rows_per_rank(m, ctx.world)
@@ -176,14 +152,13 @@ def gemm_reduce_scatter(x: torch.Tensor, w_shard: torch.Tensor, ctx: TPContext,
             res = torch.cat([res, res.new_zeros(rpr - res.shape[0], n)])
         elif res.data_ptr() % 16:
             res = res.clone()
-    props = torch.cuda.get_device_properties(x.device)
-    if ctx.world == 1 and _tree_pays(m, n, k_local, props.multi_processor_count):
-        scratch = torch.empty(lib.ka_gemm_tree8_scratch_bytes(props.multi_processor_count), dtype=torch.uint8,
+    sms = _native.sm_count(x.device)
+    if ctx.world == 1 and _tree_pays(m, n, k_local, sms):
+        scratch = torch.empty(lib.ka_gemm_tree8_scratch_bytes(sms), dtype=torch.uint8,
                               device=x.device)
         rc = lib.ka_gemm_tree8(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), int(trans_b), out.data_ptr(),
                                res.data_ptr() if res is not None else None, scratch.data_ptr(), m, n, k_local,
-                               status_buffer(x.device).data_ptr(), props.multi_processor_count, default_timeout_ns(),
-                               torch.cuda.current_stream(x.device).cuda_stream)
+                               status_buffer(x.device).data_ptr(), sms, default_timeout_ns(), _native.stream_ptr(x.device))
         if rc != 0:
             raise RuntimeError(f"ka_gemm_tree8 rejected its arguments (code {rc})")
         return out if keep_padding else out[:rows_valid]
@@ -193,8 +168,7 @@ def gemm_reduce_scatter(x: torch.Tensor, w_shard: torch.Tensor, ctx: TPContext,
     rc = lib.ka_gemm_reduce_scatter(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), int(trans_b), out.data_ptr(),
                                     res.data_ptr() if res is not None else None, ptrs, m, n, k_local, ctx.world,
                                     ctx.rank, epoch & 0xFFFFFFFF, status_buffer(x.device).data_ptr(),
-                                    props.multi_processor_count, default_timeout_ns(),
-                                    torch.cuda.current_stream(x.device).cuda_stream)
+                                    sms, default_timeout_ns(), _native.stream_ptr(x.device))
     if rc != 0:
         raise RuntimeError(f"ka_gemm_reduce_scatter rejected its arguments (code {rc})")
     return out if keep_padding else out[:rows_valid]
@@ -229,18 +203,17 @@ def all_gather_gemm(x_local: torch.Tensor, w_shard: torch.Tensor, ctx: TPContext
             x_full = x_local
         out = gemm_bi(x_full, w_shard, trans_b=trans_b)
         return (out, x_full.clone()) if return_gathered else out
-    lib = _lib()
+    lib = _native.cuda()
     x = x_local.contiguous()
     w = w_shard.contiguous()
     nbytes = lib.ka_ag_gemm_exchange_bytes(rows, k, ctx.world)
     arena, epoch = ctx.arena(("ag", rows, k), nbytes)
     out = torch.empty(ctx.world * rows, n_local, dtype=torch.bfloat16, device=x.device)
     ptrs = (c_void_p * ctx.world)(*arena.ptrs)
-    props = torch.cuda.get_device_properties(x.device)
+    sms = _native.sm_count(x.device)
     rc = lib.ka_all_gather_gemm(x.data_ptr(), w.data_ptr(), w.stride(0), int(trans_b), out.data_ptr(), out.stride(0), ptrs, rows,
                                 n_local, k, ctx.world, ctx.rank, epoch & 0xFFFFFFFF,
-                                status_buffer(x.device).data_ptr(), props.multi_processor_count,
-                                default_timeout_ns(), torch.cuda.current_stream(x.device).cuda_stream)
+                                status_buffer(x.device).data_ptr(), sms, default_timeout_ns(), _native.stream_ptr(x.device))
     if rc != 0:
         raise RuntimeError(f"ka_all_gather_gemm rejected its arguments (code {rc})")
     if return_gathered:

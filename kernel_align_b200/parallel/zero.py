@@ -13,7 +13,6 @@ The reference has no optimizer and no training loop.
 """
 from __future__ import annotations
 
-from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import Optional
 
 import torch
@@ -78,13 +77,10 @@ class ShardedAdamW:
                 new.copy_(st["master"].to(p.dtype))
             else:
                 fn = _native.cuda().ka_adamw_step
-                fn.restype = c_int
-                fn.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_float, c_float,
-                               c_float, c_float, c_float, c_int, c_float, c_int, c_void_p]
-                sms = torch.cuda.get_device_properties(p.device).multi_processor_count
+                sms = _native.sm_count(p.device)
                 rc = fn(new.data_ptr(), st["master"].data_ptr(), g.data_ptr(), int(g.dtype == torch.bfloat16),
                         st["m"].data_ptr(), st["v"].data_ptr(), shard, self.lr, b1, b2, self.eps, self.weight_decay,
-                        self.step_count, grad_scale, sms, torch.cuda.current_stream(p.device).cuda_stream)
+                        self.step_count, grad_scale, sms, _native.stream_ptr(p.device))
                 if rc != 0:
                     raise RuntimeError(f"ka_adamw_step failed ({rc})")
             # every rank's updated slice -> the whole parameter
