@@ -75,8 +75,15 @@ struct Unit {
 };
 
 __device__ __forceinline__ void decode_unit(const GemmParams& p, int tiles_m, int tiles_n, int u, Unit& out) {
-  const int t = u / p.k_slices;
+  int t = u / p.k_slices;
   out.slice = u - t * p.k_slices;
+  if (p.c_slice_stride != 0) {
+    // slices apart: all tiles of one slice follow one another, so that pairs that run together share operands
+    // (2048 x 4096 x 14336: 183 us, 198 us with all slices of one tile following one another)
+    const int tiles = tiles_m * tiles_n;
+    out.slice = u / tiles;
+    t = u - out.slice * tiles;
+  }
   const int per_group = kGroupM * tiles_n;
   const int g = t / per_group;
   const int gm = min(kGroupM, tiles_m - g * kGroupM);
@@ -210,7 +217,7 @@ __device__ __forceinline__ void store_group_warp(const GemmParams& p, const uint
              stage_offset(slice_global, p.rows_per_rank / kBM, (p.n + kBN - 1) / kBN, lr, col);
       ld = 64;  // rows of a fragment are 64 elements apart
     } else {
-      base = static_cast<__nv_bfloat16*>(p.c) + row_w0 * p.ldc + col;
+      base = static_cast<__nv_bfloat16*>(p.c) + slice_global * p.c_slice_stride + row_w0 * p.ldc + col;
       ld = p.ldc;
     }
     const int c = lane & 7, r0 = lane >> 3;   // eight lanes cover the 128 bytes of one row
@@ -751,6 +758,50 @@ inline bool narrow_tiles(int tiles_m, int tiles_n, int k, bool tree, int pairs) 
   return static_cast<long long>(tiles_m) * tiles_n * 2 <= pairs && (tree || k <= kNarrowMaxK);
 }
 
+// A product whose slices are units of their own (split) has eight times as many units: narrow ones where
+// they come out ahead in rounds, at about 0.55 of the time each.
+inline bool narrow_split_units(long long tiles, int pairs) {
+  const long long wide = (tiles * kTreeSlices + pairs - 1) / pairs, narrow = (2 * tiles * kTreeSlices + pairs - 1) / pairs;
+  return narrow * 11 < wide * 20;
+}
+
+// ---- split mode (ka_gemm_split8). A pair that keeps a tile walks its eight slices one after the other, at
+// about 0.31 us per 64-wide K block whatever the tile's width, so few tiles with a long K leave most pairs
+// idle; with the slices spread over all pairs 128 x 4096 takes 18.5 us instead of 37.7 (K = 4096), 39.7 instead
+// of 86.0 (14336), 60 instead of 152 (28672); 512 x 4096 37.3 / 40.3, 80 / 90, 143 / 156; 512 x 1024 15.4 / 36.3
+// (4096). The price is a pass over the partials, 3 to 6 us (they stay in L2). Second half: the eight bf16 partials
+// of every element summed in the order of the reduce-scatter tail, ((0+1)+(2+3))+((4+5)+(6+7)) in fp32,
+// rounded, the residual added after that.
+constexpr int kSumThreads = 256;
+
+__global__ void __launch_bounds__(kSumThreads)
+slice_sum_kernel(const uint4* __restrict__ part, long long vecs, const uint4* __restrict__ residual, uint4* __restrict__ out) {
+  const long long i = static_cast<long long>(blockIdx.x) * kSumThreads + threadIdx.x;
+  if (i >= vecs) return;
+  uint4 v[kTreeSlices];
+#pragma unroll
+  for (int s = 0; s < kTreeSlices; ++s) v[s] = __ldcg(part + s * vecs + i);
+  uint4 r = make_uint4(0u, 0u, 0u, 0u);
+  if (residual) r = __ldg(residual + i);
+  auto word = [&](auto get) {
+    float lo[kTreeSlices], hi[kTreeSlices];
+#pragma unroll
+    for (int s = 0; s < kTreeSlices; ++s) {
+      lo[s] = bf16_lo(get(v[s]));
+      hi[s] = bf16_hi(get(v[s]));
+    }
+    auto tree = [](const float(&a)[kTreeSlices]) {
+      return __fadd_rn(__fadd_rn(__fadd_rn(a[0], a[1]), __fadd_rn(a[2], a[3])),
+                       __fadd_rn(__fadd_rn(a[4], a[5]), __fadd_rn(a[6], a[7])));
+    };
+    uint32_t o = pack_bf16(tree(lo), tree(hi));
+    if (residual) o = pack_bf16(__fadd_rn(bf16_lo(o), bf16_lo(get(r))), __fadd_rn(bf16_hi(o), bf16_hi(get(r))));
+    return o;
+  };
+  out[i] = make_uint4(word([](const uint4& a) { return a.x; }), word([](const uint4& a) { return a.y; }),
+                      word([](const uint4& a) { return a.z; }), word([](const uint4& a) { return a.w; }));
+}
+
 }  // namespace
 
 // Shared by the plain entry point and the tensor-parallel ones (tp_gemm.cu): build the
@@ -766,7 +817,10 @@ int gemm_launch(const void* a, long long lda, const void* b, long long ldb, cons
   int ctas = tree ? max_ctas<true, kBN>(num_sms) : max_ctas<false, kBN>(num_sms);
   if (ctas <= 0) return -10;
   const int tiles_m = (p.m + kBM * kG - 1) / (kBM * kG);
-  const bool narrow = !full_grid && narrow_tiles(tiles_m, (p.n + kBN - 1) / kBN, p.k, tree, ctas / kG);
+  const int wide_n = (p.n + kBN - 1) / kBN;
+  const bool split = p.c_slice_stride != 0;
+  const bool narrow = !full_grid && (split ? narrow_split_units(static_cast<long long>(tiles_m) * wide_n, ctas / kG)
+                                           : narrow_tiles(tiles_m, wide_n, p.k, tree, ctas / kG));
   if (narrow) ctas = tree ? max_ctas<true, kBN / 2>(num_sms) : max_ctas<false, kBN / 2>(num_sms);
   if (ctas <= 0) return -10;
   const int bn = narrow ? kBN / 2 : kBN;
@@ -865,6 +919,42 @@ extern "C" int ka_gemm_tree8(const void* a, long long lda, const void* b, long l
   p.status = status;
   p.timeout_ns = timeout_ns;
   return ka::gemm_launch(a, lda, b, ldb, p, num_sms, false, static_cast<cudaStream_t>(stream));
+}
+
+// Elements (bf16) of scratch ka_gemm_split8 needs.
+extern "C" size_t ka_gemm_split8_scratch_elems(int m, int n) { return static_cast<size_t>(ka::kTreeSlices) * m * n; }
+
+// The same result as ka_gemm_tree8, for products of few tiles: the slices are units of their own, spread
+// over all CTA pairs, their bf16 partials go to `scratch` ([8, m, n], 16-byte aligned; it stays in L2) and a
+// second kernel sums them.
+extern "C" int ka_gemm_split8(const void* a, long long lda, const void* b, long long ldb, int b_major, void* out,
+                              const void* residual, void* scratch, int m, int n, int k, int* status, int num_sms,
+                              unsigned long long timeout_ns, void* stream) {
+  if (m <= 0 || n <= 0) return 0;
+  if (n % 8 != 0) return -51;
+  if (((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(scratch)) & 15u) != 0)
+    return -54;
+  ka::GemmParams p = {};
+  p.m = m;
+  p.n = n;
+  p.k = k;
+  p.b_major = b_major ? 1 : 0;
+  p.epilogue = ka::kEpiStoreBf16;
+  p.c = scratch;
+  p.ldc = n;
+  p.c_slice_stride = static_cast<long long>(m) * n;
+  p.k_slices = ka::kTreeSlices;
+  p.total_slices = ka::kTreeSlices;
+  p.world = 1;
+  p.status = status;
+  p.timeout_ns = timeout_ns;
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int rc = ka::gemm_launch(a, lda, b, ldb, p, num_sms, false, st);
+  if (rc != 0) return rc;
+  const long long vecs = p.c_slice_stride / 8;
+  ka::slice_sum_kernel<<<static_cast<unsigned>((vecs + ka::kSumThreads - 1) / ka::kSumThreads), ka::kSumThreads, 0, st>>>(
+      static_cast<const uint4*>(scratch), vecs, static_cast<const uint4*>(residual), static_cast<uint4*>(out));
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
 extern "C" int ka_lmhead_logits_grad(const void* hidden, const void* weight, const long long* ids, const float* lse,

@@ -34,6 +34,7 @@ struct GemmParams {
   int epilogue;
   void* c;                // kEpiStoreBf16 / kEpiStoreF32 output
   long long ldc;
+  long long c_slice_stride;   // kEpiStoreBf16 with k_slices > 1: elements between the slices' results (0: no slices apart)
   // --- K-slice partials + reduce-scatter (kEpiPartialF32)
   int k_slices;           // local slices (each k / k_slices wide, multiple of 64)
   int slice_base;         // global index of the first local slice (rank * k_slices)

@@ -106,6 +106,8 @@ def cuda() -> ctypes.CDLL:
     _bind(lib, "ka_gemm_reduce_scatter", c_int, [p, ll, p, ll, i, p, p, p, i, i, i, i, i, c_uint, p, i, ull, p])
     _bind(lib, "ka_gemm_tree8_scratch_bytes", c_size_t, [i])
     _bind(lib, "ka_gemm_tree8", c_int, [p, ll, p, ll, i, p, p, p, i, i, i, p, i, ull, p])
+    _bind(lib, "ka_gemm_split8_scratch_elems", c_size_t, [i, i])
+    _bind(lib, "ka_gemm_split8", c_int, [p, ll, p, ll, i, p, p, p, i, i, i, p, i, ull, p])
     _bind(lib, "ka_all_gather_gemm", c_int, [p, p, ll, i, p, ll, p, i, i, i, i, i, c_uint, p, i, ull, p])
     return lib
 

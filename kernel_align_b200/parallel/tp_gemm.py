@@ -107,18 +107,30 @@ def _gemm_reduce_scatter_cpu(x, w_shard, ctx, residual, trans_b, keep_padding):
     return out if keep_padding else out[:rows_valid]
 
 
-def _tree_pays(m: int, n: int, k: int, num_sms: int) -> bool:
-    """Whether one rank sums the eight K slices of a tile in the kernel that computes them
-    (``ka_gemm_tree8``) or stages them (``ka_gemm_reduce_scatter``). The bits are the same.
+def _split_pays(m: int, n: int, k: int) -> bool:
+    """Whether one rank that sums its eight K slices itself makes them units of their own
+    (``ka_gemm_split8``: eight times as many units, a pass over the partials) or keeps a tile's slices on one
+    CTA pair (``ka_gemm_tree8``). Measured split / kept in us on 74 pairs, tiles counted as 256 x 256: 4 tiles:
+    10 / 26 (K = 1024), 13 / 36 (4096); 16 tiles: 16 / 26 (1024), 18.5 / 38 (4096), 40 / 86 (14336), 60 / 152
+    (28672); 32 tiles: 27 / 27 (1024), 28 / 24 (1536), 37 / 40 (4096), 42 / 43 (6144), 80 / 90 (14336),
+    143 / 156 (28672); 48 tiles: 43 / 53 (4096), 46 / 51 (6144), 81 / 104 (14336); 64 tiles: 52 / 54 (4096),
+    54 / 53 (6144), 96 / 106 (14336), 161 / 171 (28672); with more tiles the partials outgrow what the rest saves
+    (256 tiles: 196 / 185 at 6144, 688 / 706 at 28672, with half a gigabyte of scratch)."""
+    tiles = -(-m // 256) * -(-n // 256)
+    return tiles <= 24 or (tiles <= 48 and k >= 4096) or (tiles <= 64 and k >= 12288)
 
-    A CTA pair that keeps a tile walks its eight slices one after the other, while staged slices
-    spread over all pairs but cost a pass over the partials and the wait for them. Measured on
-    148 SMs, staged / kept in us, tiles counted as 256 x 256 (the kept form cuts up to 37 of them into
-    halves of 128 columns): 256 tiles: 385 / 156 (K = 4096), 1025 / 738 (28672); 32 tiles: 72 / 35 (4096),
-    109 / 90 (14336), 150 / 163 (28672); 16 tiles: 48 / 33 (4096), 57 / 44 (6144), 70 / 85 (14336),
-    101 / 156 (28672); 8 tiles: 39 / 33 (4096), 42 / 43 (6144), 54 / 82 (14336); 4 tiles: 39 / 33 (4096),
-    40 / 42 (6144). A slice round takes about 5.4e-3 us per K column, staging about 20 us plus 1.2 us per
-    tile; the rule compares the two."""
+
+def _tree_pays(m: int, n: int, k: int, num_sms: int) -> bool:
+    """Whether one rank sums its eight K slices itself, in one of the two forms of :func:`_split_pays`, or
+    stages them as several ranks do (``ka_gemm_reduce_scatter``). The bits are the same.
+
+    Staged slices spread over all pairs but cost fences, flags and the wait for them. Measured on
+    148 SMs, staged / own in us, tiles counted as 256 x 256: 256 tiles: 385 / 156 (K = 4096), 1025 / 738 (28672);
+    32 tiles: 72 / 37 (4096), 109 / 80 (14336), 150 / 143 (28672); 16 tiles: 48 / 18 (4096), 57 / 26 (6144),
+    70 / 40 (14336), 101 / 60 (28672); 4 tiles: 39 / 13 (4096). A slice round of a kept tile takes about 5.4e-3 us
+    per K column, staging about 20 us plus 1.2 us per tile; the rule compares the two."""
+    if _split_pays(m, n, k):
+        return True
     pairs = max(1, num_sms // 2)
     tiles = -(-m // 256) * -(-n // 256)
     extra_rounds = -(-tiles // pairs) * 8 - -(-8 * tiles // pairs)
@@ -154,13 +166,17 @@ def gemm_reduce_scatter(x: torch.Tensor, w_shard: torch.Tensor, ctx: TPContext,
             res = res.clone()
     sms = _native.sm_count(x.device)
     if ctx.world == 1 and _tree_pays(m, n, k_local, sms):
-        scratch = torch.empty(lib.ka_gemm_tree8_scratch_bytes(sms), dtype=torch.uint8,
-                              device=x.device)
-        rc = lib.ka_gemm_tree8(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), int(trans_b), out.data_ptr(),
-                               res.data_ptr() if res is not None else None, scratch.data_ptr(), m, n, k_local,
-                               status_buffer(x.device).data_ptr(), sms, default_timeout_ns(), _native.stream_ptr(x.device))
+        if _split_pays(m, n, k_local):
+            scratch = torch.empty(lib.ka_gemm_split8_scratch_elems(m, n), dtype=torch.bfloat16, device=x.device)
+            fn = lib.ka_gemm_split8
+        else:
+            scratch = torch.empty(lib.ka_gemm_tree8_scratch_bytes(sms), dtype=torch.uint8, device=x.device)
+            fn = lib.ka_gemm_tree8
+        rc = fn(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), int(trans_b), out.data_ptr(),
+                res.data_ptr() if res is not None else None, scratch.data_ptr(), m, n, k_local,
+                status_buffer(x.device).data_ptr(), sms, default_timeout_ns(), _native.stream_ptr(x.device))
         if rc != 0:
-            raise RuntimeError(f"ka_gemm_tree8 rejected its arguments (code {rc})")
+            raise RuntimeError(f"the row-parallel product rejected its arguments (code {rc})")
         return out if keep_padding else out[:rows_valid]
     nbytes = lib.ka_gemm_rs_exchange_bytes(m, n, ctx.world)
     arena, epoch = ctx.arena(("rs", m, n), nbytes)

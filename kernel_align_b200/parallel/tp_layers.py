@@ -8,8 +8,8 @@ Activations between blocks are sequence-sharded (each rank holds ``rows_per_rank
 Their backward passes are the mirrored fused kernels (the gradient of an all-gather is a
 reduce-scatter and vice versa), so forward and backward both overlap NVLink traffic with the
 MMAs and both use the fixed 8-slice reduction order. With one rank there is nothing to gather, and
-the eight slices are summed in the kernel that computes them, or staged in a local buffer
-(``tp_gemm._tree_pays``): the same bits as on several ranks.
+the eight slices are summed in the kernel that computes them, or by a second one from local partials
+(``tp_gemm._split_pays``): the same bits as on several ranks.
 """
 from __future__ import annotations
 

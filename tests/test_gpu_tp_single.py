@@ -63,3 +63,24 @@ def test_slices_summed_in_the_kernel_equal_the_staged_ones_bitwise(cuda_device, 
         outs += [[gemm_reduce_scatter(x, w, ctx, residual=res, trans_b=trans_b) for res in (None, r)]]
     gemm.check_status(cuda_device)
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("m,n,k,trans_b", [(1, 8, 512, False), (127, 264, 1024, True), (300, 1032, 512, False),
+                                           (1000, 4096, 1536, True), (1100, 4104, 512, False)])
+def test_slices_as_units_of_their_own_equal_the_kept_ones_bitwise(cuda_device, m, n, k, trans_b, monkeypatch):
+    """The eight K slices as separate units (narrow and wide ones, one round and several) and a sum over
+    their partials: the bits of a tile that keeps its slices."""
+    from kernel_align_b200.parallel import tp_gemm
+
+    ctx = TPContext(device=cuda_device)
+    g = torch.Generator(device=cuda_device).manual_seed(m + n)
+    x = torch.randn(m, k, device=cuda_device, generator=g).to(torch.bfloat16)
+    w = (torch.randn(*((k, n) if trans_b else (n, k)), device=cuda_device, generator=g) * 0.05).to(torch.bfloat16)
+    r = torch.randn(m, n, device=cuda_device, generator=g).to(torch.bfloat16)
+    outs = []
+    monkeypatch.setattr(tp_gemm, "_tree_pays", lambda *a: True)
+    for split in (False, True):
+        monkeypatch.setattr(tp_gemm, "_split_pays", lambda *a, s=split: s)
+        outs += [[gemm_reduce_scatter(x, w, ctx, residual=res, trans_b=trans_b) for res in (None, r)]]
+    gemm.check_status(cuda_device)
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
