@@ -2,9 +2,9 @@
 //
 //   delta[b, h, i] = sum_d dO[i, d] * O[i, d]
 //   P  = exp(scale * Q K^T - lse),   dP = dO V^T,   dS = P * (dP - delta) * scale
-//   dQ = dS K            kernel attention_bwd_dq_kernel : one CTA per (sequence, q head, q tile),
+//   dQ = dS K            bwd_dq: one CTA per (sequence, q head, q tile),
 //                        walks the KV tiles in increasing order, dQ accumulates in TMEM
-//   dV = P^T dO, dK = dS^T Q   kernel attention_bwd_dkv_kernel: one CTA per (sequence, kv head,
+//   dV = P^T dO, dK = dS^T Q   bwd_dkv: one CTA per (sequence, kv head,
 //                        kv tile), walks (q head of the group, q tile) in a fixed order; it
 //                        works on S^T = K Q^T so that its threads own KV rows
 //
@@ -148,10 +148,9 @@ struct CtlDq {
 // ------------------------------------------------------------------------------------------------
 // dQ kernel. TMEM: S (two buffers), dP, dQ. Shared memory: Q, dO, two stages of (K, V).
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads, 1)
-attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                        const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                        const __grid_constant__ BwdParams p) {
+__device__ __forceinline__ void
+bwd_dq(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_do,
+       const BwdParams& p, int block) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
   const uint32_t q_tile = base, do_tile = base + kTileBytes, ring = base + 2 * kTileBytes;  // stage: K, V
@@ -159,8 +158,8 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_qt = (p.seq_len + kT - 1) / kT;
-  const int qt = n_qt - 1 - static_cast<int>(blockIdx.x % n_qt);
-  const int bh = blockIdx.x / n_qt;
+  const int qt = n_qt - 1 - block % n_qt;
+  const int bh = block / n_qt;
   const int h = bh % p.hq, b = bh / p.hq;
   const int hk = h / (p.hq / p.hkv);
   const int q_row0 = qt * kT, tok0 = b * p.seq_len;
@@ -372,10 +371,9 @@ struct CtlDkv {
   alignas(16) float neg_delta[2][kT];
 };
 
-__global__ void __launch_bounds__(kThreads, 1)
-attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                         const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                         const __grid_constant__ BwdParams p) {
+__device__ __forceinline__ void
+bwd_dkv(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_do,
+        const BwdParams& p, int block) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
   const uint32_t k_tile = base, v_tile = base + kTileBytes, ring = base + 2 * kTileBytes,   // stage: Q, dO
@@ -388,8 +386,8 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   // All CTAs of the early (causal: heavy) kv tiles first: the last CTAs to start are the lightest
   // (sequence by sequence the last heavy ones started when the rest was done: 1074 against 833 us).
   const int n_bh = p.batch * p.hkv;
-  const int jt = static_cast<int>(blockIdx.x) / n_bh;
-  const int bh = static_cast<int>(blockIdx.x) % n_bh;
+  const int jt = block / n_bh;
+  const int bh = block % n_bh;
   const int hk = bh % p.hkv, b = bh / p.hkv;
   const int group = p.hq / p.hkv;
   const int kv_row0 = jt * kT, tok0 = b * p.seq_len;
@@ -646,6 +644,22 @@ attention_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   }
 }
 
+// Both in one launch: the first n_dkv CTAs do a dK / dV tile each, the others a dQ tile. The two need only
+// delta from each other's direction, and a dK / dV CTA walks a whole group of query heads, so a call of few
+// sequences or KV heads leaves most SMs idle until the last of them is done, and a call of many its last
+// round: dQ tiles fill both. dQ + dK / dV apart, together (us, 32 / 8 heads): 8 x 512 133, 126; 4 x 1000, no mask,
+// 310, 290; 1 x 700 82, 61; 2 x 4000 1043, 1037; 4 / 1 heads, 1 x 4000 325, 268.
+__global__ void __launch_bounds__(kThreads, 1)
+attention_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
+                     const __grid_constant__ BwdParams p, int n_dkv) {
+  const int block = static_cast<int>(blockIdx.x);
+  if (block < n_dkv)
+    bwd_dkv(tm_q, tm_k, tm_v, tm_do, p, block);
+  else
+    bwd_dq(tm_q, tm_k, tm_v, tm_do, p, block - n_dkv);
+}
+
 }  // namespace
 }  // namespace ka
 
@@ -666,10 +680,9 @@ extern "C" int ka_attention_bwd(const void* q, long long q_stride, const void* k
   constexpr int kSmemDq = 6 * kTileBytes + 256;
   constexpr int kSmemDkv = 7 * kTileBytes + 2304;
   static_assert(sizeof(CtlDq) <= 256 && sizeof(CtlDkv) <= 2304 && kSmemDkv <= 227 * 1024, "shared memory layout");
-  static PerDevice once_dq, once_dkv;
-  if (!smem_opt_in(once_dq, attention_bwd_dq_kernel, kSmemDq) ||
-      !smem_opt_in(once_dkv, attention_bwd_dkv_kernel, kSmemDkv))
-    return -10;
+  constexpr int kSmem = kSmemDkv > kSmemDq ? kSmemDkv : kSmemDq;
+  static PerDevice once;
+  if (!smem_opt_in(once, attention_bwd_kernel, kSmem)) return -10;
   const uint64_t tokens = static_cast<uint64_t>(batch) * seq_len;
   CUtensorMap tq, tk, tv, tdo;
   int rc = make_tmap_2d_16bit_sw128(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, q, tokens, static_cast<uint64_t>(hq) * kD,
@@ -707,7 +720,7 @@ extern "C" int ka_attention_bwd(const void* q, long long q_stride, const void* k
   p.status = status;
   p.timeout_ns = timeout_ns;
   const int n_t = (seq_len + kT - 1) / kT;
-  attention_bwd_dq_kernel<<<static_cast<unsigned>(batch) * hq * n_t, kThreads, kSmemDq, st>>>(tq, tk, tv, tdo, p);
-  attention_bwd_dkv_kernel<<<static_cast<unsigned>(batch) * hkv * n_t, kThreads, kSmemDkv, st>>>(tq, tk, tv, tdo, p);
+  const int n_dkv = batch * hkv * n_t;
+  attention_bwd_kernel<<<static_cast<unsigned>(batch) * (hq + hkv) * n_t, kThreads, kSmem, st>>>(tq, tk, tv, tdo, p, n_dkv);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
