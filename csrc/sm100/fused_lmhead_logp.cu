@@ -229,6 +229,15 @@ __device__ __forceinline__ void fold32(const uint32_t (&v)[32], int col0, int va
   m = mn;
 }
 
+// The first n (a multiple of 8) of 32 accumulator columns of a row, written past the caches' working set.
+__device__ __forceinline__ void store32(float* dst, const uint32_t (&v)[32], int n) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 4)
+    if (j < n)
+      __stcs(reinterpret_cast<float4*>(dst + j), make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
+                                                             __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])));
+}
+
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // Merge this rank's sub-slice partials of one row: chains inside each slice, then the local
@@ -598,6 +607,9 @@ fused_lmhead_logp_kernel(const __grid_constant__ CUtensorMap tm_h,
         const int tcol = tcol_item - nt * kBN;
         const uint32_t trow = tmem_base + (static_cast<uint32_t>(warp * 32) << 16) +
                               static_cast<uint32_t>(abuf * kBN);
+        float* const lrow = p.logits != nullptr && row_ok
+                                ? p.logits + rr.out_row * p.v_local + it.col_begin + nt * kBN
+                                : nullptr;
         uint32_t va[32], vb[32];
         tmem_ld_32x32(trow, va);
         tmem_ld_wait_dep(va);
@@ -605,10 +617,12 @@ fused_lmhead_logp_kernel(const __grid_constant__ CUtensorMap tm_h,
         for (int g = 0; g < kBN / 32; g += 2) {
           __syncwarp();
           tmem_ld_32x32(trow + (g + 1) * 32, vb);
+          if (lrow) store32(lrow + g * 32, va, valid - g * 32);
           if (g * 32 < valid) fold32(va, g * 32, valid, tcol, s2, m, l, t);
           __syncwarp();
           tmem_ld_wait_dep(vb);
           if (g + 2 < kBN / 32) tmem_ld_32x32(trow + (g + 2) * 32, va);
+          if (lrow) store32(lrow + (g + 1) * 32, vb, valid - (g + 1) * 32);
           if ((g + 1) * 32 < valid) fold32(vb, (g + 1) * 32, valid, tcol, s2, m, l, t);
           __syncwarp();
           if (g + 2 < kBN / 32) tmem_ld_wait_dep(va);
@@ -889,6 +903,7 @@ struct FwdArgs {
   int panel_rows, sharded, out_all, cta_group, cg_pref, m_fast, l2_hint, num_sms;
   unsigned long long timeout_ns;
   cudaStream_t stream;
+  float* logits = nullptr;
 };
 
 int forward_impl(const FwdArgs& a) {
@@ -941,6 +956,8 @@ int forward_impl(const FwdArgs& a) {
   p.ids = a.ids;
   p.logp = a.logp;
   p.lse = a.lse;
+  if (a.logits != nullptr && (a.world != 1 || a.v_local % 64 != 0 || (reinterpret_cast<uintptr_t>(a.logits) & 15u) != 0)) return -16;
+  p.logits = a.logits;
   p.m = a.m;
   p.k = a.k;
   p.v_global = a.v_global;
@@ -1095,6 +1112,19 @@ int ka_lmhead_logp_forward_sched(const void* hidden, const void* weight, const l
                    m, k, v_global, v_local, vocab_offset, world, rank, epoch_base, scale, panel_rows,
                    0, 1, cta_group, cg_pref, m_fast, l2_hint, num_sms, timeout_ns,
                    static_cast<cudaStream_t>(stream_ptr)};
+  return ka::forward_impl(a);
+}
+
+// The same for a whole vocabulary on one GPU, keeping the products: logits [m, v] fp32, v % 64 == 0.
+int ka_lmhead_logp_forward_keep(const void* hidden, const void* weight, const long long* ids, float* logp, float* lse,
+                                float* logits, void* workspace, size_t workspace_bytes, int m, int k, int v,
+                                unsigned epoch_base, float scale, int panel_rows, int cta_group, int cg_pref, int m_fast,
+                                int l2_hint, int num_sms, unsigned long long timeout_ns, void* stream_ptr) {
+  ka::FwdArgs a = {hidden, weight, ids, logp, lse, workspace, workspace_bytes, nullptr, nullptr,
+                   m, k, v, v, 0, 1, 0, epoch_base, scale, panel_rows,
+                   0, 1, cta_group, cg_pref, m_fast, l2_hint, num_sms, timeout_ns,
+                   static_cast<cudaStream_t>(stream_ptr)};
+  a.logits = logits;
   return ka::forward_impl(a);
 }
 

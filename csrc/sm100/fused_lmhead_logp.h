@@ -32,6 +32,7 @@ struct LogpParams {
   int world, rank;
   unsigned epoch;        // value the flags of this launch carry
   float scale;           // logits are scale * <h, w>; must be > 0
+  float* logits;         // [m, v_local] or nullptr: the products as they are, for a backward pass (world 1, v_local % 64 == 0)
   unsigned long long timeout_ns;
   int mt_rot;            // rotation of the row-tile order (row-sharded input: own rows first)
   int l2_hint;           // L2 eviction hints of the operand loads, see the producer

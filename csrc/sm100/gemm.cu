@@ -957,6 +957,61 @@ extern "C" int ka_gemm_split8(const void* a, long long lda, const void* b, long 
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
+namespace ka {
+namespace {
+
+// d_logits from kept logits: the arithmetic of the kEpiLogitsGrad epilogue, so the bits are those of the
+// recomputed ones. A stream: 4 bytes read and 2 written per logit.
+constexpr int kGradThreads = 256, kGradVecs = 4;   // vectors of 8 columns per thread
+
+__global__ void __launch_bounds__(kGradThreads)
+kept_logits_grad_kernel(const float* __restrict__ logits, const long long* __restrict__ ids, const float* __restrict__ lse,
+                        const float* __restrict__ g, __nv_bfloat16* __restrict__ out, int n, float scale) {
+  const int row = blockIdx.y;
+  const float s2 = scale * 1.4426950408889634f, neg_lse2 = __fmul_rn(-lse[row], 1.4426950408889634f);
+  const float gs = __fmul_rn(g[row], scale);
+  const long long tgt = ids[row];
+  const float* src = logits + static_cast<long long>(row) * n;
+  __nv_bfloat16* dst = out + static_cast<long long>(row) * n;
+  const int c0 = (blockIdx.x * kGradThreads * kGradVecs + threadIdx.x) * 8;
+  float4 a[kGradVecs], b[kGradVecs];
+#pragma unroll
+  for (int u = 0; u < kGradVecs; ++u) {
+    const int c = c0 + u * kGradThreads * 8;
+    if (c < n) {
+      a[u] = __ldcs(reinterpret_cast<const float4*>(src + c));
+      b[u] = __ldcs(reinterpret_cast<const float4*>(src + c + 4));
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kGradVecs; ++u) {
+    const int c = c0 + u * kGradThreads * 8;
+    if (c >= n) break;
+    const float v[8] = {a[u].x, a[u].y, a[u].z, a[u].w, b[u].x, b[u].y, b[u].z, b[u].w};
+    float d[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      d[j] = __fmul_rn(gs, __fsub_rn(c + j == tgt ? 1.f : 0.f, ex2_approx(__fmaf_rn(v[j], s2, neg_lse2))));
+    *reinterpret_cast<uint4*>(dst + c) = make_uint4(pack_bf16(d[0], d[1]), pack_bf16(d[2], d[3]), pack_bf16(d[4], d[5]),
+                                                    pack_bf16(d[6], d[7]));
+  }
+}
+
+}  // namespace
+}  // namespace ka
+
+// d_logits [m, n] bf16 from logits [m, n] fp32 that ka_lmhead_logp_forward_keep wrote; n % 8 == 0, 16-byte aligned.
+extern "C" int ka_lmhead_kept_logits_grad(const float* logits, const long long* ids, const float* lse, const float* g,
+                                          void* d_logits, int m, int n, float scale, void* stream) {
+  if (m <= 0 || n <= 0) return 0;
+  if (n % 8 != 0 || m > 65535 || ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(d_logits)) & 15u) != 0)
+    return -1;
+  constexpr int per = ka::kGradThreads * ka::kGradVecs * 8;
+  ka::kept_logits_grad_kernel<<<dim3((n + per - 1) / per, m), ka::kGradThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+      logits, ids, lse, g, static_cast<__nv_bfloat16*>(d_logits), n, scale);
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
 extern "C" int ka_lmhead_logits_grad(const void* hidden, const void* weight, const long long* ids, const float* lse,
                                      const float* g, void* d_logits, long long ldd, int m, int n, int k, float scale,
                                      int col_offset, int* status, int num_sms, unsigned long long timeout_ns,

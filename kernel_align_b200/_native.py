@@ -100,6 +100,9 @@ def cuda() -> ctypes.CDLL:
     _bind(lib, "ka_gemm_bf16", c_int, [p, ll, i, p, ll, i, p, ll, i, i, i, i, p, i, ull, p])
     _bind(lib, "ka_gemm_skinny_bf16", c_int, [p, ll, p, ll, p, ll, i, i, i, p, ull, p])
     _bind(lib, "ka_lmhead_logits_grad", c_int, [p, p, p, p, p, p, ll, i, i, i, f, i, p, i, ull, p])
+    _bind(lib, "ka_lmhead_kept_logits_grad", c_int, [p, p, p, p, p, i, i, f, p])
+    _bind(lib, "ka_lmhead_logp_forward_keep", c_int,
+          [p, p, p, p, p, p, p, c_size_t, i, i, i, c_uint, f, i, i, i, i, i, i, ull, p])
     _bind(lib, "ka_gemm_rs_exchange_bytes", c_size_t, [i, i, i])
     _bind(lib, "ka_gemm_rs_rows_per_rank", c_int, [i, i])
     _bind(lib, "ka_ag_gemm_exchange_bytes", c_size_t, [i, i, i])

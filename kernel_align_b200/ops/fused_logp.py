@@ -1,7 +1,8 @@
 """Fused LM-head + per-token log-probability.
 
 ``lmhead_logp(hidden, weight, ids)`` returns ``log_softmax(scale * hidden @ weight.T)[ids]``
-without ever materialising the ``[rows, vocab]`` logits. On CUDA it runs the hand-written
+without materialising the ``[rows, vocab]`` logits (calls with gradients keep them for the backward pass
+while they are few, see ``_KEEP_BYTES``). On CUDA it runs the hand-written
 tcgen05/TMA kernel of ``csrc/sm100/fused_lmhead_logp.cu``; on CPU the C++ implementation of
 ``csrc/cpu/fused_logp_cpu.cpp``. Both follow the same canonical decomposition of the
 vocabulary (8 slices, 1792-column sub-slices, balanced merge tree), so a row's result does
@@ -15,6 +16,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from dataclasses import dataclass, field
 from typing import Optional
 
@@ -220,13 +222,14 @@ def _lmhead_logp_forward(
     check: bool = False,
     row_sharded: bool = False,
     gather_output: bool = False,
+    logits: Optional[torch.Tensor] = None,
 ):
     """Per-token log-probabilities of ``ids`` under ``softmax(scale * hidden @ weight.T)``.
 
     hidden: ``[..., K]`` bf16; weight: ``[V_local, K]`` bf16 (this rank's vocabulary shard,
     whole canonical slices, see :func:`vocab_shard_range`); ids: ``[...]`` integer, global
     ids. Ids outside ``[0, vocab)`` give 0. Returns fp32 ``[...]`` (and the log-sum-exp if
-    ``return_lse``). With ``row_sharded`` the rank passes only its rows of the batch (the same
+    ``return_lse``). ``logits`` (CUDA, one rank, see :func:`_kept_logits`) receives the products. With ``row_sharded`` the rank passes only its rows of the batch (the same
     number on every rank) and gets their results, or, with ``gather_output``, the flat
     ``[world * rows]`` results of the whole batch.
     """
@@ -339,6 +342,13 @@ def _lmhead_logp_forward(
                 epoch & 0xFFFFFFFF, float(scale), panel_rows, 1 if gather_output else 0, g, cg, m_fast, hint,
                 sms, default_timeout_ns(), stream,
             )
+        elif logits is not None:
+            rc = lib.ka_lmhead_logp_forward_keep(
+                h2.data_ptr(), w.data_ptr(), ids64.data_ptr(), logp.data_ptr(),
+                lse.data_ptr() if lse is not None else None, logits.data_ptr(), ws.buf.data_ptr(), ws.nbytes,
+                m, k, v_global, epoch & 0xFFFFFFFF, float(scale), panel_rows, g, cg, m_fast, hint, sms,
+                default_timeout_ns(), stream,
+            )
         else:
             rc = lib.ka_lmhead_logp_forward_sched(
                 h2.data_ptr(), w.data_ptr(), ids64.data_ptr(), logp.data_ptr(),
@@ -376,10 +386,56 @@ def last_status(device: torch.device, vocab: int, panel_rows: int = DEFAULT_PANE
 
 _GRAD_PANEL_BYTES = 8 << 30
 
+# ---- logits kept for the backward pass --------------------------------------------------------
+# The backward pass needs every logit once more. Recomputing them is the fourth of four products of the
+# same size; keeping them (fp32, as the forward kernel has them: the gradients are the same bits) costs a
+# write of 4 bytes per logit under the forward's products and a read: 2000 x 4096 x 128256, forward and
+# backward: 6.9 -> 5.7 ms. It is done while what all live graphs of a device keep stays below
+# _KEEP_BYTES (1.1 % of its memory, two calls of 2000 rows at 128256 columns); beyond that, or when the
+# allocation fails, the logits are recomputed and never materialised.
+_KEEP_BYTES = 2 << 30
+_kept_bytes: dict[int, int] = {}
+_kept_lock = threading.Lock()
 
-def _logp_backward(hidden, weight, ids, lse, g, scale, vocab, group, need_dh, need_dw):
+
+class _Kept:
+    """A share of a device's allowance for kept logits, given back when the graph node that holds it goes."""
+
+    def __init__(self, index: int, nbytes: int):
+        self.index, self.nbytes = index, nbytes
+
+    @classmethod
+    def take(cls, index: int, nbytes: int) -> Optional["_Kept"]:
+        with _kept_lock:
+            if _kept_bytes.get(index, 0) + nbytes > _KEEP_BYTES:
+                return None
+            _kept_bytes[index] = _kept_bytes.get(index, 0) + nbytes
+        return cls(index, nbytes)
+
+    def __del__(self):
+        with _kept_lock:
+            _kept_bytes[self.index] -= self.nbytes
+
+
+def _kept_logits(hidden, weight, vocab, group):
+    """``(share, logits)`` for a forward call whose logits are kept, or ``(None, None)``."""
+    v = int(weight.shape[0])
+    m = hidden.numel() // max(1, hidden.shape[-1])
+    if (hidden.device.type != "cuda" or group is not None or v % 64 != 0 or not 0 < m <= 65535
+            or (vocab is not None and int(vocab) != v)):
+        return None, None
+    share = _Kept.take(_native._device_index(hidden.device), 4 * m * v)
+    if share is None:
+        return None, None
+    try:
+        return share, torch.empty(m, v, dtype=torch.float32, device=hidden.device)
+    except torch.OutOfMemoryError:
+        return None, None
+
+
+def _logp_backward(hidden, weight, ids, lse, g, scale, vocab, group, need_dh, need_dw, logits=None):
     """Gradients of the log-probabilities with respect to ``hidden`` (all rows, summed over the
-    vocabulary shards of the group) and to this rank's ``weight`` shard. The logits are
+    vocabulary shards of the group) and to this rank's ``weight`` shard. Without kept ``logits`` they are
     recomputed tile by tile inside the GEMM kernel (``kEpiLogitsGrad`` epilogue of
     ``csrc/sm100/gemm.cu``), which writes ``d_logits = g * scale * (onehot - softmax)`` as bf16
     for a panel of rows; two GEMMs follow: ``d_hidden = d_logits @ W``, ``d_W = d_logits^T @ hidden``."""
@@ -434,12 +490,19 @@ def _logp_backward(hidden, weight, ids, lse, g, scale, vocab, group, need_dh, ne
     for r0 in range(0, m, rows_per_panel):
         r1 = min(m, r0 + rows_per_panel)
         d_logits = torch.empty(r1 - r0, v_local, dtype=torch.bfloat16, device=h2.device)
-        rc = fn(h2[r0:r1].data_ptr(), w.data_ptr(), ids64[r0:r1].data_ptr(), lse32[r0:r1].data_ptr(),
-                g32[r0:r1].data_ptr(), d_logits.data_ptr(), v_local, r1 - r0, v_local, k, float(scale), lo,
-                _gemm.status_buffer(h2.device).data_ptr(), sms, default_timeout_ns(),
-                stream)
+        if logits is not None:
+            n_real = min(m_real, r1) - r0
+            rc = lib.ka_lmhead_kept_logits_grad(logits[r0:].data_ptr(), ids64[r0:].data_ptr(), lse32[r0:].data_ptr(),
+                                                g32[r0:].data_ptr(), d_logits.data_ptr(), n_real, v_local, float(scale),
+                                                stream)
+            if n_real < r1 - r0:
+                d_logits[n_real:].zero_()
+        else:
+            rc = fn(h2[r0:r1].data_ptr(), w.data_ptr(), ids64[r0:r1].data_ptr(), lse32[r0:r1].data_ptr(),
+                    g32[r0:r1].data_ptr(), d_logits.data_ptr(), v_local, r1 - r0, v_local, k, float(scale), lo,
+                    _gemm.status_buffer(h2.device).data_ptr(), sms, default_timeout_ns(), stream)
         if rc != 0:
-            raise RuntimeError(f"ka_lmhead_logits_grad rejected its arguments (code {rc})")
+            raise RuntimeError(f"the gradient of the logits rejected its arguments (code {rc})")
         if need_dh:
             d_hidden[r0:r1] = _gemm.gemm_bi(d_logits, w, trans_b=True)
         if need_dw:
@@ -463,18 +526,21 @@ class _LmheadLogpFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, hidden, weight, ids, scale, vocab, group, panel_rows, cta_group):
+        share, logits = _kept_logits(hidden, weight, vocab, group)
         logp, lse = _lmhead_logp_forward(hidden, weight, ids, scale=scale, vocab=vocab, group=group,
-                                         return_lse=True, panel_rows=panel_rows, cta_group=cta_group)
-        ctx.save_for_backward(hidden, weight, ids, lse)
+                                         return_lse=True, panel_rows=panel_rows, cta_group=cta_group, logits=logits)
+        ctx.save_for_backward(hidden, weight, ids, lse, *(() if logits is None else (logits,)))
+        ctx.share = share
         ctx.scale, ctx.vocab, ctx.group = scale, vocab, group
         ctx.mark_non_differentiable(lse)
         return logp, lse
 
     @staticmethod
     def backward(ctx, g, _g_lse):
-        hidden, weight, ids, lse = ctx.saved_tensors
+        hidden, weight, ids, lse, *logits = ctx.saved_tensors
         d_hidden, d_weight = _logp_backward(hidden, weight, ids, lse, g, ctx.scale, ctx.vocab, ctx.group,
-                                            ctx.needs_input_grad[0], ctx.needs_input_grad[1])
+                                            ctx.needs_input_grad[0], ctx.needs_input_grad[1],
+                                            logits[0] if logits else None)
         return (d_hidden.reshape(hidden.shape) if d_hidden is not None else None), d_weight, None, None, None, None, \
             None, None
 

@@ -147,3 +147,32 @@ def test_fused_logp_backward_matches_autograd(cuda_device):
     h2, w2 = h.clone().requires_grad_(), w.clone().requires_grad_()
     fused_logp.lmhead_logp(h2, w2, ids, scale=1 / 0.7).backward(g)
     assert torch.equal(h2.grad, hq.grad) and torch.equal(w2.grad, wq.grad)
+
+
+@pytest.mark.parametrize("m,k,v,scale", [(1, 64, 64, 1.0), (37, 128, 1920, 0.7), (300, 256, 16448, 1.0), (129, 64, 50304, 1.3)])
+def test_kept_logits_give_the_gradients_of_recomputed_ones(cuda_device, m, k, v, scale, monkeypatch):
+    """Bit for bit, for one sub-slice of the vocabulary and several, ignored ids, a second pass through
+    the graph, and a graph that finds the allowance used up."""
+    from kernel_align_b200.ops import fused_logp
+
+    g = torch.Generator(device=cuda_device).manual_seed(v)
+    h = torch.randn(m, k, device=cuda_device, generator=g).to(torch.bfloat16).requires_grad_()
+    w = (torch.randn(v, k, device=cuda_device, generator=g) * 0.2).to(torch.bfloat16).requires_grad_()
+    ids = torch.randint(-1, v + 1, (m,), device=cuda_device, generator=g)
+    up = torch.randn(m, device=cuda_device, generator=g)
+    before = dict(fused_logp._kept_bytes)
+    monkeypatch.setattr(fused_logp, "_KEEP_BYTES", sum(before.values()) + 4 * m * v)
+
+    def call():
+        return fused_logp.lmhead_logp(h, w, ids, scale=scale)
+
+    kept, other = call(), call()          # the second one recomputes
+    assert len(kept.grad_fn.saved_tensors) == 5 and len(other.grad_fn.saved_tensors) == 4
+    want = torch.autograd.grad(other, (h, w), up)
+    for _ in range(2):
+        got = torch.autograd.grad(kept, (h, w), up, retain_graph=True)
+        assert torch.equal(kept, other) and all(torch.equal(a, b) for a, b in zip(got, want))
+    with torch.no_grad():
+        assert torch.equal(call(), other)
+    del kept, other
+    assert {i: n for i, n in fused_logp._kept_bytes.items() if n} == {i: n for i, n in before.items() if n}
