@@ -176,3 +176,30 @@ def test_kept_logits_give_the_gradients_of_recomputed_ones(cuda_device, m, k, v,
         assert torch.equal(call(), other)
     del kept, other
     assert {i: n for i, n in fused_logp._kept_bytes.items() if n} == {i: n for i, n in before.items() if n}
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("vocab", [1, 7, 8, 17, 33, 4095, 16385, 50257])
+@pytest.mark.parametrize("times", [1, 200])
+def test_logits_logp_does_not_depend_on_where_a_row_starts(cuda_device, dtype, vocab, times):
+    """The same bits for a row on a 16-byte boundary and at every offset from one, in few rows and in many."""
+    from kernel_align_b200.ops.logits_logp import logits_logp
+
+    g = torch.Generator(device=cuda_device).manual_seed(vocab)
+    width = (vocab + 15) // 8 * 8
+    x = torch.full((3, width), float("nan"), device=cuda_device, dtype=dtype)
+    x[:, :vocab] = (torch.randn(3, vocab, device=cuda_device, generator=g) * 2).to(dtype)
+    ids = torch.tensor([0, vocab - 1, vocab // 2], device=cuda_device)
+    want, want_lse = logits_logp(x[:, :vocab], ids, return_lse=True)
+    exact = torch.log_softmax(x[:, :vocab].double(), -1).gather(1, ids[:, None])[:, 0]
+    # 32-bit sums of at most 50257 terms and two approximate functions of 2^-22 relative error
+    assert torch.allclose(want.double(), exact, rtol=1e-6, atol=4e-6)
+    rows = 3 * times
+    x, ids, want, want_lse = x.repeat(times, 1), ids.repeat(times), want.repeat(times), want_lse.repeat(times)
+    for off in range(16 // x.element_size()):
+        buf = torch.full((rows * (width + 1) + 8,), float("nan"), device=cuda_device, dtype=dtype)
+        for stride in (width, width + 1):
+            part = buf[off:off + rows * stride].view(rows, stride)[:, :vocab]
+            part.copy_(x[:, :vocab])
+            got, got_lse = logits_logp(part, ids, return_lse=True)
+            assert torch.equal(got, want) and torch.equal(got_lse, want_lse), (off, stride)
