@@ -17,6 +17,7 @@ from __future__ import annotations
 import ctypes
 import os
 import threading
+from collections import deque
 from dataclasses import dataclass, field
 from typing import Optional
 
@@ -396,6 +397,14 @@ _GRAD_PANEL_BYTES = 8 << 30
 _KEEP_BYTES = 2 << 30
 _kept_bytes: dict[int, int] = {}
 _kept_lock = threading.Lock()
+_given_back: deque = deque()      # (device, bytes) of shares that are gone and not yet subtracted
+
+
+def _subtract_given_back() -> None:
+    """Call with ``_kept_lock`` held."""
+    while _given_back:
+        index, nbytes = _given_back.popleft()
+        _kept_bytes[index] -= nbytes
 
 
 class _Kept:
@@ -407,14 +416,21 @@ class _Kept:
     @classmethod
     def take(cls, index: int, nbytes: int) -> Optional["_Kept"]:
         with _kept_lock:
+            _subtract_given_back()
             if _kept_bytes.get(index, 0) + nbytes > _KEEP_BYTES:
                 return None
             _kept_bytes[index] = _kept_bytes.get(index, 0) + nbytes
         return cls(index, nbytes)
 
     def __del__(self):
-        with _kept_lock:
-            _kept_bytes[self.index] -= self.nbytes
+        # May run inside take(), on the thread that holds the lock (a collection frees a share that sat in a
+        # reference cycle): it never waits, and leaves the subtraction to the lock's holder or the next take().
+        _given_back.append((self.index, self.nbytes))
+        if _kept_lock.acquire(blocking=False):
+            try:
+                _subtract_given_back()
+            finally:
+                _kept_lock.release()
 
 
 def _kept_logits(hidden, weight, vocab, group):
