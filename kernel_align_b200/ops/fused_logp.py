@@ -545,7 +545,13 @@ class _LmheadLogpFn(torch.autograd.Function):
         share, logits = _kept_logits(hidden, weight, vocab, group)
         logp, lse = _lmhead_logp_forward(hidden, weight, ids, scale=scale, vocab=vocab, group=group,
                                          return_lse=True, panel_rows=panel_rows, cta_group=cta_group, logits=logits)
-        ctx.save_for_backward(hidden, weight, ids, lse, *(() if logits is None else (logits,)))
+        # The saved tensors are the same whether logits are kept or not: checkpointing compares their number and
+        # shapes between a call and its repetition, and hooks move what is saved to the host. Kept logits hang
+        # on an alias of the ids that nobody else has, so autograd keeps and drops them with it, and a hook
+        # that puts another tensor in its place leaves a backward pass that recomputes them.
+        ids = ids.detach()
+        ids._ka_logits = logits
+        ctx.save_for_backward(hidden, weight, ids, lse)
         ctx.share = share
         ctx.scale, ctx.vocab, ctx.group = scale, vocab, group
         ctx.mark_non_differentiable(lse)
@@ -553,10 +559,10 @@ class _LmheadLogpFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g, _g_lse):
-        hidden, weight, ids, lse, *logits = ctx.saved_tensors
+        hidden, weight, ids, lse = ctx.saved_tensors
         d_hidden, d_weight = _logp_backward(hidden, weight, ids, lse, g, ctx.scale, ctx.vocab, ctx.group,
                                             ctx.needs_input_grad[0], ctx.needs_input_grad[1],
-                                            logits[0] if logits else None)
+                                            getattr(ids, "_ka_logits", None))
         return (d_hidden.reshape(hidden.shape) if d_hidden is not None else None), d_weight, None, None, None, None, \
             None, None
 

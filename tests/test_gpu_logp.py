@@ -167,7 +167,9 @@ def test_kept_logits_give_the_gradients_of_recomputed_ones(cuda_device, m, k, v,
         return fused_logp.lmhead_logp(h, w, ids, scale=scale)
 
     kept, other = call(), call()          # the second one recomputes
-    assert len(kept.grad_fn.saved_tensors) == 5 and len(other.grad_fn.saved_tensors) == 4
+    logits = [getattr(x.grad_fn.saved_tensors[2], "_ka_logits", None) for x in (kept, other)]
+    assert logits[0].shape == (m, v) and logits[1] is None
+    del logits
     want = torch.autograd.grad(other, (h, w), up)
     for _ in range(2):
         got = torch.autograd.grad(kept, (h, w), up, retain_graph=True)
@@ -203,3 +205,26 @@ def test_logits_logp_does_not_depend_on_where_a_row_starts(cuda_device, dtype, v
             part.copy_(x[:, :vocab])
             got, got_lse = logits_logp(part, ids, return_lse=True)
             assert torch.equal(got, want) and torch.equal(got_lse, want_lse), (off, stride)
+
+
+def test_kept_logits_under_checkpoint(cuda_device, monkeypatch):
+    """Checkpointed calls of more than half the allowance, and chunks that use it up: the repetition of a
+    call may find another part of the allowance free than the call itself."""
+    from torch.utils.checkpoint import checkpoint
+
+    from kernel_align_b200.ops import fused_logp
+
+    g = torch.Generator(device=cuda_device).manual_seed(5)
+    m, k, v = 256, 128, 1920
+    h = torch.randn(m, k, device=cuda_device, generator=g).to(torch.bfloat16).requires_grad_()
+    w = (torch.randn(v, k, device=cuda_device, generator=g) * 0.2).to(torch.bfloat16).requires_grad_()
+    ids = torch.randint(0, v, (m,), device=cuda_device, generator=g)
+    for chunks, allowance in ((1, m * 6), (4, m * 4), (4, m)):       # bytes per column, 4 * m in all
+        monkeypatch.setattr(fused_logp, "_KEEP_BYTES", sum(fused_logp._kept_bytes.values()) + allowance * v)
+        grads = []
+        for use in (False, True):
+            parts = [checkpoint(fused_logp.lmhead_logp, a, w, b, use_reentrant=False) if use
+                     else fused_logp.lmhead_logp(a, w, b) for a, b in zip(h.chunk(chunks), ids.chunk(chunks))]
+            grads.append(torch.autograd.grad(torch.cat(parts).sum(), (h, w)))
+            del parts
+        assert all(torch.equal(a, b) for a, b in zip(*grads))

@@ -3,6 +3,12 @@ import subprocess
 import sys
 import textwrap
 
+import pytest
+import torch
+from torch.utils.checkpoint import checkpoint
+
+from kernel_align_b200.ops import fused_logp
+
 _SHARES_IN_CYCLES = """
 import gc, threading
 from kernel_align_b200.ops import fused_logp as f
@@ -31,3 +37,46 @@ def test_share_collected_while_another_is_taken():
     r = subprocess.run([sys.executable, "-c", textwrap.dedent(_SHARES_IN_CYCLES)], timeout=120, capture_output=True,
                        text=True)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def _keep_on_cpu(monkeypatch, allowance):
+    """Calls on the CPU take shares and keep (unused) logits as calls on a GPU do."""
+    def kept_logits(hidden, weight, vocab, group):
+        m, v = hidden.numel() // hidden.shape[-1], weight.shape[0]
+        share = fused_logp._Kept.take(99, 4 * m * v)
+        return (None, None) if share is None else (share, torch.empty(m, v))
+
+    monkeypatch.setattr(fused_logp, "_kept_logits", kept_logits)
+    monkeypatch.setattr(fused_logp, "_KEEP_BYTES", fused_logp._kept_bytes.get(99, 0) + allowance)
+
+
+def _inputs(m=8, k=16, v=64):
+    g = torch.Generator().manual_seed(m)
+    h = torch.randn(m, k, generator=g).to(torch.bfloat16).requires_grad_()
+    w = torch.randn(v, k, generator=g).to(torch.bfloat16).requires_grad_()
+    return h, w, torch.randint(0, v, (m,), generator=g)
+
+
+@pytest.mark.parametrize("chunks,allowance", [(1, 6 * 8 * 64), (4, 4 * 8 * 64), (4, 8 * 64)])
+def test_checkpoint_with_an_allowance_that_is_used_up(monkeypatch, chunks, allowance):
+    """The repetition of a checkpointed call may find another part of the allowance free than the call."""
+    _keep_on_cpu(monkeypatch, allowance)
+    h, w, ids = _inputs()
+    grads = []
+    for use in (False, True):
+        parts = [checkpoint(fused_logp.lmhead_logp, a, w, b, use_reentrant=False) if use
+                 else fused_logp.lmhead_logp(a, w, b) for a, b in zip(h.chunk(chunks), ids.chunk(chunks))]
+        grads.append(torch.autograd.grad(torch.cat(parts).sum(), (h, w)))
+        del parts
+    assert all(torch.equal(a, b) for a, b in zip(*grads))
+
+
+def test_saved_tensors_do_not_depend_on_what_is_kept(monkeypatch):
+    h, w, ids = _inputs()
+    _keep_on_cpu(monkeypatch, 4 * 8 * 64)
+    seen = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: seen.append((tuple(t.shape), t.dtype)) or t, lambda t: t):
+        first = fused_logp.lmhead_logp(h, w, ids)
+        second = fused_logp.lmhead_logp(h, w, ids)     # finds the allowance used up
+    assert seen[:len(seen) // 2] == seen[len(seen) // 2:] and len(seen) == 8
+    assert torch.equal(first, second)
