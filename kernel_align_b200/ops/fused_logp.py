@@ -408,10 +408,11 @@ def _subtract_given_back() -> None:
 
 
 class _Kept:
-    """A share of a device's allowance for kept logits, given back when the graph node that holds it goes."""
+    """Kept logits and their share of a device's allowance, given back when they are dropped."""
 
     def __init__(self, index: int, nbytes: int):
         self.index, self.nbytes = index, nbytes
+        self.logits: Optional[torch.Tensor] = None
 
     @classmethod
     def take(cls, index: int, nbytes: int) -> Optional["_Kept"]:
@@ -433,20 +434,21 @@ class _Kept:
                 _kept_lock.release()
 
 
-def _kept_logits(hidden, weight, vocab, group):
-    """``(share, logits)`` for a forward call whose logits are kept, or ``(None, None)``."""
+def _kept_logits(hidden, weight, vocab, group) -> Optional[_Kept]:
+    """Room for the logits of a forward call, or None if they are not kept."""
     v = int(weight.shape[0])
     m = hidden.numel() // max(1, hidden.shape[-1])
     if (hidden.device.type != "cuda" or group is not None or v % 64 != 0 or not 0 < m <= 65535
             or (vocab is not None and int(vocab) != v)):
-        return None, None
-    share = _Kept.take(_native._device_index(hidden.device), 4 * m * v)
-    if share is None:
-        return None, None
+        return None
+    kept = _Kept.take(_native._device_index(hidden.device), 4 * m * v)
+    if kept is None:
+        return None
     try:
-        return share, torch.empty(m, v, dtype=torch.float32, device=hidden.device)
+        kept.logits = torch.empty(m, v, dtype=torch.float32, device=hidden.device)
     except torch.OutOfMemoryError:
-        return None, None
+        return None
+    return kept
 
 
 def _logp_backward(hidden, weight, ids, lse, g, scale, vocab, group, need_dh, need_dw, logits=None):
@@ -542,17 +544,18 @@ class _LmheadLogpFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, hidden, weight, ids, scale, vocab, group, panel_rows, cta_group):
-        share, logits = _kept_logits(hidden, weight, vocab, group)
-        logp, lse = _lmhead_logp_forward(hidden, weight, ids, scale=scale, vocab=vocab, group=group,
-                                         return_lse=True, panel_rows=panel_rows, cta_group=cta_group, logits=logits)
+        kept = _kept_logits(hidden, weight, vocab, group)
+        logp, lse = _lmhead_logp_forward(hidden, weight, ids, scale=scale, vocab=vocab, group=group, return_lse=True,
+                                         panel_rows=panel_rows, cta_group=cta_group,
+                                         logits=kept.logits if kept is not None else None)
         # The saved tensors are the same whether logits are kept or not: checkpointing compares their number and
         # shapes between a call and its repetition, and hooks move what is saved to the host. Kept logits hang
-        # on an alias of the ids that nobody else has, so autograd keeps and drops them with it, and a hook
-        # that puts another tensor in its place leaves a backward pass that recomputes them.
+        # on an alias of the ids that nobody else has, so autograd keeps and drops them (and their share of the
+        # allowance) with it, and a hook that puts another tensor in its place leaves a backward pass that
+        # recomputes them.
         ids = ids.detach()
-        ids._ka_logits = logits
+        ids._ka_kept = kept
         ctx.save_for_backward(hidden, weight, ids, lse)
-        ctx.share = share
         ctx.scale, ctx.vocab, ctx.group = scale, vocab, group
         ctx.mark_non_differentiable(lse)
         return logp, lse
@@ -560,9 +563,10 @@ class _LmheadLogpFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g, _g_lse):
         hidden, weight, ids, lse = ctx.saved_tensors
+        kept = getattr(ids, "_ka_kept", None)
         d_hidden, d_weight = _logp_backward(hidden, weight, ids, lse, g, ctx.scale, ctx.vocab, ctx.group,
                                             ctx.needs_input_grad[0], ctx.needs_input_grad[1],
-                                            getattr(ids, "_ka_logits", None))
+                                            kept.logits if kept is not None else None)
         return (d_hidden.reshape(hidden.shape) if d_hidden is not None else None), d_weight, None, None, None, None, \
             None, None
 

@@ -167,9 +167,9 @@ def test_kept_logits_give_the_gradients_of_recomputed_ones(cuda_device, m, k, v,
         return fused_logp.lmhead_logp(h, w, ids, scale=scale)
 
     kept, other = call(), call()          # the second one recomputes
-    logits = [getattr(x.grad_fn.saved_tensors[2], "_ka_logits", None) for x in (kept, other)]
-    assert logits[0].shape == (m, v) and logits[1] is None
-    del logits
+    holders = [x.grad_fn.saved_tensors[2]._ka_kept for x in (kept, other)]
+    assert holders[0].logits.shape == (m, v) and holders[1] is None
+    del holders
     want = torch.autograd.grad(other, (h, w), up)
     for _ in range(2):
         got = torch.autograd.grad(kept, (h, w), up, retain_graph=True)
@@ -228,3 +228,25 @@ def test_kept_logits_under_checkpoint(cuda_device, monkeypatch):
             grads.append(torch.autograd.grad(torch.cat(parts).sum(), (h, w)))
             del parts
         assert all(torch.equal(a, b) for a, b in zip(*grads))
+
+
+def test_kept_logits_are_gone_after_the_backward_pass(cuda_device):
+    """Their share of the allowance as well, whoever holds the result; and with a hook that moves what is
+    saved to the host."""
+    from kernel_align_b200.ops import fused_logp
+
+    h, w, ids = _inputs(cuda_device, 64, 128, 1920, seed=3)
+    h.requires_grad_()
+    before = dict(fused_logp._kept_bytes).get(cuda_device.index or 0, 0)
+    nbytes = 4 * 64 * 1920
+    results, grads = [], []
+    for _ in range(3):
+        results.append(fused_logp.lmhead_logp(h, w, ids))
+        assert fused_logp._kept_bytes[cuda_device.index or 0] == before + nbytes
+        grads += torch.autograd.grad(results[-1].sum(), h)
+        assert fused_logp._kept_bytes[cuda_device.index or 0] == before
+    with torch.autograd.graph.save_on_cpu():
+        results.append(fused_logp.lmhead_logp(h, w, ids))
+        assert fused_logp._kept_bytes[cuda_device.index or 0] == before
+        grads += torch.autograd.grad(results[-1].sum(), h)
+    assert all(torch.equal(a, grads[0]) for a in grads)

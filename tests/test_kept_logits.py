@@ -43,8 +43,10 @@ def _keep_on_cpu(monkeypatch, allowance):
     """Calls on the CPU take shares and keep (unused) logits as calls on a GPU do."""
     def kept_logits(hidden, weight, vocab, group):
         m, v = hidden.numel() // hidden.shape[-1], weight.shape[0]
-        share = fused_logp._Kept.take(99, 4 * m * v)
-        return (None, None) if share is None else (share, torch.empty(m, v))
+        kept = fused_logp._Kept.take(99, 4 * m * v)
+        if kept is not None:
+            kept.logits = torch.empty(m, v)
+        return kept
 
     monkeypatch.setattr(fused_logp, "_kept_logits", kept_logits)
     monkeypatch.setattr(fused_logp, "_KEEP_BYTES", fused_logp._kept_bytes.get(99, 0) + allowance)
@@ -80,3 +82,35 @@ def test_saved_tensors_do_not_depend_on_what_is_kept(monkeypatch):
         second = fused_logp.lmhead_logp(h, w, ids)     # finds the allowance used up
     assert seen[:len(seen) // 2] == seen[len(seen) // 2:] and len(seen) == 8
     assert torch.equal(first, second)
+
+
+def _kept_now():
+    return fused_logp._kept_bytes.get(99, 0)
+
+
+def test_allowance_follows_the_logits_and_not_the_node(monkeypatch):
+    """After a backward pass, behind a checkpoint and with a hook that copies, the logits are gone and so is
+    their share, whoever still holds the result; a retained graph keeps both."""
+    nbytes = 4 * 8 * 64
+    _keep_on_cpu(monkeypatch, nbytes)
+    before = _kept_now()
+    h, w, ids = _inputs()
+    results = []
+    for _ in range(2):
+        logp = fused_logp.lmhead_logp(h, w, ids)
+        assert _kept_now() == before + nbytes
+        logp.sum().backward(retain_graph=True)
+        assert _kept_now() == before + nbytes
+        logp.sum().backward()
+        assert _kept_now() == before
+        results.append(logp)
+    results.append(checkpoint(fused_logp.lmhead_logp, h, w, ids, use_reentrant=False))
+    assert _kept_now() == before
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.clone(), lambda t: t):
+        results.append(fused_logp.lmhead_logp(h, w, ids))
+        assert _kept_now() == before
+        want = torch.autograd.grad(results[-1].sum(), (h, w))
+    logp = fused_logp.lmhead_logp(h, w, ids)
+    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(logp.sum(), (h, w)), want))
+    fused_logp.lmhead_logp(h, w, ids)          # dropped without a backward pass
+    assert _kept_now() == before
