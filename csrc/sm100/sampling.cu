@@ -1223,7 +1223,8 @@ __device__ __forceinline__ unsigned long long warp_incl_u64(unsigned long long v
 //   * Counters are 16 bits, two per word (128 KiB), named by the value's bits as they are; only what reads
 //     them puts them in the order of keys, by groups of 32. An overflow loses at least 65535 from the sum
 //     of the counters, so "sum == v" says that none happened; a row in which one value fills more than
-//     65535 places takes the older search, and so does a row with NaNs.
+//     65535 places takes the older search. NaNs, which have many bit patterns and one key, are moved to that
+//     key's counter, if there are any, and the groups are counted once more.
 //   * Only groups that occur are visited when masses are added up (150 of 2048 for bf16 logits).
 //   * The masses of the keys above the threshold go to a table in the counters' place if there are fewer
 //     than 16384 of them (a few hundred for top-p on bf16 logits). Its entries are 64 bits, so that a tie at
@@ -1527,8 +1528,9 @@ __device__ bool sample_row16(const T* rp, int v, float inv_temp, int top_k, floa
   }
   __syncthreads();
   // ---- counts per group of 32 keys (four threads' vectors of eight counters), their sum, which groups occur
-  {
-    constexpr uint32_t kInf = Elem<T>::kInf2 & 0xFFFFu;
+  constexpr uint32_t kInf = Elem<T>::kInf2 & 0xFFFFu;
+#pragma unroll 1
+  for (bool again = false;; again = true) {
     constexpr int kN = kHistWords / 4 / kThreads;
     unsigned int n[kN], occurs[kN], sum = 0, nans = 0, top = 0, found = 0;
     const bool lead = (lane & 3) == 0;
@@ -1576,9 +1578,21 @@ __device__ bool sample_row16(const T* rp, int v, float inv_temp, int top_k, floa
       if (nans) atomicAdd(&f.nans, nans);
       atomicMax(&f.top_group, top);
     }
+    __syncthreads();
+    if (f.total != static_cast<unsigned int>(v)) return false;   // a counter overflowed
+    const unsigned int n_nan = f.nans;
+    if (again || n_nan == 0) break;
+    if (n_nan > 0xFFFFu) return false;
+    __syncthreads();
+    // the patterns above infinity's, of both signs, hold nothing any more; key 0 (0xFFFF's counter) holds them all
+    for (uint32_t w = (kInf >> 1) + tid; w < 0x4000u; w += kThreads) {
+      const bool inf = w == kInf >> 1;         // infinity's own counter is the lower half
+      f.words[w] = inf ? f.words[w] & 0xFFFFu : 0u;
+      f.words[w + 0x4000u] = (inf ? f.words[w + 0x4000u] & 0xFFFFu : 0u) | (w == 0x3FFFu ? n_nan << 16 : 0u);
+    }
+    if (tid == 0) f.n_list = f.total = f.top_group = 0;
+    __syncthreads();
   }
-  __syncthreads();
-  if (f.total != static_cast<unsigned int>(v) || f.nans != 0) return false;   // a counter overflowed, or NaNs
   uint32_t max_key;
   {
     const uint32_t key = f.top_group * 32u + static_cast<uint32_t>(lane);

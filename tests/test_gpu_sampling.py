@@ -180,3 +180,29 @@ def test_sampler_without_small_top_k_special_values(cuda_device, dtype, vocab):
                 tok = sample(logits, top_k=k, top_p=top_p, temperature=temperature, seed=8, step=off)
                 ref = _cpu(logits, k, top_p, temperature, 8, off)
                 assert torch.equal(tok.cpu(), ref), (name, off, k, top_p)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("vocab", [1025, 33001, 140001])
+def test_sampler_nan_patterns(cuda_device, dtype, vocab):
+    """NaNs of every bit pattern and both signs are one key, the lowest: among plain values, as most of a
+    row (more of them than a 16-bit counter holds, too), below a maximum next to their own patterns, alone."""
+    g = torch.Generator(device=cuda_device).manual_seed(vocab)
+    x = torch.randn(4, vocab, device=cuda_device, generator=g) * 2
+    u = torch.rand(x.shape, device=cuda_device, generator=g)
+    inf = torch.tensor(float("inf"), dtype=dtype).view(torch.int16).item()
+    nan = (torch.randint(inf + 1, 0x8000, x.shape, device=cuda_device, generator=g) -
+           0x8000 * torch.randint(0, 2, x.shape, device=cuda_device, generator=g)).to(torch.int16).view(dtype)
+    assert nan.isnan().all()
+    low = torch.full_like(x, torch.finfo(dtype).min).to(dtype)
+    low.view(torch.int16)[:, ::3] -= 40               # 40 steps above the lowest value
+    x = x.to(dtype)
+    for name, val in {"few": torch.where(u < 0.01, nan, x), "most": torch.where(u < 0.9, nan, x),
+                      "masked": torch.where(u < 0.3, nan, torch.where(u < 0.9, float("-inf"), x)),
+                      "lowest": torch.where(u < 0.5, nan, low), "one_left": torch.where(u < u.max(), nan, x),
+                      "all": nan}.items():
+        for top_k, top_p, temperature in ((None, 0.9, 1.0), (None, 0.9999, 2.0), (1024, 0.8, 1.0), (1100, None, 0.3),
+                                          (20000, 0.99, 1.0), (None, 0.5, 1e30)):
+            k = None if top_k is not None and top_k >= vocab else top_k
+            tok = sample(val, top_k=k, top_p=top_p, temperature=temperature, seed=6, step=3)
+            assert torch.equal(tok.cpu(), _cpu(val, k, top_p, temperature, 6, 3)), (name, k, top_p, temperature)
