@@ -362,13 +362,17 @@ __device__ __forceinline__ uint32_t kth_of_warp_tops(uint32_t w, int kk, TopkSme
   return s.bound;
 }
 
-// A bound that at least kk of the keys in the block's words reach.
+// A bound that at least kk of the keys in the block's words reach; nvec: vectors of the row that the block
+// holds, thread by thread. In a short row only a few warps have keys to bring, and with fewer than kk of them
+// the bound would be 0 and every element a candidate: while they bring less than 2 kk, the block searches
+// (bf16, 200 rows of 1000 columns, k = 50: 24.3 us with the warps' keys, 11.6 with the search).
 template <int NW, int kBits, int kBlockWarps>
-__device__ __forceinline__ uint32_t bound_of(const uint32_t (&w)[NW], int kk, TopkSmem& s) {
-  if constexpr (NW == 1)
-    return kth_of_warp_tops<kBits, kBlockWarps>(w[0], kk, s);
-  else
-    return kth_key<NW, kBits>(w, kk, s.hits);
+__device__ __forceinline__ uint32_t bound_of(const uint32_t (&w)[NW], int kk, int nvec, TopkSmem& s) {
+  if constexpr (NW == 1) {
+    const int warps = min(kBlockWarps, (nvec + 31) / 32);
+    if (warps * (kWarpTops / kBlockWarps) >= 2 * kk) return kth_of_warp_tops<kBits, kBlockWarps>(w[0], kk, s);
+  }
+  return kth_key<NW, kBits>(w, kk, s.hits);
 }
 
 // s.sorted[0 .. 1023] descending, by 256 threads that hold four neighbours each: partners at distance 1
@@ -775,7 +779,7 @@ sample_topk_kernel(const T* __restrict__ logits, long long row_stride, int v, co
                                          : static_cast<unsigned long long>(row);
   const uint32_t u24 = uniform_u24(seed, rid, step);
   words_to_keys<T>(mx);
-  const Bound<T> bound(bound_of<NW, Elem<T>::kPacked ? 16 : 32, kTopkThreads / 32>(mx, kk, s));
+  const Bound<T> bound(bound_of<NW, Elem<T>::kPacked ? 16 : 32, kTopkThreads / 32>(mx, kk, nvec, s));
   auto push = [&](uint32_t key, int idx) {
     const int slot = atomicAdd(&s.count, 1);
     if (slot < kCandCap) s.cand[slot] = cand_of(key, idx);
@@ -892,7 +896,7 @@ sample_topk_held_kernel(const T* __restrict__ logits, long long row_stride, int 
 #pragma unroll
   for (int u = 0; u < kHeldVecs; ++u) mx[u % NW] = Elem<T>::wmax(mx[u % NW], vec_max<T>(raw[u]));
   words_to_keys<T>(mx);
-  uint32_t low16 = bound_of<NW, 16, kHeldThreads / 32>(mx, kk, s);
+  uint32_t low16 = bound_of<NW, 16, kHeldThreads / 32>(mx, kk, v1 - v0, s);
   if constexpr (C > 1) {
     cluster_wait_acquire();                            // every CTA of the cluster runs, its counter is zero
     if constexpr (NW > 1) {
