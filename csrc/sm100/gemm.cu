@@ -758,18 +758,13 @@ inline bool narrow_tiles(int tiles_m, int tiles_n, int k, bool tree, int pairs) 
   return static_cast<long long>(tiles_m) * tiles_n * 2 <= pairs && (tree || k <= kNarrowMaxK);
 }
 
-// A product whose slices are units of their own (split) has eight times as many units: narrow ones where
-// they come out ahead in rounds, at about 0.55 of the time each.
-inline bool narrow_split_units(long long tiles, int pairs) {
-  const long long wide = (tiles * kTreeSlices + pairs - 1) / pairs, narrow = (2 * tiles * kTreeSlices + pairs - 1) / pairs;
-  return narrow * 11 < wide * 20;
-}
-
-// ---- split mode (ka_gemm_split8). A pair that keeps a tile walks its eight slices one after the other, at
-// about 0.31 us per 64-wide K block whatever the tile's width, so few tiles with a long K leave most pairs
-// idle; with the slices spread over all pairs 128 x 4096 takes 18.5 us instead of 37.7 (K = 4096), 39.7 instead
-// of 86.0 (14336), 60 instead of 152 (28672); 512 x 4096 37.3 / 40.3, 80 / 90, 143 / 156; 512 x 1024 15.4 / 36.3
-// (4096). The price is a pass over the partials, 3 to 6 us (they stay in L2). Second half: the eight bf16 partials
+// ---- split mode (ka_gemm_split8). A pair that keeps a tile walks its eight slices one after the other, so few
+// tiles with a long K leave most pairs idle; the times of both are with the rule (_split_pays in
+// parallel/tp_gemm.py). The price is a pass over the partials, 3 to 6 us (they stay in L2). A unit is always a
+// tile of 256 columns: with 128 there are twice as many, and one takes 0.7 (K = 4096) to 0.9 (28672) of the
+// time. Wide / narrow units in us: 512 x 1024 19.6 / 19.3 (K = 4096), 34.3 / 50.3 (28672), 128 x 5120 24.1 / 28.1,
+// 79.3 / 105.5; 512 x 4096 32.2 / 36.8, 101.5 / 143.8; 768 x 4096 44.7 / 52.7, 148.6 / 218.6; 128 x 1024, where
+// both are one round, 19.3 / 19.2, 32.3 / 31.5. Second half: the eight bf16 partials
 // of every element summed in the order of the reduce-scatter tail, ((0+1)+(2+3))+((4+5)+(6+7)) in fp32,
 // rounded, the residual added after that.
 constexpr int kSumThreads = 256;
@@ -817,10 +812,8 @@ int gemm_launch(const void* a, long long lda, const void* b, long long ldb, cons
   int ctas = tree ? max_ctas<true, kBN>(num_sms) : max_ctas<false, kBN>(num_sms);
   if (ctas <= 0) return -10;
   const int tiles_m = (p.m + kBM * kG - 1) / (kBM * kG);
-  const int wide_n = (p.n + kBN - 1) / kBN;
-  const bool split = p.c_slice_stride != 0;
-  const bool narrow = !full_grid && (split ? narrow_split_units(static_cast<long long>(tiles_m) * wide_n, ctas / kG)
-                                           : narrow_tiles(tiles_m, wide_n, p.k, tree, ctas / kG));
+  const bool narrow = !full_grid && p.c_slice_stride == 0 &&
+                      narrow_tiles(tiles_m, (p.n + kBN - 1) / kBN, p.k, tree, ctas / kG);
   if (narrow) ctas = tree ? max_ctas<true, kBN / 2>(num_sms) : max_ctas<false, kBN / 2>(num_sms);
   if (ctas <= 0) return -10;
   const int bn = narrow ? kBN / 2 : kBN;

@@ -110,12 +110,14 @@ def _gemm_reduce_scatter_cpu(x, w_shard, ctx, residual, trans_b, keep_padding):
 def _split_pays(m: int, n: int, k: int) -> bool:
     """Whether one rank that sums its eight K slices itself makes them units of their own
     (``ka_gemm_split8``: eight times as many units, a pass over the partials) or keeps a tile's slices on one
-    CTA pair (``ka_gemm_tree8``). Measured split / kept in us on 74 pairs, tiles counted as 256 x 256: 4 tiles:
-    10 / 26 (K = 1024), 13 / 36 (4096); 16 tiles: 16 / 26 (1024), 18.5 / 38 (4096), 40 / 86 (14336), 60 / 152
-    (28672); 32 tiles: 27 / 27 (1024), 28 / 24 (1536), 37 / 40 (4096), 42 / 43 (6144), 80 / 90 (14336),
-    143 / 156 (28672); 48 tiles: 43 / 53 (4096), 46 / 51 (6144), 81 / 104 (14336); 64 tiles: 52 / 54 (4096),
-    54 / 53 (6144), 96 / 106 (14336), 161 / 171 (28672); with more tiles the partials outgrow what the rest saves
-    (256 tiles: 196 / 185 at 6144, 688 / 706 at 28672, with half a gigabyte of scratch)."""
+    CTA pair (``ka_gemm_tree8``). Measured split / kept in us on 74 pairs, calls after one another (19 us is what
+    the host takes for one), tiles counted as 256 x 256: 4 tiles: 19 / 27 (K = 1024), 19 / 33 (4096); 16 tiles:
+    20 / 27 (1024), 20 / 35 (4096), 37 / 67 (14336), 58 / 98 (28672); 32 tiles: 32 / 35 (4096), 37 / 46 (6144),
+    61 / 87 (14336), 101 / 147 (28672); 48 tiles: 45 / 45 (4096), 49 / 54 (6144), 83 / 95 (14336), 149 / 165 (28672);
+    64 tiles: 99 / 101 (14336), 180 / 185 (28672). One row instead of 128 or 512, whose tiles are mostly
+    padding: 16 tiles 42 / 49 (14336), 63 / 75 (28672); 20 tiles 49 / 60, 84 / 98; 32 tiles 72 / 98, 109 / 129. With
+    more tiles the partials outgrow what the rest saves (256 tiles: 196 / 185 at 6144, 688 / 706 at 28672,
+    with half a gigabyte of scratch)."""
     tiles = -(-m // 256) * -(-n // 256)
     return tiles <= 24 or (tiles <= 48 and k >= 4096) or (tiles <= 64 and k >= 12288)
 

@@ -68,8 +68,8 @@ def test_slices_summed_in_the_kernel_equal_the_staged_ones_bitwise(cuda_device, 
 @pytest.mark.parametrize("m,n,k,trans_b", [(1, 8, 512, False), (127, 264, 1024, True), (300, 1032, 512, False),
                                            (1000, 4096, 1536, True), (1100, 4104, 512, False)])
 def test_slices_as_units_of_their_own_equal_the_kept_ones_bitwise(cuda_device, m, n, k, trans_b, monkeypatch):
-    """The eight K slices as separate units (narrow and wide ones, one round and several) and a sum over
-    their partials: the bits of a tile that keeps its slices."""
+    """The eight K slices as separate units (one round and several) and a sum over their partials: the bits
+    of a tile that keeps its slices."""
     from kernel_align_b200.parallel import tp_gemm
 
     ctx = TPContext(device=cuda_device)
