@@ -206,3 +206,25 @@ def test_sampler_nan_patterns(cuda_device, dtype, vocab):
             k = None if top_k is not None and top_k >= vocab else top_k
             tok = sample(val, top_k=k, top_p=top_p, temperature=temperature, seed=6, step=3)
             assert torch.equal(tok.cpu(), _cpu(val, k, top_p, temperature, 6, 3)), (name, k, top_p, temperature)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("vocab,rows", [(1000, 3), (4088, 3), (4104, 3), (50257, 2), (128256, 2), (200064, 2), (128256, 80)])
+def test_sampler_small_k_candidates_in_few_places(cuda_device, dtype, vocab, rows):
+    """Bounds from the warps' keys that are far too low for a part of a row (few finite elements in it, its
+    largest in a few warps, none at all) and more candidates than fit: by the hundred and by the thousand."""
+    g = torch.Generator(device=cuda_device).manual_seed(vocab)
+    x = torch.randn(rows, vocab, device=cuda_device, generator=g) * 2
+    u = torch.rand(x.shape, device=cuda_device, generator=g)
+    at = torch.arange(vocab, device=cuda_device)
+    few = torch.where(u < 1 - 130 / vocab, float("-inf"), x)
+    values = {"few_finite": few, "fewer": torch.where(u < 1 - 30 / vocab, float("-inf"), x),
+              "one": torch.where(at == vocab // 3, 1.0, torch.full_like(x, float("-inf"))),
+              "first_half": torch.where(at < vocab // 2, x, float("-inf")), "last": torch.where(at < vocab - 300, float("-inf"), x),
+              "sorted": x.sort(1, descending=True).values, "rising": x.sort(1).values, "equal": torch.ones_like(x),
+              "two_values": (u < 0.3).float(), "nan": torch.where(few.isinf(), float("nan"), few)}
+    for name, val in values.items():
+        val = val.to(dtype)
+        for top_k, top_p in ((1, None), (20, 0.9), (50, None), (64, 0.8)):
+            tok = sample(val, top_k=top_k, top_p=top_p, temperature=0.7, seed=2, step=top_k)
+            assert torch.equal(tok[:3].cpu(), _cpu(val[:3], top_k, top_p, 0.7, 2, top_k)), (name, top_k, top_p)
