@@ -70,7 +70,7 @@ class _GrpoLossFn(torch.autograd.Function):
             return loss, out
         m = mask.to(torch.uint8).contiguous() if mask is not None else None
         grad = torch.empty_like(ln)
-        out = torch.empty(3, dtype=torch.float32)
+        out = torch.empty(3, dtype=torch.float32, device=ln.device)
         fn = _native.cpu().ka_cpu_grpo_loss
         fn.restype = c_int
         fn.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_float, c_float,

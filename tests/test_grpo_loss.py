@@ -60,6 +60,16 @@ def test_grpo_loss_cpu():
     _check(torch.device("cpu"))
 
 
+def test_grpo_loss_follows_its_inputs_and_not_the_default_device():
+    ln, lo = torch.randn(4, 8, requires_grad=True), torch.randn(4, 8)
+    adv = torch.randn(4)
+    want, want_stats = grpo_loss(ln, lo, adv, return_stats=True)
+    with torch.device("meta"):
+        got, stats = grpo_loss(ln, lo, adv, return_stats=True)
+        assert torch.equal(grpo_loss(ln, lo, adv), want)
+    assert torch.equal(got, want) and torch.equal(stats, want_stats)
+
+
 @pytest.mark.gpu
 def test_grpo_loss_gpu(cuda_device):
     _check(cuda_device)
