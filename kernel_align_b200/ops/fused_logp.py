@@ -392,12 +392,41 @@ _GRAD_PANEL_BYTES = 8 << 30
 # same size; keeping them (fp32, as the forward kernel has them: the gradients are the same bits) costs a
 # write of 4 bytes per logit under the forward's products and a read: 2000 x 4096 x 128256, forward and
 # backward: 6.9 -> 5.7 ms. It is done while what all live graphs of a device keep stays below
-# _KEEP_BYTES (1.1 % of its memory, two calls of 2000 rows at 128256 columns); beyond that, or when the
-# allocation fails, the logits are recomputed and never materialised.
+# _KEEP_BYTES (1.1 % of its memory, two calls of 2000 rows at 128256 columns; KA_LOGP_KEEP_BYTES sets
+# another limit, 0 for none at all) and a sixteenth of the device's memory stays available; otherwise the
+# logits are recomputed and never materialised.
 _KEEP_BYTES = 2 << 30
+# Asking for the available memory costs 8 us, and 72 more when the allocator's cache is not enough: it is done
+# for logits of at least this size, whose products take the GPU a quarter of a millisecond and more.
+_KEEP_UNASKED_BYTES = 64 << 20
 _kept_bytes: dict[int, int] = {}
 _kept_lock = threading.Lock()
 _given_back: deque = deque()      # (device, bytes) of shares that are gone and not yet subtracted
+
+
+def _keep_limit() -> int:
+    env = os.environ.get("KA_LOGP_KEEP_BYTES")
+    if not env:
+        return _KEEP_BYTES
+    try:
+        return int(env)
+    except ValueError:
+        raise ValueError("KA_LOGP_KEEP_BYTES must be a number of bytes") from None
+
+
+def _memory_to_spare(device: torch.device, nbytes: int) -> bool:
+    """Whether ``nbytes`` more leave a sixteenth of the device's memory free or in the allocator's cache: kept
+    logits must not be what a step runs out of memory for, and an allocation that fails empties the cache. A
+    capture, which allocates once, is not asked."""
+    if nbytes < _KEEP_UNASKED_BYTES or torch.cuda.is_current_stream_capturing():
+        return True
+    need = nbytes + torch.cuda.get_device_properties(device).total_memory // 16
+    try:
+        stats = torch.cuda.memory_stats_as_nested_dict(device)
+        cached = stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"]
+    except (RuntimeError, KeyError):      # an allocator without statistics
+        cached = 0
+    return cached >= need or cached + torch.cuda.mem_get_info(device)[0] >= need
 
 
 def _subtract_given_back() -> None:
@@ -418,7 +447,7 @@ class _Kept:
     def take(cls, index: int, nbytes: int) -> Optional["_Kept"]:
         with _kept_lock:
             _subtract_given_back()
-            if _kept_bytes.get(index, 0) + nbytes > _KEEP_BYTES:
+            if _kept_bytes.get(index, 0) + nbytes > _keep_limit():
                 return None
             _kept_bytes[index] = _kept_bytes.get(index, 0) + nbytes
         return cls(index, nbytes)
@@ -442,7 +471,7 @@ def _kept_logits(hidden, weight, vocab, group) -> Optional[_Kept]:
             or (vocab is not None and int(vocab) != v)):
         return None
     kept = _Kept.take(_native._device_index(hidden.device), 4 * m * v)
-    if kept is None:
+    if kept is None or not _memory_to_spare(hidden.device, 4 * m * v):
         return None
     try:
         kept.logits = torch.empty(m, v, dtype=torch.float32, device=hidden.device)

@@ -250,3 +250,22 @@ def test_kept_logits_are_gone_after_the_backward_pass(cuda_device):
         assert fused_logp._kept_bytes[cuda_device.index or 0] == before
         grads += torch.autograd.grad(results[-1].sum(), h)
     assert all(torch.equal(a, grads[0]) for a in grads)
+
+
+def test_kept_logits_need_memory_to_spare(cuda_device, monkeypatch):
+    """Neither with the limit at 0 nor while memory is short are logits kept; the gradients are the same."""
+    from kernel_align_b200.ops import fused_logp
+
+    h, w, ids = _inputs(cuda_device, 64, 128, 1920, seed=4)
+    h.requires_grad_()
+    monkeypatch.setattr(fused_logp, "_KEEP_UNASKED_BYTES", 0)
+    grads = []
+    for env, free, kept in (("", None, True), ("0", None, False), ("", 0, False)):
+        monkeypatch.setenv("KA_LOGP_KEEP_BYTES", env)
+        if free is not None:
+            torch.cuda.empty_cache()
+            monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: (free, 0))
+        logp = fused_logp.lmhead_logp(h, w, ids)
+        assert (logp.grad_fn.saved_tensors[2]._ka_kept is not None) == kept
+        grads += torch.autograd.grad(logp.sum(), h)
+    assert torch.equal(grads[0], grads[1]) and torch.equal(grads[0], grads[2])

@@ -114,3 +114,33 @@ def test_allowance_follows_the_logits_and_not_the_node(monkeypatch):
     assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(logp.sum(), (h, w)), want))
     fused_logp.lmhead_logp(h, w, ids)          # dropped without a backward pass
     assert _kept_now() == before
+
+
+def test_limit_from_the_environment(monkeypatch):
+    _keep_on_cpu(monkeypatch, 4 * 8 * 64)
+    before = _kept_now()
+    h, w, ids = _inputs()
+    for env, kept in (("0", 0), (str(before + 4 * 8 * 64), 4 * 8 * 64), (str(before + 4 * 8 * 64 - 1), 0)):
+        monkeypatch.setenv("KA_LOGP_KEEP_BYTES", env)
+        logp = fused_logp.lmhead_logp(h, w, ids)
+        assert _kept_now() == before + kept
+        del logp
+    monkeypatch.setenv("KA_LOGP_KEEP_BYTES", "2G")
+    with pytest.raises(ValueError, match="KA_LOGP_KEEP_BYTES"):
+        fused_logp.lmhead_logp(h, w, ids)
+
+
+@pytest.mark.parametrize("free,cached,nbytes,spare", [
+    (100 << 30, 0, 1 << 30, True), (0, 13 << 30, 1 << 30, True), (6 << 30, 6 << 30, 1 << 30, False),
+    (7 << 30, 6 << 30, 1 << 30, True), (0, 0, 1 << 20, True), (0, 0, 64 << 20, False)])
+def test_nothing_is_kept_when_memory_is_short(monkeypatch, free, cached, nbytes, spare):
+    """192 GiB in all, of which a sixteenth, 12 GiB, has to stay available."""
+    class Props:
+        total_memory = 192 << 30
+
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda d: Props)
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: (free, 192 << 30))
+    stats = {"reserved_bytes": {"all": {"current": 20 << 30}}, "allocated_bytes": {"all": {"current": (20 << 30) - cached}}}
+    monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda d: stats)
+    assert fused_logp._memory_to_spare(torch.device("cuda", 0), nbytes) is spare
