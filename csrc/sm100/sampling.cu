@@ -362,17 +362,25 @@ __device__ __forceinline__ uint32_t kth_of_warp_tops(uint32_t w, int kk, TopkSme
   return s.bound;
 }
 
-// A bound that at least kk of the keys in the block's words reach; nvec: vectors of the row that the block
-// holds, thread by thread. In a short row only a few warps have keys to bring, and with fewer than kk of them
-// the bound would be 0 and every element a candidate: while they bring less than 2 kk, the block searches
-// (bf16, 200 rows of 1000 columns, k = 50: 24.3 us with the warps' keys, 11.6 with the search).
-template <int NW, int kBits, int kBlockWarps>
-__device__ __forceinline__ uint32_t bound_of(const uint32_t (&w)[NW], int kk, int nvec, TopkSmem& s) {
-  if constexpr (NW == 1) {
-    const int warps = min(kBlockWarps, (nvec + 31) / 32);
-    if (warps * (kWarpTops / kBlockWarps) >= 2 * kk) return kth_of_warp_tops<kBits, kBlockWarps>(w[0], kk, s);
-  }
-  return kth_key<NW, kBits>(w, kk, s.hits);
+// How a block finds the bound: from the keys that the warps bring (one word per thread), or by a search among
+// all its maxima, one or four words per thread.
+enum BoundFrom : int { kWarpKeys = 0, kOneWord = 1, kFourWords = 4 };
+constexpr int words_of(int from) { return from == kFourWords ? 4 : 1; }
+
+// A bound that at least kk of the keys in the block's words reach.
+template <int kFrom, int kBits, int kBlockWarps>
+__device__ __forceinline__ uint32_t bound_of(const uint32_t (&w)[words_of(kFrom)], int kk, TopkSmem& s) {
+  if constexpr (kFrom == kWarpKeys)
+    return kth_of_warp_tops<kBits, kBlockWarps>(w[0], kk, s);
+  else
+    return kth_key<words_of(kFrom), kBits>(w, kk, s.hits);
+}
+
+// The search of one word, out of line: for a path that is rarely taken (inline it costs the one-CTA cluster 0.3 us
+// of 6.7, out of line it costs two CTAs 0.3 us of 9.1).
+__device__ __noinline__ uint32_t kth_key16_far(uint32_t w, int kk, TopkSmem& s) {
+  const uint32_t words[1] = {w};
+  return kth_key<1, 16>(words, kk, s.hits);
 }
 
 // s.sorted[0 .. 1023] descending, by 256 threads that hold four neighbours each: partners at distance 1
@@ -448,12 +456,15 @@ __device__ __forceinline__ T from_bits16(uint32_t h) {
   return *reinterpret_cast<const T*>(&us);
 }
 
-// The words a thread's largest elements are kept in: one up to this k, four for a larger one, so that the
-// number of maxima stays well above k (with as many maxima as k the bound would be the smallest of them and
-// the row's exact search the rule: k = 1000 took 334 us for 1 row of 128256 and 1365 us for 256, with four
-// words 33 and 59 us). Up to it the bound comes from what the warps bring (kth_of_warp_tops).
+// k up to which the bound may come from what the warps bring (bound_from has the rule)
 constexpr int kFewK = 64;
-constexpr int kRankSort = 512;   // candidates that are sorted by counting
+// Candidates that are ranked by counting, from more the k largest are searched first: eight steps over 16-bit keys,
+// sixteen over 32-bit ones, so the line lies higher there. On the GPU, us, counting / search: bf16, 500 candidates, 200
+// rows, k = 200: 26.0 / 15.9; 64 rows of 128256 columns, k = 200: 20.6 / 18.1; 8 rows of 8000, k = 400:
+// 17.9 / 16.9; fp32, 8 rows of 16000, k = 200: 12.6 / 14.4, k = 400 18.8 / 20.8; 200 rows
+// of 500, k = 200 (500): 27.0 / 20.0.
+template <typename T>
+constexpr int kRankSort = Elem<T>::kPacked ? 256 : 480;
 
 // Key of an element given as the low bits of a register word.
 template <typename T>
@@ -593,7 +604,7 @@ __device__ __forceinline__ void topk_finish(TopkSmem& s, int n_cand, const T* __
   }
 
   // ---- the kk survivors, sorted by (key desc, id asc)
-  if (n_cand <= kRankSort) {
+  if (n_cand <= kRankSort<T>) {
     // eight lanes count for one candidate
     for (int i0 = 0; i0 < n_cand; i0 += nt >> 3) {
       const int i = i0 + (tid >> 3);
@@ -688,17 +699,30 @@ __device__ __forceinline__ void topk_finish(TopkSmem& s, int n_cand, const T* __
           s.sorted[atomicAdd(&s.n_sorted, 1)] = c;
       }
     }
-    if (kk <= nt >> 3) {
-      // eight lanes count for one survivor, in place
+    if (kk <= nt >> 1) {
+      // eight lanes count for up to four survivors, in place
       __syncthreads();
-      const int i = tid >> 3;
-      const unsigned long long mine = i < kk ? s.sorted[i] : ~0ull;
-      uint32_t rank = 0;
-      for (int j = tid & 7; j < kk; j += 8) rank += s.sorted[j] > mine ? 1u : 0u;
+      const int group = tid >> 3, groups = nt >> 3;
+      unsigned long long mine[4];
+      uint32_t rank[4];
 #pragma unroll
-      for (int o = 1; o < 8; o <<= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
+      for (int c = 0; c < 4; ++c) {
+        mine[c] = group + c * groups < kk ? s.sorted[group + c * groups] : ~0ull;
+        rank[c] = 0;
+      }
+      for (int j = tid & 7; j < kk; j += 8) {
+        const unsigned long long other = s.sorted[j];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) rank[c] += other > mine[c] ? 1u : 0u;
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) rank[c] += __shfl_xor_sync(0xffffffffu, rank[c], o);
       __syncthreads();
-      if ((tid & 7) == 0 && i < kk) s.sorted[rank] = mine;
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if ((tid & 7) == 0 && group + c * groups < kk) s.sorted[rank[c]] = mine[c];
       __syncthreads();
     } else {
       for (int i = kk + tid; i < kMaxTopK; i += nt) s.sorted[i] = 0;   // sorts behind every candidate
@@ -761,14 +785,14 @@ __device__ __forceinline__ void topk_finish(TopkSmem& s, int n_cand, const T* __
 // block's maxima bounds the kk-th largest element from below. Bound by the two passes: bf16 [256, 128256],
 // k = 50, 33 us (49 us with the keys of all elements computed); fp32 [256, 128256] 66 us (70 us), 128255
 // columns 76 us (255 us when rows off a 16-byte boundary were read by scalars).
-template <typename T, int NW>
+template <typename T, int kFrom>
 __global__ void __launch_bounds__(kTopkThreads, 2)
 sample_topk_kernel(const T* __restrict__ logits, long long row_stride, int v, const long long* __restrict__ row_ids,
                    float inv_temp, int top_k, float top_p, unsigned long long seed, unsigned long long step,
                    int* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TopkSmem& s = *reinterpret_cast<TopkSmem*>(smem_raw);
-  constexpr int kVec = Elem<T>::kVec, nt = kTopkThreads;
+  constexpr int kVec = Elem<T>::kVec, nt = kTopkThreads, NW = words_of(kFrom);
   constexpr int kU = 8;                       // 16-byte loads in flight per thread
   static_assert(kU % NW == 0, "every word gets its share of a batch");
   const int tid = threadIdx.x;
@@ -801,7 +825,7 @@ sample_topk_kernel(const T* __restrict__ logits, long long row_stride, int v, co
                                          : static_cast<unsigned long long>(row);
   const uint32_t u24 = uniform_u24(seed, rid, step);
   words_to_keys<T>(mx);
-  const Bound<T> bound(bound_of<NW, Elem<T>::kPacked ? 16 : 32, kTopkThreads / 32>(mx, kk, nvec, s));
+  const Bound<T> bound(bound_of<kFrom, Elem<T>::kPacked ? 16 : 32, kTopkThreads / 32>(mx, kk, s));
   auto push = [&](uint32_t key, int idx) {
     const int slot = atomicAdd(&s.count, 1);
     if (slot < kCandCap) s.cand[slot] = cand_of(key, idx);
@@ -829,9 +853,9 @@ sample_topk_kernel(const T* __restrict__ logits, long long row_stride, int v, co
 // once and keeps it, so the row is read once and the collection costs no second pass. One CTA
 // with eight loads per thread and step needs several round trips to memory and the same again to L2.
 //   1. CTA r keeps its 1/C of the row and finds, as above, a bound that at least kk of its own
-//      elements reach. For a large k the bounds are exchanged through distributed shared memory and the
-//      largest serves the whole row (the part that produced it alone holds kk elements at or above it);
-//      for a small one the few more candidates cost less than the exchange.
+//      elements reach. One from a search is exchanged through distributed shared memory and the largest
+//      serves the whole row (the part that produced it alone holds kk elements at or above it); with the
+//      warps' keys, for a small k, the few more candidates cost less than the exchange.
 //   2. Every CTA collects the elements of its part that reach its bound; the others store theirs into
 //      CTA 0's shared memory, all meet at the cluster barrier, the others leave and CTA 0 finishes as the
 //      one-CTA kernel does. If the candidates of a small k do not fit, there is a second try with a bound
@@ -874,12 +898,13 @@ constexpr int kHeldThreads = 1024;
 constexpr int kHeldVecs = 8;                                          // 16-byte vectors a thread keeps
 constexpr int kHeldElems = kHeldThreads * kHeldVecs * 8;              // 16-bit elements a CTA keeps
 
-template <typename T, int C, int NW>
+template <typename T, int C, int kFrom>
 __global__ void __launch_bounds__(kHeldThreads, 1)
 sample_topk_held_kernel(const T* __restrict__ logits, long long row_stride, int v,
                         const long long* __restrict__ row_ids, float inv_temp, int top_k, float top_p,
                         unsigned long long seed, unsigned long long step, int* __restrict__ out) {
   static_assert(Elem<T>::kPacked, "the kernel takes 16-bit logits");
+  constexpr int NW = words_of(kFrom);
   static_assert(kHeldVecs % NW == 0, "every word gets its share of the vectors");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TopkSmem& s = *reinterpret_cast<TopkSmem*>(smem_raw);
@@ -914,10 +939,10 @@ sample_topk_held_kernel(const T* __restrict__ logits, long long row_stride, int 
 #pragma unroll
   for (int u = 0; u < kHeldVecs; ++u) mx[u % NW] = Elem<T>::wmax(mx[u % NW], vec_max<T>(raw[u]));
   words_to_keys<T>(mx);
-  uint32_t low16 = bound_of<NW, 16, kHeldThreads / 32>(mx, kk, v1 - v0, s);
+  uint32_t low16 = bound_of<kFrom, 16, kHeldThreads / 32>(mx, kk, s);
   if constexpr (C > 1) {
     cluster_wait_acquire();                            // every CTA of the cluster runs, its counter is zero
-    if constexpr (NW > 1) {
+    if constexpr (kFrom != kWarpKeys) {
       if (tid < C) st_remote_u32(map_to_cta(&x.low[cr], static_cast<uint32_t>(tid)), low16);
       cluster_arrive_release();
       cluster_wait_acquire();
@@ -934,15 +959,15 @@ sample_topk_held_kernel(const T* __restrict__ logits, long long row_stride, int 
   constexpr int kPart = C > 1 ? 1536 : 0, kList = kCandCap - (C - 1) * kPart;
   int total;
 #pragma unroll 1
-  for (bool again = NW > 1;; again = true) {
+  for (bool again = kFrom != kWarpKeys;; again = true) {
     const Bound<T> bound(low16);
     auto push = [&](uint32_t key, int idx) {
       const int slot = atomicAdd(&s.count, 1);
       if (slot < kCandCap) s.cand[slot] = cand_of(key, idx);
     };
-    // a thread with more than a few hits says that the bound is too low: no need to list them all
+    // with room for 1536 candidates a part, a thread with more than a few says that the bound is too low
     if (!visit_hits<T>(raw, (left + kHeldThreads - 1) / kHeldThreads, head + (v0 + tid) * 8, kHeldThreads * 8, bound,
-                       again ? kHeldVecs * 8 : 8, push))
+                       again || C == 1 ? kHeldVecs * 8 : 8, push))
       atomicAdd(&s.count, kCandCap + 1);
     if (has_scal) {
       const uint32_t key = key_of_bits<T>(scal_word);
@@ -975,15 +1000,32 @@ sample_topk_held_kernel(const T* __restrict__ logits, long long row_stride, int 
       if (!fits) total = kCandCap + 1;         // the row is searched exactly
       break;
     }
-    uint32_t wide[1] = {mx[0]};
-    low16 = max(low16, kth_key<1, 16>(wide, kk, s.hits));   // its barriers: everybody has read s.count
+    uint32_t wide;
+    if constexpr (C == 1) {
+      wide = kth_key16_far(mx[0], kk, s);
+    } else {
+      const uint32_t word[1] = {mx[0]};
+      wide = kth_key<1, 16>(word, kk, s.hits);
+    }
+    const uint32_t best = max(low16, wide);    // the search has barriers: everybody has read s.count
+    bool better = best > low16;
     if (tid == 0) s.count = 0;
     if constexpr (C > 1) {
-      if (tid < C) st_remote_u32(map_to_cta(&x.low[cr], static_cast<uint32_t>(tid)), low16);
+      if (tid < C) st_remote_u32(map_to_cta(&x.low[cr], static_cast<uint32_t>(tid)), (low16 << 16) | best);
       cluster_arrive_release();
       cluster_wait_acquire();                  // everybody has read x.cnt as well
+      low16 = best;
 #pragma unroll
-      for (int r = 0; r < C; ++r) low16 = max(low16, x.low[r]);
+      for (int r = 0; r < C; ++r) low16 = max(low16, x.low[r] & 0xFFFFu);
+      better = false;
+#pragma unroll
+      for (int r = 0; r < C; ++r) better = better || low16 > (x.low[r] >> 16);
+    } else {
+      low16 = best;
+    }
+    if (!better) {                             // ties: no bound leaves fewer
+      total = kCandCap + 1;
+      break;
     }
     __syncthreads();
   }
@@ -1914,7 +1956,22 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
   if (tid == 0) out[row] = last < 0 ? 0 : last;
 }
 
-template <typename T, int NW>
+// Which maxima bound a row of which a block of `threads` holds `elems` elements. The warps' keys (eight or four
+// each, kth_of_warp_tops) take the least time, but in a short row only a few warps have any, and with fewer than
+// k the bound is 0 and every element a candidate. One word per thread is enough while its maxima are
+// four times k or more (about a quarter more candidates than k then; with as many maxima as k the bound would be the
+// smallest of them), or if a thread has no more than one vector anyway. On the GPU, us: k = 50, 200 bf16 rows of 1000 columns: warps' keys 20.6, four words 10.7, one 8.1; 8
+// rows 17.2, 11.5, 8.5; k = 100, four words / one: 200 rows of 4000 columns, bf16 13.8 / 11.3, fp32 15.4 / 13.3,
+// 64 bf16 rows of 128256 16.8 / 14.3; k = 1000, 64 rows: 28 / 345 (ranked by counting). 64 bf16 rows of 128256
+// columns, k = 50, with the warps' keys: 9.0.
+template <typename T>
+BoundFrom bound_from(int elems, int threads, int k) {
+  const int with_keys = min(threads, elems / Elem<T>::kVec), warps = (with_keys + 31) / 32;
+  if (k <= kFewK && warps * (kWarpTops / (threads / 32)) >= k) return kWarpKeys;
+  return elems / Elem<T>::kVec <= threads || 4 * k <= with_keys * (Elem<T>::kPacked ? 2 : 1) ? kOneWord : kFourWords;
+}
+
+template <typename T>
 int launch_topk(const T* lp, long long row_stride, int rows, int v, const long long* row_ids, float inv_temp, int top_k,
                 float top_p, unsigned long long seed, unsigned long long step, int* out, cudaStream_t stream) {
   // 16-bit rows that 1, 2 or 4 CTAs can keep in registers take the kernel that reads them once, as long as
@@ -1934,10 +1991,17 @@ int launch_topk(const T* lp, long long row_stride, int rows, int v, const long l
       cluster = 0;
     if (cluster > 0) {
       const int smem = static_cast<int>(sizeof(TopkSmem) + sizeof(ClusterXchg));
-      auto* kernel = cluster == 1 ? sample_topk_held_kernel<T, 1, NW>
-                                  : (cluster == 2 ? sample_topk_held_kernel<T, 2, NW> : sample_topk_held_kernel<T, 4, NW>);
-      static PerDevice once[3];
-      if (!smem_opt_in(once[cluster / 2], kernel, smem)) return -10;
+      auto of = [&](auto from) {
+        constexpr int kFrom = decltype(from)::value;
+        return cluster == 1 ? sample_topk_held_kernel<T, 1, kFrom>
+                            : (cluster == 2 ? sample_topk_held_kernel<T, 2, kFrom> : sample_topk_held_kernel<T, 4, kFrom>);
+      };
+      const BoundFrom from = bound_from<T>(v / cluster, kHeldThreads, min(top_k, v));
+      auto* kernel = from == kWarpKeys  ? of(std::integral_constant<int, kWarpKeys>{})
+                     : from == kOneWord ? of(std::integral_constant<int, kOneWord>{})
+                                        : of(std::integral_constant<int, kFourWords>{});
+      static PerDevice once[9];
+      if (!smem_opt_in(once[cluster / 2 * 3 + (from + 1) / 2], kernel, smem)) return -10;
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(static_cast<unsigned>(rows) * cluster);
       cfg.blockDim = dim3(kHeldThreads);
@@ -1956,10 +2020,13 @@ int launch_topk(const T* lp, long long row_stride, int rows, int v, const long l
                  : -11;
     }
   }
-  static PerDevice once;
-  if (!smem_opt_in(once, sample_topk_kernel<T, NW>, static_cast<int>(sizeof(TopkSmem)))) return -10;
-  sample_topk_kernel<T, NW><<<rows, kTopkThreads, sizeof(TopkSmem), stream>>>(lp, row_stride, v, row_ids, inv_temp, top_k,
-                                                                           top_p, seed, step, out);
+  const BoundFrom from = bound_from<T>(v, kTopkThreads, min(top_k, v));
+  auto* kernel = from == kWarpKeys  ? sample_topk_kernel<T, kWarpKeys>
+                 : from == kOneWord ? sample_topk_kernel<T, kOneWord>
+                                    : sample_topk_kernel<T, kFourWords>;
+  static PerDevice once[3];
+  if (!smem_opt_in(once[(from + 1) / 2], kernel, static_cast<int>(sizeof(TopkSmem)))) return -10;
+  kernel<<<rows, kTopkThreads, sizeof(TopkSmem), stream>>>(lp, row_stride, v, row_ids, inv_temp, top_k, top_p, seed, step, out);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -1969,8 +2036,7 @@ int launch_sampling(const void* logits, long long row_stride, int rows, int v, c
                     int* out, cudaStream_t stream) {
   const T* lp = static_cast<const T*>(logits);
   if (top_k >= 1 && top_k <= kMaxTopK) {
-    return top_k <= kFewK ? launch_topk<T, 1>(lp, row_stride, rows, v, row_ids, inv_temp, top_k, top_p, seed, step, out, stream)
-                          : launch_topk<T, 4>(lp, row_stride, rows, v, row_ids, inv_temp, top_k, top_p, seed, step, out, stream);
+    return launch_topk<T>(lp, row_stride, rows, v, row_ids, inv_temp, top_k, top_p, seed, step, out, stream);
   } else {
     constexpr int smem = kGeneralSmemBytes + (Elem<T>::kPacked ? static_cast<int>(sizeof(FastSmem)) : 0);
     static_assert(sizeof(FastSmem) >= kHistBytes, "the older search keeps its histogram there");

@@ -210,7 +210,7 @@ def test_sampler_nan_patterns(cuda_device, dtype, vocab):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("vocab,rows", [(1000, 3), (4088, 3), (4104, 3), (50257, 2), (128256, 2), (200064, 2), (128256, 80)])
-def test_sampler_small_k_candidates_in_few_places(cuda_device, dtype, vocab, rows):
+def test_sampler_candidates_in_few_places(cuda_device, dtype, vocab, rows):
     """Bounds from the warps' keys that are far too low for a part of a row (few finite elements in it, its
     largest in a few warps, none at all) and more candidates than fit: by the hundred and by the thousand."""
     g = torch.Generator(device=cuda_device).manual_seed(vocab)
@@ -225,6 +225,6 @@ def test_sampler_small_k_candidates_in_few_places(cuda_device, dtype, vocab, row
               "two_values": (u < 0.3).float(), "nan": torch.where(few.isinf(), float("nan"), few)}
     for name, val in values.items():
         val = val.to(dtype)
-        for top_k, top_p in ((1, None), (20, 0.9), (50, None), (64, 0.8)):
+        for top_k, top_p in ((1, None), (20, 0.9), (50, None), (64, 0.8), (65, 0.9), (200, None), (257, 0.9), (600, 0.95)):
             tok = sample(val, top_k=top_k, top_p=top_p, temperature=0.7, seed=2, step=top_k)
             assert torch.equal(tok[:3].cpu(), _cpu(val[:3], top_k, top_p, 0.7, 2, top_k)), (name, top_k, top_p)
