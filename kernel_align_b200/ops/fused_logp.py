@@ -364,9 +364,10 @@ def _lmhead_logp_forward(
 
     if cta_group is None:
         # keyed and sized by quantities that are the same on every rank of a group, so that all
-        # ranks tune (a collective sequence of calls when the vocabulary is sharded) or none does
+        # ranks tune (a collective sequence of calls when the vocabulary is sharded) or none does; a call that
+        # also writes its logits loads the epilogue and the memory in another way and is tuned for itself
         rows_total = m * world if sharded else m
-        key = (hidden.device.index, rows_total, k, v_global, world, sharded)
+        key = (hidden.device.index, rows_total, k, v_global, world, sharded, logits is not None)
         sched = _choose_schedule(key, float(rows_total) * k * (v_global / world), hidden.device, launch,
                                  shard_bytes=int(v_global / world) * k * 2)
     else:

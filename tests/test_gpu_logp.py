@@ -149,12 +149,12 @@ def test_fused_logp_backward_matches_autograd(cuda_device):
     assert torch.equal(h2.grad, hq.grad) and torch.equal(w2.grad, wq.grad)
 
 
-@pytest.mark.parametrize("m,k,v,scale", [(1, 64, 64, 1.0), (37, 128, 1920, 0.7), (300, 256, 16448, 1.0), (129, 64, 50304, 1.3)])
-def test_kept_logits_give_the_gradients_of_recomputed_ones(cuda_device, m, k, v, scale, monkeypatch):
-    """Bit for bit, for one sub-slice of the vocabulary and several, ignored ids, a second pass through
-    the graph, and a graph that finds the allowance used up."""
-    from kernel_align_b200.ops import fused_logp
-
+@pytest.mark.parametrize("cta_group,panel_rows", [(None, fused_logp.DEFAULT_PANEL_ROWS), (1, 256), (2, 256)])
+@pytest.mark.parametrize("m,k,v,scale", [(1, 64, 64, 1.0), (37, 128, 1920, 0.7), (300, 256, 16448, 1.0), (129, 64, 50304, 1.3),
+                                         (700, 64, 1920, 1.0)])
+def test_kept_logits_give_the_gradients_of_recomputed_ones(cuda_device, m, k, v, scale, cta_group, panel_rows, monkeypatch):
+    """Bit for bit, for one sub-slice of the vocabulary and several, both tile variants, several panels of
+    rows, ignored ids, a second pass through the graph, and a graph that finds the allowance used up."""
     g = torch.Generator(device=cuda_device).manual_seed(v)
     h = torch.randn(m, k, device=cuda_device, generator=g).to(torch.bfloat16).requires_grad_()
     w = (torch.randn(v, k, device=cuda_device, generator=g) * 0.2).to(torch.bfloat16).requires_grad_()
@@ -164,7 +164,7 @@ def test_kept_logits_give_the_gradients_of_recomputed_ones(cuda_device, m, k, v,
     monkeypatch.setattr(fused_logp, "_KEEP_BYTES", sum(before.values()) + 4 * m * v)
 
     def call():
-        return fused_logp.lmhead_logp(h, w, ids, scale=scale)
+        return fused_logp.lmhead_logp(h, w, ids, scale=scale, cta_group=cta_group, panel_rows=panel_rows)
 
     kept, other = call(), call()          # the second one recomputes
     holders = [x.grad_fn.saved_tensors[2]._ka_kept for x in (kept, other)]
@@ -212,8 +212,6 @@ def test_kept_logits_under_checkpoint(cuda_device, monkeypatch):
     call may find another part of the allowance free than the call itself."""
     from torch.utils.checkpoint import checkpoint
 
-    from kernel_align_b200.ops import fused_logp
-
     g = torch.Generator(device=cuda_device).manual_seed(5)
     m, k, v = 256, 128, 1920
     h = torch.randn(m, k, device=cuda_device, generator=g).to(torch.bfloat16).requires_grad_()
@@ -233,8 +231,6 @@ def test_kept_logits_under_checkpoint(cuda_device, monkeypatch):
 def test_kept_logits_are_gone_after_the_backward_pass(cuda_device):
     """Their share of the allowance as well, whoever holds the result; and with a hook that moves what is
     saved to the host."""
-    from kernel_align_b200.ops import fused_logp
-
     h, w, ids = _inputs(cuda_device, 64, 128, 1920, seed=3)
     h.requires_grad_()
     before = dict(fused_logp._kept_bytes).get(cuda_device.index or 0, 0)
@@ -254,8 +250,6 @@ def test_kept_logits_are_gone_after_the_backward_pass(cuda_device):
 
 def test_kept_logits_need_memory_to_spare(cuda_device, monkeypatch):
     """Neither with the limit at 0 nor while memory is short are logits kept; the gradients are the same."""
-    from kernel_align_b200.ops import fused_logp
-
     h, w, ids = _inputs(cuda_device, 64, 128, 1920, seed=4)
     h.requires_grad_()
     monkeypatch.setattr(fused_logp, "_KEEP_UNASKED_BYTES", 0)
@@ -269,3 +263,16 @@ def test_kept_logits_need_memory_to_spare(cuda_device, monkeypatch):
         assert (logp.grad_fn.saved_tensors[2]._ka_kept is not None) == kept
         grads += torch.autograd.grad(logp.sum(), h)
     assert torch.equal(grads[0], grads[1]) and torch.equal(grads[0], grads[2])
+
+
+def test_schedule_of_a_call_that_keeps_its_logits_is_its_own(cuda_device, monkeypatch):
+    """Scoring and training calls of one shape are tuned apart, in whichever order they come."""
+    monkeypatch.setattr(fused_logp, "_tuned", {})
+    monkeypatch.setattr(fused_logp, "_AUTOTUNE_MIN_MACS", 0.0)
+    monkeypatch.setattr(fused_logp, "_TUNE_MIN_MS", 0.1)
+    h, w, ids = _inputs(cuda_device, 300, 64, 1920, seed=6)
+    want = fused_logp.lmhead_logp(h, w, ids)
+    h.requires_grad_()
+    for _ in range(2):
+        assert torch.equal(fused_logp.lmhead_logp(h, w, ids), want)
+    assert sorted(key[-1] for key in fused_logp._tuned) == [False, True]
