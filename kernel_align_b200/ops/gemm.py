@@ -48,7 +48,6 @@ def check_status(device: torch.device) -> None:
 SKINNY_MAX_ROWS = 64
 
 
-@profiled("gemm_skinny")
 def _check_out(out: torch.Tensor, m: int, n: int, dtype: torch.dtype) -> None:
     if out.shape != (m, n) or out.dtype != dtype or out.stride(1) != 1 or out.stride(0) % 8 != 0 or \
             out.data_ptr() % 16 != 0:
@@ -56,6 +55,7 @@ def _check_out(out: torch.Tensor, m: int, n: int, dtype: torch.dtype) -> None:
                          "multiple of 8 and a 16-byte aligned start")
 
 
+@profiled("gemm_skinny")
 def gemm_skinny(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``a [M <= 64, K] @ w[N, K].T`` on the weight-streaming kernel (bf16 in, bf16 out).
     ``out``: write into this ``[M, N]`` view (rows may be strided, e.g. a column block)."""

@@ -90,3 +90,7 @@ def test_gpu_decoder_layer_has_a_range_for_every_operator(cuda_device):
     assert s["rope"]["calls"] == 2          # forward and backward
     for name in ("rmsnorm", "attention", "attention_backward", "swiglu", "gemm_reduce_scatter"):
         assert name in s, name
+
+
+def test_the_skinny_product_is_profiled_and_the_check_of_its_output_is_not():
+    assert hasattr(gemm.gemm_skinny, "__wrapped__") and not hasattr(gemm._check_out, "__wrapped__")
