@@ -1065,7 +1065,6 @@ struct GeneralSmem {
   int red[kWarps];
   uint32_t max_key;
   // results of a descent
-  uint32_t prefix;
   unsigned long long above_cnt;
   unsigned long long above_mass;
   int sel_bin;
