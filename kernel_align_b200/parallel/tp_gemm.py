@@ -128,8 +128,8 @@ def _tree_pays(m: int, n: int, k: int, num_sms: int) -> bool:
 
     Staged slices spread over all pairs but cost fences, flags and the wait for them. Measured on
     148 SMs, staged / own in us, tiles counted as 256 x 256: 256 tiles: 385 / 156 (K = 4096), 1025 / 738 (28672);
-    32 tiles: 72 / 37 (4096), 109 / 80 (14336), 150 / 143 (28672); 16 tiles: 48 / 18 (4096), 57 / 26 (6144),
-    70 / 40 (14336), 101 / 60 (28672); 4 tiles: 39 / 13 (4096). A slice round of a kept tile takes about 5.4e-3 us
+    32 tiles: 72 / 32 (4096), 109 / 61 (14336), 150 / 101 (28672); 16 tiles: 48 / 20 (4096), 57 / 24 (6144),
+    70 / 37 (14336), 101 / 58 (28672); 4 tiles: 39 / 19 (4096). A slice round of a kept tile takes about 5.4e-3 us
     per K column, staging about 20 us plus 1.2 us per tile; the rule compares the two."""
     if _split_pays(m, n, k):
         return True

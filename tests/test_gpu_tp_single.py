@@ -46,12 +46,13 @@ def test_reduce_scatter_matches_cpu_rank_emulator(cuda_device):
 
 
 @pytest.mark.parametrize("m,n,k,trans_b", [(1, 8, 512, False), (300, 264, 512, False), (1000, 768, 1536, True),
-                                           (2049, 1032, 1024, False), (19000, 256, 512, True)])
+                                           (2049, 1032, 1024, False), (1000, 2056, 512, False), (19000, 256, 512, True)])
 def test_slices_summed_in_the_kernel_equal_the_staged_ones_bitwise(cuda_device, m, n, k, trans_b, monkeypatch):
-    """One rank may sum the eight K slices of a tile where they are computed; the staged path,
-    which the multi-rank kernels share, defines the bits."""
+    """One rank may sum the eight K slices of a tile where they are computed (in narrow tiles and in wide
+    ones); the staged path, which the multi-rank kernels share, defines the bits."""
     from kernel_align_b200.parallel import tp_gemm
 
+    monkeypatch.setattr(tp_gemm, "_split_pays", lambda *a: False)
     ctx = TPContext(device=cuda_device)
     g = torch.Generator(device=cuda_device).manual_seed(m + n)
     x = torch.randn(m, k, device=cuda_device, generator=g).to(torch.bfloat16)
@@ -66,10 +67,10 @@ def test_slices_summed_in_the_kernel_equal_the_staged_ones_bitwise(cuda_device, 
 
 
 @pytest.mark.parametrize("m,n,k,trans_b", [(1, 8, 512, False), (127, 264, 1024, True), (300, 1032, 512, False),
-                                           (1000, 4096, 1536, True), (1100, 4104, 512, False)])
-def test_slices_as_units_of_their_own_equal_the_kept_ones_bitwise(cuda_device, m, n, k, trans_b, monkeypatch):
+                                           (1000, 2056, 512, False), (1000, 4096, 1536, True), (1100, 4104, 512, False)])
+def test_slices_as_units_of_their_own_equal_the_kept_and_the_staged_ones_bitwise(cuda_device, m, n, k, trans_b, monkeypatch):
     """The eight K slices as separate units (one round and several) and a sum over their partials: the bits
-    of a tile that keeps its slices."""
+    of a tile that keeps its slices, and of the staged path, which defines them."""
     from kernel_align_b200.parallel import tp_gemm
 
     ctx = TPContext(device=cuda_device)
@@ -78,9 +79,10 @@ def test_slices_as_units_of_their_own_equal_the_kept_ones_bitwise(cuda_device, m
     w = (torch.randn(*((k, n) if trans_b else (n, k)), device=cuda_device, generator=g) * 0.05).to(torch.bfloat16)
     r = torch.randn(m, n, device=cuda_device, generator=g).to(torch.bfloat16)
     outs = []
-    monkeypatch.setattr(tp_gemm, "_tree_pays", lambda *a: True)
-    for split in (False, True):
+    for own, split in ((False, False), (True, False), (True, True)):
+        monkeypatch.setattr(tp_gemm, "_tree_pays", lambda *a, o=own: o)
         monkeypatch.setattr(tp_gemm, "_split_pays", lambda *a, s=split: s)
         outs += [[gemm_reduce_scatter(x, w, ctx, residual=res, trans_b=trans_b) for res in (None, r)]]
     gemm.check_status(cuda_device)
-    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    for other in outs[1:]:
+        assert torch.equal(outs[0][0], other[0]) and torch.equal(outs[0][1], other[1])
