@@ -394,12 +394,13 @@ _GRAD_PANEL_BYTES = 8 << 30
 # write of 4 bytes per logit under the forward's products and a read: 2000 x 4096 x 128256, forward and
 # backward: 6.9 -> 5.7 ms. It is done while what all live graphs of a device keep stays below
 # _KEEP_BYTES (1.1 % of its memory, two calls of 2000 rows at 128256 columns; KA_LOGP_KEEP_BYTES sets
-# another limit, 0 for none at all) and a sixteenth of the device's memory stays available; otherwise the
+# another limit, 0 for none at all) and a sixteenth of the device's memory stays unallocated; otherwise the
 # logits are recomputed and never materialised.
 _KEEP_BYTES = 2 << 30
-# Asking for the available memory costs 8 us, and 72 more when the allocator's cache is not enough: it is done
-# for logits of at least this size, whose products take the GPU a quarter of a millisecond and more.
-_KEEP_UNASKED_BYTES = 64 << 20
+# Asking the allocator costs the host 20 us, which a call of few products notices (1000 x 1024 x 50304, checkpointed:
+# 890 -> 955 us): it is done for logits of at least this size, or once an allocation has failed.
+_KEEP_UNASKED_BYTES = 256 << 20
+_capacity: dict[int, int] = {}    # of a device on which an allocation failed: what could not be had any more
 _kept_bytes: dict[int, int] = {}
 _kept_lock = threading.Lock()
 _given_back: deque = deque()      # (device, bytes) of shares that are gone and not yet subtracted
@@ -415,19 +416,22 @@ def _keep_limit() -> int:
         raise ValueError("KA_LOGP_KEEP_BYTES must be a number of bytes") from None
 
 
-def _memory_to_spare(device: torch.device, nbytes: int) -> bool:
-    """Whether ``nbytes`` more leave a sixteenth of the device's memory free or in the allocator's cache: kept
-    logits must not be what a step runs out of memory for, and an allocation that fails empties the cache. A
-    capture, which allocates once, is not asked."""
-    if nbytes < _KEEP_UNASKED_BYTES or torch.cuda.is_current_stream_capturing():
-        return True
-    need = nbytes + torch.cuda.get_device_properties(device).total_memory // 16
+def _allocated(index: int) -> int:
     try:
-        stats = torch.cuda.memory_stats_as_nested_dict(device)
-        cached = stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"]
+        return torch.cuda.memory_stats_as_nested_dict(index)["allocated_bytes"]["all"]["current"]
     except (RuntimeError, KeyError):      # an allocator without statistics
-        cached = 0
-    return cached >= need or cached + torch.cuda.mem_get_info(device)[0] >= need
+        return 0
+
+
+def _memory_to_spare(index: int, nbytes: int) -> bool:
+    """Whether ``nbytes`` more leave a sixteenth of the device's memory unallocated: kept logits must not be what a
+    step runs out of memory for. The allocator's figures know nothing of other processes and libraries; what those
+    hold shows in an allocation that fails, which is not tried again (the driver's own figure, cudaMemGetInfo, is no
+    choice: 70 us on an idle host, 1 to 40 ms on a busy one)."""
+    if nbytes < _KEEP_UNASKED_BYTES and index not in _capacity:
+        return True
+    capacity = _capacity.get(index) or torch.cuda.get_device_properties(index).total_memory
+    return _allocated(index) + nbytes <= capacity - capacity // 16
 
 
 def _subtract_given_back() -> None:
@@ -471,12 +475,14 @@ def _kept_logits(hidden, weight, vocab, group) -> Optional[_Kept]:
     if (hidden.device.type != "cuda" or group is not None or v % 64 != 0 or not 0 < m <= 65535
             or (vocab is not None and int(vocab) != v)):
         return None
-    kept = _Kept.take(_native._device_index(hidden.device), 4 * m * v)
-    if kept is None or not _memory_to_spare(hidden.device, 4 * m * v):
+    index, nbytes = _native._device_index(hidden.device), 4 * m * v
+    kept = _Kept.take(index, nbytes)
+    if kept is None or not _memory_to_spare(index, nbytes):
         return None
     try:
         kept.logits = torch.empty(m, v, dtype=torch.float32, device=hidden.device)
     except torch.OutOfMemoryError:
+        _capacity[index] = _allocated(index) + nbytes
         return None
     return kept
 

@@ -249,20 +249,30 @@ def test_kept_logits_are_gone_after_the_backward_pass(cuda_device):
 
 
 def test_kept_logits_need_memory_to_spare(cuda_device, monkeypatch):
-    """Neither with the limit at 0 nor while memory is short are logits kept; the gradients are the same."""
+    """Neither with the limit at 0 nor while memory is short are logits kept, an allocation that failed is not
+    tried again, and the gradients are the same."""
     h, w, ids = _inputs(cuda_device, 64, 128, 1920, seed=4)
     h.requires_grad_()
     monkeypatch.setattr(fused_logp, "_KEEP_UNASKED_BYTES", 0)
-    grads = []
-    for env, free, kept in (("", None, True), ("0", None, False), ("", 0, False)):
+    monkeypatch.setattr(fused_logp, "_capacity", {})
+    grads, tries, empty = [], [], torch.empty
+
+    def full(*args, **kwargs):
+        if args == (64, 1920) and kwargs["dtype"] == torch.float32:
+            tries.append(args)
+            raise torch.OutOfMemoryError("no room")
+        return empty(*args, **kwargs)
+
+    for env, capacity, alloc, kept in (("", {}, empty, True), ("0", {}, empty, False), ("", {0: 1 << 20}, empty, False),
+                                       ("", {}, full, False), ("", None, full, False)):
         monkeypatch.setenv("KA_LOGP_KEEP_BYTES", env)
-        if free is not None:
-            torch.cuda.empty_cache()
-            monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: (free, 0))
+        monkeypatch.setattr(torch, "empty", alloc)
+        if capacity is not None:
+            monkeypatch.setattr(fused_logp, "_capacity", capacity)
         logp = fused_logp.lmhead_logp(h, w, ids)
         assert (logp.grad_fn.saved_tensors[2]._ka_kept is not None) == kept
         grads += torch.autograd.grad(logp.sum(), h)
-    assert torch.equal(grads[0], grads[1]) and torch.equal(grads[0], grads[2])
+    assert len(tries) == 1 and all(torch.equal(g, grads[0]) for g in grads)
 
 
 def test_schedule_of_a_call_that_keeps_its_logits_is_its_own(cuda_device, monkeypatch):
