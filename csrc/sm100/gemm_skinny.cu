@@ -16,10 +16,11 @@
 // accumulator rows that nobody stores. M = 64 matters because those reads share the shared-memory
 // port with the arriving tiles: 39 cycles per MMA at M = 128, N = 16, 23 at M = 64, and N = 4096,
 // K = 14336 took 32.6 us with M = 128, 27.1 us with M = 64.
-// A CTA walks its tiles persistently; the ring of 128-wide K blocks runs on across tiles and the
-// accumulator is double-buffered.
+// A CTA walks its tiles persistently; the ring of K blocks (128 to 512 columns, see launch) runs on across
+// tiles and the accumulator is double-buffered.
 // Measured, 8 rows (64 rows): the four products of a Llama-3-8B decoder layer (436 MB of weights)
-// take 90 us (102 us); with 128 weight rows per CTA everywhere they took 157 us (164 us).
+// take 83 us (98 us), 90 us (102 us) with K blocks of 128 columns throughout; with 128 weight rows per CTA
+// everywhere they took 157 us (164 us).
 //
 // The reference has no GEMM of its own (it names backends in rl_engine/kernels/registry.py:41-55).
 #include <cstdint>
@@ -34,7 +35,6 @@ namespace {
 
 constexpr int kMaxRows = 128;  // largest M of the MMA (rows of shared memory it reads per K step)
 constexpr int kBox = 64;       // K columns of a TMA box: one 128-byte swizzled row
-constexpr int kBoxes = 2;      // boxes per stage
 constexpr int kThreads = 192;  // four epilogue warps, one TMA warp, one MMA warp
 constexpr int kMaxStages = 32;
 constexpr int kRingBytes = 192 * 1024;
@@ -54,6 +54,7 @@ struct SkinnyParams {
   long long ldc;
   int m, n, k;
   int tile_rows, n_tiles, stages;
+  bool joined;          // K is whole boxes: one copy per operand and stage
   int* status;
   unsigned long long timeout_ns;
 };
@@ -64,8 +65,8 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
-// NB: batch rows padded (the MMA's N); MR: weight rows of the MMA (its M)
-template <int NB, int MR>
+// NB: batch rows padded (the MMA's N); MR: weight rows of the MMA (its M); kBoxes: boxes per stage
+template <int NB, int MR, int kBoxes>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                    const __grid_constant__ SkinnyParams p) {
@@ -120,11 +121,18 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
           const uint32_t full = smem_u32(&ctl->full[s]);
           const uint32_t dst = base + s * stage_bytes;
           const int boxes = min(kBoxes, n_boxes - kb * kBoxes);
-          mbar_arrive_expect_tx(full, boxes * box_bytes);
-          for (int x = 0; x < boxes; ++x) {
-            const int k0 = (kb * kBoxes + x) * kBox;
-            tma_load_2d(dst + x * w_bytes, &tm_w, k0, t * p.tile_rows, full);
-            tma_load_2d(dst + kBoxes * w_bytes + x * kXBytes, &tm_x, k0, 0, full);
+          if (p.joined) {
+            // boxes behind the last one are filled with zeros and counted like the others
+            mbar_arrive_expect_tx(full, kBoxes * box_bytes);
+            tma_load_3d(dst, &tm_w, 0, t * p.tile_rows, kb * kBoxes, full);
+            tma_load_3d(dst + kBoxes * w_bytes, &tm_x, 0, 0, kb * kBoxes, full);
+          } else {
+            mbar_arrive_expect_tx(full, boxes * box_bytes);
+            for (int x = 0; x < boxes; ++x) {
+              const int k0 = (kb * kBoxes + x) * kBox;
+              tma_load_2d(dst + x * w_bytes, &tm_w, k0, t * p.tile_rows, full);
+              tma_load_2d(dst + kBoxes * w_bytes + x * kXBytes, &tm_x, k0, 0, full);
+            }
           }
           if (++s == p.stages) {
             s = 0;
@@ -224,23 +232,43 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   }
 }
 
-template <int NB, int MR>
-int launch(const void* a, long long lda, const void* w, long long ldw, SkinnyParams p, int sms, cudaStream_t stream) {
-  if (cudaFuncSetAttribute(gemm_skinny_kernel<NB, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) !=
+template <int NB, int MR, int kBoxes>
+int launch_boxes(const void* a, long long lda, const void* w, long long ldw, SkinnyParams p, int sms, cudaStream_t stream) {
+  if (cudaFuncSetAttribute(gemm_skinny_kernel<NB, MR, kBoxes>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) !=
       cudaSuccess)
     return -10;
   const int stage_bytes = kBoxes * (p.tile_rows + NB) * kBox * 2;
   p.stages = kRingBytes / stage_bytes < kMaxStages ? kRingBytes / stage_bytes : kMaxStages;
   CUtensorMap tw, tx;
-  int rc = make_tmap_2d_16bit_sw128(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, w, static_cast<uint64_t>(p.n),
-                                    static_cast<uint64_t>(p.k), ldw, static_cast<uint32_t>(p.tile_rows), kBox);
+  p.joined = p.k % kBox == 0;
+  auto map = [&](CUtensorMap* t, const void* base, int rows, long long ld, int box_rows) {
+    return p.joined ? make_tmap_3d_16bit_sw128(t, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, static_cast<uint64_t>(rows),
+                                               static_cast<uint64_t>(p.k), ld, static_cast<uint32_t>(box_rows), kBoxes)
+                    : make_tmap_2d_16bit_sw128(t, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, static_cast<uint64_t>(rows),
+                                               static_cast<uint64_t>(p.k), ld, static_cast<uint32_t>(box_rows), kBox);
+  };
+  int rc = map(&tw, w, p.n, ldw, p.tile_rows);
   if (rc) return -20 + rc;
-  rc = make_tmap_2d_16bit_sw128(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a, static_cast<uint64_t>(p.m),
-                                static_cast<uint64_t>(p.k), lda, NB, kBox);
+  rc = map(&tx, a, p.m, lda, NB);
   if (rc) return -40 + rc;
   const unsigned grid = static_cast<unsigned>(p.n_tiles < sms ? p.n_tiles : sms);
-  gemm_skinny_kernel<NB, MR><<<grid, kThreads, kSmemBytes, stream>>>(tw, tx, p);
+  gemm_skinny_kernel<NB, MR, kBoxes><<<grid, kThreads, kSmemBytes, stream>>>(tw, tx, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
+// Boxes per stage: the most that leave four stages in the ring and that K fills. A stage costs the MMA warp about
+// 220 cycles on top of its MMAs (27 cycles each for 16 batch rows: 8 rows x 1184 columns, K = 4096, where only the
+// chain of MMAs counts, takes 10.6 us with two boxes, 8.9 with four, 8.2 with eight), but with fewer than four
+// stages the loads no longer keep ahead. us, boxes 2 / 4 / 8: 8 rows, 4096 columns, K = 14336 28.1 / 23.5 / 22.9, K = 4096
+// 10.8 / 9.8 / 9.4; 6144 columns 12.3 / 11.6 / 11.7; 28672 columns 39.9 / 39.5 / 51.9 (six, three and one stage);
+// 64 rows, 4096 columns, K = 14336 32.4 / 29.5 / 36.7; 6144 columns 14.2 / 14.5 / 20.8.
+template <int NB, int MR>
+int launch(const void* a, long long lda, const void* w, long long ldw, SkinnyParams p, int sms, cudaStream_t stream) {
+  const int bytes = (p.tile_rows + NB) * kBox * 2;
+  auto fits = [&](int boxes) { return 4 * boxes * bytes <= kRingBytes && boxes * kBox <= p.k; };
+  if (fits(8)) return launch_boxes<NB, MR, 8>(a, lda, w, ldw, p, sms, stream);
+  if (fits(4)) return launch_boxes<NB, MR, 4>(a, lda, w, ldw, p, sms, stream);
+  return launch_boxes<NB, MR, 2>(a, lda, w, ldw, p, sms, stream);
 }
 
 }  // namespace

@@ -77,6 +77,21 @@ def test_skinny_gemm_equals_tiled_kernel_bitwise(cuda_device, m, n, k, monkeypat
     assert torch.equal(gemm.gemm_bi(a[:m], w), tiled[:m])
 
 
+@pytest.mark.parametrize("m", [3, 30, 64])
+@pytest.mark.parametrize("n,k", [(40, 64), (4104, 320), (6144, 576), (19000, 448), (1184, 4160), (40, 72)])
+def test_skinny_gemm_boxes_behind_the_last_one(cuda_device, m, n, k):
+    """K that is no multiple of a stage, in operands whose rows go on behind K: what lies there (NaN) is not
+    multiplied, also where one copy brings several boxes."""
+    g = torch.Generator(device=cuda_device).manual_seed(k)
+    a = torch.full((80, k + 640), float("nan"), device=cuda_device, dtype=torch.bfloat16)
+    w = torch.full((n + 130, k + 640), float("nan"), device=cuda_device, dtype=torch.bfloat16)
+    a[:, :k] = torch.randn(80, k, device=cuda_device, generator=g).to(torch.bfloat16)
+    w[:n, :k] = (torch.randn(n, k, device=cuda_device, generator=g) * 0.05).to(torch.bfloat16)
+    got = gemm.gemm_skinny(a[:m, :k], w[:n, :k])
+    gemm.check_status(cuda_device)
+    assert torch.equal(got, gemm.gemm_bi(a[:, :k].contiguous(), w[:n, :k].contiguous())[:m])
+
+
 @pytest.mark.parametrize("n,k", [(8, 64), (136, 200), (1032, 512), (4096, 1024)])
 @pytest.mark.parametrize("trans_a,trans_b,dtype", [(False, False, torch.bfloat16), (False, True, torch.bfloat16),
                                                    (True, True, torch.float32)])
