@@ -13,13 +13,15 @@
 // the batch size, the launch shape or the schedule, and the C++ CPU path reproduces it bit
 // for bit.
 //
-// Three kernels:
+// Four kernels:
 //   sample_topk_kernel     top_k in [1, 1024] (greedy = top_k 1), optional top_p
 //   sample_topk_held_kernel  the same for 16-bit rows that 1, 2 or 4 CTAs hold in registers
 //                          (a cluster; candidates exchanged through distributed shared memory)
 //   sample_general_kernel  no top_k (or k > 1024), optional top_p: 16-bit rows by one histogram of
 //                          counts per key (sample_row16), fp32 rows and the few 16-bit rows that
 //                          does not take by radix descent on (count, mass) histograms
+//   sample_parts_kernel    the same for bf16 rows with a filter where part_ctas says so: a histogram for every
+//                          part of the row, one to eight CTAs per row
 #include <cstdint>
 #include <cstdlib>
 #include <type_traits>
@@ -1077,7 +1079,7 @@ constexpr int kGeneralSmemBytes = (static_cast<int>(sizeof(GeneralSmem)) + 15) /
 // that crosses `limit` lies among the keys equal to tau. `by_mass` selects the criterion:
 //   by count: first key where count_above + count(key) >  limit  (limit = k - 1)
 //   by mass : first key where mass_above  + mass(key)  >  limit
-template <typename T>
+template <typename T, int kT>
 __device__ void descend(const T* rp, int v, float inv_temp, float y_max, bool by_mass,
                         unsigned long long limit, GeneralSmem& s, uint32_t& tau, unsigned long long& above_cnt,
                         unsigned long long& above_mass) {
@@ -1090,7 +1092,7 @@ __device__ void descend(const T* rp, int v, float inv_temp, float y_max, bool by
   for (int round = 0; round < 3; ++round) {
     const int w = widths[round];
     const int shift = 32 - known_bits - w;
-    for (int b = tid; b < kBins; b += kThreads) {
+    for (int b = tid; b < kBins; b += kT) {
       s.cnt[b] = 0;
       s.mass[b] = 0;
     }
@@ -1510,10 +1512,10 @@ __device__ __forceinline__ void sum_range(const T* rp, int begin, int end, const
 }
 
 // First element, in token-id order, whose cumulative kept mass exceeds the target: the row is cut into
-// 32 contiguous segments, one per warp, whose kept masses are order-free integer sums (coalesced loads),
-// the segment that holds the target is cut into 32 again, and only the last hundred elements are walked
+// as many contiguous segments as there are warps (kW), whose kept masses are order-free integer sums (coalesced loads),
+// the segment that holds the target is cut again, and only the last hundred elements are walked
 // in order. With kAll the kept mass is what the first level adds up; false if it is 0.
-template <typename T, int kMode>
+template <typename T, int kMode, int kW = kWarps>
 __device__ bool draw(const T* rp, int v, const Kept& k, unsigned long long kept_mass, uint32_t u24, DrawSmem& d, int* out) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int begin = 0, end = v;
@@ -1524,7 +1526,7 @@ __device__ bool draw(const T* rp, int v, const Kept& k, unsigned long long kept_
   }
 #pragma unroll 1
   for (int level = 0; level < 2; ++level) {
-    const int len = ((end - begin + kWarps - 1) / kWarps + 7) / 8 * 8;
+    const int len = ((end - begin + kW - 1) / kW + 7) / 8 * 8;
     const int b = min(end, begin + warp * len), e = min(end, b + len);
     unsigned long long mass, ties;
     sum_range<T, kMode>(rp, b, e, k, mass, ties);
@@ -1534,10 +1536,10 @@ __device__ bool draw(const T* rp, int v, const Kept& k, unsigned long long kept_
     }
     __syncthreads();
     if (warp == 0) {
-      const unsigned long long t = d.seg_ties[lane];
+      const unsigned long long t = lane < kW ? d.seg_ties[lane] : 0ull;
       const unsigned long long t0 = d.ties_before + warp_incl_u64(t) - t;
       const unsigned long long left = k.tie_keep > t0 ? k.tie_keep - t0 : 0ull;
-      const unsigned long long m = d.seg_mass[lane] + (t < left ? t : left) * k.q_tau;
+      const unsigned long long m = (lane < kW ? d.seg_mass[lane] : 0ull) + (t < left ? t : left) * k.q_tau;
       const unsigned long long inc = warp_incl_u64(m);
       unsigned long long target = d.target;
       if (kMode == kAll && level == 0) target = mass_scale_u24(u24, __shfl_sync(0xffffffffu, inc, 31));
@@ -1775,10 +1777,10 @@ __device__ bool sample_row16(const T* rp, int v, float inv_temp, int top_k, floa
 }
 
 // The last kept element of a row in which nothing has a mass (-1: none is kept).
-template <typename T>
+template <typename T, int kT>
 __device__ int last_kept(const T* rp, int v, uint32_t tau, unsigned long long tie_keep, GeneralSmem& s) {
   const int tid = threadIdx.x;
-  const int chunk = (v + kThreads - 1) / kThreads;
+  const int chunk = (v + kT - 1) / kT;
   const int begin = min(v, tid * chunk), end = min(v, begin + chunk);
   unsigned long long ties = 0, total;
   for (int i = begin; i < end; ++i) ties += float_to_key(Elem<T>::to_float(rp[i])) == tau ? 1u : 0u;
@@ -1799,17 +1801,17 @@ __device__ int last_kept(const T* rp, int v, uint32_t tau, unsigned long long ti
 }
 
 // Largest key of the row, for the whole block.
-template <typename T>
+template <typename T, int kT>
 __device__ uint32_t row_max_key(const T* rp, int v, GeneralSmem& s) {
   constexpr int kVec = Elem<T>::kVec, kU = 8;
   const int tid = threadIdx.x;
   const int head = row_head(rp, v), nvec = (v - head) / kVec, scal = v - nvec * kVec;
   const uint4* vp = reinterpret_cast<const uint4*>(rp + head);
   uint32_t w[1] = {~0u};                      // NaN: key 0
-  for (int j = tid; j < nvec; j += kThreads * kU) {
+  for (int j = tid; j < nvec; j += kT * kU) {
     uint4 raw[kU];
 #pragma unroll
-    for (int u = 0; u < kU; ++u) raw[u] = j + kThreads * u < nvec ? __ldg(vp + j + kThreads * u) : make_uint4(~0u, ~0u, ~0u, ~0u);
+    for (int u = 0; u < kU; ++u) raw[u] = j + kT * u < nvec ? __ldg(vp + j + kT * u) : make_uint4(~0u, ~0u, ~0u, ~0u);
 #pragma unroll
     for (int u = 0; u < kU; ++u) w[0] = Elem<T>::wmax(w[0], vec_max<T>(raw[u]));
   }
@@ -1830,35 +1832,19 @@ __device__ uint32_t row_max_key(const T* rp, int v, GeneralSmem& s) {
   return s.max_key;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 1)
-sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v, const long long* __restrict__ row_ids,
-                      float inv_temp, int top_k, float top_p, unsigned long long seed, unsigned long long step,
-                      int* __restrict__ out) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ DrawSmem d;
-  GeneralSmem& s = *reinterpret_cast<GeneralSmem*>(smem_raw);
-  constexpr bool kKey16 = std::is_same<T, __nv_bfloat16>::value;
-  unsigned int* hist = reinterpret_cast<unsigned int*>(smem_raw + kGeneralSmemBytes);  // kKey16 only
+// One row by radix descent, any type; kHist: with descend16's histogram (kThreads threads, bf16).
+template <typename T, int kT, bool kHist>
+__device__ void general_row(const T* rp, int v, float inv_temp, int top_k, float top_p, uint32_t u24, GeneralSmem& s,
+                            unsigned int* hist, DrawSmem& d, int* out) {
   const int tid = threadIdx.x;
-  const int row = blockIdx.x;
-  const T* rp = logits + static_cast<long long>(row) * row_stride;
-  const unsigned long long rid = row_ids ? static_cast<unsigned long long>(row_ids[row])
-                                         : static_cast<unsigned long long>(row);
-  const uint32_t u24 = uniform_u24(seed, rid, step);
   const bool has_k = top_k > 0 && top_k < v;
-  if constexpr (Elem<T>::kPacked) {
-    FastSmem& f = *reinterpret_cast<FastSmem*>(smem_raw + kGeneralSmemBytes);
-    if ((has_k || top_p < 1.0f) && sample_row16<T>(rp, v, inv_temp, top_k, top_p, u24, s, f, d, out + row)) return;
-    __syncthreads();
-  }
-  const float y_max = mul_rn(key_to_float(row_max_key(rp, v, s)), inv_temp);
+  const float y_max = mul_rn(key_to_float(row_max_key<T, kT>(rp, v, s)), inv_temp);
   Kept k;
   k.args = {inv_temp, -y_max};
   k.q_tau = 0;
   if (!has_k && top_p >= 1.0f) {              // everything is kept: the sums of the draw are the only pass
     k.tie_keep = 0;
-    if (!draw<T, kAll>(rp, v, k, 0, u24, d, out + row) && tid == 0) out[row] = v - 1;
+    if (!draw<T, kAll, kT / 32>(rp, v, k, 0, u24, d, out) && tid == 0) *out = v - 1;
     return;
   }
 
@@ -1873,12 +1859,12 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
     unsigned long long k_ties = ~0ull;
     unsigned long long zk;
     if (has_k) {
-      if constexpr (kKey16) {
+      if constexpr (kHist) {
         unsigned long long unused;
         descend16<T>(rp, v, inv_temp, y_max, false, static_cast<unsigned long long>(top_k - 1), s, hist, k_tau,
                      k_above_cnt, k_above_mass, unused);
       } else {
-        descend<T>(rp, v, inv_temp, y_max, false, static_cast<unsigned long long>(top_k - 1), s, k_tau, k_above_cnt,
+        descend<T, kT>(rp, v, inv_temp, y_max, false, static_cast<unsigned long long>(top_k - 1), s, k_tau, k_above_cnt,
                    k_above_mass);
       }
       k_ties = static_cast<unsigned long long>(top_k) - k_above_cnt;
@@ -1886,7 +1872,7 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
       zk = k_above_mass + k_ties * mass_fixed(exp_det(sub_rn(y, y_max)));
     } else {
       // everything is kept by the count criterion: Z = total mass
-      const int len = ((v + kWarps - 1) / kWarps + 7) / 8 * 8;
+      const int len = ((v + kT / 32 - 1) / (kT / 32) + 7) / 8 * 8;
       const int b = min(v, (tid >> 5) * len);
       unsigned long long part, unused, total;
       sum_range<T, kAll>(rp, b, min(v, b + len), k, part, unused);
@@ -1900,10 +1886,10 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
       const unsigned long long limit = mass_fraction(static_cast<double>(top_p), zk);
       uint32_t p_tau;
       unsigned long long p_above_cnt, p_above_mass, p_present = 0;
-      if constexpr (kKey16) {
+      if constexpr (kHist) {
         descend16<T>(rp, v, inv_temp, y_max, true, limit, s, hist, p_tau, p_above_cnt, p_above_mass, p_present);
       } else {
-        descend<T>(rp, v, inv_temp, y_max, true, limit, s, p_tau, p_above_cnt, p_above_mass);
+        descend<T, kT>(rp, v, inv_temp, y_max, true, limit, s, p_tau, p_above_cnt, p_above_mass);
       }
       // element i (in sorted order) is kept while the mass before it is <= limit
       const float y = mul_rn(key_to_float(p_tau), inv_temp);
@@ -1930,7 +1916,7 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
         tie_keep = p_ties;
         // the kept mass follows from the number of ties actually present
         unsigned long long present;
-        if constexpr (kKey16) {
+        if constexpr (kHist) {
           present = p_present;  // the histogram had the count
         } else {
           int local = 0;
@@ -1948,11 +1934,818 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
   k.tau = tau;
   k.tie_keep = tie_keep;
   k.q_tau = mass_fixed(exp_det(sub_rn(mul_rn(key_to_float(tau), inv_temp), y_max)));
-  if (draw<T, kByExp>(rp, v, k, kept_mass, u24, d, out + row)) return;
+  if (draw<T, kByExp, kT / 32>(rp, v, k, kept_mass, u24, d, out)) return;
   // target == kept_mass can only happen when kept_mass is 0 (all masses underflowed):
   // fall back to the last kept element
-  const int last = last_kept<T>(rp, v, tau, tie_keep, s);
-  if (tid == 0) out[row] = last < 0 ? 0 : last;
+  const int last = last_kept<T, kT>(rp, v, tau, tie_keep, s);
+  if (tid == 0) *out = last < 0 ? 0 : last;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 1)
+sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v, const long long* __restrict__ row_ids,
+                      float inv_temp, int top_k, float top_p, unsigned long long seed, unsigned long long step,
+                      int* __restrict__ out) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ DrawSmem d;
+  GeneralSmem& s = *reinterpret_cast<GeneralSmem*>(smem_raw);
+  unsigned int* hist = reinterpret_cast<unsigned int*>(smem_raw + kGeneralSmemBytes);  // bf16 only
+  const int row = blockIdx.x;
+  const T* rp = logits + static_cast<long long>(row) * row_stride;
+  const unsigned long long rid = row_ids ? static_cast<unsigned long long>(row_ids[row])
+                                         : static_cast<unsigned long long>(row);
+  const uint32_t u24 = uniform_u24(seed, rid, step);
+  if constexpr (Elem<T>::kPacked) {
+    FastSmem& f = *reinterpret_cast<FastSmem*>(smem_raw + kGeneralSmemBytes);
+    const bool has_k = top_k > 0 && top_k < v;
+    if ((has_k || top_p < 1.0f) && sample_row16<T>(rp, v, inv_temp, top_k, top_p, u24, s, f, d, out + row)) return;
+    __syncthreads();
+  }
+  general_row<T, kThreads, std::is_same<T, __nv_bfloat16>::value>(rp, v, inv_temp, top_k, top_p, u24, s, hist, d, out + row);
+}
+
+// ---- bf16 rows: histograms per part of the row -------------------------------------------------
+// What bounds the general path is one shared-memory atomic per element: a histogram of 148 rows of
+// 128256 columns, one row per SM, takes 12.5 us whatever the counters' width (5.9 cycles per warp, the
+// conflicts of 32 random banks), and nothing else has to be done per element:
+//   * A row is cut into C * 2 contiguous sub-parts, C CTAs (a cluster) with a histogram for each of their
+//     two. The kept mass of a sub-part follows from its histogram, so only the one that holds the target is
+//     read again by the draw (a sixteenth to a half of the row; the draw over whole rows took as long as the counting).
+//   * C is chosen by part_ctas: few rows fill the GPU, and 200 rows are 400 CTAs, at most three half rows per SM, where one CTA
+//     of 1024 threads per row and SM takes two rounds.
+//   * For three CTAs per SM the two histograms must fit 64 KiB: 16-bit counters (a sub-part has at most 65535 elements) of the
+//     values whose magnitude lies in 64 binades, [2^-54, 2^10). What lies outside is sorted out element by
+//     element: zeros have counters of their own, NaN has no mass, and what is low enough to have no mass
+//     (-inf, the type's lowest value, -1e4) need not be counted. A look at the row's first elements shifts the 64 binades for
+//     rows of large values; if something with a mass is left out all the same, the row is counted again with the binades
+//     that its maximum asks for, and if that leaves out a nonzero value with a mass, one CTA takes the radix descent.
+// [200, 128256] ~ N(0, 2), T = 1, top_p = 0.9: 58.4 us with one CTA per row, 46.7 us now: counting takes 31k to 50k cycles of an
+// SM with three half rows, what follows 29k, which is latency (searches 10k, barriers 6k, the draw 12k).
+constexpr int kPartThreads = 512, kPartWarps = kPartThreads / 32;
+constexpr int kPartsPerCta = 2;
+constexpr int kMaxPartCtas = 8;
+constexpr int kPartBinades = 64;
+constexpr int kPartMags = kPartBinades * 128;                        // magnitudes counted per sign
+constexpr int kPartBase = (127 + 10 - kPartBinades) * 128;           // bits of the smallest of them: 2^-54
+constexpr int kPartHistBytes = kPartMags * 2 * 2;
+constexpr int kPartGroups = 2 * kPartMags / 32 + 1;                  // descending: positive values, zeros, negative values
+constexpr int kPartZeroGroup = kPartMags / 32;
+constexpr int kPartMaxElems = 65535;                                 // of a sub-part: what a counter holds
+constexpr int kNothing = 0x7FFFFFFF;                                 // below every counted value
+
+constexpr int kPartMaxBlocks = kPartMaxElems / 256 + 3;              // of 256 elements, and the scalars at both ends
+
+constexpr int kPartUnits = 2 * kPartMags / 128;                      // of 128 neighbouring counters
+
+struct PartInfo {
+  uint32_t max_key;             // 16-bit key of the largest element, 0 if there is no number
+  uint32_t flags;
+  uint32_t units[kPartUnits / 32];   // which units of counters are not empty
+};
+constexpr int kInfoWords = static_cast<int>(sizeof(PartInfo) / 4);
+enum PartFlags : uint32_t { kBig = 1, kLow = 2, kTiny = 4 };         // values outside the counted magnitudes
+
+struct PartSmem {
+  unsigned long long mass[kPartGroups];
+  unsigned int cnt[kPartGroups];
+  unsigned int zeros[kPartsPerCta][2];                               // +0, -0
+  PartInfo mine;
+  PartInfo info[kMaxPartCtas];
+  unsigned long long scan[kPartWarps];
+  unsigned long long sub_mass[kMaxPartCtas * kPartsPerCta], sub_ties[kMaxPartCtas * kPartsPerCta];
+  unsigned long long acc[kPartsPerCta];
+  // result of a search
+  unsigned long long above_cnt, above_mass, present;
+  int group, sel;
+  int owner, n_units;
+  unsigned char units[kPartUnits];   // those of the row that are not empty
+  uint32_t u24;
+  uint32_t look[kPartWarps];
+  unsigned long long target, ties_before;      // of the draw inside the owner's sub-part
+  unsigned long long blocks[kPartMaxBlocks];   // ties << kTieShift | mass
+};
+constexpr int kPartSmemBytes = kPartsPerCta * kPartHistBytes + static_cast<int>(sizeof(PartSmem));
+static_assert(kPartGroups <= 2 * kPartThreads, "a thread sums two groups");
+static_assert(kGeneralSmemBytes <= kPartsPerCta * kPartHistBytes, "the radix descent works where the histograms were");
+
+// Counted values in descending order: d = 0 .. kPartMags - 1 are the positive ones, then +0 and -0, then the negative ones.
+__device__ __forceinline__ uint32_t part_bits(int d, uint32_t base) {
+  if (d < kPartMags) return base + static_cast<uint32_t>(kPartMags - 1 - d);
+  return d < kPartMags + 2 ? (d == kPartMags ? 0u : 0x8000u) : 0x8000u + base + static_cast<uint32_t>(d - kPartMags - 2);
+}
+__device__ __forceinline__ uint32_t part_offset(int d) {             // of its counter; not for zeros
+  return d < kPartMags ? static_cast<uint32_t>(kPartMags - 1 - d) * 2 : static_cast<uint32_t>(d - 2) * 2;
+}
+__device__ __forceinline__ int part_rank(uint32_t bits, uint32_t base) {   // d of the largest value
+  const uint32_t mag = bits & 0x7FFFu;
+  if (mag == 0) return kPartMags;            // the first of the zeros
+  return bits & 0x8000u ? kPartMags + 2 + static_cast<int>(mag - base) : kPartMags - 1 - static_cast<int>(mag - base);
+}
+__device__ __forceinline__ float bits16_float(uint32_t bits) { return __uint_as_float(bits << 16); }
+__device__ __forceinline__ unsigned long long bits16_mass(uint32_t bits, float inv_temp, float y_max) {
+  return mass_fixed(exp_det(sub_rn(mul_rn(bits16_float(bits), inv_temp), y_max)));
+}
+__device__ __forceinline__ uint32_t ld_remote_u16(uint32_t a) {
+  unsigned short v;
+  asm volatile("ld.shared::cluster.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_remote_u32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 ld_remote_u32x2(uint32_t a) {
+  uint2 v;
+  asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t map_addr(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+
+// Sub-part q of n_sub in token order: scalars in front of the row's first 16-byte boundary (q = 0), whole vectors,
+// scalars behind the last one (the last sub-part).
+struct PartRange {
+  int n_head;                   // scalars, from the row's start
+  int first, n_vec;             // first element of the vectors, vectors
+  int tail, n_tail;
+};
+__device__ __forceinline__ PartRange part_range(int q, int n_sub, int head, int v) {
+  const int nvec = (v - head) / 8, per = (nvec + n_sub - 1) / n_sub;
+  const int v0 = min(nvec, q * per), v1 = q == n_sub - 1 ? nvec : min(nvec, (q + 1) * per);
+  PartRange r;
+  r.n_head = q == 0 ? head : 0;
+  r.first = head + 8 * v0;
+  r.n_vec = v1 - v0;
+  r.tail = head + 8 * nvec;
+  r.n_tail = q == n_sub - 1 ? v - r.tail : 0;
+  return r;
+}
+
+// The largest magnitude that can have a mass if the largest value is x, and the 64 binades up to it.
+__device__ __forceinline__ float part_reach(float x, float inv_temp) {
+  return fminf(fmaxf(fabsf(x), fabsf(x - 24.f / inv_temp)), 3.0e38f);
+}
+__device__ __forceinline__ uint32_t part_base(float reach) {
+  const uint32_t top = min(((__float_as_uint(reach) >> 23) + 1u) << 7, 0x7F80u);
+  return top > kPartMags ? top - kPartMags : 1u;
+}
+
+// Histogram of this CTA's sub-parts (zeroed before), its largest element, which values were not counted.
+__device__ __forceinline__ void part_count(const __nv_bfloat16* rp, int v, uint32_t base, int rank, int ctas, unsigned char* hist,
+                                           PartSmem& s) {
+  using T = __nv_bfloat16;
+  constexpr int kTs = kPartThreads / kPartsPerCta, kU = 4;
+  const int tid = threadIdx.x, sub = tid / kTs, t = tid % kTs;
+  const PartRange pr = part_range(rank * kPartsPerCta + sub, ctas * kPartsPerCta, row_head(rp, v), v);
+  const int n_vec = pr.n_vec;
+  unsigned char* mine = hist + sub * kPartHistBytes;
+  uint32_t top = 0xFFFFFFFFu, flags = 0;
+  unsigned int zeros = 0, neg_zeros = 0;
+  auto count = [&](uint32_t a) {       // a: bits - base in the low half; a counter of 16 bits is half a word
+    const uint32_t off = ((a << 1) & 0x3FFCu) | ((a >> 1) & 0x4000u);
+    atomicAdd(reinterpret_cast<unsigned int*>(mine + off), max((a << 16) & 0x10000u, 1u));
+  };
+  // h: 16 bits. What is not counted: zeros, tiny values, large ones and NaN
+  auto count_or_note = [&](uint32_t h) {
+    const uint32_t mag = h & 0x7FFFu, above = mag - (base + kPartMags);
+    zeros += h == 0u ? 1u : 0u;
+    neg_zeros += h == 0x8000u ? 1u : 0u;
+    flags |= mag - 1u < base - 1u ? kTiny : 0u;
+    flags |= above <= 0x7F80u - (base + kPartMags) ? (h >> 15) + kBig : 0u;
+    if (((h - base) & 0x6000u) == 0) count(h - base);
+  };
+  const uint4* vp = reinterpret_cast<const uint4*>(rp + pr.first);
+  for (int j = t; j < n_vec; j += kTs * kU) {
+    uint4 raw[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      if (j + kTs * u < n_vec) raw[u] = __ldg(vp + j + kTs * u);
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (j + kTs * u >= n_vec) break;
+      const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
+      uint32_t a[8], out = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a[2 * i] = w[i] - base;
+        a[2 * i + 1] = (w[i] >> 16) - base;
+        out |= (a[2 * i] | a[2 * i + 1]) & 0x6000u;
+      }
+      top = Elem<T>::wmax(top, vec_max<T>(raw[u]));
+      if (__any_sync(__activemask(), out != 0) == 0) {     // one path for the warp: lanes apart would take both
+#pragma unroll
+        for (int i = 0; i < 8; ++i) count(a[i]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          count_or_note(w[i] & 0xFFFFu);
+          count_or_note(w[i] >> 16);
+        }
+      }
+    }
+  }
+  // scalars in front of the first vector and behind the last one (fewer than eight each)
+  const unsigned short* hp = reinterpret_cast<const unsigned short*>(rp);
+  if (t < pr.n_head + pr.n_tail) {
+    const uint32_t h = hp[t < pr.n_head ? t : pr.tail + (t - pr.n_head)];
+    count_or_note(h);
+    top = Elem<T>::wmax(top, h | 0xFFFF0000u);
+  }
+  top = key16x2<T>(top);
+  top = __reduce_max_sync(0xffffffffu, max(top >> 16, top & 0xFFFFu));
+  flags = __reduce_or_sync(0xffffffffu, flags);
+  zeros = __reduce_add_sync(0xffffffffu, zeros);
+  neg_zeros = __reduce_add_sync(0xffffffffu, neg_zeros);
+  if ((tid & 31) == 0) {
+    atomicMax(&s.mine.max_key, top);
+    if (flags) atomicOr(&s.mine.flags, flags);
+    if (zeros) atomicAdd(&s.zeros[sub][0], zeros);
+    if (neg_zeros) atomicAdd(&s.zeros[sub][1], neg_zeros);
+  }
+  __syncthreads();
+  // which units of 128 counters are not empty
+  const int lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int i = 0; i < kPartUnits / kPartWarps; ++i) {
+    const int u = warp + i * kPartWarps;
+    const uint2 c0 = *reinterpret_cast<const uint2*>(hist + u * 256 + lane * 8);
+    const uint2 c1 = *reinterpret_cast<const uint2*>(hist + kPartHistBytes + u * 256 + lane * 8);
+    if (__any_sync(0xffffffffu, (c0.x | c0.y | c1.x | c1.y) != 0) && lane == 0)
+      atomicOr(&s.mine.units[u >> 5], 1u << (u & 31));
+  }
+}
+static_assert(kPartsPerCta == 2, "both histograms of a CTA");
+
+// Zeros of one sign in the whole row.
+__device__ __forceinline__ unsigned int part_zeros(int sign, int ctas, const PartSmem& s) {
+  unsigned int n = 0;
+#pragma unroll
+  for (int r = 0; r < kMaxPartCtas; ++r)
+    if (r < ctas)
+#pragma unroll
+      for (int sub = 0; sub < kPartsPerCta; ++sub) n += ld_remote_u32(map_to_cta(&s.zeros[sub][sign], r));
+  return n;
+}
+
+__device__ __forceinline__ void part_barrier(int ctas) {
+  if (ctas == 1) {
+    __syncthreads();
+  } else {
+    cluster_arrive_release();
+    cluster_wait_acquire();
+  }
+}
+
+// The counted value that crosses `limit`, by count or by mass, from the prefix sums of this thread's two groups (what
+// lies above them); s.sel = kNothing if none does. above_cnt is only valid if counts were summed.
+__device__ void part_search(bool by_mass, unsigned long long limit, float inv_temp, float y_max, uint32_t base, int ctas,
+                            unsigned long long pre_c, unsigned long long pre_m, uint32_t hist, PartSmem& s) {
+  const int tid = threadIdx.x, lane = tid & 31, g0 = 2 * tid, g1 = g0 + 1;
+  if (tid == 0) s.group = -1;
+  __syncthreads();
+  const unsigned long long c0 = g0 < kPartGroups ? s.cnt[g0] : 0, c1 = g1 < kPartGroups ? s.cnt[g1] : 0;
+  const unsigned long long m0 = g0 < kPartGroups ? s.mass[g0] : 0, m1 = g1 < kPartGroups ? s.mass[g1] : 0;
+  const unsigned long long pre = by_mass ? pre_m : pre_c, mid = pre + (by_mass ? m0 : c0), end = mid + (by_mass ? m1 : c1);
+  if (pre <= limit && end > limit) {
+    const bool second = mid <= limit;
+    s.group = second ? g1 : g0;
+    s.above_cnt = second ? pre_c + c0 : pre_c;
+    s.above_mass = second ? pre_m + m0 : pre_m;
+  }
+  __syncthreads();
+  const int g = s.group;
+  if (g < 0) {
+    if (tid == 0) s.sel = kNothing;
+  } else if (tid < 32) {
+    const bool zero = g == kPartZeroGroup;
+    const int d = (g <= kPartZeroGroup ? 32 * g : 32 * g - 30) + lane;
+    unsigned int n = 0;
+    if (zero) {
+      if (lane < 2) n = part_zeros(lane, ctas, s);
+    } else {
+      const uint32_t a = hist + part_offset(d);
+#pragma unroll
+      for (int r = 0; r < kMaxPartCtas; ++r)
+        if (r < ctas)
+#pragma unroll
+          for (int sub = 0; sub < kPartsPerCta; ++sub) n += ld_remote_u16(map_addr(a + sub * kPartHistBytes, r));
+    }
+    const unsigned long long kc = n, km = n ? n * bits16_mass(part_bits(d, base), inv_temp, y_max) : 0ull;
+    const unsigned long long ic = warp_incl_u64(kc), im = warp_incl_u64(km);
+    const unsigned long long above_c = s.above_cnt, above_m = s.above_mass;
+    const bool crosses = by_mass ? above_m + im > limit : above_c + ic > limit;
+    const int first = __ffs(static_cast<int>(__ballot_sync(0xffffffffu, crosses))) - 1;
+    if (lane == first) {
+      s.sel = d;
+      s.above_cnt = above_c + ic - kc;
+      s.above_mass = above_m + im - km;
+      s.present = kc;
+    }
+  }
+  __syncthreads();
+}
+
+// First element of the sub-part, in token-id order, whose cumulative kept mass exceeds s.target. The kept mass of every
+// 256 elements (a vector per lane) is summed, order-free, and the block that holds the target is walked by one warp,
+// so the sub-part is read once and that block again.
+template <int kMode>
+__device__ __forceinline__ void part_draw(const __nv_bfloat16* rp, const PartRange& r, const Kept& k, PartSmem& s, int* out) {
+  using T = __nv_bfloat16;
+  constexpr int kU = 4;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned short* hp = reinterpret_cast<const unsigned short*>(rp);
+  const uint4* vp = reinterpret_cast<const uint4*>(rp + r.first);
+  const int n_blocks = (r.n_vec + 31) / 32;
+  const float y_max = -k.args.neg_y_max;
+  auto mass_of = [&](uint32_t h) {         // ties << kTieShift | mass
+    const uint32_t key = float_to_key(bits16_float(h));
+    if (kMode != kAll && key <= k.tau) return key == k.tau ? 1ull << kTieShift : 0ull;
+    return static_cast<unsigned long long>(mass_fixed(exp_det(sub_rn(mul_rn(key_to_float(key), k.args.inv_temp), y_max))));
+  };
+  const int tau_o = static_cast<int>(k.tau ^ 0x80000000u);
+  auto take_word = [&](uint32_t w, unsigned long long& m) {
+    if constexpr (kMode == kByTable) {
+      const uint32_t not_key = ~(w ^ (((w >> 15) & 0x00010001u) * 0x7FFFu));
+      const uint32_t i2 = __viaddmin_u16x2(not_key, k.top2, k.last2);
+      m += k.table[i2 & 0xFFFFu];
+      m += k.table[i2 >> 16];
+    } else {
+      float x0 = __uint_as_float(w << 16), x1 = __uint_as_float(w & 0xFFFF0000u);
+      if constexpr (kMode != kAll) {
+        auto ordered = [](float x) {
+          const int b = __float_as_int(x);
+          return b ^ ((b >> 31) & 0x7FFFFFFF);
+        };
+        const int o0 = ordered(x0), o1 = ordered(x1);
+        m += static_cast<unsigned long long>((o0 == tau_o ? 1u : 0u) + (o1 == tau_o ? 1u : 0u)) << kTieShift;
+        x0 = o0 > tau_o ? x0 : __uint_as_float(0xFF800000u);
+        x1 = o1 > tau_o ? x1 : __uint_as_float(0xFF800000u);
+      }
+      mass_pair(x0, x1, k.args, m);
+    }
+  };
+#pragma unroll 1
+  for (int b0 = warp; b0 < n_blocks; b0 += kPartWarps * kU) {
+    uint4 raw[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int j = (b0 + u * kPartWarps) * 32 + lane;
+      if (j < r.n_vec) raw[u] = __ldg(vp + j);
+    }
+    unsigned long long m[kU] = {};
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if ((b0 + u * kPartWarps) * 32 + lane < r.n_vec) {
+        take_word(raw[u].x, m[u]);
+        take_word(raw[u].y, m[u]);
+        take_word(raw[u].z, m[u]);
+        take_word(raw[u].w, m[u]);
+      }
+    }
+    // the sums of four blocks together: lanes 8 i .. 8 i + 7 end up with block i's
+    static_assert(kU == 4, "two exchanges of halves");
+    const bool hi = lane & 16, odd = lane & 8;
+    unsigned long long a = (hi ? m[2] : m[0]) + __shfl_xor_sync(0xffffffffu, hi ? m[0] : m[2], 16);
+    unsigned long long c = (hi ? m[3] : m[1]) + __shfl_xor_sync(0xffffffffu, hi ? m[1] : m[3], 16);
+    a = (odd ? c : a) + __shfl_xor_sync(0xffffffffu, odd ? a : c, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    const int b = b0 + (lane >> 3) * kPartWarps;
+    if ((lane & 7) == 0 && b < n_blocks) s.blocks[1 + b] = a;
+  }
+  if (warp >= kPartWarps - 2) {            // the scalars at the ends: first and last block
+    const bool last = warp == kPartWarps - 1;
+    const unsigned long long m =
+        warp_sum_u64(last ? (lane < r.n_tail ? mass_of(hp[r.tail + lane]) : 0ull) : (lane < r.n_head ? mass_of(hp[lane]) : 0ull));
+    if (lane == 0) s.blocks[last ? 1 + n_blocks : 0] = m;
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  const int n = n_blocks + 2, per = (n + 31) / 32;
+  constexpr unsigned long long kMassMask = (1ull << kTieShift) - 1;
+  unsigned long long target = s.target, t0 = s.ties_before;
+  int sel = -1;
+  {
+    // ties in front of this lane's blocks, then their kept mass
+    const int e0 = min(n, lane * per), e1 = min(n, e0 + per);
+    unsigned long long ties = 0, mass = 0;
+    for (int e = e0; e < e1; ++e) ties += s.blocks[e] >> kTieShift;
+    unsigned long long t = t0 + warp_incl_u64(ties) - ties;
+    const unsigned long long t_lane = t;
+    auto kept = [&](unsigned long long m) {
+      const unsigned long long left = k.tie_keep > t ? k.tie_keep - t : 0ull, here = m >> kTieShift;
+      t += here;
+      return (m & kMassMask) + (here < left ? here : left) * k.q_tau;
+    };
+    for (int e = e0; e < e1; ++e) mass += kept(s.blocks[e]);
+    const unsigned long long inc = warp_incl_u64(mass);
+    const int first = __ffs(static_cast<int>(__ballot_sync(0xffffffffu, inc > target))) - 1;
+    unsigned long long before = inc - mass;
+    if (lane == first) {
+      t = t_lane;
+      for (int e = e0; e < e1; ++e) {
+        const unsigned long long tb = t, m = kept(s.blocks[e]);
+        if (before + m > target) {
+          sel = e;
+          t0 = tb;
+          break;
+        }
+        before += m;
+      }
+    }
+    if (first < 0) return;                 // cannot happen: the sub-part holds the target
+    sel = __shfl_sync(0xffffffffu, sel, first);
+    t0 = __shfl_sync(0xffffffffu, t0, first);
+    target -= __shfl_sync(0xffffffffu, before, first);
+  }
+  // the block: eight elements per lane, or a scalar
+  uint32_t w[4] = {0u, 0u, 0u, 0u};
+  int have = 0, i0;
+  if (sel == 0 || sel == n - 1) {
+    const bool last = sel != 0;
+    i0 = (last ? r.tail : 0) + lane;
+    if (lane < (last ? r.n_tail : r.n_head)) {
+      w[0] = hp[i0];
+      have = 1;
+    }
+  } else {
+    const int j = (sel - 1) * 32 + lane;
+    i0 = r.first + 8 * j;
+    if (j < r.n_vec) {
+      const uint4 raw = __ldg(vp + j);
+      w[0] = raw.x;
+      w[1] = raw.y;
+      w[2] = raw.z;
+      w[3] = raw.w;
+      have = 8;
+    }
+  }
+  unsigned long long q[8], ties = 0;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    q[e] = e < have ? mass_of((w[e >> 1] >> (16 * (e & 1))) & 0xFFFFu) : 0ull;
+    ties += q[e] >> kTieShift;
+  }
+  unsigned long long rank = t0 + warp_incl_u64(ties) - ties, mass = 0;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    if (q[e] >> kTieShift) {
+      q[e] = rank < k.tie_keep ? k.q_tau : 0ull;
+      ++rank;
+    }
+    mass += q[e];
+  }
+  const unsigned long long inc = warp_incl_u64(mass);
+  const int first = __ffs(static_cast<int>(__ballot_sync(0xffffffffu, inc > target))) - 1;
+  if (lane == first) {
+    unsigned long long acc = inc - mass;
+    int at = -1;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      acc += q[e];
+      if (at < 0 && acc > target) at = e;
+    }
+    *out = i0 + at;
+  }
+}
+
+// Out of line: rows that the histograms cannot answer. Run by one CTA of the cluster.
+__device__ __noinline__ void part_general(const __nv_bfloat16* rp, int v, float inv_temp, int top_k, float top_p, uint32_t u24,
+                                          unsigned char* smem, DrawSmem& d, int* out) {
+  general_row<__nv_bfloat16, kPartThreads, false>(rp, v, inv_temp, top_k, top_p, u24, *reinterpret_cast<GeneralSmem*>(smem),
+                                                  nullptr, d, out);
+}
+
+__global__ void __launch_bounds__(kPartThreads, 3)
+sample_parts_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stride, int v,
+                    const long long* __restrict__ row_ids, float inv_temp, int top_k, float top_p, unsigned long long seed,
+                    unsigned long long step, int ctas, int* __restrict__ out) {
+  using T = __nv_bfloat16;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ DrawSmem d;
+  unsigned char* hist = smem_raw;
+  PartSmem& s = *reinterpret_cast<PartSmem*>(smem_raw + kPartsPerCta * kPartHistBytes);
+  const uint32_t hist_addr = static_cast<uint32_t>(__cvta_generic_to_shared(hist));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = static_cast<int>(cluster_rank()), row = static_cast<int>(blockIdx.x) / ctas;
+  const T* rp = logits + static_cast<long long>(row) * row_stride;
+  const bool has_k = top_k > 0 && top_k < v;
+
+  // a look at the row's first 4096 elements, for the magnitudes to count
+  uint32_t look = 0xFFFFFFFFu;
+  {
+    const int head = row_head(rp, v);
+    if (tid < (v - head) / 8) look = vec_max<T>(__ldg(reinterpret_cast<const uint4*>(rp + head) + tid));
+  }
+  // ---- count; the largest element and what was left out are known to all CTAs of the row behind the barrier
+  uint32_t base = kPartBase;
+  float y_max = 0.f;
+  uint32_t max_key = 0, max_bits = 0;
+#pragma unroll 1
+  for (int attempt = 0;; ++attempt) {
+    for (int i = tid; i < kPartsPerCta * kPartHistBytes / 16; i += kPartThreads)
+      reinterpret_cast<uint4*>(hist)[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = tid; i < kPartGroups; i += kPartThreads) {
+      s.mass[i] = 0;
+      s.cnt[i] = 0;
+    }
+    if (tid < kPartsPerCta * 2) s.zeros[tid >> 1][tid & 1] = 0;
+    if (tid < kPartsPerCta) s.acc[tid] = 0;
+    if (tid < kInfoWords) reinterpret_cast<uint32_t*>(&s.mine)[tid] = 0;
+    if (attempt == 0) {
+      look = Elem<T>::wmax(look, __byte_perm(look, 0, 0x1032));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) look = Elem<T>::wmax(look, __shfl_xor_sync(0xffffffffu, look, o));
+      if (lane == 0) s.look[warp] = look | 0xFFFF0000u;
+    }
+    __syncthreads();
+    if (attempt == 0) {
+      uint32_t m = 0xFFFFFFFFu;
+#pragma unroll
+      for (int w = 0; w < kPartWarps; ++w) m = Elem<T>::wmax(m, s.look[w]);
+      const float x = bits16_float(m & 0xFFFFu), reach = 2.f * part_reach(x, inv_temp);
+      if (reach >= 1024.f && reach < 1e38f) base = part_base(reach);     // no number, an infinity: as usual
+    }
+    part_count(rp, v, base, rank, ctas, hist, s);
+    __syncthreads();
+    if (tid < ctas * kInfoWords)
+      st_remote_u32(map_to_cta(reinterpret_cast<uint32_t*>(&s.info[rank]) + tid % kInfoWords, tid / kInfoWords),
+                    reinterpret_cast<const uint32_t*>(&s.mine)[tid % kInfoWords]);
+    if (tid == kPartThreads - 1)
+      s.u24 = uniform_u24(seed, row_ids ? static_cast<unsigned long long>(row_ids[row]) : static_cast<unsigned long long>(row), step);
+    part_barrier(ctas);
+    uint32_t flags = 0;
+    max_key = 0;
+    for (int r = 0; r < ctas; ++r) {
+      flags |= s.info[r].flags;
+      max_key = max(max_key, s.info[r].max_key);
+    }
+    max_bits = max_key == 0 ? 0x7FFFu : (max_key & 0x8000u ? max_key & 0x7FFFu : 0xFFFFu - max_key);
+    const float x_max = bits16_float(max_bits);
+    y_max = mul_rn(x_max, inv_temp);
+    if (!(fabsf(y_max) <= 3.402823466e38f)) {
+      // no number, or an infinite one: nothing has a mass, the last kept element is the answer
+      if (rank != 0) return;
+      if (has_k)
+        part_general(rp, v, inv_temp, top_k, top_p, s.u24, smem_raw, d, out + row);
+      else if (tid == 0)
+        out[row] = v - 1;
+      return;
+    }
+    // below 2^-33 of the maximum's weight a mass is 0 (2^-32 is the smallest that counts)
+    auto massive = [&](uint32_t bits) { return (bits16_float(bits) * inv_temp - y_max) * 1.4426950408889634f > -33.f; };
+    const uint32_t lowest = 0x8000u + base + kPartMags;
+    const bool low = (flags & kLow) && massive(lowest), tiny = (flags & kTiny) && massive(base);
+    if (!(flags & kBig) && !low && !tiny) break;
+    if (attempt > 0) {
+      if (rank == 0)
+        part_general(rp, v, inv_temp, top_k, top_p, s.u24, smem_raw, d, out + row);
+      return;
+    }
+    // the 64 binades up to the largest magnitude that can have a mass; if all values are tiny, up to theirs
+    const bool all_tiny = !(flags & (kBig | kLow)) && (max_bits & 0x7FFFu) < base;
+    base = part_base(all_tiny ? 4.f * fabsf(x_max) : part_reach(x_max, inv_temp));
+    part_barrier(ctas);               // s.info is written again
+  }
+
+  // ---- masses of the groups: units of four groups are dealt over the CTAs, whose sums go to all of them
+  if (tid < kPartUnits) {
+    unsigned int before = 0, word = 0;
+#pragma unroll
+    for (int i = 0; i < kPartUnits / 32; ++i) {
+      unsigned int w = 0;
+      for (int r = 0; r < ctas; ++r) w |= s.info[r].units[i];
+      if (i < warp) before += __popc(w);
+      if (i == warp) word = w;
+    }
+    if (word >> lane & 1u) s.units[before + __popc(word & ((1u << lane) - 1u))] = static_cast<unsigned char>(tid);
+    if (tid == kPartUnits - 1) s.n_units = before + __popc(word);
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int i = rank + ctas * warp; i < s.n_units; i += ctas * kPartWarps) {
+    const int u = s.units[i];
+    const int at = u * 128 + lane * 4;                      // four neighbours' counters, in rising order of magnitude
+    unsigned int n[4] = {0, 0, 0, 0};
+#pragma unroll 1
+    for (int r0 = 0; r0 < ctas; r0 += 4) {                  // four CTAs' counters in flight
+      uint2 c[4 * kPartsPerCta];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int sub = 0; sub < kPartsPerCta; ++sub) {
+          c[r * kPartsPerCta + sub] = make_uint2(0u, 0u);
+          if (r0 + r < ctas)
+            c[r * kPartsPerCta + sub] =
+                ld_remote_u32x2(map_addr(hist_addr + static_cast<uint32_t>(at) * 2 + sub * kPartHistBytes, r0 + r));
+        }
+#pragma unroll
+      for (int i = 0; i < 4 * kPartsPerCta; ++i) {
+        n[0] += c[i].x & 0xFFFFu;
+        n[1] += c[i].x >> 16;
+        n[2] += c[i].y & 0xFFFFu;
+        n[3] += c[i].y >> 16;
+      }
+    }
+    unsigned int cnt = n[0] + n[1] + n[2] + n[3];
+    const bool neg = at >= kPartMags;
+    const uint32_t bits = neg ? 0x8000u + base + static_cast<uint32_t>(at - kPartMags) : base + static_cast<uint32_t>(at);
+    unsigned long long m = 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) m += n[e] * bits16_mass(bits + e, inv_temp, y_max);
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      m += __shfl_xor_sync(0xffffffffu, m, o);
+      cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    }
+    const int g = neg ? kPartZeroGroup + 1 + (at - kPartMags) / 32 : kPartZeroGroup - 1 - at / 32;
+    if ((lane & 7) < ctas && cnt) {
+      st_remote_u64(map_to_cta(&s.mass[g], lane & 7), m);
+      st_remote_u32(map_to_cta(&s.cnt[g], lane & 7), cnt);
+    }
+  }
+  if (rank == 0 && warp == kPartWarps - 1) {
+    unsigned int n = lane < 2 ? part_zeros(lane, ctas, s) : 0u;
+    unsigned long long m = n ? n * bits16_mass(0u, inv_temp, y_max) : 0ull;      // both zeros weigh the same
+    m += __shfl_down_sync(0xffffffffu, m, 1);
+    n += __shfl_down_sync(0xffffffffu, n, 1);
+    m = __shfl_sync(0xffffffffu, m, 0);
+    n = __shfl_sync(0xffffffffu, n, 0);
+    if (lane < ctas && n) {
+      st_remote_u64(map_to_cta(&s.mass[kPartZeroGroup], lane), m);
+      st_remote_u32(map_to_cta(&s.cnt[kPartZeroGroup], lane), n);
+    }
+  }
+  part_barrier(ctas);
+
+  // ---- where the kept prefix ends, in every CTA: the same decisions as in general_row
+  int tau = kNothing;
+  unsigned long long tie_keep = ~0ull, kept_mass;
+  {
+    const int g0 = 2 * tid, g1 = g0 + 1;
+    unsigned long long pre_c = 0, tot_c;
+    const unsigned long long pre_m = block_exscan_u64((g0 < kPartGroups ? s.mass[g0] : 0ull) + (g1 < kPartGroups ? s.mass[g1] : 0ull),
+                                                      s.scan, kept_mass);
+    if (has_k) {
+      pre_c = block_exscan_u64((g0 < kPartGroups ? s.cnt[g0] : 0u) + (g1 < kPartGroups ? s.cnt[g1] : 0u), s.scan, tot_c);
+      // if fewer elements than that are counted, every element with a mass is among the k largest
+      part_search(false, static_cast<unsigned long long>(top_k - 1), inv_temp, y_max, base, ctas, pre_c, pre_m, hist_addr, s);
+      if (s.sel != kNothing) {
+        tau = s.sel;
+        tie_keep = static_cast<unsigned long long>(top_k) - s.above_cnt;
+        kept_mass = s.above_mass + tie_keep * bits16_mass(part_bits(tau, base), inv_temp, y_max);
+      }
+    }
+    if (top_p < 1.0f) {
+      const unsigned long long limit = mass_fraction(static_cast<double>(top_p), kept_mass);
+      __syncthreads();
+      part_search(true, limit, inv_temp, y_max, base, ctas, pre_c, pre_m, hist_addr, s);
+      if (s.sel != kNothing) {
+        const int p_tau = s.sel;
+        const unsigned long long q = bits16_mass(part_bits(p_tau, base), inv_temp, y_max);   // not 0: it crosses
+        const unsigned long long p_ties = (limit - s.above_mass) / q + 1;
+        if (p_tau != tau ? p_tau < tau : p_ties < tie_keep) {
+          tau = p_tau;
+          tie_keep = p_ties < s.present ? p_ties : s.present;
+          kept_mass = s.above_mass + tie_keep * q;
+        }
+      }
+    }
+  }
+
+  // ---- kept mass and ties of this CTA's sub-parts, from their histograms
+  {
+    unsigned long long m[kPartsPerCta] = {};
+    const int d_end = min(tau, 2 * kPartMags + 2);
+#pragma unroll 1
+    for (int i = part_rank(max_bits, base) + tid; i < d_end; i += kPartThreads) {
+      unsigned int n[kPartsPerCta], any = 0;
+      const bool zero = i == kPartMags || i == kPartMags + 1;
+#pragma unroll
+      for (int sub = 0; sub < kPartsPerCta; ++sub) {
+        n[sub] = zero ? s.zeros[sub][i - kPartMags]
+                      : *reinterpret_cast<const unsigned short*>(hist + sub * kPartHistBytes + part_offset(i));
+        any |= n[sub];
+      }
+      if (any == 0) continue;
+      const unsigned long long q = bits16_mass(part_bits(i, base), inv_temp, y_max);
+#pragma unroll
+      for (int sub = 0; sub < kPartsPerCta; ++sub) m[sub] += n[sub] * q;
+    }
+#pragma unroll
+    for (int sub = 0; sub < kPartsPerCta; ++sub) {
+      m[sub] = warp_sum_u64(m[sub]);
+      if (lane == 0 && m[sub]) atomicAdd(&s.acc[sub], m[sub]);
+    }
+    __syncthreads();
+    if (tid < ctas * kPartsPerCta) {
+      const int to = tid / kPartsPerCta, sub = tid % kPartsPerCta, q = rank * kPartsPerCta + sub;
+      unsigned long long ties = 0;
+      if (tau != kNothing)
+        ties = tau == kPartMags || tau == kPartMags + 1
+                   ? s.zeros[sub][tau - kPartMags]
+                   : *reinterpret_cast<const unsigned short*>(hist + sub * kPartHistBytes + part_offset(tau));
+      st_remote_u64(map_to_cta(&s.sub_mass[q], to), s.acc[sub]);
+      st_remote_u64(map_to_cta(&s.sub_ties[q], to), ties);
+    }
+    part_barrier(ctas);
+  }
+
+  // ---- the sub-part that holds the target; its CTA draws, nobody reads another CTA's memory any more
+  Kept k;
+  const uint32_t tau_bits = tau == kNothing ? 0u : part_bits(tau, base);
+  const uint32_t tau16 = tau == kNothing ? 0u : (tau_bits & 0x8000u ? 0xFFFFu - tau_bits : tau_bits + 0x8000u);
+  k.tau = tau == kNothing ? 0u : float_to_key(bits16_float(tau_bits));
+  k.tie_keep = tau == kNothing ? 0ull : tie_keep;
+  k.q_tau = tau == kNothing ? 0ull : bits16_mass(tau_bits, inv_temp, y_max);
+  k.args = {inv_temp, -y_max};
+  const int n_sub = ctas * kPartsPerCta;
+  if (warp == 0) {
+    const unsigned long long target = mass_scale_u24(s.u24, kept_mass);
+    const unsigned long long t = lane < n_sub ? s.sub_ties[lane] : 0ull, t0 = warp_incl_u64(t) - t;
+    const unsigned long long left = k.tie_keep > t0 ? k.tie_keep - t0 : 0ull;
+    const unsigned long long m = (lane < n_sub ? s.sub_mass[lane] : 0ull) + (t < left ? t : left) * k.q_tau;
+    const unsigned long long inc = warp_incl_u64(m);
+    const int first = __ffs(static_cast<int>(__ballot_sync(0xffffffffu, inc > target))) - 1;
+    if (lane == first) {
+      s.owner = first;
+      s.target = target - (inc - m);
+      s.ties_before = t0;
+    }
+  }
+  __syncthreads();
+  const int q = s.owner;
+  if (q / kPartsPerCta != rank) return;
+  const PartRange r = part_range(q, n_sub, row_head(rp, v), v);
+  if (tau == kNothing) {
+    part_draw<kAll>(rp, r, k, s, out + row);
+    return;
+  }
+  const uint32_t range = max_key - tau16;
+  unsigned long long* table = reinterpret_cast<unsigned long long*>(hist);
+  if (range + 2 <= kPartsPerCta * kPartHistBytes / 8) {
+    for (uint32_t i = tid; i < range; i += kPartThreads) table[i] = key16_mass_of<T>(max_key - i, inv_temp, y_max);
+    if (tid == 0) {
+      table[range] = 1ull << kTieShift;
+      table[range + 1] = 0;
+    }
+    k.table = table;
+    k.top2 = ((max_key + 0x8001u) & 0xFFFFu) * 0x00010001u;
+    k.last2 = (range + 1) * 0x00010001u;
+    __syncthreads();
+    part_draw<kByTable>(rp, r, k, s, out + row);
+    return;
+  }
+  part_draw<kByExp>(rp, r, k, s, out + row);
+}
+
+// How many CTAs share a row, 0 for the one of 1024 threads that counts and draws by itself. Counting is bound by the
+// atomics an SM can do, so more CTAs than SMs help only to deal rows that do not fill a whole number of rounds, and what is behind the
+// counting (searches, two barriers of the cluster, the draw: 14 us) is paid by any number of CTAs. us, one CTA per row
+// of 1024 threads / parts, top_p = 0.9: 8 rows of 128256 29.1 / 17.1 (8 CTAs), 30 rows 29.1 / 18.8 (4; 8 CTAs 21.1), 64 rows
+// 29.7 / 24.8 (2), 148 rows 31.3 / 35.2; 32000 columns: 8 rows 15.7 / 15.1, 64 rows 15.7 / 17.3. With more rows than SMs
+// that kernel needs another round, parts have them all resident, three per SM: 200 rows of 128256 58.3 / 46.4 (2 CTAs; 1: 51.9),
+// 256 59.0 / 52.4 (1; 2: 60.8); 32000 columns 30.4 / 25.5 (1; 2: 27.1), 1000 columns 21.9 / 16.8.
+inline int part_ctas(int rows, int v, int sms) {
+  // a sub-part's vectors are rounded up, its ends have up to seven scalars each
+  auto fits = [&](int ctas) { return v / (ctas * kPartsPerCta) + 32 <= kPartMaxElems; };
+  int ctas = 1;
+  if (rows > sms) {
+    if (v >= 65536 && 2ll * rows <= 3ll * sms) ctas = 2;
+  } else {
+    // an eighth of the SMs stays free: clusters of eight do not find a place on all of them
+    while (ctas < kMaxPartCtas && 16ll * ctas * rows <= 7ll * sms) ctas *= 2;
+    if (v < (ctas >= 4 ? 28672 : 49152) || ctas == 1) return 0;
+  }
+  while (ctas < kMaxPartCtas && !fits(ctas)) ctas *= 2;
+  return fits(ctas) ? ctas : 0;
+}
+
+inline int launch_parts(const __nv_bfloat16* lp, long long row_stride, int rows, int v, const long long* row_ids, float inv_temp,
+                        int top_k, float top_p, unsigned long long seed, unsigned long long step, int ctas, int* out,
+                        cudaStream_t stream) {
+  static PerDevice once;
+  if (!smem_opt_in(once, sample_parts_kernel, kPartSmemBytes)) return -10;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(rows) * ctas);
+  cfg.blockDim = dim3(kPartThreads);
+  cfg.dynamicSmemBytes = kPartSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(ctas);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, sample_parts_kernel, lp, row_stride, v, row_ids, inv_temp, top_k, top_p, seed, step, ctas, out) ==
+                 cudaSuccess
+             ? 0
+             : -11;
 }
 
 // Which maxima bound a row of which a block of `threads` holds `elems` elements. The warps' keys (eight or four
@@ -2037,6 +2830,14 @@ int launch_sampling(const void* logits, long long row_stride, int rows, int v, c
   if (top_k >= 1 && top_k <= kMaxTopK) {
     return launch_topk<T>(lp, row_stride, rows, v, row_ids, inv_temp, top_k, top_p, seed, step, out, stream);
   } else {
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+      // without a filter the sums of the draw are the only pass, and less work than counting
+      int dev = 0, sms = 0;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      const int ctas = (top_k > 0 && top_k < v) || top_p < 1.0f ? part_ctas(rows, v, sms) : 0;
+      if (ctas > 0) return launch_parts(lp, row_stride, rows, v, row_ids, inv_temp, top_k, top_p, seed, step, ctas, out, stream);
+    }
     constexpr int smem = kGeneralSmemBytes + (Elem<T>::kPacked ? static_cast<int>(sizeof(FastSmem)) : 0);
     static_assert(sizeof(FastSmem) >= kHistBytes, "the older search keeps its histogram there");
     static PerDevice once;

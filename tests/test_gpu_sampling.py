@@ -228,3 +228,32 @@ def test_sampler_candidates_in_few_places(cuda_device, dtype, vocab, rows):
         for top_k, top_p in ((1, None), (20, 0.9), (50, None), (64, 0.8), (65, 0.9), (200, None), (257, 0.9), (600, 0.95)):
             tok = sample(val, top_k=top_k, top_p=top_p, temperature=0.7, seed=2, step=top_k)
             assert torch.equal(tok[:3].cpu(), _cpu(val[:3], top_k, top_p, 0.7, 2, top_k)), (name, top_k, top_p)
+
+
+@pytest.mark.parametrize("top_k,top_p,temperature", [(None, 0.9, 1.0), (None, None, 0.7), (2000, 0.95, 1.0), (None, 0.9, 40.0)])
+@pytest.mark.parametrize("vocab,rows", [(31, 150), (49155, 3), (33001, 30), (50003, 74), (8193, 300), (131075, 2), (65541, 180)])
+def test_sampler_bf16_parts_of_a_row(cuda_device, vocab, rows, top_k, top_p, temperature):
+    """bf16 rows without a small top-k: one to eight CTAs per row, rows that start off a 16-byte boundary, and values
+    inside and outside the magnitudes that are counted at first: plain, far above and below them, next to zero, zeros of
+    both signs, one value throughout, masked three ways, thresholds among negative values."""
+    g = torch.Generator(device=cuda_device).manual_seed(vocab + rows)
+    x = torch.randn(rows, vocab, device=cuda_device, generator=g) * 2
+    u = torch.rand(x.shape, device=cuda_device, generator=g)
+    values = {"plain": x, "negative": x - 20, "above": x * 8 + 3000, "below": x * 8 - 5000, "wide": x * 2000, "tiny": x * 1e-18,
+              "few_tiny": torch.where(u < 0.01, x * 1e-18, x), "zeros": torch.where(u < 0.5, 0.0, -0.0),
+              "half_zero": torch.where(u < 0.5, 0.0, x), "one_value": torch.full_like(x, 3.0),
+              "inf_mask": torch.where(u < 0.99, float("-inf"), x), "lowest": torch.where(u < 0.9, torch.finfo(torch.bfloat16).min, x),
+              "mask_1e4": torch.where(u < 0.9, -1e4, x), "nan": torch.where(u < 0.1, float("nan"), x),
+              "all_nan": torch.full_like(x, float("nan")), "all_inf": torch.full_like(x, float("-inf")),
+              "plus_inf": torch.where(u > 0.999, float("inf"), x)}
+    buf = torch.empty(rows * (vocab + 1) + 3, dtype=torch.bfloat16, device=cuda_device)
+    some = torch.arange(0, rows, max(1, rows // 3))[:4]
+    for name, val in values.items():
+        for off, width in ((0, vocab), (3, vocab + 1)):
+            logits = buf[off:off + rows * width].view(rows, width)[:, :vocab]
+            logits.copy_(val)
+            tok = sample(logits, top_k=top_k, top_p=top_p, temperature=temperature, seed=5, step=1).cpu()
+            ref = _cpu(logits[some.to(cuda_device)], top_k, top_p, temperature, 5, 1, row_ids=some)
+            assert torch.equal(tok[some], ref), (name, off)
+            alone = sample(logits[:2], top_k=top_k, top_p=top_p, temperature=temperature, seed=5, step=1)
+            assert torch.equal(alone.cpu(), tok[:2]), (name, off)
