@@ -1,8 +1,9 @@
-"""In-tree native build: nvcc for the sm_100a kernels, g++ for the CPU oracle library.
+"""In-tree native build: nvcc for the sm_100a kernels, g++ for the CPU oracle library and for the
+operators that are C++ autograd nodes.
 
-Both libraries are plain shared objects with ``extern "C"`` entry points, loaded through
-``ctypes``; they sit next to the package so that a built tree can be copied to a GPU host
-as is. A content hash of the sources and flags decides whether a rebuild is needed.
+The first two are plain shared objects with ``extern "C"`` entry points, loaded through
+``ctypes``, the third is an extension module against the installed torch; they sit next to the package so that a
+built tree can be copied to a GPU host as is. A content hash of the sources and flags decides whether a rebuild is needed.
 """
 from __future__ import annotations
 
@@ -11,6 +12,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -21,6 +23,7 @@ OBJ_DIR = ROOT / "build" / "obj"
 
 CUDA_LIB = LIB_DIR / "libka_sm100.so"
 CPU_LIB = LIB_DIR / "libka_cpu.so"
+TORCH_LIB = LIB_DIR / "_ka_torch.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -104,6 +107,32 @@ def build_cpu(force: bool = False) -> Path | None:
     return CPU_LIB
 
 
+def build_torch(force: bool = False) -> Path | None:
+    """Compile ``csrc/torch/*.cpp`` into the extension module ``_ka_torch.so`` (C++ autograd nodes)."""
+    try:
+        import torch
+    except ImportError:      # an isolated package build: the first call that needs the module builds it
+        return TORCH_LIB if TORCH_LIB.exists() else None
+    srcs = sorted((CSRC / "torch").glob("*.cpp"))
+    if not srcs:
+        return TORCH_LIB if TORCH_LIB.exists() else None
+    inc, lib = Path(torch.__file__).parent / "include", Path(torch.__file__).parent / "lib"
+    cuda_home = os.environ.get("CUDA_HOME") or "/usr/local/cuda"
+    flags = ["-O2", "-std=c++17", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
+    digest = _digest(srcs, [*flags, torch.__version__, sys.version])
+    if not force and _stamp_ok(TORCH_LIB, digest):
+        return TORCH_LIB
+    cxx = shutil.which("g++")
+    if cxx is None:
+        return TORCH_LIB if TORCH_LIB.exists() else None
+    LIB_DIR.mkdir(parents=True, exist_ok=True)
+    _run([cxx, *flags, "-shared", "-o", str(TORCH_LIB), *[str(s) for s in srcs], f"-I{inc}",
+          f"-I{inc / 'torch' / 'csrc' / 'api' / 'include'}", f"-I{sysconfig.get_paths()['include']}",
+          f"-I{cuda_home}/include", f"-L{lib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"])
+    TORCH_LIB.with_suffix(".hash").write_text(digest)
+    return TORCH_LIB
+
+
 def build_cpu_sanitized(force: bool = False) -> Path | None:
     """The CPU library once more with AddressSanitizer and UndefinedBehaviorSanitizer
     (``libka_cpu_asan.so``): the sanitizer tier of the tests loads it in a child process that
@@ -137,9 +166,10 @@ def sanitizer_runtime() -> str | None:
 
 def build_all(force: bool = False, verbose: bool = False) -> None:
     build_cpu(force)
+    build_torch(force)
     build_cuda(force, verbose)
 
 
 if __name__ == "__main__":
     build_all(force="--force" in sys.argv, verbose="-v" in sys.argv)
-    print("built:", [str(p) for p in (CPU_LIB, CUDA_LIB) if p.exists()])
+    print("built:", [str(p) for p in (CPU_LIB, TORCH_LIB, CUDA_LIB) if p.exists()])

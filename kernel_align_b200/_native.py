@@ -1,12 +1,14 @@
-"""ctypes bindings to the two in-tree native libraries.
+"""Bindings to the in-tree native libraries: ctypes for two, an extension module for the third.
 
 ``cuda()`` returns the sm_100a kernel library and raises if it is missing: on a GPU host the
 hand-written kernels are the only code path, there is no silent PyTorch fallback.
 ``cpu()`` returns the C++ CPU library (oracle for the tests and the CPU device path).
+``torch_ops()`` returns the extension module with the operators that are C++ autograd nodes.
 """
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 from ctypes import c_char_p, c_float, c_int, c_longlong, c_size_t, c_uint, c_ulonglong, c_void_p
 from functools import lru_cache
@@ -74,15 +76,6 @@ def cuda() -> ctypes.CDLL:
         c_int,
         [c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p],
     )
-    _bind(lib, "ka_grpo_advantages", c_int, [c_void_p, c_void_p, c_int, c_int, c_float, c_void_p])
-    _bind(
-        lib,
-        "ka_grpo_loss_fwd",
-        c_int,
-        [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_float, c_float, c_int,
-         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
-    )
-    _bind(lib, "ka_grpo_loss_bwd", c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p])
     # prototypes are set here, once: setting them costs a call several microseconds
     p, i, ll, f, ull = c_void_p, c_int, c_longlong, c_float, c_ulonglong
     _bind(lib, "ka_rmsnorm", c_int, [p, p, p, p, p, i, i, f, i, p])
@@ -113,6 +106,23 @@ def cuda() -> ctypes.CDLL:
     _bind(lib, "ka_gemm_split8", c_int, [p, ll, p, ll, i, p, p, p, i, i, i, p, i, ull, p])
     _bind(lib, "ka_all_gather_gemm", c_int, [p, p, ll, i, p, ll, p, i, i, i, i, i, c_uint, p, i, ull, p])
     return lib
+
+
+@lru_cache(maxsize=None)
+def torch_ops():
+    """The extension module with the operators that are C++ autograd nodes, bound to the kernels of :func:`cuda`."""
+    path = _build.build_torch()
+    if path is None or not path.exists():
+        raise NativeLibraryMissing(
+            "_ka_torch.so is not built; run `python -m kernel_align_b200._build` on a host with g++"
+        )
+    spec = importlib.util.spec_from_file_location("_ka_torch", str(path))
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    lib = cuda()
+    mod.bind(*[ctypes.cast(getattr(lib, name), c_void_p).value
+               for name in ("ka_grpo_advantages", "ka_grpo_loss_fwd", "ka_grpo_loss_bwd")])
+    return mod
 
 
 def _device_index(device) -> int:

@@ -1,6 +1,6 @@
 """``python -m kernel_align_b200.doctor``: what this installation can do on this host.
 
-Prints the package version, the state of the two native libraries (built / stale / missing,
+Prints the package version, the state of the native libraries (built / stale / missing,
 with the compiler that would build them), the visible GPUs with their compute capability (the
 kernels need sm_100), peer access between them, the distributed backends PyTorch offers, and
 runs a two-second CPU self-test of the C++ library against PyTorch. Exit code 0 when at least
@@ -24,6 +24,7 @@ def collect() -> dict:
     info["cxx"] = shutil.which("g++")
     info["libka_sm100"] = str(_build.CUDA_LIB) if _build.CUDA_LIB.exists() else None
     info["libka_cpu"] = str(_build.CPU_LIB) if _build.CPU_LIB.exists() else None
+    info["ka_torch"] = str(_build.TORCH_LIB) if _build.TORCH_LIB.exists() else None
     gpus = []
     if torch.cuda.is_available():
         for i in range(torch.cuda.device_count()):
@@ -83,6 +84,7 @@ def main(argv=None) -> int:
         print(f"kernel_align_b200 {info['version']}  (torch {info['torch']}, CUDA runtime {info['cuda_runtime']})")
         print(f"  sm_100a kernel library : {info['libka_sm100'] or 'not built'}   (nvcc: {info['nvcc'] or 'not found'})")
         print(f"  C++ CPU library        : {info['libka_cpu'] or 'not built'}   (g++: {info['cxx'] or 'not found'})")
+        print(f"  autograd nodes (C++)   : {info['ka_torch'] or 'not built'}   (g++: {info['cxx'] or 'not found'})")
         if info["gpus"]:
             for gpu in info["gpus"]:
                 mark = "ok" if gpu["supported"] else "unsupported: the kernels are written for sm_100a"

@@ -1,7 +1,7 @@
-"""Packaging: the Python package plus the two in-tree native libraries.
+"""Packaging: the Python package plus the in-tree native libraries.
 
 ``python setup.py build_ext --inplace`` (or any ``pip install``) compiles
-``csrc/sm100/*.cu`` for sm_100a with nvcc and ``csrc/cpu/*.cpp`` with g++ into
+``csrc/sm100/*.cu`` for sm_100a with nvcc, ``csrc/cpu/*.cpp`` and ``csrc/torch/*.cpp`` with g++ into
 ``kernel_align_b200/_lib`` through ``kernel_align_b200/_build.py``; every sub-package is a real
 package (the reference's setup.py:6 silently dropped four of its six).
 """

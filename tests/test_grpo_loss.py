@@ -83,3 +83,78 @@ def test_grpo_loss_gpu(cuda_device):
     assert a.item() == b.item()
     a.backward()
     assert torch.isfinite(ln.grad).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,strided,mask_dtype", [(torch.float32, False, torch.bool), (torch.bfloat16, True, torch.int64),
+                                                      (torch.float64, True, torch.float32), (torch.float32, True, None)])
+def test_grpo_loss_gpu_takes_what_the_cpu_takes(cuda_device, dtype, strided, mask_dtype):
+    """Types and strides are brought to fp32 rows on both devices; the gradient has the input's type and shape."""
+    ln, lo, lr, rewards, mask = (t.to(dtype) if t.is_floating_point() else t for t in _case(torch.device("cpu")))
+    grids = [t.t().contiguous().t() if strided else t for t in (ln, lo, lr)]
+    m = None if mask_dtype is None else mask.to(mask_dtype)
+    got = []
+    for dev in (torch.device("cpu"), cuda_device):
+        x, o, r = (t.to(dev) for t in grids)
+        x = x.detach().requires_grad_()
+        adv = group_advantages(rewards.to(dev).view(3, 4), 4)
+        assert adv.shape == (3, 4) and adv.dtype == torch.float32
+        loss, stats = grpo_loss(x, o, adv.view(-1), mask=None if m is None else m.to(dev), logp_ref=r, beta=0.04, return_stats=True)
+        (g,) = torch.autograd.grad(loss, x, torch.tensor(3.0, device=dev, dtype=torch.float64).to(loss.dtype))
+        assert g.dtype == dtype and g.shape == x.shape and not stats.requires_grad
+        got.append([loss.detach().cpu(), stats.cpu(), g.float().cpu()])
+    for a, b in zip(*got):      # sums of 840 fp32 terms in two orders, exponentials of 2 ulp; gradients rounded to 8 bits
+        assert (a - b).abs().max().item() <= (1e-5 if dtype != torch.bfloat16 else 1e-2) * max(1.0, a.abs().max().item())
+
+
+@pytest.mark.gpu
+def test_grpo_loss_gpu_as_an_autograd_node(cuda_device):
+    """Hooks on saved tensors see them, transforms that read no memory are refused, nothing is recorded without
+    gradients, a second derivative is none, another stream and thread work."""
+    import threading
+
+    ln, lo, lr, rewards, mask = _case(cuda_device)
+    adv = group_advantages(rewards, 4)
+    x = ln.clone().requires_grad_()
+    (want,) = torch.autograd.grad(grpo_loss(x, lo, adv, mask=mask), x)
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (packed.append(t.shape), t.cpu())[1], lambda t: t.to(cuda_device)):
+        loss = grpo_loss(x, lo, adv, mask=mask)
+    assert len(packed) == 2 and torch.equal(torch.autograd.grad(loss, x)[0], want)
+    for refused in (lambda: torch.func.vmap(lambda a: grpo_loss(ln, lo, a, mask=mask))(torch.stack([adv, adv])),
+                    lambda: torch.func.grad(lambda a: grpo_loss(a, lo, adv, mask=mask))(ln),
+                    lambda: torch.func.jvp(lambda a: grpo_loss(a, lo, adv, mask=mask), (ln,), (ln,)),
+                    lambda: grpo_loss(x, lo.cpu(), adv), lambda: grpo_loss(x[0], lo[0], adv)):
+        with pytest.raises((RuntimeError, ValueError, NotImplementedError)):
+            refused()
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(ln.clone(), torch.ones_like(ln))
+        with pytest.raises((RuntimeError, NotImplementedError)):
+            grpo_loss(dual, lo, adv, mask=mask)
+    for mode in (torch.no_grad, torch.inference_mode):
+        with mode():
+            assert grpo_loss(x, lo, adv, mask=mask).item() == loss.item() and not grpo_loss(x, lo, adv).requires_grad
+    (g,) = torch.autograd.grad(grpo_loss(x, lo, adv, mask=mask), x, create_graph=True)
+    assert torch.equal(g, want) and not g.requires_grad
+    out = {}
+
+    def work():
+        s = torch.cuda.Stream(cuda_device)
+        with torch.cuda.stream(s):
+            y = ln.clone().requires_grad_()
+            out["g"] = torch.autograd.grad(grpo_loss(y, lo, adv, mask=mask), y)[0]
+        s.synchronize()
+
+    torch.cuda.synchronize(cuda_device)
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert torch.equal(out["g"], want)
+    graph_in = ln.clone()
+    grpo_loss(graph_in, lo, adv, mask=mask)
+    torch.cuda.synchronize(cuda_device)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = grpo_loss(graph_in, lo, adv, mask=mask)
+    graph.replay()
+    assert captured.item() == loss.item()
