@@ -132,8 +132,9 @@ __device__ __forceinline__ constexpr uint32_t tcol(int kk) { return (kk >> 1) * 
 // dQ 891 -> 500 us, dK / dV 1466 -> 530 us; B = 8, L = 512: dQ 114 -> 66 us, dK / dV 173 -> 62 us.
 // ------------------------------------------------------------------------------------------------
 struct CtlDq {
-  uint64_t qdo_full;                 // Q and dO tiles loaded
-  uint64_t kv_full[2], kv_empty[2];
+  uint64_t qdo_full, do_full;        // Q tile loaded, dO tile loaded
+  uint64_t kv_full[3], kv_empty[3];  // K tiles: read by S and, an elementwise pass later, by dQ
+  uint64_t v_full[2], v_empty[2];    // V tiles: read by dP alone
   uint64_t s_full[2];                // S ready in its TMEM buffer
   uint64_t dp_full, dp_read;         // dP ready / read into registers (count: softmax warps)
   // dS written over S (count: softmax warps), one per S buffer: S(j + 1) and dP(j + 1) are issued before
@@ -146,15 +147,21 @@ struct CtlDq {
 };
 
 // ------------------------------------------------------------------------------------------------
-// dQ kernel. TMEM: S (two buffers), dP, dQ. Shared memory: Q, dO, two stages of (K, V).
+// dQ kernel. TMEM: S (two buffers), dP, dQ. Shared memory: Q, dO, three stages of K, two of V.
+// An SM gets about 85 GB/s, so a pair of tiles takes 1400 cycles and the latency on top. With two stages of (K, V)
+// that were handed back together, behind dQ(j), the load of tile j + 2 and then S(j + 2) followed one another in the time in which the warps
+// took tile j + 1, and an iteration was 3800 cycles; V is handed back by dP(j) now and K has a third stage: 2770
+// cycles, what the products of one CTA take to issue (S 590, dP 660, dQ 960: shared memory).
 // ------------------------------------------------------------------------------------------------
+constexpr int kKStages = 3;
 __device__ __forceinline__ void
 bwd_dq(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v, const CUtensorMap& tm_do,
        const BwdParams& p, int block) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t base = smem_u32(smem_raw);
-  const uint32_t q_tile = base, do_tile = base + kTileBytes, ring = base + 2 * kTileBytes;  // stage: K, V
-  CtlDq* ctl = reinterpret_cast<CtlDq*>(smem_raw + 6 * kTileBytes);
+  const uint32_t q_tile = base, do_tile = base + kTileBytes, k_ring = base + 2 * kTileBytes,
+                 v_ring = base + (2 + kKStages) * kTileBytes;
+  CtlDq* ctl = reinterpret_cast<CtlDq*>(smem_raw + (4 + kKStages) * kTileBytes);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_qt = (p.seq_len + kT - 1) / kT;
@@ -169,9 +176,14 @@ bwd_dq(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v
 
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&ctl->qdo_full), 1);
-    for (int s = 0; s < 2; ++s) {
+    mbar_init(smem_u32(&ctl->do_full), 1);
+    for (int s = 0; s < kKStages; ++s) {
       mbar_init(smem_u32(&ctl->kv_full[s]), 1);
       mbar_init(smem_u32(&ctl->kv_empty[s]), 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(smem_u32(&ctl->v_full[s]), 1);
+      mbar_init(smem_u32(&ctl->v_empty[s]), 1);
       mbar_init(smem_u32(&ctl->s_full[s]), 1);
       mbar_init(smem_u32(&ctl->ds_full[s]), kSoftThreads / 32);
     }
@@ -193,62 +205,78 @@ bwd_dq(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v
 
   if (warp == kWarpTma) {
     if (lane == 0) {
-      const uint32_t f = smem_u32(&ctl->qdo_full);
-      mbar_arrive_expect_tx(f, 2 * kTileBytes);
-      tma_load_2d(q_tile, &tm_q, h * kD, tok0 + q_row0, f);
-      tma_load_2d(q_tile + 16384, &tm_q, h * kD + 64, tok0 + q_row0, f);
-      tma_load_2d(do_tile, &tm_do, h * kD, tok0 + q_row0, f);
-      tma_load_2d(do_tile + 16384, &tm_do, h * kD + 64, tok0 + q_row0, f);
+      auto load = [&](uint32_t dst, const CUtensorMap& tm, int col, int row, uint64_t* bar) {
+        const uint32_t full = smem_u32(bar);
+        mbar_arrive_expect_tx(full, kTileBytes);
+        tma_load_2d(dst, &tm, col, row, full);
+        tma_load_2d(dst + 16384, &tm, col + 64, row, full);
+      };
+      load(q_tile, tm_q, h * kD, tok0 + q_row0, &ctl->qdo_full);
+      load(k_ring, tm_k, hk * kD, tok0, &ctl->kv_full[0]);
+      load(do_tile, tm_do, h * kD, tok0 + q_row0, &ctl->do_full);
+      // V(j), then K(j + 1): the products that hand the stages back come in that order
+      int ks = 1;
+      uint32_t kphase = 1;
       for (int j = 0; j < n_kv; ++j) {
-        const int s = j & 1;
-        if (!mbar_wait_bounded(smem_u32(&ctl->kv_empty[s]), ((j >> 1) & 1) ^ 1u, wctx, 41, j)) break;
-        const uint32_t full = smem_u32(&ctl->kv_full[s]);
-        const uint32_t k_tile = ring + s * 2 * kTileBytes, v_tile = k_tile + kTileBytes;
-        mbar_arrive_expect_tx(full, 2 * kTileBytes);
-        const int row = tok0 + j * kT;
-        tma_load_2d(k_tile, &tm_k, hk * kD, row, full);
-        tma_load_2d(k_tile + 16384, &tm_k, hk * kD + 64, row, full);
-        tma_load_2d(v_tile, &tm_v, hk * kD, row, full);
-        tma_load_2d(v_tile + 16384, &tm_v, hk * kD + 64, row, full);
+        if (!mbar_wait_bounded(smem_u32(&ctl->v_empty[j & 1]), ((j >> 1) & 1) ^ 1u, wctx, 41, j)) break;
+        load(v_ring + (j & 1) * kTileBytes, tm_v, hk * kD, tok0 + j * kT, &ctl->v_full[j & 1]);
+        if (j + 1 == n_kv) break;
+        if (!mbar_wait_bounded(smem_u32(&ctl->kv_empty[ks]), kphase, wctx, 41, j + 1)) break;
+        load(k_ring + ks * kTileBytes, tm_k, hk * kD, tok0 + (j + 1) * kT, &ctl->kv_full[ks]);
+        if (++ks == kKStages) {
+          ks = 0;
+          kphase ^= 1u;
+        }
       }
     }
   } else if (warp == kWarpMma) {
     if (lane == 0) {
       const uint32_t idesc_kk = umma_idesc_bf16_f32(kT, kT);             // both operands K-major
       const uint32_t idesc_kmn = umma_idesc_bf16_f32(kT, kD) | (1u << 16);  // B MN-major
-      const uint64_t d_q = desc_kmajor(q_tile, 0), d_do = desc_kmajor(do_tile, 0), d_ring = desc_kmajor(ring, 0),
-                     d_ring_mn = desc_mnmajor(ring, 0);
-      constexpr uint64_t kStage = (2 * kTileBytes) >> 4, kTile = kTileBytes >> 4;
-      auto issue_s = [&](int j) {      // S = Q K^T
-        const uint64_t dk = d_ring + (j & 1) * kStage;
+      const uint64_t d_q = desc_kmajor(q_tile, 0), d_do = desc_kmajor(do_tile, 0), d_k = desc_kmajor(k_ring, 0),
+                     d_k_mn = desc_mnmajor(k_ring, 0), d_v = desc_kmajor(v_ring, 0);
+      constexpr uint64_t kTile = kTileBytes >> 4;
+      auto issue_s = [&](int j, int ks) {      // S = Q K^T
+        const uint64_t dk = d_k + ks * kTile;
 #pragma unroll
         for (int kk = 0; kk < kD / 16; ++kk)
           umma_bf16<1>(tmem_base + (j & 1) * 128, d_q + kstep(kk), dk + kstep(kk), idesc_kk, kk > 0 ? 1u : 0u);
         umma_commit<1>(smem_u32(&ctl->s_full[j & 1]));
       };
       auto issue_dp = [&](int j) {     // dP = dO V^T
-        const uint64_t dv = d_ring + (j & 1) * kStage + kTile;
+        const uint64_t dv = d_v + (j & 1) * kTile;
 #pragma unroll
         for (int kk = 0; kk < kD / 16; ++kk)
           umma_bf16<1>(tmem_dp, d_do + kstep(kk), dv + kstep(kk), idesc_kk, kk > 0 ? 1u : 0u);
         umma_commit<1>(smem_u32(&ctl->dp_full));
+        umma_commit<1>(smem_u32(&ctl->v_empty[j & 1]));
       };
       bool ok = mbar_wait_bounded(smem_u32(&ctl->qdo_full), 0, wctx, 42, 0) &&
                 mbar_wait_bounded(smem_u32(&ctl->kv_full[0]), 0, wctx, 43, 0);
       if (ok) {
         tc_fence_after_sync();
-        issue_s(0);
+        issue_s(0, 0);
+        ok = mbar_wait_bounded(smem_u32(&ctl->do_full), 0, wctx, 42, 1) &&
+             mbar_wait_bounded(smem_u32(&ctl->v_full[0]), 0, wctx, 43, 0);
+      }
+      if (ok) {
+        tc_fence_after_sync();
         issue_dp(0);
       }
+      int ks = 0;                      // stage of K(j)
+      uint32_t kphase = 0;             // of K(j + 1)
       for (int j = 0; j < n_kv && ok; ++j) {
+        const int ks_next = ks + 1 == kKStages ? 0 : ks + 1;
+        if (ks_next == 0) kphase ^= 1u;
         if (j + 1 < n_kv) {
           // S(j + 1) goes over dS(j - 1), whose product was issued an iteration ago; the tensor
           // core executes in issue order
-          ok = mbar_wait_bounded(smem_u32(&ctl->kv_full[(j + 1) & 1]), ((j + 1) >> 1) & 1, wctx, 43, j + 1);
+          ok = mbar_wait_bounded(smem_u32(&ctl->kv_full[ks_next]), kphase, wctx, 43, j + 1);
           if (!ok) break;
           tc_fence_after_sync();
-          issue_s(j + 1);
-          ok = mbar_wait_bounded(smem_u32(&ctl->dp_read), j & 1, wctx, 47, j);
+          issue_s(j + 1, ks_next);
+          ok = mbar_wait_bounded(smem_u32(&ctl->v_full[(j + 1) & 1]), ((j + 1) >> 1) & 1, wctx, 43, j + 1) &&
+               mbar_wait_bounded(smem_u32(&ctl->dp_read), j & 1, wctx, 47, j);
           if (!ok) break;
           tc_fence_after_sync();
           issue_dp(j + 1);
@@ -256,13 +284,14 @@ bwd_dq(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v
         ok = mbar_wait_bounded(smem_u32(&ctl->ds_full[j & 1]), (j >> 1) & 1, wctx, 44, j);
         if (!ok) break;
         tc_fence_after_sync();
-        const uint64_t dk = d_ring_mn + (j & 1) * kStage;
+        const uint64_t dk = d_k_mn + ks * kTile;
 #pragma unroll
         for (int kk = 0; kk < kT / 16; ++kk)  // dQ += dS K
           umma_bf16_ts(tmem_dq, tmem_base + (j & 1) * 128 + tcol(kk), dk + mnstep(kk), idesc_kmn,
                        (j > 0 || kk > 0) ? 1u : 0u);
-        umma_commit<1>(smem_u32(&ctl->kv_empty[j & 1]));
+        umma_commit<1>(smem_u32(&ctl->kv_empty[ks]));
         if (j + 1 == n_kv) umma_commit<1>(smem_u32(&ctl->acc_full));
+        ks = ks_next;
       }
     }
   } else {
@@ -358,8 +387,9 @@ bwd_dq(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v
 // stages of (Q, dO), dS^T.
 // ------------------------------------------------------------------------------------------------
 struct CtlDkv {
-  uint64_t kv_full;                  // K and V tiles loaded (once)
-  uint64_t qdo_full[2], qdo_empty[2];
+  uint64_t kv_full, v_full;          // K tile loaded, V tile loaded (once)
+  uint64_t qdo_full[2], qdo_empty[2];  // Q tiles: read by S^T and, last of all, by dK
+  uint64_t do_full[2], do_empty[2];    // dO tiles: read by dP^T and dV
   uint64_t st_full;                  // S^T ready in TMEM
   uint64_t p_full;                   // P^T written over S^T (count: softmax warps)
   uint64_t dp_full, dp_read;         // dP^T ready / read into registers (count: softmax warps)
@@ -398,9 +428,12 @@ bwd_dkv(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_
 
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&ctl->kv_full), 1);
+    mbar_init(smem_u32(&ctl->v_full), 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(smem_u32(&ctl->qdo_full[s]), 1);
       mbar_init(smem_u32(&ctl->qdo_empty[s]), 1);
+      mbar_init(smem_u32(&ctl->do_full[s]), 1);
+      mbar_init(smem_u32(&ctl->do_empty[s]), 1);
     }
     mbar_init(smem_u32(&ctl->st_full), 1);
     mbar_init(smem_u32(&ctl->p_full), kSoftThreads / 32);
@@ -424,24 +457,30 @@ bwd_dkv(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_
 
   if (warp == kWarpTma) {
     if (lane == 0) {
-      const uint32_t f = smem_u32(&ctl->kv_full);
-      mbar_arrive_expect_tx(f, 2 * kTileBytes);
-      tma_load_2d(k_tile, &tm_k, hk * kD, tok0 + kv_row0, f);
-      tma_load_2d(k_tile + 16384, &tm_k, hk * kD + 64, tok0 + kv_row0, f);
-      tma_load_2d(v_tile, &tm_v, hk * kD, tok0 + kv_row0, f);
-      tma_load_2d(v_tile + 16384, &tm_v, hk * kD + 64, tok0 + kv_row0, f);
-      for (int n = 0; n < n_iter; ++n) {
+      auto load = [&](uint32_t dst, const CUtensorMap& tm, int col, int row, uint64_t* bar) {
+        const uint32_t full = smem_u32(bar);
+        mbar_arrive_expect_tx(full, kTileBytes);
+        tma_load_2d(dst, &tm, col, row, full);
+        tma_load_2d(dst + 16384, &tm, col + 64, row, full);
+      };
+      auto load_q = [&](int n) {
         const int h = hk * group + n / n_q, qt = qt0 + n % n_q, s = n & 1;
-        if (!mbar_wait_bounded(smem_u32(&ctl->qdo_empty[s]), ((n >> 1) & 1) ^ 1u, wctx, 51, n)) break;
-        const uint32_t full = smem_u32(&ctl->qdo_full[s]);
-        const uint32_t q_tile = ring + s * 2 * kTileBytes, do_tile = q_tile + kTileBytes;
-        mbar_arrive_expect_tx(full, 2 * kTileBytes);
-        const int row = tok0 + qt * kT;
-        tma_load_2d(q_tile, &tm_q, h * kD, row, full);
-        tma_load_2d(q_tile + 16384, &tm_q, h * kD + 64, row, full);
-        tma_load_2d(do_tile, &tm_do, h * kD, row, full);
-        tma_load_2d(do_tile + 16384, &tm_do, h * kD + 64, row, full);
-      }
+        if (!mbar_wait_bounded(smem_u32(&ctl->qdo_empty[s]), ((n >> 1) & 1) ^ 1u, wctx, 51, n)) return false;
+        load(ring + s * 2 * kTileBytes, tm_q, h * kD, tok0 + qt * kT, &ctl->qdo_full[s]);
+        return true;
+      };
+      auto load_do = [&](int n) {
+        const int h = hk * group + n / n_q, qt = qt0 + n % n_q, s = n & 1;
+        if (!mbar_wait_bounded(smem_u32(&ctl->do_empty[s]), ((n >> 1) & 1) ^ 1u, wctx, 51, n)) return false;
+        load(ring + (s * 2 + 1) * kTileBytes, tm_do, h * kD, tok0 + qt * kT, &ctl->do_full[s]);
+        return true;
+      };
+      load(k_tile, tm_k, hk * kD, tok0 + kv_row0, &ctl->kv_full);
+      bool ok = n_iter > 0 && load_q(0);
+      load(v_tile, tm_v, hk * kD, tok0 + kv_row0, &ctl->v_full);
+      ok = ok && load_do(0);
+      // dO(n - 2) is handed back by dV(n - 2), Q(n - 2) by dK(n - 2)
+      for (int n = 1; n < n_iter && ok; ++n) ok = load_do(n) && load_q(n);
     }
   } else if (warp == kWarpMma) {
     if (lane == 0) {
@@ -469,6 +508,11 @@ bwd_dkv(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_
       if (ok) {
         tc_fence_after_sync();
         issue_st(0);
+        ok = mbar_wait_bounded(smem_u32(&ctl->v_full), 0, wctx, 52, 1) &&
+             mbar_wait_bounded(smem_u32(&ctl->do_full[0]), 0, wctx, 53, 0);
+      }
+      if (ok) {
+        tc_fence_after_sync();
         issue_dpt(0);
       }
       for (int n = 0; n < n_iter && ok; ++n) {
@@ -479,13 +523,15 @@ bwd_dkv(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_
 #pragma unroll
         for (int kk = 0; kk < kT / 16; ++kk)  // dV += P^T dO
           umma_bf16_ts(tmem_dv, tmem_st + tcol(kk), ddo + mnstep(kk), idesc_kmn, (n > 0 || kk > 0) ? 1u : 0u);
+        umma_commit<1>(smem_u32(&ctl->do_empty[n & 1]));
         if (n + 1 < n_iter) {
           // S^T(n + 1) goes over P^T(n): the tensor core executes in issue order
           ok = mbar_wait_bounded(smem_u32(&ctl->qdo_full[(n + 1) & 1]), ((n + 1) >> 1) & 1, wctx, 53, n + 1);
           if (!ok) break;
           tc_fence_after_sync();
           issue_st(n + 1);
-          ok = mbar_wait_bounded(smem_u32(&ctl->dp_read), n & 1, wctx, 57, n);
+          ok = mbar_wait_bounded(smem_u32(&ctl->do_full[(n + 1) & 1]), ((n + 1) >> 1) & 1, wctx, 53, n + 1) &&
+               mbar_wait_bounded(smem_u32(&ctl->dp_read), n & 1, wctx, 57, n);
           if (!ok) break;
           tc_fence_after_sync();
           issue_dpt(n + 1);
@@ -677,7 +723,7 @@ extern "C" int ka_attention_bwd(const void* q, long long q_stride, const void* k
   // q, k, v and d_o are checked with their tensor maps; o is read by the delta kernel alone
   if ((reinterpret_cast<uintptr_t>(o) & 15u) != 0 || o_stride % 8 != 0) return -2;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  constexpr int kSmemDq = 6 * kTileBytes + 256;
+  constexpr int kSmemDq = (4 + kKStages) * kTileBytes + 256;
   constexpr int kSmemDkv = 7 * kTileBytes + 2304;
   static_assert(sizeof(CtlDq) <= 256 && sizeof(CtlDkv) <= 2304 && kSmemDkv <= 227 * 1024, "shared memory layout");
   constexpr int kSmem = kSmemDkv > kSmemDq ? kSmemDkv : kSmemDq;
