@@ -70,10 +70,12 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// Arrive on a barrier that lives in another CTA of the cluster (shared::cluster address).
+// Arrive on a barrier that lives in another CTA of the cluster (shared::cluster address), for handing over TMEM:
+// what the arriving threads did there is complete (tcgen05.wait, tcgen05.fence). The release is CTA-wide, the default:
+// one at cluster scope first waits for all of the thread's global stores, more than a thousand cycles behind an epilogue
+// or under load, and orders memory that nobody reads here.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar)
-               : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
