@@ -83,7 +83,7 @@ def attention_backward(q, k, v, out, d_out, lse, *, causal: bool = True, scale: 
     dq = torch.empty(b, l, hq, d, dtype=torch.bfloat16, device=q.device)
     dk = torch.empty(b, l, hkv, d, dtype=torch.bfloat16, device=q.device)
     dv = torch.empty(b, l, hkv, d, dtype=torch.bfloat16, device=q.device)
-    delta = torch.empty(b, hq, l, dtype=torch.float32, device=q.device)
+    delta = torch.empty(b * hq * l + 2, dtype=torch.float32, device=q.device)   # and two counters
     lse = lse.contiguous()
     rc = _native.cuda().ka_attention_bwd(
         q.data_ptr(), q.stride(1), k.data_ptr(), k.stride(1), v.data_ptr(), v.stride(1), out.data_ptr(),

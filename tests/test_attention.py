@@ -109,3 +109,28 @@ def test_gpu_attention_backward_reads_views_of_a_fused_projection(cuda_device, c
     strided = attention_backward(*views, wide[:, :, :hq], wide[:, :, hq:], lse, causal=causal)
     packed = attention_backward(*(t.contiguous() for t in views), o, wide[:, :, hq:].contiguous(), lse, causal=causal)
     assert all(torch.equal(s, p) for s, p in zip(strided, packed))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("b,l,hq,hkv,causal", [(40, 130, 8, 2, True), (200, 70, 4, 4, True), (20, 300, 8, 8, False),
+                                                (12, 513, 8, 4, True), (150, 128, 2, 1, False)])
+def test_gpu_attention_backward_of_many_tiles(cuda_device, b, l, hq, hkv, causal):
+    """More tiles than SMs: CTAs that take one tile after the other give the bits of a sequence on its own, which has a
+    CTA per tile, and the gradients of the fp32 oracle."""
+    from kernel_align_b200.ops.attention import attention_backward
+    from kernel_align_b200.ops.gemm import check_status
+
+    g = torch.Generator(device=cuda_device).manual_seed(b + l)
+    q, k, v, d_o = (torch.randn(b, l, h, 128, device=cuda_device, generator=g).to(torch.bfloat16) for h in (hq, hkv, hkv, hq))
+    o, lse = attention(q, k, v, causal=causal, return_lse=True)
+    got = attention_backward(q, k, v, o, d_o, lse, causal=causal)
+    check_status(cuda_device)
+    for again in range(2):
+        assert all(torch.equal(x, y) for x, y in zip(got, attention_backward(q, k, v, o, d_o, lse, causal=causal)))
+    for i in (0, b // 2, b - 1):
+        one = attention_backward(*(t[i:i + 1] for t in (q, k, v, o, d_o, lse)), causal=causal)
+        assert all(torch.equal(x[i:i + 1], y) for x, y in zip(got, one)), i
+    qr, kr, vr = (t[-2:].float().requires_grad_() for t in (q, k, v))
+    _sdpa(qr, kr, vr, causal).backward(d_o[-2:].float())
+    for x, ref in zip(got, (qr.grad, kr.grad, vr.grad)):
+        assert (x[-2:].float() - ref).abs().max().item() <= 0.03 * ref.abs().max().item() + 1e-3
