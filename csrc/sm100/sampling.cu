@@ -1979,9 +1979,10 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
 //     (-inf, the type's lowest value, -1e4) need not be counted. A look at the row's first elements shifts the 64 binades for
 //     rows of large values; if something with a mass is left out all the same, the row is counted again with the binades
 //     that its maximum asks for, and if that leaves out a nonzero value with a mass, one CTA takes the radix descent.
-// [200, 128256] ~ N(0, 2), T = 1, top_p = 0.9: 58.4 us with one CTA per row, 46.7 us now: counting takes 31k to 50k cycles of an
-// SM with three half rows, what follows 29k, which is latency (searches 10k, barriers 6k, the draw 12k).
-constexpr int kPartThreads = 512, kPartWarps = kPartThreads / 32;
+// [200, 128256] ~ N(0, 2), T = 1, top_p = 0.9: 58.4 us with one CTA per row, 41.6 us now: counting takes 31k cycles of an
+// SM with three half rows, the rest is latency (searches, barriers, the draw).
+// With 512 threads (40 registers each, three CTAs) the loops spilled: 46.8 us for 200 rows of 128256, 41.6 with 384; 320 41.9, 288 41.8.
+constexpr int kPartThreads = 384, kPartWarps = kPartThreads / 32;
 constexpr int kPartsPerCta = 2;
 constexpr int kMaxPartCtas = 8;
 constexpr int kPartBinades = 64;
@@ -2169,9 +2170,8 @@ __device__ __forceinline__ void part_count(const __nv_bfloat16* rp, int v, uint3
   __syncthreads();
   // which units of 128 counters are not empty
   const int lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-  for (int i = 0; i < kPartUnits / kPartWarps; ++i) {
-    const int u = warp + i * kPartWarps;
+#pragma unroll 4
+  for (int u = warp; u < kPartUnits; u += kPartWarps) {
     const uint2 c0 = *reinterpret_cast<const uint2*>(hist + u * 256 + lane * 8);
     const uint2 c1 = *reinterpret_cast<const uint2*>(hist + kPartHistBytes + u * 256 + lane * 8);
     if (__any_sync(0xffffffffu, (c0.x | c0.y | c1.x | c1.y) != 0) && lane == 0)
@@ -2706,10 +2706,10 @@ sample_parts_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stri
 // How many CTAs share a row, 0 for the one of 1024 threads that counts and draws by itself. Counting is bound by the
 // atomics an SM can do, so more CTAs than SMs help only to deal rows that do not fill a whole number of rounds, and what is behind the
 // counting (searches, two barriers of the cluster, the draw: 14 us) is paid by any number of CTAs. us, one CTA per row
-// of 1024 threads / parts, top_p = 0.9: 8 rows of 128256 29.1 / 17.1 (8 CTAs), 30 rows 29.1 / 18.8 (4; 8 CTAs 21.1), 64 rows
-// 29.7 / 24.8 (2), 148 rows 31.3 / 35.2; 32000 columns: 8 rows 15.7 / 15.1, 64 rows 15.7 / 17.3. With more rows than SMs
-// that kernel needs another round, parts have them all resident, three per SM: 200 rows of 128256 58.3 / 46.4 (2 CTAs; 1: 51.9),
-// 256 59.0 / 52.4 (1; 2: 60.8); 32000 columns 30.4 / 25.5 (1; 2: 27.1), 1000 columns 21.9 / 16.8.
+// of 1024 threads / parts, top_p = 0.9: 8 rows of 128256 29.1 / 16.4 (8 CTAs), 30 rows 29.1 / 18.7 (4), 64 rows
+// 29.7 / 25.0 (2), 148 rows 31.3 / 35 (2, with 512 threads); 32000 columns: 8 rows 15.7 / 14.6, 64 rows 15.7 / 17.3. With more
+// rows than SMs that kernel needs another round, parts have them all resident, three per SM: 200 rows of 128256 58.3 / 41.7
+// (2 CTAs), 256 59.0 / 49.1 (1; 2 with 512 threads: 60.8); 32000 columns 30.4 / 23.8 (1), 1000 columns 21.9 / 16.8.
 inline int part_ctas(int rows, int v, int sms) {
   // a sub-part's vectors are rounded up, its ends have up to seven scalars each
   auto fits = [&](int ctas) { return v / (ctas * kPartsPerCta) + 32 <= kPartMaxElems; };
