@@ -1979,7 +1979,7 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
 //     (-inf, the type's lowest value, -1e4) need not be counted. A look at the row's first elements shifts the 64 binades for
 //     rows of large values; if something with a mass is left out all the same, the row is counted again with the binades
 //     that its maximum asks for, and if that leaves out a nonzero value with a mass, one CTA takes the radix descent.
-// [200, 128256] ~ N(0, 2), T = 1, top_p = 0.9: 58.4 us with one CTA per row, 41.6 us now: counting takes 31k cycles of an
+// [200, 128256] ~ N(0, 2), T = 1, top_p = 0.9: 58.4 us with one CTA per row, 41.2 us now: counting takes 31k cycles of an
 // SM with three half rows, the rest is latency (searches, barriers, the draw).
 // With 512 threads (40 registers each, three CTAs) the loops spilled: 46.8 us for 200 rows of 128256, 41.6 with 384; 320 41.9, 288 41.8.
 constexpr int kPartThreads = 384, kPartWarps = kPartThreads / 32;
@@ -2099,7 +2099,9 @@ __device__ __forceinline__ uint32_t part_base(float reach) {
 __device__ __forceinline__ void part_count(const __nv_bfloat16* rp, int v, uint32_t base, int rank, int ctas, unsigned char* hist,
                                            PartSmem& s) {
   using T = __nv_bfloat16;
-  constexpr int kTs = kPartThreads / kPartsPerCta, kU = 4;
+  // Three vectors in flight per thread: 200 / 256 rows of 128256 take 41.2 / 48.3 us, with four 42.1 / 49.1, with two 40.3 / 49.4
+  // in another run, so 256 rows lose; short rows do not care (256 x 8000: 17.9 against 17.7).
+  constexpr int kTs = kPartThreads / kPartsPerCta, kU = 3;
   const int tid = threadIdx.x, sub = tid / kTs, t = tid % kTs;
   const PartRange pr = part_range(rank * kPartsPerCta + sub, ctas * kPartsPerCta, row_head(rp, v), v);
   const int n_vec = pr.n_vec;
