@@ -111,13 +111,13 @@ def _split_pays(m: int, n: int, k: int) -> bool:
     """Whether one rank that sums its eight K slices itself makes them units of their own
     (``ka_gemm_split8``: eight times as many units, a pass over the partials) or keeps a tile's slices on one
     CTA pair (``ka_gemm_tree8``). Measured split / kept in us on 74 pairs, calls after one another (19 us is what
-    the host takes for one), tiles counted as 256 x 256: 4 tiles: 19 / 27 (K = 1024), 19 / 33 (4096); 16 tiles:
-    20 / 27 (1024), 20 / 35 (4096), 37 / 67 (14336), 58 / 98 (28672); 32 tiles: 32 / 35 (4096), 37 / 46 (6144),
-    61 / 87 (14336), 101 / 147 (28672); 48 tiles: 45 / 45 (4096), 49 / 54 (6144), 83 / 95 (14336), 149 / 165 (28672);
-    64 tiles: 99 / 101 (14336), 180 / 185 (28672). One row instead of 128 or 512, whose tiles are mostly
-    padding: 16 tiles 42 / 49 (14336), 63 / 75 (28672); 20 tiles 49 / 60, 84 / 98; 32 tiles 72 / 98, 109 / 129. With
-    more tiles the partials outgrow what the rest saves (256 tiles: 196 / 185 at 6144, 688 / 706 at 28672,
-    with half a gigabyte of scratch)."""
+    the host takes for one, so K = 1024 tells little), tiles counted as 256 x 256: 16 tiles: 27 / 34 (K = 4096),
+    34 / 83 (14336), 55 / 153 (28672); 24 tiles: 21 / 20 (1024), 26 / 34 (4096), 47 / 84 (14336); 32 tiles: 23 / 20
+    (1024), 29 / 34 (4096), 58 / 86 (14336), 103 / 157 (28672); 48 tiles: 33 / 32 (1024), 44 / 46 (4096), 51 / 56
+    (6144), 85 / 99 (14336), 148 / 175 (28672); 64 tiles: 39 / 32 (1024), 53 / 49 (4096), 63 / 60 (6144), 102 / 105
+    (14336), 180 / 188 (28672). One row instead, whose tiles are mostly padding: 20 tiles 25 / 34 (4096),
+    83 / 157 (28672); 32 tiles 29 / 38, 107 / 171. With more tiles the partials outgrow what the rest saves, with half a
+    gigabyte of scratch at 256 of them."""
     tiles = -(-m // 256) * -(-n // 256)
     return tiles <= 24 or (tiles <= 48 and k >= 4096) or (tiles <= 64 and k >= 12288)
 
@@ -127,7 +127,8 @@ def _tree_pays(m: int, n: int, k: int, num_sms: int) -> bool:
     stages them as several ranks do (``ka_gemm_reduce_scatter``). The bits are the same.
 
     Staged slices spread over all pairs but cost fences, flags and the wait for them. Measured on
-    148 SMs, staged / own in us, tiles counted as 256 x 256: 256 tiles: 385 / 156 (K = 4096), 1025 / 738 (28672);
+    148 SMs, staged / own in us, tiles counted as 256 x 256: 256 tiles: 385 / 156 (K = 4096; 139 since TMEM is
+    handed back without waiting for stores), 1025 / 738 (28672);
     32 tiles: 72 / 32 (4096), 109 / 61 (14336), 150 / 101 (28672); 16 tiles: 48 / 20 (4096), 57 / 24 (6144),
     70 / 37 (14336), 101 / 58 (28672); 4 tiles: 39 / 19 (4096). A slice round of a kept tile takes about 5.4e-3 us
     per K column, staging about 20 us plus 1.2 us per tile; the rule compares the two."""
