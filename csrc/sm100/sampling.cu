@@ -2436,8 +2436,9 @@ sample_parts_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stri
   const int rank = static_cast<int>(cluster_rank()), row = static_cast<int>(blockIdx.x) / ctas;
   const T* rp = logits + static_cast<long long>(row) * row_stride;
   const bool has_k = top_k > 0 && top_k < v;
+  if (ctas > 1) cluster_arrive_release();          // waited for before the first remote access
 
-  // a look at the row's first 4096 elements, for the magnitudes to count
+  // a look at the row's first 8 * kPartThreads elements, for the magnitudes to count
   uint32_t look = 0xFFFFFFFFu;
   {
     const int head = row_head(rp, v);
@@ -2474,6 +2475,7 @@ sample_parts_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stri
     }
     part_count(rp, v, base, rank, ctas, hist, s);
     __syncthreads();
+    if (attempt == 0 && ctas > 1) cluster_wait_acquire();            // every CTA of the cluster runs
     if (tid < ctas * kInfoWords)
       st_remote_u32(map_to_cta(reinterpret_cast<uint32_t*>(&s.info[rank]) + tid % kInfoWords, tid / kInfoWords),
                     reinterpret_cast<const uint32_t*>(&s.mine)[tid % kInfoWords]);
