@@ -3,7 +3,9 @@
 ``cuda()`` returns the sm_100a kernel library and raises if it is missing: on a GPU host the
 hand-written kernels are the only code path, there is no silent PyTorch fallback.
 ``cpu()`` returns the C++ CPU library (oracle for the tests and the CPU device path).
-``torch_ops()`` returns the extension module with the operators that are C++ autograd nodes.
+``torch_ops()`` returns the extension module with the operators that are C++ autograd nodes, or None: it is
+made for one torch, which an isolated package build does not have, and the operators then reach the same kernels
+through ``cuda()``.
 """
 from __future__ import annotations
 
@@ -76,6 +78,15 @@ def cuda() -> ctypes.CDLL:
         c_int,
         [c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p],
     )
+    _bind(lib, "ka_grpo_advantages", c_int, [c_void_p, c_void_p, c_int, c_int, c_float, c_void_p])
+    _bind(
+        lib,
+        "ka_grpo_loss_fwd",
+        c_int,
+        [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_float, c_float, c_int,
+         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
+    )
+    _bind(lib, "ka_grpo_loss_bwd", c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p])
     # prototypes are set here, once: setting them costs a call several microseconds
     p, i, ll, f, ull = c_void_p, c_int, c_longlong, c_float, c_ulonglong
     _bind(lib, "ka_rmsnorm", c_int, [p, p, p, p, p, i, i, f, i, p])
@@ -110,12 +121,11 @@ def cuda() -> ctypes.CDLL:
 
 @lru_cache(maxsize=None)
 def torch_ops():
-    """The extension module with the operators that are C++ autograd nodes, bound to the kernels of :func:`cuda`."""
+    """The extension module with the operators that are C++ autograd nodes, bound to the kernels of :func:`cuda`; None
+    if there is none for this torch and it cannot be built."""
     path = _build.build_torch()
     if path is None or not path.exists():
-        raise NativeLibraryMissing(
-            "_ka_torch.so is not built; run `python -m kernel_align_b200._build` on a host with g++"
-        )
+        return None
     spec = importlib.util.spec_from_file_location("_ka_torch", str(path))
     mod = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(mod)

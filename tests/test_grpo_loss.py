@@ -1,7 +1,13 @@
 """GRPO objective: CPU library and CUDA kernels against an autograd PyTorch reference."""
+import os
+import shutil
+import subprocess
+import sys
+
 import pytest
 import torch
 
+from kernel_align_b200 import _native
 from kernel_align_b200.ops.grpo_loss import group_advantages, grpo_loss
 
 
@@ -68,6 +74,38 @@ def test_grpo_loss_follows_its_inputs_and_not_the_default_device():
         got, stats = grpo_loss(ln, lo, adv, return_stats=True)
         assert torch.equal(grpo_loss(ln, lo, adv), want)
     assert torch.equal(got, want) and torch.equal(stats, want_stats)
+
+
+def test_an_installed_package_without_the_module_has_the_loss(tmp_path):
+    """A package built without torch carries the two plain libraries and no sources: the operators take them."""
+    package = os.path.dirname(_native.__file__)
+    shutil.copytree(package, tmp_path / "kernel_align_b200", ignore=shutil.ignore_patterns("__pycache__", "_ka_torch*", "*.hash"))
+    code = ("import torch; from kernel_align_b200 import _native; from kernel_align_b200.ops import grpo_loss as g\n"
+            "assert _native.torch_ops() is None and _native.cuda().ka_grpo_loss_fwd.argtypes\n"
+            "x = torch.randn(2, 3, requires_grad=True); g.grpo_loss(x, x.detach(), torch.ones(2)).backward(); print(x.grad.shape)")
+    r = subprocess.run([sys.executable, "-c", code], cwd=tmp_path, capture_output=True, text=True, timeout=300,
+                       env={**os.environ, "PYTHONPATH": str(tmp_path)})
+    assert r.returncode == 0 and "torch.Size([2, 3])" in r.stdout, r.stderr
+
+
+@pytest.mark.gpu
+def test_grpo_loss_gpu_without_the_module(cuda_device, monkeypatch):
+    """The Python node reaches the same kernels: the same bits, and what is refused stays refused."""
+    ln, lo, lr, rewards, mask = _case(cuda_device)
+    got = []
+    for gone in (False, True):
+        if gone:
+            monkeypatch.setattr(_native, "torch_ops", lambda: None)
+        assert (_native.torch_ops() is None) == gone
+        x = ln.clone().requires_grad_()
+        adv = group_advantages(rewards, 4)
+        loss, stats = grpo_loss(x, lo, adv, mask=mask, logp_ref=lr, beta=0.04, return_stats=True)
+        got.append([adv, loss.detach(), stats, *torch.autograd.grad(loss, x)])
+        for bad in ((x, lo.cpu(), adv), (x[0], lo[0], adv)):
+            with pytest.raises((RuntimeError, ValueError)):
+                grpo_loss(*bad)
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+    _check(cuda_device)
 
 
 @pytest.mark.gpu
