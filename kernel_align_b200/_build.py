@@ -107,28 +107,50 @@ def build_cpu(force: bool = False) -> Path | None:
     return CPU_LIB
 
 
-def build_torch(force: bool = False) -> Path | None:
-    """Compile ``csrc/torch/*.cpp`` into the extension module ``_ka_torch.so`` (C++ autograd nodes)."""
+def torch_missing() -> str | None:
+    """Why ``_ka_torch.so`` cannot be compiled on this host, or None if it can."""
     try:
         import torch
-    except ImportError:      # an isolated package build: the first call that needs the module builds it
-        return TORCH_LIB if TORCH_LIB.exists() else None
+    except ImportError:
+        return "torch is not installed"
+    if torch.version.cuda is None or not (Path(torch.__file__).parent / "lib" / "libc10_cuda.so").exists():
+        return "this torch was built without CUDA"
+    if _cuda_include() is None:
+        return "no CUDA headers (cuda_runtime_api.h) under CUDA_HOME, beside nvcc or under /usr/local/cuda"
+    if shutil.which("g++") is None:
+        return "no g++"
+    return None
+
+
+def _cuda_include() -> Path | None:
+    nvcc = _nvcc()
+    homes = [os.environ.get("CUDA_HOME"), nvcc and Path(nvcc).resolve().parent.parent, "/usr/local/cuda"]
+    for home in homes:
+        if home and (Path(home) / "include" / "cuda_runtime_api.h").exists():
+            return Path(home) / "include"
+    return None
+
+
+def build_torch(force: bool = False) -> Path | None:
+    """Compile ``csrc/torch/*.cpp`` into the extension module ``_ka_torch.so`` (C++ autograd nodes). None where that is not
+    possible (:func:`torch_missing`): the operators then reach the kernels from Python."""
     srcs = sorted((CSRC / "torch").glob("*.cpp"))
-    if not srcs:
+    if not srcs or torch_missing() is not None:
         return TORCH_LIB if TORCH_LIB.exists() else None
+    import torch
+
     inc, lib = Path(torch.__file__).parent / "include", Path(torch.__file__).parent / "lib"
-    cuda_home = os.environ.get("CUDA_HOME") or "/usr/local/cuda"
     flags = ["-O2", "-std=c++17", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
     digest = _digest(srcs, [*flags, torch.__version__, sys.version])
     if not force and _stamp_ok(TORCH_LIB, digest):
         return TORCH_LIB
-    cxx = shutil.which("g++")
-    if cxx is None:
-        return TORCH_LIB if TORCH_LIB.exists() else None
     LIB_DIR.mkdir(parents=True, exist_ok=True)
-    _run([cxx, *flags, "-shared", "-o", str(TORCH_LIB), *[str(s) for s in srcs], f"-I{inc}",
-          f"-I{inc / 'torch' / 'csrc' / 'api' / 'include'}", f"-I{sysconfig.get_paths()['include']}",
-          f"-I{cuda_home}/include", f"-L{lib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"])
+    try:
+        _run(["g++", *flags, "-shared", "-o", str(TORCH_LIB), *[str(s) for s in srcs], f"-I{inc}",
+              f"-I{inc / 'torch' / 'csrc' / 'api' / 'include'}", f"-I{sysconfig.get_paths()['include']}",
+              f"-I{_cuda_include()}", f"-L{lib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"])
+    except RuntimeError:     # the compiler's message is on stderr; the other libraries do not need this one
+        return None
     TORCH_LIB.with_suffix(".hash").write_text(digest)
     return TORCH_LIB
 
@@ -166,8 +188,8 @@ def sanitizer_runtime() -> str | None:
 
 def build_all(force: bool = False, verbose: bool = False) -> None:
     build_cpu(force)
-    build_torch(force)
     build_cuda(force, verbose)
+    build_torch(force)
 
 
 if __name__ == "__main__":

@@ -25,6 +25,7 @@ def collect() -> dict:
     info["libka_sm100"] = str(_build.CUDA_LIB) if _build.CUDA_LIB.exists() else None
     info["libka_cpu"] = str(_build.CPU_LIB) if _build.CPU_LIB.exists() else None
     info["ka_torch"] = str(_build.TORCH_LIB) if _build.TORCH_LIB.exists() else None
+    info["ka_torch_missing"] = _build.torch_missing()
     gpus = []
     if torch.cuda.is_available():
         for i in range(torch.cuda.device_count()):
@@ -84,7 +85,8 @@ def main(argv=None) -> int:
         print(f"kernel_align_b200 {info['version']}  (torch {info['torch']}, CUDA runtime {info['cuda_runtime']})")
         print(f"  sm_100a kernel library : {info['libka_sm100'] or 'not built'}   (nvcc: {info['nvcc'] or 'not found'})")
         print(f"  C++ CPU library        : {info['libka_cpu'] or 'not built'}   (g++: {info['cxx'] or 'not found'})")
-        print(f"  autograd nodes (C++)   : {info['ka_torch'] or 'not built'}   (g++: {info['cxx'] or 'not found'})")
+        print(f"  autograd nodes (C++)   : {info['ka_torch'] or 'not built: the Python ones are used'}   "
+              f"(g++: {info['cxx'] or 'not found'}{'; cannot be built: ' + info['ka_torch_missing'] if info['ka_torch_missing'] else ''})")
         if info["gpus"]:
             for gpu in info["gpus"]:
                 mark = "ok" if gpu["supported"] else "unsupported: the kernels are written for sm_100a"
