@@ -13,6 +13,7 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+import threading
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -23,7 +24,6 @@ OBJ_DIR = ROOT / "build" / "obj"
 
 CUDA_LIB = LIB_DIR / "libka_sm100.so"
 CPU_LIB = LIB_DIR / "libka_cpu.so"
-TORCH_LIB = LIB_DIR / "_ka_torch.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -107,8 +107,19 @@ def build_cpu(force: bool = False) -> Path | None:
     return CPU_LIB
 
 
+def torch_lib() -> Path | None:
+    """Where the extension module for this Python and this torch is, or would be; None without torch. An extension of
+    another torch must not be loaded, so both versions are part of its name: a package that was built beside
+    another torch has none."""
+    try:
+        import torch
+    except ImportError:
+        return None
+    return LIB_DIR / f"_ka_torch.cp{sys.version_info.major}{sys.version_info.minor}.torch{torch.__version__}.so"
+
+
 def torch_missing() -> str | None:
-    """Why ``_ka_torch.so`` cannot be compiled on this host, or None if it can."""
+    """Why the extension module cannot be compiled on this host, or None if it can."""
     try:
         import torch
     except ImportError:
@@ -132,27 +143,37 @@ def _cuda_include() -> Path | None:
 
 
 def build_torch(force: bool = False) -> Path | None:
-    """Compile ``csrc/torch/*.cpp`` into the extension module ``_ka_torch.so`` (C++ autograd nodes). None where that is not
-    possible (:func:`torch_missing`): the operators then reach the kernels from Python."""
+    """Compile ``csrc/torch/*.cpp`` into the extension module ``_ka_torch.*.so`` (C++ autograd nodes). None where that is
+    not possible (:func:`torch_missing`): the operators then reach the kernels from Python."""
+    out = torch_lib()
+    if out is None:
+        return None
     srcs = sorted((CSRC / "torch").glob("*.cpp"))
-    if not srcs or torch_missing() is not None:
-        return TORCH_LIB if TORCH_LIB.exists() else None
+    if not srcs:             # an installed wheel carries the built module, not the sources
+        return out if out.exists() else None
     import torch
 
     inc, lib = Path(torch.__file__).parent / "include", Path(torch.__file__).parent / "lib"
     flags = ["-O2", "-std=c++17", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
     digest = _digest(srcs, [*flags, torch.__version__, sys.version])
-    if not force and _stamp_ok(TORCH_LIB, digest):
-        return TORCH_LIB
+    if not force and _stamp_ok(out, digest):
+        return out
+    if torch_missing() is not None:
+        return None
     LIB_DIR.mkdir(parents=True, exist_ok=True)
+    # ranks that build at the same time, at their first call, each find a whole file
+    part = out.with_name(f"{out.stem}.{os.getpid()}.{threading.get_ident()}.part")
     try:
-        _run(["g++", *flags, "-shared", "-o", str(TORCH_LIB), *[str(s) for s in srcs], f"-I{inc}",
+        _run(["g++", *flags, "-shared", "-o", str(part), *[str(s) for s in srcs], f"-I{inc}",
               f"-I{inc / 'torch' / 'csrc' / 'api' / 'include'}", f"-I{sysconfig.get_paths()['include']}",
               f"-I{_cuda_include()}", f"-L{lib}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"])
+        os.replace(part, out)
     except RuntimeError:     # the compiler's message is on stderr; the other libraries do not need this one
         return None
-    TORCH_LIB.with_suffix(".hash").write_text(digest)
-    return TORCH_LIB
+    finally:
+        part.unlink(missing_ok=True)
+    out.with_suffix(".hash").write_text(digest)
+    return out
 
 
 def build_cpu_sanitized(force: bool = False) -> Path | None:
@@ -194,4 +215,4 @@ def build_all(force: bool = False, verbose: bool = False) -> None:
 
 if __name__ == "__main__":
     build_all(force="--force" in sys.argv, verbose="-v" in sys.argv)
-    print("built:", [str(p) for p in (CPU_LIB, TORCH_LIB, CUDA_LIB) if p.exists()])
+    print("built:", [str(p) for p in (CPU_LIB, torch_lib(), CUDA_LIB) if p is not None and p.exists()])

@@ -124,7 +124,7 @@ def torch_ops():
     """The extension module with the operators that are C++ autograd nodes, bound to the kernels of :func:`cuda`; None
     if there is none for this torch and it cannot be built."""
     path = _build.build_torch()
-    if path is None or not path.exists():
+    if path is None:
         return None
     spec = importlib.util.spec_from_file_location("_ka_torch", str(path))
     mod = importlib.util.module_from_spec(spec)

@@ -24,7 +24,7 @@ def collect() -> dict:
     info["cxx"] = shutil.which("g++")
     info["libka_sm100"] = str(_build.CUDA_LIB) if _build.CUDA_LIB.exists() else None
     info["libka_cpu"] = str(_build.CPU_LIB) if _build.CPU_LIB.exists() else None
-    info["ka_torch"] = str(_build.TORCH_LIB) if _build.TORCH_LIB.exists() else None
+    info["ka_torch"] = str(_build.torch_lib()) if _build.torch_lib().exists() else None
     info["ka_torch_missing"] = _build.torch_missing()
     gpus = []
     if torch.cuda.is_available():

@@ -10,7 +10,6 @@ from kernel_align_b200 import _build
 def elsewhere(tmp_path, monkeypatch):
     """The extension module goes to a folder of its own, and nothing is taken for built."""
     monkeypatch.setattr(_build, "LIB_DIR", tmp_path)
-    monkeypatch.setattr(_build, "TORCH_LIB", tmp_path / "_ka_torch.so")
     return tmp_path
 
 
@@ -34,9 +33,41 @@ def test_a_host_without_what_the_autograd_module_needs(elsewhere, monkeypatch, l
         monkeypatch.setattr(_build, "CSRC", elsewhere / "csrc")
         monkeypatch.setattr(_build, "ROOT", elsewhere)
     assert _build.build_torch() is None
-    assert not (elsewhere / "_ka_torch.so").exists()
+    assert not [p for p in elsewhere.iterdir() if p.suffix in (".so", ".part", ".hash")]
     if lacks != "a source that compiles":
         assert _build.torch_missing()
+
+
+def test_a_module_of_another_torch_or_of_other_sources_is_not_loaded(elsewhere, monkeypatch):
+    import torch
+
+    (elsewhere / "csrc" / "torch").mkdir(parents=True)
+    monkeypatch.setattr(_build, "CSRC", elsewhere / "csrc")                # an installed package: no sources
+    mine = _build.torch_lib()
+    mine.write_bytes(b"")
+    assert _build.build_torch() == mine
+    with monkeypatch.context() as m:
+        m.setattr(torch, "__version__", "2.99.0")
+        assert _build.torch_lib() != mine and _build.build_torch() is None
+    (elsewhere / "csrc" / "torch" / "node.cpp").write_text("")             # a checkout whose module is older than its sources
+    monkeypatch.setattr(_build, "ROOT", elsewhere)
+    monkeypatch.setattr(_build, "torch_missing", lambda: "no compiler")
+    assert _build.build_torch() is None
+
+
+def test_ranks_that_build_at_once_find_a_whole_module(elsewhere, monkeypatch):
+    """The compiler writes beside the module, which is put in place when it is whole."""
+    seen = []
+
+    def run(cmd):
+        out = cmd[cmd.index("-o") + 1]
+        seen.append((out, _build.torch_lib().exists()))
+        with open(out, "w") as f:
+            f.write("whole")
+
+    monkeypatch.setattr(_build, "_run", run)
+    path = _build.build_torch()
+    assert seen == [(seen[0][0], False)] and seen[0][0] != str(path) and path.read_text() == "whole"
 
 
 def test_the_kernel_library_is_built_before_the_module(monkeypatch):
