@@ -1079,7 +1079,7 @@ constexpr int kGeneralSmemBytes = (static_cast<int>(sizeof(GeneralSmem)) + 15) /
 // that crosses `limit` lies among the keys equal to tau. `by_mass` selects the criterion:
 //   by count: first key where count_above + count(key) >  limit  (limit = k - 1)
 //   by mass : first key where mass_above  + mass(key)  >  limit
-template <typename T, int kT>
+template <typename T>
 __device__ void descend(const T* rp, int v, float inv_temp, float y_max, bool by_mass,
                         unsigned long long limit, GeneralSmem& s, uint32_t& tau, unsigned long long& above_cnt,
                         unsigned long long& above_mass) {
@@ -1092,7 +1092,7 @@ __device__ void descend(const T* rp, int v, float inv_temp, float y_max, bool by
   for (int round = 0; round < 3; ++round) {
     const int w = widths[round];
     const int shift = 32 - known_bits - w;
-    for (int b = tid; b < kBins; b += kT) {
+    for (int b = tid; b < kBins; b += kThreads) {
       s.cnt[b] = 0;
       s.mass[b] = 0;
     }
@@ -1370,7 +1370,7 @@ struct DrawSmem {
   unsigned long long ties_before, target;
   int sel;
 };
-enum : int { kAll = 0, kByExp = 1, kByTable = 2 };   // all elements are kept / masses computed / looked up
+enum : int { kAll = 0, kByExp = 1, kByTable = 2, kByCount = 3 };   // all are kept / masses computed / looked up / 1 each
 
 template <typename T>
 __device__ __forceinline__ float key16_float(uint32_t k16) {
@@ -1512,10 +1512,10 @@ __device__ __forceinline__ void sum_range(const T* rp, int begin, int end, const
 }
 
 // First element, in token-id order, whose cumulative kept mass exceeds the target: the row is cut into
-// as many contiguous segments as there are warps (kW), whose kept masses are order-free integer sums (coalesced loads),
-// the segment that holds the target is cut again, and only the last hundred elements are walked
+// 32 contiguous segments, one per warp, whose kept masses are order-free integer sums (coalesced loads),
+// the segment that holds the target is cut into 32 again, and only the last hundred elements are walked
 // in order. With kAll the kept mass is what the first level adds up; false if it is 0.
-template <typename T, int kMode, int kW = kWarps>
+template <typename T, int kMode>
 __device__ bool draw(const T* rp, int v, const Kept& k, unsigned long long kept_mass, uint32_t u24, DrawSmem& d, int* out) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int begin = 0, end = v;
@@ -1526,7 +1526,7 @@ __device__ bool draw(const T* rp, int v, const Kept& k, unsigned long long kept_
   }
 #pragma unroll 1
   for (int level = 0; level < 2; ++level) {
-    const int len = ((end - begin + kW - 1) / kW + 7) / 8 * 8;
+    const int len = ((end - begin + kWarps - 1) / kWarps + 7) / 8 * 8;
     const int b = min(end, begin + warp * len), e = min(end, b + len);
     unsigned long long mass, ties;
     sum_range<T, kMode>(rp, b, e, k, mass, ties);
@@ -1536,10 +1536,10 @@ __device__ bool draw(const T* rp, int v, const Kept& k, unsigned long long kept_
     }
     __syncthreads();
     if (warp == 0) {
-      const unsigned long long t = lane < kW ? d.seg_ties[lane] : 0ull;
+      const unsigned long long t = d.seg_ties[lane];
       const unsigned long long t0 = d.ties_before + warp_incl_u64(t) - t;
       const unsigned long long left = k.tie_keep > t0 ? k.tie_keep - t0 : 0ull;
-      const unsigned long long m = (lane < kW ? d.seg_mass[lane] : 0ull) + (t < left ? t : left) * k.q_tau;
+      const unsigned long long m = d.seg_mass[lane] + (t < left ? t : left) * k.q_tau;
       const unsigned long long inc = warp_incl_u64(m);
       unsigned long long target = d.target;
       if (kMode == kAll && level == 0) target = mass_scale_u24(u24, __shfl_sync(0xffffffffu, inc, 31));
@@ -1777,10 +1777,10 @@ __device__ bool sample_row16(const T* rp, int v, float inv_temp, int top_k, floa
 }
 
 // The last kept element of a row in which nothing has a mass (-1: none is kept).
-template <typename T, int kT>
+template <typename T>
 __device__ int last_kept(const T* rp, int v, uint32_t tau, unsigned long long tie_keep, GeneralSmem& s) {
   const int tid = threadIdx.x;
-  const int chunk = (v + kT - 1) / kT;
+  const int chunk = (v + kThreads - 1) / kThreads;
   const int begin = min(v, tid * chunk), end = min(v, begin + chunk);
   unsigned long long ties = 0, total;
   for (int i = begin; i < end; ++i) ties += float_to_key(Elem<T>::to_float(rp[i])) == tau ? 1u : 0u;
@@ -1801,17 +1801,17 @@ __device__ int last_kept(const T* rp, int v, uint32_t tau, unsigned long long ti
 }
 
 // Largest key of the row, for the whole block.
-template <typename T, int kT>
+template <typename T>
 __device__ uint32_t row_max_key(const T* rp, int v, GeneralSmem& s) {
   constexpr int kVec = Elem<T>::kVec, kU = 8;
   const int tid = threadIdx.x;
   const int head = row_head(rp, v), nvec = (v - head) / kVec, scal = v - nvec * kVec;
   const uint4* vp = reinterpret_cast<const uint4*>(rp + head);
   uint32_t w[1] = {~0u};                      // NaN: key 0
-  for (int j = tid; j < nvec; j += kT * kU) {
+  for (int j = tid; j < nvec; j += kThreads * kU) {
     uint4 raw[kU];
 #pragma unroll
-    for (int u = 0; u < kU; ++u) raw[u] = j + kT * u < nvec ? __ldg(vp + j + kT * u) : make_uint4(~0u, ~0u, ~0u, ~0u);
+    for (int u = 0; u < kU; ++u) raw[u] = j + kThreads * u < nvec ? __ldg(vp + j + kThreads * u) : make_uint4(~0u, ~0u, ~0u, ~0u);
 #pragma unroll
     for (int u = 0; u < kU; ++u) w[0] = Elem<T>::wmax(w[0], vec_max<T>(raw[u]));
   }
@@ -1832,19 +1832,35 @@ __device__ uint32_t row_max_key(const T* rp, int v, GeneralSmem& s) {
   return s.max_key;
 }
 
-// One row by radix descent, any type; kHist: with descend16's histogram (kThreads threads, bf16).
-template <typename T, int kT, bool kHist>
-__device__ void general_row(const T* rp, int v, float inv_temp, int top_k, float top_p, uint32_t u24, GeneralSmem& s,
-                            unsigned int* hist, DrawSmem& d, int* out) {
+template <typename T>
+__global__ void __launch_bounds__(kThreads, 1)
+sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v, const long long* __restrict__ row_ids,
+                      float inv_temp, int top_k, float top_p, unsigned long long seed, unsigned long long step,
+                      int* __restrict__ out) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ DrawSmem d;
+  GeneralSmem& s = *reinterpret_cast<GeneralSmem*>(smem_raw);
+  constexpr bool kKey16 = std::is_same<T, __nv_bfloat16>::value;
+  unsigned int* hist = reinterpret_cast<unsigned int*>(smem_raw + kGeneralSmemBytes);  // kKey16 only
   const int tid = threadIdx.x;
+  const int row = blockIdx.x;
+  const T* rp = logits + static_cast<long long>(row) * row_stride;
+  const unsigned long long rid = row_ids ? static_cast<unsigned long long>(row_ids[row])
+                                         : static_cast<unsigned long long>(row);
+  const uint32_t u24 = uniform_u24(seed, rid, step);
   const bool has_k = top_k > 0 && top_k < v;
-  const float y_max = mul_rn(key_to_float(row_max_key<T, kT>(rp, v, s)), inv_temp);
+  if constexpr (Elem<T>::kPacked) {
+    FastSmem& f = *reinterpret_cast<FastSmem*>(smem_raw + kGeneralSmemBytes);
+    if ((has_k || top_p < 1.0f) && sample_row16<T>(rp, v, inv_temp, top_k, top_p, u24, s, f, d, out + row)) return;
+    __syncthreads();
+  }
+  const float y_max = mul_rn(key_to_float(row_max_key(rp, v, s)), inv_temp);
   Kept k;
   k.args = {inv_temp, -y_max};
   k.q_tau = 0;
   if (!has_k && top_p >= 1.0f) {              // everything is kept: the sums of the draw are the only pass
     k.tie_keep = 0;
-    if (!draw<T, kAll, kT / 32>(rp, v, k, 0, u24, d, out) && tid == 0) *out = v - 1;
+    if (!draw<T, kAll>(rp, v, k, 0, u24, d, out + row) && tid == 0) out[row] = v - 1;
     return;
   }
 
@@ -1859,12 +1875,12 @@ __device__ void general_row(const T* rp, int v, float inv_temp, int top_k, float
     unsigned long long k_ties = ~0ull;
     unsigned long long zk;
     if (has_k) {
-      if constexpr (kHist) {
+      if constexpr (kKey16) {
         unsigned long long unused;
         descend16<T>(rp, v, inv_temp, y_max, false, static_cast<unsigned long long>(top_k - 1), s, hist, k_tau,
                      k_above_cnt, k_above_mass, unused);
       } else {
-        descend<T, kT>(rp, v, inv_temp, y_max, false, static_cast<unsigned long long>(top_k - 1), s, k_tau, k_above_cnt,
+        descend<T>(rp, v, inv_temp, y_max, false, static_cast<unsigned long long>(top_k - 1), s, k_tau, k_above_cnt,
                    k_above_mass);
       }
       k_ties = static_cast<unsigned long long>(top_k) - k_above_cnt;
@@ -1872,7 +1888,7 @@ __device__ void general_row(const T* rp, int v, float inv_temp, int top_k, float
       zk = k_above_mass + k_ties * mass_fixed(exp_det(sub_rn(y, y_max)));
     } else {
       // everything is kept by the count criterion: Z = total mass
-      const int len = ((v + kT / 32 - 1) / (kT / 32) + 7) / 8 * 8;
+      const int len = ((v + kWarps - 1) / kWarps + 7) / 8 * 8;
       const int b = min(v, (tid >> 5) * len);
       unsigned long long part, unused, total;
       sum_range<T, kAll>(rp, b, min(v, b + len), k, part, unused);
@@ -1886,10 +1902,10 @@ __device__ void general_row(const T* rp, int v, float inv_temp, int top_k, float
       const unsigned long long limit = mass_fraction(static_cast<double>(top_p), zk);
       uint32_t p_tau;
       unsigned long long p_above_cnt, p_above_mass, p_present = 0;
-      if constexpr (kHist) {
+      if constexpr (kKey16) {
         descend16<T>(rp, v, inv_temp, y_max, true, limit, s, hist, p_tau, p_above_cnt, p_above_mass, p_present);
       } else {
-        descend<T, kT>(rp, v, inv_temp, y_max, true, limit, s, p_tau, p_above_cnt, p_above_mass);
+        descend<T>(rp, v, inv_temp, y_max, true, limit, s, p_tau, p_above_cnt, p_above_mass);
       }
       // element i (in sorted order) is kept while the mass before it is <= limit
       const float y = mul_rn(key_to_float(p_tau), inv_temp);
@@ -1916,7 +1932,7 @@ __device__ void general_row(const T* rp, int v, float inv_temp, int top_k, float
         tie_keep = p_ties;
         // the kept mass follows from the number of ties actually present
         unsigned long long present;
-        if constexpr (kHist) {
+        if constexpr (kKey16) {
           present = p_present;  // the histogram had the count
         } else {
           int local = 0;
@@ -1934,34 +1950,11 @@ __device__ void general_row(const T* rp, int v, float inv_temp, int top_k, float
   k.tau = tau;
   k.tie_keep = tie_keep;
   k.q_tau = mass_fixed(exp_det(sub_rn(mul_rn(key_to_float(tau), inv_temp), y_max)));
-  if (draw<T, kByExp, kT / 32>(rp, v, k, kept_mass, u24, d, out)) return;
+  if (draw<T, kByExp>(rp, v, k, kept_mass, u24, d, out + row)) return;
   // target == kept_mass can only happen when kept_mass is 0 (all masses underflowed):
   // fall back to the last kept element
-  const int last = last_kept<T, kT>(rp, v, tau, tie_keep, s);
-  if (tid == 0) *out = last < 0 ? 0 : last;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 1)
-sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v, const long long* __restrict__ row_ids,
-                      float inv_temp, int top_k, float top_p, unsigned long long seed, unsigned long long step,
-                      int* __restrict__ out) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ DrawSmem d;
-  GeneralSmem& s = *reinterpret_cast<GeneralSmem*>(smem_raw);
-  unsigned int* hist = reinterpret_cast<unsigned int*>(smem_raw + kGeneralSmemBytes);  // bf16 only
-  const int row = blockIdx.x;
-  const T* rp = logits + static_cast<long long>(row) * row_stride;
-  const unsigned long long rid = row_ids ? static_cast<unsigned long long>(row_ids[row])
-                                         : static_cast<unsigned long long>(row);
-  const uint32_t u24 = uniform_u24(seed, rid, step);
-  if constexpr (Elem<T>::kPacked) {
-    FastSmem& f = *reinterpret_cast<FastSmem*>(smem_raw + kGeneralSmemBytes);
-    const bool has_k = top_k > 0 && top_k < v;
-    if ((has_k || top_p < 1.0f) && sample_row16<T>(rp, v, inv_temp, top_k, top_p, u24, s, f, d, out + row)) return;
-    __syncthreads();
-  }
-  general_row<T, kThreads, std::is_same<T, __nv_bfloat16>::value>(rp, v, inv_temp, top_k, top_p, u24, s, hist, d, out + row);
+  const int last = last_kept<T>(rp, v, tau, tie_keep, s);
+  if (tid == 0) out[row] = last < 0 ? 0 : last;
 }
 
 // ---- bf16 rows: histograms per part of the row -------------------------------------------------
@@ -1974,11 +1967,18 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
 //   * C is chosen by part_ctas: few rows fill the GPU, and 200 rows are 400 CTAs, at most three half rows per SM, where one CTA
 //     of 1024 threads per row and SM takes two rounds.
 //   * For three CTAs per SM the two histograms must fit 64 KiB: 16-bit counters (a sub-part has at most 65535 elements) of the
-//     values whose magnitude lies in 64 binades, [2^-54, 2^10). What lies outside is sorted out element by
-//     element: zeros have counters of their own, NaN has no mass, and what is low enough to have no mass
-//     (-inf, the type's lowest value, -1e4) need not be counted. A look at the row's first elements shifts the 64 binades for
-//     rows of large values; if something with a mass is left out all the same, the row is counted again with the binades
-//     that its maximum asks for, and if that leaves out a nonzero value with a mass, one CTA takes the radix descent.
+//     values whose magnitude lies in 64 binades, [2^-51, 2^13) at first. What lies outside is sorted out element by
+//     element: NaN has no mass, what is low enough to have none (-inf, the type's lowest value) need not be counted, and zeros
+//     and "small" values below the 64 binades have four counters, one per kind and sign: they weigh the same to the last bit
+//     while the maximum is far larger than they are or all of them are next to nothing (part_small_alike). A look at the row's
+//     first elements moves the 64 binades for rows of large or of small values; if they turn out not to serve the row, it is
+//     counted again with those that its maximum asks for, which always do.
+//     The 64 binades end at 2^13 because of finite masks: 200 rows of 128256 columns, 90 % of them -1e4, 49 us, and 118 if these
+//     are counted (one counter for all). One value of 1e-18 in each of 8 / 64 / 200 rows: 18 / 25 / 41 us, as
+//     without it (31 / 31 / 59 by one CTA per row; 243 / 260 / 502 when such a row was searched by radix descent); zeros or NaN
+//     in 1 % / 10 % of the places 62 / 49 us for 200 rows (70 / 66).
+//   * A threshold among the small values, whose order their counters do not tell, is found by rank (part_select), and so is
+//     the last kept element of a row in which nothing has a mass.
 // [200, 128256] ~ N(0, 2), T = 1, top_p = 0.9: 58.4 us with one CTA per row, 41.2 us now: counting takes 31k cycles of an
 // SM with three half rows, the rest is latency (searches, barriers, the draw).
 // With 512 threads (40 registers each, three CTAs) the loops spilled: 46.8 us for 200 rows of 128256, 41.6 with 384; 320 41.9, 288 41.8.
@@ -1987,10 +1987,11 @@ constexpr int kPartsPerCta = 2;
 constexpr int kMaxPartCtas = 8;
 constexpr int kPartBinades = 64;
 constexpr int kPartMags = kPartBinades * 128;                        // magnitudes counted per sign
-constexpr int kPartBase = (127 + 10 - kPartBinades) * 128;           // bits of the smallest of them: 2^-54
+constexpr int kPartBase = (127 + 13 - kPartBinades) * 128;           // bits of the smallest of them: 2^-51
 constexpr int kPartHistBytes = kPartMags * 2 * 2;
-constexpr int kPartGroups = 2 * kPartMags / 32 + 1;                  // descending: positive values, zeros, negative values
-constexpr int kPartZeroGroup = kPartMags / 32;
+constexpr int kPartGroups = 2 * kPartMags / 32 + 1;                  // descending: positive values, small ones, negative values
+constexpr int kPartSmallGroup = kPartMags / 32;
+constexpr int kPartSmall = 4;                                        // small and positive, +0, -0, small and negative
 constexpr int kPartMaxElems = 65535;                                 // of a sub-part: what a counter holds
 constexpr int kNothing = 0x7FFFFFFF;                                 // below every counted value
 
@@ -2000,16 +2001,17 @@ constexpr int kPartUnits = 2 * kPartMags / 128;                      // of 128 n
 
 struct PartInfo {
   uint32_t max_key;             // 16-bit key of the largest element, 0 if there is no number
-  uint32_t flags;
+  uint32_t any_small;           // a nonzero value below the counted magnitudes
   uint32_t units[kPartUnits / 32];   // which units of counters are not empty
 };
 constexpr int kInfoWords = static_cast<int>(sizeof(PartInfo) / 4);
-enum PartFlags : uint32_t { kBig = 1, kLow = 2, kTiny = 4 };         // values outside the counted magnitudes
+constexpr int kPartBins = kPartsPerCta * kPartHistBytes / 4;         // of part_select: 32-bit counters of four keys each
+static_assert(kPartBins == 65536 / 4, "every key has a counter");
 
 struct PartSmem {
   unsigned long long mass[kPartGroups];
   unsigned int cnt[kPartGroups];
-  unsigned int zeros[kPartsPerCta][2];                               // +0, -0
+  unsigned int small[kPartsPerCta][kPartSmall];
   PartInfo mine;
   PartInfo info[kMaxPartCtas];
   unsigned long long scan[kPartWarps];
@@ -2024,23 +2026,32 @@ struct PartSmem {
   uint32_t look[kPartWarps];
   unsigned long long target, ties_before;      // of the draw inside the owner's sub-part
   unsigned long long blocks[kPartMaxBlocks];   // ties << kTieShift | mass
+  // part_select: elements in each CTA's slice of the bins, the bin that holds the rank and what lies above it, and
+  // per sub-part the elements above that bin and those of its keys
+  unsigned int slice[kMaxPartCtas], bin, above_bin, sel_above;
+  uint32_t sel_key;
+  unsigned int mine_keys[kPartsPerCta][5], keys[kMaxPartCtas * kPartsPerCta][5];
 };
 constexpr int kPartSmemBytes = kPartsPerCta * kPartHistBytes + static_cast<int>(sizeof(PartSmem));
 static_assert(kPartGroups <= 2 * kPartThreads, "a thread sums two groups");
-static_assert(kGeneralSmemBytes <= kPartsPerCta * kPartHistBytes, "the radix descent works where the histograms were");
 
-// Counted values in descending order: d = 0 .. kPartMags - 1 are the positive ones, then +0 and -0, then the negative ones.
+// Counted values in descending order: d = 0 .. kPartMags - 1 are the positive ones, then the four kinds of small ones (which
+// all weigh what a zero does), then the negative ones.
 __device__ __forceinline__ uint32_t part_bits(int d, uint32_t base) {
   if (d < kPartMags) return base + static_cast<uint32_t>(kPartMags - 1 - d);
-  return d < kPartMags + 2 ? (d == kPartMags ? 0u : 0x8000u) : 0x8000u + base + static_cast<uint32_t>(d - kPartMags - 2);
+  return d < kPartMags + kPartSmall ? (d == kPartMags + 2 ? 0x8000u : 0u)
+                                    : 0x8000u + base + static_cast<uint32_t>(d - kPartMags - kPartSmall);
 }
-__device__ __forceinline__ uint32_t part_offset(int d) {             // of its counter; not for zeros
-  return d < kPartMags ? static_cast<uint32_t>(kPartMags - 1 - d) * 2 : static_cast<uint32_t>(d - 2) * 2;
+__device__ __forceinline__ uint32_t part_offset(int d) {             // of its counter; not for small ones
+  return d < kPartMags ? static_cast<uint32_t>(kPartMags - 1 - d) * 2 : static_cast<uint32_t>(d - kPartSmall) * 2;
 }
 __device__ __forceinline__ int part_rank(uint32_t bits, uint32_t base) {   // d of the largest value
   const uint32_t mag = bits & 0x7FFFu;
-  if (mag == 0) return kPartMags;            // the first of the zeros
-  return bits & 0x8000u ? kPartMags + 2 + static_cast<int>(mag - base) : kPartMags - 1 - static_cast<int>(mag - base);
+  if (mag < base) return kPartMags;          // the first of the small ones
+  return bits & 0x8000u ? kPartMags + kPartSmall + static_cast<int>(mag - base) : kPartMags - 1 - static_cast<int>(mag - base);
+}
+__device__ __forceinline__ uint32_t key16_of_bits(uint32_t bits) {        // NaN: 0
+  return (bits & 0x7FFFu) > 0x7F80u ? 0u : (bits & 0x8000u ? 0xFFFFu - bits : bits + 0x8000u);
 }
 __device__ __forceinline__ float bits16_float(uint32_t bits) { return __uint_as_float(bits << 16); }
 __device__ __forceinline__ unsigned long long bits16_mass(uint32_t bits, float inv_temp, float y_max) {
@@ -2095,41 +2106,61 @@ __device__ __forceinline__ uint32_t part_base(float reach) {
   return top > kPartMags ? top - kPartMags : 1u;
 }
 
-// Histogram of this CTA's sub-parts (zeroed before), its largest element, which values were not counted.
+// Do all values below magnitude `base` weigh the same as a zero, to the last bit? They do if their weights have one
+// argument, and if the arguments are so close to 0 that the weight is 1 (exp_det rounds to it below 2^-26).
+__device__ __forceinline__ bool part_small_alike(uint32_t base, float inv_temp, float y_max) {
+  const float y = mul_rn(bits16_float(base - 1), inv_temp);
+  return sub_rn(y, y_max) == sub_rn(-y, y_max) || (fabsf(y) <= 0x1p-28f && fabsf(y_max) <= 0x1p-28f);
+}
+
+// Histogram of this CTA's sub-parts (zeroed before), its largest element, its small values.
 __device__ __forceinline__ void part_count(const __nv_bfloat16* rp, int v, uint32_t base, int rank, int ctas, unsigned char* hist,
                                            PartSmem& s) {
   using T = __nv_bfloat16;
-  // Three vectors in flight per thread: 200 / 256 rows of 128256 take 41.2 / 48.3 us, with four 42.1 / 49.1, with two 40.3 / 49.4
-  // in another run, so 256 rows lose; short rows do not care (256 x 8000: 17.9 against 17.7).
+  // Vectors in flight per thread, us with two / three / four: 64 rows of 128256 27.3 / 25.6 / 25.6, 200 rows 41.4 / 41.2 / 42.3,
+  // 256 rows 49.9 / 47.8 / 48.5; short rows do not care (256 x 8000: 18.2 / 18.4 / 18.5).
   constexpr int kTs = kPartThreads / kPartsPerCta, kU = 3;
-  const int tid = threadIdx.x, sub = tid / kTs, t = tid % kTs;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = tid / kTs, t = tid % kTs;
+  static_assert(kTs % 32 == 0, "a warp works on one sub-part");
   const PartRange pr = part_range(rank * kPartsPerCta + sub, ctas * kPartsPerCta, row_head(rp, v), v);
   const int n_vec = pr.n_vec;
   unsigned char* mine = hist + sub * kPartHistBytes;
-  uint32_t top = 0xFFFFFFFFu, flags = 0;
-  unsigned int zeros = 0, neg_zeros = 0;
+  uint32_t top = 0xFFFFFFFFu;
+  uint32_t below2 = 0, below_pos2 = 0, zero2 = 0, zero_pos2 = 0;     // values below base, zeros; of both signs / positive ones
   auto count = [&](uint32_t a) {       // a: bits - base in the low half; a counter of 16 bits is half a word
     const uint32_t off = ((a << 1) & 0x3FFCu) | ((a >> 1) & 0x4000u);
     atomicAdd(reinterpret_cast<unsigned int*>(mine + off), max((a << 16) & 0x10000u, 1u));
   };
-  // h: 16 bits. What is not counted: zeros, tiny values, large ones and NaN
-  auto count_or_note = [&](uint32_t h) {
-    const uint32_t mag = h & 0x7FFFu, above = mag - (base + kPartMags);
-    zeros += h == 0u ? 1u : 0u;
-    neg_zeros += h == 0x8000u ? 1u : 0u;
-    flags |= mag - 1u < base - 1u ? kTiny : 0u;
-    flags |= above <= 0x7F80u - (base + kPartMags) ? (h >> 15) + kBig : 0u;
-    if (((h - base) & 0x6000u) == 0) count(h - base);
+  // the same under a predicate: eight branches a vector cost more than the atomics
+  const uint32_t mine_addr = static_cast<uint32_t>(__cvta_generic_to_shared(mine));
+  auto count_if = [&](bool inside, uint32_t a) {
+    const uint32_t off = ((a << 1) & 0x3FFCu) | ((a >> 1) & 0x4000u);
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p red.shared.add.u32 [%1], %2;\n\t}" ::"r"(inside ? 1u : 0u),
+                 "r"(mine_addr + off), "r"(max((a << 16) & 0x10000u, 1u))
+                 : "memory");
+  };
+  const uint32_t base2 = (base + 1) * 0x00010001u;
+  // per half of a word: 1 where the magnitude is below the limit (limit2: limit + 1 in both halves)
+  auto below = [](uint32_t w, uint32_t limit2) { return __viaddmin_s16x2_relu(~w | 0x80008000u, limit2, 0x00010001u); };
+  auto positive = [](uint32_t w, uint32_t ones) { return ones & ~(w >> 15); };
+  auto note = [&](uint32_t w, uint32_t small) {
+    const uint32_t zero = below(w, 0x00020002u);
+    below2 += small;
+    below_pos2 += positive(w, small);
+    zero2 += zero;
+    zero_pos2 += positive(w, zero);
   };
   const uint4* vp = reinterpret_cast<const uint4*>(rp + pr.first);
-  for (int j = t; j < n_vec; j += kTs * kU) {
+  for (int j0 = t - lane; j0 < n_vec; j0 += kTs * kU) {
     uint4 raw[kU];
 #pragma unroll
-    for (int u = 0; u < kU; ++u)
-      if (j + kTs * u < n_vec) raw[u] = __ldg(vp + j + kTs * u);
+    for (int u = 0; u < kU; ++u) {
+      const int j = j0 + kTs * u + lane;
+      raw[u] = j < n_vec ? __ldg(vp + j) : make_uint4(~0u, ~0u, ~0u, ~0u);     // NaN: neither counted nor noted
+    }
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
-      if (j + kTs * u >= n_vec) break;
+      if (j0 + kTs * u >= n_vec) break;
       const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
       uint32_t a[8], out = 0;
 #pragma unroll
@@ -2139,14 +2170,21 @@ __device__ __forceinline__ void part_count(const __nv_bfloat16* rp, int v, uint3
         out |= (a[2 * i] | a[2 * i + 1]) & 0x6000u;
       }
       top = Elem<T>::wmax(top, vec_max<T>(raw[u]));
-      if (__any_sync(__activemask(), out != 0) == 0) {     // one path for the warp: lanes apart would take both
+      const bool have = j0 + kTs * u + lane < n_vec;
+      if (__any_sync(0xffffffffu, have && out != 0) == 0) {     // one path for the warp: lanes apart would take both
+        if (have) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) count(a[i]);
+          for (int i = 0; i < 8; ++i) count(a[i]);
+        }
       } else {
+        uint32_t small[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          count_or_note(w[i] & 0xFFFFu);
-          count_or_note(w[i] >> 16);
+        for (int i = 0; i < 4; ++i) small[i] = below(w[i], base2);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) count_if((a[i] & 0x6000u) == 0, a[i]);
+        if (__any_sync(0xffffffffu, (small[0] | small[1] | small[2] | small[3]) != 0)) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) note(w[i], small[i]);
         }
       }
     }
@@ -2154,24 +2192,27 @@ __device__ __forceinline__ void part_count(const __nv_bfloat16* rp, int v, uint3
   // scalars in front of the first vector and behind the last one (fewer than eight each)
   const unsigned short* hp = reinterpret_cast<const unsigned short*>(rp);
   if (t < pr.n_head + pr.n_tail) {
-    const uint32_t h = hp[t < pr.n_head ? t : pr.tail + (t - pr.n_head)];
-    count_or_note(h);
-    top = Elem<T>::wmax(top, h | 0xFFFF0000u);
+    const uint32_t h = hp[t < pr.n_head ? t : pr.tail + (t - pr.n_head)] | 0xFFFF0000u;
+    if (((h - base) & 0x6000u) == 0) count(h - base);
+    note(h, below(h, base2));
+    top = Elem<T>::wmax(top, h);
   }
   top = key16x2<T>(top);
   top = __reduce_max_sync(0xffffffffu, max(top >> 16, top & 0xFFFFu));
-  flags = __reduce_or_sync(0xffffffffu, flags);
-  zeros = __reduce_add_sync(0xffffffffu, zeros);
-  neg_zeros = __reduce_add_sync(0xffffffffu, neg_zeros);
-  if ((tid & 31) == 0) {
+  auto total = [](uint32_t c) { return __reduce_add_sync(0xffffffffu, (c & 0xFFFFu) + (c >> 16)); };
+  const unsigned int n_below = total(below2), n_pos = total(below_pos2), n_zero = total(zero2), n_zero_pos = total(zero_pos2);
+  if (lane == 0) {
     atomicMax(&s.mine.max_key, top);
-    if (flags) atomicOr(&s.mine.flags, flags);
-    if (zeros) atomicAdd(&s.zeros[sub][0], zeros);
-    if (neg_zeros) atomicAdd(&s.zeros[sub][1], neg_zeros);
+    if (n_below) {
+      if (n_below != n_zero) s.mine.any_small = 1u;
+      const unsigned int n[kPartSmall] = {n_pos - n_zero_pos, n_zero_pos, n_zero - n_zero_pos, n_below - n_pos - (n_zero - n_zero_pos)};
+#pragma unroll
+      for (int i = 0; i < kPartSmall; ++i)
+        if (n[i]) atomicAdd(&s.small[sub][i], n[i]);
+    }
   }
   __syncthreads();
   // which units of 128 counters are not empty
-  const int lane = tid & 31, warp = tid >> 5;
 #pragma unroll 4
   for (int u = warp; u < kPartUnits; u += kPartWarps) {
     const uint2 c0 = *reinterpret_cast<const uint2*>(hist + u * 256 + lane * 8);
@@ -2182,14 +2223,14 @@ __device__ __forceinline__ void part_count(const __nv_bfloat16* rp, int v, uint3
 }
 static_assert(kPartsPerCta == 2, "both histograms of a CTA");
 
-// Zeros of one sign in the whole row.
-__device__ __forceinline__ unsigned int part_zeros(int sign, int ctas, const PartSmem& s) {
+// Small values of one kind in the whole row.
+__device__ __forceinline__ unsigned int part_smalls(int kind, int ctas, const PartSmem& s) {
   unsigned int n = 0;
 #pragma unroll
   for (int r = 0; r < kMaxPartCtas; ++r)
     if (r < ctas)
 #pragma unroll
-      for (int sub = 0; sub < kPartsPerCta; ++sub) n += ld_remote_u32(map_to_cta(&s.zeros[sub][sign], r));
+      for (int sub = 0; sub < kPartsPerCta; ++sub) n += ld_remote_u32(map_to_cta(&s.small[sub][kind], r));
   return n;
 }
 
@@ -2223,11 +2264,11 @@ __device__ void part_search(bool by_mass, unsigned long long limit, float inv_te
   if (g < 0) {
     if (tid == 0) s.sel = kNothing;
   } else if (tid < 32) {
-    const bool zero = g == kPartZeroGroup;
-    const int d = (g <= kPartZeroGroup ? 32 * g : 32 * g - 30) + lane;
+    const bool small = g == kPartSmallGroup;
+    const int d = (g <= kPartSmallGroup ? 32 * g : 32 * g - (32 - kPartSmall)) + lane;
     unsigned int n = 0;
-    if (zero) {
-      if (lane < 2) n = part_zeros(lane, ctas, s);
+    if (small) {
+      if (lane < kPartSmall) n = part_smalls(lane, ctas, s);
     } else {
       const uint32_t a = hist + part_offset(d);
 #pragma unroll
@@ -2266,6 +2307,7 @@ __device__ __forceinline__ void part_draw(const __nv_bfloat16* rp, const PartRan
   auto mass_of = [&](uint32_t h) {         // ties << kTieShift | mass
     const uint32_t key = float_to_key(bits16_float(h));
     if (kMode != kAll && key <= k.tau) return key == k.tau ? 1ull << kTieShift : 0ull;
+    if (kMode == kByCount) return 1ull;
     return static_cast<unsigned long long>(mass_fixed(exp_det(sub_rn(mul_rn(key_to_float(key), k.args.inv_temp), y_max))));
   };
   const int tau_o = static_cast<int>(k.tau ^ 0x80000000u);
@@ -2275,6 +2317,8 @@ __device__ __forceinline__ void part_draw(const __nv_bfloat16* rp, const PartRan
       const uint32_t i2 = __viaddmin_u16x2(not_key, k.top2, k.last2);
       m += k.table[i2 & 0xFFFFu];
       m += k.table[i2 >> 16];
+    } else if constexpr (kMode == kByCount) {
+      m += mass_of(w & 0xFFFFu) + mass_of(w >> 16);
     } else {
       float x0 = __uint_as_float(w << 16), x1 = __uint_as_float(w & 0xFFFF0000u);
       if constexpr (kMode != kAll) {
@@ -2415,11 +2459,163 @@ __device__ __forceinline__ void part_draw(const __nv_bfloat16* rp, const PartRan
   }
 }
 
-// Out of line: rows that the histograms cannot answer. Run by one CTA of the cluster.
-__device__ __noinline__ void part_general(const __nv_bfloat16* rp, int v, float inv_temp, int top_k, float top_p, uint32_t u24,
-                                          unsigned char* smem, DrawSmem& d, int* out) {
-  general_row<__nv_bfloat16, kPartThreads, false>(rp, v, inv_temp, top_k, top_p, u24, *reinterpret_cast<GeneralSmem*>(smem),
-                                                  nullptr, d, out);
+// The sub-part that holds s.target of the kept mass, from s.sub_mass and s.sub_ties; the target and the ties in front inside it.
+// By one warp.
+__device__ __forceinline__ void part_owner(int n_sub, const Kept& k, unsigned long long target, PartSmem& s) {
+  const int lane = threadIdx.x & 31;
+  const unsigned long long t = lane < n_sub ? s.sub_ties[lane] : 0ull, t0 = warp_incl_u64(t) - t;
+  const unsigned long long left = k.tie_keep > t0 ? k.tie_keep - t0 : 0ull;
+  const unsigned long long m = (lane < n_sub ? s.sub_mass[lane] : 0ull) + (t < left ? t : left) * k.q_tau;
+  const unsigned long long inc = warp_incl_u64(m);
+  const int first = __ffs(static_cast<int>(__ballot_sync(0xffffffffu, inc > target))) - 1;
+  if (lane == first) {
+    s.owner = first;
+    s.target = target - (inc - m);
+    s.ties_before = t0;
+  }
+}
+
+// By rank: the key of the n-th largest of the row's elements whose 16-bit keys lie in [lo, hi] (there are that many), and
+// how many of these elements lie above that key. s.sub_mass gets, per sub-part, `each` for every one of them on top of what
+// it holds, s.sub_ties the elements of that key. Out of line, by all CTAs of the row: bins of four keys, of which each
+// CTA adds up a slice, then a look at the four keys of the bin that holds the rank. The histograms are overwritten.
+// What bounds it is its instructions, two passes of about 15 per element, and no earnest row comes here: half of the values
+// nonzero and below 2^-51, us, one CTA of 1024 threads per row / here: 8 rows of 128256 34.6 / 36.8, 64 rows 35.2 / 70.7, 200 rows
+// 65.9 / 128; rows with an infinity, k = 2000: 148 / 40, 150 / 64, 296 / 116.
+__device__ __noinline__ void part_select(const __nv_bfloat16* rp, int v, int rank, int ctas, uint32_t lo, uint32_t hi, unsigned int n,
+                                         unsigned long long each, unsigned int* bins, PartSmem& s) {
+  constexpr int kTs = kPartThreads / kPartsPerCta;
+  const int tid = threadIdx.x, lane = tid & 31, sub = tid / kTs, t = tid % kTs;
+  const PartRange pr = part_range(rank * kPartsPerCta + sub, ctas * kPartsPerCta, row_head(rp, v), v);
+  const uint4* vp = reinterpret_cast<const uint4*>(rp + pr.first);
+  const unsigned short* hp = reinterpret_cast<const unsigned short*>(rp);
+  auto each_key = [&](auto&& f) {        // keys of this thread's elements that lie in [lo, hi]
+    auto one = [&](uint32_t h) {
+      const uint32_t key = key16_of_bits(h);
+      if (key >= lo && key <= hi) f(key);
+    };
+    for (int j = t; j < pr.n_vec; j += kTs) {
+      const uint4 raw = __ldg(vp + j);
+      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        one(w[i] & 0xFFFFu);
+        one(w[i] >> 16);
+      }
+    }
+    if (t < pr.n_head + pr.n_tail) one(hp[t < pr.n_head ? t : pr.tail + (t - pr.n_head)]);
+  };
+  part_barrier(ctas);                    // nobody reads the histograms any more
+  for (int i = tid; i < kPartBins / 4; i += kPartThreads) reinterpret_cast<uint4*>(bins)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (tid < kPartsPerCta * 5) s.mine_keys[tid / 5][tid % 5] = 0;
+  __syncthreads();
+  each_key([&](uint32_t key) { atomicAdd(&bins[key >> 2], 1u); });
+  part_barrier(ctas);
+  // this CTA's slice: bins top - from ... top - (to - 1), each thread a run of them, summed over the row's CTAs
+  const int top = static_cast<int>(hi >> 2), n_bins = top - static_cast<int>(lo >> 2) + 1, per = (n_bins + ctas - 1) / ctas;
+  const int from = min(n_bins, rank * per), to = min(n_bins, from + per), run = (to - from + kPartThreads - 1) / kPartThreads;
+  const int b0 = min(to, from + tid * run), b1 = min(to, b0 + run);
+  auto bin_sum = [&](int b) {
+    unsigned int c = 0;
+#pragma unroll
+    for (int r = 0; r < kMaxPartCtas; ++r)
+      if (r < ctas) c += ld_remote_u32(map_to_cta(bins + (top - b), r));
+    return c;
+  };
+  unsigned int mine = 0;
+  for (int b = b0; b < b1; ++b) mine += bin_sum(b);
+  unsigned long long all;
+  unsigned long long before = block_exscan_u64(mine, s.scan, all);
+  if (tid < ctas) st_remote_u32(map_to_cta(&s.slice[rank], tid), static_cast<unsigned int>(all));
+  part_barrier(ctas);
+  for (int r = 0; r < rank; ++r) before += s.slice[r];
+  if (before < n && n <= before + mine) {
+    for (int b = b0; b < b1; ++b) {
+      const unsigned int c = bin_sum(b);
+      if (n <= before + c) {
+        for (int r = 0; r < ctas; ++r) {
+          st_remote_u32(map_to_cta(&s.bin, r), static_cast<uint32_t>(top - b));
+          st_remote_u32(map_to_cta(&s.above_bin, r), static_cast<uint32_t>(before));
+        }
+        break;
+      }
+      before += c;
+    }
+  }
+  part_barrier(ctas);
+  const uint32_t bin = s.bin;
+  unsigned int c[5] = {0, 0, 0, 0, 0};   // above the bin, then its keys from the top
+  each_key([&](uint32_t key) {
+    c[0] += (key >> 2) > bin ? 1u : 0u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[1 + i] += key == 4 * bin + 3 - i ? 1u : 0u;
+  });
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    c[i] = __reduce_add_sync(0xffffffffu, c[i]);
+    if (lane == 0 && c[i]) atomicAdd(&s.mine_keys[sub][i], c[i]);
+  }
+  __syncthreads();
+  if (tid < ctas * kPartsPerCta * 5) {
+    const int to_cta = tid / (kPartsPerCta * 5), at = tid % (kPartsPerCta * 5);
+    st_remote_u32(map_to_cta(&s.keys[rank * kPartsPerCta + at / 5][at % 5], to_cta), s.mine_keys[at / 5][at % 5]);
+  }
+  part_barrier(ctas);
+  unsigned int above = s.above_bin;
+  int at = 0;
+  for (;; ++at) {                        // the key of the four that holds the rank
+    unsigned int here = 0;
+    for (int q = 0; q < ctas * kPartsPerCta; ++q) here += s.keys[q][1 + at];
+    if (at == 3 || n <= above + here) break;
+    above += here;
+  }
+  if (tid == 0) {
+    s.sel_key = 4 * bin + 3 - at;
+    s.sel_above = above;
+  }
+  if (tid < ctas * kPartsPerCta) {
+    unsigned int kept = 0;
+    for (int i = 0; i <= at; ++i) kept += s.keys[tid][i];
+    s.sub_mass[tid] += kept * each;
+    s.sub_ties[tid] = s.keys[tid][1 + at];
+  }
+  __syncthreads();
+}
+
+// The draw where the kept elements end among the small ones of one sign, of which the first n by rank are kept: the rest of
+// the kernel, with q the mass of a small value and s.sub_mass what is kept above them.
+__device__ __noinline__ void part_draw_small(const __nv_bfloat16* rp, int v, int rank, int ctas, uint32_t base, bool neg, unsigned int n,
+                                             unsigned long long q, MassArgs args, unsigned long long target, unsigned int* bins,
+                                             PartSmem& s, int* out) {
+  part_select(rp, v, rank, ctas, neg ? 0x8000u - base : 0x8001u, neg ? 0x7FFEu : 0x7FFFu + base, n, q, bins, s);
+  Kept k;
+  k.tau = float_to_key(key16_float<__nv_bfloat16>(s.sel_key));
+  k.tie_keep = n - s.sel_above;
+  k.q_tau = q;
+  k.args = args;
+  const int n_sub = ctas * kPartsPerCta;
+  if (threadIdx.x < 32) part_owner(n_sub, k, target, s);
+  __syncthreads();
+  if (s.owner / kPartsPerCta != rank) return;
+  part_draw<kByExp>(rp, part_range(s.owner, n_sub, row_head(rp, v), v), k, s, out);
+}
+
+// A row in which nothing has a mass (its maximum is infinite or there is no number): the last of its top_k largest elements in
+// token-id order.
+__device__ __noinline__ void part_last(const __nv_bfloat16* rp, int v, int rank, int ctas, int top_k, unsigned int* bins,
+                                       PartSmem& s, int* out) {
+  const int n_sub = ctas * kPartsPerCta;
+  if (threadIdx.x < n_sub) s.sub_mass[threadIdx.x] = 0;
+  part_select(rp, v, rank, ctas, 0u, 0xFFFFu, static_cast<unsigned int>(top_k), 1ull, bins, s);
+  Kept k;
+  k.tau = s.sel_key == 0 ? 0u : float_to_key(key16_float<__nv_bfloat16>(s.sel_key));
+  k.tie_keep = static_cast<unsigned int>(top_k) - s.sel_above;
+  k.q_tau = 1;
+  k.args = {0.f, 0.f};
+  if (threadIdx.x < 32) part_owner(n_sub, k, static_cast<unsigned long long>(top_k) - 1, s);
+  __syncthreads();
+  if (s.owner / kPartsPerCta != rank) return;
+  part_draw<kByCount>(rp, part_range(s.owner, n_sub, row_head(rp, v), v), k, s, out);
 }
 
 __global__ void __launch_bounds__(kPartThreads, 3)
@@ -2428,7 +2624,6 @@ sample_parts_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stri
                     unsigned long long step, int ctas, int* __restrict__ out) {
   using T = __nv_bfloat16;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ DrawSmem d;
   unsigned char* hist = smem_raw;
   PartSmem& s = *reinterpret_cast<PartSmem*>(smem_raw + kPartsPerCta * kPartHistBytes);
   const uint32_t hist_addr = static_cast<uint32_t>(__cvta_generic_to_shared(hist));
@@ -2456,7 +2651,7 @@ sample_parts_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stri
       s.mass[i] = 0;
       s.cnt[i] = 0;
     }
-    if (tid < kPartsPerCta * 2) s.zeros[tid >> 1][tid & 1] = 0;
+    if (tid < kPartsPerCta * kPartSmall) s.small[tid / kPartSmall][tid % kPartSmall] = 0;
     if (tid < kPartsPerCta) s.acc[tid] = 0;
     if (tid < kInfoWords) reinterpret_cast<uint32_t*>(&s.mine)[tid] = 0;
     if (attempt == 0) {
@@ -2471,7 +2666,8 @@ sample_parts_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stri
 #pragma unroll
       for (int w = 0; w < kPartWarps; ++w) m = Elem<T>::wmax(m, s.look[w]);
       const float x = bits16_float(m & 0xFFFFu), reach = 2.f * part_reach(x, inv_temp);
-      if (reach >= 1024.f && reach < 1e38f) base = part_base(reach);     // no number, an infinity: as usual
+      if (reach >= 0x1p13f && reach < 1e38f) base = part_base(reach);     // no number, an infinity: as usual
+      if (x > 0.f && x < 0x1p-51f) base = part_base(4.f * x);
     }
     part_count(rp, v, base, rank, ctas, hist, s);
     __syncthreads();
@@ -2482,10 +2678,10 @@ sample_parts_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stri
     if (tid == kPartThreads - 1)
       s.u24 = uniform_u24(seed, row_ids ? static_cast<unsigned long long>(row_ids[row]) : static_cast<unsigned long long>(row), step);
     part_barrier(ctas);
-    uint32_t flags = 0;
+    bool small = false;
     max_key = 0;
     for (int r = 0; r < ctas; ++r) {
-      flags |= s.info[r].flags;
+      small |= s.info[r].any_small != 0;
       max_key = max(max_key, s.info[r].max_key);
     }
     max_bits = max_key == 0 ? 0x7FFFu : (max_key & 0x8000u ? max_key & 0x7FFFu : 0xFFFFu - max_key);
@@ -2493,26 +2689,21 @@ sample_parts_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stri
     y_max = mul_rn(x_max, inv_temp);
     if (!(fabsf(y_max) <= 3.402823466e38f)) {
       // no number, or an infinite one: nothing has a mass, the last kept element is the answer
-      if (rank != 0) return;
       if (has_k)
-        part_general(rp, v, inv_temp, top_k, top_p, s.u24, smem_raw, d, out + row);
-      else if (tid == 0)
+        part_last(rp, v, rank, ctas, top_k, reinterpret_cast<unsigned int*>(hist), s, out + row);
+      else if (rank == 0 && tid == 0)
         out[row] = v - 1;
       return;
     }
-    // below 2^-33 of the maximum's weight a mass is 0 (2^-32 is the smallest that counts)
-    auto massive = [&](uint32_t bits) { return (bits16_float(bits) * inv_temp - y_max) * 1.4426950408889634f > -33.f; };
-    const uint32_t lowest = 0x8000u + base + kPartMags;
-    const bool low = (flags & kLow) && massive(lowest), tiny = (flags & kTiny) && massive(base);
-    if (!(flags & kBig) && !low && !tiny) break;
-    if (attempt > 0) {
-      if (rank == 0)
-        part_general(rp, v, inv_temp, top_k, top_p, s.u24, smem_raw, d, out + row);
-      return;
-    }
-    // the 64 binades up to the largest magnitude that can have a mass; if all values are tiny, up to theirs
-    const bool all_tiny = !(flags & (kBig | kLow)) && (max_bits & 0x7FFFu) < base;
-    base = part_base(all_tiny ? 4.f * fabsf(x_max) : part_reach(x_max, inv_temp));
+    if (attempt > 0) break;              // the second 64 binades serve every row
+    // What the first ones may miss: the largest value; values below all of them that have a mass, which is 0 below
+    // 2^-33 of the maximum's (2^-32 is the smallest that counts); small values that weigh other than a zero
+    const uint32_t max_mag = max_bits & 0x7FFFu;
+    const float lowest = -bits16_float(base + kPartMags);
+    const bool big = max_mag >= base + kPartMags, low = (lowest * inv_temp - y_max) * 1.4426950408889634f > -33.f;
+    const bool differ = small && !part_small_alike(base, inv_temp, y_max);
+    if (!big && !low && !differ) break;
+    base = part_base(part_reach(x_max, inv_temp));
     part_barrier(ctas);               // s.info is written again
   }
 
@@ -2566,27 +2757,22 @@ sample_parts_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stri
       m += __shfl_xor_sync(0xffffffffu, m, o);
       cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     }
-    const int g = neg ? kPartZeroGroup + 1 + (at - kPartMags) / 32 : kPartZeroGroup - 1 - at / 32;
+    const int g = neg ? kPartSmallGroup + 1 + (at - kPartMags) / 32 : kPartSmallGroup - 1 - at / 32;
     if ((lane & 7) < ctas && cnt) {
       st_remote_u64(map_to_cta(&s.mass[g], lane & 7), m);
       st_remote_u32(map_to_cta(&s.cnt[g], lane & 7), cnt);
     }
   }
   if (rank == 0 && warp == kPartWarps - 1) {
-    unsigned int n = lane < 2 ? part_zeros(lane, ctas, s) : 0u;
-    unsigned long long m = n ? n * bits16_mass(0u, inv_temp, y_max) : 0ull;      // both zeros weigh the same
-    m += __shfl_down_sync(0xffffffffu, m, 1);
-    n += __shfl_down_sync(0xffffffffu, n, 1);
-    m = __shfl_sync(0xffffffffu, m, 0);
-    n = __shfl_sync(0xffffffffu, n, 0);
+    const unsigned int n = __reduce_add_sync(0xffffffffu, lane < kPartSmall ? part_smalls(lane, ctas, s) : 0u);
     if (lane < ctas && n) {
-      st_remote_u64(map_to_cta(&s.mass[kPartZeroGroup], lane), m);
-      st_remote_u32(map_to_cta(&s.cnt[kPartZeroGroup], lane), n);
+      st_remote_u64(map_to_cta(&s.mass[kPartSmallGroup], lane), n * bits16_mass(0u, inv_temp, y_max));
+      st_remote_u32(map_to_cta(&s.cnt[kPartSmallGroup], lane), n);
     }
   }
   part_barrier(ctas);
 
-  // ---- where the kept prefix ends, in every CTA: the same decisions as in general_row
+  // ---- where the kept prefix ends, in every CTA: the same decisions as in sample_general_kernel
   int tau = kNothing;
   unsigned long long tie_keep = ~0ull, kept_mass;
   {
@@ -2621,18 +2807,23 @@ sample_parts_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stri
     }
   }
 
+  // small values without a mass: everything that has one is kept
+  const bool among_small = tau == kPartMags || tau == kPartMags + kPartSmall - 1;
+  const unsigned long long q_small = among_small ? bits16_mass(0u, inv_temp, y_max) : 0ull;
+  if (among_small && q_small == 0) tau = kNothing;
+
   // ---- kept mass and ties of this CTA's sub-parts, from their histograms
   {
     unsigned long long m[kPartsPerCta] = {};
-    const int d_end = min(tau, 2 * kPartMags + 2);
+    const int d_end = min(tau, 2 * kPartMags + kPartSmall);
 #pragma unroll 1
     for (int i = part_rank(max_bits, base) + tid; i < d_end; i += kPartThreads) {
       unsigned int n[kPartsPerCta], any = 0;
-      const bool zero = i == kPartMags || i == kPartMags + 1;
+      const bool small = i >= kPartMags && i < kPartMags + kPartSmall;
 #pragma unroll
       for (int sub = 0; sub < kPartsPerCta; ++sub) {
-        n[sub] = zero ? s.zeros[sub][i - kPartMags]
-                      : *reinterpret_cast<const unsigned short*>(hist + sub * kPartHistBytes + part_offset(i));
+        n[sub] = small ? s.small[sub][i - kPartMags]
+                       : *reinterpret_cast<const unsigned short*>(hist + sub * kPartHistBytes + part_offset(i));
         any |= n[sub];
       }
       if (any == 0) continue;
@@ -2650,8 +2841,8 @@ sample_parts_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stri
       const int to = tid / kPartsPerCta, sub = tid % kPartsPerCta, q = rank * kPartsPerCta + sub;
       unsigned long long ties = 0;
       if (tau != kNothing)
-        ties = tau == kPartMags || tau == kPartMags + 1
-                   ? s.zeros[sub][tau - kPartMags]
+        ties = tau >= kPartMags && tau < kPartMags + kPartSmall
+                   ? s.small[sub][tau - kPartMags]
                    : *reinterpret_cast<const unsigned short*>(hist + sub * kPartHistBytes + part_offset(tau));
       st_remote_u64(map_to_cta(&s.sub_mass[q], to), s.acc[sub]);
       st_remote_u64(map_to_cta(&s.sub_ties[q], to), ties);
@@ -2662,25 +2853,18 @@ sample_parts_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stri
   // ---- the sub-part that holds the target; its CTA draws, nobody reads another CTA's memory any more
   Kept k;
   const uint32_t tau_bits = tau == kNothing ? 0u : part_bits(tau, base);
-  const uint32_t tau16 = tau == kNothing ? 0u : (tau_bits & 0x8000u ? 0xFFFFu - tau_bits : tau_bits + 0x8000u);
-  k.tau = tau == kNothing ? 0u : float_to_key(bits16_float(tau_bits));
+  const uint32_t tau16 = tau == kNothing ? 0u : key16_of_bits(tau_bits);
+  if (q_small != 0) {
+    part_draw_small(rp, v, rank, ctas, base, tau != kPartMags, static_cast<unsigned int>(tie_keep), q_small, {inv_temp, -y_max},
+                    mass_scale_u24(s.u24, kept_mass), reinterpret_cast<unsigned int*>(hist), s, out + row);
+    return;
+  }
+  k.tau = tau == kNothing ? 0u : float_to_key(key16_float<T>(tau16));
   k.tie_keep = tau == kNothing ? 0ull : tie_keep;
   k.q_tau = tau == kNothing ? 0ull : bits16_mass(tau_bits, inv_temp, y_max);
   k.args = {inv_temp, -y_max};
   const int n_sub = ctas * kPartsPerCta;
-  if (warp == 0) {
-    const unsigned long long target = mass_scale_u24(s.u24, kept_mass);
-    const unsigned long long t = lane < n_sub ? s.sub_ties[lane] : 0ull, t0 = warp_incl_u64(t) - t;
-    const unsigned long long left = k.tie_keep > t0 ? k.tie_keep - t0 : 0ull;
-    const unsigned long long m = (lane < n_sub ? s.sub_mass[lane] : 0ull) + (t < left ? t : left) * k.q_tau;
-    const unsigned long long inc = warp_incl_u64(m);
-    const int first = __ffs(static_cast<int>(__ballot_sync(0xffffffffu, inc > target))) - 1;
-    if (lane == first) {
-      s.owner = first;
-      s.target = target - (inc - m);
-      s.ties_before = t0;
-    }
-  }
+  if (warp == 0) part_owner(n_sub, k, mass_scale_u24(s.u24, kept_mass), s);
   __syncthreads();
   const int q = s.owner;
   if (q / kPartsPerCta != rank) return;
@@ -2709,11 +2893,17 @@ sample_parts_kernel(const __nv_bfloat16* __restrict__ logits, long long row_stri
 
 // How many CTAs share a row, 0 for the one of 1024 threads that counts and draws by itself. Counting is bound by the
 // atomics an SM can do, so more CTAs than SMs help only to deal rows that do not fill a whole number of rounds, and what is behind the
-// counting (searches, two barriers of the cluster, the draw: 14 us) is paid by any number of CTAs. us, one CTA per row
-// of 1024 threads / parts, top_p = 0.9: 8 rows of 128256 29.1 / 16.4 (8 CTAs), 30 rows 29.1 / 18.7 (4), 64 rows
-// 29.7 / 25.0 (2), 148 rows 31.3 / 35 (2, with 512 threads); 32000 columns: 8 rows 15.7 / 14.6, 64 rows 15.7 / 17.3. With more
-// rows than SMs that kernel needs another round, parts have them all resident, three per SM: 200 rows of 128256 58.3 / 41.7
-// (2 CTAs), 256 59.0 / 49.1 (1; 2 with 512 threads: 60.8); 32000 columns 30.4 / 23.8 (1), 1000 columns 21.9 / 16.8.
+// counting (searches, two barriers of the cluster, the draw: 14 us) is paid by any number of CTAs. us, top_p = 0.9, the CTA
+// of 1024 threads / one / two / four / eight CTAs:
+//   128256 columns, rows of 9: 29.2 / 31.5 / 22.5 / 18.4 / 16.7; 18: 29.4 / 31.4 / 22.6 / 18.4 / 19.0; 37: 29.4 / 31.8 / 22.9 / 21.8;
+//     64: 30.1 / 36.3 / 25.4 / 23.9; 100: 31.1 / 36.9 / 31.4; 148: 31.5 / 37.3 / 32.0. So as many as leave an eighth of the SMs free, and from
+//     65 rows on the one of 1024 (two would still win up to 74, 30.3 / 25.9).
+//   8 rows, four or eight CTAs only in rows of 28672 columns and more: 16384 13.7 / 14.5 (eight), 24576 14.9 / 15.0, 28672 15.3 / 15.0,
+//     32000 15.7 / 15.0, 49152 18.2 / 15.5. 64 rows, two CTAs only from 49152 on: 32000 15.7 / 16.7, 40960 17.1 / 17.1, 49152 18.5 / 17.7.
+//   More rows than SMs: the CTA of 1024 threads needs another round, parts have them all resident, three per SM. 149 rows of 128256
+//     56.6 / 45.9 / 39.9; 222 58.9 / 47.3 / 41.4; 223, where two CTAs per row are more than three per SM, 58.9 / 47.1 / 54.8; 200 rows of 4096
+//     22.9 / 16.7 / 18.8, 28672 29.4 / 23.3 / 23.3, 49152 36.6 / 29.3 / 27.9, 65536 40.6 / 33.1 / 31.1: two from 65536 on, which leaves
+//     1 to 2 us between 32000 and there.
 inline int part_ctas(int rows, int v, int sms) {
   // a sub-part's vectors are rounded up, its ends have up to seven scalars each
   auto fits = [&](int ctas) { return v / (ctas * kPartsPerCta) + 32 <= kPartMaxElems; };

@@ -230,22 +230,32 @@ def test_sampler_candidates_in_few_places(cuda_device, dtype, vocab, rows):
             assert torch.equal(tok[:3].cpu(), _cpu(val[:3], top_k, top_p, 0.7, 2, top_k)), (name, top_k, top_p)
 
 
-@pytest.mark.parametrize("top_k,top_p,temperature", [(None, 0.9, 1.0), (None, None, 0.7), (2000, 0.95, 1.0), (None, 0.9, 40.0)])
-@pytest.mark.parametrize("vocab,rows", [(31, 150), (49155, 3), (33001, 30), (50003, 74), (8193, 300), (131075, 2), (65541, 180)])
+@pytest.mark.parametrize("top_k,top_p,temperature", [(None, 0.9, 1.0), (None, None, 0.7), (2000, 0.95, 1.0), (None, 0.9, 40.0),
+                                                     (3000, None, 1e-3), (None, 0.6, 1e30)])
+@pytest.mark.parametrize("vocab,rows", [(31, 150), (49155, 3), (33001, 30), (50003, 74), (8193, 300), (131075, 2), (65541, 180),
+                                        (50003, 60), (131000, 230), (131201, 230)])
 def test_sampler_bf16_parts_of_a_row(cuda_device, vocab, rows, top_k, top_p, temperature):
-    """bf16 rows without a small top-k: one to eight CTAs per row, rows that start off a 16-byte boundary, and values
-    inside and outside the magnitudes that are counted at first: plain, far above and below them, next to zero, zeros of
-    both signs, one value throughout, masked three ways, thresholds among negative values."""
+    """bf16 rows without a small top-k: one to eight CTAs per row (on 148 SMs (50003, 74) stays with the one that takes whole
+    rows), rows that start off a 16-byte boundary, counters close to their limit (one value, 131000 columns) and rows that take
+    more CTAs because of it, and values inside and outside the magnitudes that are counted at first: plain, far above and
+    below them, next to zero, zeros of both signs, one value throughout, masked three ways, thresholds among negative values
+    and among values next to zero."""
     g = torch.Generator(device=cuda_device).manual_seed(vocab + rows)
     x = torch.randn(rows, vocab, device=cuda_device, generator=g) * 2
     u = torch.rand(x.shape, device=cuda_device, generator=g)
+    at = torch.arange(vocab, device=cuda_device)
     values = {"plain": x, "negative": x - 20, "above": x * 8 + 3000, "below": x * 8 - 5000, "wide": x * 2000, "tiny": x * 1e-18,
               "few_tiny": torch.where(u < 0.01, x * 1e-18, x), "zeros": torch.where(u < 0.5, 0.0, -0.0),
               "half_zero": torch.where(u < 0.5, 0.0, x), "one_value": torch.full_like(x, 3.0),
               "inf_mask": torch.where(u < 0.99, float("-inf"), x), "lowest": torch.where(u < 0.9, torch.finfo(torch.bfloat16).min, x),
               "mask_1e4": torch.where(u < 0.9, -1e4, x), "nan": torch.where(u < 0.1, float("nan"), x),
               "all_nan": torch.full_like(x, float("nan")), "all_inf": torch.full_like(x, float("-inf")),
-              "plus_inf": torch.where(u > 0.999, float("inf"), x)}
+              "plus_inf": torch.where(u > 0.999, float("inf"), x), "one_tiny": torch.where(at == vocab // 2, 1e-18, x),
+              "half_tiny": torch.where(u < 0.5, x * 1e-18, x), "tiny_above": torch.where(u < 0.5, x.abs() * 1e-18, -x.abs()),
+              "tiny_below": torch.where(u < 0.9, -x.abs() * 1e-12, x), "subnormal": x * 1e-39,
+              "next_to_zero": torch.where(u < 0.3, 0.0, torch.where(u < 0.6, -0.0, x * 10 ** (-40 * u))),
+              "small": x * 1e-6, "late": torch.where(at == vocab - 2, 3e12, x), "minus": -x.abs() - 3e9,
+              "inf_and_nan": torch.where(u < 0.5, float("nan"), torch.where(u < 0.9, float("-inf"), float("inf")))}
     buf = torch.empty(rows * (vocab + 1) + 3, dtype=torch.bfloat16, device=cuda_device)
     some = torch.arange(0, rows, max(1, rows // 3))[:4]
     for name, val in values.items():
