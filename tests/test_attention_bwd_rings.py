@@ -1,15 +1,32 @@
 """The barrier protocol of the attention backward kernel, a persistent CTA that takes one tile after the other with a ring
-for every streamed operand, run through every interleaving on the CPU: as in ``test_attention_bwd_barriers`` a wait is for
-the parity of a phase, so every reachable state must let somebody move, and no wait may end before its phase is over."""
+for every streamed operand, run through every interleaving on the CPU. A CTA of its own per tile is the case of one tile.
+
+An mbarrier is waited for by the parity of a phase, so a waiter that is overtaken by two phases sees the parity it started
+from and waits on. The model holds what each party of a CTA waits for and arrives at; how many barriers of a kind there are is
+read from the kernel's source (barrier ``j % n`` serves number ``j``, with parity ``j / n``). Every reachable state must let
+somebody move, and no wait may end before the phase it is meant for.
+"""
+import os
+import re
+
 import pytest
 
-import test_attention_bwd_barriers as model
+SRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "csrc", "sm100", "attention_bwd.cu")
+WARPS = 2       # element-wise warps: two are enough for one to be ahead of the other
 
-WARPS = 2
+
+def _barriers(struct):
+    with open(SRC) as f:
+        body = re.search(r"struct %s \{(.*?)\n\};" % struct, f.read(), re.S).group(1)
+    out = {}
+    for decl in re.findall(r"uint64_t ([^;]+);", body):
+        for name, n in re.findall(r"(\w+)(?:\[(\d)\])?", decl):
+            out[name] = int(n or 1)
+    return out
 
 
 def _bars(kernel):
-    return dict(model._barriers(kernel), item_full=2, item_empty=2, join=1 << 20)   # the named barrier has no parity to miss
+    return dict(_barriers(kernel), item_full=2, item_empty=2, join=1 << 20)   # the named barrier has no parity to miss
 
 
 def _programs(kernel, sizes, bars):
