@@ -51,7 +51,7 @@ def main():
 
         x = (torch.randn(args.rows, args.vocab, device=dev, generator=g) * 2).to(torch.bfloat16)
         fn = lambda: sample(x, top_k=50, top_p=0.9, temperature=0.7, seed=1, step=0)  # noqa: E731
-    elif args.op == "sampling_top_p":       # no top-k: sample_general_kernel
+    elif args.op == "sampling_top_p":       # no top-k: sample_parts_kernel for more rows than SMs, else sample_general_kernel
         from kernel_align_b200.ops.sampling import sample
 
         x = (torch.randn(args.rows, args.vocab, device=dev, generator=g) * 2).to(torch.bfloat16)

@@ -2,12 +2,13 @@
 //
 //   delta[b, h, i] = sum_d dO[i, d] * O[i, d]
 //   P  = exp(scale * Q K^T - lse),   dP = dO V^T,   dS = P * (dP - delta) * scale
-//   dQ = dS K            bwd_dq: per (sequence, q head, q tile) a CTA
-//                        walks the KV tiles in increasing order, dQ accumulates in TMEM
-//   dV = P^T dO, dK = dS^T Q   bwd_dkv: per (sequence, kv head, kv tile) a CTA
-//                        walks (q head of the group, q tile) in a fixed order; it
+//   dQ = dS K            bwd_dq: a dQ tile per (sequence, q head, q tile), made by one CTA that
+//                        walks the KV tiles in increasing order; dQ accumulates in TMEM
+//   dV = P^T dO, dK = dS^T Q   bwd_dkv: a dK / dV tile per (sequence, kv head, kv tile), made by one CTA
+//                        that walks (q head of the group, q tile) in a fixed order; it
 //                        works on S^T = K Q^T so that its threads own KV rows
-// Which CTA takes which of these tiles, and when, is left to a counter; a tile's result does not depend on it.
+// One kernel makes both kinds of tiles. With tiles enough a CTA per SM takes one after the other from a counter, with few of
+// them each has a CTA of its own; a tile's result does not depend on it.
 //
 // All five products are tcgen05.mma 128 x 128 tiles; operands that are needed "transposed"
 // (K and Q as [d, rows], dO as [d, rows]) are read through MN-major descriptors from the same
@@ -126,16 +127,17 @@ __device__ __forceinline__ constexpr uint64_t mnstep(int kk) { return (kk * 2048
 __device__ __forceinline__ constexpr uint32_t tcol(int kk) { return (kk >> 1) * kPartCols + (kk & 1) * 8; }
 
 // ------------------------------------------------------------------------------------------------
-// Both kernels overlap the tensor core with the element-wise work: the operand of the next
-// iteration is in a second shared-memory stage, the next S and dP products are issued as soon as
+// Both kinds of tiles overlap the tensor core with the element-wise work: the operands of the next
+// iteration are in other stages of their rings, the next S and dP products are issued as soon as
 // their TMEM columns have been read, and the 16-bit operand that comes out of S goes back to TMEM
 // over the columns of S (the A operand of the product that follows), which leaves shared memory
 // to the loaded tiles. Sixteen warps share a tile (eight issued in a quarter of the cycles: with two
 // warps per scheduler nothing covers the TMEM loads and barriers), and tiles that need no mask
 // run a loop of their own, without comparisons.
 // One iteration is three products of 512 cycles (dQ) or four (dK / dV); with a single stage and
-// everything in sequence it took about 9000 cycles. B = 2, L = 4000, 32 / 8 heads, causal:
-// dQ 891 -> 500 us, dK / dV 1466 -> 530 us; B = 8, L = 512: dQ 114 -> 66 us, dK / dV 173 -> 62 us.
+// everything in sequence it took about 9000 cycles. B = 2, L = 4000, 32 / 8 heads, causal, dQ and dK / dV as launches of their
+// own: 891 and 1466 us with a single stage, 500 and 530 so, 902 for both in one launch with a ring for every operand; B = 8,
+// L = 512: 114 and 173, 66 and 62, 115.
 // ------------------------------------------------------------------------------------------------
 // The loading thread takes the next tile of its kind and tells the others, a tile ahead of them.
 struct Items {
@@ -185,11 +187,12 @@ struct CtlDq {
 };
 
 // ------------------------------------------------------------------------------------------------
-// dQ kernel. TMEM: S (two buffers), dP, dQ. Shared memory: Q, dO, three stages of K, two of V.
+// dQ tiles. TMEM: S (two buffers), dP, dQ. Shared memory: Q, dO, three stages of K, two of V.
 // An SM gets about 85 GB/s, so a pair of tiles takes 1400 cycles and the latency on top. With two stages of (K, V)
 // that were handed back together, behind dQ(j), the load of tile j + 2 and then S(j + 2) followed one another in the time in which the warps
 // took tile j + 1, and an iteration was 3800 cycles; V is handed back by dP(j) now and K has a third stage: 2770
-// cycles, what the products of one CTA take to issue (S 590, dP 660, dQ 960: shared memory).
+// cycles, all of them the issuing thread's: S 590, dP 660 and dQ 960 (512 each at the tensor core's rate) and 560 for its waits, 130
+// to 200 for a barrier that is ready and 75 until the tensor core, whose queue has run empty, starts again.
 // ------------------------------------------------------------------------------------------------
 constexpr int kKStages = 3;
 struct DqTile {
@@ -429,7 +432,7 @@ bwd_dq(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v
 }
 
 // ------------------------------------------------------------------------------------------------
-// dK / dV kernel. TMEM: S^T (then P^T as bf16 over it), dP^T, dV, dK. Shared memory: K, V, two
+// dK / dV tiles. TMEM: S^T (then P^T as bf16 over it), dP^T, dV, dK. Shared memory: K, V, two
 // stages of (Q, dO), dS^T.
 // ------------------------------------------------------------------------------------------------
 // Does the condition hold for any element-wise thread? A barrier of all of them.

@@ -1959,8 +1959,8 @@ sample_general_kernel(const T* __restrict__ logits, long long row_stride, int v,
 
 // ---- bf16 rows: histograms per part of the row -------------------------------------------------
 // What bounds the general path is one shared-memory atomic per element: a histogram of 148 rows of
-// 128256 columns, one row per SM, takes 12.5 us whatever the counters' width (5.9 cycles per warp, the
-// conflicts of 32 random banks), and nothing else has to be done per element:
+// 128256 columns, one row per SM, takes 14.5 us whatever the counters' width, 12.5 of them atomics (5.9 cycles per
+// warp, the conflicts of 32 random banks), and nothing else has to be done per element:
 //   * A row is cut into C * 2 contiguous sub-parts, C CTAs (a cluster) with a histogram for each of their
 //     two. The kept mass of a sub-part follows from its histogram, so only the one that holds the target is
 //     read again by the draw (a sixteenth to a half of the row; the draw over whole rows took as long as the counting).
