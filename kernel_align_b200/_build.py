@@ -1,9 +1,11 @@
-"""In-tree native build: nvcc for the sm_100a kernels, g++ for the CPU oracle library and for the
+"""Native build, in-tree: nvcc for the sm_100a kernels, g++ for the CPU oracle library and for the
 operators that are C++ autograd nodes.
 
 The first two are plain shared objects with ``extern "C"`` entry points, loaded through
 ``ctypes``, the third is an extension module against the installed torch; they sit next to the package so that a
 built tree can be copied to a GPU host as is. A content hash of the sources and flags decides whether a rebuild is needed.
+An installed package carries the built libraries and the sources of the third alone, which ``python -m kernel_align_b200._build``
+compiles there if the package was built without a torch, or beside another one.
 """
 from __future__ import annotations
 
@@ -142,15 +144,20 @@ def _cuda_include() -> Path | None:
     return None
 
 
-def build_torch(force: bool = False) -> Path | None:
+def build_torch(force: bool = False, installed: bool = False) -> Path | None:
     """Compile ``csrc/torch/*.cpp`` into the extension module ``_ka_torch.*.so`` (C++ autograd nodes). None where that is
-    not possible (:func:`torch_missing`): the operators then reach the kernels from Python."""
+    not possible (:func:`torch_missing`): the operators then reach the kernels from Python. An installed package compiles
+    nothing unless ``installed`` is set: it takes the module that it was built with, if that is one for this torch."""
     out = torch_lib()
     if out is None:
         return None
     srcs = sorted((CSRC / "torch").glob("*.cpp"))
-    if not srcs:             # an installed wheel carries the built module, not the sources
-        return out if out.exists() else None
+    if not srcs:
+        if not installed or out.exists():
+            return out if out.exists() else None
+        srcs = sorted((LIB_DIR.parent / "_src").glob("*.cpp"))
+        if not srcs:
+            return None
     import torch
 
     inc, lib = Path(torch.__file__).parent / "include", Path(torch.__file__).parent / "lib"
@@ -210,7 +217,7 @@ def sanitizer_runtime() -> str | None:
 def build_all(force: bool = False, verbose: bool = False) -> None:
     build_cpu(force)
     build_cuda(force, verbose)
-    build_torch(force)
+    build_torch(force, installed=True)
 
 
 if __name__ == "__main__":

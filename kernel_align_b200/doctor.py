@@ -85,7 +85,7 @@ def main(argv=None) -> int:
         print(f"kernel_align_b200 {info['version']}  (torch {info['torch']}, CUDA runtime {info['cuda_runtime']})")
         print(f"  sm_100a kernel library : {info['libka_sm100'] or 'not built'}   (nvcc: {info['nvcc'] or 'not found'})")
         print(f"  C++ CPU library        : {info['libka_cpu'] or 'not built'}   (g++: {info['cxx'] or 'not found'})")
-        print(f"  autograd nodes (C++)   : {info['ka_torch'] or 'not built: the Python ones are used'}   "
+        print(f"  autograd nodes (C++)   : {info['ka_torch'] or 'not built: the Python ones are used; python -m kernel_align_b200._build makes them'}   "
               f"(g++: {info['cxx'] or 'not found'}{'; cannot be built: ' + info['ka_torch_missing'] if info['ka_torch_missing'] else ''})")
         if info["gpus"]:
             for gpu in info["gpus"]:

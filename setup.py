@@ -5,8 +5,10 @@
 ``kernel_align_b200/_lib`` through ``kernel_align_b200/_build.py``; every sub-package is a real
 package (the reference's setup.py:6 silently dropped four of its six).
 """
+import glob
 import importlib.util
 import os
+import shutil
 
 from setuptools import Command, find_packages, setup
 from setuptools.command.build_py import build_py
@@ -39,6 +41,11 @@ class BuildPyWithNative(build_py):
     def run(self):
         _native_build()
         super().run()
+        # the extension module is made for one torch: its sources go along, to be compiled beside another one
+        out = os.path.join(self.build_lib, "kernel_align_b200", "_src")
+        os.makedirs(out, exist_ok=True)
+        for src in glob.glob(os.path.join(HERE, "csrc", "torch", "*.cpp")):
+            shutil.copy(src, out)
 
 
 setup(

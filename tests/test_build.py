@@ -55,6 +55,27 @@ def test_a_module_of_another_torch_or_of_other_sources_is_not_loaded(elsewhere, 
     assert _build.build_torch() is None
 
 
+def test_an_installed_package_compiles_the_module_when_it_is_told_to(tmp_path, monkeypatch):
+    root = tmp_path / "site"
+    package = root / "kernel_align_b200"
+    (package / "_src").mkdir(parents=True)
+    (package / "_src" / "node.cpp").write_text("")
+    for name, value in (("ROOT", root), ("CSRC", root / "csrc"), ("LIB_DIR", package / "_lib")):
+        monkeypatch.setattr(_build, name, value)
+    compiled = []
+
+    def run(cmd):
+        compiled.append(cmd)
+        with open(cmd[cmd.index("-o") + 1], "w") as f:
+            f.write("module")
+
+    monkeypatch.setattr(_build, "_run", run)
+    assert _build.build_torch() is None and not compiled                  # as the first call of an operator does
+    path = _build.build_torch(installed=True)
+    assert path.read_text() == "module" and str(package / "_src" / "node.cpp") in compiled[0]
+    assert _build.build_torch() == path and _build.build_torch(installed=True) == path and len(compiled) == 1
+
+
 def test_ranks_that_build_at_once_find_a_whole_module(elsewhere, monkeypatch):
     """The compiler writes beside the module, which is put in place when it is whole."""
     seen = []
@@ -73,6 +94,6 @@ def test_ranks_that_build_at_once_find_a_whole_module(elsewhere, monkeypatch):
 def test_the_kernel_library_is_built_before_the_module(monkeypatch):
     order = []
     for name in ("build_cpu", "build_cuda", "build_torch"):
-        monkeypatch.setattr(_build, name, lambda *a, name=name: order.append(name))
+        monkeypatch.setattr(_build, name, lambda *a, name=name, **k: order.append(name))
     _build.build_all()
     assert order == ["build_cpu", "build_cuda", "build_torch"]
